@@ -15,9 +15,11 @@
 #include <string>
 #include <vector>
 
+#include "engine_mat.h"
 #include "fnx_common.cuh"
 #include "iq3s_tile.h"
-#include "mmv_core.cuh"
+#include "nat_image.cuh"
+#include "nat_tile.h"
 
 namespace fnxb {
 
@@ -50,11 +52,24 @@ static Nccl* nccl() {
     return n.lib && n.GetUniqueId && n.CommInitRank && n.AllReduce ? &n : nullptr;
 }
 
+// A weight matrix (or a stack of n of them, one per local expert).  The engine holds it in its own layout (nat_tile.h).  A caller that asks
+// for the tensor by name gets it in the interchange layout (iq3s_tile.h): it is converted then, and because that memory may be
+// written afterwards, it is what the windows and prompts read from then on (the operators of the C ABI).
+struct Mat {
+    size_t rows = 0, cols = 0;
+    int n = 1;
+    bool gate_up = false;        // [gate; up] stacked: the halves of a native tile are theirs
+    uint8_t *nat = nullptr, *tiles = nullptr;   // one of the two
+    Mat* with = nullptr;         // the matrix that the same launches read (routed and shared experts): converted together
+    size_t nat_stride() const { return nat_bytes(rows, cols); }
+    size_t tile_stride() const { return iq3s_bytes(rows, cols); }
+};
+
 struct LayerW {
     bool attn = false;
     float *norm1 = nullptr, *norm2 = nullptr;
     // mixer
-    uint8_t *w_in = nullptr, *w_out = nullptr;   // attention: [q|gate per head; k; v] x H and H x (nq hd); DeltaNet: [q|k|v|z|alpha|beta] x H and H x (nv hs)
+    Mat w_in, w_out;   // attention: [q|gate per head; k; v] x H and H x (nq hd); DeltaNet: [q|k|v|z|alpha|beta] x H and H x (nv hs)
     int in_rows = 0;
     float *qn = nullptr, *kn = nullptr;          // attention head norms
     __half *kc = nullptr, *vc = nullptr;         // [n_seq][cache_rows][nkv hd]
@@ -62,7 +77,7 @@ struct LayerW {
     float *S_pool = nullptr, *hist_pool = nullptr;   // [n_seq][NS]...
     // MoE
     float* wr = nullptr;
-    uint8_t *wgu = nullptr, *wdn = nullptr, *wsh_gu = nullptr, *wsh_dn = nullptr;
+    Mat wgu, wdn, wsh_gu, wsh_dn;
 };
 
 struct SeqState {
@@ -88,11 +103,11 @@ struct fnx_engine {
     std::vector<LayerW> layers;
     LayerW mtp;
     float *mtp_hnorm = nullptr, *mtp_enorm = nullptr, *mtp_onorm = nullptr, *out_norm = nullptr;
-    uint8_t *mtp_fc_hid = nullptr, *mtp_fc_emb = nullptr, *head = nullptr;
+    Mat mtp_fc_hid, mtp_fc_emb, head;
+    std::map<std::string, Mat*> mats;
     __half* embed = nullptr;
     std::vector<SeqState> seqs;
     int NS = 0, cache_rows = 0, E_local = 0, e_lo = 0, e_hi = 0;
-    size_t gu_bytes = 0, dn_bytes = 0;
     // window buffers
     float *R = nullptr, *Rm = nullptr, *Rsrc = nullptr, *Emb = nullptr, *proj = nullptr, *mix = nullptr, *logits = nullptr;
     float *rlogits = nullptr, *topw = nullptr, *hbuf = nullptr, *part = nullptr, *moe_out = nullptr, *best_v = nullptr, *cand_v = nullptr;
@@ -110,9 +125,9 @@ struct fnx_engine {
     fnx_job* jobs = nullptr;
     unsigned* err = nullptr;
     void* att_scratch = nullptr;
-    // the image of the new residual rows that the combine leaves for the next projection (single rank; one per FNX_DENSE_ROWS rows)
-    uint8_t* d_img = nullptr;
-    bool use_img = true;
+    // images of the window's rows (nat_image.cuh): of the residual rows for the next projection, of the mixers' output rows, of the MoE
+    // block's input rows
+    uint8_t *img_r = nullptr, *img_m = nullptr, *img_x = nullptr;
     // the prompt pass (fnx_engine_prompt): buffers for a chunk of prompt_chunk rows, made at its first call
     int prompt_chunk = 40960;
     float *pR = nullptr, *pproj = nullptr, *pmix = nullptr, *plogits = nullptr, *ptopw = nullptr;
@@ -123,7 +138,7 @@ struct fnx_engine {
     void *p_router_scratch = nullptr, *p_moe_scratch = nullptr, *p_dense_scratch = nullptr, *p_gdn_scratch = nullptr, *p_attn_scratch = nullptr;
     // the draft layer's own head over a draft vocabulary (config draft_vocab > 0): dvn rows, row -> token id in d_dvocab;
     // otherwise the main head and no map
-    uint8_t* mtp_head = nullptr;
+    Mat mtp_head;
     int* d_dvocab = nullptr;
     int dvn = 0;
     int *h_stage = nullptr;      // pinned host staging
@@ -179,6 +194,47 @@ static int dalloc(fnx_engine* e, T** p, size_t count, const char* name = nullptr
     e->bytes += bytes;
     *p = (T*) q;
     if (name) e->tensors[name] = {q, bytes};
+    return FNX_OK;
+}
+
+static int alloc_mat(fnx_engine* e, Mat& m, size_t rows, size_t cols, const std::string& name, int n = 1, bool gate_up = false) {
+    m.rows = rows; m.cols = cols; m.n = n; m.gate_up = gate_up;
+    FNX_TRY(dalloc(e, &m.nat, m.nat_stride() * n));
+    e->mats[name] = &m;
+    return FNX_OK;
+}
+static int put_rows(Mat& m, int index, size_t row0, size_t n, const uint8_t* ggml, cudaStream_t st) {
+    if (m.nat) return nat_pack(ggml, m.nat + (size_t) index * m.nat_stride(), m.rows, row0, n, m.cols, m.gate_up, st);
+    return fnx_iq3s_retile(ggml, m.tiles + (size_t) index * m.tile_stride() + iq3s_bytes(row0, m.cols), n, m.cols, st);
+}
+int engine_put_matrix(fnx_engine* e, const std::string& name, int index, size_t rows, size_t cols, const uint8_t* ggml, cudaStream_t st) {
+    auto it = e->mats.find(name);
+    if (it == e->mats.end()) return fail(FNX_E_STATE, "load: the engine has no matrix %s", name.c_str());
+    Mat& m = *it->second;
+    FNX_REQUIRE(rows == m.rows && cols == m.cols && index >= 0 && index < m.n, "load: engine matrix %s is %d of %zu x %zu, the loader fills number %d of %zu x %zu", name.c_str(),
+                m.n, m.rows, m.cols, index, rows, cols);
+    return put_rows(m, index, 0, rows, ggml, st);
+}
+static void dfree(fnx_engine* e, void* p, size_t bytes) {
+    for (auto& q : e->owned)
+        if (q == p) {
+            cudaFree(p);
+            q = e->owned.back();
+            e->owned.pop_back();
+            e->bytes -= bytes;
+            return;
+        }
+}
+static int to_tiles(fnx_engine* e, Mat& m) {
+    if (!m.nat) return FNX_OK;
+    uint8_t* t = nullptr;
+    FNX_TRY(dalloc(e, &t, m.tile_stride() * m.n));
+    FNX_CUDA_OK(cudaDeviceSynchronize());   // (the zeroing above runs on another stream than the engine's)
+    for (int i = 0; i < m.n; ++i) FNX_TRY(nat_unpack(m.nat + (size_t) i * m.nat_stride(), t + (size_t) i * m.tile_stride(), m.rows, m.cols, m.gate_up, e->st));
+    FNX_CUDA_OK(cudaStreamSynchronize(e->st));
+    dfree(e, m.nat, m.nat_stride() * m.n);
+    m.nat = nullptr;
+    m.tiles = t;
     return FNX_OK;
 }
 
@@ -339,6 +395,15 @@ __global__ void k_fill_dvocab(int* map, int dv, int V) {
     if (r < dv) map[r] = (int) ((long long) r * V / dv);
 }
 
+// moe_prefill.cu, moe_route.cu: the prompt products and the combine over either weight layout / with the next projection's image
+int prompt_dense(const void* W, bool nat, int rows, int cols, const float* x, int T, const float* norm_w, float eps, float* y, int ldy, int accumulate, void* scratch,
+                 unsigned* err, cudaStream_t st);
+int prompt_moe(const void* Wgu, size_t gu_stride, const void* Wsh_gu, bool gu_nat, const void* Wdn, size_t dn_stride, const void* Wsh_dn, bool dn_nat, int e_base, int E,
+               int K, int e_lo, int e_hi, int add_shared, const int* topi, const float* topw, const float* logits, const float* x, const float* norm_w, float eps, int T,
+               int H, int F, float* out, int accumulate, void* scratch, unsigned* err, cudaStream_t st);
+int moe_combine_nat(const float* part, const int* topi, const float* topw, const float* logits, int T, int E, int H, int K, float* R, uint8_t* img, const float* img_norm_w,
+                    cudaStream_t st);
+
 struct Dims {
     int H, E, K, F, nq, nkv, hd, nrot, nk, nv, hs, V, MAXR, q_rows, kv_rows, attn_in, gdn_ch, gdn_in, P;
 };
@@ -357,17 +422,16 @@ static Dims dims(const fnx_model_config& c) {
     return d;
 }
 
-// an IQ3_S tile matrix of N(0, sigma) weights: generate, quantise, re-tile, in chunks of whole 16-row tiles
-static int synth_iq3s(fnx_engine* e, uint8_t* dst, size_t rows, size_t cols, float sigma, uint64_t seed, uint32_t stream_id, float* tmp_f,
-                      uint8_t* tmp_g, size_t tmp_weights) {
-    size_t chunk_rows = tmp_weights / cols / 16 * 16;
-    if (chunk_rows == 0) return fail(FNX_E_ARG, "synthetic init: staging buffer too small for %zu columns", cols);
+// matrix `index` of m from N(0, sigma) weights: generate, quantise, lay out, in chunks of whole 16-row tiles
+static int synth_iq3s(fnx_engine* e, Mat& m, int index, float sigma, uint64_t seed, uint32_t stream_id, float* tmp_f, uint8_t* tmp_g, size_t tmp_weights) {
+    size_t chunk_rows = tmp_weights / m.cols / 16 * 16;
+    if (chunk_rows == 0) return fail(FNX_E_ARG, "synthetic init: staging buffer too small for %zu columns", m.cols);
     uint32_t sub = 0;
-    for (size_t r0 = 0; r0 < rows; r0 += chunk_rows, ++sub) {
-        const size_t nr = rows - r0 < chunk_rows ? rows - r0 : chunk_rows;
-        FNX_TRY(fnx_fill_normal(tmp_f, nr * cols, sigma, seed, stream_id + sub, e->st));
-        FNX_TRY(fnx_iq3s_quantize(tmp_f, tmp_g, nr * cols, e->st));
-        FNX_TRY(fnx_iq3s_retile(tmp_g, dst + iq3s_bytes(r0, cols), nr, cols, e->st));
+    for (size_t r0 = 0; r0 < m.rows; r0 += chunk_rows, ++sub) {
+        const size_t nr = m.rows - r0 < chunk_rows ? m.rows - r0 : chunk_rows;
+        FNX_TRY(fnx_fill_normal(tmp_f, nr * m.cols, sigma, seed, stream_id + sub, e->st));
+        FNX_TRY(fnx_iq3s_quantize(tmp_f, tmp_g, nr * m.cols, e->st));
+        FNX_TRY(put_rows(m, index, r0, nr, tmp_g, e->st));
     }
     return FNX_OK;
 }
@@ -380,16 +444,16 @@ static int alloc_layer(fnx_engine* e, LayerW& L, bool attn, const std::string& p
     FNX_TRY(dalloc(e, &L.norm2, d.H, (pre + "norm2").c_str()));
     if (attn) {
         L.in_rows = d.attn_in;
-        FNX_TRY(dalloc(e, &L.w_in, iq3s_bytes(d.attn_in, d.H), (pre + "w_in").c_str()));
-        FNX_TRY(dalloc(e, &L.w_out, iq3s_bytes(d.H, d.nq * d.hd), (pre + "w_out").c_str()));
+        FNX_TRY(alloc_mat(e, L.w_in, d.attn_in, d.H, pre + "w_in"));
+        FNX_TRY(alloc_mat(e, L.w_out, d.H, d.nq * d.hd, pre + "w_out"));
         FNX_TRY(dalloc(e, &L.qn, d.hd, (pre + "q_norm").c_str()));
         FNX_TRY(dalloc(e, &L.kn, d.hd, (pre + "k_norm").c_str()));
         FNX_TRY(dalloc(e, &L.kc, (size_t) ns * e->cache_rows * d.kv_rows, (pre + "k_cache").c_str()));
         FNX_TRY(dalloc(e, &L.vc, (size_t) ns * e->cache_rows * d.kv_rows, (pre + "v_cache").c_str()));
     } else {
         L.in_rows = d.gdn_in;
-        FNX_TRY(dalloc(e, &L.w_in, iq3s_bytes(d.gdn_in, d.H), (pre + "w_in").c_str()));
-        FNX_TRY(dalloc(e, &L.w_out, iq3s_bytes(d.H, d.nv * d.hs), (pre + "w_out").c_str()));
+        FNX_TRY(alloc_mat(e, L.w_in, d.gdn_in, d.H, pre + "w_in"));
+        FNX_TRY(alloc_mat(e, L.w_out, d.H, d.nv * d.hs, pre + "w_out"));
         FNX_TRY(dalloc(e, &L.convw, (size_t) d.gdn_ch * 4, (pre + "conv_w").c_str()));
         FNX_TRY(dalloc(e, &L.dt, d.nv, (pre + "dt").c_str()));
         FNX_TRY(dalloc(e, &L.a, d.nv, (pre + "a").c_str()));
@@ -398,10 +462,12 @@ static int alloc_layer(fnx_engine* e, LayerW& L, bool attn, const std::string& p
         FNX_TRY(dalloc(e, &L.hist_pool, (size_t) ns * e->NS * 3 * d.gdn_ch, (pre + "conv_hist").c_str()));
     }
     FNX_TRY(dalloc(e, &L.wr, (size_t) (d.E + 1) * d.H, (pre + "router").c_str()));
-    FNX_TRY(dalloc(e, &L.wgu, e->gu_bytes * e->E_local, (pre + "experts_gu").c_str()));
-    FNX_TRY(dalloc(e, &L.wdn, e->dn_bytes * e->E_local, (pre + "experts_dn").c_str()));
-    FNX_TRY(dalloc(e, &L.wsh_gu, e->gu_bytes, (pre + "shared_gu").c_str()));
-    FNX_TRY(dalloc(e, &L.wsh_dn, e->dn_bytes, (pre + "shared_dn").c_str()));
+    FNX_TRY(alloc_mat(e, L.wgu, 2 * d.F, d.H, pre + "experts_gu", e->E_local, true));
+    FNX_TRY(alloc_mat(e, L.wdn, d.H, d.F, pre + "experts_dn", e->E_local));
+    FNX_TRY(alloc_mat(e, L.wsh_gu, 2 * d.F, d.H, pre + "shared_gu", 1, true));
+    FNX_TRY(alloc_mat(e, L.wsh_dn, d.H, d.F, pre + "shared_dn"));
+    L.wgu.with = &L.wsh_gu; L.wsh_gu.with = &L.wgu;
+    L.wdn.with = &L.wsh_dn; L.wsh_dn.with = &L.wdn;
     return FNX_OK;
 }
 
@@ -416,13 +482,13 @@ static int init_layer(fnx_engine* e, LayerW& L, int li, uint64_t seed, float sig
     auto sid = [&](int kind, int ex) { return (uint32_t) (((li * 16 + kind) << 12) | ex); };
     FNX_TRY(fill_const(e, L.norm1, d.H, 1.0f));
     FNX_TRY(fill_const(e, L.norm2, d.H, 1.0f));
-    FNX_TRY(synth_iq3s(e, L.w_in, L.in_rows, d.H, sigma, seed, sid(0, 0), tf, tg, tw));
+    FNX_TRY(synth_iq3s(e, L.w_in, 0, sigma, seed, sid(0, 0), tf, tg, tw));
     if (L.attn) {
-        FNX_TRY(synth_iq3s(e, L.w_out, d.H, d.nq * d.hd, sigma, seed, sid(1, 0), tf, tg, tw));
+        FNX_TRY(synth_iq3s(e, L.w_out, 0, sigma, seed, sid(1, 0), tf, tg, tw));
         FNX_TRY(fill_const(e, L.qn, d.hd, 1.0f));
         FNX_TRY(fill_const(e, L.kn, d.hd, 1.0f));
     } else {
-        FNX_TRY(synth_iq3s(e, L.w_out, d.H, d.nv * d.hs, sigma, seed, sid(1, 0), tf, tg, tw));
+        FNX_TRY(synth_iq3s(e, L.w_out, 0, sigma, seed, sid(1, 0), tf, tg, tw));
         FNX_TRY(fnx_fill_normal(L.convw, (size_t) d.gdn_ch * 4, 0.5f, seed, sid(2, 0), e->st));
         k_gdn_params<<<(d.nv + 63) / 64, 64, 0, e->st>>>(L.dt, L.a, d.nv);
         FNX_LAUNCH_OK("gdn_params");
@@ -431,11 +497,11 @@ static int init_layer(fnx_engine* e, LayerW& L, int li, uint64_t seed, float sig
     FNX_TRY(fnx_fill_normal(L.wr, (size_t) (d.E + 1) * d.H, sigma, seed, sid(3, 0), e->st));
     for (int x = 0; x < e->E_local; ++x) {
         const int ge = e->e_lo + x;   // the global expert: every rank draws the same weights for it
-        FNX_TRY(synth_iq3s(e, L.wgu + (size_t) x * e->gu_bytes, 2 * d.F, d.H, sigma, seed, sid(4, ge), tf, tg, tw));
-        FNX_TRY(synth_iq3s(e, L.wdn + (size_t) x * e->dn_bytes, d.H, d.F, sigma, seed, sid(5, ge), tf, tg, tw));
+        FNX_TRY(synth_iq3s(e, L.wgu, x, sigma, seed, sid(4, ge), tf, tg, tw));
+        FNX_TRY(synth_iq3s(e, L.wdn, x, sigma, seed, sid(5, ge), tf, tg, tw));
     }
-    FNX_TRY(synth_iq3s(e, L.wsh_gu, 2 * d.F, d.H, sigma, seed, sid(6, 0), tf, tg, tw));
-    FNX_TRY(synth_iq3s(e, L.wsh_dn, d.H, d.F, sigma, seed, sid(7, 0), tf, tg, tw));
+    FNX_TRY(synth_iq3s(e, L.wsh_gu, 0, sigma, seed, sid(6, 0), tf, tg, tw));
+    FNX_TRY(synth_iq3s(e, L.wsh_dn, 0, sigma, seed, sid(7, 0), tf, tg, tw));
     return FNX_OK;
 }
 
@@ -450,8 +516,7 @@ __global__ void __launch_bounds__(32) k_ep_exchange(const float* __restrict__ pa
                                                     float* const* __restrict__ peer_x, unsigned* const* __restrict__ peer_flag, size_t flag_off,
                                                     const float* __restrict__ xbuf, const unsigned* __restrict__ xflag, int rank, int R, int maxr,
                                                     float* __restrict__ out, unsigned* __restrict__ seqs, unsigned* __restrict__ err,
-                                                    unsigned wait_limit, uint8_t* __restrict__ img_out, const float* __restrict__ img_norm_w,
-                                                    size_t img_stride) {
+                                                    unsigned wait_limit, uint8_t* __restrict__ img_out, const float* __restrict__ img_norm_w) {
     const int blk = blockIdx.x, t = blockIdx.y, lane = threadIdx.x, KB = H / 256;
     const int nblk = gridDim.x * gridDim.y, bid = t * gridDim.x + blk;
     const size_t col = (size_t) blk * 256 + lane * 8;
@@ -498,17 +563,9 @@ __global__ void __launch_bounds__(32) k_ep_exchange(const float* __restrict__ pa
     const bool all = __all_sync(0xffffffffu, mine);
     if (!all && lane == 0) atomicOr(err, (unsigned) FNX_ERR_TIMEOUT);
     if (all) {
-        QuantTask q[QUANT_BATCH];
-        float v[QUANT_BATCH][8], nw[QUANT_BATCH][8];
-#pragma unroll
-        for (int j = 0; j < QUANT_BATCH; ++j) {
-            q[j].src = nullptr;
-            q[j].t = q[j].blk = 0;
-        }
-        q[0].src = out + (size_t) t * H + (size_t) blk * 256;
-        q[0].t = t % FNX_DENSE_ROWS;
-        q[0].blk = blk;
-        quant_fetch(q[0], img_out ? img_norm_w : nullptr, lane, v[0], nw[0]);
+        float* dst = out + (size_t) t * H + col;
+        const float4 o0 = *reinterpret_cast<const float4*>(dst), o1 = *reinterpret_cast<const float4*>(dst + 4);
+        float v[8] = {o0.x, o0.y, o0.z, o0.w, o1.x, o1.y, o1.z, o1.w};
         float a[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) a[i] = 0.f;
@@ -526,26 +583,12 @@ __global__ void __launch_bounds__(32) k_ep_exchange(const float* __restrict__ pa
             a[4] += g * a1.x; a[5] += g * a1.y; a[6] += g * a1.z; a[7] += g * a1.w;
         }
 #pragma unroll
-        for (int i = 0; i < 8; ++i) v[0][i] += a[i];
-        float* dst = out + (size_t) t * H + col;
-        *reinterpret_cast<float4*>(dst) = make_float4(v[0][0], v[0][1], v[0][2], v[0][3]);
-        *reinterpret_cast<float4*>(dst + 4) = make_float4(v[0][4], v[0][5], v[0][6], v[0][7]);
+        for (int i = 0; i < 8; ++i) v[i] += a[i];
+        *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+        *reinterpret_cast<float4*>(dst + 4) = make_float4(v[4], v[5], v[6], v[7]);
         if (img_out) {
-            const int t0 = t - t % FNX_DENSE_ROWS, nt = min((int) FNX_DENSE_ROWS, T - t0), NG = (nt + 3) / 4;
-            uint2* cells = reinterpret_cast<uint2*>(img_out + (size_t) (t0 / FNX_DENSE_ROWS) * img_stride);
-            float* scales = reinterpret_cast<float*>(cells + (size_t) NG * (H / 32) * 32);
-            float* rs = scales + (size_t) NG * KB * 8;
-            quant_finish(q, v, nw, H, img_norm_w, cells, scales, rs, lane);
-            if (t == t0 + nt - 1)
-                for (int td = nt; td < 4 * NG; ++td) {
-                    const int ng = td >> 2, n = td & 3;
-                    for (int i = lane; i < 64; i += 32) {
-                        const int sbG = blk * 8 + (i >> 3), lvl = (i >> 2) & 1, qq = i & 3;
-                        cells[((size_t) (ng * (H / 32) + sbG) * 8 + n + 4 * lvl) * 4 + qq] = make_uint2(0u, 0u);
-                    }
-                    if (lane < 2) scales[(size_t) (ng * KB + blk) * 8 + n + 4 * lane] = 0.f;
-                    if (lane == 2) rs[td * 16 + blk] = 0.f;
-                }
+            const float ss = ni_norm8(v, img_norm_w + col);
+            ni_quant(img_out, KB, v, ss, t, blk, lane);
         }
     }
     __syncwarp();
@@ -628,29 +671,35 @@ __global__ void k_dp_recv(const float* __restrict__ xrows, const unsigned* __res
 }
 
 // ---- one MoE block on T rows of residual R: R += experts(rmsnorm(R))
-// next_norm: the norm weights of the projection that reads R next; with them (single rank) the combine leaves that projection's
-// image of the rows in e->d_img and *img_ready is set
-static int enqueue_moe(fnx_engine* e, const LayerW& L, float* R, int T, const float* next_norm = nullptr, bool* img_ready = nullptr) {
+// next, next_norm: the projection that reads R next and its norm weights; where it reads the rows' image, whatever completes the rows
+// leaves it in e->img_r and *img_ready is set
+static int enqueue_moe(fnx_engine* e, const LayerW& L, float* R, int T, const Mat* next = nullptr, const float* next_norm = nullptr, bool* img_ready = nullptr) {
     const Dims d = dims(e->c);
-    const bool ep = e->c.ep_size > 1;
+    const bool ep = e->c.ep_size > 1, img = next && next->nat && next_norm;
     if (img_ready) *img_ready = false;
+    if (L.wgu.nat) FNX_TRY(nat_rows_image(R, d.H, T, d.H, L.norm2, e->img_x, e->st));
     FNX_TRY(fnx_router_route(L.wr, R, L.norm2, e->c.eps, T, d.E, d.H, d.K, e->e_lo, e->e_hi, 1, e->rlogits, e->topi, e->topw, e->jobs, e->njobs,
                              e->d_stats, e->err, e->st));
     const int njobs_max = T * d.K + (T + FNX_JOB_TOK - 1) / FNX_JOB_TOK;
-    FNX_TRY(fnx_moe_gate_up(L.wgu, e->gu_bytes, e->e_lo, L.wsh_gu, d.E, e->jobs, e->njobs, njobs_max, R, L.norm2, e->c.eps, d.H, d.F, e->hbuf,
-                            e->err, e->st));
-    FNX_TRY(fnx_moe_down(L.wdn, e->dn_bytes, e->e_lo, L.wsh_dn, d.E, e->jobs, e->njobs, njobs_max, e->hbuf, d.H, d.F, e->part, e->err, e->st));
-    if (!ep && next_norm && e->use_img) {
+    if (L.wgu.nat)
+        FNX_TRY(nat_gate_up(L.wgu.nat, L.wgu.nat_stride(), e->e_lo, L.wsh_gu.nat, d.E, e->jobs, e->njobs, njobs_max, e->img_x, e->c.eps, d.H, d.F, e->hbuf, e->st));
+    else
+        FNX_TRY(fnx_moe_gate_up(L.wgu.tiles, L.wgu.tile_stride(), e->e_lo, L.wsh_gu.tiles, d.E, e->jobs, e->njobs, njobs_max, R, L.norm2, e->c.eps, d.H, d.F, e->hbuf,
+                                e->err, e->st));
+    if (L.wdn.nat)
+        FNX_TRY(nat_down(L.wdn.nat, L.wdn.nat_stride(), e->e_lo, L.wsh_dn.nat, d.E, e->jobs, e->njobs, njobs_max, e->hbuf, d.H, d.F, e->part, e->st));
+    else
+        FNX_TRY(fnx_moe_down(L.wdn.tiles, L.wdn.tile_stride(), e->e_lo, L.wsh_dn.tiles, d.E, e->jobs, e->njobs, njobs_max, e->hbuf, d.H, d.F, e->part, e->err, e->st));
+    if (!ep && img) {
         if (img_ready) *img_ready = true;
-        return fnx_moe_combine_image(e->part, e->topi, e->topw, e->rlogits, T, d.E, d.H, d.K, R, e->d_img, next_norm, e->st);
+        return moe_combine_nat(e->part, e->topi, e->topw, e->rlogits, T, d.E, d.H, d.K, R, e->img_r, next_norm, e->st);
     }
     if (!ep) return fnx_moe_combine(e->part, e->topi, e->topw, e->rlogits, T, d.E, d.H, d.K, 0, d.E, 1, R, 1, e->st);
     if (e->ep_peers && e->ep_one_kernel && d.H % 256 == 0) {
-        const bool img = next_norm && e->use_img;
         if (img_ready) *img_ready = img;
         k_ep_exchange<<<dim3(d.H / 256, T), 32, 0, e->st>>>(e->part, e->topi, e->topw, e->rlogits, T, d.E, d.H, d.K, e->e_lo, e->e_hi, e->d_peer_x, e->d_peer_flag,
                                                              (size_t) 4 * e->c.ep_size, e->xbuf, e->xflag, e->c.ep_rank, e->c.ep_size, d.MAXR, R, e->d_xseq, e->err,
-                                                             e->wait_limit, img ? e->d_img : nullptr, next_norm, fnx_dense_image_bytes(d.H));
+                                                             e->wait_limit, img ? e->img_r : nullptr, next_norm);
         FNX_LAUNCH_OK("k_ep_exchange");
         return FNX_OK;
     }
@@ -671,19 +720,18 @@ static int enqueue_moe(fnx_engine* e, const LayerW& L, float* R, int T, const fl
     return fnx_moe_combine(e->part, e->topi, e->topw, e->rlogits, T, d.E, d.H, d.K, 0, 0, 1, R, 1, e->st);
 }
 
-// dense projection of up to MAXR rows in calls of fnx_dense_rows(cols) rows
-// (img: the rows' image in e->d_img is that of x normed by norm_w: the blocks copy it instead of quantising the rows)
-static int enqueue_dense(fnx_engine* e, const uint8_t* W, int rows, int cols, const float* x, int ldx, int T, const float* norm_w, float* y, int ldy,
-                         int accumulate, bool img = false) {
-    const int per = img ? FNX_DENSE_ROWS : fnx_dense_rows(cols);   // (an image holds FNX_DENSE_ROWS rows: its products have <= 2048 columns)
+// y (+)= W x over up to MAXR rows; img: where the image of x (normed by norm_w) is or goes, ready: it is there
+static int enqueue_dense(fnx_engine* e, const Mat& W, const float* x, int ldx, int T, const float* norm_w, float* y, int ldy, int accumulate, uint8_t* img,
+                         bool ready = false) {
+    const int rows = (int) W.rows, cols = (int) W.cols;
+    if (W.nat) {
+        if (!ready) FNX_TRY(nat_rows_image(x, ldx, T, cols, norm_w, img, e->st));
+        return nat_dense(W.nat, rows, cols, img, norm_w != nullptr, e->c.eps, T, y, ldy, accumulate, e->st);
+    }
+    const int per = fnx_dense_rows(cols);
     for (int t0 = 0; t0 < T; t0 += per) {
         const int nt = T - t0 < per ? T - t0 : per;
-        if (img) {
-            FNX_TRY(fnx_dense_image(W, rows, cols, e->d_img + (size_t) (t0 / FNX_DENSE_ROWS) * fnx_dense_image_bytes(cols), nt, norm_w != nullptr, e->c.eps,
-                                    y + (size_t) t0 * ldy, ldy, accumulate, e->err, e->st));
-            continue;
-        }
-        FNX_TRY(fnx_dense(W, rows, cols, x + (size_t) t0 * ldx, ldx, nt, norm_w, e->c.eps, y + (size_t) t0 * ldy, ldy, accumulate, e->err, e->st));
+        FNX_TRY(fnx_dense(W.tiles, rows, cols, x + (size_t) t0 * ldx, ldx, nt, norm_w, e->c.eps, y + (size_t) t0 * ldy, ldy, accumulate, e->err, e->st));
     }
     return FNX_OK;
 }
@@ -691,7 +739,7 @@ static int enqueue_dense(fnx_engine* e, const uint8_t* W, int rows, int cols, co
 static int enqueue_attention(fnx_engine* e, const LayerW& L, float* R, int T, int seq, const int* d_parent, const int* d_depth, const int* d_pos,
                              bool img = false) {
     const Dims d = dims(e->c);
-    FNX_TRY(enqueue_dense(e, L.w_in, L.in_rows, d.H, R, d.H, T, L.norm1, e->proj, e->proj_ld, 0, img));
+    FNX_TRY(enqueue_dense(e, L.w_in, R, d.H, T, L.norm1, e->proj, e->proj_ld, 0, e->img_r, img));
     __half* kc = L.kc + (size_t) seq * e->cache_rows * d.kv_rows;
     __half* vc = L.vc + (size_t) seq * e->cache_rows * d.kv_rows;
     float* qg = e->proj;
@@ -700,17 +748,17 @@ static int enqueue_attention(fnx_engine* e, const LayerW& L, float* R, int T, in
     FNX_TRY(fnx_attn_prep_append(qg, e->proj_ld, k, e->proj_ld, v, e->proj_ld, L.qn, L.kn, kc, vc, T, d.nq, d.nkv, d.hd, d.nrot, d_pos, d_depth,
                                  e->c.eps, e->c.rope_base, e->st));
     FNX_TRY(fnx_attn(qg, e->proj_ld, kc, vc, e->mix, T, d.nq, d.nkv, d.hd, d_pos, d_parent, e->att_scratch, e->st));
-    return enqueue_dense(e, L.w_out, d.H, d.nq * d.hd, e->mix, d.nq * d.hd, T, nullptr, R, d.H, 1);
+    return enqueue_dense(e, L.w_out, e->mix, d.nq * d.hd, T, nullptr, R, d.H, 1, e->img_m);
 }
 
 static int enqueue_gdn(fnx_engine* e, const LayerW& L, float* R, int T, int seq, const int* d_parent, bool img = false) {
     const Dims d = dims(e->c);
-    FNX_TRY(enqueue_dense(e, L.w_in, L.in_rows, d.H, R, d.H, T, L.norm1, e->proj, e->proj_ld, 0, img));
+    FNX_TRY(enqueue_dense(e, L.w_in, R, d.H, T, L.norm1, e->proj, e->proj_ld, 0, e->img_r, img));
     float* S = L.S_pool + (size_t) seq * e->NS * d.nv * d.hs * d.hs;
     float* hist = L.hist_pool + (size_t) seq * e->NS * 3 * d.gdn_ch;
     FNX_TRY(fnx_gdn_core(e->proj, e->proj_ld, e->proj + d.gdn_ch + d.nv * d.hs, e->proj_ld, hist, L.convw, L.dt, L.a, L.gnorm, S, e->d_cur + seq,
                          e->NS, d_parent, e->mix, d.nk, d.nv, d.hs, T, e->c.eps, e->st));
-    return enqueue_dense(e, L.w_out, d.H, d.nv * d.hs, e->mix, d.nv * d.hs, T, nullptr, R, d.H, 1);
+    return enqueue_dense(e, L.w_out, e->mix, d.nv * d.hs, T, nullptr, R, d.H, 1, e->img_m);
 }
 
 // the whole verify window: embed, layers, head, argmax, greedy acceptance
@@ -719,15 +767,16 @@ static int enqueue_verify(fnx_engine* e, int seq, int T, bool tree) {
     const int* par = tree ? e->d_parent : nullptr;
     k_depths<<<1, 32, 0, e->st>>>(par, e->d_depth, T);
     FNX_LAUNCH_OK("depths");
-    FNX_TRY(fnx_embed_rows(e->embed, e->d_tok, T, d.H, e->R, e->st));
-    bool img = false;   // the rows' image for the next projection is ready (left by the layer before)
+    bool img = e->layers[0].w_in.nat != nullptr;   // the rows' image for the next projection is ready (left by whatever completed the rows)
+    FNX_TRY(nat_embed_image(e->embed, e->d_tok, T, d.H, e->R, e->layers[0].norm1, img ? e->img_r : nullptr, e->st));
     for (size_t l = 0; l < e->layers.size(); ++l) {
         const LayerW& L = e->layers[l];
         if (L.attn) FNX_TRY(enqueue_attention(e, L, e->R, T, seq, par, e->d_depth, e->d_pos + seq, img));
         else FNX_TRY(enqueue_gdn(e, L, e->R, T, seq, par, img));
-        FNX_TRY(enqueue_moe(e, L, e->R, T, l + 1 < e->layers.size() ? e->layers[l + 1].norm1 : e->out_norm, &img));
+        const bool last = l + 1 == e->layers.size();
+        FNX_TRY(enqueue_moe(e, L, e->R, T, last ? &e->head : &e->layers[l + 1].w_in, last ? e->out_norm : e->layers[l + 1].norm1, &img));
     }
-    FNX_TRY(enqueue_dense(e, e->head, d.V, d.H, e->R, d.H, T, e->out_norm, e->logits, d.V, 0, img));
+    FNX_TRY(enqueue_dense(e, e->head, e->R, d.H, T, e->out_norm, e->logits, d.V, 0, e->img_r, img));
     if (e->rules_on)   // the request's logit_bias and penalties, before either rule looks at the logits
         FNX_TRY(fnx_logit_adjust(e->logits, T, d.V, e->d_ctx + (size_t) seq * e->cache_rows, e->d_ctx_n + seq, e->d_tok, e->rules.last_n, e->rules.repeat,
                                  e->rules.freq, e->rules.present, e->d_bias_tok, e->d_bias_val, e->rules.bias_n, e->st));
@@ -741,14 +790,28 @@ static int enqueue_verify(fnx_engine* e, int seq, int T, bool tree) {
     return fnx_accept_greedy(e->d_tok, par, e->best_i, T, e->result, e->st);
 }
 
-// one MTP call on T rows: Rm = fc_hid(rms(src)) + fc_emb(rms(emb(tok))), the draft block, the head on the last row
+// the draft layer's input rows: Rm = fc_hid(rms(src)) + fc_emb(rms(emb(tok)))   (fnx_mtp_input)
+static int enqueue_mtp_input(fnx_engine* e, int T, const float* src) {
+    const Dims d = dims(e->c);
+    if (!e->mtp_fc_hid.nat)
+        return fnx_mtp_input(e->mtp_fc_hid.tiles, e->mtp_fc_emb.tiles, e->embed, e->mtp_hnorm, e->mtp_enorm, e->c.eps, src, d.H, e->d_mtok, T, d.H, e->Emb, e->Rm, e->err,
+                             e->st);
+    FNX_TRY(nat_rows_image(src, d.H, T, d.H, e->mtp_hnorm, e->img_x, e->st));
+    FNX_TRY(nat_embed_image(e->embed, e->d_mtok, T, d.H, e->Emb, e->mtp_enorm, e->img_r, e->st));
+    FNX_TRY(nat_dense(e->mtp_fc_hid.nat, d.H, d.H, e->img_x, true, e->c.eps, T, e->Rm, d.H, 0, e->st));
+    return nat_dense(e->mtp_fc_emb.nat, d.H, d.H, e->img_r, true, e->c.eps, T, e->Rm, d.H, 1, e->st);
+}
+
+// one MTP call on T rows: the draft block on the input rows, the head on the last row
 static int enqueue_mtp(fnx_engine* e, int seq, int T, const float* src) {
     const Dims d = dims(e->c);
-    FNX_TRY(fnx_mtp_input(e->mtp_fc_hid, e->mtp_fc_emb, e->embed, e->mtp_hnorm, e->mtp_enorm, e->c.eps, src, d.H, e->d_mtok, T, d.H, e->Emb, e->Rm, e->err, e->st));
+    const Mat& head = e->mtp_head.rows ? e->mtp_head : e->head;
+    FNX_TRY(enqueue_mtp_input(e, T, src));
     FNX_TRY(enqueue_attention(e, e->mtp, e->Rm, T, seq, nullptr, nullptr, e->d_mpos));
-    FNX_TRY(enqueue_moe(e, e->mtp, e->Rm, T));
-    return fnx_dense(e->mtp_head ? e->mtp_head : e->head, e->dvn, d.H, e->Rm + (size_t) (T - 1) * d.H, d.H, 1, e->mtp_onorm, e->c.eps, e->logits, e->dvn, 0,
-                     e->err, e->st);
+    bool img = false;
+    FNX_TRY(enqueue_moe(e, e->mtp, e->Rm, T, &head, e->mtp_onorm, &img));
+    return enqueue_dense(e, head, e->Rm + (size_t) (T - 1) * d.H, d.H, 1, e->mtp_onorm, e->logits, e->dvn, 0,
+                         img ? e->img_r + (size_t) (T - 1) * ni_row_bytes(d.H / 256) : e->img_r, img);
 }
 
 // ------------------------------------------------------------------------------------------------ batched lanes
@@ -826,7 +889,7 @@ static int enqueue_mixer_lanes(fnx_engine* e, const LayerW& L, float* R, int T, 
     // for the others', which the lane kernels skip) and the output rows are gathered before the output projection
     const bool dp = e->c.ep_size > 1 && e->ep_peers && e->dp_mixers;
     const int* lanes = dp ? e->d_lane_own : d_lane_seq;
-    FNX_TRY(enqueue_dense(e, L.w_in, L.in_rows, d.H, R, d.H, T, L.norm1, e->proj, e->proj_ld, 0, img));
+    FNX_TRY(enqueue_dense(e, L.w_in, R, d.H, T, L.norm1, e->proj, e->proj_ld, 0, e->img_r, img));
     if (L.attn) {
         float* qg = e->proj;
         float* k = e->proj + d.q_rows;
@@ -835,25 +898,26 @@ static int enqueue_mixer_lanes(fnx_engine* e, const LayerW& L, float* R, int T, 
                                            d.nkv, d.hd, d.nrot, d_pos, lanes, d_row0, e->c.eps, e->c.rope_base, e->st));
         FNX_TRY(fnx_attn_lanes(qg, e->proj_ld, L.kc, L.vc, (size_t) e->cache_rows, e->mix, T, n_lanes, d.nq, d.nkv, d.hd, d_pos, lanes, d_row0, e->att_scratch, e->st));
         if (dp) FNX_TRY(enqueue_dp_gather(e, d.nq * d.hd, n_lanes, d_row0));
-        return enqueue_dense(e, L.w_out, d.H, d.nq * d.hd, e->mix, d.nq * d.hd, T, nullptr, R, d.H, 1);
+        return enqueue_dense(e, L.w_out, e->mix, d.nq * d.hd, T, nullptr, R, d.H, 1, e->img_m);
     }
     FNX_TRY(fnx_gdn_core_lanes(e->proj, e->proj_ld, e->proj + d.gdn_ch + d.nv * d.hs, e->proj_ld, L.hist_pool, (size_t) e->NS * 3 * d.gdn_ch, L.convw, L.dt, L.a, L.gnorm,
                                L.S_pool, (size_t) e->NS * d.nv * d.hs * d.hs, e->d_cur, e->NS, lanes, d_row0, n_lanes, max_lane_rows, e->mix, d.nk, d.nv, d.hs,
                                e->c.eps, e->st));
     if (dp) FNX_TRY(enqueue_dp_gather(e, d.nv * d.hs, n_lanes, d_row0));
-    return enqueue_dense(e, L.w_out, d.H, d.nv * d.hs, e->mix, d.nv * d.hs, T, nullptr, R, d.H, 1);
+    return enqueue_dense(e, L.w_out, e->mix, d.nv * d.hs, T, nullptr, R, d.H, 1, e->img_m);
 }
 
 static int enqueue_verify_lanes(fnx_engine* e, int n_lanes, int rows, int T) {   // rows: the longest lane's; T: rows in all
     const Dims d = dims(e->c);
-    FNX_TRY(fnx_embed_rows(e->embed, e->d_tok, T, d.H, e->R, e->st));
-    bool img = false;
+    bool img = e->layers[0].w_in.nat != nullptr;
+    FNX_TRY(nat_embed_image(e->embed, e->d_tok, T, d.H, e->R, e->layers[0].norm1, img ? e->img_r : nullptr, e->st));
     for (size_t l = 0; l < e->layers.size(); ++l) {
         const LayerW& L = e->layers[l];
         FNX_TRY(enqueue_mixer_lanes(e, L, e->R, T, n_lanes, rows, e->d_lane_seq, e->d_lane_row0, e->d_pos, img));
-        FNX_TRY(enqueue_moe(e, L, e->R, T, l + 1 < e->layers.size() ? e->layers[l + 1].norm1 : e->out_norm, &img));
+        const bool last = l + 1 == e->layers.size();
+        FNX_TRY(enqueue_moe(e, L, e->R, T, last ? &e->head : &e->layers[l + 1].w_in, last ? e->out_norm : e->layers[l + 1].norm1, &img));
     }
-    FNX_TRY(enqueue_dense(e, e->head, d.V, d.H, e->R, d.H, T, e->out_norm, e->logits, d.V, 0, img));
+    FNX_TRY(enqueue_dense(e, e->head, e->R, d.H, T, e->out_norm, e->logits, d.V, 0, e->img_r, img));
     if (e->sampling_on) {
         FNX_TRY(fnx_top_tokens(e->logits, T, d.V, e->cand_v, e->cand_i, e->st));
         return fnx_accept_sample_lanes(e->cand_v, e->cand_i, e->d_tok, e->sampling, e->sample_seed, e->d_lane_seq, e->d_lane_row0, n_lanes, rows, e->d_step,
@@ -867,12 +931,12 @@ static int enqueue_verify_lanes(fnx_engine* e, int n_lanes, int rows, int T) {  
 // through the head and their best tokens land in best_i[0 .. n_lanes)
 static int enqueue_mtp_lanes(fnx_engine* e, int n_lanes, int Tm, int max_rows, const int* d_row0, const float* src) {
     const Dims d = dims(e->c);
-    FNX_TRY(fnx_mtp_input(e->mtp_fc_hid, e->mtp_fc_emb, e->embed, e->mtp_hnorm, e->mtp_enorm, e->c.eps, src, d.H, e->d_mtok, Tm, d.H, e->Emb, e->Rm, e->err, e->st));
+    FNX_TRY(enqueue_mtp_input(e, Tm, src));
     FNX_TRY(enqueue_mixer_lanes(e, e->mtp, e->Rm, Tm, n_lanes, max_rows, e->d_lane_seq, d_row0, e->d_mpos_seq));
     FNX_TRY(enqueue_moe(e, e->mtp, e->Rm, Tm));
     k_last_rows<<<dim3((d.H + 255) / 256, n_lanes), 256, 0, e->st>>>(e->Rlast, e->Rm, d_row0, d.H);
     FNX_LAUNCH_OK("draft last rows");
-    FNX_TRY(enqueue_dense(e, e->mtp_head ? e->mtp_head : e->head, e->dvn, d.H, e->Rlast, d.H, n_lanes, e->mtp_onorm, e->logits, e->dvn, 0));
+    FNX_TRY(enqueue_dense(e, e->mtp_head.rows ? e->mtp_head : e->head, e->Rlast, d.H, n_lanes, e->mtp_onorm, e->logits, e->dvn, 0, e->img_r));
     return fnx_argmax_mapped(e->logits, n_lanes, e->dvn, e->d_dvocab, e->best_i, nullptr, e->err, e->st);
 }
 
@@ -948,8 +1012,6 @@ extern "C" int fnx_engine_create(const fnx_model_config* cfg, fnx_engine** out) 
     e->E_local = c.n_expert / c.ep_size;
     e->e_lo = c.ep_rank * e->E_local;
     e->e_hi = e->e_lo + e->E_local;
-    e->gu_bytes = iq3s_bytes((size_t) 2 * d.F, d.H);
-    e->dn_bytes = iq3s_bytes((size_t) d.H, d.F);
     e->seqs.resize(c.n_seq);
     int rc = FNX_OK;
     auto body = [&]() -> int {
@@ -963,13 +1025,14 @@ extern "C" int fnx_engine_create(const fnx_model_config* cfg, fnx_engine** out) 
         FNX_TRY(dalloc(e, &e->mtp_enorm, d.H, "mtp.e_norm"));
         FNX_TRY(dalloc(e, &e->mtp_onorm, d.H, "mtp.out_norm"));
         FNX_TRY(dalloc(e, &e->out_norm, d.H, "out_norm"));
-        FNX_TRY(dalloc(e, &e->mtp_fc_hid, iq3s_bytes(d.H, d.H), "mtp.fc_hid"));
-        FNX_TRY(dalloc(e, &e->mtp_fc_emb, iq3s_bytes(d.H, d.H), "mtp.fc_emb"));
-        FNX_TRY(dalloc(e, &e->head, iq3s_bytes(d.V, d.H), "head"));
+        FNX_TRY(alloc_mat(e, e->mtp_fc_hid, d.H, d.H, "mtp.fc_hid"));
+        FNX_TRY(alloc_mat(e, e->mtp_fc_emb, d.H, d.H, "mtp.fc_emb"));
+        e->mtp_fc_hid.with = &e->mtp_fc_emb; e->mtp_fc_emb.with = &e->mtp_fc_hid;
+        FNX_TRY(alloc_mat(e, e->head, d.V, d.H, "head"));
         e->dvn = d.V;
         if (c.draft_vocab > 0) {
             e->dvn = c.draft_vocab;
-            FNX_TRY(dalloc(e, &e->mtp_head, iq3s_bytes(e->dvn, d.H), "mtp.head"));
+            FNX_TRY(alloc_mat(e, e->mtp_head, e->dvn, d.H, "mtp.head"));
             FNX_TRY(dalloc(e, &e->d_dvocab, (size_t) e->dvn, "mtp.vocab"));
         }
         FNX_TRY(dalloc(e, &e->embed, (size_t) d.V * d.H, "embed"));
@@ -990,9 +1053,9 @@ extern "C" int fnx_engine_create(const fnx_model_config* cfg, fnx_engine** out) 
         FNX_TRY(dalloc(e, &e->hbuf, (size_t) d.P * d.F, "buf.h"));
         FNX_TRY(dalloc(e, &e->part, (size_t) d.P * d.H, "buf.part"));
         FNX_TRY(dalloc(e, &e->moe_out, (size_t) d.MAXR * d.H, "buf.moe_out"));
-        FNX_TRY(dalloc(e, &e->d_img, (size_t) ((d.MAXR + FNX_DENSE_ROWS - 1) / FNX_DENSE_ROWS) * fnx_dense_image_bytes(d.H)));
-        if (const char* nf = getenv("FNX_NO_IMAGE")) e->use_img = nf[0] != '1';
-        if (d.H > 2048) e->use_img = false;   // (an image's product takes FNX_DENSE_ROWS rows a call, which wider rows do not fit)
+        FNX_TRY(dalloc(e, &e->img_r, ni_bytes(d.MAXR, d.H)));
+        FNX_TRY(dalloc(e, &e->img_x, ni_bytes(d.MAXR, d.H)));
+        FNX_TRY(dalloc(e, &e->img_m, ni_bytes(d.MAXR, mixw)));
         if (c.ep_size > 1) {
             e->mix_width = mixw;
             e->x_off_rows = (size_t) 2 * c.ep_size * d.MAXR * d.H;
@@ -1085,11 +1148,11 @@ extern "C" int fnx_engine_init_synthetic(fnx_engine* e, uint64_t seed, float sig
         FNX_TRY(fill_const(e, e->mtp_enorm, d.H, 1.0f));
         FNX_TRY(fill_const(e, e->mtp_onorm, d.H, 1.0f));
         FNX_TRY(fill_const(e, e->out_norm, d.H, 1.0f));
-        FNX_TRY(synth_iq3s(e, e->mtp_fc_hid, d.H, d.H, sigma, seed, (61u * 16 + 0) << 12, tf, tg, tw));
-        FNX_TRY(synth_iq3s(e, e->mtp_fc_emb, d.H, d.H, sigma, seed, (61u * 16 + 1) << 12, tf, tg, tw));
-        FNX_TRY(synth_iq3s(e, e->head, d.V, d.H, sigma, seed, (62u * 16) << 12, tf, tg, tw));
-        if (e->mtp_head) {
-            FNX_TRY(synth_iq3s(e, e->mtp_head, e->dvn, d.H, sigma, seed, (61u * 16 + 2) << 12, tf, tg, tw));
+        FNX_TRY(synth_iq3s(e, e->mtp_fc_hid, 0, sigma, seed, (61u * 16 + 0) << 12, tf, tg, tw));
+        FNX_TRY(synth_iq3s(e, e->mtp_fc_emb, 0, sigma, seed, (61u * 16 + 1) << 12, tf, tg, tw));
+        FNX_TRY(synth_iq3s(e, e->head, 0, sigma, seed, (62u * 16) << 12, tf, tg, tw));
+        if (e->mtp_head.rows) {
+            FNX_TRY(synth_iq3s(e, e->mtp_head, 0, sigma, seed, (61u * 16 + 2) << 12, tf, tg, tw));
             k_fill_dvocab<<<(e->dvn + 255) / 256, 256, 0, e->st>>>(e->d_dvocab, e->dvn, d.V);
             FNX_LAUNCH_OK("draft vocabulary");
         }
@@ -1117,6 +1180,18 @@ extern "C" size_t fnx_engine_device_bytes(const fnx_engine* e) { return e ? e->b
 extern "C" void* fnx_engine_tensor(fnx_engine* e, const char* name, size_t* bytes) {
     if (bytes) *bytes = 0;
     if (!e || !name) return nullptr;
+    auto mt = e->mats.find(name);
+    if (mt != e->mats.end()) {
+        Mat& m = *mt->second;
+        if (m.nat) {   // the captured graphs name the layout that goes
+            cudaStreamSynchronize(e->st);
+            for (auto& g : e->graphs) cudaGraphExecDestroy(g.second);
+            e->graphs.clear();
+            if (to_tiles(e, m) != FNX_OK || (m.with && to_tiles(e, *m.with) != FNX_OK)) return nullptr;
+        }
+        if (bytes) *bytes = m.tile_stride() * m.n;
+        return m.tiles;
+    }
     auto it = e->tensors.find(name);
     if (it == e->tensors.end()) return nullptr;
     if (bytes) *bytes = it->second.second;
@@ -1330,7 +1405,7 @@ extern "C" int fnx_engine_prompt(fnx_engine* e, int seq, const int* h_tok, int n
             const LayerW& L = e->layers[l];
             e->launches += 3 + (L.attn ? 3 : 3) + 3 + 2 + 7;   // this layer's kernels: projections 3 + 3, mixer 3, router 2, experts 7
             mark(PH_INPROJ, true);
-            FNX_TRY(fnx_dense_prompt(L.w_in, L.in_rows, d.H, e->pR, nt, L.norm1, e->c.eps, e->pproj, e->proj_ld, 0, e->p_dense_scratch, e->err, e->st));
+            FNX_TRY(prompt_dense(L.w_in.nat ? L.w_in.nat : L.w_in.tiles, L.w_in.nat != nullptr, L.in_rows, d.H, e->pR, nt, L.norm1, e->c.eps, e->pproj, e->proj_ld, 0, e->p_dense_scratch, e->err, e->st));
             mark(PH_INPROJ, false);
             mark(L.attn ? PH_ATTN : PH_GDN, true);
             int mixw_l;
@@ -1353,14 +1428,18 @@ extern "C" int fnx_engine_prompt(fnx_engine* e, int seq, const int* h_tok, int n
             }
             mark(0, false);
             mark(PH_OUTPROJ, true);
-            FNX_TRY(fnx_dense_prompt(L.w_out, d.H, mixw_l, e->pmix, nt, nullptr, e->c.eps, e->pR, d.H, 1, e->p_dense_scratch, e->err, e->st));
+            FNX_TRY(prompt_dense(L.w_out.nat ? L.w_out.nat : L.w_out.tiles, L.w_out.nat != nullptr, d.H, mixw_l, e->pmix, nt, nullptr, e->c.eps, e->pR, d.H, 1, e->p_dense_scratch, e->err, e->st));
             mark(0, false);
             mark(PH_ROUTER, true);
             FNX_TRY(fnx_router_rows(L.wr, e->pR, L.norm2, e->c.eps, nt, d.E, d.H, d.K, e->plogits, e->ptopi, e->ptopw, e->p_router_scratch, e->err, e->st));
             mark(0, false);
             mark(PH_MOE, true);
-            FNX_TRY(fnx_moe_prefill(L.wgu, e->gu_bytes, L.wdn, e->dn_bytes, L.wsh_gu, L.wsh_dn, 0, d.E, d.K, 0, d.E, 1, e->ptopi, e->ptopw, e->plogits, e->pR, L.norm2,
-                                    e->c.eps, nt, d.H, d.F, e->pR, 1, e->p_moe_scratch, e->err, e->st));
+            {
+                const bool gn = L.wgu.nat != nullptr, dn = L.wdn.nat != nullptr;
+                FNX_TRY(prompt_moe(gn ? L.wgu.nat : L.wgu.tiles, gn ? L.wgu.nat_stride() : L.wgu.tile_stride(), gn ? L.wsh_gu.nat : L.wsh_gu.tiles, gn,
+                                   dn ? L.wdn.nat : L.wdn.tiles, dn ? L.wdn.nat_stride() : L.wdn.tile_stride(), dn ? L.wsh_dn.nat : L.wsh_dn.tiles, dn, 0, d.E, d.K, 0, d.E, 1,
+                                   e->ptopi, e->ptopw, e->plogits, e->pR, L.norm2, e->c.eps, nt, d.H, d.F, e->pR, 1, e->p_moe_scratch, e->err, e->st));
+            }
             mark(0, false);
         }
         if (phases) {

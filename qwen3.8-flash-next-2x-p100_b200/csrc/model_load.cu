@@ -1,16 +1,17 @@
 // Model loader: a GGUF file's tensors (llama.cpp's names for this architecture) into an engine's device tensors.  The
 // counterpart of the reference's load (engine/src/model.cpp:837-905 dense models, :932-1097 the MoE model; expert slicing
-// :1063-1069; small-tensor conversion engine/src/tensor_convert.hpp): every matrix ends up in the IQ3_S tile layout the
+// :1063-1069; small-tensor conversion engine/src/tensor_convert.hpp): every matrix ends up in the IQ3_S layout the
 // kernels stream, every vector in f32.
 //   - an IQ3_S tensor is copied block for block and re-tiled: bit-exact;
 //   - a matrix of another type (F32, F16, BF16, Q8_0) is converted to f32 on the host and quantised to IQ3_S on the
 //     GPU by fnx_iq3s_quantize: lossy, counted in *h_converted (the verify path has no kernels for other formats);
 //   - stacked expert tensors ([experts][rows][cols]) are sliced to this rank's experts.
-// Written against the public entry points only (fnx_engine_tensor names the destinations).
+// Vectors and tables go to the places fnx_engine_tensor names, matrices through engine_put_matrix (engine_mat.h).
 #include <cstring>
 #include <string>
 #include <vector>
 
+#include "engine_mat.h"
 #include "fnx_common.cuh"
 
 namespace fnxb {
@@ -76,13 +77,7 @@ struct Loader {
 
     // A matrix of `rows` x `cols` from pieces stacked by rows, in order; rows past the pieces' are zero.  Every piece has
     // `cols` columns (n_cols) and its rows land after the previous piece's.
-    int matrix(const std::string& dst_name, size_t rows, size_t cols, const std::vector<Piece>& pieces) {
-        void* dst = nullptr;
-        FNX_TRY(dest(dst_name, fnx_iq3s_bytes(rows, cols), &dst));
-        return matrix_to(dst, dst_name, rows, cols, pieces);
-    }
-
-    int matrix_to(void* dst, const std::string& what, size_t rows, size_t cols, const std::vector<Piece>& pieces) {
+    int matrix(const std::string& what, size_t rows, size_t cols, const std::vector<Piece>& pieces, int index = 0) {
         FNX_REQUIRE(rows % 16 == 0 && cols % 256 == 0, "load: %s is %zu x %zu (rows in 16s, columns in 256s)", what.c_str(), rows, cols);
         const size_t row_bytes = cols / 256 * IQ3S_BLOCK;
         FNX_TRY(need_g(rows * row_bytes));
@@ -116,7 +111,7 @@ struct Loader {
             }
             r += (size_t) p.n_rows;
         }
-        FNX_TRY(fnx_iq3s_retile(d_g, dst, rows, cols, st));
+        FNX_TRY(engine_put_matrix(e, what, index, rows, cols, d_g, st));
         FNX_CUDA_OK(cudaStreamSynchronize(st));
         return FNX_OK;
     }
@@ -200,16 +195,11 @@ struct Loader {
         FNX_REQUIRE(tg.ne[0] == H && tg.ne[1] == F && tg.ne[2] == c.n_expert && tu.ne[0] == H && tu.ne[1] == F && tu.ne[2] == c.n_expert && td.ne[0] == F &&
                         td.ne[1] == H && td.ne[2] == c.n_expert,
                     "load: layer %d: the stacked expert tensors are not [%d][%d][%d] (gate, up) and [%d][%d][%d] (down)", l, c.n_expert, F, H, c.n_expert, H, F);
-        const size_t gu_bytes = fnx_iq3s_bytes((size_t) 2 * F, (size_t) H), dn_bytes = fnx_iq3s_bytes((size_t) H, (size_t) F);
-        void *wgu = nullptr, *wdn = nullptr;
-        FNX_TRY(dest(dst + "experts_gu", gu_bytes * E_local, &wgu));
-        FNX_TRY(dest(dst + "experts_dn", dn_bytes * E_local, &wdn));
         const int conv0 = converted;
         for (int x = 0; x < E_local; ++x) {
             const int64_t ge = e_lo + x;
-            FNX_TRY(matrix_to((uint8_t*) wgu + (size_t) x * gu_bytes, dst + "experts_gu", (size_t) 2 * F, (size_t) H,
-                              {Piece{tg, ge * F, F, 0, H}, Piece{tu, ge * F, F, 0, H}}));
-            FNX_TRY(matrix_to((uint8_t*) wdn + (size_t) x * dn_bytes, dst + "experts_dn", (size_t) H, (size_t) F, {Piece{td, ge * H, H, 0, F}}));
+            FNX_TRY(matrix(dst + "experts_gu", (size_t) 2 * F, (size_t) H, {Piece{tg, ge * F, F, 0, H}, Piece{tu, ge * F, F, 0, H}}, x));
+            FNX_TRY(matrix(dst + "experts_dn", (size_t) H, (size_t) F, {Piece{td, ge * H, H, 0, F}}, x));
         }
         if (converted > conv0) converted = conv0 + (tg.type != 21) + (tu.type != 21) + (td.type != 21);   // counted per tensor, not per expert
         FNX_TRY(find(src + "ffn_gate_shexp.weight", &tg));

@@ -19,6 +19,7 @@
 #include "fnx_common.cuh"
 #include "iq3s_grid.h"
 #include "iq3s_tile.h"
+#include "nat_tile.h"
 
 namespace fnxb {
 
@@ -102,6 +103,40 @@ __device__ __forceinline__ void pf_load_raw(const uint8_t* tile, int lane, PfRaw
     r.d1 = __half2float(*reinterpret_cast<const __half*>(tile + TILE_D + (g + 8) * 2));
 }
 
+// the same of half a tile in the engine's own layout (nat_tile.h): the nibbles of rows g and g + 8, a word per sub-block
+struct PfRawNat {
+    uint32_t w[2][8];
+    uint32_t sn0, sn1;
+    float d0, d1;
+};
+__device__ __forceinline__ void pf_load_raw(const uint8_t* half, int lane, PfRawNat& r) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const uint4 v = *reinterpret_cast<const uint4*>(half + j * 512 + lane * 16);
+        r.w[j >> 1][(j & 1) * 4] = v.x; r.w[j >> 1][(j & 1) * 4 + 1] = v.y; r.w[j >> 1][(j & 1) * 4 + 2] = v.z; r.w[j >> 1][(j & 1) * 4 + 3] = v.w;
+    }
+    const uint4 m = *reinterpret_cast<const uint4*>(half + NAT_META + (lane >> 2) * 16);
+    const float2 d = __half22float2(*reinterpret_cast<const __half2*>(&m.z));
+    r.sn0 = m.x; r.sn1 = m.y; r.d0 = d.x; r.d1 = d.y;
+}
+// the eight weights of a word as halves, times the sub-block scale: a nibble t becomes the byte 2 (t + 8) = m + 15, the half
+// 0x6400 | byte is 1024 + m + 15
+__device__ __forceinline__ uint4 pf_halves8_nat(uint32_t w, __half2 f2) {
+    const __half2 bias = __floats2half2_rn(1039.0f, 1039.0f);
+    const uint32_t lo = ((w << 1) & 0x1E1E1E1Eu) ^ 0x10101010u, hi = ((w >> 3) & 0x1E1E1E1Eu) ^ 0x10101010u;
+    uint32_t h[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const uint32_t u = j < 2 ? lo : hi;
+        uint32_t pair;
+        if (j & 1) asm("prmt.b32 %0, %1, %2, 0x4342;" : "=r"(pair) : "r"(u), "r"(0x64646464u));
+        else asm("prmt.b32 %0, %1, %2, 0x4140;" : "=r"(pair) : "r"(u), "r"(0x64646464u));
+        const __half2 v = __hmul2(__hsub2(*reinterpret_cast<const __half2*>(&pair), bias), f2);
+        h[j] = *reinterpret_cast<const uint32_t*>(&v);
+    }
+    return make_uint4(h[0], h[1], h[2], h[3]);
+}
+
 // eight signed codebook bytes (two lookups) times the sub-block scale -> eight f16 at (row, k .. k + 7): one core-matrix
 // row.  Bytes become halves without the conversion unit: 0x6400 | (b + 128) is the f16 1024 + (b + 128), exactly.
 __device__ __forceinline__ uint4 pf_halves8(uint32_t lo4, uint32_t hi4, __half2 f2) {
@@ -134,6 +169,13 @@ __device__ __forceinline__ uint32_t pf_decode(const uint32_t (&S)[5], const uint
 // chunk).  Lane q of a row holds the sub-block's columns 8 q .. 8 q + 7: lookup 2 SB the first four, 2 SB + 1 the others
 // (the tile layout pairs them with the activation cells of 8 consecutive columns, iq3s_tile.h).
 template <int SB>
+__device__ __forceinline__ void pf_sub_block(const PfRawNat& r, uint8_t* tileA, int row0, int lane, uint32_t) {
+    const int g = lane >> 2, q = lane & 3, k0 = (SB & 1) * 32 + 8 * q;
+    const __half2 f0 = __float2half2_rn(r.d0 * (float) (1 + 2 * (int) ((r.sn0 >> (4 * SB)) & 15u))), f1 = __float2half2_rn(r.d1 * (float) (1 + 2 * (int) ((r.sn1 >> (4 * SB)) & 15u)));
+    *reinterpret_cast<uint4*>(tileA + pf_off(row0 + g, k0)) = pf_halves8_nat(r.w[0][SB], f0);
+    *reinterpret_cast<uint4*>(tileA + pf_off(row0 + g + 8, k0)) = pf_halves8_nat(r.w[1][SB], f1);
+}
+template <int SB>
 __device__ __forceinline__ void pf_sub_block(const PfRaw& r, uint8_t* tileA, int row0, int lane, uint32_t table_s) {
     const int g = lane >> 2, q = lane & 3, k0 = (SB & 1) * 32 + 8 * q;
     const __half2 f0 = __float2half2_rn(r.d0 * (float) (1 + 2 * (int) ((r.sn0 >> (8 * (SB >> 1) + 4 * (SB & 1))) & 15u)));
@@ -142,8 +184,8 @@ __device__ __forceinline__ void pf_sub_block(const PfRaw& r, uint8_t* tileA, int
     pf_store8(tileA, row0 + g + 8, k0, pf_decode<2 * SB>(r.S1, r.G1, table_s), pf_decode<2 * SB + 1>(r.S1, r.G1, table_s), f1);
 }
 // the warp's share of quarter Q of a tile block (sub-blocks 2 Q, 2 Q + 1): gate|up: both; down (two warps per tile): one
-template <int Q, int MODE>
-__device__ __forceinline__ void pf_quarter(const PfRaw& r, uint8_t* tileA, int row0, int lane, uint32_t table_s, int sel) {
+template <int Q, int MODE, typename Raw>
+__device__ __forceinline__ void pf_quarter(const Raw& r, uint8_t* tileA, int row0, int lane, uint32_t table_s, int sel) {
     if (MODE == 1) {
         pf_sub_block<2 * Q>(r, tileA, row0, lane, table_s);
         pf_sub_block<2 * Q + 1>(r, tileA, row0, lane, table_s);
@@ -174,7 +216,8 @@ struct PfParams {
 };
 
 // MODE 0: out = x W^T (down).  MODE 1: out = silu(x Wg^T) * (x Wu^T) (gate|up; W = [gate (rows); up (rows)]).
-template <int MODE>
+// NAT: the weights lie in the engine's own layout.
+template <int MODE, bool NAT>
 __global__ void __launch_bounds__(PF_BLOCK, 1) k_pf_gemm(const PfParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
     constexpr int NA = MODE == 1 ? 2 : 1;                      // weight tiles per stage
@@ -191,7 +234,8 @@ __global__ void __launch_bounds__(PF_BLOCK, 1) k_pf_gemm(const PfParams p) {
     const PfJob job = p.jobs[blockIdx.x];
     const int ft = blockIdx.y, KB = p.K / 256, nchunk = p.K / PF_KC;
     const uint8_t* W = job.w >= p.E ? p.Wsh : p.W + (size_t) (job.w - p.e_base) * p.expert_stride;
-    for (int i = tid; i < 512 * PF_REP; i += PF_BLOCK) table[i] = g_grid_pf[i / PF_REP];
+    if (!NAT)
+        for (int i = tid; i < 512 * PF_REP; i += PF_BLOCK) table[i] = g_grid_pf[i / PF_REP];
     if (tid < PF_N) {
         int src = -1, o = 0;
         if (tid < job.n) {
@@ -244,15 +288,17 @@ __global__ void __launch_bounds__(PF_BLOCK, 1) k_pf_gemm(const PfParams p) {
     } else {
         // 16 warps: warp w decodes tile row (w % 8) of the 128-feature slab; gate|up: of the gate (w < 8) or the up matrix
         // (all four sub-blocks of the chunk); down: sub-block pair w / 8 of the chunk
-        PfRaw raw, nxt;
+        using Raw = typename std::conditional<NAT, PfRawNat, PfRaw>::type;
+        Raw raw, nxt;
         const int sel = warp >> 3;
         const int trow = (MODE == 1 && sel ? p.rows / 16 : 0) + ft * (PF_M / 16) + (warp & 7);
         const int a_off = MODE == 1 && sel ? PF_TILE_A : 0, row0 = (warp & 7) * 16;
         // (a slab past the matrix's last tile row, when the features are not a multiple of 128, decodes zero weights)
         const bool live_row = MODE == 1 || trow < p.rows / 16;
-        auto load_raw = [&](int kb, PfRaw& r) {
-            if (live_row) pf_load_raw(W + ((size_t) trow * KB + kb) * TILE_BYTES, lane, r);
-            else r = PfRaw{};
+        const int n16 = (MODE == 1 ? 2 : 1) * (p.rows / 16);
+        auto load_raw = [&](int kb, Raw& r) {
+            if (live_row) pf_load_raw(NAT ? W + nat_half_at(trow, n16, kb, KB, MODE == 1) : W + ((size_t) trow * KB + kb) * TILE_BYTES, lane, r);
+            else r = Raw{};
         };
         load_raw(0, raw);
         // the activations of chunk c into its stage: 16-byte pieces (8 columns of one row = one core-matrix row) by async copies;
@@ -549,11 +595,33 @@ __global__ void __launch_bounds__(256) k_pf_decode_f16(const uint8_t* __restrict
         sub(std::integral_constant<int, 4>{}); sub(std::integral_constant<int, 5>{}); sub(std::integral_constant<int, 6>{}); sub(std::integral_constant<int, 7>{});
     }
 }
+// the same from n matrices in the engine's own layout, one after another; one warp per half tile
+__global__ void __launch_bounds__(256) k_pf_decode_nat(const uint8_t* __restrict__ W, size_t stride, int n, int rows, int K, int gate_up, __half* __restrict__ out) {
+    const int lane = threadIdx.x & 31, KB = K / 256, n16 = rows / 16;
+    const size_t per = (size_t) n16 * KB, nblk = (size_t) n * per;
+    const int g = lane >> 2, q = lane & 3;
+    for (size_t b = (size_t) blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5); b < nblk; b += (size_t) gridDim.x * (blockDim.x / 32)) {
+        const size_t m = b / per, i = b % per, trow = i / KB;
+        const int kb = (int) (i % KB);
+        PfRawNat r;
+        pf_load_raw(W + m * stride + nat_half_at(trow, n16, kb, KB, gate_up), lane, r);
+        __half* o0 = out + ((size_t) m * rows + trow * 16 + g) * K + (size_t) kb * 256 + 8 * q;
+        __half* o1 = o0 + (size_t) 8 * K;
+#pragma unroll
+        for (int sb = 0; sb < 8; ++sb) {
+            const __half2 f0 = __float2half2_rn(r.d0 * (float) (1 + 2 * (int) ((r.sn0 >> (4 * sb)) & 15u))), f1 = __float2half2_rn(r.d1 * (float) (1 + 2 * (int) ((r.sn1 >> (4 * sb)) & 15u)));
+            *reinterpret_cast<uint4*>(o0 + sb * 32) = pf_halves8_nat(r.w[0][sb], f0);
+            *reinterpret_cast<uint4*>(o1 + sb * 32) = pf_halves8_nat(r.w[1][sb], f1);
+        }
+    }
+}
 
-int pf_decode_f16_launch(const void* W, int rows, int K, __half* out, cudaStream_t st) {
-    const size_t nblk = (size_t) (rows / 16) * (K / 256);
+// n matrices of rows x K (tiles: one stacked matrix)
+static int pf_decode_f16_launch(const void* W, bool nat, size_t stride, int n, int rows, int K, int gate_up, __half* out, cudaStream_t st) {
+    const size_t nblk = (size_t) n * (rows / 16) * (K / 256);
     const unsigned blocks = (unsigned) (nblk / 8 < 148 * 8 ? (nblk + 7) / 8 : 148 * 8);
-    k_pf_decode_f16<<<blocks, 256, 0, st>>>((const uint8_t*) W, rows, K, out);
+    if (nat) k_pf_decode_nat<<<blocks, 256, 0, st>>>((const uint8_t*) W, stride, n, rows, K, gate_up, out);
+    else k_pf_decode_f16<<<blocks, 256, 0, st>>>((const uint8_t*) W, n * rows, K, out);
     FNX_LAUNCH_OK("k_pf_decode_f16");
     return FNX_OK;
 }
@@ -603,16 +671,16 @@ extern "C" size_t fnx_moe_prefill_scratch_bytes(int T, int K, int E, int H, int 
            (T >= 1024 ? pf_staged_bytes(pairs, E, H, F) : 0);
 }
 
-extern "C" int fnx_moe_prefill(const void* Wgu, size_t gu_stride, const void* Wdn, size_t dn_stride, const void* Wsh_gu, const void* Wsh_dn, int e_base,
-                               int E, int K, int e_lo, int e_hi, int add_shared, const int* topi, const float* topw, const float* logits, const float* x,
-                               const float* norm_w, float eps, int T, int H, int F, float* out, int accumulate, void* scratch, unsigned* err, fnx_stream st_) {
+namespace fnxb {
+int prompt_moe(const void* Wgu, size_t gu_stride, const void* Wsh_gu, bool gu_nat, const void* Wdn, size_t dn_stride, const void* Wsh_dn, bool dn_nat, int e_base, int E,
+               int K, int e_lo, int e_hi, int add_shared, const int* topi, const float* topw, const float* logits, const float* x, const float* norm_w, float eps, int T,
+               int H, int F, float* out, int accumulate, void* scratch, unsigned* err, cudaStream_t st) {
     FNX_REQUIRE(Wgu && Wdn && topi && topw && logits && x && out && scratch && err, "fnx_moe_prefill: null pointer");
     FNX_REQUIRE(T >= 1 && K >= 1 && K <= 32, "fnx_moe_prefill: %d rows, top %d", T, K);
     FNX_REQUIRE(E >= 1 && E <= 1024, "fnx_moe_prefill: %d experts (at most 1024)", E);
     FNX_REQUIRE(H % 256 == 0 && F % 256 == 0 && F % PF_M == 0 && H % PF_M == 0, "fnx_moe_prefill: hidden %d, ffn %d (multiples of 256)", H, F);
     FNX_REQUIRE(0 <= e_lo && e_lo <= e_hi && e_hi <= E && (!add_shared || (Wsh_gu && Wsh_dn)), "fnx_moe_prefill: expert range [%d, %d) of %d", e_lo, e_hi, E);
     FNX_REQUIRE((long long) T * K + T < (1ll << 30), "fnx_moe_prefill: %d rows are too many", T);
-    cudaStream_t st = as_stream(st_);
     const size_t pairs = (size_t) T * K + T;
     uint8_t* b = (uint8_t*) scratch;
     __half* hbuf = (__half*) b; b += pf_align(pairs * F * sizeof(__half));
@@ -638,15 +706,15 @@ extern "C" int fnx_moe_prefill(const void* Wgu, size_t gu_stride, const void* Wd
     FNX_LAUNCH_OK("k_pf_xnorm");
     // From 1,024 rows on, with every expert on this rank and stacked without gaps: the experts' matrices decoded to f16 once, the
     // rows copied into job order, and the two grouped products with both operands by tensor copies (gemm_tma.cu).
-    if (T >= 1024 && !pf_gemm_off() && e_base == 0 && e_lo == 0 && e_hi == E && add_shared && gu_stride == fnx_iq3s_bytes((size_t) 2 * F, (size_t) H) &&
-        dn_stride == fnx_iq3s_bytes((size_t) H, (size_t) F)) {
+    if (T >= 1024 && !pf_gemm_off() && e_base == 0 && e_lo == 0 && e_hi == E && add_shared && (gu_nat || gu_stride == fnx_iq3s_bytes((size_t) 2 * F, (size_t) H)) &&
+        (dn_nat || dn_stride == fnx_iq3s_bytes((size_t) H, (size_t) F))) {
         __half* xs = (__half*) b; b += pf_align(pairs * H * sizeof(__half));
         __half* gu16 = (__half*) b; b += pf_align((size_t) (E + 1) * 2 * F * H * sizeof(__half));
         __half* dn16 = (__half*) b;
-        FNX_TRY(pf_decode_f16_launch(Wgu, E * 2 * F, H, gu16, st));
-        FNX_TRY(pf_decode_f16_launch(Wsh_gu, 2 * F, H, gu16 + (size_t) E * 2 * F * H, st));
-        FNX_TRY(pf_decode_f16_launch(Wdn, E * H, F, dn16, st));
-        FNX_TRY(pf_decode_f16_launch(Wsh_dn, H, F, dn16 + (size_t) E * H * F, st));
+        FNX_TRY(pf_decode_f16_launch(Wgu, gu_nat, gu_stride, E, 2 * F, H, 1, gu16, st));
+        FNX_TRY(pf_decode_f16_launch(Wsh_gu, gu_nat, gu_stride, 1, 2 * F, H, 1, gu16 + (size_t) E * 2 * F * H, st));
+        FNX_TRY(pf_decode_f16_launch(Wdn, dn_nat, dn_stride, E, H, F, 0, dn16, st));
+        FNX_TRY(pf_decode_f16_launch(Wsh_dn, dn_nat, dn_stride, 1, H, F, 0, dn16 + (size_t) E * H * F, st));
         k_pf_gather_rows<<<(unsigned) pairs, 256, 0, st>>>(xh, order, n, K, H, xs);
         FNX_LAUNCH_OK("k_pf_gather_rows");
         const int nj = (int) ((size_t) n / PF_N) + ne + (T + PF_N - 1) / PF_N;
@@ -655,8 +723,10 @@ extern "C" int fnx_moe_prefill(const void* Wgu, size_t gu_stride, const void* Wd
         FNX_LAUNCH_OK("k_pf_combine");
         return FNX_OK;
     }
-    if (int rc = set_smem_limit((const void*) k_pf_gemm<0>, (int) pf_smem(0))) return rc;
-    if (int rc = set_smem_limit((const void*) k_pf_gemm<1>, (int) pf_smem(1))) return rc;
+    auto gu_kernel = gu_nat ? k_pf_gemm<1, true> : k_pf_gemm<1, false>;
+    auto dn_kernel = dn_nat ? k_pf_gemm<0, true> : k_pf_gemm<0, false>;
+    if (int rc = set_smem_limit((const void*) gu_kernel, (int) pf_smem(1))) return rc;
+    if (int rc = set_smem_limit((const void*) dn_kernel, (int) pf_smem(0))) return rc;
     // the job count is known on the device only: the grids cover the largest it can be (an expert's pairs in jobs of PF_N rows:
     // at most one ragged job per expert beyond pairs / PF_N) and the blocks past the count leave at once; nothing is read back
     {
@@ -664,16 +734,24 @@ extern "C" int fnx_moe_prefill(const void* Wgu, size_t gu_stride, const void* Wd
         PfParams p{};
         p.W = (const uint8_t*) Wgu; p.expert_stride = gu_stride; p.e_base = e_base; p.E = E; p.Wsh = (const uint8_t*) Wsh_gu;
         p.jobs = jobs; p.njobs = njobs; p.order = order; p.TKp = n; p.Kp = K; p.x = xh; p.rows = F; p.K = H; p.outh = hbuf; p.err = err;
-        k_pf_gemm<1><<<dim3(nj, F / PF_M), PF_BLOCK, pf_smem(1), st>>>(p);
+        gu_kernel<<<dim3(nj, F / PF_M), PF_BLOCK, pf_smem(1), st>>>(p);
         FNX_LAUNCH_OK("k_pf_gemm (gate|up)");
         p.W = (const uint8_t*) Wdn; p.expert_stride = dn_stride; p.Wsh = (const uint8_t*) Wsh_dn;
         p.x = hbuf; p.rows = H; p.K = F; p.out = part; p.outh = nullptr;
-        k_pf_gemm<0><<<dim3(nj, H / PF_M), PF_BLOCK, pf_smem(0), st>>>(p);
+        dn_kernel<<<dim3(nj, H / PF_M), PF_BLOCK, pf_smem(0), st>>>(p);
         FNX_LAUNCH_OK("k_pf_gemm (down)");
     }
     k_pf_combine<<<dim3((H / 4 + 255) / 256, T), 256, 0, st>>>(part, topi, topw, logits, T, E, H, K, e_lo, e_hi, add_shared, out, accumulate);
     FNX_LAUNCH_OK("k_pf_combine");
     return FNX_OK;
+}
+}  // namespace fnxb
+
+extern "C" int fnx_moe_prefill(const void* Wgu, size_t gu_stride, const void* Wdn, size_t dn_stride, const void* Wsh_gu, const void* Wsh_dn, int e_base,
+                               int E, int K, int e_lo, int e_hi, int add_shared, const int* topi, const float* topw, const float* logits, const float* x,
+                               const float* norm_w, float eps, int T, int H, int F, float* out, int accumulate, void* scratch, unsigned* err, fnx_stream st) {
+    return prompt_moe(Wgu, gu_stride, Wsh_gu, false, Wdn, dn_stride, Wsh_dn, false, e_base, E, K, e_lo, e_hi, add_shared, topi, topw, logits, x, norm_w, eps, T, H, F, out,
+                      accumulate, scratch, err, as_stream(st));
 }
 
 // ------------------------------------------------------------------------------------------------ dense product for prompts
@@ -693,11 +771,11 @@ extern "C" size_t fnx_dense_prompt_scratch_bytes(int T, int rows, int cols) {
            pf_align((size_t) rows * cols * sizeof(__half));
 }
 
-extern "C" int fnx_dense_prompt(const void* W, int rows, int cols, const float* x, int T, const float* norm_w, float eps, float* y, int ldy, int accumulate,
-                                void* scratch, unsigned* err, fnx_stream st_) {
+namespace fnxb {
+int prompt_dense(const void* W, bool nat, int rows, int cols, const float* x, int T, const float* norm_w, float eps, float* y, int ldy, int accumulate, void* scratch,
+                 unsigned* err, cudaStream_t st) {
     FNX_REQUIRE(W && x && y && scratch && err, "fnx_dense_prompt: null pointer");
     FNX_REQUIRE(T >= 1 && rows >= 16 && rows % 16 == 0 && cols >= 256 && cols % 256 == 0 && ldy >= rows, "fnx_dense_prompt: %d rows x %d columns over %d rows", rows, cols, T);
-    cudaStream_t st = as_stream(st_);
     uint8_t* b = (uint8_t*) scratch;
     __half* xh = (__half*) b; b += pf_align((size_t) T * cols * sizeof(__half));
     int* order = (int*) b; b += pf_align((size_t) T * sizeof(int));
@@ -708,17 +786,24 @@ extern "C" int fnx_dense_prompt(const void* W, int rows, int cols, const float* 
     k_pf_xnorm<<<T, 256, 0, st>>>(x, norm_w, cols, eps, xh);
     FNX_LAUNCH_OK("k_pf_xnorm");
     if (T >= pf_tma_rows()) {   // the matrix to f16 once, then one product with both operands by tensor copies
-        FNX_TRY(pf_decode_f16_launch(W, rows, cols, w16, st));
+        FNX_TRY(pf_decode_f16_launch(W, nat, 0, 1, rows, cols, 0, w16, st));
         return gemm_tma_launch(w16, nullptr, xh, nullptr, y, ldy, T, rows, cols, accumulate, 1.0f, err, st);
     }
     k_pf_dense_jobs<<<(T + 255) / 256, 256, 0, st>>>(T, jobs, njobs, order);
     FNX_LAUNCH_OK("k_pf_dense_jobs");
-    if (int rc = set_smem_limit((const void*) k_pf_gemm<0>, (int) pf_smem(0))) return rc;
+    auto kernel = nat ? k_pf_gemm<0, true> : k_pf_gemm<0, false>;
+    if (int rc = set_smem_limit((const void*) kernel, (int) pf_smem(0))) return rc;
     PfParams p{};
     p.W = (const uint8_t*) W; p.expert_stride = 0; p.e_base = 0; p.E = 1; p.Wsh = nullptr;
     p.jobs = jobs; p.njobs = njobs; p.order = order; p.TKp = T; p.Kp = 1; p.x = xh; p.rows = rows; p.K = cols; p.out = y; p.outh = nullptr; p.err = err;
     p.ldo = ldy; p.accumulate = accumulate;
-    k_pf_gemm<0><<<dim3(nj, (rows + PF_M - 1) / PF_M), PF_BLOCK, pf_smem(0), st>>>(p);
+    kernel<<<dim3(nj, (rows + PF_M - 1) / PF_M), PF_BLOCK, pf_smem(0), st>>>(p);
     FNX_LAUNCH_OK("k_pf_gemm (dense)");
     return FNX_OK;
+}
+}  // namespace fnxb
+
+extern "C" int fnx_dense_prompt(const void* W, int rows, int cols, const float* x, int T, const float* norm_w, float eps, float* y, int ldy, int accumulate,
+                                void* scratch, unsigned* err, fnx_stream st) {
+    return prompt_dense(W, false, rows, cols, x, T, norm_w, eps, y, ldy, accumulate, scratch, err, as_stream(st));
 }

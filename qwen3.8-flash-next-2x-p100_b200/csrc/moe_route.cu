@@ -10,7 +10,7 @@
 #include <cstdlib>
 
 #include "moe_route.cuh"
-#include "mmv_core.cuh"
+#include "nat_image.cuh"
 
 namespace fnxb {
 
@@ -379,6 +379,59 @@ __global__ void __launch_bounds__(32) k_combine_image(const float* __restrict__ 
             if (lane < 2) scales[(size_t) (ng * KB + blk) * 8 + n + 4 * lane] = 0.f;
             if (lane == 2) rs[td * 16 + blk] = 0.f;
         }
+}
+
+// k_combine for an engine's window: the new rows' image (nat_image.cuh) for the next projection rides along.  One warp per (256-column
+// block, row); the addends' loads are in flight together, sixteen picks at a time.
+__global__ void __launch_bounds__(32) k_combine_nat(const float* __restrict__ part, const int* __restrict__ topi, const float* __restrict__ topw,
+                                                    const float* __restrict__ logits, int T, int E, int H, int K, float* __restrict__ out, uint8_t* __restrict__ img,
+                                                    const float* __restrict__ img_norm_w) {
+    const int blk = blockIdx.x, t = blockIdx.y, lane = threadIdx.x, KB = H / 256;
+    const size_t col = (size_t) blk * 256 + lane * 8;
+    pdl_wait();
+    pdl_launch_dependents();
+    float* dst = out + (size_t) t * H + col;
+    const float4 o0 = *reinterpret_cast<const float4*>(dst), o1 = *reinterpret_cast<const float4*>(dst + 4);
+    const float shl = logits[(size_t) t * (E + 1) + E], mw = lane < K ? topw[t * K + lane] : 0.f;
+    const float4* sh = reinterpret_cast<const float4*>(part + ((size_t) T * K + t) * H + col);
+    const float4 h0 = sh[0], h1 = sh[1];
+    unsigned long long s[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s[i] = 0ull;
+    for (int k0 = 0; k0 < K; k0 += 16) {
+        float4 a[16][2];
+#pragma unroll
+        for (int k = 0; k < 16; ++k)
+            if (k0 + k < K) {
+                const float4* src = reinterpret_cast<const float4*>(part + ((size_t) t * K + k0 + k) * H + col);
+                a[k][0] = src[0];
+                a[k][1] = src[1];
+            }
+#pragma unroll
+        for (int k = 0; k < 16; ++k)
+            if (k0 + k < K) {
+                const float wk = __shfl_sync(0xffffffffu, mw, k0 + k);
+                const float e8[8] = {a[k][0].x, a[k][0].y, a[k][0].z, a[k][0].w, a[k][1].x, a[k][1].y, a[k][1].z, a[k][1].w};
+#pragma unroll
+                for (int i = 0; i < 8; ++i) s[i] += fix_from_float(wk * e8[i]);
+            }
+    }
+    const float g = sigmoidf_(shl);
+    const float e8[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
+    float v[8] = {o0.x, o0.y, o0.z, o0.w, o1.x, o1.y, o1.z, o1.w};
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] += fix_to_float(s[i] + fix_from_float(g * e8[i]));
+    *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+    *reinterpret_cast<float4*>(dst + 4) = make_float4(v[4], v[5], v[6], v[7]);
+    const float ss = ni_norm8(v, img_norm_w + col);
+    ni_quant(img, KB, v, ss, t, blk, lane);
+}
+
+int moe_combine_nat(const float* part, const int* topi, const float* topw, const float* logits, int T, int E, int H, int K, float* R, uint8_t* img, const float* img_norm_w,
+                    cudaStream_t st) {
+    FNX_REQUIRE(T >= 1 && T <= FNX_MAX_ROWS && K >= 1 && K <= 32 && H % 256 == 0, "moe_combine_nat: %d rows of %d, top %d", T, H, K);
+    const cudaError_t le = launch_dep(k_combine_nat, dim3(H / 256, T), dim3(32), 0, st, part, topi, topw, logits, T, E, H, K, R, img, img_norm_w);
+    return le == cudaSuccess ? FNX_OK : fail(FNX_E_CUDA, "k_combine_nat: launch failed: %s", cudaGetErrorString(le));
 }
 
 }  // namespace fnxb

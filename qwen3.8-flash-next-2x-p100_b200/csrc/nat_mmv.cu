@@ -1,0 +1,682 @@
+// The windows' matrix x few-rows products on the engine's own weight layout (nat_tile.h): dense projections, the experts' gate|up with
+// SwiGLU, and down.  The arithmetic is that of iq3s_mmv.cu (integer products of exact odd weights with two-level int8 activations,
+// integer sub-block scales, float scales once per 256-column block); what differs is everything around it:
+//   - no codebook: an operand register is a mask (and a shift) of the stored nibbles, so an item (one 16 x 256 tile against the rows)
+//     takes about 200 warp instructions for four rows instead of about 600, and a block needs no 64 KB table;
+//   - the rows come as their image (nat_image.cuh): a dense or gate|up block copies the rows it needs into shared memory and quantises
+//     nothing (read through L1 from global memory instead, the operands cost more than the weights); down quantises its few rows itself;
+//   - every lane copies its own 64 bytes of the next tiles into shared memory (cp.async): no mbarriers, no issuing lane;
+//   - a block takes half an SM's registers and shared memory at most, so that the next kernel of the window can be resident while
+//     this one drains (programmatic dependent launch): its first tiles are on their way before the rows it waits for are written.
+// Bound by HBM for the large expert products, by the launch and its dependent loads for the small dense ones.
+#include <cooperative_groups.h>
+#include <cuda_fp16.h>
+#include <cuda_runtime.h>
+
+#include "fnx_common.cuh"
+#include "iq3s_grid.h"
+#include "nat_image.cuh"
+#include "nat_tile.h"
+
+namespace cg = cooperative_groups;
+
+namespace fnxb {
+
+__device__ static const uint32_t g_grid_nat[512] = {FNX_IQ3S_GRID_VALUES};
+
+struct NatParams {
+    const uint8_t* W;
+    size_t expert_stride;
+    int e_base;
+    const uint8_t* Wsh;
+    int E;
+    const fnx_job* jobs;
+    const int* njobs;
+    int njobs_max;
+    int T;
+    const uint8_t* img;
+    int normed;
+    float eps;
+    const float* x;      // down: h rows
+    float* out;
+    int ldo;
+    int rows, K;         // output rows per job (gate|up: F), columns
+    int accumulate;
+    int rmax;            // expert modes: rows a block holds at once
+    int umax;            // dense with split columns: units of a cluster
+};
+
+template <int NG, int MODE>
+struct NatPiece {
+    using AccT = typename MatAcc<MODE>::type;
+    int unit;            // -1: none, -2: the warp had no items at all
+    int b_hi;
+    AccT v[2 * NG * 64];   // [half][group][16 lanes][4]
+};
+
+__device__ __forceinline__ void nm_mma(int (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+        : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(0));
+}
+
+// four nibbles of x -> bytes 8 m = 16 t + 8 (the high ones as they lie, the low ones shifted up)
+__device__ __forceinline__ uint32_t nm_hi(uint32_t x) { return (x & 0xF0F0F0F0u) | 0x08080808u; }
+__device__ __forceinline__ uint32_t nm_lo(uint32_t x) { return ((x * 16u) & 0xF0F0F0F0u) | 0x08080808u; }
+
+// the two rows' eight sub-block scales 1 + 2 s as bytes: even sub-blocks in .x, odd ones in .y
+struct NmScales {
+    uint2 r0, r1;
+};
+__device__ __forceinline__ uint2 nm_scale_bytes(uint32_t n) {
+    return make_uint2((n & 0x0F0F0F0Fu) * 2u + 0x01010101u, ((n >> 4) & 0x0F0F0F0Fu) * 2u + 0x01010101u);
+}
+template <int H>
+__device__ __forceinline__ NmScales nm_scales(uint32_t am) {
+    const uint2 sn = lds_v2<H * NAT_HALF_BYTES + NAT_META>(am);
+    return NmScales{nm_scale_bytes(sn.x), nm_scale_bytes(sn.y)};
+}
+// One half of a tile (16 rows) over four sub-blocks (4 hf ..): decoded operands and the two rows' sub-block scales
+struct NmHalf {
+    uint32_t a[4][4];
+    int f0[4], f1[4];
+};
+template <int H>
+__device__ __forceinline__ void nm_decode(uint32_t a16, const NmScales& sc, int hf, NmHalf& w) {
+    const uint4 w0 = lds_v4<H * NAT_HALF_BYTES>(a16 + hf * 512), w1 = lds_v4<H * NAT_HALF_BYTES + 1024>(a16 + hf * 512);
+    const uint32_t wa[4] = {w0.x, w0.y, w0.z, w0.w}, wb[4] = {w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        w.a[k][0] = nm_lo(wa[k]);
+        w.a[k][1] = nm_lo(wb[k]);
+        w.a[k][2] = nm_hi(wa[k]);
+        w.a[k][3] = nm_hi(wb[k]);
+        const uint32_t sel = 0x4440u + 2 * hf + (k >> 1);   // sub-block 4 hf + k: byte 2 hf + k / 2 of the even or the odd ones
+        asm("prmt.b32 %0, %1, %2, %3;" : "=r"(w.f0[k]) : "r"(k & 1 ? sc.r0.y : sc.r0.x), "r"(0u), "r"(sel));
+        asm("prmt.b32 %0, %1, %2, %3;" : "=r"(w.f1[k]) : "r"(k & 1 ? sc.r1.y : sc.r1.x), "r"(0u), "r"(sel));
+    }
+}
+__device__ __forceinline__ void nm_products(const NmHalf& w, const uint4& x0, const uint4& x1, int (&accI)[4]) {
+    const uint32_t b[4][2] = {{x0.x, x0.y}, {x0.z, x0.w}, {x1.x, x1.y}, {x1.z, x1.w}};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        int c[4];
+        nm_mma(c, w.a[k], b[k][0], b[k][1]);
+        accI[0] += w.f0[k] * c[0];
+        accI[1] += w.f0[k] * c[1];
+        accI[2] += w.f1[k] * c[2];
+        accI[3] += w.f1[k] * c[3];
+    }
+}
+template <int H, typename AccT>
+__device__ __forceinline__ void nm_flush(uint32_t am, float s0, float s1, const int (&accI)[4], AccT (&acc)[4]) {
+    const uint32_t dw = lds_u32<H * NAT_HALF_BYTES + NAT_META + 8>(am);
+    const float2 d = __half22float2(*reinterpret_cast<const __half2*>(&dw));
+    const float d0 = d.x * 0.125f, d1 = d.y * 0.125f;   // (exact: the integers are 8 times the sums)
+    if constexpr (sizeof(AccT) == 8) {
+        acc[0] += (double) (d0 * s0) * (double) accI[0];
+        acc[1] += (double) (d0 * s1) * (double) accI[1];
+        acc[2] += (double) (d1 * s0) * (double) accI[2];
+        acc[3] += (double) (d1 * s1) * (double) accI[3];
+    } else {
+        acc[0] += d0 * s0 * (float) accI[0];
+        acc[1] += d0 * s1 * (float) accI[1];
+        acc[2] += d1 * s0 * (float) accI[2];
+        acc[3] += d1 * s1 * (float) accI[3];
+    }
+}
+template <int H, int NG, typename AccT>
+__device__ __forceinline__ void nm_half_item(uint32_t a16, uint32_t am, uint32_t xb, uint32_t x0, uint32_t x1, uint32_t group, AccT (&acc)[NG][4]) {
+    int accI[NG][4];
+#pragma unroll
+    for (int ng = 0; ng < NG; ++ng)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) accI[ng][i] = 0;
+    const NmScales sc = nm_scales<H>(am);
+#pragma unroll 1
+    for (int hf = 0; hf < 2; ++hf) {
+        NmHalf w;
+        nm_decode<H>(a16, sc, hf, w);
+#pragma unroll
+        for (int ng = 0; ng < NG; ++ng) nm_products(w, lds_v4(xb + ng * group + hf * 128), lds_v4<64>(xb + ng * group + hf * 128), accI[ng]);
+    }
+#pragma unroll
+    for (int ng = 0; ng < NG; ++ng) nm_flush<H>(am, lds_f32(x0 + ng * group), lds_f32(x1 + ng * group), accI[ng], acc[ng]);
+}
+
+// One item: the tile at shared address tile_s against one block of the rows; adds into acc[half][ng][0..3] = (row g, column 2 q),
+// (g, 2 q + 1), (g + 8, 2 q), (g + 8, 2 q + 1).  xb: shared address of the lane's cells in its column's row of group 0, x0 / x1: of its
+// two C columns' scales; groups lie `group` bytes apart.  The integers are exact (8 times the sums of iq3s_mmv.cu's items).
+// AccT double (expert modes): the rounded result does not depend on where a row's K-sum was cut, as there.
+// Up to two row groups load the rows' operands once for both half tiles; more would not leave the registers.  (The loops over four
+// sub-blocks stay rolled: unrolled, every load would be hoisted into registers.)
+template <int NG, typename AccT>
+__device__ __forceinline__ void nm_item(uint32_t tile_s, uint32_t xb, uint32_t x0, uint32_t x1, uint32_t group, int lane, AccT (&acc)[2][NG][4]) {
+    const uint32_t a16 = tile_s + lane * 16, am = tile_s + (lane >> 2) * 16;
+    if constexpr (NG > 2) {
+        nm_half_item<0, NG>(a16, am, xb, x0, x1, group, acc[0]);
+        nm_half_item<1, NG>(a16, am, xb, x0, x1, group, acc[1]);
+    } else {
+        int accI[2][NG][4];
+#pragma unroll
+        for (int i = 0; i < 2 * NG * 4; ++i) accI[i / (4 * NG)][(i / 4) % NG][i & 3] = 0;
+        const NmScales sc0 = nm_scales<0>(am), sc1 = nm_scales<1>(am);
+#pragma unroll 1
+        for (int hf = 0; hf < 2; ++hf) {
+            uint4 b0[NG], b1[NG];
+#pragma unroll
+            for (int ng = 0; ng < NG; ++ng) {
+                b0[ng] = lds_v4(xb + ng * group + hf * 128);
+                b1[ng] = lds_v4<64>(xb + ng * group + hf * 128);
+            }
+            {
+                NmHalf w;
+                nm_decode<0>(a16, sc0, hf, w);
+#pragma unroll
+                for (int ng = 0; ng < NG; ++ng) nm_products(w, b0[ng], b1[ng], accI[0][ng]);
+            }
+            {
+                NmHalf w;
+                nm_decode<1>(a16, sc1, hf, w);
+#pragma unroll
+                for (int ng = 0; ng < NG; ++ng) nm_products(w, b0[ng], b1[ng], accI[1][ng]);
+            }
+        }
+#pragma unroll
+        for (int ng = 0; ng < NG; ++ng) {
+            const float s0 = lds_f32(x0 + ng * group), s1 = lds_f32(x1 + ng * group);
+            nm_flush<0>(am, s0, s1, accI[0][ng], acc[0][ng]);
+            nm_flush<1>(am, s0, s1, accI[1][ng], acc[1][ng]);
+        }
+    }
+}
+
+// the results of a unit, held by threads q < 2; rf: lane i holds 1 / rms of row i (normed rows; else 1); orow: the job's output rows
+template <int NG, int MODE, typename AccT>
+__device__ __forceinline__ void nm_write(const NatParams& p, int lu, const int* orow, int ntok, float rf, int lane, const AccT (&acc)[2][NG][4]) {
+    const int g = lane >> 2, q = lane & 3;
+#pragma unroll
+    for (int ng = 0; ng < NG; ++ng)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int tok = 4 * ng + 2 * (q & 1) + (k & 1);
+            const float r = MODE == MAT_DOWN ? 1.0f : __shfl_sync(0xffffffffu, rf, tok);
+            if (q >= 2 || tok >= ntok) continue;
+            float* out = p.out + (size_t) (MODE == MAT_DENSE ? tok : orow[tok]) * p.ldo;
+            if (MODE == MAT_GATEUP) {
+                out[lu * 16 + g + 8 * (k >> 1)] = siluf_((float) acc[0][ng][k] * r) * ((float) acc[1][ng][k] * r);
+            } else {
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int row = lu * 32 + h * 16 + g + 8 * (k >> 1);
+                    const float v = MODE == MAT_DOWN ? (float) acc[h][ng][k] : (float) acc[h][ng][k] * r;
+                    if (row < p.rows) out[row] = MODE == MAT_DENSE && p.accumulate ? out[row] + v : v;
+                }
+            }
+        }
+}
+
+// 1 / rms of a row from its image (shared address of its first block)
+__device__ __forceinline__ float nm_row_factor(uint32_t row_s, int KB, float eps) {
+    float ss = 0.f;
+    for (int c = 0; c < KB; ++c) ss += lds_f32<NI_RS>(row_s + c * NI_BYTES);
+    return rsqrtf(ss / (float) (KB * 256) + eps);
+}
+
+// A block's items are the tiles of units [u0, u1) (a unit: one tile row across the columns), dealt to its warps in equal contiguous
+// shares (mmv_core.cuh: units cut by share boundaries leave their pieces in shared memory, and after one barrier the warp with a
+// unit's first piece adds the others in warp order).
+// C > 1 (dense, long rows): C blocks of a cluster share the units and split the columns, each holding its part of the rows' image;
+// the partial sums are added in block order through distributed shared memory.  A 2048 x 4096 product at five rows would otherwise
+// have every block copy 48 KB of image for one unit.
+template <int NG, int MODE, int NW, int SLOTS, int C>
+__device__ __forceinline__ void nm_body(const NatParams& p, uint8_t* smem) {
+    using AccT = typename MatAcc<MODE>::type;
+    using Piece = NatPiece<NG, MODE>;
+    constexpr bool MOE = MODE != MAT_DENSE;
+    constexpr int NT = NW * 32;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int KB = p.K / 256, KBc = KB / C, nbu = KBc, upj = MODE == MAT_GATEUP ? p.rows / 16 : (p.rows + 31) / 32;
+    const int crank = C > 1 ? (int) (blockIdx.x % C) : 0, bid = C > 1 ? (int) (blockIdx.x / C) : (int) blockIdx.x, nblk = (int) gridDim.x / C;
+    const uint32_t RS = (uint32_t) ni_row_bytes(KBc);
+    Piece* pieces = reinterpret_cast<Piece*>(smem + (size_t) NW * SLOTS * NAT_TILE_BYTES);   // [NW][2]
+    uint8_t* pool = reinterpret_cast<uint8_t*>(pieces + NW * 2);                             // row images
+    const int pool_rows = MOE ? p.rmax + 3 : 4 * NG;                                         // (a group's missing rows are read and dropped)
+    fnx_job* jobs_s = reinterpret_cast<fnx_job*>(pool + (size_t) pool_rows * RS);
+    float* ub = reinterpret_cast<float*>(pool + (size_t) pool_rows * RS);                    // C > 1: the units' partial sums
+    const uint32_t slots_s = smem_u32(smem) + (uint32_t) warp * (SLOTS * NAT_TILE_BYTES), pool_s = smem_u32(pool);
+    // gate|up: the job list is the previous kernel's; down: it is older than the kernel whose rows this one waits for, and that
+    // kernel lets dependents start only once it has itself waited for the list
+    if (MODE == MAT_GATEUP) {
+        pdl_wait();
+        pdl_launch_dependents();
+    }
+    int njobs = 1;
+    if (MOE) {
+        njobs = min(__ldcg(p.njobs), p.njobs_max);
+        const int n8 = p.njobs_max * (int) sizeof(fnx_job) / 8;   // 40 bytes a job
+        for (int i = tid; i < n8; i += NT) reinterpret_cast<uint2*>(jobs_s)[i] = __ldcg(reinterpret_cast<const uint2*>(p.jobs) + i);
+        __syncthreads();
+    }
+    const unsigned total = (unsigned) njobs * upj;
+    const int u0 = (int) (total * bid / nblk), u1 = (int) (total * (bid + 1) / nblk);
+    bool waited = MODE == MAT_GATEUP;
+    for (int uc = u0; uc < u1 || !waited;) {
+        // the pass's jobs: as many as fit the row pool
+        const int j0 = uc / upj;
+        int j1 = njobs, nrow = p.T;
+        if (MOE) {
+            const int jend = uc < u1 ? (u1 - 1) / upj + 1 : j0;
+            nrow = 0;
+            for (j1 = j0; j1 < jend; ++j1) {
+                const int n = min(jobs_s[j1].n, 4);
+                if (j1 > j0 && nrow + n > p.rmax) break;
+                nrow += n;
+            }
+        }
+        const int ue = min(u1, j1 * upj);
+        const unsigned N = ue > uc ? (unsigned) (ue - uc) * nbu : 0u;
+        const int i0 = (int) (N * warp / NW), i1 = (int) (N * (warp + 1) / NW);
+        if (MODE == MAT_GATEUP) {   // the jobs' rows
+            const int per = KB * (NI_BYTES / 16);
+            for (int i = tid; i < nrow * per; i += NT) {
+                int r = i / per, j = j0;
+                const int at = i - r * per, dr = r;
+                for (int n; r >= (n = min(jobs_s[j].n, 4)); ++j) r -= n;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(pool_s + dr * RS + at * 16), "l"(p.img + (size_t) jobs_s[j].y[r] * RS + at * 16) : "memory");
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        }
+        // ---- the copies run ahead of the items: each lane's 128 bytes of a tile, and one of eight lanes' 32 bytes of its scales
+        auto job_base = [&](int j) {
+            if (!MOE) return p.W;
+            const int e = jobs_s[j].w;
+            return e >= p.E ? p.Wsh : p.W + (size_t) (e - p.e_base) * p.expert_stride;
+        };
+        // the next item to fetch: block ab of unit au (of the job, in expert modes)
+        int aj = MOE ? (uc + i0 / nbu) / upj : 0, au = MOE ? (uc + i0 / nbu) % upj : uc + i0 / nbu, ab = i0 % nbu;
+        const uint8_t* asrc = i0 < i1 ? job_base(aj) + ((size_t) au * KB + crank * KBc + ab) * NAT_TILE_BYTES + lane * 16 : nullptr;
+        auto fetch = [&](int item, int into) {   // (items in order, every one once)
+            if (item < i1) {
+                const uint32_t dst = slots_s + (uint32_t) (into * NAT_TILE_BYTES + lane * 16);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + h * NAT_HALF_BYTES + j * 512), "l"(asrc + h * NAT_HALF_BYTES + j * 512) : "memory");
+                    if (lane < 8)
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + h * NAT_HALF_BYTES + NAT_META), "l"(asrc + h * NAT_HALF_BYTES + NAT_META) : "memory");
+                }
+                asrc += NAT_TILE_BYTES;
+                if (MOE || C > 1) {
+                    if (++ab == nbu) {
+                        ab = 0;
+                        if (C > 1) asrc += (size_t) (KB - KBc) * NAT_TILE_BYTES;
+                        if (MOE && ++au == upj) {
+                            au = 0;
+                            ++aj;
+                            if (item + 1 < i1) asrc = job_base(aj) + lane * 16;
+                        }
+                    }
+                }
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+#pragma unroll
+        for (int k = 0; k < SLOTS; ++k) fetch(i0 + k, k);
+        if (!waited) {
+            pdl_wait();   // from here on: what the previous kernel wrote (the rows)
+            pdl_launch_dependents();
+            waited = true;
+            if (C == 1 && u0 >= u1) break;
+        }
+        if (MODE == MAT_DENSE) {
+            const int per = KBc * (NI_BYTES / 16);
+            const uint8_t* src = p.img + (size_t) crank * KBc * NI_BYTES;
+            const size_t grs = ni_row_bytes(KB);
+            for (int i = tid; i < nrow * per; i += NT) {
+                const int r = i / per, at = i - r * per;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(pool_s + r * RS + at * 16), "l"(src + r * grs + at * 16) : "memory");
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        } else if (MODE == MAT_DOWN) {   // the rows of the pass's jobs, quantised here (two 256-column blocks a row at 512 columns)
+            for (int id = warp; id < nrow * KB; id += NW) {
+                int r = id % nrow, j = j0;
+                const int dr = r, blk = id / nrow;
+                for (int n; r >= (n = min(jobs_s[j].n, 4)); ++j) r -= n;
+                const float* src = p.x + (size_t) jobs_s[j].out[r] * p.K + blk * 256 + lane * 8;
+                const float4 a = *reinterpret_cast<const float4*>(src), b = *reinterpret_cast<const float4*>(src + 4);
+                const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+                ni_quant_at(pool + dr * RS + blk * NI_BYTES, v, 0.f, lane);
+            }
+        } else {
+            asm volatile("cp.async.wait_group %0;" ::"n"(SLOTS) : "memory");   // the rows were the first group
+        }
+        __syncthreads();
+        Piece* mine = pieces + warp * 2;
+        if (lane == 0) {
+            mine[0].unit = i0 < i1 ? -1 : -2;
+            mine[1].unit = -1;
+        }
+        // the lane's columns: row n & 3 of its group at level n / 4
+        const int g = lane >> 2, q = lane & 3;
+        const uint32_t xb0 = pool_s + (uint32_t) (g & 3) * RS + (uint32_t) (g >> 2) * 256u + q * 16;
+        const uint32_t x00 = pool_s + (uint32_t) ((2 * q) & 3) * RS + NI_SCALE + (uint32_t) (q >> 1) * 4u, x10 = x00 + RS;
+        uint32_t jrow = 0;   // expert modes: the current job's first row in the pool
+        int cur_job = -1, ntok = p.T, b_lo = 0;
+        float rf = 1.0f;
+        if (MODE == MAT_DENSE && p.normed && lane < p.T) rf = nm_row_factor(pool_s + lane * RS, KB, p.eps);   // (normed rows are never split: C == 1)
+        AccT acc[2][NG][4];
+        int b = i0 % nbu, u = uc + i0 / nbu, slot = 0;
+        // a unit's sums: written, or (columns split) left for the cluster
+        auto done = [&](int unit) {
+            if (C > 1) {
+                if ((lane & 3) < 2) {
+                    const int l16 = (lane >> 2) * 2 + (lane & 3);
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+#pragma unroll
+                        for (int ng = 0; ng < NG; ++ng)
+                            *reinterpret_cast<float4*>(ub + (((size_t) (unit - u0) * 2 + h) * NG + ng) * 64 + l16 * 4) =
+                                make_float4((float) acc[h][ng][0], (float) acc[h][ng][1], (float) acc[h][ng][2], (float) acc[h][ng][3]);
+                }
+            } else {
+                nm_write<NG, MODE, AccT>(p, MOE ? unit % upj : unit, MOE ? jobs_s[unit / upj].out : nullptr, ntok, rf, lane, acc);
+            }
+        };
+        for (int s = i0; s < i1; ++s) {
+            if (b == 0 || s == i0) {
+                b_lo = b;
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int ng = 0; ng < NG; ++ng)
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) acc[h][ng][k] = 0;
+                if (MOE && u / upj != cur_job) {
+                    cur_job = u / upj;
+                    int r = 0;
+                    for (int j = j0; j < cur_job; ++j) r += min(jobs_s[j].n, 4);
+                    jrow = (uint32_t) r * RS;
+                    ntok = min(jobs_s[cur_job].n, 4);
+                    if (MODE == MAT_GATEUP && p.normed) rf = lane < ntok ? nm_row_factor(pool_s + jrow + lane * RS, KB, p.eps) : 1.0f;
+                }
+            }
+            asm volatile("cp.async.wait_group %0;" ::"n"(SLOTS - 1) : "memory");
+            __syncwarp();   // (the scales came in by other lanes' copies)
+            const uint32_t off = jrow + (uint32_t) b * NI_BYTES;
+            nm_item<NG, AccT>(slots_s + (uint32_t) (slot * NAT_TILE_BYTES), xb0 + off, x00 + off, x10 + off, 4u * RS, lane, acc);
+            __syncwarp();   // every lane is done with the slot
+            fetch(s + SLOTS, slot);
+            slot = slot + 1 == SLOTS ? 0 : slot + 1;
+            if (b == nbu - 1 || s == i1 - 1) {
+                // level 1 (threads q = 0, 1) + level 2 (q = 2, 3) of the same rows
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int ng = 0; ng < NG; ++ng)
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) acc[h][ng][k] += __shfl_xor_sync(0xffffffffu, acc[h][ng][k], 2);
+                if (b_lo == 0 && b == nbu - 1) {
+                    done(u);
+                } else {
+                    Piece* ps = mine + (b_lo == 0 ? 1 : 0);
+                    if (lane == 0) {
+                        ps->unit = u;
+                        ps->b_hi = b + 1;
+                    }
+                    if ((lane & 3) < 2) {
+                        const int l16 = (lane >> 2) * 2 + (lane & 3);
+#pragma unroll
+                        for (int h = 0; h < 2; ++h)
+#pragma unroll
+                            for (int ng = 0; ng < NG; ++ng)
+#pragma unroll
+                                for (int k = 0; k < 4; ++k) ps->v[((h * NG + ng) * 16 + l16) * 4 + k] = acc[h][ng][k];
+                    }
+                }
+            }
+            if (++b == nbu) {
+                b = 0;
+                ++u;
+            }
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+        {   // units cut by share boundaries (the warp's last unit: ntok and rf are those of its job)
+            const Piece* first = pieces + warp * 2 + 1;
+            const int fu = first->unit;
+            if (fu >= 0) {
+                const int l16 = (lane >> 2) * 2 + (lane & 3);
+                const bool holder = (lane & 3) < 2;
+#pragma unroll
+                for (int i = 0; i < 2 * NG * 4; ++i) acc[i / (4 * NG)][(i / 4) % NG][i & 3] = holder ? first->v[((i / 4) * 16 + l16) * 4 + (i & 3)] : (AccT) 0;
+                for (int ww = warp + 1; ww < NW; ++ww) {
+                    const Piece* c = pieces + ww * 2;
+                    if (c->unit == -2) continue;
+                    if (c->unit != fu) break;
+                    if (holder)
+#pragma unroll
+                        for (int i = 0; i < 2 * NG * 4; ++i) acc[i / (4 * NG)][(i / 4) % NG][i & 3] += c->v[((i / 4) * 16 + l16) * 4 + (i & 3)];
+                    if (c->b_hi == nbu) break;
+                }
+                done(fu);
+            }
+        }
+        uc = ue;
+        if (uc < u1) __syncthreads();   // the row images and the pieces are rewritten by the next pass
+        if (C > 1) break;
+    }
+    if constexpr (C > 1) {
+        cg::cluster_group cluster = cg::this_cluster();
+        const int n = (u1 - u0) * 2 * NG * 64;
+        cluster.sync();
+        for (int i = crank * NT + tid; i < n; i += C * NT) {
+            const int k = i & 3, l16 = (i >> 2) & 15, ng = (i >> 6) % NG, h = ((i >> 6) / NG) & 1, un = (i >> 6) / NG / 2;
+            const int tok = 4 * ng + 2 * (l16 & 1) + (k & 1), row = (u0 + un) * 32 + h * 16 + (l16 >> 1) + 8 * (k >> 1);
+            if (tok >= p.T || row >= p.rows) continue;
+            float* dst = p.out + (size_t) tok * p.ldo + row;
+            const float old = p.accumulate ? *dst : 0.f;
+            float s = 0.f;
+#pragma unroll
+            for (int r = 0; r < C; ++r) s += cluster.map_shared_rank(ub, r)[i];
+            *dst = p.accumulate ? old + s : s;
+        }
+        cluster.sync();   // no block may leave while a neighbour still reads its sums
+    }
+}
+
+// two blocks an SM: the next kernel's may be resident while this one's drain
+template <int NG, int MODE, int NW, int SLOTS>
+__global__ void __launch_bounds__(NW * 32, NW > 12 ? 1 : 2) k_nat_mmv(const NatParams p) {
+    extern __shared__ __align__(128) uint8_t smem[];
+    nm_body<NG, MODE, NW, SLOTS, 1>(p, smem);
+}
+constexpr int NM_SPLIT = 4;
+template <int NG, int NW, int SLOTS>
+__global__ void __cluster_dims__(NM_SPLIT, 1, 1) __launch_bounds__(NW * 32, NW > 12 ? 1 : 2) k_nat_mmv_split(const NatParams p) {
+    extern __shared__ __align__(128) uint8_t smem[];
+    nm_body<NG, MAT_DENSE, NW, SLOTS, NM_SPLIT>(p, smem);
+}
+
+template <int NG, int MODE, int NW, int SLOTS>
+static int launch_nat(NatParams p, cudaStream_t st) {
+    constexpr size_t LIMIT = 220 * 1024;
+    const size_t fixed = (size_t) NW * SLOTS * NAT_TILE_BYTES + (size_t) NW * 2 * sizeof(NatPiece<NG, MODE>);
+    const size_t row = ni_row_bytes(p.K / 256);
+    size_t smem = fixed;
+    if (MODE == MAT_DENSE) {
+        smem += 4 * NG * row;
+    } else {
+        p.rmax = 12;   // rows of the jobs a block meets in one pass: a few (its units lie in one to three jobs); at most ~40 KB of them
+        while (p.rmax > 4 && (p.rmax + 3) * row > 40 * 1024) --p.rmax;
+        smem += (p.rmax + 3) * row + (size_t) p.njobs_max * sizeof(fnx_job);
+    }
+    if (smem > LIMIT) return fail(FNX_E_ARG, "nat_mmv: %d columns, %d rows, %d jobs need %zu bytes of shared memory", p.K, 4 * NG, p.njobs_max, smem);
+    if (int rc = set_smem_limit((const void*) k_nat_mmv<NG, MODE, NW, SLOTS>, (int) LIMIT)) return rc;
+    const cudaError_t le = launch_dep(k_nat_mmv<NG, MODE, NW, SLOTS>, dim3(sm_count()), dim3(NW * 32), smem, st, p);
+    return le == cudaSuccess ? FNX_OK : fail(FNX_E_CUDA, "nat_mmv: launch failed: %s", cudaGetErrorString(le));
+}
+
+template <int NG, int NW, int SLOTS>
+static int launch_nat_split(NatParams p, cudaStream_t st) {
+    constexpr size_t LIMIT = 220 * 1024;
+    const int units = (p.rows + 31) / 32, most = sm_count() / NM_SPLIT, per = (units + most - 1) / most, clusters = (units + per - 1) / per;
+    p.umax = per;
+    const size_t smem = (size_t) NW * SLOTS * NAT_TILE_BYTES + (size_t) NW * 2 * sizeof(NatPiece<NG, MAT_DENSE>) + 4 * NG * ni_row_bytes(p.K / 256 / NM_SPLIT) +
+                        (size_t) per * 2 * NG * 64 * sizeof(float);
+    if (smem > LIMIT) return fail(FNX_E_ARG, "nat_mmv: %d columns, %d rows need %zu bytes of shared memory", p.K, 4 * NG, smem);
+    if (int rc = set_smem_limit((const void*) k_nat_mmv_split<NG, NW, SLOTS>, (int) LIMIT)) return rc;
+    const cudaError_t le = launch_dep(k_nat_mmv_split<NG, NW, SLOTS>, dim3(clusters * NM_SPLIT), dim3(NW * 32), smem, st, p);
+    return le == cudaSuccess ? FNX_OK : fail(FNX_E_CUDA, "nat_mmv: launch failed: %s", cudaGetErrorString(le));
+}
+
+int nat_dense(const uint8_t* W, int rows, int K, const uint8_t* img, bool normed, float eps, int T, float* y, int ldy, int accumulate, cudaStream_t st) {
+    FNX_REQUIRE(T >= 1 && T <= FNX_MAX_ROWS && rows % 16 == 0 && K % 256 == 0, "nat_dense: %d rows of %d x %d", T, rows, K);
+    const size_t row = ni_row_bytes(K / 256);
+    // columns split over a cluster: long rows that are not normed, and few enough units that their partial sums fit
+    const bool split = K >= 4096 && K % (256 * NM_SPLIT) == 0 && !normed && (rows + 31) / 32 <= 8 * (sm_count() / NM_SPLIT);
+    // up to five groups of four rows a launch (more would leave no registers), fewer where their image would not fit beside the tiles
+    int most = 5;
+    while (most > 1 && 4 * most * (split ? ni_row_bytes(K / 256 / NM_SPLIT) : row) > 100 * 1024) --most;
+    const int groups = (T + 3) / 4, calls = (groups + most - 1) / most, per = (groups + calls - 1) / calls;
+    for (int g0 = 0; g0 < groups; g0 += per) {
+        NatParams p{};
+        const int ng = groups - g0 < per ? groups - g0 : per;
+        p.W = W; p.T = T - 4 * g0 < 4 * ng ? T - 4 * g0 : 4 * ng; p.img = img + (size_t) 4 * g0 * row; p.normed = normed; p.eps = eps;
+        p.out = y + (size_t) 4 * g0 * ldy; p.ldo = ldy; p.rows = rows; p.K = K; p.accumulate = accumulate;
+        int rc;
+        if (split) {
+            switch (ng) {
+                case 1: rc = launch_nat_split<1, 8, 2>(p, st); break;
+                case 2: rc = launch_nat_split<2, 8, 2>(p, st); break;
+                case 3: rc = launch_nat_split<3, 8, 2>(p, st); break;
+                case 4: rc = launch_nat_split<4, 8, 2>(p, st); break;
+                default: rc = launch_nat_split<5, 8, 2>(p, st); break;
+            }
+        } else {
+            switch (ng) {
+                case 1: rc = launch_nat<1, MAT_DENSE, 8, 3>(p, st); break;
+                case 2: rc = launch_nat<2, MAT_DENSE, 8, 3>(p, st); break;
+                case 3: rc = launch_nat<3, MAT_DENSE, 8, 2>(p, st); break;
+                case 4: rc = launch_nat<4, MAT_DENSE, 8, 2>(p, st); break;
+                default: rc = launch_nat<5, MAT_DENSE, 8, 2>(p, st); break;
+            }
+        }
+        if (rc != FNX_OK) return rc;
+    }
+    return FNX_OK;
+}
+
+int nat_gate_up(const uint8_t* Wgu, size_t stride, int e_base, const uint8_t* Wsh, int E, const fnx_job* jobs, const int* njobs, int njobs_max, const uint8_t* img,
+                float eps, int H, int F, float* h, cudaStream_t st) {
+    NatParams p{};
+    p.W = Wgu; p.expert_stride = stride; p.e_base = e_base; p.Wsh = Wsh; p.E = E; p.jobs = jobs; p.njobs = njobs; p.njobs_max = njobs_max; p.img = img; p.normed = 1;
+    p.eps = eps; p.out = h; p.ldo = F; p.rows = F; p.K = H;
+    return launch_nat<1, MAT_GATEUP, 8, 3>(p, st);
+}
+
+int nat_down(const uint8_t* Wdn, size_t stride, int e_base, const uint8_t* Wsh, int E, const fnx_job* jobs, const int* njobs, int njobs_max, const float* h, int H,
+             int F, float* part, cudaStream_t st) {
+    NatParams p{};
+    p.W = Wdn; p.expert_stride = stride; p.e_base = e_base; p.Wsh = Wsh; p.E = E; p.jobs = jobs; p.njobs = njobs; p.njobs_max = njobs_max; p.x = h;
+    p.out = part; p.ldo = H; p.rows = H; p.K = F;
+    return launch_nat<1, MAT_DOWN, 8, 2>(p, st);
+}
+
+// ------------------------------------------------------------------------------------------------ images of rows
+// one warp per (256-column block, row)
+__global__ void __launch_bounds__(32) k_nat_rows_image(const float* __restrict__ x, int ldx, const float* __restrict__ norm_w, uint8_t* __restrict__ img) {
+    pdl_wait();
+    pdl_launch_dependents();
+    const int blk = blockIdx.x, t = blockIdx.y, lane = threadIdx.x, c = blk * 256 + lane * 8;
+    const float4 a = *reinterpret_cast<const float4*>(x + (size_t) t * ldx + c), b = *reinterpret_cast<const float4*>(x + (size_t) t * ldx + c + 4);
+    float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    const float ss = ni_norm8(v, norm_w ? norm_w + c : nullptr);
+    ni_quant(img, gridDim.x, v, ss, t, blk, lane);
+}
+
+__global__ void __launch_bounds__(32) k_nat_embed_image(const __half* __restrict__ table, const int* __restrict__ tok, float* __restrict__ R,
+                                                        const float* __restrict__ norm_w, uint8_t* __restrict__ img) {
+    pdl_wait();
+    pdl_launch_dependents();
+    const int blk = blockIdx.x, t = blockIdx.y, lane = threadIdx.x, c = blk * 256 + lane * 8, H = gridDim.x * 256;
+    const uint4 h = *reinterpret_cast<const uint4*>(table + (size_t) tok[t] * H + c);
+    const __half2* h2 = reinterpret_cast<const __half2*>(&h);
+    float v[8];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float2 f = __half22float2(h2[i]);
+        v[2 * i] = f.x;
+        v[2 * i + 1] = f.y;
+    }
+    float* o = R + (size_t) t * H + c;
+    *reinterpret_cast<float4*>(o) = make_float4(v[0], v[1], v[2], v[3]);
+    *reinterpret_cast<float4*>(o + 4) = make_float4(v[4], v[5], v[6], v[7]);
+    if (!img) return;
+    const float ss = ni_norm8(v, norm_w ? norm_w + c : nullptr);
+    ni_quant(img, gridDim.x, v, ss, t, blk, lane);
+}
+
+int nat_rows_image(const float* x, int ldx, int T, int K, const float* norm_w, uint8_t* img, cudaStream_t st) {
+    FNX_REQUIRE(x && img && T >= 1 && K % 256 == 0 && ldx % 4 == 0, "nat_rows_image: %d rows of %d", T, K);
+    const cudaError_t le = launch_dep(k_nat_rows_image, dim3(K / 256, T), dim3(32), 0, st, x, ldx, norm_w, img);
+    return le == cudaSuccess ? FNX_OK : fail(FNX_E_CUDA, "nat_rows_image: launch failed: %s", cudaGetErrorString(le));
+}
+
+int nat_embed_image(const __half* table, const int* tok, int T, int H, float* R, const float* norm_w, uint8_t* img, cudaStream_t st) {
+    FNX_REQUIRE(table && tok && R && T >= 1 && H % 256 == 0, "nat_embed_image: %d rows of %d", T, H);
+    const cudaError_t le = launch_dep(k_nat_embed_image, dim3(H / 256, T), dim3(32), 0, st, table, tok, R, norm_w, img);
+    return le == cudaSuccess ? FNX_OK : fail(FNX_E_CUDA, "nat_embed_image: launch failed: %s", cudaGetErrorString(le));
+}
+
+// ------------------------------------------------------------------------------------------------ layouts
+__global__ void __launch_bounds__(128) k_nat_pack(const uint8_t* __restrict__ ggml, uint8_t* __restrict__ nat, size_t rows, size_t row0, size_t n, int KB, int gate_up) {
+    __shared__ uint32_t grid[512];
+    for (int i = threadIdx.x; i < 512; i += blockDim.x) grid[i] = g_grid_nat[i];
+    __syncthreads();
+    const size_t i = (size_t) blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n * KB) return;
+    const size_t row = row0 + i / KB;
+    const int b = (int) (i % KB);
+    uint8_t blk[IQ3S_BLOCK_BYTES];
+    const uint8_t* src = ggml + i * IQ3S_BLOCK_BYTES;
+    for (int k = 0; k < IQ3S_BLOCK_BYTES; ++k) blk[k] = src[k];
+    nat_put_block(nat + nat_half_at(row / 16, rows / 16, b, KB, gate_up), (int) (row % 16), blk, grid);
+}
+
+__global__ void __launch_bounds__(128) k_nat_unpack(const uint8_t* __restrict__ nat, uint8_t* __restrict__ tiles, size_t rows, int KB, int gate_up) {
+    __shared__ uint16_t inv[4096];
+    for (int e = threadIdx.x; e < 512; e += blockDim.x) {
+        uint32_t key = 0;
+        for (int j = 0; j < 4; ++j) key |= ((g_grid_nat[e] >> (8 * j + 1)) & 7u) << (3 * j);
+        inv[key] = (uint16_t) e;
+    }
+    __syncthreads();
+    const size_t i = (size_t) blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= rows * KB) return;
+    const size_t row = i / KB;
+    const int b = (int) (i % KB);
+    uint8_t blk[IQ3S_BLOCK_BYTES];
+    nat_get_block(nat + nat_half_at(row / 16, rows / 16, b, KB, gate_up), (int) (row % 16), blk, inv);
+    tile_put_block(tiles + ((row / 16) * KB + b) * TILE_BYTES, (int) (row % 16), blk);
+}
+
+int nat_pack(const uint8_t* ggml, uint8_t* nat, size_t rows, size_t row0, size_t n, size_t cols, bool gate_up, cudaStream_t st) {
+    FNX_REQUIRE(ggml && nat && rows % (gate_up ? 32 : 16) == 0 && row0 % 16 == 0 && n % 16 == 0 && n && row0 + n <= rows && cols % 256 == 0, "nat_pack: rows [%zu, + %zu) of %zu x %zu", row0, n, rows, cols);
+    const size_t w = n * (cols / 256);
+    k_nat_pack<<<(unsigned) ((w + 127) / 128), 128, 0, st>>>(ggml, nat, rows, row0, n, (int) (cols / 256), gate_up);
+    FNX_LAUNCH_OK("nat_pack");
+    return FNX_OK;
+}
+
+int nat_unpack(const uint8_t* nat, uint8_t* tiles, size_t rows, size_t cols, bool gate_up, cudaStream_t st) {
+    FNX_REQUIRE(nat && tiles && rows % (gate_up ? 32 : 16) == 0 && cols % 256 == 0, "nat_unpack: %zu x %zu", rows, cols);
+    const size_t w = rows * (cols / 256);
+    k_nat_unpack<<<(unsigned) ((w + 127) / 128), 128, 0, st>>>(nat, tiles, rows, (int) (cols / 256), gate_up);
+    FNX_LAUNCH_OK("nat_unpack");
+    return FNX_OK;
+}
+
+}  // namespace fnxb

@@ -1,0 +1,114 @@
+"""The engine's own weight layout against the interchange layout: the same weights, windows and prompts, two engines.
+
+fnx_engine_tensor hands a weight matrix out in the interchange layout, and windows read it there from then on; an engine whose
+matrices were never asked for reads its own four-bit layout.  Both hold the same numbers and quantise the rows the same way, so
+their results differ by the order of f32 sums and by rows whose codes move by one step of 1 / 65,024 of a block's largest value."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+import fnx_b200 as F  # noqa: E402
+
+MATRICES = ("w_in", "w_out", "experts_gu", "experts_dn", "shared_gu", "shared_dn")
+
+
+def small(**over):
+    d = dict(n_layer=4, hidden=1024, n_expert=32, top_k=4, ffn=256, n_q_head=8, n_kv_head=1, gdn_k_head=2, gdn_v_head=4, vocab=2048, max_ctx=2048, max_rows=32, n_seq=4)
+    d.update(over)
+    return F.flash_next_config(**d)
+
+
+def wide():   # the benchmark's widths: 4,096-column output projections (split over clusters), 16-row padding of the draft head
+    return F.flash_next_config(n_layer=4, n_expert=32, vocab=4096, max_ctx=512, max_rows=32, n_seq=4, draft_vocab=1040)
+
+
+def pair(cfg):
+    engines = []
+    for tiles in (False, True):
+        e = F.Engine(cfg)
+        e.init_synthetic(seed=5, sigma=0.02)
+        if tiles:
+            names = [f"l{l}.{m}" for l in range(cfg.n_layer) for m in MATRICES] + ["mtp." + m for m in MATRICES] + ["mtp.fc_hid", "mtp.fc_emb", "head"]
+            for n in names + (["mtp.head"] if cfg.draft_vocab else []):
+                e.tensor(n, torch.uint8)
+        engines.append(e)
+    return engines
+
+
+def rows(e, cfg, T):
+    r = e.tensor("buf.R", torch.float32).cpu().numpy().reshape(cfg.max_rows, cfg.hidden)[:T]
+    lg = e.tensor("buf.logits", torch.float32).cpu().numpy().reshape(cfg.max_rows, cfg.vocab)[:T]
+    return r.copy(), lg.copy()
+
+
+def close(a, b, what):
+    err = float(np.linalg.norm(a.astype(np.float64) - b) / np.linalg.norm(b))
+    assert err < 3e-4, (what, err)
+
+
+@pytest.mark.parametrize("make", [small, wide])
+def test_windows_and_drafts_agree_between_the_layouts(make):
+    cfg = make()
+    a, b = pair(cfg)
+    try:
+        rng = np.random.default_rng(3)
+        for T in (1, 4, 5, 9, 16, 20, 21, 32):   # row groups 1 .. 5, one launch and two
+            toks = rng.integers(0, cfg.vocab, size=T).tolist()
+            got = [e.verify(toks) for e in (a, b)]
+            for x, y, w in zip(rows(a, cfg, T), rows(b, cfg, T), ("rows", "logits")):
+                close(x, y, (T, w))
+            assert got[0] == got[1]
+            keep = list(range(min(T, 3)))
+            for e in (a, b):
+                e.commit(keep)
+            assert a.draft(3) == b.draft(3)
+        par = [-1, 0, 1, 0, 3, 1, 2]
+        toks = rng.integers(0, cfg.vocab, size=7).tolist()
+        assert a.verify(toks, par) == b.verify(toks, par)
+        for x, y in zip(rows(a, cfg, 7), rows(b, cfg, 7)):
+            close(x, y, "tree")
+        lanes = [rng.integers(0, cfg.vocab, size=n).tolist() for n in (1, 4, 5)]
+        assert a.verify_lanes_rows([1, 2, 3], lanes) == b.verify_lanes_rows([1, 2, 3], lanes)
+        for x, y in zip(rows(a, cfg, 10), rows(b, cfg, 10)):
+            close(x, y, "lanes")
+        for e in (a, b):
+            e.commit_lanes([1, 2, 3], [1, 2, 5])
+        assert a.draft_lanes([1, 2, 3], 2) == b.draft_lanes([1, 2, 3], 2)
+    finally:
+        a.close()
+        b.close()
+
+
+@pytest.mark.parametrize("n", [70, 1200])   # the products that decode as they go, and the ones from weights decoded once
+def test_prompts_agree_between_the_layouts(n):
+    cfg = small()
+    a, b = pair(cfg)
+    try:
+        toks = np.random.default_rng(4).integers(0, cfg.vocab, size=n).tolist()
+        for e in (a, b):
+            e.prompt(toks)
+        close(rows(a, cfg, 1)[1], rows(b, cfg, 1)[1], n)
+    finally:
+        a.close()
+        b.close()
+
+
+def test_a_matrix_asked_for_comes_back_in_the_interchange_layout():
+    """Bit for bit the tiles that the same seeded weights give through the operators, padded rows included."""
+    cfg = small(draft_vocab=1040)
+    e = F.Engine(cfg)
+    try:
+        e.init_synthetic(seed=5, sigma=0.02)
+        w = torch.empty(1040 * cfg.hidden, device="cuda")
+        F.fill_normal(w, 0.02, 5, (61 * 16 + 2) << 12)
+        want = F.iq3s_retile(F.iq3s_quantize(w), 1040, cfg.hidden)
+        assert torch.equal(e.tensor("mtp.head", torch.uint8), want)
+        gu = 2 * cfg.ffn
+        w = torch.empty(gu * cfg.hidden, device="cuda")
+        F.fill_normal(w, 0.02, 5, ((1 * 16 + 4) << 12) | 7)
+        per = F.iq3s_bytes(gu, cfg.hidden)
+        assert torch.equal(e.tensor("l1.experts_gu", torch.uint8)[7 * per:8 * per], F.iq3s_retile(F.iq3s_quantize(w), gu, cfg.hidden))
+    finally:
+        e.close()
