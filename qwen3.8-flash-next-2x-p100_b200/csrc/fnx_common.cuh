@@ -61,10 +61,12 @@ inline cudaError_t launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, siz
     cfg.numAttrs = pdl_enabled() ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
 }
-// the same for a kernel that leaves room for its successor on the SM (registers and shared memory of two blocks fit): it may start
-// while its predecessor drains
+// A kernel of an engine's window, which leaves room for its successor on the SM (registers and shared memory of two blocks fit): it may
+// start while its predecessor drains.  Before pdl_wait() it may read what no kernel since the last but one before it writes (weights,
+// the starting states); an operator of the C ABI, whose caller may have filled any input just before, is launched with early = false
+// unless the kernel reads nothing before pdl_wait().  Every block must reach pdl_wait(): a kernel's end implies its predecessors'.
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_dep(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
+inline cudaError_t launch_dep(bool early, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -74,7 +76,7 @@ inline cudaError_t launch_dep(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = early ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
 }
 #endif

@@ -430,7 +430,7 @@ __global__ void __launch_bounds__(32) k_combine_nat(const float* __restrict__ pa
 int moe_combine_nat(const float* part, const int* topi, const float* topw, const float* logits, int T, int E, int H, int K, float* R, uint8_t* img, const float* img_norm_w,
                     cudaStream_t st) {
     FNX_REQUIRE(T >= 1 && T <= FNX_MAX_ROWS && K >= 1 && K <= 32 && H % 256 == 0, "moe_combine_nat: %d rows of %d, top %d", T, H, K);
-    const cudaError_t le = launch_dep(k_combine_nat, dim3(H / 256, T), dim3(32), 0, st, part, topi, topw, logits, T, E, H, K, R, img, img_norm_w);
+    const cudaError_t le = launch_dep(true, k_combine_nat, dim3(H / 256, T), dim3(32), 0, st, part, topi, topw, logits, T, E, H, K, R, img, img_norm_w);
     return le == cudaSuccess ? FNX_OK : fail(FNX_E_CUDA, "k_combine_nat: launch failed: %s", cudaGetErrorString(le));
 }
 

@@ -43,7 +43,6 @@ struct NatParams {
     int rows, K;         // output rows per job (gate|up: F), columns
     int accumulate;
     int rmax;            // expert modes: rows a block holds at once
-    int umax;            // dense with split columns: units of a cluster
 };
 
 template <int NG, int MODE>
@@ -62,7 +61,12 @@ __device__ __forceinline__ void nm_mma(int (&c)[4], const uint32_t (&a)[4], uint
 
 // four nibbles of x -> bytes 8 m = 16 t + 8 (the high ones as they lie, the low ones shifted up)
 __device__ __forceinline__ uint32_t nm_hi(uint32_t x) { return (x & 0xF0F0F0F0u) | 0x08080808u; }
-__device__ __forceinline__ uint32_t nm_lo(uint32_t x) { return ((x * 16u) & 0xF0F0F0F0u) | 0x08080808u; }
+// (the factor is hidden from the compiler: the shift it would make of it competes with the masks for the integer-logic pipe)
+__device__ __forceinline__ uint32_t nm_lo(uint32_t x) {
+    uint32_t k;
+    asm("mov.u32 %0, 16;" : "=r"(k));
+    return ((x * k) & 0xF0F0F0F0u) | 0x08080808u;
+}
 
 // the two rows' eight sub-block scales 1 + 2 s as bytes: even sub-blocks in .x, odd ones in .y
 struct NmScales {
@@ -148,8 +152,10 @@ __device__ __forceinline__ void nm_half_item(uint32_t a16, uint32_t am, uint32_t
 // (g, 2 q + 1), (g + 8, 2 q), (g + 8, 2 q + 1).  xb: shared address of the lane's cells in its column's row of group 0, x0 / x1: of its
 // two C columns' scales; groups lie `group` bytes apart.  The integers are exact (8 times the sums of iq3s_mmv.cu's items).
 // AccT double (expert modes): the rounded result does not depend on where a row's K-sum was cut, as there.
-// Up to two row groups load the rows' operands once for both half tiles; more would not leave the registers.  (The loops over four
-// sub-blocks stay rolled: unrolled, every load would be hoisted into registers.)
+// Up to two row groups load the rows' operands once for both half tiles; more would not leave the registers.  (Most jobs have one
+// row, two of the eight columns; a form with half of the integer work for them was slower: 52 against 46 us for 205 jobs, the second
+// copy of the code.)  Their loop over four
+// sub-blocks stays rolled (unrolled, every load would be hoisted into registers), the short one is worth unrolling: 50 -> 47 us for 205 jobs.
 template <int NG, typename AccT>
 __device__ __forceinline__ void nm_item(uint32_t tile_s, uint32_t xb, uint32_t x0, uint32_t x1, uint32_t group, int lane, AccT (&acc)[2][NG][4]) {
     const uint32_t a16 = tile_s + lane * 16, am = tile_s + (lane >> 2) * 16;
@@ -161,7 +167,7 @@ __device__ __forceinline__ void nm_item(uint32_t tile_s, uint32_t xb, uint32_t x
 #pragma unroll
         for (int i = 0; i < 2 * NG * 4; ++i) accI[i / (4 * NG)][(i / 4) % NG][i & 3] = 0;
         const NmScales sc0 = nm_scales<0>(am), sc1 = nm_scales<1>(am);
-#pragma unroll 1
+#pragma unroll
         for (int hf = 0; hf < 2; ++hf) {
             uint4 b0[NG], b1[NG];
 #pragma unroll
@@ -241,7 +247,7 @@ __device__ __forceinline__ void nm_body(const NatParams& p, uint8_t* smem) {
     const uint32_t RS = (uint32_t) ni_row_bytes(KBc);
     Piece* pieces = reinterpret_cast<Piece*>(smem + (size_t) NW * SLOTS * NAT_TILE_BYTES);   // [NW][2]
     uint8_t* pool = reinterpret_cast<uint8_t*>(pieces + NW * 2);                             // row images
-    const int pool_rows = MOE ? p.rmax + 3 : 4 * NG;                                         // (a group's missing rows are read and dropped)
+    const int pool_rows = MOE ? p.rmax : 4 * NG;
     fnx_job* jobs_s = reinterpret_cast<fnx_job*>(pool + (size_t) pool_rows * RS);
     float* ub = reinterpret_cast<float*>(pool + (size_t) pool_rows * RS);                    // C > 1: the units' partial sums
     const uint32_t slots_s = smem_u32(smem) + (uint32_t) warp * (SLOTS * NAT_TILE_BYTES), pool_s = smem_u32(pool);
@@ -359,14 +365,22 @@ __device__ __forceinline__ void nm_body(const NatParams& p, uint8_t* smem) {
             mine[0].unit = i0 < i1 ? -1 : -2;
             mine[1].unit = -1;
         }
-        // the lane's columns: row n & 3 of its group at level n / 4
+        // the lane's columns: row n & 3 of its group at level n / 4.  Expert modes: a job's missing rows read its last one (a dense group's
+        // lie in the pool, whatever they hold); either way the columns are dropped.
         const int g = lane >> 2, q = lane & 3;
-        const uint32_t xb0 = pool_s + (uint32_t) (g & 3) * RS + (uint32_t) (g >> 2) * 256u + q * 16;
-        const uint32_t x00 = pool_s + (uint32_t) ((2 * q) & 3) * RS + NI_SCALE + (uint32_t) (q >> 1) * 4u, x10 = x00 + RS;
-        uint32_t jrow = 0;   // expert modes: the current job's first row in the pool
+        uint32_t xb0 = 0, x00 = 0, x10 = 0;
+        auto columns = [&](uint32_t base, int n) {
+            const int last = MOE ? n - 1 : 4 * NG, r0 = (2 * q) & 3;
+            xb0 = base + (uint32_t) min(g & 3, last) * RS + (uint32_t) (g >> 2) * 256u + q * 16;
+            x00 = base + (uint32_t) min(r0, last) * RS + NI_SCALE + (uint32_t) (q >> 1) * 4u;
+            x10 = base + (uint32_t) min(r0 + 1, last) * RS + NI_SCALE + (uint32_t) (q >> 1) * 4u;
+        };
         int cur_job = -1, ntok = p.T, b_lo = 0;
         float rf = 1.0f;
-        if (MODE == MAT_DENSE && p.normed && lane < p.T) rf = nm_row_factor(pool_s + lane * RS, KB, p.eps);   // (normed rows are never split: C == 1)
+        if (!MOE) {
+            columns(pool_s, p.T);
+            if (p.normed && lane < p.T) rf = nm_row_factor(pool_s + lane * RS, KB, p.eps);   // (normed rows are never split: C == 1)
+        }
         AccT acc[2][NG][4];
         int b = i0 % nbu, u = uc + i0 / nbu, slot = 0;
         // a unit's sums: written, or (columns split) left for the cluster
@@ -398,15 +412,15 @@ __device__ __forceinline__ void nm_body(const NatParams& p, uint8_t* smem) {
                     cur_job = u / upj;
                     int r = 0;
                     for (int j = j0; j < cur_job; ++j) r += min(jobs_s[j].n, 4);
-                    jrow = (uint32_t) r * RS;
                     ntok = min(jobs_s[cur_job].n, 4);
-                    if (MODE == MAT_GATEUP && p.normed) rf = lane < ntok ? nm_row_factor(pool_s + jrow + lane * RS, KB, p.eps) : 1.0f;
+                    columns(pool_s + (uint32_t) r * RS, ntok);
+                    if (MODE == MAT_GATEUP && p.normed) rf = lane < ntok ? nm_row_factor(pool_s + (uint32_t) (r + lane) * RS, KB, p.eps) : 1.0f;
                 }
             }
             asm volatile("cp.async.wait_group %0;" ::"n"(SLOTS - 1) : "memory");
             __syncwarp();   // (the scales came in by other lanes' copies)
-            const uint32_t off = jrow + (uint32_t) b * NI_BYTES;
-            nm_item<NG, AccT>(slots_s + (uint32_t) (slot * NAT_TILE_BYTES), xb0 + off, x00 + off, x10 + off, 4u * RS, lane, acc);
+            const uint32_t off = (uint32_t) b * NI_BYTES, tile_s = slots_s + (uint32_t) (slot * NAT_TILE_BYTES);
+            nm_item<NG, AccT>(tile_s, xb0 + off, x00 + off, x10 + off, 4u * RS, lane, acc);
             __syncwarp();   // every lane is done with the slot
             fetch(s + SLOTS, slot);
             slot = slot + 1 == SLOTS ? 0 : slot + 1;
@@ -509,13 +523,16 @@ static int launch_nat(NatParams p, cudaStream_t st) {
     if (MODE == MAT_DENSE) {
         smem += 4 * NG * row;
     } else {
-        p.rmax = 12;   // rows of the jobs a block meets in one pass: a few (its units lie in one to three jobs); at most ~40 KB of them
-        while (p.rmax > 4 && (p.rmax + 3) * row > 40 * 1024) --p.rmax;
-        smem += (p.rmax + 3) * row + (size_t) p.njobs_max * sizeof(fnx_job);
+        // rows of the jobs a block meets in one pass: its units lie in one to three jobs of a row or so each, one of them perhaps the shared
+        // expert's four (a second pass drains the copies: four rows instead of eight cost 1.3 us at five rows); with eight a gate|up
+        // and a down block fit an SM together
+        p.rmax = 8;
+        while (p.rmax > 4 && p.rmax * row > 40 * 1024) --p.rmax;
+        smem += p.rmax * row + (size_t) p.njobs_max * sizeof(fnx_job);
     }
     if (smem > LIMIT) return fail(FNX_E_ARG, "nat_mmv: %d columns, %d rows, %d jobs need %zu bytes of shared memory", p.K, 4 * NG, p.njobs_max, smem);
     if (int rc = set_smem_limit((const void*) k_nat_mmv<NG, MODE, NW, SLOTS>, (int) LIMIT)) return rc;
-    const cudaError_t le = launch_dep(k_nat_mmv<NG, MODE, NW, SLOTS>, dim3(sm_count()), dim3(NW * 32), smem, st, p);
+    const cudaError_t le = launch_dep(true, k_nat_mmv<NG, MODE, NW, SLOTS>, dim3(sm_count()), dim3(NW * 32), smem, st, p);
     return le == cudaSuccess ? FNX_OK : fail(FNX_E_CUDA, "nat_mmv: launch failed: %s", cudaGetErrorString(le));
 }
 
@@ -523,12 +540,11 @@ template <int NG, int NW, int SLOTS>
 static int launch_nat_split(NatParams p, cudaStream_t st) {
     constexpr size_t LIMIT = 220 * 1024;
     const int units = (p.rows + 31) / 32, most = sm_count() / NM_SPLIT, per = (units + most - 1) / most, clusters = (units + per - 1) / per;
-    p.umax = per;
     const size_t smem = (size_t) NW * SLOTS * NAT_TILE_BYTES + (size_t) NW * 2 * sizeof(NatPiece<NG, MAT_DENSE>) + 4 * NG * ni_row_bytes(p.K / 256 / NM_SPLIT) +
                         (size_t) per * 2 * NG * 64 * sizeof(float);
     if (smem > LIMIT) return fail(FNX_E_ARG, "nat_mmv: %d columns, %d rows need %zu bytes of shared memory", p.K, 4 * NG, smem);
     if (int rc = set_smem_limit((const void*) k_nat_mmv_split<NG, NW, SLOTS>, (int) LIMIT)) return rc;
-    const cudaError_t le = launch_dep(k_nat_mmv_split<NG, NW, SLOTS>, dim3(clusters * NM_SPLIT), dim3(NW * 32), smem, st, p);
+    const cudaError_t le = launch_dep(true, k_nat_mmv_split<NG, NW, SLOTS>, dim3(clusters * NM_SPLIT), dim3(NW * 32), smem, st, p);
     return le == cudaSuccess ? FNX_OK : fail(FNX_E_CUDA, "nat_mmv: launch failed: %s", cudaGetErrorString(le));
 }
 
@@ -537,6 +553,8 @@ int nat_dense(const uint8_t* W, int rows, int K, const uint8_t* img, bool normed
     const size_t row = ni_row_bytes(K / 256);
     // columns split over a cluster: long rows that are not normed, and few enough units that their partial sums fit
     const bool split = K >= 4096 && K % (256 * NM_SPLIT) == 0 && !normed && (rows + 31) / 32 <= 8 * (sm_count() / NM_SPLIT);
+    // a matrix that streams for some 10 us (a vocabulary's): sixteen warps, as for many expert jobs below
+    const bool large = !split && nat_bytes(rows, K) > ((size_t) 64 << 20);
     // up to five groups of four rows a launch (more would leave no registers), fewer where their image would not fit beside the tiles
     int most = 5;
     while (most > 1 && 4 * most * (split ? ni_row_bytes(K / 256 / NM_SPLIT) : row) > 100 * 1024) --most;
@@ -557,8 +575,8 @@ int nat_dense(const uint8_t* W, int rows, int K, const uint8_t* img, bool normed
             }
         } else {
             switch (ng) {
-                case 1: rc = launch_nat<1, MAT_DENSE, 8, 3>(p, st); break;
-                case 2: rc = launch_nat<2, MAT_DENSE, 8, 3>(p, st); break;
+                case 1: rc = large ? launch_nat<1, MAT_DENSE, 16, 2>(p, st) : launch_nat<1, MAT_DENSE, 8, 3>(p, st); break;
+                case 2: rc = large ? launch_nat<2, MAT_DENSE, 16, 2>(p, st) : launch_nat<2, MAT_DENSE, 8, 3>(p, st); break;
                 case 3: rc = launch_nat<3, MAT_DENSE, 8, 2>(p, st); break;
                 case 4: rc = launch_nat<4, MAT_DENSE, 8, 2>(p, st); break;
                 default: rc = launch_nat<5, MAT_DENSE, 8, 2>(p, st); break;
@@ -569,12 +587,16 @@ int nat_dense(const uint8_t* W, int rows, int K, const uint8_t* img, bool normed
     return FNX_OK;
 }
 
+// From this many jobs on the expert products stream long enough (some 15 us) that sixteen warps, which hide more of an item's latency,
+// are worth more than a second resident block: 205 jobs 50 -> 45 us (gate|up) and 28 -> 24 us (down); 52 jobs are level.
+constexpr int NM_MANY_JOBS = 80;
+
 int nat_gate_up(const uint8_t* Wgu, size_t stride, int e_base, const uint8_t* Wsh, int E, const fnx_job* jobs, const int* njobs, int njobs_max, const uint8_t* img,
                 float eps, int H, int F, float* h, cudaStream_t st) {
     NatParams p{};
     p.W = Wgu; p.expert_stride = stride; p.e_base = e_base; p.Wsh = Wsh; p.E = E; p.jobs = jobs; p.njobs = njobs; p.njobs_max = njobs_max; p.img = img; p.normed = 1;
     p.eps = eps; p.out = h; p.ldo = F; p.rows = F; p.K = H;
-    return launch_nat<1, MAT_GATEUP, 8, 3>(p, st);
+    return njobs_max > NM_MANY_JOBS ? launch_nat<1, MAT_GATEUP, 16, 2>(p, st) : launch_nat<1, MAT_GATEUP, 8, 2>(p, st);
 }
 
 int nat_down(const uint8_t* Wdn, size_t stride, int e_base, const uint8_t* Wsh, int E, const fnx_job* jobs, const int* njobs, int njobs_max, const float* h, int H,
@@ -582,7 +604,7 @@ int nat_down(const uint8_t* Wdn, size_t stride, int e_base, const uint8_t* Wsh, 
     NatParams p{};
     p.W = Wdn; p.expert_stride = stride; p.e_base = e_base; p.Wsh = Wsh; p.E = E; p.jobs = jobs; p.njobs = njobs; p.njobs_max = njobs_max; p.x = h;
     p.out = part; p.ldo = H; p.rows = H; p.K = F;
-    return launch_nat<1, MAT_DOWN, 8, 2>(p, st);
+    return njobs_max > NM_MANY_JOBS ? launch_nat<1, MAT_DOWN, 16, 2>(p, st) : launch_nat<1, MAT_DOWN, 8, 2>(p, st);
 }
 
 // ------------------------------------------------------------------------------------------------ images of rows
@@ -621,13 +643,13 @@ __global__ void __launch_bounds__(32) k_nat_embed_image(const __half* __restrict
 
 int nat_rows_image(const float* x, int ldx, int T, int K, const float* norm_w, uint8_t* img, cudaStream_t st) {
     FNX_REQUIRE(x && img && T >= 1 && K % 256 == 0 && ldx % 4 == 0, "nat_rows_image: %d rows of %d", T, K);
-    const cudaError_t le = launch_dep(k_nat_rows_image, dim3(K / 256, T), dim3(32), 0, st, x, ldx, norm_w, img);
+    const cudaError_t le = launch_dep(true, k_nat_rows_image, dim3(K / 256, T), dim3(32), 0, st, x, ldx, norm_w, img);
     return le == cudaSuccess ? FNX_OK : fail(FNX_E_CUDA, "nat_rows_image: launch failed: %s", cudaGetErrorString(le));
 }
 
 int nat_embed_image(const __half* table, const int* tok, int T, int H, float* R, const float* norm_w, uint8_t* img, cudaStream_t st) {
     FNX_REQUIRE(table && tok && R && T >= 1 && H % 256 == 0, "nat_embed_image: %d rows of %d", T, H);
-    const cudaError_t le = launch_dep(k_nat_embed_image, dim3(H / 256, T), dim3(32), 0, st, table, tok, R, norm_w, img);
+    const cudaError_t le = launch_dep(true, k_nat_embed_image, dim3(H / 256, T), dim3(32), 0, st, table, tok, R, norm_w, img);
     return le == cudaSuccess ? FNX_OK : fail(FNX_E_CUDA, "nat_embed_image: launch failed: %s", cudaGetErrorString(le));
 }
 
