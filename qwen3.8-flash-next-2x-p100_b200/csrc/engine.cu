@@ -17,6 +17,7 @@
 
 #include "engine_mat.h"
 #include "fnx_common.cuh"
+#include "gdn_core.h"
 #include "iq3s_tile.h"
 #include "nat_image.cuh"
 #include "nat_tile.h"
@@ -756,9 +757,11 @@ static int enqueue_gdn(fnx_engine* e, const LayerW& L, float* R, int T, int seq,
     FNX_TRY(enqueue_dense(e, L.w_in, R, d.H, T, L.norm1, e->proj, e->proj_ld, 0, e->img_r, img));
     float* S = L.S_pool + (size_t) seq * e->NS * d.nv * d.hs * d.hs;
     float* hist = L.hist_pool + (size_t) seq * e->NS * 3 * d.gdn_ch;
-    FNX_TRY(fnx_gdn_core(e->proj, e->proj_ld, e->proj + d.gdn_ch + d.nv * d.hs, e->proj_ld, hist, L.convw, L.dt, L.a, L.gnorm, S, e->d_cur + seq,
-                         e->NS, d_parent, e->mix, d.nk, d.nv, d.hs, T, e->c.eps, e->st));
-    return enqueue_dense(e, L.w_out, e->mix, d.nv * d.hs, T, nullptr, R, d.H, 1, e->img_m);
+    const bool mi = L.w_out.nat && d.nv % 2 == 0;   // (a 256-column block of the image is two heads)
+    FNX_TRY(gdn_window(GdnArgs{e->proj, e->proj_ld, e->proj + d.gdn_ch + d.nv * d.hs, e->proj_ld, hist, L.convw, L.dt, L.a, L.gnorm, S, e->NS, d_parent, e->mix,
+                               mi ? e->img_m : nullptr, d.nk, d.nv, T, e->c.eps},
+                       e->d_cur + seq, true, e->st));
+    return enqueue_dense(e, L.w_out, e->mix, d.nv * d.hs, T, nullptr, R, d.H, 1, e->img_m, mi);
 }
 
 // the whole verify window: embed, layers, head, argmax, greedy acceptance
@@ -900,11 +903,12 @@ static int enqueue_mixer_lanes(fnx_engine* e, const LayerW& L, float* R, int T, 
         if (dp) FNX_TRY(enqueue_dp_gather(e, d.nq * d.hd, n_lanes, d_row0));
         return enqueue_dense(e, L.w_out, e->mix, d.nq * d.hd, T, nullptr, R, d.H, 1, e->img_m);
     }
-    FNX_TRY(fnx_gdn_core_lanes(e->proj, e->proj_ld, e->proj + d.gdn_ch + d.nv * d.hs, e->proj_ld, L.hist_pool, (size_t) e->NS * 3 * d.gdn_ch, L.convw, L.dt, L.a, L.gnorm,
-                               L.S_pool, (size_t) e->NS * d.nv * d.hs * d.hs, e->d_cur, e->NS, lanes, d_row0, n_lanes, max_lane_rows, e->mix, d.nk, d.nv, d.hs,
-                               e->c.eps, e->st));
+    const bool mi = L.w_out.nat && d.nv % 2 == 0 && !dp;
+    FNX_TRY(gdn_window_lanes(GdnArgs{e->proj, e->proj_ld, e->proj + d.gdn_ch + d.nv * d.hs, e->proj_ld, L.hist_pool, L.convw, L.dt, L.a, L.gnorm, L.S_pool, e->NS, nullptr, e->mix,
+                                     mi ? e->img_m : nullptr, d.nk, d.nv, max_lane_rows, e->c.eps},
+                             (size_t) e->NS * 3 * d.gdn_ch, (size_t) e->NS * d.nv * d.hs * d.hs, e->d_cur, lanes, d_row0, n_lanes, max_lane_rows, true, e->st));
     if (dp) FNX_TRY(enqueue_dp_gather(e, d.nv * d.hs, n_lanes, d_row0));
-    return enqueue_dense(e, L.w_out, e->mix, d.nv * d.hs, T, nullptr, R, d.H, 1, e->img_m);
+    return enqueue_dense(e, L.w_out, e->mix, d.nv * d.hs, T, nullptr, R, d.H, 1, e->img_m, mi);
 }
 
 static int enqueue_verify_lanes(fnx_engine* e, int n_lanes, int rows, int T) {   // rows: the longest lane's; T: rows in all

@@ -11,217 +11,304 @@
 //     through distributed shared memory, where the reference uses a global scratch buffer and atomic counters.
 #include <cooperative_groups.h>
 
-#include "fnx_common.cuh"
+#include "gdn_core.h"
+#include "nat_image.cuh"
 
 namespace cg = cooperative_groups;
 
 namespace fnxb {
 
-constexpr int GDN_HS = 128, GDN_Q = 4, GDN_QC = GDN_HS / GDN_Q, GDN_THREADS = 128;
+constexpr int GDN_HS = 128, GDN_Q = 4, GDN_QC = GDN_HS / GDN_Q, GDN_THREADS = 2 * GDN_HS + GDN_QC, GDS_THREADS = 128;
 
-// One block of the (value head, column quarter) grid: the cluster's four blocks share a value head.
-__device__ __forceinline__ void gdn_body(const float* __restrict__ qkvz, int stride, const float* __restrict__ ab, int ldab, float* __restrict__ hist_pool,
-                                         const float* __restrict__ convw, const float* __restrict__ dt, const float* __restrict__ a_,
-                                         const float* __restrict__ nw, float* __restrict__ S_pool, int cur, int NS, const int* __restrict__ parent,
-                                         float* __restrict__ y, int nk, int nv, int T, float eps, float* sm, bool last_only = false) {
-    // (last_only: a prompt's window, every row of which is kept: only the last row's state and history are written)
+// two f32 in a 64-bit register and the packed multiply-add on them (fma.rn.f32x2: each half rounded as the scalar fmaf is, so the
+// products are those of the scalar form, at half the arithmetic instructions)
+__device__ __forceinline__ uint64_t f2_pack(float x, float y) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ void f2_unpack(uint64_t r, float& x, float& y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(r)); }
+__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+
+// One block = a quarter (32 columns) of a value head; the four blocks of a head, and with an image the two heads of a 256-column
+// block of it, form a cluster.  288 threads: one per conv channel the block needs (the head's q and k, its own v columns).  Four of the nine
+// warps run the delta rule: a warp holds 8 columns of the state, lane = 8 rg + c: column c, key rows 16 j + 4 rg + i (j < 8, i < 4),
+// so that a row's sums over the key rows are two shuffles inside the warp and nothing in the rows' chain is block-wide, and a warp's
+// 16-byte reads of k and q fall on four different bank groups.  (Eight warps of 4 columns halve the chain's instructions, but their
+// 16-byte pieces of the states' rows cost more than that: 36 us against 25 at 20 rows.)  The starting state, the history and the constants depend on no
+// kernel of this window: they are loaded before the projections are waited for.
+// Bound by latency at a few rows (the loads, the chain, the exchange over the cluster), by the states' 2 MB a row at many; one block
+// barrier a row and every load after the wait before.
+template <int CL>
+__device__ __forceinline__ void gdn_body(const GdnArgs& p, int cur, float* sm) {
     cg::cluster_group cluster = cg::this_cluster();
-    const int lv = blockIdx.x / GDN_Q, qq = blockIdx.x % GDN_Q, kh = lv % nk, tid = threadIdx.x;
+    const int lv = blockIdx.x / GDN_Q, qq = blockIdx.x % GDN_Q, kh = lv % p.nk, tid = threadIdx.x, T = p.T, NS = p.NS;
     const int warp = tid >> 5, lane = tid & 31;
-    const int ch = (2 * nk + nv) * GDN_HS;
-    const size_t hsz = (size_t) 3 * ch, ssz = (size_t) nv * GDN_HS * GDN_HS;
-    float* xq = sm;                              // [T][HS] q after conv, silu, norm
+    const int ch = (2 * p.nk + p.nv) * GDN_HS;
+    const size_t hsz = (size_t) 3 * ch, ssz = (size_t) p.nv * GDN_HS * GDN_HS;
+    float* xq = sm;                              // [T][HS] q after conv and silu (its norm's factor is applied to the sums)
     float* xk = xq + (size_t) T * GDN_HS;        // [T][HS]
     float* vs = xk + (size_t) T * GDN_HS;        // [T][QC]
-    float* gates = vs + (size_t) T * GDN_QC;     // [T][2]
-    float* kred = gates + 2 * T;                 // [2][4][QC]
-    float* ared = kred + 2 * 4 * GDN_QC;         // [T][4][QC]
-    float* osum = ared + (size_t) T * 4 * GDN_QC;   // [T] this block's square sums (read by the cluster)
-    float* red = osum + T;                       // [4][2 T]
-    float* xin = red + 8 * T;                    // [T + 3][2 HS + QC] conv inputs
-    int* anc = reinterpret_cast<int*>(xin + (size_t) (T + 3) * (2 * GDN_HS + GDN_QC));   // [T][3]
-    const float* hin = hist_pool + (size_t) cur * hsz;
-    // the starting state of the warp's key rows is on its way before anything else: row 0's parent is the root
-    const int part = warp, col = qq * GDN_QC + lane;
-    const size_t soff = (size_t) lv * GDN_HS * GDN_HS + (size_t) part * 32 * GDN_HS + col;
-    float s[32];
-    {
-        const float* src = S_pool + (size_t) cur * ssz + soff;
-#pragma unroll
-        for (int r = 0; r < 32; ++r) s[r] = src[(size_t) r * GDN_HS];
-    }
-    if (tid < T) {
-        const float* abt = ab + (size_t) tid * ldab;
-        const float x = abt[lv] + dt[lv];
-        gates[2 * tid] = expf((x > 20.0f ? x : log1pf(expf(x))) * a_[lv]);
-        gates[2 * tid + 1] = 1.0f / (1.0f + expf(-abt[nv + lv]));
-    }
-    // ---- the conv inputs this block needs, staged with every load in flight at once: rows 0..2 = the starting
-    // history (oldest first), row 3 + t = window row t; columns = the head's q (HS), k (HS), this block's v (QC)
-    constexpr int NC = 2 * GDN_HS + GDN_QC;
-    auto chan = [&](int e) {
-        return e < GDN_HS ? kh * GDN_HS + e : e < 2 * GDN_HS ? nk * GDN_HS + kh * GDN_HS + (e - GDN_HS) : 2 * nk * GDN_HS + lv * GDN_HS + qq * GDN_QC + (e - 2 * GDN_HS);
+    float* os = vs + (size_t) T * GDN_QC;        // [T][QC] the rows' outputs
+    float* gates = os + (size_t) T * GDN_QC;     // [T][2]
+    float* fac = gates + 2 * T;                  // [T][2] 1 / |q|, 1 / |k|
+    float* osum = fac + 2 * T;                   // [T][2] this block's square sums and maxima (read by the cluster)
+    float* gath = osum + 2 * T;                  // [T][2 CL] the blocks' square sums and maxima
+    float* xin = gath + 2 * CL * T;              // trees: [T + 3][2 HS + QC] conv inputs
+    constexpr int NC = GDN_THREADS;
+    int* anc = reinterpret_cast<int*>(xin + (size_t) (T + 3) * NC);   // trees: [T][3]
+    auto slot_of = [&](int t) {   // the ring slot of row t's result (cur + 1 + t < 2 NS)
+        const int v = cur + 1 + t;
+        return v >= NS ? v - NS : v;
     };
-    constexpr int SB = 20;   // loads in flight per thread: a 5-row window's conv inputs in one round
-    // the conv weights of this thread's channels ride along
-    float4 cw3[3];
+    const int cc = (warp & 3) * 8 + (lane & 7), rg = lane >> 3;
+    const size_t soff = (size_t) lv * GDN_HS * GDN_HS + (size_t) (4 * rg) * GDN_HS + qq * GDN_QC + cc;
+    uint64_t s[16];   // pairs of key rows: s[2 j + h] = rows 16 j + 4 rg + 2 h, + 1
+    auto load_state = [&](int slot) {
+        const float* src = p.S_pool + (size_t) slot * ssz + soff;
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const int e = tid + k * GDN_THREADS;
-        cw3[k] = e < NC ? *reinterpret_cast<const float4*>(convw + chan(e) * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int j = 0; j < 8; ++j)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) s[2 * j + h] = f2_pack(src[(size_t) (16 * j + 2 * h) * GDN_HS], src[(size_t) (16 * j + 2 * h + 1) * GDN_HS]);
+    };
+    if (warp < 4) load_state(cur);
+    // this thread's channel: q, k or v element
+    const int part = tid < GDN_HS ? 0 : tid < 2 * GDN_HS ? 1 : 2, el = part < 2 ? tid - part * GDN_HS : tid - 2 * GDN_HS;
+    const int c = part == 0 ? kh * GDN_HS + el : part == 1 ? p.nk * GDN_HS + kh * GDN_HS + el : 2 * p.nk * GDN_HS + lv * GDN_HS + qq * GDN_QC + el;
+    const float* hin = p.hist_pool + (size_t) cur * hsz;
+    const float4 cw = *reinterpret_cast<const float4*>(p.convw + c * 4);
+    float h0 = hin[c], h1 = hin[ch + c], h2 = hin[2 * ch + c];
+    const float dtv = p.dt[lv], av = p.a[lv], nwv = p.nw[qq * GDN_QC + lane];
+    pdl_wait();   // from here on: the projections
+    pdl_launch_dependents();
+    if (tid >= NC - 32 && lane < T) {
+        const float* abt = p.ab + (size_t) lane * p.ldab;
+        const float x = abt[lv] + dtv, be = abt[p.nv + lv];
+        gates[2 * lane] = expf((x > 20.0f ? x : log1pf(expf(x))) * av);
+        gates[2 * lane + 1] = 1.0f / (1.0f + expf(-be));
     }
-    for (int i0 = tid; i0 < (T + 3) * NC; i0 += SB * GDN_THREADS) {
-        float v[SB];
+    const bool writes = part == 2 || (lv < p.nk && qq == 0);   // one block per channel writes its history
+    float* xout = part == 0 ? xq + el : part == 1 ? xk + el : vs + el;
+    const int xstr = part < 2 ? GDN_HS : GDN_QC;
+    auto put = [&](int t, float x3, float x2, float x1, float x0) {
+        const float x = cw.x * x3 + cw.y * x2 + cw.z * x1 + cw.w * x0;
+        xout[t * xstr] = x / (1.0f + expf(-x));
+        if (writes) {
+            float* hout = p.hist_pool + (size_t) slot_of(t) * hsz + c;
+            hout[0] = x2;
+            hout[ch] = x1;
+            hout[2 * ch] = x0;
+        }
+    };
+    const float* src = p.qkvz + c;
+    if (!p.parent) {   // a chain: the channel's inputs pass through registers, eight rows' loads in flight
+        for (int t0 = 0; t0 < T; t0 += 8) {
+            float x[8];
 #pragma unroll
-        for (int j = 0; j < SB; ++j) {
-            const int i = i0 + j * GDN_THREADS;
-            v[j] = 0.f;
-            if (i < (T + 3) * NC) {
-                const int r = i / NC, c = chan(i % NC);
-                v[j] = r < 3 ? hin[(size_t) r * ch + c] : qkvz[(size_t) (r - 3) * stride + c];
+            for (int i = 0; i < 8; ++i) x[i] = t0 + i < T ? src[(size_t) (t0 + i) * p.stride] : 0.f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                if (t0 + i >= T) break;
+                put(t0 + i, h0, h1, h2, x[i]);
+                h0 = h1;
+                h1 = h2;
+                h2 = x[i];
             }
         }
+    } else {   // a tree: the inputs staged, rows 0..2 = the starting history (oldest first), row 3 + t = window row t
+        xin[tid] = h0;
+        xin[NC + tid] = h1;
+        xin[2 * NC + tid] = h2;
+        for (int t0 = 0; t0 < T; t0 += 16) {
+            float x[16];
 #pragma unroll
-        for (int j = 0; j < SB; ++j) {
-            const int i = i0 + j * GDN_THREADS;
-            if (i < (T + 3) * NC) xin[i] = v[j];
-        }
-    }
-    // the three rows before each window row on its path, as rows of xin (past the root: the history)
-    if (tid < T) {
-        int a = tid;
-        for (int k = 1; k <= 3; ++k) {
-            if (a >= 0) a = parent ? parent[a] : a - 1;
-            else --a;                      // a = -1 - (rows past the root)
-            anc[tid * 3 + k - 1] = a >= 0 ? 3 + a : 3 + a;   // -1 -> row 2 (newest history), -2 -> row 1, -3 -> row 0
-        }
-    }
-    __syncthreads();
+            for (int i = 0; i < 16; ++i) x[i] = t0 + i < T ? src[(size_t) (t0 + i) * p.stride] : 0.f;
 #pragma unroll
-    for (int k3 = 0; k3 < 3; ++k3) {
-        const int e = tid + k3 * GDN_THREADS;
-        if (e >= NC) continue;
-        const int part = e < GDN_HS ? 0 : e < 2 * GDN_HS ? 1 : 2, i = part < 2 ? e - part * GDN_HS : e - 2 * GDN_HS;
-        const int c = chan(e);
-        const float4 cw = cw3[k3];
-        const float w0 = cw.x, w1 = cw.y, w2 = cw.z, w3 = cw.w;
-        const bool writes = part == 2 || (lv < nk && qq == 0);   // one block per channel writes its history
-        for (int t = 0; t < T; ++t) {
-            const float x3 = xin[anc[t * 3 + 2] * NC + e], x2 = xin[anc[t * 3 + 1] * NC + e], x1 = xin[anc[t * 3] * NC + e];
-            const float x0 = xin[(3 + t) * NC + e];
-            const float x = w0 * x3 + w1 * x2 + w2 * x1 + w3 * x0;
-            const float v = x / (1.0f + expf(-x));
-            if (part == 0) xq[t * GDN_HS + i] = v;
-            else if (part == 1) xk[t * GDN_HS + i] = v;
-            else vs[t * GDN_QC + i] = v;
-            if (writes && (!last_only || t == T - 1)) {
-                float* hout = hist_pool + (size_t) ((cur + 1 + t) % NS) * hsz;
-                hout[c] = x2;
-                hout[ch + c] = x1;
-                hout[2 * ch + c] = x0;
+            for (int i = 0; i < 16; ++i)
+                if (t0 + i < T) xin[(size_t) (3 + t0 + i) * NC + tid] = x[i];
+        }
+        // the three rows before each window row on its path, as rows of xin (past the root: the history)
+        if (tid < T) {
+            int a = tid;
+            for (int k = 1; k <= 3; ++k) {
+                if (a >= 0) a = p.parent[a];
+                else --a;                      // a = -1 - (rows past the root)
+                anc[tid * 3 + k - 1] = 3 + a;  // -1 -> row 2 (newest history), -2 -> row 1, -3 -> row 0
             }
         }
-    }
-    __syncthreads();
-    // ---- L2 norms of q and k per row: thread = element (HS == GDN_THREADS)
-    for (int t = 0; t < T; ++t) {
-        const float qv = xq[t * GDN_HS + tid], kv = xk[t * GDN_HS + tid];
-        const float sq = warp_sum(qv * qv), sk = warp_sum(kv * kv);
-        if (lane == 0) { red[warp * 2 * T + t] = sq; red[warp * 2 * T + T + t] = sk; }
-    }
-    __syncthreads();
-    for (int t = 0; t < T; ++t) {
-        float sq = 0.f, sk = 0.f;
-        for (int w = 0; w < 4; ++w) { sq += red[w * 2 * T + t]; sk += red[w * 2 * T + T + t]; }
-        xq[t * GDN_HS + tid] *= rsqrtf(sq + 1e-6f);
-        xk[t * GDN_HS + tid] *= rsqrtf(sk + 1e-6f);
-    }
-    __syncthreads();
-    // ---- the delta rule: warp `part` holds key rows [32 part, +32) of the block's QC value columns, lane = column
-    int have = -1;   // the row whose result the registers hold (-1: the starting state)
-    const float scale = rsqrtf((float) GDN_HS);
-#pragma unroll 1
-    for (int t = 0; t < T; ++t) {
-        const int par = parent ? parent[t] : t - 1;
-        if (par != have) {
-            const float* src = S_pool + (size_t) (par < 0 ? cur : (cur + 1 + par) % NS) * ssz + soff;
-#pragma unroll
-            for (int r = 0; r < 32; ++r) s[r] = src[(size_t) r * GDN_HS];
-        }
-        const float gv = gates[2 * t], bv = gates[2 * t + 1];
-        const float* kt = xk + t * GDN_HS + part * 32;
-        const float* qt = xq + t * GDN_HS + part * 32;
-        float kvd = 0.f;
-#pragma unroll
-        for (int r = 0; r < 32; ++r) kvd = fmaf(s[r], kt[r], kvd);
-        float* kr = kred + (t & 1) * 4 * GDN_QC;
-        kr[part * GDN_QC + lane] = kvd;
         __syncthreads();
-        const float kvs = (kr[lane] + kr[GDN_QC + lane]) + (kr[2 * GDN_QC + lane] + kr[3 * GDN_QC + lane]);
-        const float delta = (vs[t * GDN_QC + lane] - gv * kvs) * bv;
-        float at = 0.f;
-        float* dst = S_pool + (size_t) ((cur + 1 + t) % NS) * ssz + soff;
-        const bool keep = !last_only || t == T - 1;
+        for (int t = 0; t < T; ++t) put(t, xin[anc[t * 3 + 2] * NC + tid], xin[anc[t * 3 + 1] * NC + tid], xin[anc[t * 3] * NC + tid], xin[(3 + t) * NC + tid]);
+    }
+    __syncthreads();
+    // ---- the L2 norms of q and k: a warp per (row, vector)
+    for (int i = warp; i < 2 * T; i += NC / 32) {
+        const float4 v = *reinterpret_cast<const float4*>((i & 1 ? xk : xq) + (i >> 1) * GDN_HS + lane * 4);
+        const float ss = warp_sum((v.x * v.x + v.y * v.y) + (v.z * v.z + v.w * v.w));
+        if (lane == 0) fac[i] = rsqrtf(ss + 1e-6f);
+    }
+    __syncthreads();
+    // ---- the delta rule
+    if (warp < 4) {
+        int have = -1;   // the row whose result the registers hold (-1: the starting state)
+        const float scale = rsqrtf((float) GDN_HS);
+#pragma unroll 1
+        for (int t = 0; t < T; ++t) {
+            if (p.parent) {
+                const int par = p.parent[t];
+                if (par != have) load_state(par < 0 ? cur : slot_of(par));
+            }
+            const float gv = gates[2 * t], bv = gates[2 * t + 1], fq = fac[2 * t], fk = fac[2 * t + 1];
+            const float* kt = xk + t * GDN_HS + 4 * rg;
+            const float* qt = xq + t * GDN_HS + 4 * rg;
+            uint64_t kp[16], acc[4];
 #pragma unroll
-        for (int r = 0; r < 32; ++r) {
-            s[r] = fmaf(kt[r], delta, gv * s[r]);
-            at = fmaf(s[r], qt[r], at);
-            if (keep) dst[(size_t) r * GDN_HS] = s[r];
+            for (int i = 0; i < 4; ++i) acc[i] = 0ull;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const ulonglong2 k2 = *reinterpret_cast<const ulonglong2*>(kt + 16 * j);
+                kp[2 * j] = k2.x;
+                kp[2 * j + 1] = k2.y;
+                acc[(2 * j) & 3] = f2_fma(s[2 * j], k2.x, acc[(2 * j) & 3]);
+                acc[(2 * j + 1) & 3] = f2_fma(s[2 * j + 1], k2.y, acc[(2 * j + 1) & 3]);
+            }
+            float a0, a1, a2, a3, a4, a5, a6, a7;
+            f2_unpack(acc[0], a0, a1);
+            f2_unpack(acc[1], a2, a3);
+            f2_unpack(acc[2], a4, a5);
+            f2_unpack(acc[3], a6, a7);
+            float kv = ((a0 + a1) + (a2 + a3)) + ((a4 + a5) + (a6 + a7));
+            kv += __shfl_xor_sync(0xffffffffu, kv, 8);
+            kv += __shfl_xor_sync(0xffffffffu, kv, 16);
+            const float dk = (vs[t * GDN_QC + cc] - gv * (kv * fk)) * bv * fk;
+            const uint64_t d2 = f2_pack(dk, dk), g2 = f2_pack(gv, gv);
+            float* dst = p.S_pool + (size_t) slot_of(t) * ssz + soff;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[i] = 0ull;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const ulonglong2 q2 = *reinterpret_cast<const ulonglong2*>(qt + 16 * j);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int i = 2 * j + h;
+                    s[i] = f2_fma(kp[i], d2, f2_mul(g2, s[i]));
+                    acc[i & 3] = f2_fma(s[i], h ? q2.y : q2.x, acc[i & 3]);
+                    float lo, hi;
+                    f2_unpack(s[i], lo, hi);
+                    dst[(size_t) (16 * j + 2 * h) * GDN_HS] = lo;
+                    dst[(size_t) (16 * j + 2 * h + 1) * GDN_HS] = hi;
+                }
+            }
+            f2_unpack(acc[0], a0, a1);
+            f2_unpack(acc[1], a2, a3);
+            f2_unpack(acc[2], a4, a5);
+            f2_unpack(acc[3], a6, a7);
+            float at = ((a0 + a1) + (a2 + a3)) + ((a4 + a5) + (a6 + a7));
+            at += __shfl_xor_sync(0xffffffffu, at, 8);
+            at += __shfl_xor_sync(0xffffffffu, at, 16);
+            if (rg == 0) os[t * GDN_QC + cc] = at * fq * scale;
+            have = t;
         }
-        ared[(t * 4 + part) * GDN_QC + lane] = at;
-        have = t;
+    }
+    // the gate inputs of the warp's output rows (warp, warp + 9, ...), fetched while the rule runs
+    constexpr int OR = (FNX_MAX_ROWS + NC / 32 - 1) / (NC / 32);
+    float u[OR];
+#pragma unroll
+    for (int j = 0; j < OR; ++j) {
+        const int t = warp + j * (NC / 32);
+        u[j] = t < T ? p.qkvz[(size_t) t * p.stride + ch + lv * GDN_HS + qq * GDN_QC + lane] : 0.f;
     }
     __syncthreads();
-    // ---- this block's outputs and their square sums per row
-    float ov[FNX_MAX_ROWS / 4];   // warp w keeps rows w, w + 4, ... of column `lane`
-    for (int t = warp, j = 0; t < T; t += 4, ++j) {
-        const float o = ((ared[(t * 4 + 0) * GDN_QC + lane] + ared[(t * 4 + 1) * GDN_QC + lane]) +
-                         (ared[(t * 4 + 2) * GDN_QC + lane] + ared[(t * 4 + 3) * GDN_QC + lane])) * scale;
-        ov[j] = o;
-        const float sq = warp_sum(o * o);
-        if (lane == 0) osum[t] = sq;
+    // ---- the outputs times their norm weight and gate; their square sums and maxima
+#pragma unroll
+    for (int j = 0; j < OR; ++j) {
+        const int t = warp + j * (NC / 32);
+        if (t >= T) break;
+        const float o = os[t * GDN_QC + lane];
+        u[j] = o * nwv / (1.0f + expf(-u[j]));
+        const float sq = warp_sum(o * o), mx = CL > GDN_Q ? warp_max(fabsf(u[j])) : 0.f;
+        if (lane == 0) *reinterpret_cast<float2*>(osum + 2 * t) = make_float2(sq, mx);
     }
-    // the gate inputs z, fetched while the cluster gathers (they do not depend on it)
-    float zv[FNX_MAX_ROWS / 4];
-    for (int t = warp, j = 0; t < T; t += 4, ++j) zv[j] = qkvz[(size_t) t * stride + ch + lv * GDN_HS + col];
-    const float nwv = nw[col];
     cluster.sync();
-    // every block's T square sums into this block's shared memory, one remote read per thread
-    float* msum = red;   // [T] (red is free by now)
-    for (int i = tid; i < T * GDN_Q; i += GDN_THREADS) kred[i] = cluster.map_shared_rank(osum, i % GDN_Q)[i / GDN_Q];
+    for (int i = tid; i < T * CL; i += NC) {   // every block's, one remote read per thread
+        const int t = i / CL, r = i % CL;
+        const float2 v = *reinterpret_cast<const float2*>(cluster.map_shared_rank(osum, r) + 2 * t);
+        gath[t * 2 * CL + r] = v.x;
+        gath[t * 2 * CL + CL + r] = v.y;
+    }
     __syncthreads();
-    if (tid < T) msum[tid] = ((kred[tid * GDN_Q] + kred[tid * GDN_Q + 1]) + (kred[tid * GDN_Q + 2] + kred[tid * GDN_Q + 3])) / (float) GDN_HS;
-    __syncthreads();
-    for (int t = warp, j = 0; t < T; t += 4, ++j)
-        y[(size_t) t * nv * GDN_HS + lv * GDN_HS + col] = ov[j] * rsqrtf(msum[t] + eps) * nwv / (1.0f + expf(-zv[j]));
+    const int hb = CL > GDN_Q ? (lv & 1) * GDN_Q : 0;   // the head's blocks in the cluster
+#pragma unroll
+    for (int j = 0; j < OR; ++j) {
+        const int t = warp + j * (NC / 32);
+        if (t >= T) break;
+        const float* gt = gath + t * 2 * CL;
+        const float r = rsqrtf(((gt[hb] + gt[hb + 1]) + (gt[hb + 2] + gt[hb + 3])) / (float) GDN_HS + p.eps), yv = u[j] * r;
+        p.y[(size_t) t * p.nv * GDN_HS + lv * GDN_HS + qq * GDN_QC + lane] = yv;
+        if (CL > GDN_Q) {   // the image: the block's 32 columns are a sub-block of it, eight lanes a cell of each level
+            const int ob = GDN_Q - hb;
+            const float ro = rsqrtf(((gt[ob] + gt[ob + 1]) + (gt[ob + 2] + gt[ob + 3])) / (float) GDN_HS + p.eps);
+            const float* gm = gt + CL;
+            const float am = fmaxf(fmaxf(fmaxf(gm[hb], gm[hb + 1]), fmaxf(gm[hb + 2], gm[hb + 3])) * r, fmaxf(fmaxf(gm[ob], gm[ob + 1]), fmaxf(gm[ob + 2], gm[ob + 3])) * ro);
+            uint32_t w1, w2;
+            float d;
+            ni_code(yv, am, w1, w2, d);
+            w1 <<= 8 * (lane & 3);
+            w2 <<= 8 * (lane & 3);
+#pragma unroll
+            for (int o = 1; o < 4; o <<= 1) {
+                w1 |= __shfl_xor_sync(0xffffffffu, w1, o);
+                w2 |= __shfl_xor_sync(0xffffffffu, w2, o);
+            }
+            const int KB = p.nv * GDN_HS / 256, sb = (lv & 1) * 4 + qq;
+            uint8_t* rec = p.img + (size_t) t * ni_row_bytes(KB) + (size_t) (lv >> 1) * NI_BYTES;
+            uint8_t* cell = rec + (sb >> 1) * 64 + (lane >> 3) * 16 + (sb & 1) * 8 + (lane & 4);
+            if ((lane & 3) == 0) *reinterpret_cast<uint32_t*>(cell) = w1;
+            if ((lane & 3) == 1) *reinterpret_cast<uint32_t*>(cell + 256) = w2;
+            if (sb == 0 && lane == 2) *reinterpret_cast<float4*>(rec + NI_SCALE) = make_float4(d, d * (1.0f / 256.0f), 0.f, 0.f);
+        }
+    }
     cluster.sync();   // no block may leave while a neighbour still reads its shared memory
 }
 
-__global__ void __cluster_dims__(GDN_Q, 1, 1) __launch_bounds__(GDN_THREADS)
-    k_gdn_core(const float* __restrict__ qkvz, int stride, const float* __restrict__ ab, int ldab, float* __restrict__ hist_pool,
-               const float* __restrict__ convw, const float* __restrict__ dt, const float* __restrict__ a_,
-               const float* __restrict__ nw, float* __restrict__ S_pool, const int* __restrict__ curp, int NS,
-               const int* __restrict__ parent, float* __restrict__ y, int nk, int nv, int T, float eps, int cur_off, int last_only) {
-    pdl_wait();
-    pdl_launch_dependents();
+template <int CL>
+__global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(GDN_THREADS, 2) k_gdn_core(const GdnArgs p, const int* __restrict__ curp) {
     extern __shared__ __align__(16) float sm[];
-    gdn_body(qkvz, stride, ab, ldab, hist_pool, convw, dt, a_, nw, S_pool, (*curp + cur_off) % NS, NS, parent, y, nk, nv, T, eps, sm, last_only != 0);
+    gdn_body<CL>(p, *curp % p.NS, sm);
 }
 
 // Batched lanes: blockIdx.y = lane j, the rows [lane_row0[j], lane_row0[j + 1]) of sequence lane_seq[j], a chain from
 // that sequence's state slot cur[seq] in its own rings (hist_pool + seq * hist_stride, S_pool + seq * s_stride)
 // (gdn_core_segs, engine/src/kernels.cu:2112-2156).  Every block of a cluster has the same lane, so all of them take
 // the same path.
-__global__ void __cluster_dims__(GDN_Q, 1, 1) __launch_bounds__(GDN_THREADS)
-    k_gdn_core_lanes(const float* __restrict__ qkvz, int stride, const float* __restrict__ ab, int ldab, float* __restrict__ hist_pool, size_t hist_stride,
-                     const float* __restrict__ convw, const float* __restrict__ dt, const float* __restrict__ a_, const float* __restrict__ nw,
-                     float* __restrict__ S_pool, size_t s_stride, const int* __restrict__ cur, int NS, const int* __restrict__ lane_seq,
-                     const int* __restrict__ lane_row0, float* __restrict__ y, int nk, int nv, float eps) {
+template <int CL>
+__global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(GDN_THREADS, 2)
+    k_gdn_core_lanes(const GdnArgs p0, size_t hist_stride, size_t s_stride, const int* __restrict__ cur, const int* __restrict__ lane_seq,
+                     const int* __restrict__ lane_row0) {
     extern __shared__ __align__(16) float sm[];
     const int lane = blockIdx.y, row0 = lane_row0[lane], T = lane_row0[lane + 1] - row0, seq = lane_seq[lane];
-    if (T <= 0 || seq < 0) return;   // (a negative sequence: another rank's lane)
-    gdn_body(qkvz + (size_t) row0 * stride, stride, ab + (size_t) row0 * ldab, ldab, hist_pool + seq * hist_stride, convw, dt, a_, nw, S_pool + seq * s_stride,
-             cur[seq], NS, nullptr, y + (size_t) row0 * nv * GDN_HS, nk, nv, T, eps, sm);
+    if (T <= 0 || seq < 0) {   // (a negative sequence: another rank's lane)
+        pdl_wait();
+        return;
+    }
+    GdnArgs p = p0;
+    p.qkvz += (size_t) row0 * p.stride;
+    p.ab += (size_t) row0 * p.ldab;
+    p.hist_pool += seq * hist_stride;
+    p.S_pool += seq * s_stride;
+    p.y += (size_t) row0 * p.nv * GDN_HS;
+    if (p.img) p.img += (size_t) row0 * ni_row_bytes(p.nv * GDN_HS / 256);
+    p.T = T;
+    p.parent = nullptr;
+    gdn_body<CL>(p, cur[seq], sm);
 }
 
 // ------------------------------------------------------------------------------------------------ prompts
@@ -279,28 +366,8 @@ __global__ void __launch_bounds__(GDP_THREADS) k_gdn_pre(const float* __restrict
 
 // block = (value head, column quarter) as in the window kernel: warp `part` holds key rows [32 part, +32) of the block's 32 value
 // columns, lane = column.  Rows stream through two shared-memory tiles of GDS_ROWS rows.
-// two f32 in a 64-bit register and the packed multiply-add on them (fma.rn.f32x2: each half rounded as the scalar fmaf is, so the
-// scan's products are those of its scalar form, at half the arithmetic instructions: the scan is bound by instruction issue, with
-// one warp per scheduler)
-__device__ __forceinline__ uint64_t f2_pack(float x, float y) {
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
-    return r;
-}
-__device__ __forceinline__ void f2_unpack(uint64_t r, float& x, float& y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(r)); }
-__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
-    uint64_t d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-
 constexpr int GDS_ROWS = 16;
-__global__ void __launch_bounds__(GDN_THREADS) k_gdn_scan(const float* __restrict__ xq, const float* __restrict__ xk, const float* __restrict__ xv,
+__global__ void __launch_bounds__(GDS_THREADS) k_gdn_scan(const float* __restrict__ xq, const float* __restrict__ xk, const float* __restrict__ xv,
                                                           const float* __restrict__ gates, const float* __restrict__ S_in, float* __restrict__ S_out,
                                                           float* __restrict__ o, int nk, int nv, int T) {
     constexpr int ROWF = 2 * GDN_HS + GDN_QC + 2;   // floats of a staged row: k, q, the block's v, the two gates
@@ -314,7 +381,7 @@ __global__ void __launch_bounds__(GDN_THREADS) k_gdn_scan(const float* __restric
     for (int r = 0; r < 32; r += 2) s[r / 2] = f2_pack(S_in[soff + (size_t) r * GDN_HS], S_in[soff + (size_t) (r + 1) * GDN_HS]);
     auto stage = [&](int buf, int t0) {
         const int nr = min(GDS_ROWS, T - t0);
-        for (int i = tid; i < nr * (ROWF / 2); i += GDN_THREADS) {   // 8-byte pieces
+        for (int i = tid; i < nr * (ROWF / 2); i += GDS_THREADS) {   // 8-byte pieces
             const int r = i / (ROWF / 2), e = (i % (ROWF / 2)) * 2, t = t0 + r;
             const float* src;
             if (e < GDN_HS) src = xk + ((size_t) t * nk + kh) * GDN_HS + e;
@@ -388,7 +455,7 @@ __global__ void __launch_bounds__(GDN_THREADS) k_gdn_scan(const float* __restric
             ared[r0][part][lane] = ((a0 + a1) + (a2 + a3)) + ((a4 + a5) + (a6 + a7));
         }
         __syncthreads();   // the tile's sums are complete; its buffer may be refilled two tiles on
-        for (int i = tid; i < nr * GDN_QC; i += GDN_THREADS) {
+        for (int i = tid; i < nr * GDN_QC; i += GDS_THREADS) {
             const int r0 = i / GDN_QC, c = i % GDN_QC;
             o[((size_t) (t0 + r0) * nv + lv) * GDN_HS + qq * GDN_QC + c] = ((ared[r0][0][c] + ared[r0][1][c]) + (ared[r0][2][c] + ared[r0][3][c])) * scale;
         }
@@ -422,9 +489,26 @@ __global__ void __launch_bounds__(GDP_THREADS) k_gdn_post(const float* __restric
     }
 }
 
-static size_t gdn_smem_bytes(int T) {
-    return sizeof(float) * ((size_t) 2 * T * GDN_HS + (size_t) T * GDN_QC + 2 * T + 2 * 4 * GDN_QC + (size_t) T * 4 * GDN_QC + T + 8 * T +
-                            (size_t) (T + 3) * (2 * GDN_HS + GDN_QC) + 3 * T);
+static size_t gdn_smem_bytes(int T, int CL, bool tree) {
+    return sizeof(float) * ((size_t) 2 * T * GDN_HS + (size_t) 2 * T * GDN_QC + 6 * T + 2 * CL * T + (tree ? (size_t) (T + 3) * (2 * GDN_HS + GDN_QC) + 3 * T : 0));
+}
+
+// an image needs the two heads of its 256-column blocks in one cluster
+int gdn_window(const GdnArgs& p, const int* cur, bool early, cudaStream_t st) {
+    const int CL = p.img ? 2 * GDN_Q : GDN_Q;
+    auto kernel = p.img ? k_gdn_core<2 * GDN_Q> : k_gdn_core<GDN_Q>;
+    if (int rc = set_smem_limit((const void*) kernel, 112 * 1024)) return rc;
+    const cudaError_t le = launch_dep(early, kernel, dim3(p.nv * GDN_Q), dim3(GDN_THREADS), gdn_smem_bytes(p.T, CL, p.parent != nullptr), st, p, cur);
+    return le == cudaSuccess ? FNX_OK : fail(FNX_E_CUDA, "k_gdn_core: launch failed: %s", cudaGetErrorString(le));
+}
+int gdn_window_lanes(const GdnArgs& p, size_t hist_seq_stride, size_t s_seq_stride, const int* cur, const int* lane_seq, const int* lane_row0, int n_lanes, int max_rows,
+                     bool early, cudaStream_t st) {
+    const int CL = p.img ? 2 * GDN_Q : GDN_Q;
+    auto kernel = p.img ? k_gdn_core_lanes<2 * GDN_Q> : k_gdn_core_lanes<GDN_Q>;
+    if (int rc = set_smem_limit((const void*) kernel, 112 * 1024)) return rc;
+    const cudaError_t le = launch_dep(early, kernel, dim3(p.nv * GDN_Q, n_lanes), dim3(GDN_THREADS), gdn_smem_bytes(max_rows, CL, false), st, p, hist_seq_stride, s_seq_stride, cur,
+                                      lane_seq, lane_row0);
+    return le == cudaSuccess ? FNX_OK : fail(FNX_E_CUDA, "k_gdn_core_lanes: launch failed: %s", cudaGetErrorString(le));
 }
 
 }  // namespace fnxb
@@ -438,14 +522,7 @@ extern "C" int fnx_gdn_core(const float* qkvz, int ldx, const float* ab, int lda
     FNX_REQUIRE(hs == GDN_HS, "fnx_gdn_core: head dim %d (this build: %d)", hs, GDN_HS);
     FNX_REQUIRE(T >= 1 && T <= FNX_MAX_ROWS && NS >= T + 1, "fnx_gdn_core: %d rows need at least %d state slots, have %d", T, T + 1, NS);
     FNX_REQUIRE(nk >= 1 && nv >= nk && nv % nk == 0, "fnx_gdn_core: %d key heads, %d value heads", nk, nv);
-    const size_t smem = gdn_smem_bytes(T);
-    if (int rc = set_smem_limit((const void*) k_gdn_core, 96 * 1024)) return rc;
-    {
-        const cudaError_t le_ = launch_k(k_gdn_core, dim3(nv * GDN_Q), dim3(GDN_THREADS), smem, as_stream(st), qkvz, ldx, ab, ldab, hist_pool, convw, dt, a, nw, S_pool, cur, NS, parent, y, nk, nv, T, eps, 0, 0);
-        if (le_ != cudaSuccess) return fail(FNX_E_CUDA, "k_gdn_core: launch failed: %s", cudaGetErrorString(le_));
-    }
-    FNX_LAUNCH_OK("fnx_gdn_core");
-    return FNX_OK;
+    return gdn_window(GdnArgs{qkvz, ldx, ab, ldab, hist_pool, convw, dt, a, nw, S_pool, NS, parent, y, nullptr, nk, nv, T, eps}, cur, false, as_stream(st));
 }
 
 extern "C" size_t fnx_gdn_prompt_scratch_bytes(int T, int nk, int nv, int hs) {
@@ -473,7 +550,7 @@ extern "C" int fnx_gdn_prompt(const float* qkvz, int ldx, const float* ab, int l
     k_gdn_pre<<<T, GDP_THREADS, 0, s>>>(qkvz, ldx, ab, ldab, hin, hist_pool + (size_t) out_slot * hsz, convw, dt, a, xq, xk, xv, gates, nk,
                                          nv, T);
     FNX_LAUNCH_OK("k_gdn_pre");
-    k_gdn_scan<<<nv * GDN_Q, GDN_THREADS, 0, s>>>(xq, xk, xv, gates, S_pool + (size_t) cur_host * ssz, S_pool + (size_t) out_slot * ssz, o, nk, nv, T);
+    k_gdn_scan<<<nv * GDN_Q, GDS_THREADS, 0, s>>>(xq, xk, xv, gates, S_pool + (size_t) cur_host * ssz, S_pool + (size_t) out_slot * ssz, o, nk, nv, T);
     FNX_LAUNCH_OK("k_gdn_scan");
     k_gdn_post<<<T, GDP_THREADS, 0, s>>>(o, qkvz, ldx, nw, y, nk, nv, eps);
     FNX_LAUNCH_OK("k_gdn_post");
@@ -489,10 +566,6 @@ extern "C" int fnx_gdn_core_lanes(const float* qkvz, int ldx, const float* ab, i
     FNX_REQUIRE(n_lanes >= 1 && n_lanes <= FNX_MAX_ROWS && max_lane_rows >= 1 && NS >= max_lane_rows + 1, "fnx_gdn_core_lanes: %d lanes of up to %d rows, %d state slots",
                 n_lanes, max_lane_rows, NS);
     FNX_REQUIRE(nk >= 1 && nv >= nk && nv % nk == 0, "fnx_gdn_core_lanes: %d key heads, %d value heads", nk, nv);
-    if (int rc = set_smem_limit((const void*) k_gdn_core_lanes, 96 * 1024)) return rc;
-    const cudaError_t le = launch_k(k_gdn_core_lanes, dim3(nv * GDN_Q, n_lanes), dim3(GDN_THREADS), gdn_smem_bytes(max_lane_rows), as_stream(st), qkvz, ldx, ab, ldab,
-                                    hist_pool, hist_seq_stride, convw, dt, a, nw, S_pool, s_seq_stride, cur, NS, lane_seq, lane_row0, y, nk, nv, eps);
-    if (le != cudaSuccess) return fail(FNX_E_CUDA, "k_gdn_core_lanes: launch failed: %s", cudaGetErrorString(le));
-    FNX_LAUNCH_OK("fnx_gdn_core_lanes");
-    return FNX_OK;
+    return gdn_window_lanes(GdnArgs{qkvz, ldx, ab, ldab, hist_pool, convw, dt, a, nw, S_pool, NS, nullptr, y, nullptr, nk, nv, max_lane_rows, eps}, hist_seq_stride,
+                            s_seq_stride, cur, lane_seq, lane_row0, n_lanes, max_lane_rows, false, as_stream(st));
 }

@@ -16,6 +16,15 @@ constexpr int NI_SCALE = 512, NI_RS = 520, NI_BYTES = 528;
 __host__ __device__ __forceinline__ size_t ni_row_bytes(int KB) { return ((size_t) KB * NI_BYTES + 127) / 128 * 128 + 64; }
 __host__ __device__ inline size_t ni_bytes(int T, int K) { return (size_t) T * ni_row_bytes(K / 256); }
 
+// one value's two codes (in the words' low bytes: core_quant_cell's) and its block's scale, given the block's maximum
+__device__ __forceinline__ void ni_code(float x, float am, uint32_t& a, uint32_t& b, float& d) {
+    constexpr float MAGIC = 12582912.0f;
+    d = am * (1.0f / 127.0f);
+    const float inv = am > 0.f ? __fdividef(127.0f, am) : 0.f, ta = fmaf(x, inv, MAGIC);
+    a = __float_as_uint(ta) & 255u;
+    b = __float_as_uint(fminf(fmaf(fmaf(-(ta - MAGIC), d, x), inv * 256.0f, MAGIC), MAGIC + 127.0f)) & 255u;
+}
+
 // One warp, one 256-column block of a row: v = the lane's 8 values (columns 8 lane ..), times the norm weight where there is one;
 // ss = the lane's share of the raw values' sum of squares (not normed: 0).
 __device__ __forceinline__ void ni_quant_at(uint8_t* rec, const float (&v)[8], float ss, int lane) {
