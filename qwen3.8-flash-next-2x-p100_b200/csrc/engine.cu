@@ -402,6 +402,8 @@ int prompt_dense(const void* W, bool nat, int rows, int cols, const float* x, in
 int prompt_moe(const void* Wgu, size_t gu_stride, const void* Wsh_gu, bool gu_nat, const void* Wdn, size_t dn_stride, const void* Wsh_dn, bool dn_nat, int e_base, int E,
                int K, int e_lo, int e_hi, int add_shared, const int* topi, const float* topw, const float* logits, const float* x, const float* norm_w, float eps, int T,
                int H, int F, float* out, int accumulate, void* scratch, unsigned* err, cudaStream_t st);
+int router_window(const float* Wr, const float* x, const float* norm_w, float eps, int T, int E, int H, int K, int e_lo, int e_hi, int add_shared, float* logits, int* topi,
+                  float* topw, fnx_job* jobs, int* njobs, unsigned long long* stats, unsigned* err, uint8_t* img, bool early, cudaStream_t st);
 int moe_combine_nat(const float* part, const int* topi, const float* topw, const float* logits, int T, int E, int H, int K, float* R, uint8_t* img, const float* img_norm_w,
                     cudaStream_t st);
 
@@ -678,9 +680,8 @@ static int enqueue_moe(fnx_engine* e, const LayerW& L, float* R, int T, const Ma
     const Dims d = dims(e->c);
     const bool ep = e->c.ep_size > 1, img = next && next->nat && next_norm;
     if (img_ready) *img_ready = false;
-    if (L.wgu.nat) FNX_TRY(nat_rows_image(R, d.H, T, d.H, L.norm2, e->img_x, e->st));
-    FNX_TRY(fnx_router_route(L.wr, R, L.norm2, e->c.eps, T, d.E, d.H, d.K, e->e_lo, e->e_hi, 1, e->rlogits, e->topi, e->topw, e->jobs, e->njobs,
-                             e->d_stats, e->err, e->st));
+    FNX_TRY(router_window(L.wr, R, L.norm2, e->c.eps, T, d.E, d.H, d.K, e->e_lo, e->e_hi, 1, e->rlogits, e->topi, e->topw, e->jobs, e->njobs, e->d_stats, e->err,
+                          L.wgu.nat ? e->img_x : nullptr, true, e->st));
     const int njobs_max = T * d.K + (T + FNX_JOB_TOK - 1) / FNX_JOB_TOK;
     if (L.wgu.nat)
         FNX_TRY(nat_gate_up(L.wgu.nat, L.wgu.nat_stride(), e->e_lo, L.wsh_gu.nat, d.E, e->jobs, e->njobs, njobs_max, e->img_x, e->c.eps, d.H, d.F, e->hbuf, e->st));

@@ -1,9 +1,8 @@
 // MoE routing and combine.
 //
 // fnx_router_route replaces router_route / k_router_route (engine/src/kernels.hpp:294-296, engine/src/moe.cuh:258-515)
-// and its simple form route / k_topk + k_jobs (engine/src/kernels.cu:338-398): one launch computes the router logits
-// (f32 weights, a warp per expert row, fixed summation order), and the last block to finish picks the top K per row,
-// renormalises their softmax and lists the jobs.  fnx_moe_combine replaces k_combine (engine/src/kernels.cu:412-419).
+// and its simple form route / k_topk + k_jobs (engine/src/kernels.cu:338-398): router logits (f32 weights, fixed summation order), the
+// top K per row with their renormalised softmax, the job list.  fnx_moe_combine replaces k_combine (engine/src/kernels.cu:412-419).
 #include <algorithm>
 
 #include "fnx_common.cuh"
@@ -14,257 +13,216 @@
 
 namespace fnxb {
 
-constexpr int RT_WARPS = 8, RT_TOK = 8, RT_SPLIT = 2, RT_ROWS = RT_WARPS / RT_SPLIT;
+// ---- the window form, in two launches: the logits over the whole chip, then one block that picks and lists the jobs (with programmatic
+// launch the second costs about 1.3 us; an arrival counter and fences inside the first cost more).
+//
+// Block = ROWS expert rows, warp = one 256-column slice of all of them, lane = 8 consecutive columns (so that a warp holds a block
+// of the rows' image in the quantiser's order): a row's slice feeds ROWS x 8 products per lane straight from registers.  TOK rows
+// at a time make TOK x ROWS = 32 sums per lane, which cross the warp by halving (31 shuffles: lane i ends with sum i); the slices
+// are then added in double.  A row's logits do not depend on the rows it comes with, nor on ROWS.  Everything that depends on no
+// other kernel (the weights, the norm weights) is loaded before the rows are waited for.  f32 products and sums.
+// Windows: 4 expert rows a block (129 blocks), block y = 0 of block column t also leaves row t's image (nat_image.cuh) for the experts'
+// products; bound by the rows' way to every block (T x 8 KB each) and latency: 5 rows 14 -> 4.5 us, 20 rows 34 -> 10 us (with the pick
+// 10 and 20), when one launch did both, eight rows at a time through shared memory.
+// Prompts: 16 expert rows a block, so that the rows cross L2 33 times instead of 129; bound by the products from a few hundred rows
+// on (8 rows a block walking all 513 expert rows took 145 us at any number of rows up to 1,023).
+constexpr int RT_ROWS = 4, RT_PROMPT_ROWS = 16;
 
-// Grid: ceil((E + 1) / RT_ROWS) blocks of RT_WARPS warps; a block computes RT_ROWS logit rows, RT_SPLIT warps per row
-// (each a contiguous share of the columns, summed in share order).
-__global__ void __launch_bounds__(RT_WARPS * 32) k_router(const float* __restrict__ Wr, const float* __restrict__ x,
-                                                          const float* __restrict__ norm_w, float eps, int T, int E, int H, int K,
-                                                          int e_lo, int e_hi, int add_shared, float* __restrict__ logits,
-                                                          int* __restrict__ topi, float* __restrict__ topw, fnx_job* __restrict__ jobs,
-                                                          int* __restrict__ njobs, unsigned long long* __restrict__ stats, unsigned* __restrict__ err) {
+template <int ROWS, int THREADS>
+__global__ void __launch_bounds__(THREADS, 1) k_router_logits(const float* __restrict__ Wr, const float* __restrict__ x, const float* __restrict__ norm_w, float eps, int T,
+                                                          int per, int E, int H, float* __restrict__ logits, unsigned* __restrict__ err, uint8_t* __restrict__ img) {
+    constexpr int TOK = 32 / ROWS;
+    extern __shared__ float sm[];                 // two buffers of psum [warps][32], ss [warps][TOK]
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, NW = H / 256;
+    const int row0 = blockIdx.x * ROWS, c = warp * 256 + lane * 8, t_lo = blockIdx.y * per, t_hi = min(T, t_lo + per);
+    float w[ROWS][8], nw[8];
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+        if (row0 + r <= E) {
+            const float4* p = reinterpret_cast<const float4*>(Wr + (size_t) (row0 + r) * H + c);
+            a = __ldg(p);
+            b = __ldg(p + 1);
+        }
+        w[r][0] = a.x; w[r][1] = a.y; w[r][2] = a.z; w[r][3] = a.w;
+        w[r][4] = b.x; w[r][5] = b.y; w[r][6] = b.z; w[r][7] = b.w;
+    }
+    if (norm_w) {
+        const float4 a = __ldg(reinterpret_cast<const float4*>(norm_w + c)), b = __ldg(reinterpret_cast<const float4*>(norm_w + c) + 1);
+        nw[0] = a.x; nw[1] = a.y; nw[2] = a.z; nw[3] = a.w;
+        nw[4] = b.x; nw[5] = b.y; nw[6] = b.z; nw[7] = b.w;
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) nw[i] = 1.0f;
+    }
     pdl_wait();
     pdl_launch_dependents();
-    extern __shared__ __align__(16) float xs[];   // [RT_TOK][H]: x * norm_w (the row's 1 / rms is applied to the sums)
-    __shared__ float rs[RT_TOK], ssw[RT_TOK][RT_WARPS], psum[RT_ROWS][RT_SPLIT][RT_TOK];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int row = blockIdx.x * RT_ROWS + warp / RT_SPLIT, share = warp % RT_SPLIT;
-    constexpr int NT = RT_WARPS * 32;
-    const int HS = H / RT_SPLIT, c_lo = share * HS;   // this warp's columns
-    // the warp's first weights are on their way before anything else (they depend on nothing)
-    float4 w[8];
-    if (row <= E) {
-        const float* wr = Wr + (size_t) row * H + c_lo;
+    constexpr int LD = THREADS <= 256 ? TOK : 4;   // rows whose loads are in flight together
+    float4 xa[LD], xb[LD];
+    auto fetch = [&](int t) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int i = lane * 4 + j * 128;
-            w[j] = i < HS ? *reinterpret_cast<const float4*>(wr + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-    }
-    for (int t0 = 0; t0 < T; t0 += RT_TOK) {
-        const int nt = min(RT_TOK, T - t0);
-        __syncthreads();
-        // stage the rows with 16-byte async copies, all in flight at once; then, from shared memory, each thread's
-        // columns of every row: the sum of squares and the product with the norm weight
-        for (int i = tid; i < nt * (H / 4); i += NT)
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(xs + (size_t) i * 4)), "l"(x + (size_t) t0 * H + (size_t) i * 4) : "memory");
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        float4 nw4[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int c = tid * 4 + j * NT * 4;
-            nw4[j] = norm_w && c < H ? *reinterpret_cast<const float4*>(norm_w + c) : make_float4(1.f, 1.f, 1.f, 1.f);
-        }
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncthreads();
-        for (int t = 0; t < nt; ++t) {
-            float ss = 0.f;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int c = tid * 4 + j * NT * 4;
-                if (c >= H) continue;
-                float4 v = *reinterpret_cast<const float4*>(xs + (size_t) t * H + c);
-                ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
-                v.x *= nw4[j].x; v.y *= nw4[j].y; v.z *= nw4[j].z; v.w *= nw4[j].w;
-                *reinterpret_cast<float4*>(xs + (size_t) t * H + c) = v;
+        for (int i = 0; i < LD; ++i) {
+            xa[i] = xb[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (t + i < t_hi) {
+                const float4* p = reinterpret_cast<const float4*>(x + (size_t) (t + i) * H + c);
+                xa[i] = p[0];
+                xb[i] = p[1];
             }
-            ss = warp_sum(ss);
-            if (lane == 0) ssw[t][warp] = ss;
         }
-        __syncthreads();
-        if (tid < nt) {
-            float ss = 0.f;
-            for (int wq = 0; wq < RT_WARPS; ++wq) ss += ssw[tid][wq];
-            rs[tid] = norm_w ? rsqrtf(ss / (float) H + eps) : 1.0f;
-        }
-        float acc[RT_TOK];
+    };
+    constexpr bool AHEAD = THREADS <= 256;   // the next rows' loads run under the products (where the registers allow)
+    if (AHEAD) fetch(t_lo);
+    int buf = 0;
+    for (int t0 = t_lo; t0 < t_hi; t0 += TOK, buf ^= 1) {
+        float v[32];   // sum t ROWS + r
+        float sq[TOK];
 #pragma unroll
-        for (int t = 0; t < RT_TOK; ++t) acc[t] = 0.f;
-        if (row <= E) {
-            const float* wr = Wr + (size_t) row * H + c_lo;
-            for (int i0 = 0; i0 < HS; i0 += 1024) {   // 8 float4 of the weight row in flight per lane
-                if (i0 > 0 || t0 > 0) {
+        for (int h = 0; h < TOK; h += LD) {
+            if (!AHEAD) fetch(t0 + h);
+            float e[LD][8];
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        const int i = i0 + lane * 4 + j * 128;
-                        w[j] = i < HS ? *reinterpret_cast<const float4*>(wr + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-                    }
+            for (int t = 0; t < LD; ++t) {
+                e[t][0] = xa[t].x; e[t][1] = xa[t].y; e[t][2] = xa[t].z; e[t][3] = xa[t].w;
+                e[t][4] = xb[t].x; e[t][5] = xb[t].y; e[t][6] = xb[t].z; e[t][7] = xb[t].w;
+            }
+            if (AHEAD) fetch(t0 + h + LD);
+#pragma unroll
+            for (int t = 0; t < LD; ++t) {
+                float ss = 0.f;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    ss = fmaf(e[t][i], e[t][i], ss);
+                    e[t][i] *= nw[i];
                 }
+                sq[h + t] = ss;
+                if (img && t0 + h + t == (int) blockIdx.x && t0 + h + t < t_hi) ni_quant(img, NW, e[t], norm_w ? ss : 0.f, t0 + h + t, warp, lane);
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const int i = i0 + lane * 4 + j * 128;
-                    if (i >= HS) continue;
+                for (int r = 0; r < ROWS; ++r) {
+                    float s = 0.f;
 #pragma unroll
-                    for (int t = 0; t < RT_TOK; ++t)
-                        if (t < nt) {
-                            const float4 v = *reinterpret_cast<const float4*>(xs + (size_t) t * H + c_lo + i);
-                            acc[t] = fmaf(w[j].x, v.x, acc[t]);
-                            acc[t] = fmaf(w[j].y, v.y, acc[t]);
-                            acc[t] = fmaf(w[j].z, v.z, acc[t]);
-                            acc[t] = fmaf(w[j].w, v.w, acc[t]);
-                        }
+                    for (int i = 0; i < 8; ++i) s = fmaf(w[r][i], e[t][i], s);
+                    v[(h + t) * ROWS + r] = s;
                 }
             }
-#pragma unroll
-            for (int t = 0; t < RT_TOK; ++t)
-                if (t < nt) {
-                    const float s = warp_sum(acc[t]);
-                    if (lane == 0) psum[warp / RT_SPLIT][share][t] = s;
-                }
         }
-        __syncthreads();
-        if (tid < RT_ROWS * RT_TOK) {
-            const int r = tid / RT_TOK, t = tid % RT_TOK, grow = blockIdx.x * RT_ROWS + r;
-            if (t < nt && grow <= E) {
-                float s = 0.f;
+        // 32 sums over 32 lanes: at step o a lane keeps the half of its values whose index has the bit its lane number has
 #pragma unroll
-                for (int q = 0; q < RT_SPLIT; ++q) s += psum[r][q][t];
-                s *= rs[t];
-                logits[(size_t) (t0 + t) * (E + 1) + grow] = s;
+        for (int o = 16; o >= 1; o >>= 1) {
+            const bool up = lane & o;
+#pragma unroll
+            for (int i = 0; i < o; ++i) {
+                const float keep = up ? v[i + o] : v[i], give = up ? v[i] : v[i + o];
+                v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+            }
+        }
+#pragma unroll
+        for (int o = TOK / 2; o >= 1; o >>= 1) {
+            const bool up = lane & o;
+#pragma unroll
+            for (int i = 0; i < o; ++i) {
+                const float keep = up ? sq[i + o] : sq[i], give = up ? sq[i] : sq[i + o];
+                sq[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+            }
+        }
+        float ss = sq[0];
+#pragma unroll
+        for (int o = TOK; o < 32; o <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        float* psum = sm + buf * NW * (32 + TOK);
+        float* sqs = psum + NW * 32;
+        psum[warp * 32 + lane] = v[0];
+        if (lane < TOK) sqs[warp * TOK + lane] = ss;
+        __syncthreads();   // (the buffers alternate: the last readers of this one passed the barrier of the step between)
+        if (tid < 32) {
+            const int t = tid / ROWS, r = tid % ROWS;
+            double sd = 0.0, q = 0.0;   // (a handful of additions: the slices' own rounding is what the logits keep)
+            for (int j = 0; j < NW; ++j) {
+                sd += (double) psum[j * 32 + tid];
+                q += (double) sqs[j * TOK + t];
+            }
+            float s = (float) sd;
+            if (norm_w) s *= rsqrtf((float) q / (float) H + eps);
+            if (t0 + t < t_hi && row0 + r <= E) {
+                logits[(size_t) (t0 + t) * (E + 1) + row0 + r] = s;
                 if (!isfinite(s)) atomicOr(err, (unsigned) FNX_ERR_NONFINITE);
             }
         }
     }
-    // ---- the last block to get here routes
-    __shared__ bool last;
-    __shared__ int s_topi[FNX_MAX_ROWS * 32];
-    __shared__ int s_cnt[RT_MAXE];
-    __shared__ int s_base[RT_MAXE];
-    __shared__ int wsum_[32];
-    __shared__ int total_[2];
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) last = atomicAdd(&njobs[1], 1) == (int) gridDim.x - 1;
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    // top K per row: a warp per row, K rounds of (value, index) maximum, ties to the lower index
-    for (int t = warp; t < T; t += RT_WARPS) {
-        const volatile float* l = logits + (size_t) t * (E + 1);
-        if (E <= 512) rt_topk_row<16>(l, E, K, lane, topi + t * K, s_topi + t * K, topw + t * K, nullptr);
-        else rt_topk_row<RT_MAXE / 32>(l, E, K, lane, topi + t * K, s_topi + t * K, topw + t * K, nullptr);
+}
+
+// the logits of T rows; windows (img may be given) or prompts
+static int router_logits(const float* Wr, const float* x, const float* norm_w, float eps, int T, int E, int H, float* logits, unsigned* err, uint8_t* img, bool early,
+                         cudaStream_t st) {
+    const int NW = H / 256;
+    cudaError_t le;
+    if (T <= FNX_MAX_ROWS || H > 2048) {   // (sixteen rows' weights of wider slices do not fit the registers)
+        const int blocks = (E + RT_ROWS) / RT_ROWS;
+        le = launch_dep(early, H <= 2048 ? k_router_logits<RT_ROWS, 256> : k_router_logits<RT_ROWS, 512>,
+                        dim3(img && blocks < T ? T : blocks, (T + FNX_MAX_ROWS - 1) / FNX_MAX_ROWS), dim3(NW * 32), (size_t) 2 * NW * (32 + 32 / RT_ROWS) * sizeof(float), st, Wr,
+                        x, norm_w, eps, T, (int) FNX_MAX_ROWS, E, H, logits, err, img);
+    } else {   // about two blocks an SM, at least eight rows each (their weights are 128 KB)
+        const int blocks = (E + RT_PROMPT_ROWS) / RT_PROMPT_ROWS, want = (2 * sm_count() + blocks - 1) / blocks;
+        int per = (T + want - 1) / want;
+        per = per < 8 ? 8 : (per + 1) / 2 * 2;
+        le = launch_dep(early, k_router_logits<RT_PROMPT_ROWS, 256>, dim3(blocks, (T + per - 1) / per), dim3(NW * 32),
+                        (size_t) 2 * NW * (32 + 32 / RT_PROMPT_ROWS) * sizeof(float), st, Wr, x, norm_w, eps, T, per, E, H, logits, err, img);
     }
-    __syncthreads();
-    // the job list is built in the rows' shared memory (free by now) and copied out
+    return le == cudaSuccess ? FNX_OK : fail(FNX_E_CUDA, "k_router_logits: launch failed: %s", cudaGetErrorString(le));
+}
+
+// One block: the top K of every row (a warp per row), their weights, and the job list, built in shared memory and copied out.
+constexpr int RT_PICK = 1024;   // a warp per row
+__global__ void __launch_bounds__(RT_PICK) k_router_pick(const float* __restrict__ logits, int T, int E, int K, int e_lo, int e_hi, int add_shared, int* __restrict__ topi,
+                                                         float* __restrict__ topw, fnx_job* __restrict__ jobs, int* __restrict__ njobs,
+                                                         unsigned long long* __restrict__ stats) {
+    extern __shared__ __align__(16) uint8_t pick_smem[];   // the job list
+    __shared__ int s_topi[FNX_MAX_ROWS * 32];
+    __shared__ unsigned s_rows[RT_MAXE];
+    __shared__ int s_base[RT_MAXE], wsum_[32], total_[2];
+    __shared__ __align__(16) unsigned scr_[RT_PICK / 32][64];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     RtJobSmem js;
-    js.s_topi = s_topi; js.s_cnt = s_cnt; js.s_base = s_base; js.wsum = wsum_; js.total = total_;
-    js.js = reinterpret_cast<fnx_job*>(xs);
-    rt_build_jobs<NT>(js, tid, T, E, K, e_lo, e_hi, add_shared);
+    js.s_topi = s_topi; js.s_rows = s_rows; js.s_base = s_base; js.wsum = wsum_; js.total = total_;
+    js.js = reinterpret_cast<fnx_job*>(pick_smem);
+    pdl_wait();
+    pdl_launch_dependents();
+    for (int t = warp; t < T; t += RT_PICK / 32) {
+        const float* l = logits + (size_t) t * (E + 1);
+        int* ti = topi + t * K;
+        float* tw = topw + t * K;
+        if (E <= 512) rt_topk_row<16>(l, E, K, lane, scr_[warp], ti, s_topi + t * K, tw, nullptr);
+        else rt_topk_row<RT_MAXE / 32>(l, E, K, lane, scr_[warp], ti, s_topi + t * K, tw, nullptr);
+    }
+    rt_build_jobs<RT_PICK>(js, tid, T, E, K, e_lo, e_hi, add_shared);
+    __syncthreads();
     const int total = total_[0];
     if (tid == 0) {
         njobs[0] = total;
-        njobs[1] = 0;
         if (stats) {
             atomicAdd(&stats[0], (unsigned long long) total_[1]);
             atomicAdd(&stats[1], 1ull);
         }
     }
     constexpr int JW = sizeof(fnx_job) / 4;
-    for (int w = tid; w < total * JW; w += NT) reinterpret_cast<int*>(jobs)[w] = reinterpret_cast<const int*>(js.js)[w];
+    for (int w = tid; w < total * JW; w += RT_PICK) reinterpret_cast<int*>(jobs)[w] = reinterpret_cast<const int*>(js.js)[w];
 }
 
-// Routing for prompt-sized row counts: the logits of any number of rows, then the top K of every row by one warp each.
-// A block stages eight window rows once (normed, as k_router does) and its sixteen warps walk the expert rows, four per warp at
-// a time: a warp keeps a 512-column piece of its four weight rows in registers, so every 16-byte read of a staged row feeds
-// sixteen multiply-adds, and carries its 4 x 8 sums in registers across the row's pieces; nothing in the walk is block-wide,
-// so the warps hide one another's weight loads.  f32 throughout; the sums' order differs from k_router's, the values by rounding.
-constexpr int RP_WARPS = 16, RP_RPW = 4, RP_TOK = 8;
-
-__global__ void __launch_bounds__(RP_WARPS * 32) k_router_rows(const float* __restrict__ Wr, const float* __restrict__ x, const float* __restrict__ norm_w,
-                                                               float eps, int T, int E, int H, float* __restrict__ logits, unsigned* __restrict__ err) {
-    extern __shared__ __align__(16) float xs[];   // [RP_TOK][H]: x * norm_w (the row's 1 / rms is applied to the sums)
-    __shared__ float rs[RP_TOK], ssw[RP_TOK][RP_WARPS];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    constexpr int NT = RP_WARPS * 32;
-    const int t0 = blockIdx.x * RP_TOK, nt = min(RP_TOK, T - t0);
-    for (int i = tid; i < nt * (H / 4); i += NT)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(xs + (size_t) i * 4)), "l"(x + (size_t) t0 * H + (size_t) i * 4) : "memory");
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    float4 nw4[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const int c = tid * 4 + j * NT * 4;
-        nw4[j] = norm_w && c < H ? *reinterpret_cast<const float4*>(norm_w + c) : make_float4(1.f, 1.f, 1.f, 1.f);
-    }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();
-    for (int t = 0; t < nt; ++t) {
-        float ss = 0.f;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int c = tid * 4 + j * NT * 4;
-            if (c >= H) continue;
-            float4 v = *reinterpret_cast<const float4*>(xs + (size_t) t * H + c);
-            ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
-            v.x *= nw4[j].x; v.y *= nw4[j].y; v.z *= nw4[j].z; v.w *= nw4[j].w;
-            *reinterpret_cast<float4*>(xs + (size_t) t * H + c) = v;
-        }
-        ss = warp_sum(ss);
-        if (lane == 0) ssw[t][warp] = ss;
-    }
-    __syncthreads();
-    if (tid < nt) {
-        float ss = 0.f;
-        for (int wq = 0; wq < RP_WARPS; ++wq) ss += ssw[tid][wq];
-        rs[tid] = norm_w ? rsqrtf(ss / (float) H + eps) : 1.0f;
-    }
-    __syncthreads();
-    bool bad = false;
-    for (int row0 = warp * RP_RPW; row0 <= E; row0 += RP_WARPS * RP_RPW) {
-        float acc[RP_RPW][RP_TOK];
-#pragma unroll
-        for (int r = 0; r < RP_RPW; ++r)
-#pragma unroll
-            for (int t = 0; t < RP_TOK; ++t) acc[r][t] = 0.f;
-        for (int i0 = 0; i0 < H; i0 += 512) {
-            float4 w[RP_RPW][4];
-#pragma unroll
-            for (int r = 0; r < RP_RPW; ++r)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const int i = i0 + lane * 4 + j * 128;
-                    w[r][j] = row0 + r <= E && i < H ? *reinterpret_cast<const float4*>(Wr + (size_t) (row0 + r) * H + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-                }
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int i = i0 + lane * 4 + j * 128;
-                if (i >= H) continue;
-#pragma unroll
-                for (int t = 0; t < RP_TOK; ++t)
-                    if (t < nt) {
-                        const float4 v = *reinterpret_cast<const float4*>(xs + (size_t) t * H + i);
-#pragma unroll
-                        for (int r = 0; r < RP_RPW; ++r) {
-                            acc[r][t] = fmaf(w[r][j].x, v.x, acc[r][t]);
-                            acc[r][t] = fmaf(w[r][j].y, v.y, acc[r][t]);
-                            acc[r][t] = fmaf(w[r][j].z, v.z, acc[r][t]);
-                            acc[r][t] = fmaf(w[r][j].w, v.w, acc[r][t]);
-                        }
-                    }
-            }
-        }
-#pragma unroll
-        for (int r = 0; r < RP_RPW; ++r)
-#pragma unroll
-            for (int t = 0; t < RP_TOK; ++t)
-                if (t < nt && row0 + r <= E) {
-                    const float s = warp_sum(acc[r][t]) * rs[t];
-                    if (lane == 0) {
-                        logits[(size_t) (t0 + t) * (E + 1) + row0 + r] = s;
-                        bad |= !isfinite(s);
-                    }
-                }
-    }
-    if (bad) atomicOr(err, (unsigned) FNX_ERR_NONFINITE);
+int router_window(const float* Wr, const float* x, const float* norm_w, float eps, int T, int E, int H, int K, int e_lo, int e_hi, int add_shared, float* logits, int* topi,
+                  float* topw, fnx_job* jobs, int* njobs, unsigned long long* stats, unsigned* err, uint8_t* img, bool early, cudaStream_t st) {
+    FNX_TRY(router_logits(Wr, x, norm_w, eps, T, E, H, logits, err, img, early, st));
+    const size_t smem = ((size_t) T * K + (T + FNX_JOB_TOK - 1) / FNX_JOB_TOK) * sizeof(fnx_job);
+    if (int rc = set_smem_limit((const void*) k_router_pick, 64 * 1024)) return rc;
+    const cudaError_t le = launch_dep(true, k_router_pick, dim3(1), dim3(RT_PICK), smem, st, (const float*) logits, T, E, K, e_lo, e_hi, add_shared, topi, topw, jobs, njobs, stats);
+    return le == cudaSuccess ? FNX_OK : fail(FNX_E_CUDA, "k_router_pick: launch failed: %s", cudaGetErrorString(le));
 }
 
 // one warp per row: the top K of its E logits and their renormalised softmax weights
 __global__ void __launch_bounds__(256) k_topk_rows(const float* __restrict__ logits, int T, int E, int K, int* __restrict__ topi, float* __restrict__ topw) {
-    const int t = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    __shared__ __align__(16) unsigned scr_[8][64];
+    const int warp = threadIdx.x >> 5, t = blockIdx.x * 8 + warp, lane = threadIdx.x & 31;
     if (t >= T) return;
-    const volatile float* l = logits + (size_t) t * (E + 1);
-    if (E <= 512) rt_topk_row<16>(l, E, K, lane, topi + (size_t) t * K, nullptr, topw + (size_t) t * K, nullptr);
-    else rt_topk_row<RT_MAXE / 32>(l, E, K, lane, topi + (size_t) t * K, nullptr, topw + (size_t) t * K, nullptr);
+    const float* l = logits + (size_t) t * (E + 1);
+    if (E <= 512) rt_topk_row<16>(l, E, K, lane, scr_[warp], topi + (size_t) t * K, nullptr, topw + (size_t) t * K, nullptr);
+    else rt_topk_row<RT_MAXE / 32>(l, E, K, lane, scr_[warp], topi + (size_t) t * K, nullptr, topw + (size_t) t * K, nullptr);
 }
 
 __global__ void k_combine(const float* __restrict__ part, const int* __restrict__ topi, const float* __restrict__ topw,
@@ -446,17 +404,8 @@ extern "C" int fnx_router_route(const float* Wr, const float* x, const float* no
     FNX_REQUIRE(E >= K && E <= RT_MAXE && K >= 1 && K <= 32, "fnx_router_route: %d experts, top %d not supported", E, K);
     FNX_REQUIRE(H % 256 == 0 && H <= 4096, "fnx_router_route: hidden %d not supported", H);
     FNX_REQUIRE(0 <= e_lo && e_lo <= e_hi && e_hi <= E, "fnx_router_route: expert range [%d, %d) outside [0, %d)", e_lo, e_hi, E);
-    const size_t jobs_cap = (size_t) T * K + (T + FNX_JOB_TOK - 1) / FNX_JOB_TOK;
-    const size_t smem = std::max((size_t) RT_TOK * H * sizeof(float), jobs_cap * sizeof(fnx_job));
-    if (int rc = set_smem_limit((const void*) k_router, 160 * 1024)) return rc;
-    const int blocks = (E + 1 + RT_ROWS - 1) / RT_ROWS;
-    {
-        const cudaError_t le_ = launch_k(k_router, dim3(blocks), dim3(RT_WARPS * 32), smem, as_stream(st), Wr, x, norm_w, eps, T, E, H, K, e_lo, e_hi, add_shared, logits, topi, topw, jobs,
-                                                            njobs, stats, err);
-        if (le_ != cudaSuccess) return fail(FNX_E_CUDA, "k_router: launch failed: %s", cudaGetErrorString(le_));
-    }
-    FNX_LAUNCH_OK("fnx_router_route");
-    return FNX_OK;
+    FNX_REQUIRE(((uintptr_t) x & 15) == 0 && ((uintptr_t) Wr & 15) == 0 && ((uintptr_t) norm_w & 15) == 0, "fnx_router_route: 16-byte alignment");
+    return router_window(Wr, x, norm_w, eps, T, E, H, K, e_lo, e_hi, add_shared, logits, topi, topw, jobs, njobs, stats, err, nullptr, false, as_stream(st));
 }
 
 extern "C" int fnx_moe_combine(const float* part, const int* topi, const float* topw, const float* logits, int T, int E, int H, int K,
@@ -581,10 +530,7 @@ extern "C" int fnx_router_rows(const float* Wr, const float* x, const float* nor
         FNX_LAUNCH_OK("k_router_split_w");
         if (int rc = gemm_tma_launch(wh, wl, xh, xl, logits, E + 1, T, E, H, 0, 1.0f / 256.0f, err, as_stream(st))) return rc;
     } else {
-        const size_t smem = (size_t) RP_TOK * H * sizeof(float);
-        if (int rc = set_smem_limit((const void*) k_router_rows, 160 * 1024)) return rc;
-        k_router_rows<<<(T + RP_TOK - 1) / RP_TOK, RP_WARPS * 32, smem, as_stream(st)>>>(Wr, x, norm_w, eps, T, E, H, logits, err);
-        FNX_LAUNCH_OK("k_router_rows");
+        FNX_TRY(router_logits(Wr, x, norm_w, eps, T, E, H, logits, err, nullptr, false, as_stream(st)));
     }
     k_topk_rows<<<(T + 7) / 8, 256, 0, as_stream(st)>>>(logits, T, E, K, topi, topw);
     FNX_LAUNCH_OK("k_topk_rows");
