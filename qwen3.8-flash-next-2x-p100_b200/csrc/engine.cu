@@ -15,6 +15,7 @@
 #include <string>
 #include <vector>
 
+#include "attn_win.h"
 #include "engine_mat.h"
 #include "fnx_common.cuh"
 #include "gdn_core.h"
@@ -747,10 +748,12 @@ static int enqueue_attention(fnx_engine* e, const LayerW& L, float* R, int T, in
     float* qg = e->proj;
     float* k = e->proj + d.q_rows;
     float* v = k + d.kv_rows;
-    FNX_TRY(fnx_attn_prep_append(qg, e->proj_ld, k, e->proj_ld, v, e->proj_ld, L.qn, L.kn, kc, vc, T, d.nq, d.nkv, d.hd, d.nrot, d_pos, d_depth,
-                                 e->c.eps, e->c.rope_base, e->st));
-    FNX_TRY(fnx_attn(qg, e->proj_ld, kc, vc, e->mix, T, d.nq, d.nkv, d.hd, d_pos, d_parent, e->att_scratch, e->st));
-    return enqueue_dense(e, L.w_out, e->mix, d.nq * d.hd, T, nullptr, R, d.H, 1, e->img_m);
+    FNX_TRY(attn_prep(AttnPrep{qg, e->proj_ld, k, e->proj_ld, v, e->proj_ld, L.qn, L.kn, kc, vc, 0, d.nq, d.nkv, d.hd, d.nrot, d_pos, d_depth, nullptr, nullptr, e->c.eps,
+                               e->c.rope_base},
+                      T, 1, true, e->st));
+    FNX_TRY(attn_window(AttnWin{qg, e->proj_ld, kc, vc, 0, T, d.nq, d.nkv, d.hd, d_pos, d_parent, nullptr, nullptr, 0, e->err}, e->att_scratch, e->mix,
+                        L.w_out.nat ? e->img_m : nullptr, true, e->st));
+    return enqueue_dense(e, L.w_out, e->mix, d.nq * d.hd, T, nullptr, R, d.H, 1, e->img_m, L.w_out.nat);
 }
 
 static int enqueue_gdn(fnx_engine* e, const LayerW& L, float* R, int T, int seq, const int* d_parent, bool img = false) {
@@ -898,11 +901,14 @@ static int enqueue_mixer_lanes(fnx_engine* e, const LayerW& L, float* R, int T, 
         float* qg = e->proj;
         float* k = e->proj + d.q_rows;
         float* v = k + d.kv_rows;
-        FNX_TRY(fnx_attn_prep_append_lanes(qg, e->proj_ld, k, e->proj_ld, v, e->proj_ld, L.qn, L.kn, L.kc, L.vc, (size_t) e->cache_rows, n_lanes, max_lane_rows, d.nq,
-                                           d.nkv, d.hd, d.nrot, d_pos, lanes, d_row0, e->c.eps, e->c.rope_base, e->st));
-        FNX_TRY(fnx_attn_lanes(qg, e->proj_ld, L.kc, L.vc, (size_t) e->cache_rows, e->mix, T, n_lanes, d.nq, d.nkv, d.hd, d_pos, lanes, d_row0, e->att_scratch, e->st));
+        const bool mi = L.w_out.nat && !dp;
+        FNX_TRY(attn_prep(AttnPrep{qg, e->proj_ld, k, e->proj_ld, v, e->proj_ld, L.qn, L.kn, L.kc, L.vc, (size_t) e->cache_rows, d.nq, d.nkv, d.hd, d.nrot, d_pos, nullptr,
+                                   lanes, d_row0, e->c.eps, e->c.rope_base},
+                          max_lane_rows, n_lanes, true, e->st));
+        FNX_TRY(attn_window(AttnWin{qg, e->proj_ld, L.kc, L.vc, (size_t) e->cache_rows, T, d.nq, d.nkv, d.hd, d_pos, nullptr, lanes, d_row0, n_lanes, e->err}, e->att_scratch, e->mix,
+                            mi ? e->img_m : nullptr, true, e->st));
         if (dp) FNX_TRY(enqueue_dp_gather(e, d.nq * d.hd, n_lanes, d_row0));
-        return enqueue_dense(e, L.w_out, e->mix, d.nq * d.hd, T, nullptr, R, d.H, 1, e->img_m);
+        return enqueue_dense(e, L.w_out, e->mix, d.nq * d.hd, T, nullptr, R, d.H, 1, e->img_m, mi);
     }
     const bool mi = L.w_out.nat && d.nv % 2 == 0 && !dp;
     FNX_TRY(gdn_window_lanes(GdnArgs{e->proj, e->proj_ld, e->proj + d.gdn_ch + d.nv * d.hs, e->proj_ld, L.hist_pool, L.convw, L.dt, L.a, L.gnorm, L.S_pool, e->NS, nullptr, e->mix,
