@@ -68,6 +68,17 @@ __device__ __forceinline__ uint32_t nm_lo(uint32_t x) {
     return ((x * k) & 0xF0F0F0F0u) | 0x08080808u;
 }
 
+// Weights pass through L2 once a window and are the first to leave it: what they would push out (the kernels' own code, fetched from
+// DRAM again at every launch, the router's weights, activations) is read again a layer later.
+__device__ __forceinline__ uint64_t nm_stream_policy() {
+    uint64_t p;
+    asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+    return p;
+}
+__device__ __forceinline__ void nm_cp_stream(uint32_t dst, const void* src, uint64_t policy) {
+    asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "l"(policy) : "memory");
+}
+
 // the two rows' eight sub-block scales 1 + 2 s as bytes: even sub-blocks in .x, odd ones in .y
 struct NmScales {
     uint2 r0, r1;
@@ -250,6 +261,7 @@ __device__ __forceinline__ void nm_body(const NatParams& p, uint8_t* smem) {
     const int pool_rows = MOE ? p.rmax : 4 * NG;
     fnx_job* jobs_s = reinterpret_cast<fnx_job*>(pool + (size_t) pool_rows * RS);
     float* ub = reinterpret_cast<float*>(pool + (size_t) pool_rows * RS);                    // C > 1: the units' partial sums
+    const uint64_t policy = nm_stream_policy();
     const uint32_t slots_s = smem_u32(smem) + (uint32_t) warp * (SLOTS * NAT_TILE_BYTES), pool_s = smem_u32(pool);
     // gate|up: the job list is the previous kernel's; down: it is older than the kernel whose rows this one waits for, and that
     // kernel lets dependents start only once it has itself waited for the list
@@ -309,9 +321,9 @@ __device__ __forceinline__ void nm_body(const NatParams& p, uint8_t* smem) {
                 for (int h = 0; h < 2; ++h) {
 #pragma unroll
                     for (int j = 0; j < 4; ++j)
-                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + h * NAT_HALF_BYTES + j * 512), "l"(asrc + h * NAT_HALF_BYTES + j * 512) : "memory");
+                        nm_cp_stream(dst + h * NAT_HALF_BYTES + j * 512, asrc + h * NAT_HALF_BYTES + j * 512, policy);
                     if (lane < 8)
-                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + h * NAT_HALF_BYTES + NAT_META), "l"(asrc + h * NAT_HALF_BYTES + NAT_META) : "memory");
+                        nm_cp_stream(dst + h * NAT_HALF_BYTES + NAT_META, asrc + h * NAT_HALF_BYTES + NAT_META, policy);
                 }
                 asrc += NAT_TILE_BYTES;
                 if (MOE || C > 1) {
