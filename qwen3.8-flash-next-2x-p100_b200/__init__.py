@@ -192,6 +192,18 @@ def _stream():
     return C.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
+# The window operators below are called once a layer: a small window's kernels take less time than a few Python calls, so these hand
+# plain addresses (which C.c_void_p arguments take) to the library and allocate no more than they return.
+def _at(t):
+    return None if t is None else t.data_ptr()
+
+
+def _raw_stream(t):
+    """The current stream's handle on the current device (as _stream(), without the Stream object)."""
+    import torch
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+
+
 # ------------------------------------------------------------------------------------------------ weights
 def iq3s_bytes(rows: int, cols: int) -> int:
     return rows * (cols // 256) * IQ3S_BLOCK
@@ -242,10 +254,15 @@ def dense(W, rows: int, cols: int, x, norm_w=None, eps: float = 1e-6, out=None, 
     """y[t] (+)= W . x[t] (x optionally RMS-normed with norm_w first): q8s_gemv / mmvq of the reference."""
     import torch
     T = x.shape[0]
-    if out is None:
-        out = torch.zeros((T, rows), dtype=torch.float32, device=x.device)
+    if out is None:   # (sums start from zeros)
+        out = (torch.zeros if accumulate else torch.empty)((T, rows), dtype=torch.float32, device=x.device)
     err = new_err(x.device) if err is None else err
-    per = lib().fnx_dense_rows(cols)
+    L = lib()
+    per = L.fnx_dense_rows(cols)
+    if T <= per:
+        check(L.fnx_dense(W.data_ptr(), rows, cols, x.data_ptr(), x.stride(0), T, _at(norm_w), eps, out.data_ptr(), out.stride(0), 1 if accumulate else 0,
+                          err.data_ptr(), _raw_stream(x)))
+        return out, err
     for t0 in range(0, T, per):
         nt = min(per, T - t0)
         check(lib().fnx_dense(ptr(W), rows, cols, ptr(x[t0:]), x.stride(0), nt, ptr(norm_w), eps, ptr(out[t0:]), out.stride(0),
@@ -276,11 +293,13 @@ def router_route(Wr, x, K: int, norm_w=None, eps: float = 1e-6, e_lo: int = 0, e
     topi = torch.empty((T, K), dtype=torch.int32, device=dev)
     topw = torch.empty((T, K), dtype=torch.float32, device=dev)
     njobs_max = T * K + (T + JOB_TOK - 1) // JOB_TOK
-    jobs = torch.zeros(njobs_max * C.sizeof(Job), dtype=torch.uint8, device=dev)
-    njobs = torch.zeros(2, dtype=torch.int32, device=dev)
-    err = new_err(dev) if err is None else err
-    check(lib().fnx_router_route(ptr(Wr), ptr(x), ptr(norm_w), eps, T, E, H, K, e_lo, e_hi, 1 if add_shared else 0, ptr(logits), ptr(topi),
-                                 ptr(topw), ptr(jobs), ptr(njobs), None, ptr(err), _stream()))
+    # the job list, its count and the error word in one zeroed allocation
+    jb = (njobs_max * C.sizeof(Job) + 15) // 16 * 4
+    words = torch.zeros(jb + 4, dtype=torch.int32, device=dev)
+    jobs, njobs, tail = words[:njobs_max * C.sizeof(Job) // 4].view(torch.uint8), words[jb:jb + 2], words[jb + 2:jb + 3]
+    err = tail if err is None else err
+    check(lib().fnx_router_route(Wr.data_ptr(), x.data_ptr(), _at(norm_w), eps, T, E, H, K, e_lo, e_hi, 1 if add_shared else 0, logits.data_ptr(), topi.data_ptr(),
+                                 topw.data_ptr(), jobs.data_ptr(), njobs.data_ptr(), None, err.data_ptr(), _raw_stream(x)))
     return dict(logits=logits, topi=topi, topw=topw, jobs=jobs, njobs=njobs, njobs_max=njobs_max, err=err)
 
 
@@ -293,16 +312,17 @@ def moe_experts(Wgu, Wdn, Wsh_gu, Wsh_dn, route, x, F: int, K: int, norm_w=None,
     e_hi = E if e_hi is None else e_hi
     P = T * K + T
     gu_stride, dn_stride = iq3s_bytes(2 * F, H), iq3s_bytes(H, F)
-    h = torch.zeros((P, F), dtype=torch.float32, device=x.device)
-    part = torch.zeros((P, H), dtype=torch.float32, device=x.device)
-    out = torch.zeros((T, H), dtype=torch.float32, device=x.device)
-    L = lib()
-    check(L.fnx_moe_gate_up(ptr(Wgu), gu_stride, e_base, ptr(Wsh_gu), E, ptr(route["jobs"]), ptr(route["njobs"]), route["njobs_max"], ptr(x),
-                            ptr(norm_w), eps, H, F, ptr(h), ptr(route["err"]), _stream()))
-    check(L.fnx_moe_down(ptr(Wdn), dn_stride, e_base, ptr(Wsh_dn), E, ptr(route["jobs"]), ptr(route["njobs"]), route["njobs_max"], ptr(h), H, F,
-                         ptr(part), ptr(route["err"]), _stream()))
-    check(L.fnx_moe_combine(ptr(part), ptr(route["topi"]), ptr(route["topw"]), ptr(route["logits"]), T, E, H, K, e_lo, e_hi,
-                            1 if add_shared else 0, ptr(out), 0, _stream()))
+    new = torch.empty if e_lo <= 0 and e_hi >= E and add_shared else torch.zeros   # (rows of experts outside the range stay zero)
+    h = new((P, F), dtype=torch.float32, device=x.device)
+    part = new((P, H), dtype=torch.float32, device=x.device)
+    out = torch.empty((T, H), dtype=torch.float32, device=x.device)
+    L, st = lib(), _raw_stream(x)
+    jobs, njobs, njobs_max, err = route["jobs"].data_ptr(), route["njobs"].data_ptr(), route["njobs_max"], route["err"].data_ptr()
+    hp, pp = h.data_ptr(), part.data_ptr()
+    check(L.fnx_moe_gate_up(Wgu.data_ptr(), gu_stride, e_base, _at(Wsh_gu), E, jobs, njobs, njobs_max, x.data_ptr(), _at(norm_w), eps, H, F, hp, err, st))
+    check(L.fnx_moe_down(Wdn.data_ptr(), dn_stride, e_base, _at(Wsh_dn), E, jobs, njobs, njobs_max, hp, H, F, pp, err, st))
+    check(L.fnx_moe_combine(pp, route["topi"].data_ptr(), route["topw"].data_ptr(), route["logits"].data_ptr(), T, E, H, K, e_lo, e_hi, 1 if add_shared else 0,
+                            out.data_ptr(), 0, st))
     return out, h, part
 
 
@@ -426,7 +446,7 @@ def attn(qg, kc, vc, pos0, parent=None, scratch=None):
     out = torch.empty((T, nq, hd), dtype=torch.float32, device=qg.device)
     if scratch is None:
         scratch = torch.empty(lib().fnx_attn_scratch_bytes(T, nq, hd), dtype=torch.uint8, device=qg.device)
-    check(lib().fnx_attn(ptr(qg), nq * hd2, ptr(kc), ptr(vc), ptr(out), T, nq, nkv, hd, ptr(pos0), ptr(parent), ptr(scratch), _stream()))
+    check(lib().fnx_attn(qg.data_ptr(), nq * hd2, kc.data_ptr(), vc.data_ptr(), out.data_ptr(), T, nq, nkv, hd, pos0.data_ptr(), _at(parent), scratch.data_ptr(), _raw_stream(qg)))
     return out
 
 
@@ -781,8 +801,16 @@ class Engine:
     def save_state(self, seq: int = 0, kv: bool = True):
         """The sequence's state as a host buffer (a ctypes array) for load_state."""
         import ctypes as C
+        import mmap
         n = lib().fnx_engine_state_bytes(self._h, seq, 1 if kv else 0)
-        buf = (C.c_uint8 * n)()
+        # (fresh pages, large where the system gives them: a ctypes array of its own would be cleared first, page by page)
+        m = mmap.mmap(-1, n, flags=mmap.MAP_PRIVATE | mmap.MAP_ANONYMOUS)
+        if hasattr(mmap, "MADV_HUGEPAGE"):
+            try:
+                m.madvise(mmap.MADV_HUGEPAGE)
+            except OSError:
+                pass
+        buf = (C.c_uint8 * n).from_buffer(m)
         check(lib().fnx_engine_save_state(self._h, seq, 1 if kv else 0, buf, n))
         return buf
 

@@ -1,7 +1,6 @@
 // Host-side plumbing shared by every entry point: the per-thread error text and device facts.
 #include "fnx_common.cuh"
 
-#include <cstdlib>
 #include <cstring>
 #include <mutex>
 #include <set>
@@ -36,26 +35,24 @@ int sm_count() {
     return n[dev];
 }
 
-// cudaFuncAttributeMaxDynamicSharedMemorySize is a per-device attribute of a kernel: set once per (device, kernel)
+// cudaFuncAttributeMaxDynamicSharedMemorySize is a per-device attribute of a kernel: set once per (device, kernel).  A thread remembers
+// the last pairs it has seen done, so that a launch usually takes no lock.
 int set_smem_limit(const void* kernel, int bytes) {
     static std::mutex mu;
     static std::set<std::pair<int, const void*>> done;
+    constexpr size_t SEEN = 64;
+    static thread_local std::pair<int, const void*> seen[SEEN];   // (empty: a null kernel)
     int dev = 0;
     FNX_CUDA_OK(cudaGetDevice(&dev));
+    auto& mine = seen[((uintptr_t) kernel >> 4) % SEEN];
+    if (mine.second == kernel && mine.first == dev) return FNX_OK;
     std::lock_guard<std::mutex> lock(mu);
-    if (done.count({dev, kernel})) return FNX_OK;
-    FNX_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-    done.insert({dev, kernel});
-    return FNX_OK;
-}
-
-bool pdl_enabled() {
-    static int on = -1;
-    if (on < 0) {
-        const char* v = getenv("FNX_PDL");
-        on = v && v[0] == '1';
+    if (!done.count({dev, kernel})) {
+        FNX_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+        done.insert({dev, kernel});
     }
-    return on != 0;
+    mine = {dev, kernel};
+    return FNX_OK;
 }
 
 }  // namespace fnxb

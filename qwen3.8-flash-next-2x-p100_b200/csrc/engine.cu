@@ -9,10 +9,13 @@
 #include <cuda_runtime.h>
 #include <dlfcn.h>
 
+#include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <cmath>
 #include <map>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "attn_win.h"
@@ -101,6 +104,12 @@ struct fnx_engine {
     float last_ms = 0.f;
     size_t bytes = 0;
     std::vector<void*> owned;
+    struct Stage {   // one thread's pinned slots for parking and resuming sequences (copy_pieces)
+        cudaStream_t st = nullptr;
+        char* slot[2] = {nullptr, nullptr};
+        cudaEvent_t done[2] = {nullptr, nullptr};
+    };
+    std::vector<Stage> stage;
     std::map<std::string, std::pair<void*, size_t>> tensors;
     std::vector<LayerW> layers;
     LayerW mtp;
@@ -259,6 +268,8 @@ __global__ void k_gdn_params(float* dt, float* a, int nv) {
 }
 // dst[j] = src[idx[j]] rows of n floats
 __global__ void k_gather_rows(float* __restrict__ dst, const float* __restrict__ src, const int* __restrict__ idx, int n) {
+    pdl_wait();
+    pdl_launch_dependents();
     const int j = blockIdx.y, i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) dst[(size_t) j * n + i] = src[(size_t) idx[j] * n + i];
 }
@@ -344,6 +355,8 @@ __global__ void k_ep_recv(const float* __restrict__ xbuf, const unsigned* __rest
 __global__ void k_plus_one(int* dst, const int* src) { *dst = *src + 1; }
 // depth of every window row from the parent array (parent null: a chain)
 __global__ void k_depths(const int* __restrict__ parent, int* __restrict__ depth, int T) {
+    pdl_wait();
+    pdl_launch_dependents();
     const int t = threadIdx.x;
     if (t >= T) return;
     int d = 0;
@@ -380,7 +393,11 @@ __global__ void k_commit(__half* const* __restrict__ kcs, __half* const* __restr
         *cur = (*cur + 1 + path[n - 1]) % NS;
     }
 }
-__global__ void k_advance_pos(int* pos, int n) { *pos += n; }
+__global__ void k_advance_pos(int* pos, int n) {
+    pdl_wait();
+    pdl_launch_dependents();
+    *pos += n;
+}
 // the prompt pass: the chunk's tokens joining the context; position and state slot afterwards
 __global__ void k_prompt_context(int* ctx, const int* ctx_n, const int* tok, int n) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -772,7 +789,7 @@ static int enqueue_gdn(fnx_engine* e, const LayerW& L, float* R, int T, int seq,
 static int enqueue_verify(fnx_engine* e, int seq, int T, bool tree) {
     const Dims d = dims(e->c);
     const int* par = tree ? e->d_parent : nullptr;
-    k_depths<<<1, 32, 0, e->st>>>(par, e->d_depth, T);
+    launch_dep(true, k_depths, 1, 32, 0, e->st, par, e->d_depth, T);
     FNX_LAUNCH_OK("depths");
     bool img = e->layers[0].w_in.nat != nullptr;   // the rows' image for the next projection is ready (left by whatever completed the rows)
     FNX_TRY(nat_embed_image(e->embed, e->d_tok, T, d.H, e->R, e->layers[0].norm1, img ? e->img_r : nullptr, e->st));
@@ -847,6 +864,8 @@ __global__ void k_commit_lanes(const int* __restrict__ lane_seq, const int* __re
 // the draft layer's first call: its rows are the lanes' kept rows (source rows and the tokens they emitted)
 __global__ void k_mtp_gather_lanes(float* __restrict__ dst, const float* __restrict__ src, int* __restrict__ mtok, const int* __restrict__ results,
                                    const int* __restrict__ row0v, const int* __restrict__ row0m, int L, int H) {
+    pdl_wait();
+    pdl_launch_dependents();
     const int r = blockIdx.y;   // draft-layer row
     int lane = 0;
     while (lane + 1 < L && r >= row0m[lane + 1]) ++lane;
@@ -858,19 +877,27 @@ __global__ void k_mtp_gather_lanes(float* __restrict__ dst, const float* __restr
 }
 // dst[lane] = src[last row of lane]
 __global__ void k_last_rows(float* __restrict__ dst, const float* __restrict__ src, const int* __restrict__ row0, int H) {
+    pdl_wait();
+    pdl_launch_dependents();
     const int lane = blockIdx.y, i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < H) dst[(size_t) lane * H + i] = src[(size_t) (row0[lane + 1] - 1) * H + i];
 }
 // the draft layer's positions advance per lane: by the rows of its first call, then by one
 __global__ void k_mtp_advance_lanes(int* __restrict__ mpos, const int* __restrict__ lane_seq, const int* __restrict__ row0m, int L, int first) {
+    pdl_wait();
+    pdl_launch_dependents();
     const int lane = threadIdx.x;
     if (lane < L) mpos[lane_seq[lane]] += first ? row0m[lane + 1] - row0m[lane] : 1;
 }
 __global__ void k_mtp_set_pos_lanes(int* __restrict__ mpos, const int* __restrict__ lane_seq, const int* __restrict__ base, int L) {
+    pdl_wait();
+    pdl_launch_dependents();
     const int lane = threadIdx.x;
     if (lane < L) mpos[lane_seq[lane]] = base[lane];
 }
 __global__ void k_scatter_drafts(int* __restrict__ out, const int* __restrict__ best, int L, int k, int j) {
+    pdl_wait();
+    pdl_launch_dependents();
     const int lane = threadIdx.x;
     if (lane < L) out[lane * k + j] = best[lane];
 }
@@ -945,7 +972,7 @@ static int enqueue_mtp_lanes(fnx_engine* e, int n_lanes, int Tm, int max_rows, c
     FNX_TRY(enqueue_mtp_input(e, Tm, src));
     FNX_TRY(enqueue_mixer_lanes(e, e->mtp, e->Rm, Tm, n_lanes, max_rows, e->d_lane_seq, d_row0, e->d_mpos_seq));
     FNX_TRY(enqueue_moe(e, e->mtp, e->Rm, Tm));
-    k_last_rows<<<dim3((d.H + 255) / 256, n_lanes), 256, 0, e->st>>>(e->Rlast, e->Rm, d_row0, d.H);
+    launch_dep(true, k_last_rows, dim3((d.H + 255) / 256, n_lanes), 256, 0, e->st, e->Rlast, e->Rm, d_row0, d.H);
     FNX_LAUNCH_OK("draft last rows");
     FNX_TRY(enqueue_dense(e, e->mtp_head.rows ? e->mtp_head : e->head, e->Rlast, d.H, n_lanes, e->mtp_onorm, e->logits, e->dvn, 0, e->img_r));
     return fnx_argmax_mapped(e->logits, n_lanes, e->dvn, e->d_dvocab, e->best_i, nullptr, e->err, e->st);
@@ -999,7 +1026,7 @@ extern "C" int fnx_commit(void* const* k_caches, void* const* v_caches, int n_at
     k_commit<<<n_attn_layers + 1, 256, 0, as_stream(st)>>>((__half* const*) k_caches, (__half* const*) v_caches, n_attn_layers, row_halves, path, nullptr, nullptr, n,
                                                              pos0, cur, NS, nullptr, nullptr);
     FNX_LAUNCH_OK("fnx_commit");
-    k_advance_pos<<<1, 1, 0, as_stream(st)>>>(pos0, n);
+    launch_dep(true, k_advance_pos, 1, 1, 0, as_stream(st), pos0, n);
     FNX_LAUNCH_OK("fnx_commit (position)");
     return FNX_OK;
 }
@@ -1126,6 +1153,15 @@ extern "C" int fnx_engine_create(const fnx_model_config* cfg, fnx_engine** out) 
     return FNX_OK;
 }
 
+static void stage_free(fnx_engine::Stage& g) {
+    if (g.st) cudaStreamDestroy(g.st);
+    for (int k = 0; k < 2; ++k) {
+        if (g.slot[k]) cudaFreeHost(g.slot[k]);
+        if (g.done[k]) cudaEventDestroy(g.done[k]);
+    }
+    g = fnx_engine::Stage{};
+}
+
 extern "C" void fnx_engine_destroy(fnx_engine* e) {
     if (!e) return;
     if (e->st) cudaStreamSynchronize(e->st);
@@ -1136,6 +1172,7 @@ extern "C" void fnx_engine_destroy(fnx_engine* e) {
     if (e->d_bias_tok) cudaFree(e->d_bias_tok);
     if (e->d_bias_val) cudaFree(e->d_bias_val);
     if (e->h_stage) cudaFreeHost(e->h_stage);
+    for (auto& g : e->stage) stage_free(g);
     if (e->ev0) cudaEventDestroy(e->ev0);
     if (e->ev1) cudaEventDestroy(e->ev1);
     if (e->st) cudaStreamDestroy(e->st);
@@ -1535,7 +1572,7 @@ extern "C" int fnx_engine_commit(fnx_engine* e, int seq, const int* h_path, int 
     k_commit<<<nattn + 1, 256, 0, e->st>>>(tables[key].first, tables[key].second, nattn, d.kv_rows, e->d_path, e->d_tok, e->result + 1 + FNX_MAX_ROWS, n,
                                            e->d_pos + seq, e->d_cur + seq, e->NS, e->d_ctx + (size_t) seq * e->cache_rows, e->d_ctx_n + seq);
     FNX_LAUNCH_OK("commit");
-    k_advance_pos<<<1, 1, 0, e->st>>>(e->d_pos + seq, n);
+    launch_dep(true, k_advance_pos, 1, 1, 0, e->st, e->d_pos + seq, n);
     FNX_LAUNCH_OK("commit (position)");
     s.kept = n;
     s.kept_pos0 = s.pos;
@@ -1566,7 +1603,7 @@ extern "C" int fnx_engine_draft(fnx_engine* e, int seq, int k, int* h_drafts) {
     auto chain = [&]() -> int {
         // (the chain advances the position as it goes: it starts from a copy, so that running it again gives the same result)
         FNX_CUDA_OK(cudaMemcpyAsync(e->d_mpos, e->d_mpos_base, sizeof(int), cudaMemcpyDeviceToDevice, e->st));
-        k_gather_rows<<<dim3((d.H + 255) / 256, n), 256, 0, e->st>>>(e->Rsrc, e->R, e->d_path, d.H);
+        launch_dep(true, k_gather_rows, dim3((d.H + 255) / 256, n), 256, 0, e->st, e->Rsrc, e->R, e->d_path, d.H);
         FNX_LAUNCH_OK("draft gather");
         FNX_CUDA_OK(cudaMemcpyAsync(e->d_mtok, e->result + 1 + FNX_MAX_ROWS, sizeof(int) * n, cudaMemcpyDeviceToDevice, e->st));
         FNX_TRY(mtp_call(n, e->d_drafts));
@@ -1574,7 +1611,7 @@ extern "C" int fnx_engine_draft(fnx_engine* e, int seq, int k, int* h_drafts) {
             const int src_row = j == 1 ? n - 1 : 0;
             FNX_CUDA_OK(cudaMemcpyAsync(e->Rsrc, e->Rm + (size_t) src_row * d.H, sizeof(float) * d.H, cudaMemcpyDeviceToDevice, e->st));
             FNX_CUDA_OK(cudaMemcpyAsync(e->d_mtok, e->d_drafts + (j - 1), sizeof(int), cudaMemcpyDeviceToDevice, e->st));
-            k_advance_pos<<<1, 1, 0, e->st>>>(e->d_mpos, j == 1 ? n : 1);
+            launch_dep(true, k_advance_pos, 1, 1, 0, e->st, e->d_mpos, j == 1 ? n : 1);
             FNX_LAUNCH_OK("draft position");
             FNX_TRY(mtp_call(1, e->d_drafts + j));
         }
@@ -1800,21 +1837,21 @@ extern "C" int fnx_engine_draft_lanes(fnx_engine* e, int n_lanes, const int* h_s
     // one graph for the whole chain: the first call on every lane's kept rows, then k - 1 calls of one row per lane
     auto chain = [&]() -> int {
         // (the chain advances the lanes' positions as it goes: it starts from a copy, so that running it again gives the same result)
-        k_mtp_set_pos_lanes<<<1, 32, 0, e->st>>>(e->d_mpos_seq, e->d_lane_seq, e->d_mpos_base, n_lanes);
+        launch_dep(true, k_mtp_set_pos_lanes, 1, 32, 0, e->st, e->d_mpos_seq, e->d_lane_seq, e->d_mpos_base, n_lanes);
         FNX_LAUNCH_OK("draft positions (lanes)");
-        k_mtp_gather_lanes<<<dim3((d.H + 255) / 256, Tm), 256, 0, e->st>>>(e->Rsrc, e->R, e->d_mtok, e->d_results, e->d_lane_row0, e->d_mlane_row0, n_lanes, d.H);
+        launch_dep(true, k_mtp_gather_lanes, dim3((d.H + 255) / 256, Tm), 256, 0, e->st, e->Rsrc, e->R, e->d_mtok, e->d_results, e->d_lane_row0, e->d_mlane_row0, n_lanes, d.H);
         FNX_LAUNCH_OK("draft gather (lanes)");
         FNX_TRY(enqueue_mtp_lanes(e, n_lanes, Tm, maxn, e->d_mlane_row0, e->Rsrc));
-        k_scatter_drafts<<<1, 32, 0, e->st>>>(e->d_ldrafts, e->best_i, n_lanes, k, 0);
+        launch_dep(true, k_scatter_drafts, 1, 32, 0, e->st, e->d_ldrafts, e->best_i, n_lanes, k, 0);
         FNX_LAUNCH_OK("draft scatter");
         for (int j = 1; j < k; ++j) {
             // each lane's source row: its draft-layer last row (compact in Rlast), its token: the previous draft
             FNX_CUDA_OK(cudaMemcpyAsync(e->Rsrc, e->Rlast, sizeof(float) * (size_t) n_lanes * d.H, cudaMemcpyDeviceToDevice, e->st));
             FNX_CUDA_OK(cudaMemcpyAsync(e->d_mtok, e->best_i, sizeof(int) * n_lanes, cudaMemcpyDeviceToDevice, e->st));
-            k_mtp_advance_lanes<<<1, 32, 0, e->st>>>(e->d_mpos_seq, e->d_lane_seq, e->d_mlane_row0, n_lanes, j == 1 ? 1 : 0);
+            launch_dep(true, k_mtp_advance_lanes, 1, 32, 0, e->st, e->d_mpos_seq, e->d_lane_seq, e->d_mlane_row0, n_lanes, j == 1 ? 1 : 0);
             FNX_LAUNCH_OK("draft positions (lanes)");
             FNX_TRY(enqueue_mtp_lanes(e, n_lanes, n_lanes, 1, e->d_ident_row0, e->Rsrc));
-            k_scatter_drafts<<<1, 32, 0, e->st>>>(e->d_ldrafts, e->best_i, n_lanes, k, j);
+            launch_dep(true, k_scatter_drafts, 1, 32, 0, e->st, e->d_ldrafts, e->best_i, n_lanes, k, j);
             FNX_LAUNCH_OK("draft scatter");
         }
         return FNX_OK;
@@ -1878,6 +1915,102 @@ static std::vector<std::pair<char*, size_t>> state_pieces(fnx_engine* e, int seq
     layer(e->mtp);
     return v;
 }
+// Between the pieces and their places in the caller's image, in either direction.  Memory that the caller pinned is the copy engine's
+// own business.  Pageable memory goes through pinned slots, a few threads at once, each with two slots of its own (the copy engine
+// fills or drains one while the thread moves the other): the runtime's own staging moved 53 MB each way at 6 GB/s, one thread copying
+// and taking the page faults of fresh memory.  The slots live as long as the engine.
+constexpr size_t STAGE_BYTES = 1 << 20;
+constexpr int STAGE_MAX = 8;   // threads
+struct StageChunk {
+    char *dev, *host;
+    size_t bytes;
+};
+static int stage_worker(fnx_engine* e, int w, int device, const std::vector<StageChunk>& list, std::atomic<size_t>& next, bool to_host) {
+    FNX_CUDA_OK(cudaSetDevice(device));
+    fnx_engine::Stage& g = e->stage[w];
+    StageChunk held[2] = {};
+    int rc = FNX_OK;
+    auto settle = [&](int k) -> int {   // slot k's copy is done (and, coming from the device, in the caller's memory)
+        if (!held[k].bytes) return FNX_OK;
+        FNX_CUDA_OK(cudaEventSynchronize(g.done[k]));
+        if (to_host) memcpy(held[k].host, g.slot[k], held[k].bytes);
+        held[k].bytes = 0;
+        return FNX_OK;
+    };
+    auto start = [&](int k, const StageChunk& c) -> int {
+        if (to_host) FNX_CUDA_OK(cudaMemcpyAsync(g.slot[k], c.dev, c.bytes, cudaMemcpyDeviceToHost, g.st));
+        else {
+            memcpy(g.slot[k], c.host, c.bytes);
+            FNX_CUDA_OK(cudaMemcpyAsync(c.dev, g.slot[k], c.bytes, cudaMemcpyHostToDevice, g.st));
+        }
+        FNX_CUDA_OK(cudaEventRecord(g.done[k], g.st));
+        held[k] = c;
+        return FNX_OK;
+    };
+    int k = 0;
+    for (size_t i; rc == FNX_OK && (i = next++) < list.size(); k ^= 1) {
+        rc = settle(k);
+        if (rc == FNX_OK) rc = start(k, list[i]);
+    }
+    for (int j = 0; j < 2; ++j) {
+        const int rc2 = settle(k ^ j);
+        if (rc == FNX_OK) rc = rc2;
+    }
+    return rc;
+}
+static bool stage_ready(fnx_engine* e) {
+    if (!e->stage.empty()) return true;
+    const int n = (int) std::min(std::max(std::thread::hardware_concurrency(), 1u), (unsigned) STAGE_MAX);
+    std::vector<fnx_engine::Stage> v(n);
+    bool ok = true;
+    for (auto& g : v) {
+        ok = ok && cudaStreamCreateWithFlags(&g.st, cudaStreamNonBlocking) == cudaSuccess;
+        for (int k = 0; k < 2; ++k)
+            ok = ok && cudaHostAlloc(&g.slot[k], STAGE_BYTES, cudaHostAllocDefault) == cudaSuccess &&
+                 cudaEventCreateWithFlags(&g.done[k], cudaEventDisableTiming) == cudaSuccess;
+    }
+    if (!ok) {   // (no pinned memory to be had: the runtime's staging)
+        cudaGetLastError();
+        for (auto& g : v) stage_free(g);
+        return false;
+    }
+    e->stage.swap(v);
+    return true;
+}
+static int copy_pieces(fnx_engine* e, const std::vector<std::pair<char*, size_t>>& pieces, char* host, bool to_host) {
+    cudaPointerAttributes at{};
+    const bool pinned = cudaPointerGetAttributes(&at, host) == cudaSuccess && at.type == cudaMemoryTypeHost;
+    cudaGetLastError();
+    if (pinned || !stage_ready(e)) {
+        for (const auto& p : pieces) {
+            FNX_CUDA_OK(to_host ? cudaMemcpyAsync(host, p.first, p.second, cudaMemcpyDeviceToHost, e->st) : cudaMemcpyAsync(p.first, host, p.second, cudaMemcpyHostToDevice, e->st));
+            host += (p.second + 15) & ~(size_t) 15;
+        }
+        return FNX_OK;
+    }
+    std::vector<StageChunk> list;
+    for (const auto& p : pieces) {
+        for (size_t o = 0; o < p.second; o += STAGE_BYTES) list.push_back({p.first + o, host + o, std::min(STAGE_BYTES, p.second - o)});
+        host += (p.second + 15) & ~(size_t) 15;
+    }
+    int device = 0;
+    FNX_CUDA_OK(cudaGetDevice(&device));
+    std::atomic<size_t> next{0};
+    const int n = (int) std::min(e->stage.size(), list.size());
+    std::vector<int> rcs(n, FNX_OK);
+    std::vector<std::string> why(n);
+    std::vector<std::thread> threads;
+    for (int w = 1; w < n; ++w)
+        threads.emplace_back([&, w]() {
+            rcs[w] = stage_worker(e, w, device, list, next, to_host);
+            if (rcs[w] != FNX_OK) why[w] = error_buf();
+        });
+    if (n > 0) rcs[0] = stage_worker(e, 0, device, list, next, to_host);
+    for (auto& t : threads) t.join();
+    for (int w = 0; w < n; ++w)
+        if (rcs[w] != FNX_OK) return w ? fail(rcs[w], "%s", why[w].c_str()) : rcs[w];
+    return FNX_OK;
+}
 }  // namespace fnxb
 
 extern "C" size_t fnx_engine_state_bytes(fnx_engine* e, int seq, int kv) {
@@ -1898,12 +2031,8 @@ extern "C" int fnx_engine_save_state(fnx_engine* e, int seq, int kv, void* host,
     h.magic = STATE_MAGIC; h.kv = kv != 0; h.pos = s.pos; h.n_layer = e->c.n_layer; h.hidden = d.H; h.nv = d.nv; h.hs = d.hs; h.gdn_ch = d.gdn_ch;
     h.kv_rows = d.kv_rows; h.has_mtp = 1; h.step = s.step; h.bytes = need;
     memcpy(host, &h, sizeof h);
-    char* dst = (char*) host + sizeof h;
     FNX_CUDA_OK(cudaStreamSynchronize(e->st));
-    for (const auto& p : state_pieces(e, seq, s.pos, s.cur, kv != 0)) {
-        FNX_CUDA_OK(cudaMemcpyAsync(dst, p.first, p.second, cudaMemcpyDeviceToHost, e->st));
-        dst += (p.second + 15) & ~(size_t) 15;
-    }
+    FNX_TRY(copy_pieces(e, state_pieces(e, seq, s.pos, s.cur, kv != 0), (char*) host + sizeof h, true));
     FNX_CUDA_OK(cudaStreamSynchronize(e->st));
     return FNX_OK;
 }
@@ -1934,10 +2063,7 @@ extern "C" int fnx_engine_load_state(fnx_engine* e, int seq, const void* host, s
     size_t total = sizeof h;
     for (const auto& p : pieces) total += (p.second + 15) & ~(size_t) 15;
     FNX_REQUIRE(total == h.bytes, "fnx_engine_load_state: a state saved with another layout (%zu bytes against %llu)", total, (unsigned long long) h.bytes);
-    for (const auto& p : pieces) {
-        FNX_CUDA_OK(cudaMemcpyAsync(p.first, src, p.second, cudaMemcpyHostToDevice, e->st));
-        src += (p.second + 15) & ~(size_t) 15;
-    }
+    FNX_TRY(copy_pieces(e, pieces, const_cast<char*>(src), false));
     const int zero = 0;
     FNX_CUDA_OK(cudaMemcpyAsync(e->d_pos + seq, &h.pos, sizeof(int), cudaMemcpyHostToDevice, e->st));
     FNX_CUDA_OK(cudaMemcpyAsync(e->d_ctx_n + seq, &h.pos, sizeof(int), cudaMemcpyHostToDevice, e->st));

@@ -41,26 +41,8 @@ inline cudaStream_t as_stream(fnx_stream s) { return (cudaStream_t) s; }
 int sm_count();
 // raises a kernel's dynamic shared-memory limit on the current device, once per (device, kernel)
 int set_smem_limit(const void* kernel, int bytes);
-// Programmatic dependent launch: every kernel of the window is launched so that it may start while its predecessor
-// in the stream drains.  A kernel does whatever does not depend on earlier kernels (its tables, its barriers, bulk
-// copies of weights), then pdl_wait() before it touches anything an earlier kernel wrote.  Off unless FNX_PDL=1:
-// inside the window's CUDA graph the overlap measured slower than plain stream order on B200.
-bool pdl_enabled();
 #if defined(__CUDACC__)
-template <typename... KArgs, typename... Args>
-inline cudaError_t launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl_enabled() ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
-}
+// Programmatic dependent launch: a kernel may start while its predecessor in the stream drains.
 // A kernel of an engine's window, which leaves room for its successor on the SM (registers and shared memory of two blocks fit): it may
 // start while its predecessor drains.  Before pdl_wait() it may read what no kernel since the last but one before it writes (weights,
 // the starting states); an operator of the C ABI, whose caller may have filled any input just before, is launched with early = false

@@ -172,7 +172,7 @@ using namespace fnxb;
 extern "C" int fnx_argmax_mapped(const float* logits, int T, int V, const int* map, int* best_i, float* best_v, unsigned* err, fnx_stream st) {
     FNX_REQUIRE(logits && best_i && err && T >= 1 && V >= 1, "fnx_argmax: bad arguments");
     {
-        const cudaError_t le_ = launch_k(k_argmax, dim3(T, T <= ARGMAX_ROWS && V >= 65536 ? ARGMAX_NB : 1), dim3(1024), 0, as_stream(st), logits, V, map, best_i, best_v, err);
+        const cudaError_t le_ = launch_dep(true, k_argmax, dim3(T, T <= ARGMAX_ROWS && V >= 65536 ? ARGMAX_NB : 1), dim3(1024), 0, as_stream(st), logits, V, map, best_i, best_v, err);
         if (le_ != cudaSuccess) return fail(FNX_E_CUDA, "k_argmax: launch failed: %s", cudaGetErrorString(le_));
     }
     FNX_LAUNCH_OK("fnx_argmax");
@@ -186,7 +186,7 @@ extern "C" int fnx_argmax(const float* logits, int T, int V, int* best_i, float*
 extern "C" int fnx_top_tokens(const float* logits, int T, int V, float* out_v, int* out_i, fnx_stream st) {
     FNX_REQUIRE(logits && out_v && out_i && T >= 1 && V >= FNX_TOPK_N, "fnx_top_tokens: bad arguments (vocabulary of at least %d)", FNX_TOPK_N);
     {
-        const cudaError_t le_ = launch_k(k_top_tokens, dim3(T), dim3(1024), 0, as_stream(st), logits, V, out_v, out_i);
+        const cudaError_t le_ = launch_dep(true, k_top_tokens, dim3(T), dim3(1024), 0, as_stream(st), logits, V, out_v, out_i);
         if (le_ != cudaSuccess) return fail(FNX_E_CUDA, "k_top_tokens: launch failed: %s", cudaGetErrorString(le_));
     }
     FNX_LAUNCH_OK("fnx_top_tokens");
@@ -241,7 +241,7 @@ extern "C" int fnx_logit_adjust(float* logits, int T, int V, const int* ctx, con
     FNX_REQUIRE(last_n == 0 || repeat > 0.f, "fnx_logit_adjust: repeat penalty %g (> 0)", (double) repeat);
     FNX_REQUIRE(bias_n >= 0 && (bias_n == 0 || (bias_tok && bias_val)), "fnx_logit_adjust: a bias list of %d entries without its arrays", bias_n);
     {
-        const cudaError_t le_ = launch_k(k_logit_adjust, dim3(T), dim3(ADJ_THREADS), sizeof(int) * (size_t) (last_n > 0 ? last_n : 1), as_stream(st), logits, V, ctx,
+        const cudaError_t le_ = launch_dep(true, k_logit_adjust, dim3(T), dim3(ADJ_THREADS), sizeof(int) * (size_t) (last_n > 0 ? last_n : 1), as_stream(st), logits, V, ctx,
                                          ctx_n, tok, last_n, repeat, freq, present, bias_tok, bias_val, bias_n);
         if (le_ != cudaSuccess) return fail(FNX_E_CUDA, "k_logit_adjust: launch failed: %s", cudaGetErrorString(le_));
     }
@@ -252,7 +252,7 @@ extern "C" int fnx_logit_adjust(float* logits, int T, int V, const int* ctx, con
 extern "C" int fnx_embed_rows(const void* table_f16, const int* tok, int T, int H, float* R, fnx_stream st) {
     FNX_REQUIRE(table_f16 && tok && R && T >= 1, "fnx_embed_rows: bad arguments");
     {
-        const cudaError_t le_ = launch_k(k_embed_rows, dim3(dim3((H + 255) / 256, T)), dim3(256), 0, as_stream(st), (const __half*) table_f16, tok, H, R);
+        const cudaError_t le_ = launch_dep(true, k_embed_rows, dim3(dim3((H + 255) / 256, T)), dim3(256), 0, as_stream(st), (const __half*) table_f16, tok, H, R);
         if (le_ != cudaSuccess) return fail(FNX_E_CUDA, "k_embed_rows: launch failed: %s", cudaGetErrorString(le_));
     }
     FNX_LAUNCH_OK("fnx_embed_rows");
@@ -281,7 +281,7 @@ extern "C" int fnx_mtp_input(const void* fc_hid, const void* fc_emb, const void*
 extern "C" int fnx_rmsnorm(const float* x, const float* w, float* y, int rows, int n, float eps, fnx_stream st) {
     FNX_REQUIRE(x && w && y && rows >= 1 && n >= 1, "fnx_rmsnorm: bad arguments");
     {
-        const cudaError_t le_ = launch_k(k_rmsnorm, dim3(rows), dim3(256), 0, as_stream(st), x, w, y, n, eps);
+        const cudaError_t le_ = launch_dep(true, k_rmsnorm, dim3(rows), dim3(256), 0, as_stream(st), x, w, y, n, eps);
         if (le_ != cudaSuccess) return fail(FNX_E_CUDA, "k_rmsnorm: launch failed: %s", cudaGetErrorString(le_));
     }
     FNX_LAUNCH_OK("fnx_rmsnorm");

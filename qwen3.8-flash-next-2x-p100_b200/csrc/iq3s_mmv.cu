@@ -57,17 +57,18 @@ __global__ void __launch_bounds__(MMV_THREADS, 1) k_iq3s_mmv(const MmvParams p) 
     S.jobs_s = reinterpret_cast<fnx_job*>(reinterpret_cast<uint8_t*>(S.pieces) + (size_t) MMV_WARPS * 2 * sizeof(PieceSlotT<NG, MODE>));
     unsigned long long* prof = g_mmv_prof ? g_mmv_prof + (size_t) blockIdx.x * MMV_PROF_SLOTS : nullptr;
     int nstamp = 0;
-    MMV_STAMP();
+    // the codebook is replicated and the barriers are set up while the kernel before drains: five dense launches in a row of 12,352 x 2,048
+    // took 18 us each one after another
     pdl_launch_dependents();
-    pdl_wait();   // from here on: what earlier kernels of the stream wrote (activations, job lists)
-    // the job list or the first rows are fetched while the codebook is replicated and the barriers are set up
-    StageRegs h;
-    stage_begin<NG, MODE, MMV_WARPS>(p, h, tid, RowPlain());
     core_fill_table(table, tid, MMV_THREADS);
     if (lane == 0) {
         for (int i = 0; i < R; ++i) mbar_init(&S.bars[warp * R + i], 1);
         fence_barrier_init();
     }
+    pdl_wait();   // from here on: what earlier kernels of the stream wrote (weights, activations, job lists)
+    MMV_STAMP();
+    StageRegs h;
+    stage_begin<NG, MODE, MMV_WARPS>(p, h, tid, RowPlain());
     __syncthreads();
     WarpRing ring;
     ring.parity = 0;
@@ -86,7 +87,7 @@ static int launch_mmv(const MmvParams& p0, cudaStream_t st) {
     if (smem > LIMIT) return fail(FNX_E_ARG, "iq3s_mmv: %d columns x %d rows need %zu bytes of shared memory", p.K, 4 * NG, smem);
     if (int rc = set_smem_limit((const void*) k_iq3s_mmv<NG, MODE>, (int) LIMIT)) return rc;
     {
-        const cudaError_t le_ = launch_k(k_iq3s_mmv<NG, MODE>, dim3(sm_count()), dim3(MMV_THREADS), smem, st, p);
+        const cudaError_t le_ = launch_dep(true, k_iq3s_mmv<NG, MODE>, dim3(sm_count()), dim3(MMV_THREADS), smem, st, p);
         if (le_ != cudaSuccess) return fail(FNX_E_CUDA, "iq3s_mmv: launch failed: %s", cudaGetErrorString(le_));
     }
     return FNX_OK;

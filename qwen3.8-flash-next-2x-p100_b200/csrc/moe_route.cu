@@ -413,7 +413,7 @@ extern "C" int fnx_moe_combine(const float* part, const int* topi, const float* 
     FNX_REQUIRE(part && topi && topw && logits && out, "fnx_moe_combine: null pointer");
     FNX_REQUIRE(T >= 1 && T <= FNX_MAX_ROWS, "fnx_moe_combine: %d rows", T);
     {
-        const cudaError_t le_ = launch_k(k_combine, dim3(dim3((H + 255) / 256, T)), dim3(256), 0, as_stream(st), part, topi, topw, logits, T, E, H, K, e_lo, e_hi, add_shared, out, accumulate);
+        const cudaError_t le_ = launch_dep(true, k_combine, dim3(dim3((H + 255) / 256, T)), dim3(256), 0, as_stream(st), part, topi, topw, logits, T, E, H, K, e_lo, e_hi, add_shared, out, accumulate);
         if (le_ != cudaSuccess) return fail(FNX_E_CUDA, "k_combine: launch failed: %s", cudaGetErrorString(le_));
     }
     FNX_LAUNCH_OK("fnx_moe_combine");
@@ -427,7 +427,7 @@ extern "C" int fnx_moe_combine_image(const float* part, const int* topi, const f
     FNX_REQUIRE(H == 256 || H == 512 || H == 1024 || H == 2048 || H == 4096, "fnx_moe_combine_image: hidden %d", H);
     FNX_REQUIRE(((uintptr_t) img_out & 15) == 0 && ((uintptr_t) R & 15) == 0 && ((uintptr_t) part & 15) == 0, "fnx_moe_combine_image: 16-byte alignment");
     {
-        const cudaError_t le_ = launch_k(k_combine_image, dim3(H / 256, T), dim3(32), 0, as_stream(st), part, topi, topw, logits, T, E, H, K, R, (uint8_t*) img_out,
+        const cudaError_t le_ = launch_dep(true, k_combine_image, dim3(H / 256, T), dim3(32), 0, as_stream(st), part, topi, topw, logits, T, E, H, K, R, (uint8_t*) img_out,
                                          img_norm_w, fnx_dense_image_bytes(H));
         if (le_ != cudaSuccess) return fail(FNX_E_CUDA, "k_combine_image: launch failed: %s", cudaGetErrorString(le_));
     }

@@ -72,6 +72,8 @@ __global__ void k_accept_greedy(const int* __restrict__ tok, const int* __restri
 
 // batched lanes: block j walks lane j's chain (rows [lane_row0[j], lane_row0[j + 1])) into result row j
 __global__ void k_accept_greedy_lanes(const int* __restrict__ tok, const int* __restrict__ best, const int* __restrict__ lane_row0, int* __restrict__ result) {
+    pdl_wait();
+    pdl_launch_dependents();
     if (threadIdx.x != 0) return;
     const int lane = blockIdx.x, row0 = lane_row0[lane];
     accept_greedy_walk(tok + row0, nullptr, best + row0, lane_row0[lane + 1] - row0, result + (size_t) lane * (1 + 2 * FNX_MAX_ROWS));
@@ -200,6 +202,8 @@ __global__ void __launch_bounds__(1024) k_accept_sample_lanes(const float* __res
                                                               const int* __restrict__ tok, fnx_sampling sp, uint64_t seed,
                                                               const int* __restrict__ lane_seq, const int* __restrict__ lane_row0,
                                                               const uint32_t* __restrict__ steps, int* __restrict__ result) {
+    pdl_wait();
+    pdl_launch_dependents();
     extern __shared__ __align__(16) uint8_t smem[];
     const int lane = blockIdx.x, row0 = lane_row0[lane], seq = lane_seq[lane];
     accept_sample_body(cand_v + (size_t) row0 * FNX_TOPK_N, cand_i + (size_t) row0 * FNX_TOPK_N, tok + row0, lane_row0[lane + 1] - row0, sp, nullptr, nullptr, nullptr,
@@ -213,7 +217,7 @@ using namespace fnxb;
 extern "C" int fnx_lookup_draft(const int* ctx, const int* n, int lk, const int* d1, int* out, int* out_n, fnx_stream st) {
     FNX_REQUIRE(ctx && n && out && out_n && lk >= 0 && lk <= FNX_MAX_ROWS, "fnx_lookup_draft: bad arguments");
     {
-        const cudaError_t le_ = launch_k(k_lookup, dim3(1), dim3(1024), 0, as_stream(st), ctx, n, lk, d1, out, out_n);
+        const cudaError_t le_ = launch_dep(true, k_lookup, dim3(1), dim3(1024), 0, as_stream(st), ctx, n, lk, d1, out, out_n);
         if (le_ != cudaSuccess) return fail(FNX_E_CUDA, "k_lookup: launch failed: %s", cudaGetErrorString(le_));
     }
     FNX_LAUNCH_OK("fnx_lookup_draft");
@@ -223,7 +227,7 @@ extern "C" int fnx_lookup_draft(const int* ctx, const int* n, int lk, const int*
 extern "C" int fnx_accept_greedy(const int* tok, const int* parent, const int* best, int T, int* result, fnx_stream st) {
     FNX_REQUIRE(tok && best && result && T >= 1 && T <= FNX_MAX_ROWS, "fnx_accept_greedy: bad arguments");
     {
-        const cudaError_t le_ = launch_k(k_accept_greedy, dim3(1), dim3(32), 0, as_stream(st), tok, parent, best, T, result);
+        const cudaError_t le_ = launch_dep(true, k_accept_greedy, dim3(1), dim3(32), 0, as_stream(st), tok, parent, best, T, result);
         if (le_ != cudaSuccess) return fail(FNX_E_CUDA, "k_accept_greedy: launch failed: %s", cudaGetErrorString(le_));
     }
     FNX_LAUNCH_OK("fnx_accept_greedy");
@@ -238,7 +242,7 @@ extern "C" int fnx_accept_sample(const float* cand_v, const int* cand_i, const i
     const size_t smem = sizeof(DistS) * (size_t) T + sizeof(double) * FNX_TOPK_N * (size_t) T;
     if (int rc = set_smem_limit((const void*) k_accept_sample, 64 * 1024)) return rc;
     {
-        const cudaError_t le_ = launch_k(k_accept_sample, dim3(1), dim3(1024), smem, as_stream(st), cand_v, cand_i, tok, T, s, q_ids, q_p, q_n, seed, seq, step, result);
+        const cudaError_t le_ = launch_dep(true, k_accept_sample, dim3(1), dim3(1024), smem, as_stream(st), cand_v, cand_i, tok, T, s, q_ids, q_p, q_n, seed, seq, step, result);
         if (le_ != cudaSuccess) return fail(FNX_E_CUDA, "k_accept_sample: launch failed: %s", cudaGetErrorString(le_));
     }
     FNX_LAUNCH_OK("fnx_accept_sample");
@@ -248,7 +252,7 @@ extern "C" int fnx_accept_sample(const float* cand_v, const int* cand_i, const i
 // ---- batched lanes: one result row of 1 + 2 FNX_MAX_ROWS ints per lane
 extern "C" int fnx_accept_greedy_lanes(const int* tok, const int* best, const int* lane_row0, int n_lanes, int* result, fnx_stream st) {
     FNX_REQUIRE(tok && best && lane_row0 && result && n_lanes >= 1 && n_lanes <= FNX_MAX_ROWS, "fnx_accept_greedy_lanes: bad arguments");
-    const cudaError_t le = launch_k(k_accept_greedy_lanes, dim3(n_lanes), dim3(32), 0, as_stream(st), tok, best, lane_row0, result);
+    const cudaError_t le = launch_dep(true, k_accept_greedy_lanes, dim3(n_lanes), dim3(32), 0, as_stream(st), tok, best, lane_row0, result);
     if (le != cudaSuccess) return fail(FNX_E_CUDA, "k_accept_greedy_lanes: launch failed: %s", cudaGetErrorString(le));
     FNX_LAUNCH_OK("fnx_accept_greedy_lanes");
     return FNX_OK;
@@ -262,7 +266,7 @@ extern "C" int fnx_accept_sample_lanes(const float* cand_v, const int* cand_i, c
     FNX_REQUIRE(s.temperature > 0.f, "fnx_accept_sample_lanes: temperature %g", (double) s.temperature);
     const size_t smem = sizeof(DistS) * (size_t) max_lane_rows + sizeof(double) * FNX_TOPK_N * (size_t) max_lane_rows;
     if (int rc = set_smem_limit((const void*) k_accept_sample_lanes, 64 * 1024)) return rc;
-    const cudaError_t le = launch_k(k_accept_sample_lanes, dim3(n_lanes), dim3(1024), smem, as_stream(st), cand_v, cand_i, tok, s, seed, lane_seq, lane_row0, steps, result);
+    const cudaError_t le = launch_dep(true, k_accept_sample_lanes, dim3(n_lanes), dim3(1024), smem, as_stream(st), cand_v, cand_i, tok, s, seed, lane_seq, lane_row0, steps, result);
     if (le != cudaSuccess) return fail(FNX_E_CUDA, "k_accept_sample_lanes: launch failed: %s", cudaGetErrorString(le));
     FNX_LAUNCH_OK("fnx_accept_sample_lanes");
     return FNX_OK;
