@@ -20,6 +20,7 @@
 #include "iq3s_grid.h"
 #include "iq3s_tile.h"
 #include "nat_tile.h"
+#include "prompt_nat.cuh"
 
 namespace fnxb {
 
@@ -37,9 +38,7 @@ constexpr int PF_SBO = (PF_KC / 8) * PF_LBO;   // ... along the rows
 constexpr int PF_TILE_A = (PF_M / 8) * PF_SBO; // bytes of one f16 weight tile (128 features x 64)
 constexpr int PF_TILE_B = (PF_N / 8) * PF_SBO; // ... of the activation tile (256 rows x 64)
 
-struct PfJob {
-    int w, n, start;   // expert, rows, first entry of `order`
-};
+typedef PnJob PfJob;
 
 __device__ static const uint32_t g_grid_pf[512] = {FNX_IQ3S_GRID_VALUES};
 
@@ -169,13 +168,6 @@ __device__ __forceinline__ uint32_t pf_decode(const uint32_t (&S)[5], const uint
 // chunk).  Lane q of a row holds the sub-block's columns 8 q .. 8 q + 7: lookup 2 SB the first four, 2 SB + 1 the others
 // (the tile layout pairs them with the activation cells of 8 consecutive columns, iq3s_tile.h).
 template <int SB>
-__device__ __forceinline__ void pf_sub_block(const PfRawNat& r, uint8_t* tileA, int row0, int lane, uint32_t) {
-    const int g = lane >> 2, q = lane & 3, k0 = (SB & 1) * 32 + 8 * q;
-    const __half2 f0 = __float2half2_rn(r.d0 * (float) (1 + 2 * (int) ((r.sn0 >> (4 * SB)) & 15u))), f1 = __float2half2_rn(r.d1 * (float) (1 + 2 * (int) ((r.sn1 >> (4 * SB)) & 15u)));
-    *reinterpret_cast<uint4*>(tileA + pf_off(row0 + g, k0)) = pf_halves8_nat(r.w[0][SB], f0);
-    *reinterpret_cast<uint4*>(tileA + pf_off(row0 + g + 8, k0)) = pf_halves8_nat(r.w[1][SB], f1);
-}
-template <int SB>
 __device__ __forceinline__ void pf_sub_block(const PfRaw& r, uint8_t* tileA, int row0, int lane, uint32_t table_s) {
     const int g = lane >> 2, q = lane & 3, k0 = (SB & 1) * 32 + 8 * q;
     const __half2 f0 = __float2half2_rn(r.d0 * (float) (1 + 2 * (int) ((r.sn0 >> (8 * (SB >> 1) + 4 * (SB & 1))) & 15u)));
@@ -184,8 +176,8 @@ __device__ __forceinline__ void pf_sub_block(const PfRaw& r, uint8_t* tileA, int
     pf_store8(tileA, row0 + g + 8, k0, pf_decode<2 * SB>(r.S1, r.G1, table_s), pf_decode<2 * SB + 1>(r.S1, r.G1, table_s), f1);
 }
 // the warp's share of quarter Q of a tile block (sub-blocks 2 Q, 2 Q + 1): gate|up: both; down (two warps per tile): one
-template <int Q, int MODE, typename Raw>
-__device__ __forceinline__ void pf_quarter(const Raw& r, uint8_t* tileA, int row0, int lane, uint32_t table_s, int sel) {
+template <int Q, int MODE>
+__device__ __forceinline__ void pf_quarter(const PfRaw& r, uint8_t* tileA, int row0, int lane, uint32_t table_s, int sel) {
     if (MODE == 1) {
         pf_sub_block<2 * Q>(r, tileA, row0, lane, table_s);
         pf_sub_block<2 * Q + 1>(r, tileA, row0, lane, table_s);
@@ -216,8 +208,7 @@ struct PfParams {
 };
 
 // MODE 0: out = x W^T (down).  MODE 1: out = silu(x Wg^T) * (x Wu^T) (gate|up; W = [gate (rows); up (rows)]).
-// NAT: the weights lie in the engine's own layout.
-template <int MODE, bool NAT>
+template <int MODE>
 __global__ void __launch_bounds__(PF_BLOCK, 1) k_pf_gemm(const PfParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
     constexpr int NA = MODE == 1 ? 2 : 1;                      // weight tiles per stage
@@ -234,8 +225,7 @@ __global__ void __launch_bounds__(PF_BLOCK, 1) k_pf_gemm(const PfParams p) {
     const PfJob job = p.jobs[blockIdx.x];
     const int ft = blockIdx.y, KB = p.K / 256, nchunk = p.K / PF_KC;
     const uint8_t* W = job.w >= p.E ? p.Wsh : p.W + (size_t) (job.w - p.e_base) * p.expert_stride;
-    if (!NAT)
-        for (int i = tid; i < 512 * PF_REP; i += PF_BLOCK) table[i] = g_grid_pf[i / PF_REP];
+    for (int i = tid; i < 512 * PF_REP; i += PF_BLOCK) table[i] = g_grid_pf[i / PF_REP];
     if (tid < PF_N) {
         int src = -1, o = 0;
         if (tid < job.n) {
@@ -288,17 +278,15 @@ __global__ void __launch_bounds__(PF_BLOCK, 1) k_pf_gemm(const PfParams p) {
     } else {
         // 16 warps: warp w decodes tile row (w % 8) of the 128-feature slab; gate|up: of the gate (w < 8) or the up matrix
         // (all four sub-blocks of the chunk); down: sub-block pair w / 8 of the chunk
-        using Raw = typename std::conditional<NAT, PfRawNat, PfRaw>::type;
-        Raw raw, nxt;
+        PfRaw raw, nxt;
         const int sel = warp >> 3;
         const int trow = (MODE == 1 && sel ? p.rows / 16 : 0) + ft * (PF_M / 16) + (warp & 7);
         const int a_off = MODE == 1 && sel ? PF_TILE_A : 0, row0 = (warp & 7) * 16;
         // (a slab past the matrix's last tile row, when the features are not a multiple of 128, decodes zero weights)
         const bool live_row = MODE == 1 || trow < p.rows / 16;
-        const int n16 = (MODE == 1 ? 2 : 1) * (p.rows / 16);
-        auto load_raw = [&](int kb, Raw& r) {
-            if (live_row) pf_load_raw(NAT ? W + nat_half_at(trow, n16, kb, KB, MODE == 1) : W + ((size_t) trow * KB + kb) * TILE_BYTES, lane, r);
-            else r = Raw{};
+        auto load_raw = [&](int kb, PfRaw& r) {
+            if (live_row) pf_load_raw(W + ((size_t) trow * KB + kb) * TILE_BYTES, lane, r);
+            else r = PfRaw{};
         };
         load_raw(0, raw);
         // the activations of chunk c into its stage: 16-byte pieces (8 columns of one row = one core-matrix row) by async copies;
@@ -419,7 +407,7 @@ __global__ void k_pf_count(const int* __restrict__ topi, int n, int e_lo, int* _
 
 // one block: the experts' first entries and jobs (ascending expert order, then the shared expert's)
 __global__ void k_pf_plan(const int* __restrict__ cnt, int ne, int e_lo, int E, int T, int TKp, int add_shared, int* __restrict__ base, PfJob* __restrict__ jobs,
-                          int* __restrict__ njobs, int* __restrict__ order) {
+                          int* __restrict__ njobs, int* __restrict__ order, int per) {   // per: rows a job
     // counts into shared memory, one thread's running sums over them (a few hundred shared-memory steps), then every thread
     // writes its experts' jobs
     __shared__ int s_cnt[1024], s_entry[1024], s_job[1024];
@@ -432,7 +420,7 @@ __global__ void k_pf_plan(const int* __restrict__ cnt, int ne, int e_lo, int E, 
             s_entry[e] = entry;
             s_job[e] = nj;
             entry += s_cnt[e];
-            nj += (s_cnt[e] + PF_N - 1) / PF_N;
+            nj += (s_cnt[e] + per - 1) / per;
         }
         s_entries = entry;
         s_jobs = nj;
@@ -441,14 +429,14 @@ __global__ void k_pf_plan(const int* __restrict__ cnt, int ne, int e_lo, int E, 
     for (int e = threadIdx.x; e < ne; e += blockDim.x) {
         base[e] = s_entry[e];
         int j = s_job[e];
-        for (int o = 0; o < s_cnt[e]; o += PF_N) jobs[j++] = PfJob{e_lo + e, min(PF_N, s_cnt[e] - o), s_entry[e] + o};
+        for (int o = 0; o < s_cnt[e]; o += per) jobs[j++] = PfJob{e_lo + e, min(per, s_cnt[e] - o), s_entry[e] + o};
     }
     const int entry = s_entries, nj = s_jobs;
     if (add_shared) {
         for (int t = threadIdx.x; t < T; t += blockDim.x) order[entry + t] = TKp + t;
-        for (int j = threadIdx.x; j < (T + PF_N - 1) / PF_N; j += blockDim.x) jobs[nj + j] = PfJob{E, min(PF_N, T - j * PF_N), entry + j * PF_N};
+        for (int j = threadIdx.x; j < (T + per - 1) / per; j += blockDim.x) jobs[nj + j] = PfJob{E, min(per, T - j * per), entry + j * per};
     }
-    if (threadIdx.x == 0) njobs[0] = nj + (add_shared ? (T + PF_N - 1) / PF_N : 0);
+    if (threadIdx.x == 0) njobs[0] = nj + (add_shared ? (T + per - 1) / per : 0);
 }
 
 // per expert: its pairs in ascending order into order[base ..): a thread looks at four consecutive pairs per step
@@ -595,17 +583,17 @@ __global__ void __launch_bounds__(256) k_pf_decode_f16(const uint8_t* __restrict
         sub(std::integral_constant<int, 4>{}); sub(std::integral_constant<int, 5>{}); sub(std::integral_constant<int, 6>{}); sub(std::integral_constant<int, 7>{});
     }
 }
-// the same from n matrices in the engine's own layout, one after another; one warp per half tile
-__global__ void __launch_bounds__(256) k_pf_decode_nat(const uint8_t* __restrict__ W, size_t stride, int n, int rows, int K, int gate_up, __half* __restrict__ out) {
+// the same from a matrix in the engine's own layout; one warp per half tile
+__global__ void __launch_bounds__(256) k_pf_decode_nat(const uint8_t* __restrict__ W, int rows, int K, __half* __restrict__ out) {
     const int lane = threadIdx.x & 31, KB = K / 256, n16 = rows / 16;
-    const size_t per = (size_t) n16 * KB, nblk = (size_t) n * per;
+    const size_t nblk = (size_t) n16 * KB;
     const int g = lane >> 2, q = lane & 3;
     for (size_t b = (size_t) blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5); b < nblk; b += (size_t) gridDim.x * (blockDim.x / 32)) {
-        const size_t m = b / per, i = b % per, trow = i / KB;
-        const int kb = (int) (i % KB);
+        const size_t trow = b / KB;
+        const int kb = (int) (b % KB);
         PfRawNat r;
-        pf_load_raw(W + m * stride + nat_half_at(trow, n16, kb, KB, gate_up), lane, r);
-        __half* o0 = out + ((size_t) m * rows + trow * 16 + g) * K + (size_t) kb * 256 + 8 * q;
+        pf_load_raw(W + nat_half_at(trow, n16, kb, KB, false), lane, r);
+        __half* o0 = out + (trow * 16 + g) * K + (size_t) kb * 256 + 8 * q;
         __half* o1 = o0 + (size_t) 8 * K;
 #pragma unroll
         for (int sb = 0; sb < 8; ++sb) {
@@ -616,12 +604,11 @@ __global__ void __launch_bounds__(256) k_pf_decode_nat(const uint8_t* __restrict
     }
 }
 
-// n matrices of rows x K (tiles: one stacked matrix)
-static int pf_decode_f16_launch(const void* W, bool nat, size_t stride, int n, int rows, int K, int gate_up, __half* out, cudaStream_t st) {
-    const size_t nblk = (size_t) n * (rows / 16) * (K / 256);
+static int pf_decode_f16_launch(const void* W, bool nat, int rows, int K, __half* out, cudaStream_t st) {
+    const size_t nblk = (size_t) (rows / 16) * (K / 256);
     const unsigned blocks = (unsigned) (nblk / 8 < 148 * 8 ? (nblk + 7) / 8 : 148 * 8);
-    if (nat) k_pf_decode_nat<<<blocks, 256, 0, st>>>((const uint8_t*) W, stride, n, rows, K, gate_up, out);
-    else k_pf_decode_f16<<<blocks, 256, 0, st>>>((const uint8_t*) W, n * rows, K, out);
+    if (nat) k_pf_decode_nat<<<blocks, 256, 0, st>>>((const uint8_t*) W, rows, K, out);
+    else k_pf_decode_f16<<<blocks, 256, 0, st>>>((const uint8_t*) W, rows, K, out);
     FNX_LAUNCH_OK("k_pf_decode_f16");
     return FNX_OK;
 }
@@ -632,6 +619,16 @@ __global__ void k_pf_dense_jobs(int T, PfJob* __restrict__ jobs, int* __restrict
     if (i < T) order[i] = i;
     if (i < nj) jobs[i] = PfJob{0, min(PF_N, T - i * PF_N), i * PF_N};
     if (i == 0) *njobs = nj;
+}
+
+// f16 rows in place between natural and slot order (pn_slot), a warp per 32 columns
+__global__ void __launch_bounds__(256) k_pf_reorder(__half* __restrict__ h, size_t groups, int to_slots) {
+    const size_t g = (size_t) blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (g >= groups) return;
+    const int lane = threadIdx.x & 31, slot = pn_slot(lane);
+    const __half v = h[g * 32 + (to_slots ? lane : slot)];
+    __syncwarp();
+    h[g * 32 + (to_slots ? slot : lane)] = v;
 }
 
 constexpr size_t pf_smem(int mode) { return (size_t) PF_STAGES * ((mode == 1 ? 2 : 1) * PF_TILE_A + PF_TILE_B) + 2048 * PF_REP + 2 * PF_N * sizeof(int) + 64; }
@@ -667,7 +664,7 @@ static size_t pf_staged_bytes(size_t pairs, int E, int H, int F) {
 extern "C" size_t fnx_moe_prefill_scratch_bytes(int T, int K, int E, int H, int F) {
     const size_t pairs = (size_t) T * K + T;
     return pf_align(pairs * F * sizeof(__half)) + pf_align(pairs * H * sizeof(float)) + pf_align(pairs * sizeof(int)) + pf_align((size_t) (E + 1) * sizeof(int)) * 2 +
-           pf_align((pairs / PF_N + E + 2 + (size_t) T / PF_N) * sizeof(PfJob)) + pf_align((size_t) T * H * sizeof(__half)) + 256 +
+           pf_align((pairs / PN_N + E + 2 + (size_t) T / PN_N) * sizeof(PfJob)) + pf_align((size_t) T * H * sizeof(__half)) + 256 +
            (T >= 1024 ? pf_staged_bytes(pairs, E, H, F) : 0);
 }
 
@@ -688,7 +685,7 @@ int prompt_moe(const void* Wgu, size_t gu_stride, const void* Wsh_gu, bool gu_na
     int* order = (int*) b; b += pf_align(pairs * sizeof(int));
     int* cnt = (int*) b; b += pf_align((size_t) (E + 1) * sizeof(int));
     int* base = (int*) b; b += pf_align((size_t) (E + 1) * sizeof(int));
-    PfJob* jobs = (PfJob*) b; b += pf_align((pairs / PF_N + E + 2 + (size_t) T / PF_N) * sizeof(PfJob));
+    PfJob* jobs = (PfJob*) b; b += pf_align((pairs / PN_N + E + 2 + (size_t) T / PN_N) * sizeof(PfJob));
     __half* xh = (__half*) b; b += pf_align((size_t) T * H * sizeof(__half));
     int* njobs = (int*) b; b += 256;
     const int ne = e_hi - e_lo, n = T * K;
@@ -696,25 +693,29 @@ int prompt_moe(const void* Wgu, size_t gu_stride, const void* Wsh_gu, bool gu_na
         k_pf_count<<<ne, 1024, 0, st>>>(topi, n, e_lo, cnt);
         FNX_LAUNCH_OK("k_pf_count");
     }
-    k_pf_plan<<<1, 256, 0, st>>>(cnt, ne, e_lo, E, T, n, add_shared, base, jobs, njobs, order);
+    const int per = gu_nat || dn_nat ? PN_N : PF_N;
+    k_pf_plan<<<1, 256, 0, st>>>(cnt, ne, e_lo, E, T, n, add_shared, base, jobs, njobs, order, per);
     FNX_LAUNCH_OK("k_pf_plan");
     if (ne > 0) {
         k_pf_fill<<<ne, 256, 0, st>>>(topi, n, e_lo, base, order);
         FNX_LAUNCH_OK("k_pf_fill");
     }
-    k_pf_xnorm<<<T, 256, 0, st>>>(x, norm_w, H, eps, xh);
-    FNX_LAUNCH_OK("k_pf_xnorm");
-    // From 1,024 rows on, with every expert on this rank and stacked without gaps: the experts' matrices decoded to f16 once, the
-    // rows copied into job order, and the two grouped products with both operands by tensor copies (gemm_tma.cu).
-    if (T >= 1024 && !pf_gemm_off() && e_base == 0 && e_lo == 0 && e_hi == E && add_shared && (gu_nat || gu_stride == fnx_iq3s_bytes((size_t) 2 * F, (size_t) H)) &&
-        (dn_nat || dn_stride == fnx_iq3s_bytes((size_t) H, (size_t) F))) {
+    if (gu_nat) FNX_TRY(prompt_nat_rows(x, norm_w, T, H, eps, xh, st));
+    else {
+        k_pf_xnorm<<<T, 256, 0, st>>>(x, norm_w, H, eps, xh);
+        FNX_LAUNCH_OK("k_pf_xnorm");
+    }
+    // Interchange tiles from 1,024 rows on, with every expert on this rank and stacked without gaps: the experts' matrices decoded to f16
+    // once, the rows copied into job order, and the two grouped products with both operands by tensor copies (gemm_tma.cu).
+    if (T >= 1024 && !gu_nat && !dn_nat && !pf_gemm_off() && e_base == 0 && e_lo == 0 && e_hi == E && add_shared && gu_stride == fnx_iq3s_bytes((size_t) 2 * F, (size_t) H) &&
+        dn_stride == fnx_iq3s_bytes((size_t) H, (size_t) F)) {
         __half* xs = (__half*) b; b += pf_align(pairs * H * sizeof(__half));
         __half* gu16 = (__half*) b; b += pf_align((size_t) (E + 1) * 2 * F * H * sizeof(__half));
         __half* dn16 = (__half*) b;
-        FNX_TRY(pf_decode_f16_launch(Wgu, gu_nat, gu_stride, E, 2 * F, H, 1, gu16, st));
-        FNX_TRY(pf_decode_f16_launch(Wsh_gu, gu_nat, gu_stride, 1, 2 * F, H, 1, gu16 + (size_t) E * 2 * F * H, st));
-        FNX_TRY(pf_decode_f16_launch(Wdn, dn_nat, dn_stride, E, H, F, 0, dn16, st));
-        FNX_TRY(pf_decode_f16_launch(Wsh_dn, dn_nat, dn_stride, 1, H, F, 0, dn16 + (size_t) E * H * F, st));
+        FNX_TRY(pf_decode_f16_launch(Wgu, false, E * 2 * F, H, gu16, st));
+        FNX_TRY(pf_decode_f16_launch(Wsh_gu, false, 2 * F, H, gu16 + (size_t) E * 2 * F * H, st));
+        FNX_TRY(pf_decode_f16_launch(Wdn, false, E * H, F, dn16, st));
+        FNX_TRY(pf_decode_f16_launch(Wsh_dn, false, H, F, dn16 + (size_t) E * H * F, st));
         k_pf_gather_rows<<<(unsigned) pairs, 256, 0, st>>>(xh, order, n, K, H, xs);
         FNX_LAUNCH_OK("k_pf_gather_rows");
         const int nj = (int) ((size_t) n / PF_N) + ne + (T + PF_N - 1) / PF_N;
@@ -723,22 +724,33 @@ int prompt_moe(const void* Wgu, size_t gu_stride, const void* Wsh_gu, bool gu_na
         FNX_LAUNCH_OK("k_pf_combine");
         return FNX_OK;
     }
-    auto gu_kernel = gu_nat ? k_pf_gemm<1, true> : k_pf_gemm<1, false>;
-    auto dn_kernel = dn_nat ? k_pf_gemm<0, true> : k_pf_gemm<0, false>;
-    if (int rc = set_smem_limit((const void*) gu_kernel, (int) pf_smem(1))) return rc;
-    if (int rc = set_smem_limit((const void*) dn_kernel, (int) pf_smem(0))) return rc;
-    // the job count is known on the device only: the grids cover the largest it can be (an expert's pairs in jobs of PF_N rows:
-    // at most one ragged job per expert beyond pairs / PF_N) and the blocks past the count leave at once; nothing is read back
-    {
-        const int nj = (int) ((size_t) n / PF_N) + ne + (add_shared ? (T + PF_N - 1) / PF_N : 0);
-        PfParams p{};
-        p.W = (const uint8_t*) Wgu; p.expert_stride = gu_stride; p.e_base = e_base; p.E = E; p.Wsh = (const uint8_t*) Wsh_gu;
-        p.jobs = jobs; p.njobs = njobs; p.order = order; p.TKp = n; p.Kp = K; p.x = xh; p.rows = F; p.K = H; p.outh = hbuf; p.err = err;
-        gu_kernel<<<dim3(nj, F / PF_M), PF_BLOCK, pf_smem(1), st>>>(p);
+    // the job count is known on the device only: the grids cover the largest it can be (an expert's pairs in jobs of `per` rows:
+    // at most one ragged job per expert beyond pairs / per) and the blocks past the count leave at once; nothing is read back
+    const int nj = n / per + ne + (add_shared ? (T + per - 1) / per : 0);
+    PnParams q{};
+    q.e_base = e_base; q.E = E; q.jobs = jobs; q.njobs = njobs; q.order = order; q.T = T; q.TKp = n; q.Kp = K; q.err = err;
+    PfParams p{};
+    p.e_base = e_base; p.E = E; p.jobs = jobs; p.njobs = njobs; p.order = order; p.TKp = n; p.Kp = K; p.err = err;
+    if (gu_nat) {
+        q.W = (const uint8_t*) Wgu; q.stride = gu_stride; q.Wsh = (const uint8_t*) Wsh_gu; q.x = xh; q.rows = F; q.K = H; q.outh = hbuf;
+        FNX_TRY(prompt_nat(1, q, nj, st));
+    } else {
+        FNX_TRY(set_smem_limit((const void*) k_pf_gemm<1>, (int) pf_smem(1)));
+        p.W = (const uint8_t*) Wgu; p.expert_stride = gu_stride; p.Wsh = (const uint8_t*) Wsh_gu; p.x = xh; p.rows = F; p.K = H; p.outh = hbuf;
+        k_pf_gemm<1><<<dim3(nj, F / PF_M), PF_BLOCK, pf_smem(1), st>>>(p);
         FNX_LAUNCH_OK("k_pf_gemm (gate|up)");
-        p.W = (const uint8_t*) Wdn; p.expert_stride = dn_stride; p.Wsh = (const uint8_t*) Wsh_dn;
-        p.x = hbuf; p.rows = H; p.K = F; p.out = part; p.outh = nullptr;
-        dn_kernel<<<dim3(nj, H / PF_M), PF_BLOCK, pf_smem(0), st>>>(p);
+    }
+    if (gu_nat != dn_nat) {   // (one of the two matrices was asked for in the interchange layout)
+        k_pf_reorder<<<(unsigned) ((pairs * F / 32 + 7) / 8), 256, 0, st>>>(hbuf, pairs * F / 32, dn_nat);
+        FNX_LAUNCH_OK("k_pf_reorder");
+    }
+    if (dn_nat) {
+        q.W = (const uint8_t*) Wdn; q.stride = dn_stride; q.Wsh = (const uint8_t*) Wsh_dn; q.x = hbuf; q.rows = H; q.K = F; q.out = part; q.ldo = H;
+        FNX_TRY(prompt_nat(0, q, nj, st));
+    } else {
+        FNX_TRY(set_smem_limit((const void*) k_pf_gemm<0>, (int) pf_smem(0)));
+        p.W = (const uint8_t*) Wdn; p.expert_stride = dn_stride; p.Wsh = (const uint8_t*) Wsh_dn; p.x = hbuf; p.rows = H; p.K = F; p.out = part; p.outh = nullptr;
+        k_pf_gemm<0><<<dim3(nj, H / PF_M), PF_BLOCK, pf_smem(0), st>>>(p);
         FNX_LAUNCH_OK("k_pf_gemm (down)");
     }
     k_pf_combine<<<dim3((H / 4 + 255) / 256, T), 256, 0, st>>>(part, topi, topw, logits, T, E, H, K, e_lo, e_hi, add_shared, out, accumulate);
@@ -783,21 +795,26 @@ int prompt_dense(const void* W, bool nat, int rows, int cols, const float* x, in
     int* njobs = (int*) b; b += 256;
     __half* w16 = (__half*) b;
     const int nj = (T + PF_N - 1) / PF_N;
+    if (nat && T < pf_tma_rows()) {
+        FNX_TRY(prompt_nat_rows(x, norm_w, T, cols, eps, xh, st));
+        PnParams q{};
+        q.W = (const uint8_t*) W; q.T = T; q.x = xh; q.rows = rows; q.K = cols; q.out = y; q.ldo = ldy; q.accumulate = accumulate; q.err = err;
+        return prompt_nat(0, q, (T + PN_N - 1) / PN_N, st);
+    }
     k_pf_xnorm<<<T, 256, 0, st>>>(x, norm_w, cols, eps, xh);
     FNX_LAUNCH_OK("k_pf_xnorm");
     if (T >= pf_tma_rows()) {   // the matrix to f16 once, then one product with both operands by tensor copies
-        FNX_TRY(pf_decode_f16_launch(W, nat, 0, 1, rows, cols, 0, w16, st));
+        FNX_TRY(pf_decode_f16_launch(W, nat, rows, cols, w16, st));
         return gemm_tma_launch(w16, nullptr, xh, nullptr, y, ldy, T, rows, cols, accumulate, 1.0f, err, st);
     }
     k_pf_dense_jobs<<<(T + 255) / 256, 256, 0, st>>>(T, jobs, njobs, order);
     FNX_LAUNCH_OK("k_pf_dense_jobs");
-    auto kernel = nat ? k_pf_gemm<0, true> : k_pf_gemm<0, false>;
-    if (int rc = set_smem_limit((const void*) kernel, (int) pf_smem(0))) return rc;
+    FNX_TRY(set_smem_limit((const void*) k_pf_gemm<0>, (int) pf_smem(0)));
     PfParams p{};
     p.W = (const uint8_t*) W; p.expert_stride = 0; p.e_base = 0; p.E = 1; p.Wsh = nullptr;
     p.jobs = jobs; p.njobs = njobs; p.order = order; p.TKp = T; p.Kp = 1; p.x = xh; p.rows = rows; p.K = cols; p.out = y; p.outh = nullptr; p.err = err;
     p.ldo = ldy; p.accumulate = accumulate;
-    kernel<<<dim3(nj, (rows + PF_M - 1) / PF_M), PF_BLOCK, pf_smem(0), st>>>(p);
+    k_pf_gemm<0><<<dim3(nj, (rows + PF_M - 1) / PF_M), PF_BLOCK, pf_smem(0), st>>>(p);
     FNX_LAUNCH_OK("k_pf_gemm (dense)");
     return FNX_OK;
 }

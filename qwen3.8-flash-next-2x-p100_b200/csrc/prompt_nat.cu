@@ -1,0 +1,423 @@
+// Prompt products x W^T from weights in the engine's own layout (nat_tile.h): the prompt's projections below 1,024 rows and its expert
+// products at every length, on tcgen05.mma with the weights as the A operand in tensor memory.
+//
+// Replaces the reference's grouped expert GEMMs for prompts, moe_gate_up_mma / moe_down_mma (engine/src/kernels.hpp:328-330,
+// engine/src/moe_mma.cuh:301).
+//
+// What bounds it: at a few rows an expert, the weights' bytes (377 cycles of an SM's share of DRAM for 256 features x 64 columns); at
+// many, the products (8 x M128 N64 K16, 300 cycles) and the decode (16 warps x some 85 instructions, 340 cycles).  So nothing may pass
+// through shared memory that need not: f16 weight tiles written there by the decode and read back by the tensor core took 500 cycles
+// on their own, and 256-row tiles another 1,000 of products over rows that mostly were not there (thirteen rows an expert in a prompt
+// of 640).  Here
+//   - sixteen decode warps own a 16-row tile row each: 2,176-byte half tiles by their lanes' own async copies, four blocks ahead across
+//     items; nibbles to f16 with three shifts, four masks and twelve half operations a word of eight; the fragment layout is tcgen05.st's
+//     16x256b shape, so a chunk of 64 columns leaves as one store of sixteen registers;
+//   - two warps gather the job's live rows (a row of B only reaches its own column of D: the others stay what they are);
+//   - one warp issues the products, one thread each, two accumulators (gate and up, or 2 x 128 features) double-buffered in tensor memory;
+//   - four warps write the item before.
+// Tensor memory: columns [0, 256) two pairs of accumulators, [256, 512) four stages of two 128 x 64 weight tiles.  Jobs have at most 64
+// rows: wider tiles pay off in the products only from some 100 rows an expert, by 20% of a bound that the decode then has alone.
+// Measured: see prompt_nat().
+#include "attn_tc.cuh"
+#include "nat_tile.h"
+#include "prompt_nat.cuh"
+
+namespace fnxb {
+
+constexpr int PN_KC = 64;              // columns a stage
+constexpr int PN_DECODE = 16;          // warps
+constexpr int PN_EPI = 4, PN_LOAD = 2;
+constexpr int PN_W_EPI = PN_DECODE, PN_W_MMA = PN_W_EPI + PN_EPI, PN_W_LOAD = PN_W_MMA + 1;
+constexpr int PN_THREADS = (PN_W_LOAD + PN_LOAD) * 32;
+constexpr int PN_SLOTS = 4;            // half tiles in flight a decode warp
+constexpr int PN_AST = 4, PN_BST = 8;  // stages of A (tensor memory) and of B (shared memory)
+constexpr int PN_LAG = 3;              // chunks of B in flight
+constexpr int PN_BBYTES = PN_N * 128;
+constexpr int PN_RING = PN_DECODE * PN_SLOTS * NAT_HALF_BYTES;
+constexpr int PN_HEAD = 1024;
+constexpr int PN_SMEM = PN_HEAD + PN_BST * PN_BBYTES + PN_RING;
+constexpr uint32_t PN_ACC = 2 * PN_N, PN_A = 256;   // tensor memory: columns of an accumulator pair, first column of the weight stages
+static_assert(PN_SMEM <= 227 * 1024, "fits one block's shared memory");
+
+struct PnShared {
+    uint64_t full[PN_AST], empty[PN_AST];     // weights of a chunk in tensor memory
+    uint64_t bfull[PN_BST], bempty[PN_BST];   // rows of a chunk in shared memory
+    uint64_t acc_full[2], acc_empty[2];
+    uint32_t tmem;
+    volatile int gave_up;
+};
+static_assert(sizeof(PnShared) <= PN_HEAD, "the head fits");
+
+__device__ __forceinline__ bool pn_wait(uint64_t* bar, unsigned parity, PnShared& S) {
+    for (unsigned i = 0; i < TA_WAIT; ++i) {
+        if (mbar_try_wait(bar, parity)) return true;
+        if (S.gave_up) return false;
+    }
+    S.gave_up = 1;
+    return false;
+}
+
+// sixteen tensor-memory lanes x 32 columns: register 4 b + {0, 1} = columns 8 b + 2 q, + 1 of lane g, + {2, 3} the same of lane g + 8
+__device__ __forceinline__ void pn_st_tile(uint32_t taddr, const uint32_t (&v)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr), "r"(v[0]), "r"(v[1]),
+                 "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]),
+                 "r"(v[15])
+                 : "memory");
+}
+__device__ __forceinline__ uint32_t pn_h2(__half2 h) { return *reinterpret_cast<const uint32_t*>(&h); }
+__device__ __forceinline__ __half2 pn_as_h2(uint32_t u) { return *reinterpret_cast<const __half2*>(&u); }
+
+// The eight weights of a word times the sub-block's scale (in both halves of f): out[0], out[1] = columns (0, 2), (1, 3), out[2], out[3] =
+// (4, 6), (5, 7).  A nibble t at bits 1..4 of a half 0x6400 | .. is 1024 + 2 (t + 8) = 1039 + m; at bits 4..7 it is 1024 + 16 (t + 8) =
+// 8 (143 + m): both exact, so the one rounding is that of m f, as in the other forms of these products.
+__device__ __forceinline__ void pn_decode8(uint32_t w, __half2 f, uint32_t& o0, uint32_t& o1, uint32_t& o2, uint32_t& o3) {
+    const uint32_t s = w >> 8;
+    const uint32_t a = ((w * 2u) & 0x001E001Eu) ^ 0x64106410u, c = (w & 0x00F000F0u) ^ 0x64806480u;
+    const uint32_t b = ((s * 2u) & 0x001E001Eu) ^ 0x64106410u, d = (s & 0x00F000F0u) ^ 0x64806480u;
+    const __half2 k1 = pn_as_h2(0xE40FE40Fu);                                   // -1039
+    const __half2 k8 = pn_as_h2(0x30003000u), k2 = pn_as_h2(0xD878D878u);       // 1 / 8, -143
+    o0 = pn_h2(__hmul2(__hadd2(pn_as_h2(a), k1), f));
+    o1 = pn_h2(__hmul2(__hadd2(pn_as_h2(b), k1), f));
+    o2 = pn_h2(__hmul2(__hfma2(pn_as_h2(c), k8, k2), f));
+    o3 = pn_h2(__hmul2(__hfma2(pn_as_h2(d), k8, k2), f));
+}
+// a row's two scales d (1 + 2 s) of sub-blocks 2 Q and 2 Q + 1 (nibbles sn >> 8 Q); d in both halves.  d has 11 bits and 1 + 2 s five: the
+// product rounds once, as from f32
+__device__ __forceinline__ void pn_scales(uint32_t sn, int Q, __half2 d, __half2& f0, __half2& f1) {
+    const uint32_t t = sn >> (8 * Q);
+    const __half2 n = __hadd2(pn_as_h2(((t & 15u) << 1) | ((t & 0xF0u) << 13) | 0x64016401u), pn_as_h2(0xE400E400u));   // 1 + 2 s, exact
+    const __half2 f = __hmul2(n, d);
+    f0 = __low2half2(f);
+    f1 = __high2half2(f);
+}
+
+struct PnItem {
+    int w, n, start, slab;
+};
+
+template <int MODE>
+__global__ void __launch_bounds__(PN_THREADS, 1) k_prompt_nat(const PnParams p) {
+    extern __shared__ __align__(1024) uint8_t smem[];
+    PnShared& sh = *reinterpret_cast<PnShared*>(smem);
+    uint8_t* Bs = smem + PN_HEAD;
+    uint8_t* ring = Bs + PN_BST * PN_BBYTES;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid == 0) {
+        for (int i = 0; i < PN_AST; ++i) {
+            mbar_init(&sh.full[i], PN_DECODE);
+            mbar_init(&sh.empty[i], 1);
+        }
+        for (int i = 0; i < PN_BST; ++i) {
+            mbar_init(&sh.bfull[i], PN_LOAD);
+            mbar_init(&sh.bempty[i], 1);
+        }
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&sh.acc_full[i], 1);
+            mbar_init(&sh.acc_empty[i], PN_EPI);
+        }
+        sh.gave_up = smem_u32(smem) & 1023u ? 1 : 0;   // (the swizzled tiles need their 1,024-byte boundary)
+        fence_barrier_init();
+    }
+    if (warp == PN_W_MMA) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sh.tmem)), "r"(512) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    ta_fence_before();
+    __syncthreads();
+    ta_fence_after();
+    const uint32_t tmem = sh.tmem;
+    const int KB = p.K / 256, nchunk = p.K / PN_KC;
+    const int slabs = MODE == 1 ? p.rows / 128 : (p.rows + 255) / 256;
+    const int njobs = p.jobs ? *p.njobs : (p.T + PN_N - 1) / PN_N, total = njobs * slabs;
+    auto job_of = [&](int it) {
+        const int j = it / slabs;
+        PnItem x;
+        x.slab = it - j * slabs;
+        if (p.jobs) {
+            const PnJob jb = p.jobs[j];
+            x.w = jb.w; x.n = jb.n; x.start = jb.start;
+        } else {
+            x.w = 0; x.start = j * PN_N; x.n = min(PN_N, p.T - x.start);
+        }
+        return x;
+    };
+    bool ok = !sh.gave_up;
+    if (warp < PN_DECODE) {
+        // ---------------------------------------------------------------------------------------- decode
+        // tensor-memory lanes 32 (warp % 4) + 16 h of tile `mat`
+        const int lq = warp & 3, h = (warp >> 2) & 1, mat = warp >> 3;
+        const uint32_t t_lane = tmem + ((uint32_t) (32 * lq + 16 * h) << 16) + PN_A + mat * 32;
+        uint8_t* my = ring + warp * PN_SLOTS * NAT_HALF_BYTES;
+        const uint32_t my_s = smem_u32(my);
+        const int n16 = (MODE == 1 ? 2 : 1) * (p.rows / 16);
+        // the item's half tiles of this warp (null: past the matrix's last row)
+        auto expert_of = [&](int it) { return it < total && p.jobs ? p.jobs[it / slabs].w : 0; };
+        auto base_of = [&](int it, int e) -> const uint8_t* {
+            const int slab = it % slabs, i = MODE == 1 ? mat * (p.rows / 16) + slab * 8 + lq * 2 + h : slab * 16 + mat * 8 + lq * 2 + h;
+            if (MODE == 0 && i >= n16) return nullptr;
+            const uint8_t* W = !p.jobs ? p.W : e >= p.E ? p.Wsh : p.W + (size_t) (e - p.e_base) * p.stride;
+            return W + nat_half_at((size_t) i, (size_t) n16, 0, (size_t) KB, MODE == 1) + lane * 16;
+        };
+        // the copies' cursor
+        int fit = blockIdx.x, fkb = 0, fslot = 0;
+        const uint8_t* src = fit < total ? base_of(fit, expert_of(fit)) : nullptr;
+        int e_next = expert_of(fit + gridDim.x);   // (one item ahead: its load is not waited for)
+        auto fetch = [&]() {
+            if (fit < total) {
+                if (src) {
+                    const uint32_t dst = my_s + fslot * NAT_HALF_BYTES + lane * 16;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + j * 512), "l"(src + j * 512) : "memory");
+                    if (lane < 8) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + NAT_META), "l"(src + NAT_META) : "memory");
+                    src += NAT_TILE_BYTES;
+                }
+                if (++fkb == KB) {
+                    fkb = 0;
+                    fit += gridDim.x;
+                    if (fit < total) {
+                        src = base_of(fit, e_next);
+                        e_next = expert_of(fit + gridDim.x);
+                    }
+                }
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            fslot = fslot + 1 == PN_SLOTS ? 0 : fslot + 1;
+        };
+#pragma unroll
+        for (int i = 0; i < PN_SLOTS; ++i) fetch();
+        int c = 0, slot = 0;   // chunks so far
+        bool pending = false;
+        for (int it = blockIdx.x; it < total; it += gridDim.x) {
+            for (int kb = 0; kb < KB; ++kb) {
+                asm volatile("cp.async.wait_group %0;" ::"n"(PN_SLOTS - 1) : "memory");
+                __syncwarp();   // (the scales came in by other lanes' copies)
+                uint32_t w[2][8];
+                const uint8_t* t = my + slot * NAT_HALF_BYTES;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const uint4 v = *reinterpret_cast<const uint4*>(t + j * 512 + lane * 16);
+                    w[j >> 1][(j & 1) * 4] = v.x; w[j >> 1][(j & 1) * 4 + 1] = v.y; w[j >> 1][(j & 1) * 4 + 2] = v.z; w[j >> 1][(j & 1) * 4 + 3] = v.w;
+                }
+                const uint4 m = *reinterpret_cast<const uint4*>(t + NAT_META + (lane >> 2) * 16);
+                const __half2 d = pn_as_h2(m.z), d0 = __low2half2(d), d1 = __high2half2(d);
+                __syncwarp();   // every lane has the slot
+                fetch();
+                slot = slot + 1 == PN_SLOTS ? 0 : slot + 1;
+#pragma unroll
+                for (int Q = 0; Q < 4; ++Q, ++c) {
+                    uint32_t o[16];
+                    __half2 f00, f01, f10, f11;
+                    pn_scales(m.x, Q, d0, f00, f01);
+                    pn_scales(m.y, Q, d1, f10, f11);
+                    pn_decode8(w[0][2 * Q], f00, o[0], o[1], o[4], o[5]);
+                    pn_decode8(w[1][2 * Q], f10, o[2], o[3], o[6], o[7]);
+                    pn_decode8(w[0][2 * Q + 1], f01, o[8], o[9], o[12], o[13]);
+                    pn_decode8(w[1][2 * Q + 1], f11, o[10], o[11], o[14], o[15]);
+                    // the chunk before is in tensor memory by now (PN_AST and the chunks of a block are both 4: stage Q)
+                    if (pending) {
+                        ta_wait_st();
+                        ta_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&sh.full[(Q + 3) & 3]);
+                    }
+                    if (ok && c >= PN_AST) ok = __all_sync(0xffffffffu, pn_wait(&sh.empty[Q], (unsigned) ((c / PN_AST - 1) & 1), sh));
+                    ta_fence_after();
+                    pn_st_tile(t_lane + Q * 64, o);
+                    pending = true;
+                }
+            }
+        }
+        if (pending) {
+            ta_wait_st();
+            ta_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sh.full[3]);
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+    } else if (warp >= PN_W_LOAD) {
+        // ---------------------------------------------------------------------------------------- the rows
+        // thread: piece lt % 8 of the stage rows lt / 8 + 8 j
+        const int lt = tid - PN_W_LOAD * 32, piece = lt & 7, r0 = lt >> 3;
+        const uint32_t b_s = smem_u32(Bs) + r0 * 128 + ((piece ^ (r0 & 7)) * 16);   // (r0 + 8 j has the same low bits)
+        int c = 0;
+        auto landed = [&](int chunk) {
+            fence_proxy_async();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sh.bfull[chunk % PN_BST]);
+        };
+        for (int it = blockIdx.x; it < total; it += gridDim.x) {
+            const PnItem x = job_of(it);
+            const __half* src[PN_N / 8];
+#pragma unroll
+            for (int j = 0; j < PN_N / 8; ++j) {
+                const int r = r0 + 8 * j;
+                src[j] = nullptr;
+                if (r < x.n) {
+                    int row = x.start + r;
+                    if (p.jobs) {
+                        row = p.order[row];
+                        if (MODE == 1) row = row >= p.TKp ? row - p.TKp : row / p.Kp;
+                    }
+                    src[j] = p.x + (size_t) row * p.K + piece * 8;
+                }
+            }
+            for (int k = 0; k < nchunk; ++k, ++c) {
+                if (ok && c >= PN_BST) ok = __all_sync(0xffffffffu, pn_wait(&sh.bempty[c % PN_BST], (unsigned) ((c / PN_BST - 1) & 1), sh));
+                if (ok) {
+                    const uint32_t dst = b_s + (c % PN_BST) * PN_BBYTES;
+#pragma unroll
+                    for (int j = 0; j < PN_N / 8; ++j)
+                        if (src[j]) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + j * 1024), "l"(src[j] + k * PN_KC) : "memory");
+                }
+                asm volatile("cp.async.commit_group;" ::: "memory");
+                if (c >= PN_LAG) {
+                    asm volatile("cp.async.wait_group %0;" ::"n"(PN_LAG) : "memory");
+                    landed(c - PN_LAG);
+                }
+            }
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        for (int i = max(0, c - PN_LAG); i < c; ++i) landed(i);
+    } else if (warp == PN_W_MMA) {
+        // ---------------------------------------------------------------------------------------- the products
+        constexpr uint32_t IDESC = (1u << 4) | ((uint32_t) (PN_N >> 3) << 17) | ((uint32_t) (128 >> 4) << 24);
+        const uint32_t b_s = smem_u32(Bs);
+        int c = 0, nit = 0;
+        for (int it = blockIdx.x; it < total; it += gridDim.x, ++nit) {
+            const int buf = nit & 1;
+            const uint32_t acc = tmem + buf * PN_ACC;
+            if (ok && nit >= 2) ok = __all_sync(0xffffffffu, pn_wait(&sh.acc_empty[buf], (unsigned) ((nit / 2 - 1) & 1), sh));
+            for (int k = 0; k < nchunk; ++k, ++c) {
+                if (ok) ok = __all_sync(0xffffffffu, pn_wait(&sh.bfull[c % PN_BST], (unsigned) ((c / PN_BST) & 1), sh));
+                if (ok) ok = __all_sync(0xffffffffu, pn_wait(&sh.full[c % PN_AST], (unsigned) ((c / PN_AST) & 1), sh));
+                if (ok && ta_elect()) {
+                    ta_fence_after();
+                    const uint32_t a_t = tmem + PN_A + (c % PN_AST) * 64, b = b_s + (c % PN_BST) * PN_BBYTES;
+#pragma unroll
+                    for (int k16 = 0; k16 < PN_KC / 16; ++k16) {
+                        const uint64_t bd = ta_desc_sw(b + k16 * 32, 16, 1024);
+                        ta_mma_ta(acc, a_t + k16 * 8, bd, IDESC, (k | k16) != 0);
+                        ta_mma_ta(acc + PN_N, a_t + 32 + k16 * 8, bd, IDESC, (k | k16) != 0);
+                    }
+                    ta_commit(&sh.empty[c % PN_AST]);
+                    ta_commit(&sh.bempty[c % PN_BST]);
+                    if (k == nchunk - 1) ta_commit(&sh.acc_full[buf]);
+                }
+                __syncwarp();
+            }
+        }
+        if (ok && c > 0) {   // the last arrivals, before the shared memory goes
+            pn_wait(&sh.empty[(c - 1) % PN_AST], (unsigned) (((c - 1) / PN_AST) & 1), sh);
+            pn_wait(&sh.bempty[(c - 1) % PN_BST], (unsigned) (((c - 1) / PN_BST) & 1), sh);
+        }
+    } else {
+        // ---------------------------------------------------------------------------------------- the results
+        const int lq = warp & 3;
+        const uint32_t lane_base = (uint32_t) (32 * lq) << 16;
+        int nit = 0;
+        for (int it = blockIdx.x; it < total; it += gridDim.x, ++nit) {
+            const PnItem x = job_of(it);
+            const int buf = nit & 1;
+            if (ok) ok = __all_sync(0xffffffffu, pn_wait(&sh.acc_full[buf], (unsigned) ((nit / 2) & 1), sh));
+            ta_fence_after();
+            if (ok) {
+                const uint32_t acc = tmem + buf * PN_ACC + lane_base;
+#pragma unroll 1
+                for (int c0 = 0; c0 < x.n; c0 += 16) {
+                    const int e = min(c0 + (lane & 15), x.n - 1) + x.start, mine = p.jobs ? p.order[e] : e;
+                    float g[16], u[16];
+                    ta_ld16(acc + c0, g);
+                    ta_ld16(acc + PN_N + c0, u);
+                    ta_wait_ld(g, u);
+                    if (MODE == 1) {
+                        __half* o = p.outh + x.slab * 128 + lq * 32 + pn_slot(lane);
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) {
+                            const int row = __shfl_sync(0xffffffffu, mine, i);
+                            if (c0 + i < x.n) o[(size_t) row * p.rows] = __float2half_rn(siluf_(g[i]) * u[i]);
+                        }
+                    } else {
+                        const int f = x.slab * 256 + lq * 32 + lane;
+                        const bool in0 = f < p.rows, in1 = f + 128 < p.rows;
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) {
+                            const int row = __shfl_sync(0xffffffffu, mine, i);
+                            if (c0 + i < x.n) {
+                                float* o = p.out + (size_t) row * p.ldo + f;
+                                if (in0) o[0] = p.accumulate ? o[0] + g[i] : g[i];
+                                if (in1) o[128] = p.accumulate ? o[128] + u[i] : u[i];
+                            }
+                        }
+                    }
+                }
+            }
+            ta_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sh.acc_empty[buf]);
+        }
+    }
+    ta_fence_before();
+    __syncthreads();
+    if (tid == 0 && sh.gave_up) atomicOr(p.err, (unsigned) FNX_ERR_TIMEOUT);
+    if (warp == PN_W_MMA) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+}
+
+__global__ void __launch_bounds__(256) k_prompt_nat_rows(const float* __restrict__ x, const float* __restrict__ norm_w, int H, float eps, __half* __restrict__ xh) {
+    const float* xr = x + (size_t) blockIdx.x * H;
+    __shared__ float ws[8];
+    constexpr int HOLD = 4;   // the thread's pieces of up to 4,096 columns stay in registers
+    float4 v[HOLD];
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < HOLD; ++j) {
+        const int i = (threadIdx.x + j * 256) * 4;
+        v[j] = i < H ? *reinterpret_cast<const float4*>(xr + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+        ss += v[j].x * v[j].x + v[j].y * v[j].y + v[j].z * v[j].z + v[j].w * v[j].w;
+    }
+    for (int i = (threadIdx.x + HOLD * 256) * 4; i < H; i += 1024) {
+        const float4 q = *reinterpret_cast<const float4*>(xr + i);
+        ss += q.x * q.x + q.y * q.y + q.z * q.z + q.w * q.w;
+    }
+    float r = 1.0f;
+    if (norm_w) {
+        ss = warp_sum(ss);
+        if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = ss;
+        __syncthreads();
+        ss = 0.f;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) ss += ws[k];
+        r = rsqrtf(ss / (float) H + eps);
+    }
+    auto put = [&](int i, float4 q) {
+        if (norm_w) {
+            const float4 w = *reinterpret_cast<const float4*>(norm_w + i);
+            q.x *= w.x * r; q.y *= w.y * r; q.z *= w.z * r; q.w *= w.w * r;
+        }
+        const __half2 a = __floats2half2_rn(q.x, q.z), b = __floats2half2_rn(q.y, q.w);   // (pn_slot: 0, 2, 1, 3)
+        *reinterpret_cast<uint2*>(xh + (size_t) blockIdx.x * H + pn_slot(i)) = make_uint2(pn_h2(a), pn_h2(b));
+    };
+#pragma unroll
+    for (int j = 0; j < HOLD; ++j) {
+        const int i = (threadIdx.x + j * 256) * 4;
+        if (i < H) put(i, v[j]);
+    }
+    for (int i = (threadIdx.x + HOLD * 256) * 4; i < H; i += 1024) put(i, *reinterpret_cast<const float4*>(xr + i));
+}
+
+int prompt_nat_rows(const float* x, const float* norm_w, int T, int H, float eps, __half* xh, cudaStream_t st) {
+    k_prompt_nat_rows<<<T, 256, 0, st>>>(x, norm_w, H, eps, xh);
+    FNX_LAUNCH_OK("k_prompt_nat_rows");
+    return FNX_OK;
+}
+
+int prompt_nat(int mode, const PnParams& p, int max_jobs, cudaStream_t st) {
+    FNX_REQUIRE(p.K % 256 == 0 && p.rows % 16 == 0 && (mode == 0 || p.rows % 128 == 0), "prompt product: %d features x %d", p.rows, p.K);
+    auto kernel = mode == 1 ? k_prompt_nat<1> : k_prompt_nat<0>;
+    FNX_TRY(set_smem_limit((const void*) kernel, PN_SMEM));
+    const long long items = (long long) max_jobs * (mode == 1 ? p.rows / 128 : (p.rows + 255) / 256);
+    kernel<<<(unsigned) (items < sm_count() ? items : sm_count()), PN_THREADS, PN_SMEM, st>>>(p);
+    FNX_LAUNCH_OK("k_prompt_nat");
+    return FNX_OK;
+}
+
+}  // namespace fnxb

@@ -1,0 +1,47 @@
+// Prompt products from the engine's own weight layout (prompt_nat.cu).
+#pragma once
+
+#include <cuda_fp16.h>
+#include <cuda_runtime.h>
+
+#include <cstddef>
+#include <cstdint>
+
+namespace fnxb {
+
+// Activations of these products are f16 rows whose columns lie, within every 32, in the order that the weight words decode in: lane q of a
+// fragment row holds the columns 8 q .. 8 q + 7, column 8 q + j at slot 16 (j / 4) + 4 q + {0, 2, 1, 3}[j % 4].
+__host__ __device__ __forceinline__ int pn_slot(int c) {
+    const int j = c & 7, q = (c >> 3) & 3, k = j & 3;
+    return (c & ~31) + 16 * (j >> 2) + 4 * q + ((k & 1) << 1 | k >> 1);
+}
+
+constexpr int PN_N = 64;       // rows per job: the tensor core's N
+
+struct PnJob {
+    int w, n, start;           // expert (E: the shared one), rows, first entry of `order`
+};
+
+struct PnParams {
+    const uint8_t* W;          // expert matrices [e_base ..) (dense: one matrix)
+    size_t stride;
+    int e_base, E;
+    const uint8_t* Wsh;        // job.w >= E
+    const PnJob* jobs;         // null: a dense product over T rows
+    const int* njobs;
+    const int* order;          // per entry the pair t Kp + k; shared expert: TKp + t
+    int T, TKp, Kp;
+    const __half* x;           // gate|up, dense: [token][K]; down: [pair][K]
+    int rows, K;               // features (gate|up: F), inner dimension
+    float* out;                // down: [pair][rows]; dense: [token][ldo]
+    __half* outh;              // gate|up: [pair][F], in slot order
+    int ldo, accumulate;
+    unsigned* err;
+};
+
+// mode 1: outh = silu(x Wg^T) (x Wu^T); mode 0: out (+)= x W^T.  max_jobs: as many as there can be (jobs null: T rows)
+int prompt_nat(int mode, const PnParams& p, int max_jobs, cudaStream_t st);
+// xh[t] = f16(x[t] norm_w / rms(x[t])) in slot order (norm_w null: f16(x[t]))
+int prompt_nat_rows(const float* x, const float* norm_w, int T, int H, float eps, __half* xh, cudaStream_t st);
+
+}  // namespace fnxb
