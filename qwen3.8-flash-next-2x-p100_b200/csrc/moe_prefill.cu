@@ -799,7 +799,7 @@ int prompt_dense(const void* W, bool nat, int rows, int cols, const float* x, in
         FNX_TRY(prompt_nat_rows(x, norm_w, T, cols, eps, xh, st));
         PnParams q{};
         q.W = (const uint8_t*) W; q.T = T; q.x = xh; q.rows = rows; q.K = cols; q.out = y; q.ldo = ldy; q.accumulate = accumulate; q.err = err;
-        return prompt_nat(0, q, (T + PN_N - 1) / PN_N, st);
+        return prompt_nat(2, q, (T + PN_N - 1) / PN_N, st);
     }
     k_pf_xnorm<<<T, 256, 0, st>>>(x, norm_w, cols, eps, xh);
     FNX_LAUNCH_OK("k_pf_xnorm");

@@ -11,11 +11,11 @@
 // of 640).  Here
 //   - sixteen decode warps own a 16-row tile row each: 2,176-byte half tiles by their lanes' own async copies, four blocks ahead across
 //     items; nibbles to f16 with three shifts, four masks and twelve half operations a word of eight; the fragment layout is tcgen05.st's
-//     16x256b shape, so a chunk of 64 columns leaves as one store of sixteen registers;
-//   - two warps gather the job's live rows (a row of B only reaches its own column of D: the others stay what they are);
+//     16x256b shape, so 64 columns leave as one store of sixteen registers;
+//   - four warps gather the job's live rows (a row of B only reaches its own column of D: the others stay what they are);
 //   - one warp issues the products, one thread each, two accumulators (gate and up, or 2 x 128 features) double-buffered in tensor memory;
 //   - four warps write the item before.
-// Tensor memory: columns [0, 256) two pairs of accumulators, [256, 512) four stages of two 128 x 64 weight tiles.  Jobs have at most 64
+// Tensor memory: columns [0, 256) two pairs of accumulators, [256, 512) two stages of two 128 x 128 weight tiles.  Jobs have at most 64
 // rows: wider tiles pay off in the products only from some 100 rows an expert, by 20% of a bound that the decode then has alone.
 // Measured: see prompt_nat().
 #include "attn_tc.cuh"
@@ -24,15 +24,15 @@
 
 namespace fnxb {
 
-constexpr int PN_KC = 64;              // columns a stage
+constexpr int PN_KC = 128;             // columns a stage (64: every stage's waits and arrivals cost a few hundred cycles: 285 against 194 us for 513 jobs)
 constexpr int PN_DECODE = 16;          // warps
 constexpr int PN_EPI = 4, PN_LOAD = 2;
-constexpr int PN_W_EPI = PN_DECODE, PN_W_MMA = PN_W_EPI + PN_EPI, PN_W_LOAD = PN_W_MMA + 1;
-constexpr int PN_THREADS = (PN_W_LOAD + PN_LOAD) * 32;
+constexpr int PN_W_MMA = PN_EPI, PN_W_LOAD = PN_W_MMA + 1, PN_W_DECODE = 8;   // (warp 7 idles: the decode warps start at a multiple of four)
+constexpr int PN_THREADS = (PN_W_DECODE + PN_DECODE) * 32;
 constexpr int PN_SLOTS = 4;            // half tiles in flight a decode warp
-constexpr int PN_AST = 4, PN_BST = 8;  // stages of A (tensor memory) and of B (shared memory)
-constexpr int PN_LAG = 3;              // chunks of B in flight
-constexpr int PN_BBYTES = PN_N * 128;
+constexpr int PN_AST = 256 / PN_KC, PN_BST = 512 / PN_KC;  // stages of A (tensor memory) and of B (shared memory)
+constexpr int PN_LAG = 2;              // chunks of B in flight
+constexpr int PN_BBOX = PN_N * 128, PN_BBYTES = PN_KC / 64 * PN_BBOX;   // 64 rows x 64 columns, 128-byte swizzle
 constexpr int PN_RING = PN_DECODE * PN_SLOTS * NAT_HALF_BYTES;
 constexpr int PN_HEAD = 1024;
 constexpr int PN_SMEM = PN_HEAD + PN_BST * PN_BBYTES + PN_RING;
@@ -95,6 +95,7 @@ struct PnItem {
     int w, n, start, slab;
 };
 
+// MODE 1: gate|up, 0: down, 2: dense (any number of 16-row groups, sums)
 template <int MODE>
 __global__ void __launch_bounds__(PN_THREADS, 1) k_prompt_nat(const PnParams p) {
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -128,12 +129,12 @@ __global__ void __launch_bounds__(PN_THREADS, 1) k_prompt_nat(const PnParams p) 
     const uint32_t tmem = sh.tmem;
     const int KB = p.K / 256, nchunk = p.K / PN_KC;
     const int slabs = MODE == 1 ? p.rows / 128 : (p.rows + 255) / 256;
-    const int njobs = p.jobs ? *p.njobs : (p.T + PN_N - 1) / PN_N, total = njobs * slabs;
+    const int njobs = MODE != 2 ? *p.njobs : (p.T + PN_N - 1) / PN_N, total = njobs * slabs;
     auto job_of = [&](int it) {
         const int j = it / slabs;
         PnItem x;
         x.slab = it - j * slabs;
-        if (p.jobs) {
+        if (MODE != 2) {
             const PnJob jb = p.jobs[j];
             x.w = jb.w; x.n = jb.n; x.start = jb.start;
         } else {
@@ -142,20 +143,20 @@ __global__ void __launch_bounds__(PN_THREADS, 1) k_prompt_nat(const PnParams p) 
         return x;
     };
     bool ok = !sh.gave_up;
-    if (warp < PN_DECODE) {
+    if (warp >= PN_W_DECODE) {
         // ---------------------------------------------------------------------------------------- decode
         // tensor-memory lanes 32 (warp % 4) + 16 h of tile `mat`
-        const int lq = warp & 3, h = (warp >> 2) & 1, mat = warp >> 3;
-        const uint32_t t_lane = tmem + ((uint32_t) (32 * lq + 16 * h) << 16) + PN_A + mat * 32;
-        uint8_t* my = ring + warp * PN_SLOTS * NAT_HALF_BYTES;
+        const int dw = warp - PN_W_DECODE, lq = dw & 3, h = (dw >> 2) & 1, mat = dw >> 3;
+        const uint32_t t_lane = tmem + ((uint32_t) (32 * lq + 16 * h) << 16) + PN_A + mat * (PN_KC / 2);
+        uint8_t* my = ring + dw * PN_SLOTS * NAT_HALF_BYTES;
         const uint32_t my_s = smem_u32(my);
         const int n16 = (MODE == 1 ? 2 : 1) * (p.rows / 16);
         // the item's half tiles of this warp (null: past the matrix's last row)
-        auto expert_of = [&](int it) { return it < total && p.jobs ? p.jobs[it / slabs].w : 0; };
+        auto expert_of = [&](int it) { return it < total && MODE != 2 ? p.jobs[it / slabs].w : 0; };
         auto base_of = [&](int it, int e) -> const uint8_t* {
             const int slab = it % slabs, i = MODE == 1 ? mat * (p.rows / 16) + slab * 8 + lq * 2 + h : slab * 16 + mat * 8 + lq * 2 + h;
-            if (MODE == 0 && i >= n16) return nullptr;
-            const uint8_t* W = !p.jobs ? p.W : e >= p.E ? p.Wsh : p.W + (size_t) (e - p.e_base) * p.stride;
+            if (MODE == 2 && i >= n16) return nullptr;
+            const uint8_t* W = MODE == 2 ? p.W : e >= p.E ? p.Wsh : p.W + (size_t) (e - p.e_base) * p.stride;
             return W + nat_half_at((size_t) i, (size_t) n16, 0, (size_t) KB, MODE == 1) + lane * 16;
         };
         // the copies' cursor
@@ -186,7 +187,6 @@ __global__ void __launch_bounds__(PN_THREADS, 1) k_prompt_nat(const PnParams p) 
 #pragma unroll
         for (int i = 0; i < PN_SLOTS; ++i) fetch();
         int c = 0, slot = 0;   // chunks so far
-        bool pending = false;
         for (int it = blockIdx.x; it < total; it += gridDim.x) {
             for (int kb = 0; kb < KB; ++kb) {
                 asm volatile("cp.async.wait_group %0;" ::"n"(PN_SLOTS - 1) : "memory");
@@ -204,77 +204,82 @@ __global__ void __launch_bounds__(PN_THREADS, 1) k_prompt_nat(const PnParams p) 
                 fetch();
                 slot = slot + 1 == PN_SLOTS ? 0 : slot + 1;
 #pragma unroll
-                for (int Q = 0; Q < 4; ++Q, ++c) {
-                    uint32_t o[16];
-                    __half2 f00, f01, f10, f11;
-                    pn_scales(m.x, Q, d0, f00, f01);
-                    pn_scales(m.y, Q, d1, f10, f11);
-                    pn_decode8(w[0][2 * Q], f00, o[0], o[1], o[4], o[5]);
-                    pn_decode8(w[1][2 * Q], f10, o[2], o[3], o[6], o[7]);
-                    pn_decode8(w[0][2 * Q + 1], f01, o[8], o[9], o[12], o[13]);
-                    pn_decode8(w[1][2 * Q + 1], f11, o[10], o[11], o[14], o[15]);
-                    // the chunk before is in tensor memory by now (PN_AST and the chunks of a block are both 4: stage Q)
-                    if (pending) {
-                        ta_wait_st();
-                        ta_fence_before();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(&sh.full[(Q + 3) & 3]);
+                for (int st = 0; st < PN_AST; ++st, ++c) {
+#pragma unroll
+                    for (int q2 = 0; q2 < PN_KC / 64; ++q2) {
+                        const int Q = PN_KC / 64 * st + q2;
+                        uint32_t o[16];
+                        __half2 f00, f01, f10, f11;
+                        pn_scales(m.x, Q, d0, f00, f01);
+                        pn_scales(m.y, Q, d1, f10, f11);
+                        pn_decode8(w[0][2 * Q], f00, o[0], o[1], o[4], o[5]);
+                        pn_decode8(w[1][2 * Q], f10, o[2], o[3], o[6], o[7]);
+                        pn_decode8(w[0][2 * Q + 1], f01, o[8], o[9], o[12], o[13]);
+                        pn_decode8(w[1][2 * Q + 1], f11, o[10], o[11], o[14], o[15]);
+                        if (q2 == 0) {
+                            if (ok && c >= PN_AST) ok = __all_sync(0xffffffffu, pn_wait(&sh.empty[st], (unsigned) ((c / PN_AST - 1) & 1), sh));
+                            ta_fence_after();
+                        }
+                        pn_st_tile(t_lane + st * PN_KC + q2 * 32, o);
                     }
-                    if (ok && c >= PN_AST) ok = __all_sync(0xffffffffu, pn_wait(&sh.empty[Q], (unsigned) ((c / PN_AST - 1) & 1), sh));
-                    ta_fence_after();
-                    pn_st_tile(t_lane + Q * 64, o);
-                    pending = true;
+                    ta_wait_st();
+                    ta_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&sh.full[st]);
                 }
             }
         }
-        if (pending) {
-            ta_wait_st();
-            ta_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&sh.full[3]);
-        }
         asm volatile("cp.async.wait_group 0;" ::: "memory");
-    } else if (warp >= PN_W_LOAD) {
+    } else if (warp >= PN_W_LOAD && warp < PN_W_LOAD + PN_LOAD) {
         // ---------------------------------------------------------------------------------------- the rows
-        // thread: piece lt % 8 of the stage rows lt / 8 + 8 j
+        // thread: piece lt % 8 of the rows lt / 8 + 16 j, in both boxes of a stage.  Jobs and entries are loaded an item ahead, and a chunk
+        // is reported before the wait for the next one's stage, so that neither latency lies in the products' way.
+        constexpr int RJ = PN_N / (4 * PN_LOAD);
         const int lt = tid - PN_W_LOAD * 32, piece = lt & 7, r0 = lt >> 3;
-        const uint32_t b_s = smem_u32(Bs) + r0 * 128 + ((piece ^ (r0 & 7)) * 16);   // (r0 + 8 j has the same low bits)
+        const uint32_t b_s = smem_u32(Bs) + r0 * 128 + ((piece ^ (r0 & 7)) * 16);   // (r0 + 16 j has the same low bits)
         int c = 0;
         auto landed = [&](int chunk) {
             fence_proxy_async();
             __syncwarp();
             if (lane == 0) mbar_arrive(&sh.bfull[chunk % PN_BST]);
         };
-        for (int it = blockIdx.x; it < total; it += gridDim.x) {
-            const PnItem x = job_of(it);
-            const __half* src[PN_N / 8];
+        PnItem x = job_of(min((int) blockIdx.x, total - 1)), nx;
+        int e[RJ];   // the item's entries
+        auto entries = [&](const PnItem& y) {
 #pragma unroll
-            for (int j = 0; j < PN_N / 8; ++j) {
-                const int r = r0 + 8 * j;
-                src[j] = nullptr;
-                if (r < x.n) {
-                    int row = x.start + r;
-                    if (p.jobs) {
-                        row = p.order[row];
-                        if (MODE == 1) row = row >= p.TKp ? row - p.TKp : row / p.Kp;
-                    }
-                    src[j] = p.x + (size_t) row * p.K + piece * 8;
-                }
+            for (int j = 0; j < RJ; ++j) e[j] = MODE != 2 ? p.order[y.start + min(r0 + 4 * PN_LOAD * j, y.n - 1)] : y.start + r0 + 4 * PN_LOAD * j;
+        };
+        entries(x);
+        for (int it = blockIdx.x; it < total; it += gridDim.x) {
+            const __half* src[RJ];
+#pragma unroll
+            for (int j = 0; j < RJ; ++j) {
+                int row = e[j];
+                if (MODE == 1) row = row >= p.TKp ? row - p.TKp : row / p.Kp;
+                src[j] = r0 + 4 * PN_LOAD * j < x.n ? p.x + (size_t) row * p.K + piece * 8 : nullptr;
             }
+            const bool more = it + (int) gridDim.x < total;
+            if (more) nx = job_of(it + gridDim.x);
             for (int k = 0; k < nchunk; ++k, ++c) {
+                if (c >= PN_LAG) {
+                    asm volatile("cp.async.wait_group %0;" ::"n"(PN_LAG - 1) : "memory");
+                    landed(c - PN_LAG);
+                }
                 if (ok && c >= PN_BST) ok = __all_sync(0xffffffffu, pn_wait(&sh.bempty[c % PN_BST], (unsigned) ((c / PN_BST - 1) & 1), sh));
                 if (ok) {
                     const uint32_t dst = b_s + (c % PN_BST) * PN_BBYTES;
 #pragma unroll
-                    for (int j = 0; j < PN_N / 8; ++j)
-                        if (src[j]) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + j * 1024), "l"(src[j] + k * PN_KC) : "memory");
+                    for (int j = 0; j < RJ; ++j)
+                        if (src[j]) {
+                            const __half* g = src[j] + k * PN_KC;
+                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + j * (512 * PN_LOAD)), "l"(g) : "memory");
+                            if (PN_KC == 128) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + PN_BBOX + j * (512 * PN_LOAD)), "l"(g + 64) : "memory");
+                        }
                 }
                 asm volatile("cp.async.commit_group;" ::: "memory");
-                if (c >= PN_LAG) {
-                    asm volatile("cp.async.wait_group %0;" ::"n"(PN_LAG) : "memory");
-                    landed(c - PN_LAG);
-                }
+                if (k == 0 && more) entries(nx);
             }
+            x = nx;
         }
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         for (int i = max(0, c - PN_LAG); i < c; ++i) landed(i);
@@ -282,70 +287,82 @@ __global__ void __launch_bounds__(PN_THREADS, 1) k_prompt_nat(const PnParams p) 
         // ---------------------------------------------------------------------------------------- the products
         constexpr uint32_t IDESC = (1u << 4) | ((uint32_t) (PN_N >> 3) << 17) | ((uint32_t) (128 >> 4) << 24);
         const uint32_t b_s = smem_u32(Bs);
-        int c = 0, nit = 0;
-        for (int it = blockIdx.x; it < total; it += gridDim.x, ++nit) {
-            const int buf = nit & 1;
-            const uint32_t acc = tmem + buf * PN_ACC;
-            if (ok && nit >= 2) ok = __all_sync(0xffffffffu, pn_wait(&sh.acc_empty[buf], (unsigned) ((nit / 2 - 1) & 1), sh));
-            for (int k = 0; k < nchunk; ++k, ++c) {
-                if (ok) ok = __all_sync(0xffffffffu, pn_wait(&sh.bfull[c % PN_BST], (unsigned) ((c / PN_BST) & 1), sh));
-                if (ok) ok = __all_sync(0xffffffffu, pn_wait(&sh.full[c % PN_AST], (unsigned) ((c / PN_AST) & 1), sh));
-                if (ok && ta_elect()) {
+        // (one thread all through: among sixteen decoding warps every instruction of this one is paid five or six times)
+        if (ta_elect()) {
+            int c = 0, nit = 0;
+            for (int it = blockIdx.x; it < total && ok; it += gridDim.x, ++nit) {
+                const int buf = nit & 1;
+                const uint32_t acc = tmem + buf * PN_ACC;
+                if (nit >= 2) ok = pn_wait(&sh.acc_empty[buf], (unsigned) ((nit / 2 - 1) & 1), sh);
+                for (int k = 0; k < nchunk && ok; ++k, ++c) {
+                    ok = pn_wait(&sh.bfull[c % PN_BST], (unsigned) ((c / PN_BST) & 1), sh) && pn_wait(&sh.full[c % PN_AST], (unsigned) ((c / PN_AST) & 1), sh);
+                    if (!ok) break;
                     ta_fence_after();
-                    const uint32_t a_t = tmem + PN_A + (c % PN_AST) * 64, b = b_s + (c % PN_BST) * PN_BBYTES;
+                    const uint32_t a_t = tmem + PN_A + (c % PN_AST) * PN_KC, b = b_s + (c % PN_BST) * PN_BBYTES;
 #pragma unroll
                     for (int k16 = 0; k16 < PN_KC / 16; ++k16) {
-                        const uint64_t bd = ta_desc_sw(b + k16 * 32, 16, 1024);
+                        const uint64_t bd = ta_desc_sw(b + (k16 >> 2) * PN_BBOX + (k16 & 3) * 32, 16, 1024);
                         ta_mma_ta(acc, a_t + k16 * 8, bd, IDESC, (k | k16) != 0);
-                        ta_mma_ta(acc + PN_N, a_t + 32 + k16 * 8, bd, IDESC, (k | k16) != 0);
+                        ta_mma_ta(acc + PN_N, a_t + PN_KC / 2 + k16 * 8, bd, IDESC, (k | k16) != 0);
                     }
                     ta_commit(&sh.empty[c % PN_AST]);
                     ta_commit(&sh.bempty[c % PN_BST]);
                     if (k == nchunk - 1) ta_commit(&sh.acc_full[buf]);
                 }
-                __syncwarp();
+            }
+            if (ok && c > 0) {   // the last arrivals, before the shared memory goes
+                pn_wait(&sh.empty[(c - 1) % PN_AST], (unsigned) (((c - 1) / PN_AST) & 1), sh);
+                pn_wait(&sh.bempty[(c - 1) % PN_BST], (unsigned) (((c - 1) / PN_BST) & 1), sh);
             }
         }
-        if (ok && c > 0) {   // the last arrivals, before the shared memory goes
-            pn_wait(&sh.empty[(c - 1) % PN_AST], (unsigned) (((c - 1) / PN_AST) & 1), sh);
-            pn_wait(&sh.bempty[(c - 1) % PN_BST], (unsigned) (((c - 1) / PN_BST) & 1), sh);
-        }
-    } else {
+        __syncwarp();
+    } else if (warp < PN_EPI) {
         // ---------------------------------------------------------------------------------------- the results
         const int lq = warp & 3;
         const uint32_t lane_base = (uint32_t) (32 * lq) << 16;
+        const int ldo = MODE == 1 ? p.rows : p.ldo;
         int nit = 0;
         for (int it = blockIdx.x; it < total; it += gridDim.x, ++nit) {
             const PnItem x = job_of(it);
             const int buf = nit & 1;
+            int e0 = x.start + min(lane, x.n - 1), e1 = x.start + min(lane + 32, x.n - 1);   // the item's output rows, two a lane
+            if (MODE != 2) {
+                e0 = p.order[e0];
+                e1 = p.order[e1];
+            }
             if (ok) ok = __all_sync(0xffffffffu, pn_wait(&sh.acc_full[buf], (unsigned) ((nit / 2) & 1), sh));
             ta_fence_after();
             if (ok) {
                 const uint32_t acc = tmem + buf * PN_ACC + lane_base;
+                const int f = MODE == 1 ? x.slab * 128 + lq * 32 + pn_slot(lane) : x.slab * 256 + lq * 32 + lane;
+                const bool in0 = f < p.rows, in1 = f + 128 < p.rows;
 #pragma unroll 1
                 for (int c0 = 0; c0 < x.n; c0 += 16) {
-                    const int e = min(c0 + (lane & 15), x.n - 1) + x.start, mine = p.jobs ? p.order[e] : e;
-                    float g[16], u[16];
+                    const int mine = c0 < 32 ? e0 : e1;
+                    float g[16], u[16], old0[MODE == 2 ? 16 : 1], old1[MODE == 2 ? 16 : 1];
+                    if (MODE == 2) {
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) {
+                            const size_t o = (size_t) __shfl_sync(0xffffffffu, mine, (c0 & 16) + i) * ldo + f;
+                            old0[i] = p.accumulate && in0 && c0 + i < x.n ? p.out[o] : 0.f;
+                            old1[i] = p.accumulate && in1 && c0 + i < x.n ? p.out[o + 128] : 0.f;
+                        }
+                    }
                     ta_ld16(acc + c0, g);
                     ta_ld16(acc + PN_N + c0, u);
                     ta_wait_ld(g, u);
-                    if (MODE == 1) {
-                        __half* o = p.outh + x.slab * 128 + lq * 32 + pn_slot(lane);
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) {
-                            const int row = __shfl_sync(0xffffffffu, mine, i);
-                            if (c0 + i < x.n) o[(size_t) row * p.rows] = __float2half_rn(siluf_(g[i]) * u[i]);
-                        }
-                    } else {
-                        const int f = x.slab * 256 + lq * 32 + lane;
-                        const bool in0 = f < p.rows, in1 = f + 128 < p.rows;
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) {
-                            const int row = __shfl_sync(0xffffffffu, mine, i);
-                            if (c0 + i < x.n) {
-                                float* o = p.out + (size_t) row * p.ldo + f;
-                                if (in0) o[0] = p.accumulate ? o[0] + g[i] : g[i];
-                                if (in1) o[128] = p.accumulate ? o[128] + u[i] : u[i];
+                    for (int i = 0; i < 16; ++i) {
+                        const size_t o = (size_t) __shfl_sync(0xffffffffu, mine, (c0 & 16) + i) * ldo + f;
+                        if (c0 + i < x.n) {
+                            // (rounded to f16: the hardware's exponential and division are far inside that)
+                            if (MODE == 1) p.outh[o] = __float2half_rn(__fdividef(g[i], 1.0f + __expf(-g[i])) * u[i]);
+                            else if (MODE == 0) {
+                                __stcs(p.out + o, g[i]);
+                                __stcs(p.out + o + 128, u[i]);
+                            } else {
+                                if (in0) p.out[o] = old0[i] + g[i];
+                                if (in1) p.out[o + 128] = old1[i] + u[i];
                             }
                         }
                     }
@@ -411,8 +428,8 @@ int prompt_nat_rows(const float* x, const float* norm_w, int T, int H, float eps
 }
 
 int prompt_nat(int mode, const PnParams& p, int max_jobs, cudaStream_t st) {
-    FNX_REQUIRE(p.K % 256 == 0 && p.rows % 16 == 0 && (mode == 0 || p.rows % 128 == 0), "prompt product: %d features x %d", p.rows, p.K);
-    auto kernel = mode == 1 ? k_prompt_nat<1> : k_prompt_nat<0>;
+    FNX_REQUIRE(p.K % 256 == 0 && p.rows % (mode == 2 ? 16 : mode == 1 ? 128 : 256) == 0, "prompt product: %d features x %d", p.rows, p.K);
+    auto kernel = mode == 1 ? k_prompt_nat<1> : mode == 0 ? k_prompt_nat<0> : k_prompt_nat<2>;
     FNX_TRY(set_smem_limit((const void*) kernel, PN_SMEM));
     const long long items = (long long) max_jobs * (mode == 1 ? p.rows / 128 : (p.rows + 255) / 256);
     kernel<<<(unsigned) (items < sm_count() ? items : sm_count()), PN_THREADS, PN_SMEM, st>>>(p);

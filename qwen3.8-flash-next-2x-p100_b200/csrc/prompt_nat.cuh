@@ -27,7 +27,7 @@ struct PnParams {
     size_t stride;
     int e_base, E;
     const uint8_t* Wsh;        // job.w >= E
-    const PnJob* jobs;         // null: a dense product over T rows
+    const PnJob* jobs;         // (dense: the T rows in order)
     const int* njobs;
     const int* order;          // per entry the pair t Kp + k; shared expert: TKp + t
     int T, TKp, Kp;
@@ -39,7 +39,8 @@ struct PnParams {
     unsigned* err;
 };
 
-// mode 1: outh = silu(x Wg^T) (x Wu^T); mode 0: out (+)= x W^T.  max_jobs: as many as there can be (jobs null: T rows)
+// mode 1: outh = silu(x Wg^T) (x Wu^T); mode 0: out = x W^T over the jobs' pairs; mode 2: out (+)= x W^T over T rows.  max_jobs: as many
+// as there can be
 int prompt_nat(int mode, const PnParams& p, int max_jobs, cudaStream_t st);
 // xh[t] = f16(x[t] norm_w / rms(x[t])) in slot order (norm_w null: f16(x[t]))
 int prompt_nat_rows(const float* x, const float* norm_w, int T, int H, float eps, __half* xh, cudaStream_t st);
