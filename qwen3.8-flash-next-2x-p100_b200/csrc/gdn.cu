@@ -313,160 +313,296 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(GDN_THREADS, 2)
 
 // ------------------------------------------------------------------------------------------------ prompts
 // A prompt's rows are a chain of which every row is kept, so the work splits by what depends on what (gdn_prompt,
-// engine/src/kernels.cu:2158): conv + SiLU, the q / k norms and the gates of every row at once (k_gdn_pre); the delta rule, the
-// only sequential part, with the state in registers from the first row to the last and the rows' q, k, v streamed through
-// shared memory (k_gdn_scan); the gated RMS norm of every row at once (k_gdn_post).  Only the last row's state and the last
-// three rows' conv inputs are written back.
+// engine/src/kernels.cu:2158): conv + SiLU, the q / k norms, the gates and what of the rule does not involve the state, for every group
+// of eight rows at once (k_gdn_pre); the delta rule, the only sequential part, with the state in registers from the first row to the last
+// (k_gdn_scan); the gated RMS norm of every row at once (k_gdn_post).  Only the last row's state and the last three rows' conv inputs are
+// written back.
+//
+// Row by row, the rule is  S <- g S,  d = beta (v - S' k),  S <- S + k d',  o = S' q / sqrt(128).  Over the rows i = 0 .. 7 of a group
+// that starts from S, with b_i = g_0 .. g_i and r_ij = g_(j+1) .. g_i:
+//   (I + L) d = w,  w_i = beta_i v_i - beta_i b_i (S' k_i),  L_ij = beta_i r_ij (k_i . k_j), j < i
+//   o_i = (b_i (S' q_i) + sum_(j <= i) r_ij (q_i . k_j) d_j) / sqrt(128)
+//   S  <- b_7 S + sum_j r_7j k_j d_j'
+// so the state is read for all eight rows at once and updated once; (I + L)^-1, which does not involve it, is applied to the k of the update
+// beforehand:  sum_j r_7j k_j d_j' = sum_l c_l w_l',  c_l = sum_j r_7j ((I + L)^-1)_jl k_j.  All in f32.
 constexpr int GDP_THREADS = 256;
+constexpr int GDP_ROWS = 8;
+// a group's coefficients for a value head: beta, beta b, b / sqrt(128) [8 each]; b_7; what of o comes from w [8][8]
+constexpr int GC_BV = 0, GC_BK = 8, GC_BQ = 16, GC_BC = 24, GC_M = 28, GC_FLOATS = 92;
 
-// block = one row; thread = channels tid, tid + 256, ...  xq / xk [T][nk][HS], xv [T][nv][HS], gates [T][nv][2]
+// grid (groups, key heads + pairs of value heads): a key head's q and k, its dots, and its value heads' coefficients and c; or 256 channels
+// of v.  Rows past T become zeros (their coefficients leave the state as it is).  xq / xk [8 groups][nk][HS], xv / xc [..][nv][HS].
+// Bound by its reads and writes; a row's inputs are read by one block, eight rows and three before them at a time.
 __global__ void __launch_bounds__(GDP_THREADS) k_gdn_pre(const float* __restrict__ qkvz, int stride, const float* __restrict__ ab, int ldab,
                                                          const float* __restrict__ hin, float* __restrict__ hout, const float* __restrict__ convw,
                                                          const float* __restrict__ dt, const float* __restrict__ a_, float* __restrict__ xq,
-                                                         float* __restrict__ xk, float* __restrict__ xv, float* __restrict__ gates, int nk, int nv, int T) {
-    __shared__ float red[GDP_THREADS / 32];
-    const int t = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int ch = (2 * nk + nv) * GDN_HS;
-    // row t - k of the chain: a row of this call, or the history the call starts from (rows 0..2, oldest first)
-    auto xrow = [&](int r, int c) { return r >= 0 ? qkvz[(size_t) r * stride + c] : hin[(size_t) (3 + r) * ch + c]; };
-    for (int c0 = 0; c0 < ch; c0 += GDP_THREADS) {
-        const int c = c0 + tid;
-        const float4 cw = *reinterpret_cast<const float4*>(convw + (size_t) c * 4);
-        const float x3 = xrow(t - 3, c), x2 = xrow(t - 2, c), x1 = xrow(t - 1, c), x0 = xrow(t, c);
-        const float x = cw.x * x3 + cw.y * x2 + cw.z * x1 + cw.w * x0;
-        float v = x / (1.0f + expf(-x));
-        if (t == T - 1) {   // the history the next call starts from
-            hout[c] = x2;
-            hout[ch + c] = x1;
-            hout[2 * ch + c] = x0;
-        }
-        if (c < 2 * nk * GDN_HS) {
-            // q and k heads: the L2 norm over the head's 128 channels = four warps of this pass (two heads per pass)
-            const float sq = warp_sum(v * v);
-            __syncthreads();
-            if (lane == 0) red[warp] = sq;
-            __syncthreads();
-            const int w0 = warp & ~3;
-            float ssum = 0.f;
-            for (int w = 0; w < 4; ++w) ssum += red[w0 + w];
-            v *= rsqrtf(ssum + 1e-6f);
-            if (c < nk * GDN_HS) xq[(size_t) t * nk * GDN_HS + c] = v;
-            else xk[(size_t) t * nk * GDN_HS + (c - nk * GDN_HS)] = v;
-        } else {
-            xv[(size_t) t * nv * GDN_HS + (c - 2 * nk * GDN_HS)] = v;
+                                                         float* __restrict__ xk, float* __restrict__ xv, float* __restrict__ xc, float* __restrict__ coef, int nk, int nv,
+                                                         int T) {
+    constexpr int R = GDP_ROWS, HS = GDN_HS, LD = HS + 16;   // (16 banks between neighbouring rows)
+    __shared__ __align__(16) float qs[R][LD], ks[R][LD];
+    __shared__ float red[GDP_THREADS / 32][R], kk[R][R], qk[R][R], sg[2][R], sb[2][R], Lm[2][R][R], Qm[2][R][R], Ti[2][R][R];
+    const int t0 = blockIdx.x * R, y = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int ch = (2 * nk + nv) * HS, el = tid & (HS - 1), hf = tid / HS;
+    const int c = y < nk ? hf * nk * HS + y * HS + el : 2 * nk * HS + (y - nk) * GDP_THREADS + tid;
+    const float4 cw = *reinterpret_cast<const float4*>(convw + (size_t) c * 4);
+    float x[R + 3], v[R];   // rows t0 - 3 ..: of this call, or the history it starts from (rows 0..2, oldest first)
+#pragma unroll
+    for (int i = 0; i < R + 3; ++i) {
+        const int r = t0 - 3 + i;
+        x[i] = r < 0 ? hin[(size_t) (3 + r) * ch + c] : r < T ? qkvz[(size_t) r * stride + c] : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        const float s = cw.x * x[i] + cw.y * x[i + 1] + cw.z * x[i + 2] + cw.w * x[i + 3];
+        v[i] = t0 + i < T ? s / (1.0f + expf(-s)) : 0.f;
+    }
+    if (t0 + R >= T) {   // the history the next call starts from: rows T - 3 .. T - 1
+#pragma unroll
+        for (int i = 1; i < R + 3; ++i) {
+            const int k = t0 - 3 + i - (T - 3);
+            if (k >= 0 && k < 3) hout[(size_t) k * ch + c] = x[i];
         }
     }
-    if (tid < nv) {
-        const float* abt = ab + (size_t) t * ldab;
-        const float x = abt[tid] + dt[tid];
-        gates[((size_t) t * nv + tid) * 2] = expf((x > 20.0f ? x : log1pf(expf(x))) * a_[tid]);
-        gates[((size_t) t * nv + tid) * 2 + 1] = 1.0f / (1.0f + expf(-abt[nv + tid]));
+    if (y >= nk) {
+        float* dst = xv + (size_t) t0 * nv * HS + (y - nk) * GDP_THREADS + tid;
+#pragma unroll
+        for (int i = 0; i < R; ++i) dst[(size_t) i * nv * HS] = v[i];
+        return;
+    }
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        const float sq = warp_sum(v[i] * v[i]);
+        if (lane == 0) red[warp][i] = sq;
+    }
+    __syncthreads();
+    {
+        float* dst = (hf ? xk : xq) + ((size_t) t0 * nk + y) * HS + el;
+        float (*own)[LD] = hf ? ks : qs;
+        const int w0 = warp & ~3;
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const float n = v[i] * rsqrtf(((red[w0][i] + red[w0 + 1][i]) + red[w0 + 2][i]) + red[w0 + 3][i] + 1e-6f);
+            dst[(size_t) i * nk * HS] = n;
+            own[i][el] = n;
+        }
+    }
+    __syncthreads();
+    {   // four threads a pair of rows
+        const int i = tid >> 5, j = (tid >> 2) & 7, e0 = (tid & 3) * 4;
+        float dk = 0.f, dq = 0.f;
+#pragma unroll
+        for (int m = 0; m < HS / 16; ++m) {
+            const float4 a = *reinterpret_cast<const float4*>(&ks[i][e0 + 16 * m]), b = *reinterpret_cast<const float4*>(&qs[i][e0 + 16 * m]),
+                         k = *reinterpret_cast<const float4*>(&ks[j][e0 + 16 * m]);
+            dk = fmaf(a.x, k.x, fmaf(a.y, k.y, fmaf(a.z, k.z, fmaf(a.w, k.w, dk))));
+            dq = fmaf(b.x, k.x, fmaf(b.y, k.y, fmaf(b.z, k.z, fmaf(b.w, k.w, dq))));
+        }
+#pragma unroll
+        for (int o = 1; o < 4; o <<= 1) {
+            dk += __shfl_xor_sync(0xffffffffu, dk, o);
+            dq += __shfl_xor_sync(0xffffffffu, dq, o);
+        }
+        if ((tid & 3) == 0) {
+            kk[i][j] = dk;
+            qk[i][j] = dq;
+        }
+    }
+    const float scale = rsqrtf((float) HS);
+    const int ti = (el >> 3) & 7, tj = el & 7;
+    for (int lv0 = y; lv0 < nv; lv0 += 2 * nk) {   // the key head's value heads, one a half block
+        const int lv = lv0 + hf * nk;
+        const bool on = lv < nv;
+        if (on && el < R) {
+            const int t = t0 + el;
+            const float* abt = ab + (size_t) t * ldab;
+            float g = 1.f, b = 0.f;
+            if (t < T) {
+                const float p = abt[lv] + dt[lv];
+                g = expf((p > 20.0f ? p : log1pf(expf(p))) * a_[lv]);
+                b = 1.0f / (1.0f + expf(-abt[nv + lv]));
+            }
+            sg[hf][el] = g;
+            sb[hf][el] = b;
+        }
+        __syncthreads();
+        auto prod = [&](int a, int b) {   // g_a .. g_b
+            float p = 1.f;
+            for (int l = a; l <= b; ++l) p *= sg[hf][l];
+            return p;
+        };
+        if (on && el < 64) {
+            const float r = tj <= ti ? prod(tj + 1, ti) : 0.f;
+            Lm[hf][ti][tj] = tj < ti ? sb[hf][ti] * r * kk[ti][tj] : 0.f;
+            Qm[hf][ti][tj] = tj <= ti ? scale * r * qk[ti][tj] : 0.f;
+        }
+        __syncthreads();
+        if (on && el < R) {   // column el of the inverse
+            float t[R];
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                float a = i == el ? 1.f : 0.f;
+#pragma unroll
+                for (int j = 0; j < i; ++j) a = fmaf(-Lm[hf][i][j], t[j], a);
+                t[i] = i < el ? 0.f : a;
+                Ti[hf][i][el] = t[i];
+            }
+        }
+        __syncthreads();
+        if (on) {
+            float* dst = coef + ((size_t) blockIdx.x * nv + lv) * GC_FLOATS;
+            if (el < 64) {
+                float m = 0.f;
+#pragma unroll
+                for (int j = 0; j < R; ++j) m = fmaf(Qm[hf][ti][j], Ti[hf][j][tj], m);
+                dst[GC_M + el] = m;
+            } else if (el < 64 + GC_M) {
+                const int u = el - 64, i = u & 7;
+                dst[u] = u < GC_BK ? sb[hf][i] : u < GC_BQ ? sb[hf][i] * prod(0, i) : u < GC_BC ? scale * prod(0, i) : u == GC_BC ? prod(0, R - 1) : 0.f;
+            }
+            float cl[R], e = 1.f;
+#pragma unroll
+            for (int l = 0; l < R; ++l) cl[l] = 0.f;
+#pragma unroll
+            for (int j = R - 1; j >= 0; --j) {   // e = r_7j
+                const float k = e * ks[j][el];
+#pragma unroll
+                for (int l = 0; l <= j; ++l) cl[l] = fmaf(Ti[hf][j][l], k, cl[l]);
+                e *= sg[hf][j];
+            }
+            float* cd = xc + ((size_t) t0 * nv + lv) * HS + el;
+#pragma unroll
+            for (int l = 0; l < R; ++l) cd[(size_t) l * nv * HS] = cl[l];
+        }
+        __syncthreads();
     }
 }
 
-// block = (value head, column quarter) as in the window kernel: warp `part` holds key rows [32 part, +32) of the block's 32 value
-// columns, lane = column.  Rows stream through two shared-memory tiles of GDS_ROWS rows.
-constexpr int GDS_ROWS = 16;
-__global__ void __launch_bounds__(GDS_THREADS) k_gdn_scan(const float* __restrict__ xq, const float* __restrict__ xk, const float* __restrict__ xv,
-                                                          const float* __restrict__ gates, const float* __restrict__ S_in, float* __restrict__ S_out,
-                                                          float* __restrict__ o, int nk, int nv, int T) {
-    constexpr int ROWF = 2 * GDN_HS + GDN_QC + 2;   // floats of a staged row: k, q, the block's v, the two gates
-    __shared__ __align__(16) float tile[2][GDS_ROWS][ROWF + 2];
-    __shared__ float kred[2][4][GDN_QC], ared[GDS_ROWS][4][GDN_QC];
-    const int lv = blockIdx.x / GDN_Q, qq = blockIdx.x % GDN_Q, kh = lv % nk, tid = threadIdx.x;
-    const int part = tid >> 5, lane = tid & 31, col = qq * GDN_QC + lane;
-    const size_t soff = (size_t) lv * GDN_HS * GDN_HS + (size_t) part * 32 * GDN_HS + col;
-    uint64_t s[16];   // the thread's 32 state values, in pairs (rows 2 i, 2 i + 1)
+// block = (value head, 16 columns), two to an SM so that one's loads and barriers pass while the other works: a warp holds 32 key rows
+// of the state in registers, lane = 8 of them (lane / 8) x two columns.  Bound by instructions (some 430 a warp and group) and the
+// shared memory's rate: k, q and c are broadcast, two columns a lane halve their loads; then by the chain partial sums -> sums -> w ->
+// state between two barriers.  Row by row that chain took 560 cycles a row.  Groups come through three stages of shared memory.
+constexpr int GDS_COLS = 16, GDS_STAGES = 3, GDS_PARTS = 2 * GDS_THREADS / 32, GDS_PART = 2 * GDP_ROWS * GDS_COLS + GDS_COLS;   // (the parts 16 banks apart)
+constexpr int GDS_K = 0, GDS_QO = GDP_ROWS * GDN_HS, GDS_CO = 2 * GDS_QO, GDS_V = 3 * GDS_QO, GDS_C = GDS_V + GDP_ROWS * GDS_COLS, GDS_STAGE = GDS_C + GC_FLOATS;   // floats
+constexpr int GDS_SMEM = (GDS_STAGES * GDS_STAGE + GDS_PARTS * GDS_PART + 4 * GDP_ROWS * GDS_COLS) * (int) sizeof(float);
+__global__ void __launch_bounds__(GDS_THREADS, 2) k_gdn_scan(const float* __restrict__ xq, const float* __restrict__ xk, const float* __restrict__ xv,
+                                                             const float* __restrict__ xc, const float* __restrict__ coef, const float* __restrict__ S_in,
+                                                             float* __restrict__ S_out, float* __restrict__ o, int nk, int nv, int T) {
+    constexpr int R = GDP_ROWS, HS = GDN_HS, C = GDS_COLS, SL = HS / C;
+    extern __shared__ __align__(16) float gds[];
+    float* red = gds + GDS_STAGES * GDS_STAGE;             // [parts][k sums, q sums of 8 rows][columns]
+    float* ws = red + GDS_PARTS * GDS_PART;                // [8][columns]
+    float2* w2 = reinterpret_cast<float2*>(ws + R * C);    // [2][8][columns / 2]: a lane's two columns, the one whose sums it keeps first
+    const int lv = blockIdx.x / SL, col0 = blockIdx.x % SL * C, kh = lv % nk, tid = threadIdx.x;
+    const int warp = tid >> 5, lane = tid & 31, cp = lane & 7, up = lane >> 4, ng = (T + R - 1) / R;
+    const int key0 = warp * 32 + (lane >> 3) * 8, keep = cp + 8 * up, part = warp * 2 + ((lane >> 3) & 1);
+    const int row = tid / C, col = tid % C;                // of the sums that the thread completes
+    const size_t soff = (size_t) lv * HS * HS + (size_t) key0 * HS + col0;
+    uint64_t s[2][4];   // the thread's 16 state values: its column `keep` and the other, key rows (2 i, 2 i + 1)
 #pragma unroll
-    for (int r = 0; r < 32; r += 2) s[r / 2] = f2_pack(S_in[soff + (size_t) r * GDN_HS], S_in[soff + (size_t) (r + 1) * GDN_HS]);
-    auto stage = [&](int buf, int t0) {
-        const int nr = min(GDS_ROWS, T - t0);
-        for (int i = tid; i < nr * (ROWF / 2); i += GDS_THREADS) {   // 8-byte pieces
-            const int r = i / (ROWF / 2), e = (i % (ROWF / 2)) * 2, t = t0 + r;
-            const float* src;
-            if (e < GDN_HS) src = xk + ((size_t) t * nk + kh) * GDN_HS + e;
-            else if (e < 2 * GDN_HS) src = xq + ((size_t) t * nk + kh) * GDN_HS + (e - GDN_HS);
-            else if (e < 2 * GDN_HS + GDN_QC) src = xv + ((size_t) t * nv + lv) * GDN_HS + qq * GDN_QC + (e - 2 * GDN_HS);
-            else src = gates + ((size_t) t * nv + lv) * 2;
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(&tile[buf][r][e])), "l"(src) : "memory");
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) s[c][i] = f2_pack(S_in[soff + (size_t) (2 * i) * HS + (keep ^ (8 * c))], S_in[soff + (size_t) (2 * i + 1) * HS + (keep ^ (8 * c))]);
+    // the thread's 16-byte pieces of a stage: a piece of two rows of k, q and c each, and a few of v and the coefficients
+    const int pr = tid >> 5, pe = lane * 4;
+    const uint32_t tile_s = smem_u32(gds) + tid * 16;
+    const float* gk = xk + ((size_t) pr * nk + kh) * HS + pe;
+    const float* gq = xq + ((size_t) pr * nk + kh) * HS + pe;
+    const float* gc = xc + ((size_t) pr * nv + lv) * HS + pe;
+    const float* gv = tid < R * C / 4 ? xv + ((size_t) (tid / (C / 4)) * nv + lv) * HS + col0 + tid % (C / 4) * 4 : coef + (size_t) lv * GC_FLOATS + (tid - R * C / 4) * 4;
+    const size_t kstep = (size_t) R * nk * HS, cstep = (size_t) R * nv * HS, vstep = tid < R * C / 4 ? cstep : (size_t) nv * GC_FLOATS;
+    const bool has_v = tid < R * C / 4 + GC_FLOATS / 4;
+    auto cp16 = [](uint32_t dst, const float* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); };
+    auto stage = [&](int g) {
+        if (g < ng) {
+            const uint32_t d = tile_s + g % GDS_STAGES * (GDS_STAGE * 4);
+            cp16(d, gk); cp16(d + 2048, gk + (size_t) 4 * nk * HS);
+            cp16(d + GDS_QO * 4, gq); cp16(d + GDS_QO * 4 + 2048, gq + (size_t) 4 * nk * HS);
+            cp16(d + GDS_CO * 4, gc); cp16(d + GDS_CO * 4 + 2048, gc + (size_t) 4 * nv * HS);
+            if (has_v) cp16(d + GDS_V * 4, gv);
+            gk += kstep; gq += kstep; gc += cstep; gv += vstep;
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    const float scale = rsqrtf((float) GDN_HS);
-    stage(0, 0);
-    int buf = 0;
-    for (int t0 = 0; t0 < T; t0 += GDS_ROWS, buf ^= 1) {
-        const int nr = min(GDS_ROWS, T - t0);
-        if (t0 + GDS_ROWS < T) {
-            stage(buf ^ 1, t0 + GDS_ROWS);   // (its last readers passed the barrier that ended the previous tile)
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
+    static_assert(GDS_THREADS == GDP_ROWS * GDS_COLS && GDS_THREADS * 4 == 4 * GDN_HS && GDS_C == GDS_V + GDP_ROWS * GDS_COLS, "the pieces above");
+#pragma unroll
+    for (int g = 0; g < GDS_STAGES - 1; ++g) stage(g);
+    asm volatile("cp.async.wait_group %0;" ::"n"(GDS_STAGES - 2) : "memory");
+    __syncthreads();
+    float* od = o + ((size_t) row * nv + lv) * HS + col0 + col;
+    const size_t ostep = (size_t) R * nv * HS;
+#pragma unroll 1
+    for (int g = 0; g < ng; ++g, od += ostep) {
+        const float* tl = gds + g % GDS_STAGES * GDS_STAGE;
+        float* rp = red + part * GDS_PART + keep;
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const ulonglong2 k0 = *reinterpret_cast<const ulonglong2*>(tl + GDS_K + i * HS + key0), k1 = *reinterpret_cast<const ulonglong2*>(tl + GDS_K + i * HS + key0 + 4);
+            const ulonglong2 q0 = *reinterpret_cast<const ulonglong2*>(tl + GDS_QO + i * HS + key0), q1 = *reinterpret_cast<const ulonglong2*>(tl + GDS_QO + i * HS + key0 + 4);
+            float ks[2], qs[2];
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const uint64_t ka = f2_fma(s[c][3], k1.y, f2_fma(s[c][2], k1.x, f2_fma(s[c][1], k0.y, f2_mul(s[c][0], k0.x))));
+                const uint64_t qa = f2_fma(s[c][3], q1.y, f2_fma(s[c][2], q1.x, f2_fma(s[c][1], q0.y, f2_mul(s[c][0], q0.x))));
+                float lo, hi;
+                f2_unpack(ka, lo, hi);
+                ks[c] = lo + hi;
+                f2_unpack(qa, lo, hi);
+                qs[c] = lo + hi;
+            }
+            // another eight key rows' sums of the column this lane keeps
+            rp[i * C] = ks[0] + __shfl_xor_sync(0xffffffffu, ks[1], 16);
+            rp[(R + i) * C] = qs[0] + __shfl_xor_sync(0xffffffffu, qs[1], 16);
         }
         __syncthreads();
-#pragma unroll 1
-        for (int r0 = 0; r0 < nr; ++r0) {
-            const float* row = tile[buf][r0];
-            const float* kt = row + part * 32;
-            const float* qt = row + GDN_HS + part * 32;
-            const float gv = row[2 * GDN_HS + GDN_QC], bv = row[2 * GDN_HS + GDN_QC + 1];
-            // (the row's k and q for this warp's 32 key rows: eight 16-byte broadcast reads each, as pairs)
-            uint64_t kp[16], qp[16];
+        stage(g + GDS_STAGES - 1);   // (into the slot of the group before: its last readers passed the barrier above)
+        const float* cf = tl + GDS_C;
+        float ksw = 0.f, qsw = 0.f;
 #pragma unroll
-            for (int r = 0; r < 32; r += 4) {
-                const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(kt + r), b = *reinterpret_cast<const ulonglong2*>(qt + r);
-                kp[r / 2] = a.x; kp[r / 2 + 1] = a.y;
-                qp[r / 2] = b.x; qp[r / 2 + 1] = b.y;
-            }
-            // eight running sums in four pairs (row r of the 32 goes to sum r % 8): four independent chains of packed products
-            uint64_t kacc[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) kacc[i] = f2_pack(0.f, 0.f);
-#pragma unroll
-            for (int r = 0; r < 16; r += 4)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) kacc[i] = f2_fma(s[r + i], kp[r + i], kacc[i]);
-            float k0, k1, k2, k3, k4, k5, k6, k7;
-            f2_unpack(kacc[0], k0, k1);
-            f2_unpack(kacc[1], k2, k3);
-            f2_unpack(kacc[2], k4, k5);
-            f2_unpack(kacc[3], k6, k7);
-            float* kr = &kred[r0 & 1][0][0];
-            kr[part * GDN_QC + lane] = ((k0 + k1) + (k2 + k3)) + ((k4 + k5) + (k6 + k7));
-            __syncthreads();
-            const float kvs = (kr[lane] + kr[GDN_QC + lane]) + (kr[2 * GDN_QC + lane] + kr[3 * GDN_QC + lane]);
-            const float delta = (row[2 * GDN_HS + lane] - gv * kvs) * bv;
-            const uint64_t d2 = f2_pack(delta, delta), g2 = f2_pack(gv, gv);
-            uint64_t aacc[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) aacc[i] = f2_pack(0.f, 0.f);
-#pragma unroll
-            for (int r = 0; r < 16; r += 4)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    s[r + i] = f2_fma(kp[r + i], d2, f2_mul(g2, s[r + i]));
-                    aacc[i] = f2_fma(s[r + i], qp[r + i], aacc[i]);
-                }
-            float a0, a1, a2, a3, a4, a5, a6, a7;
-            f2_unpack(aacc[0], a0, a1);
-            f2_unpack(aacc[1], a2, a3);
-            f2_unpack(aacc[2], a4, a5);
-            f2_unpack(aacc[3], a6, a7);
-            ared[r0][part][lane] = ((a0 + a1) + (a2 + a3)) + ((a4 + a5) + (a6 + a7));
+        for (int p = 0; p < GDS_PARTS; ++p) {
+            ksw += red[p * GDS_PART + row * C + col];
+            qsw += red[p * GDS_PART + (R + row) * C + col];
         }
-        __syncthreads();   // the tile's sums are complete; its buffer may be refilled two tiles on
-        for (int i = tid; i < nr * GDN_QC; i += GDS_THREADS) {
-            const int r0 = i / GDN_QC, c = i % GDN_QC;
-            o[((size_t) (t0 + r0) * nv + lv) * GDN_HS + qq * GDN_QC + c] = ((ared[r0][0][c] + ared[r0][1][c]) + (ared[r0][2][c] + ared[r0][3][c])) * scale;
+        {
+            const float w = cf[GC_BV + row] * tl[GDS_V + row * C + col] - cf[GC_BK + row] * ksw;
+            const int h = col >> 3;
+            ws[row * C + col] = w;
+            (&w2[row * 8 + (col & 7)].x)[h] = w;
+            (&w2[(R + row) * 8 + (col & 7)].x)[h ^ 1] = w;
+        }
+        asm volatile("cp.async.wait_group %0;" ::"n"(GDS_STAGES - 2) : "memory");   // the next group is in
+        __syncthreads();
+        const float bc = cf[GC_BC];
+        const uint64_t bc2 = f2_pack(bc, bc);
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+#pragma unroll
+            for (int p = 0; p < 4; ++p) s[c][p] = f2_mul(bc2, s[c][p]);
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const float2 w = w2[(up * R + i) * 8 + cp];
+            const ulonglong2 c0 = *reinterpret_cast<const ulonglong2*>(tl + GDS_CO + i * HS + key0), c1 = *reinterpret_cast<const ulonglong2*>(tl + GDS_CO + i * HS + key0 + 4);
+            const uint64_t wx = f2_pack(w.x, w.x), wy = f2_pack(w.y, w.y);
+            s[0][0] = f2_fma(c0.x, wx, s[0][0]); s[0][1] = f2_fma(c0.y, wx, s[0][1]); s[0][2] = f2_fma(c1.x, wx, s[0][2]); s[0][3] = f2_fma(c1.y, wx, s[0][3]);
+            s[1][0] = f2_fma(c0.x, wy, s[1][0]); s[1][1] = f2_fma(c0.y, wy, s[1][1]); s[1][2] = f2_fma(c1.x, wy, s[1][2]); s[1][3] = f2_fma(c1.y, wy, s[1][3]);
+        }
+        {
+            const float4 m0 = *reinterpret_cast<const float4*>(cf + GC_M + row * R), m1 = *reinterpret_cast<const float4*>(cf + GC_M + row * R + 4);
+            const float m[R] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
+            float a = cf[GC_BQ + row] * qsw;
+#pragma unroll
+            for (int j = 0; j < R; ++j) a = fmaf(m[j], ws[j * C + col], a);
+            if (g * R + row < T) *od = a;
         }
     }
 #pragma unroll
-    for (int r = 0; r < 32; r += 2) {
-        float x, y;
-        f2_unpack(s[r / 2], x, y);
-        S_out[soff + (size_t) r * GDN_HS] = x;
-        S_out[soff + (size_t) (r + 1) * GDN_HS] = y;
-    }
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float x, y;
+            f2_unpack(s[c][i], x, y);
+            S_out[soff + (size_t) (2 * i) * HS + (keep ^ (8 * c))] = x;
+            S_out[soff + (size_t) (2 * i + 1) * HS + (keep ^ (8 * c))] = y;
+        }
 }
 
 // block = one row, warp = a quarter (32 columns) of a value head at a time: y = o * rsqrt(mean(o^2) + eps) * nw * sigmoid(z)
@@ -526,7 +662,8 @@ extern "C" int fnx_gdn_core(const float* qkvz, int ldx, const float* ab, int lda
 }
 
 extern "C" size_t fnx_gdn_prompt_scratch_bytes(int T, int nk, int nv, int hs) {
-    return sizeof(float) * ((size_t) T * (2 * nk + 2 * nv) * hs + (size_t) T * nv * 2 + (size_t) 3 * (2 * nk + nv) * hs) + 1024;
+    const size_t ng = ((size_t) T + GDP_ROWS - 1) / GDP_ROWS;
+    return sizeof(float) * (ng * GDP_ROWS * (2 * nk + 3 * nv) * hs + ng * nv * GC_FLOATS + (size_t) 3 * (2 * nk + nv) * hs) + 1024;
 }
 
 extern "C" int fnx_gdn_prompt(const float* qkvz, int ldx, const float* ab, int ldab, float* hist_pool, const float* convw, const float* dt, const float* a,
@@ -538,19 +675,23 @@ extern "C" int fnx_gdn_prompt(const float* qkvz, int ldx, const float* ab, int l
     FNX_REQUIRE(nk >= 1 && nv >= nk && nv % nk == 0 && nv <= GDP_THREADS && ((2 * nk + nv) * GDN_HS) % GDP_THREADS == 0, "fnx_gdn_prompt: %d key heads, %d value heads", nk, nv);
     const int ch = (2 * nk + nv) * GDN_HS, out_slot = (cur_host + T) % NS;
     const size_t hsz = (size_t) 3 * ch, ssz = (size_t) nv * GDN_HS * GDN_HS;
+    const int ng = (T + GDP_ROWS - 1) / GDP_ROWS;
+    const size_t Tp = (size_t) ng * GDP_ROWS;
     float* xq = (float*) scratch;
-    float* xk = xq + (size_t) T * nk * GDN_HS;
-    float* xv = xk + (size_t) T * nk * GDN_HS;
-    float* o = xv + (size_t) T * nv * GDN_HS;
-    float* gates = o + (size_t) T * nv * GDN_HS;
+    float* xk = xq + Tp * nk * GDN_HS;
+    float* xv = xk + Tp * nk * GDN_HS;
+    float* xc = xv + Tp * nv * GDN_HS;
+    float* o = xc + Tp * nv * GDN_HS;
+    float* coef = o + (size_t) T * nv * GDN_HS;
     cudaStream_t s = as_stream(st);
     // the history the call starts from is read from a copy: the slot it leaves its own in may be the same one
-    float* hin = gates + (size_t) T * nv * 2;
+    float* hin = coef + (size_t) ng * nv * GC_FLOATS;
     FNX_CUDA_OK(cudaMemcpyAsync(hin, hist_pool + (size_t) cur_host * hsz, hsz * sizeof(float), cudaMemcpyDeviceToDevice, s));
-    k_gdn_pre<<<T, GDP_THREADS, 0, s>>>(qkvz, ldx, ab, ldab, hin, hist_pool + (size_t) out_slot * hsz, convw, dt, a, xq, xk, xv, gates, nk,
-                                         nv, T);
+    k_gdn_pre<<<dim3(ng, nk + nv * GDN_HS / GDP_THREADS), GDP_THREADS, 0, s>>>(qkvz, ldx, ab, ldab, hin, hist_pool + (size_t) out_slot * hsz, convw, dt, a, xq, xk, xv, xc,
+                                                                               coef, nk, nv, T);
     FNX_LAUNCH_OK("k_gdn_pre");
-    k_gdn_scan<<<nv * GDN_Q, GDS_THREADS, 0, s>>>(xq, xk, xv, gates, S_pool + (size_t) cur_host * ssz, S_pool + (size_t) out_slot * ssz, o, nk, nv, T);
+    FNX_TRY(set_smem_limit((const void*) k_gdn_scan, GDS_SMEM));
+    k_gdn_scan<<<nv * (GDN_HS / GDS_COLS), GDS_THREADS, GDS_SMEM, s>>>(xq, xk, xv, xc, coef, S_pool + (size_t) cur_host * ssz, S_pool + (size_t) out_slot * ssz, o, nk, nv, T);
     FNX_LAUNCH_OK("k_gdn_scan");
     k_gdn_post<<<T, GDP_THREADS, 0, s>>>(o, qkvz, ldx, nw, y, nk, nv, eps);
     FNX_LAUNCH_OK("k_gdn_post");
