@@ -50,15 +50,7 @@ struct TaShared {
 };
 static_assert(sizeof(TaShared) <= TA_HEAD, "the head fits");
 
-// a wait that every role leaves soon after one of them gave up
-__device__ __forceinline__ bool ta_wait(uint64_t* bar, unsigned parity, TaShared& S) {
-    for (unsigned i = 0; i < TA_WAIT; ++i) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if (S.gave_up) return false;
-    }
-    S.gave_up = 1;
-    return false;
-}
+__device__ __forceinline__ bool ta_wait(uint64_t* bar, unsigned parity, TaShared& S) { return ta_wait_for(bar, parity, S.gave_up); }
 
 // grid (16-row tiles of the chunk, latest first; KV heads)
 __global__ void __launch_bounds__(TA_THREADS, 1) k_attn_prompt_tc(const float* __restrict__ qg, int ldq, const __half* __restrict__ kc,

@@ -11,7 +11,7 @@ namespace fnxb {
 
 constexpr int ATC_HD = 256;   // head dim
 constexpr int ATC_N = 64;     // positions per step
-constexpr unsigned TA_WAIT = 20000000u;
+constexpr unsigned long long TA_WAIT_NS = 2000000000ull;   // what a wait takes at most
 
 __device__ __forceinline__ uint64_t ta_desc(uint32_t saddr, int lbo, int sbo) {
     // shared-memory matrix descriptor: start address, leading and stride byte offsets in 16-byte units, version 1, no swizzle
@@ -27,6 +27,30 @@ __device__ __forceinline__ void ta_tma_3d(uint32_t dst_s, const CUtensorMap* map
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst_s), "l"(map),
                  "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(bar))
                  : "memory");
+}
+// A wait between the warps of a block, which every role leaves soon after one of them gave up.  The thread sleeps in the barrier (a time
+// hint far above any wait that is in order): polling warps took a third of the issue slots that the others need.
+__device__ __forceinline__ bool ta_wait_for(uint64_t* bar, unsigned parity, volatile int& gave_up) {
+    if (mbar_try_wait(bar, parity)) return true;
+    unsigned long long t0, t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
+    do {
+        unsigned done;
+        asm volatile(
+            "{\n"
+            ".reg .pred p;\n"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
+            "selp.u32 %0, 1, 0, p;\n"
+            "}\n"
+            : "=r"(done)
+            : "r"(smem_u32(bar)), "r"(parity), "r"(1000000u)
+            : "memory");
+        if (done) return true;
+        if (gave_up) return false;
+        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    } while (t - t0 < TA_WAIT_NS);
+    gave_up = 1;
+    return false;
 }
 // one thread of a converged warp
 __device__ __forceinline__ bool ta_elect() {

@@ -52,15 +52,7 @@ struct AwShared {
 };
 static_assert(sizeof(AwShared) <= AW_HEAD, "the head fits");
 
-// a wait that every role leaves soon after one of them gave up
-__device__ __forceinline__ bool aw_wait(uint64_t* bar, unsigned parity, AwShared& S) {
-    for (unsigned i = 0; i < TA_WAIT; ++i) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if (S.gave_up) return false;
-    }
-    S.gave_up = 1;
-    return false;
-}
+__device__ __forceinline__ bool aw_wait(uint64_t* bar, unsigned parity, AwShared& S) { return ta_wait_for(bar, parity, S.gave_up); }
 
 struct AwItem {
     int lane, row0, nr, kvh, s, n, ctx, pos0;   // rows [row0, row0 + nr) of the window; n steps

@@ -657,7 +657,7 @@ static size_t pf_staged_bytes(size_t pairs, int E, int H, int F) {
 extern "C" size_t fnx_moe_prefill_scratch_bytes(int T, int K, int E, int H, int F) {
     const size_t pairs = (size_t) T * K + T;
     return pf_align(pairs * F * sizeof(__half)) + pf_align(pairs * H * sizeof(float)) + pf_align(pairs * sizeof(int)) + pf_align((size_t) (E + 1) * sizeof(int)) * 2 +
-           pf_align((pairs / PN_N + E + 2 + (size_t) T / PN_N) * sizeof(PfJob)) + pf_align((size_t) T * H * sizeof(__half)) + 256 +
+           pf_align((pairs / 8 + E + 2 + (size_t) T / 8) * sizeof(PfJob)) + pf_align((size_t) T * H * sizeof(__half)) + 256 +
            (T >= 1024 ? pf_staged_bytes(pairs, E, H, F) : 0);
 }
 
@@ -678,11 +678,12 @@ int prompt_moe(const void* Wgu, size_t gu_stride, const void* Wsh_gu, bool gu_na
     int* order = (int*) b; b += pf_align(pairs * sizeof(int));
     int* cnt = (int*) b; b += pf_align((size_t) (E + 1) * sizeof(int));
     int* base = (int*) b; b += pf_align((size_t) (E + 1) * sizeof(int));
-    PfJob* jobs = (PfJob*) b; b += pf_align((pairs / PN_N + E + 2 + (size_t) T / PN_N) * sizeof(PfJob));
+    PfJob* jobs = (PfJob*) b; b += pf_align((pairs / 8 + E + 2 + (size_t) T / 8) * sizeof(PfJob));
     __half* xh = (__half*) b; b += pf_align((size_t) T * H * sizeof(__half));
     int* njobs = (int*) b; b += 256;
     const int ne = e_hi - e_lo, n = T * K;
-    const int per = gu_nat || dn_nat ? PN_N : PF_N, pb = (n + PF_PAIRS - 1) / PF_PAIRS;
+    const int few = gu_nat && dn_nat ? prompt_few_groups(n, E) : 0;
+    const int per = few ? 8 * few : gu_nat || dn_nat ? PN_N : PF_N, pb = (n + PF_PAIRS - 1) / PF_PAIRS;
     if (ne > 0) {
         FNX_CUDA_OK(cudaMemsetAsync(cnt, 0, sizeof(int) * ne, st));
         k_pf_count<<<pb, 512, 0, st>>>(topi, n, e_lo, ne, cnt);
@@ -694,7 +695,7 @@ int prompt_moe(const void* Wgu, size_t gu_stride, const void* Wsh_gu, bool gu_na
         k_pf_fill<<<pb, 512, 0, st>>>(topi, n, e_lo, ne, base, order);
         FNX_LAUNCH_OK("k_pf_fill");
     }
-    if (gu_nat) FNX_TRY(prompt_nat_rows(x, norm_w, T, H, eps, xh, st));
+    if (gu_nat) FNX_TRY(prompt_nat_rows(x, norm_w, T, H, eps, xh, few != 0, st));
     else {
         k_pf_xnorm<<<T, 256, 0, st>>>(x, norm_w, H, eps, xh);
         FNX_LAUNCH_OK("k_pf_xnorm");
@@ -727,7 +728,7 @@ int prompt_moe(const void* Wgu, size_t gu_stride, const void* Wsh_gu, bool gu_na
     p.e_base = e_base; p.E = E; p.jobs = jobs; p.njobs = njobs; p.order = order; p.TKp = n; p.Kp = K; p.err = err;
     if (gu_nat) {
         q.W = (const uint8_t*) Wgu; q.stride = gu_stride; q.Wsh = (const uint8_t*) Wsh_gu; q.x = xh; q.rows = F; q.K = H; q.outh = hbuf;
-        FNX_TRY(prompt_nat(1, q, nj, st));
+        FNX_TRY(few ? prompt_few(1, few, q, nj, st) : prompt_nat(1, q, nj, st));
     } else {
         FNX_TRY(set_smem_limit((const void*) k_pf_gemm<1>, (int) pf_smem(1)));
         p.W = (const uint8_t*) Wgu; p.expert_stride = gu_stride; p.Wsh = (const uint8_t*) Wsh_gu; p.x = xh; p.rows = F; p.K = H; p.outh = hbuf;
@@ -740,7 +741,7 @@ int prompt_moe(const void* Wgu, size_t gu_stride, const void* Wsh_gu, bool gu_na
     }
     if (dn_nat) {
         q.W = (const uint8_t*) Wdn; q.stride = dn_stride; q.Wsh = (const uint8_t*) Wsh_dn; q.x = hbuf; q.rows = H; q.K = F; q.out = part; q.ldo = H;
-        FNX_TRY(prompt_nat(0, q, nj, st));
+        FNX_TRY(few ? prompt_few(0, few, q, nj, st) : prompt_nat(0, q, nj, st));
     } else {
         FNX_TRY(set_smem_limit((const void*) k_pf_gemm<0>, (int) pf_smem(0)));
         p.W = (const uint8_t*) Wdn; p.expert_stride = dn_stride; p.Wsh = (const uint8_t*) Wsh_dn; p.x = hbuf; p.rows = H; p.K = F; p.out = part; p.outh = nullptr;
@@ -790,7 +791,7 @@ int prompt_dense(const void* W, bool nat, int rows, int cols, const float* x, in
     __half* w16 = (__half*) b;
     const int nj = (T + PF_N - 1) / PF_N;
     if (nat && T < pf_tma_rows()) {
-        FNX_TRY(prompt_nat_rows(x, norm_w, T, cols, eps, xh, st));
+        FNX_TRY(prompt_nat_rows(x, norm_w, T, cols, eps, xh, false, st));
         PnParams q{};
         q.W = (const uint8_t*) W; q.T = T; q.x = xh; q.rows = rows; q.K = cols; q.out = y; q.ldo = ldy; q.accumulate = accumulate; q.err = err;
         return prompt_nat(2, q, (T + PN_N - 1) / PN_N, st);

@@ -48,14 +48,7 @@ struct PnShared {
 };
 static_assert(sizeof(PnShared) <= PN_HEAD, "the head fits");
 
-__device__ __forceinline__ bool pn_wait(uint64_t* bar, unsigned parity, PnShared& S) {
-    for (unsigned i = 0; i < TA_WAIT; ++i) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if (S.gave_up) return false;
-    }
-    S.gave_up = 1;
-    return false;
-}
+__device__ __forceinline__ bool pn_wait(uint64_t* bar, unsigned parity, PnShared& S) { return ta_wait_for(bar, parity, S.gave_up); }
 
 // sixteen tensor-memory lanes x 32 columns: register 4 b + {0, 1} = columns 8 b + 2 q, + 1 of lane g, + {2, 3} the same of lane g + 8
 __device__ __forceinline__ void pn_st_tile(uint32_t taddr, const uint32_t (&v)[16]) {
@@ -67,13 +60,34 @@ __device__ __forceinline__ void pn_st_tile(uint32_t taddr, const uint32_t (&v)[1
 __device__ __forceinline__ uint32_t pn_h2(__half2 h) { return *reinterpret_cast<const uint32_t*>(&h); }
 __device__ __forceinline__ __half2 pn_as_h2(uint32_t u) { return *reinterpret_cast<const __half2*>(&u); }
 
+// (a & b) ^ c in one instruction: with two constants the compiler makes two of it, and the integer-logic pipe is what bounds the decode
+__device__ __forceinline__ uint32_t pn_and_xor(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t d;
+    asm("lop3.b32 %0, %1, %2, %3, 0x6A;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+    return d;
+}
+__device__ __forceinline__ uint32_t pn_and_or(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t d;
+    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+    return d;
+}
+// constants that stay in registers, and factors that stay multiplications (a shift would compete for the same pipe)
+struct PnConst {
+    uint32_t two, k13, m1, m4;
+    __device__ __forceinline__ PnConst() {
+        asm("mov.u32 %0, 2;" : "=r"(two));
+        asm("mov.u32 %0, 8192;" : "=r"(k13));
+        asm("mov.u32 %0, 0x001E001E;" : "=r"(m1));
+        asm("mov.u32 %0, 0x00F000F0;" : "=r"(m4));
+    }
+};
 // The eight weights of a word times the sub-block's scale (in both halves of f): out[0], out[1] = columns (0, 2), (1, 3), out[2], out[3] =
 // (4, 6), (5, 7).  A nibble t at bits 1..4 of a half 0x6400 | .. is 1024 + 2 (t + 8) = 1039 + m; at bits 4..7 it is 1024 + 16 (t + 8) =
 // 8 (143 + m): both exact, so the one rounding is that of m f, as in the other forms of these products.
-__device__ __forceinline__ void pn_decode8(uint32_t w, __half2 f, uint32_t& o0, uint32_t& o1, uint32_t& o2, uint32_t& o3) {
+__device__ __forceinline__ void pn_decode8(const PnConst& C, uint32_t w, __half2 f, uint32_t& o0, uint32_t& o1, uint32_t& o2, uint32_t& o3) {
     const uint32_t s = w >> 8;
-    const uint32_t a = ((w * 2u) & 0x001E001Eu) ^ 0x64106410u, c = (w & 0x00F000F0u) ^ 0x64806480u;
-    const uint32_t b = ((s * 2u) & 0x001E001Eu) ^ 0x64106410u, d = (s & 0x00F000F0u) ^ 0x64806480u;
+    const uint32_t a = pn_and_xor(w * C.two, C.m1, 0x64106410u), c = pn_and_xor(w, C.m4, 0x64806480u);
+    const uint32_t b = pn_and_xor(s * C.two, C.m1, 0x64106410u), d = pn_and_xor(s, C.m4, 0x64806480u);
     const __half2 k1 = pn_as_h2(0xE40FE40Fu);                                   // -1039
     const __half2 k8 = pn_as_h2(0x30003000u), k2 = pn_as_h2(0xD878D878u);       // 1 / 8, -143
     o0 = pn_h2(__hmul2(__hadd2(pn_as_h2(a), k1), f));
@@ -83,10 +97,10 @@ __device__ __forceinline__ void pn_decode8(uint32_t w, __half2 f, uint32_t& o0, 
 }
 // a row's two scales d (1 + 2 s) of sub-blocks 2 Q and 2 Q + 1 (nibbles sn >> 8 Q); d in both halves.  d has 11 bits and 1 + 2 s five: the
 // product rounds once, as from f32
-__device__ __forceinline__ void pn_scales(uint32_t sn, int Q, __half2 d, __half2& f0, __half2& f1) {
+__device__ __forceinline__ void pn_scales(const PnConst& C, uint32_t sn, int Q, __half2 d, __half2& f0, __half2& f1) {
     const uint32_t t = sn >> (8 * Q);
-    const __half2 n = __hadd2(pn_as_h2(((t & 15u) << 1) | ((t & 0xF0u) << 13) | 0x64016401u), pn_as_h2(0xE400E400u));   // 1 + 2 s, exact
-    const __half2 f = __hmul2(n, d);
+    const uint32_t x = pn_and_or(t * C.k13, 0x001E0000u, pn_and_or(t * C.two, 0x0000001Eu, 0x64016401u));
+    const __half2 f = __hmul2(__hadd2(pn_as_h2(x), pn_as_h2(0xE400E400u)), d);   // (1 + 2 s, exact) d
     f0 = __low2half2(f);
     f1 = __high2half2(f);
 }
@@ -186,6 +200,7 @@ __global__ void __launch_bounds__(PN_THREADS, 1) k_prompt_nat(const PnParams p) 
         };
 #pragma unroll
         for (int i = 0; i < PN_SLOTS; ++i) fetch();
+        const PnConst C;
         int c = 0, slot = 0;   // chunks so far
         for (int it = blockIdx.x; it < total; it += gridDim.x) {
             for (int kb = 0; kb < KB; ++kb) {
@@ -210,12 +225,12 @@ __global__ void __launch_bounds__(PN_THREADS, 1) k_prompt_nat(const PnParams p) 
                         const int Q = PN_KC / 64 * st + q2;
                         uint32_t o[16];
                         __half2 f00, f01, f10, f11;
-                        pn_scales(m.x, Q, d0, f00, f01);
-                        pn_scales(m.y, Q, d1, f10, f11);
-                        pn_decode8(w[0][2 * Q], f00, o[0], o[1], o[4], o[5]);
-                        pn_decode8(w[1][2 * Q], f10, o[2], o[3], o[6], o[7]);
-                        pn_decode8(w[0][2 * Q + 1], f01, o[8], o[9], o[12], o[13]);
-                        pn_decode8(w[1][2 * Q + 1], f11, o[10], o[11], o[14], o[15]);
+                        pn_scales(C, m.x, Q, d0, f00, f01);
+                        pn_scales(C, m.y, Q, d1, f10, f11);
+                        pn_decode8(C, w[0][2 * Q], f00, o[0], o[1], o[4], o[5]);
+                        pn_decode8(C, w[1][2 * Q], f10, o[2], o[3], o[6], o[7]);
+                        pn_decode8(C, w[0][2 * Q + 1], f01, o[8], o[9], o[12], o[13]);
+                        pn_decode8(C, w[1][2 * Q + 1], f11, o[10], o[11], o[14], o[15]);
                         if (q2 == 0) {
                             if (ok && c >= PN_AST) ok = __all_sync(0xffffffffu, pn_wait(&sh.empty[st], (unsigned) ((c / PN_AST - 1) & 1), sh));
                             ta_fence_after();
@@ -379,7 +394,202 @@ __global__ void __launch_bounds__(PN_THREADS, 1) k_prompt_nat(const PnParams p) 
     if (warp == PN_W_MMA) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
 }
 
-__global__ void __launch_bounds__(256) k_prompt_nat_rows(const float* __restrict__ x, const float* __restrict__ norm_w, int H, float eps, __half* __restrict__ xh) {
+// ------------------------------------------------------------------------------------------------ jobs of few rows
+// The expert products where an expert has up to some nine rows on average: mma.sync with the decoded fragments in registers as the A
+// operand, so that neither tensor memory nor the waits between its writers and readers are in the way.  Bound by the decode's instructions
+// (integer-logic and half pipes, two cycles each; half of either busy); the products (2 cycles an SM each) would pass it with four row groups.  An item is a job and 16
+// tiles of 32 features (gate|up: 16 gate and the 16 up of the same features), a warp each; the job's rows go through three shared-memory
+// chunks of 256 columns, a warp's tiles through two slots of its own.  513 jobs of 6 rows: 196 + 107 -> 160 + 95 us
+// (gate|up + down).
+// The rows' columns lie in fours as (0, 2, 1, 3), the order of a decoded word's pairs.
+constexpr int PW_WARPS = 16, PW_THREADS = PW_WARPS * 32, PW_BST = 3;
+constexpr int PW_ROW = 512 + 64;   // bytes of a row's chunk (neighbouring rows in different halves of the banks)
+constexpr int PW_RING = PW_WARPS * 2 * NAT_TILE_BYTES;
+template <int NG>
+constexpr int pw_smem() { return PW_RING + PW_BST * 8 * NG * PW_ROW; }
+
+__device__ __forceinline__ void pw_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+template <int MODE, int NG>
+__global__ void __launch_bounds__(PW_THREADS, 1) k_prompt_few(const PnParams p) {
+    extern __shared__ __align__(128) uint8_t smem[];
+    constexpr int NT = 8 * NG;   // rows
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
+    const int KB = p.K / 256, units = MODE == 1 ? p.rows / 16 : p.rows / 32, parts = (units + PW_WARPS - 1) / PW_WARPS, total = *p.njobs * parts;
+    if ((int) blockIdx.x >= total) return;
+    uint8_t* ring = smem + warp * 2 * NAT_TILE_BYTES;
+    uint8_t* Bs = smem + PW_RING;
+    const uint32_t ring_s = smem_u32(ring) + lane * 16, b_s = smem_u32(Bs) + warp * PW_ROW + lane * 16;
+    // the copies' cursor, two chunks ahead; the next item's job and entries are loaded ahead of it
+    int cit = blockIdx.x, ckb = 0;
+    const uint8_t* wsrc = nullptr;
+    const __half* xsrc;   // the warp's row
+    PnJob nx;
+    int e;
+    bool need_e = true;
+    auto entries = [&]() {
+        e = p.order[nx.start + min(warp, nx.n - 1)];
+        need_e = false;
+    };
+    auto enter = [&]() {   // the cursor's item: `nx`
+        if (need_e) entries();
+        const int unit = cit % parts * PW_WARPS + warp;
+        const uint8_t* W = nx.w >= p.E ? p.Wsh : p.W + (size_t) (nx.w - p.e_base) * p.stride;
+        wsrc = unit < units ? W + (size_t) unit * KB * NAT_TILE_BYTES + lane * 16 : nullptr;
+        const int row = MODE == 1 ? (e >= p.TKp ? e - p.TKp : e / p.Kp) : e;
+        xsrc = warp < min(nx.n, NT) ? p.x + (size_t) row * p.K + lane * 8 : nullptr;
+        if (cit + (int) gridDim.x < total) {
+            nx = p.jobs[(cit + gridDim.x) / parts];
+            need_e = true;
+        }
+    };
+    auto advance = [&]() {
+        if (cit >= total) return;
+        if (++ckb == KB) {
+            ckb = 0;
+            cit += gridDim.x;
+            if (cit < total) enter();
+        } else if (need_e) {
+            entries();
+        }
+    };
+    auto fetch_rows = [&](int slot) {
+        if (cit < total && xsrc) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(b_s + slot * NT * PW_ROW), "l"(xsrc + ckb * 256) : "memory");
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    auto fetch_tile = [&](int slot) {
+        if (cit < total && wsrc) {
+            const uint32_t dst = ring_s + slot * NAT_TILE_BYTES;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + h * NAT_HALF_BYTES + j * 512), "l"(wsrc + h * NAT_HALF_BYTES + j * 512) : "memory");
+                if (lane < 8) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + h * NAT_HALF_BYTES + NAT_META), "l"(wsrc + h * NAT_HALF_BYTES + NAT_META) : "memory");
+            }
+            wsrc += NAT_TILE_BYTES;
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    nx = p.jobs[cit / parts];
+    enter();
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        fetch_rows(i);
+        fetch_tile(i);
+        advance();
+    }
+    const PnConst C;
+    int c = 0, bslot = 0;
+    for (int it = blockIdx.x; it < total; it += gridDim.x) {
+        const PnJob job = p.jobs[it / parts];
+        const int unit = it % parts * PW_WARPS + warp;
+        int mine = 0;   // lane: output row `lane` of the job
+        float acc[2][NG][4];
+#pragma unroll
+        for (int i = 0; i < 2 * NG * 4; ++i) acc[i / (4 * NG)][(i / 4) % NG][i & 3] = 0.f;
+        for (int kb = 0; kb < KB; ++kb, ++c) {
+            asm volatile("cp.async.wait_group 2;" ::: "memory");
+            __syncthreads();   // the chunk's rows are in, and everyone is done with the chunk before: its place is free
+            fetch_rows(bslot == 0 ? PW_BST - 1 : bslot - 1);
+            const uint8_t* t = ring + (c & 1) * NAT_TILE_BYTES;
+            const uint8_t* b = Bs + (bslot * NT + g) * PW_ROW + q * 16;
+            if (unit < units) {
+                const uint4 m0 = *reinterpret_cast<const uint4*>(t + NAT_META + g * 16), m1 = *reinterpret_cast<const uint4*>(t + NAT_HALF_BYTES + NAT_META + g * 16);
+                const __half2 dd[2] = {pn_as_h2(m0.z), pn_as_h2(m1.z)};
+#pragma unroll 1
+                for (int jj = 0; jj < 2; ++jj) {
+                    uint4 w[2][2];
+#pragma unroll
+                    for (int hf = 0; hf < 2; ++hf)
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) w[hf][h] = *reinterpret_cast<const uint4*>(t + hf * NAT_HALF_BYTES + (2 * h + jj) * 512 + lane * 16);
+#pragma unroll
+                    for (int s2 = 0; s2 < 2; ++s2) {
+                        __half2 f[2][2][2];   // [half tile][row half][sub-block]
+#pragma unroll
+                        for (int hf = 0; hf < 2; ++hf) {
+                            pn_scales(C, (hf ? m1.x : m0.x) >> (16 * jj), s2, __low2half2(dd[hf]), f[hf][0][0], f[hf][0][1]);
+                            pn_scales(C, (hf ? m1.y : m0.y) >> (16 * jj), s2, __high2half2(dd[hf]), f[hf][1][0], f[hf][1][1]);
+                        }
+#pragma unroll
+                        for (int e2 = 0; e2 < 2; ++e2) {
+                            uint4 bv[NG];
+#pragma unroll
+                            for (int n = 0; n < NG; ++n) bv[n] = *reinterpret_cast<const uint4*>(b + n * 8 * PW_ROW + (4 * jj + 2 * s2 + e2) * 64);
+#pragma unroll
+                            for (int hf = 0; hf < 2; ++hf) {
+                                const uint32_t wa = s2 ? (e2 ? w[hf][0].w : w[hf][0].z) : (e2 ? w[hf][0].y : w[hf][0].x);
+                                const uint32_t wb = s2 ? (e2 ? w[hf][1].w : w[hf][1].z) : (e2 ? w[hf][1].y : w[hf][1].x);
+                                uint32_t a[4], d[4];
+                                pn_decode8(C, wa, f[hf][0][e2], a[0], a[1], a[2], a[3]);
+                                pn_decode8(C, wb, f[hf][1][e2], d[0], d[1], d[2], d[3]);
+#pragma unroll
+                                for (int n = 0; n < NG; ++n) {
+                                    pw_mma(acc[hf][n], a[0], d[0], a[1], d[1], bv[n].x, bv[n].y);
+                                    pw_mma(acc[hf][n], a[2], d[2], a[3], d[3], bv[n].z, bv[n].w);
+                                }
+                            }
+                        }
+                    }
+                }
+            }
+            if (kb == 0) mine = p.order[job.start + min(lane, job.n - 1)];   // (used after the last chunk)
+            __syncwarp();   // every lane is done with the tile
+            fetch_tile(c & 1);
+            advance();
+            bslot = bslot + 1 == PW_BST ? 0 : bslot + 1;
+        }
+        // a lane holds the features g and g + 8 of its unit's two half tiles for the rows 8 n + 2 q, + 1
+#pragma unroll
+        for (int n = 0; n < NG; ++n)
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const int row = 8 * n + 2 * q + r;
+                const size_t o = (size_t) __shfl_sync(0xffffffffu, mine, row);
+                if (row < job.n && unit < units) {
+                    if (MODE == 1) {
+                        __half* dst = p.outh + o * p.rows + unit * 16;
+#pragma unroll
+                        for (int i = 0; i < 2; ++i) {
+                            const int f = g + 8 * i;
+                            const float a = acc[0][n][2 * i + r], b = acc[1][n][2 * i + r];
+                            dst[(f & ~3) | ((f & 1) << 1) | ((f >> 1) & 1)] = __float2half_rn(__fdividef(a, 1.0f + __expf(-a)) * b);
+                        }
+                    } else {
+                        float* dst = p.out + o * p.ldo + unit * 32 + g;
+#pragma unroll
+                        for (int hf = 0; hf < 2; ++hf) {
+                            dst[16 * hf] = acc[hf][n][r];
+                            dst[16 * hf + 8] = acc[hf][n][2 + r];
+                        }
+                    }
+                }
+            }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+
+template <int NG>
+static int launch_few(int mode, const PnParams& p, int max_jobs, cudaStream_t st) {
+    auto kernel = mode == 1 ? k_prompt_few<1, NG> : k_prompt_few<0, NG>;
+    FNX_TRY(set_smem_limit((const void*) kernel, pw_smem<NG>()));
+    const int units = mode == 1 ? p.rows / 16 : p.rows / 32;
+    const long long items = (long long) max_jobs * ((units + PW_WARPS - 1) / PW_WARPS);
+    kernel<<<(unsigned) (items < sm_count() ? items : sm_count()), PW_THREADS, pw_smem<NG>(), st>>>(p);
+    FNX_LAUNCH_OK("k_prompt_few");
+    return FNX_OK;
+}
+int prompt_few(int mode, int groups, const PnParams& p, int max_jobs, cudaStream_t st) {
+    FNX_REQUIRE(p.K % 256 == 0 && p.rows % 32 == 0, "prompt product: %d features x %d", p.rows, p.K);
+    return groups == 1 ? launch_few<1>(mode, p, max_jobs, st) : launch_few<2>(mode, p, max_jobs, st);
+}
+
+__global__ void __launch_bounds__(256) k_prompt_nat_rows(const float* __restrict__ x, const float* __restrict__ norm_w, int H, float eps, __half* __restrict__ xh, int few) {
     const float* xr = x + (size_t) blockIdx.x * H;
     __shared__ float ws[8];
     constexpr int HOLD = 4;   // the thread's pieces of up to 4,096 columns stay in registers
@@ -411,7 +621,7 @@ __global__ void __launch_bounds__(256) k_prompt_nat_rows(const float* __restrict
             q.x *= w.x * r; q.y *= w.y * r; q.z *= w.z * r; q.w *= w.w * r;
         }
         const __half2 a = __floats2half2_rn(q.x, q.z), b = __floats2half2_rn(q.y, q.w);   // (pn_slot: 0, 2, 1, 3)
-        *reinterpret_cast<uint2*>(xh + (size_t) blockIdx.x * H + pn_slot(i)) = make_uint2(pn_h2(a), pn_h2(b));
+        *reinterpret_cast<uint2*>(xh + (size_t) blockIdx.x * H + (few ? i : pn_slot(i))) = make_uint2(pn_h2(a), pn_h2(b));
     };
 #pragma unroll
     for (int j = 0; j < HOLD; ++j) {
@@ -421,8 +631,8 @@ __global__ void __launch_bounds__(256) k_prompt_nat_rows(const float* __restrict
     for (int i = (threadIdx.x + HOLD * 256) * 4; i < H; i += 1024) put(i, *reinterpret_cast<const float4*>(xr + i));
 }
 
-int prompt_nat_rows(const float* x, const float* norm_w, int T, int H, float eps, __half* xh, cudaStream_t st) {
-    k_prompt_nat_rows<<<T, 256, 0, st>>>(x, norm_w, H, eps, xh);
+int prompt_nat_rows(const float* x, const float* norm_w, int T, int H, float eps, __half* xh, bool few, cudaStream_t st) {
+    k_prompt_nat_rows<<<T, 256, 0, st>>>(x, norm_w, H, eps, xh, few);
     FNX_LAUNCH_OK("k_prompt_nat_rows");
     return FNX_OK;
 }

@@ -42,7 +42,13 @@ struct PnParams {
 // mode 1: outh = silu(x Wg^T) (x Wu^T); mode 0: out = x W^T over the jobs' pairs; mode 2: out (+)= x W^T over T rows.  max_jobs: as many
 // as there can be
 int prompt_nat(int mode, const PnParams& p, int max_jobs, cudaStream_t st);
-// xh[t] = f16(x[t] norm_w / rms(x[t])) in slot order (norm_w null: f16(x[t]))
-int prompt_nat_rows(const float* x, const float* norm_w, int T, int H, float eps, __half* xh, cudaStream_t st);
+// xh[t] = f16(x[t] norm_w / rms(x[t])) in slot order, or in prompt_few's (norm_w null: f16(x[t]))
+int prompt_nat_rows(const float* x, const float* norm_w, int T, int H, float eps, __half* xh, bool few, cudaStream_t st);
+// modes 1 and 0 for jobs of up to 8 groups rows (groups 1 or 2)
+int prompt_few(int mode, int groups, const PnParams& p, int max_jobs, cudaStream_t st);
+// row groups of eight that suit that many pairs over E experts (0: prompt_nat's jobs).  512 experts' matrices take 255 us in jobs of up to eight
+// rows, 275 us of up to sixteen, 303 us in prompt_nat's of 64 (and 382 us of up to 32 that way, where the products pass the decode): so as long as
+// nearly every expert's rows fit one job
+inline int prompt_few_groups(long long pairs, int E) { return pairs <= 3ll * E ? 1 : pairs <= 9ll * E ? 2 : 0; }
 
 }  // namespace fnxb
