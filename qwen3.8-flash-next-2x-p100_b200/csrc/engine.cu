@@ -90,7 +90,6 @@ struct SeqState {
     uint32_t step = 0;   // windows verified under the sampling rule (the Philox step of the next one)
     int last_T = 0;              // rows of the last verify window
     int kept = 0;                // rows kept by the last commit
-    int kept_pos0 = 0;           // position of the first kept row
 };
 
 }  // namespace fnxb
@@ -152,7 +151,10 @@ struct fnx_engine {
     Mat mtp_head;
     int* d_dvocab = nullptr;
     int dvn = 0;
-    int *h_stage = nullptr;      // pinned host staging
+    // What a window takes from the host and gives back, one block on each side (IO_*): one copy in, the error word's zero included, one out.
+    // h_stage: the host's, pinned, with room behind it for what other calls exchange (IO_TOTAL ..)
+    int *io = nullptr, *h_stage = nullptr;
+    uint32_t* h_step = nullptr;   // pinned: the sequences' Philox steps on their way to d_step
     std::map<uint64_t, cudaGraphExec_t> graphs;
     std::map<int, std::pair<__half**, __half**>> commit_tables;   // per sequence: device tables of its K and V caches
     void* comm = nullptr;
@@ -194,6 +196,10 @@ struct fnx_engine {
 };
 
 namespace fnxb {
+
+// the ints of fnx_engine::io: tokens, parents, lane tables, the error word; a window's result, the lanes' results
+constexpr int IO_M = FNX_MAX_ROWS, IO_TOK = 0, IO_PAR = IO_M, IO_LSEQ = 2 * IO_M, IO_LOWN = 3 * IO_M, IO_LROW = 4 * IO_M, IO_ERR = 5 * IO_M + 4, IO_RES = IO_ERR + 4,
+              IO_NRES = 1 + 2 * IO_M, IO_LRES = IO_RES + (IO_NRES + 3) / 4 * 4, IO_TOTAL = IO_LRES + IO_M * IO_NRES;
 
 template <typename T>
 static int dalloc(fnx_engine* e, T** p, size_t count, const char* name = nullptr) {
@@ -267,12 +273,6 @@ __global__ void k_gdn_params(float* dt, float* a, int nv) {
     }
 }
 // dst[j] = src[idx[j]] rows of n floats
-__global__ void k_gather_rows(float* __restrict__ dst, const float* __restrict__ src, const int* __restrict__ idx, int n) {
-    pdl_wait();
-    pdl_launch_dependents();
-    const int j = blockIdx.y, i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) dst[(size_t) j * n + i] = src[(size_t) idx[j] * n + i];
-}
 __global__ void k_add_rows(float* __restrict__ dst, const float* __restrict__ src, size_t n) {
     const size_t i = (size_t) blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) dst[i] += src[i];
@@ -367,10 +367,10 @@ __global__ void k_depths(const int* __restrict__ parent, int* __restrict__ depth
 // the context followed by the token the window emitted last (the next window's first row, as the reference's ctx
 // keeps it, engine/src/session.cpp:501), the state slot advances.  One block per attention layer + one for the
 // bookkeeping.
-__global__ void k_commit(__half* const* __restrict__ kcs, __half* const* __restrict__ vcs, int nlayer, int row_halves,
-                         const int* __restrict__ path, const int* __restrict__ tok, const int* __restrict__ emitted, int n,
-                         int* __restrict__ pos, int* __restrict__ cur, int NS, int* __restrict__ ctx, int* __restrict__ ctx_n) {
-    const int l = blockIdx.x, p0 = *pos;
+__device__ __forceinline__ void commit_body(__half* const* __restrict__ kcs, __half* const* __restrict__ vcs, int nlayer, int row_halves, const int* path,
+                                            const int* __restrict__ tok, const int* __restrict__ emitted, int n, int p0, int* __restrict__ cur, int NS,
+                                            int* __restrict__ ctx, int* __restrict__ ctx_n) {
+    const int l = blockIdx.x;
     if (l < nlayer) {
         for (int j = 0; j < n; ++j) {
             const int src = path[j];
@@ -393,10 +393,43 @@ __global__ void k_commit(__half* const* __restrict__ kcs, __half* const* __restr
         *cur = (*cur + 1 + path[n - 1]) % NS;
     }
 }
+__global__ void k_commit(__half* const* __restrict__ kcs, __half* const* __restrict__ vcs, int nlayer, int row_halves,
+                         const int* __restrict__ path, const int* __restrict__ tok, const int* __restrict__ emitted, int n,
+                         int* __restrict__ pos, int* __restrict__ cur, int NS, int* __restrict__ ctx, int* __restrict__ ctx_n) {
+    commit_body(kcs, vcs, nlayer, row_halves, path, tok, emitted, n, *pos, cur, NS, ctx, ctx_n);
+}
+// an engine's: the path comes with the launch and is left for the draft layer, with the position its rows start at; a prefix of a chain
+// (nlayer = 0) needs one block, which moves the position on as well
+struct RowList {
+    int v[FNX_MAX_ROWS];
+};
+__global__ void k_commit_window(__half* const* __restrict__ kcs, __half* const* __restrict__ vcs, int nlayer, int row_halves, const __grid_constant__ RowList path,
+                                const int* __restrict__ tok, const int* __restrict__ emitted, int n, int* __restrict__ pos, int* __restrict__ cur, int NS,
+                                int* __restrict__ ctx, int* __restrict__ ctx_n, int* __restrict__ path_out, int* __restrict__ mpos_base) {
+    pdl_wait();
+    const int p0 = *pos;
+    if ((int) blockIdx.x == nlayer) {
+        if ((int) threadIdx.x < n) path_out[threadIdx.x] = path.v[threadIdx.x];
+        if (threadIdx.x == 0) {
+            *mpos_base = p0;
+            if (nlayer == 0) *pos = p0 + n;
+        }
+    }
+    commit_body(kcs, vcs, nlayer, row_halves, path.v, tok, emitted, n, p0, cur, NS, ctx, ctx_n);
+}
 __global__ void k_advance_pos(int* pos, int n) {
     pdl_wait();
     pdl_launch_dependents();
     *pos += n;
+}
+// a draft chain's start: the kept rows of the main model, and the positions of its calls (n rows, then one each)
+__global__ void k_draft_start(float* __restrict__ dst, const float* __restrict__ src, const int* __restrict__ path, int H, int n, int k, const int* __restrict__ base,
+                              int* __restrict__ mpos) {
+    pdl_wait();
+    pdl_launch_dependents();
+    const int t = blockIdx.y, i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < H) dst[(size_t) t * H + i] = src[(size_t) path[t] * H + i];
+    if (t == 0 && i < k) mpos[i] = *base + (i ? n + i - 1 : 0);
 }
 // the prompt pass: the chunk's tokens joining the context; position and state slot afterwards
 __global__ void k_prompt_context(int* ctx, const int* ctx_n, const int* tok, int n) {
@@ -815,23 +848,24 @@ static int enqueue_verify(fnx_engine* e, int seq, int T, bool tree) {
 }
 
 // the draft layer's input rows: Rm = fc_hid(rms(src)) + fc_emb(rms(emb(tok)))   (fnx_mtp_input)
-static int enqueue_mtp_input(fnx_engine* e, int T, const float* src) {
+static int enqueue_mtp_input(fnx_engine* e, int T, const float* src, const int* tok) {
     const Dims d = dims(e->c);
     if (!e->mtp_fc_hid.nat)
-        return fnx_mtp_input(e->mtp_fc_hid.tiles, e->mtp_fc_emb.tiles, e->embed, e->mtp_hnorm, e->mtp_enorm, e->c.eps, src, d.H, e->d_mtok, T, d.H, e->Emb, e->Rm, e->err,
+        return fnx_mtp_input(e->mtp_fc_hid.tiles, e->mtp_fc_emb.tiles, e->embed, e->mtp_hnorm, e->mtp_enorm, e->c.eps, src, d.H, tok, T, d.H, e->Emb, e->Rm, e->err,
                              e->st);
     FNX_TRY(nat_rows_image(src, d.H, T, d.H, e->mtp_hnorm, e->img_x, e->st));
-    FNX_TRY(nat_embed_image(e->embed, e->d_mtok, T, d.H, e->Emb, e->mtp_enorm, e->img_r, e->st));
+    FNX_TRY(nat_embed_image(e->embed, tok, T, d.H, e->Emb, e->mtp_enorm, e->img_r, e->st));
     FNX_TRY(nat_dense(e->mtp_fc_hid.nat, d.H, d.H, e->img_x, true, e->c.eps, T, e->Rm, d.H, 0, e->st));
     return nat_dense(e->mtp_fc_emb.nat, d.H, d.H, e->img_r, true, e->c.eps, T, e->Rm, d.H, 1, e->st);
 }
 
-// one MTP call on T rows: the draft block on the input rows, the head on the last row
-static int enqueue_mtp(fnx_engine* e, int seq, int T, const float* src) {
+// one MTP call on T rows: the draft block on the input rows (rows of the main model or of the call before, and their tokens), the head on the
+// last row
+static int enqueue_mtp(fnx_engine* e, int seq, int T, const float* src, const int* tok, const int* mpos) {
     const Dims d = dims(e->c);
     const Mat& head = e->mtp_head.rows ? e->mtp_head : e->head;
-    FNX_TRY(enqueue_mtp_input(e, T, src));
-    FNX_TRY(enqueue_attention(e, e->mtp, e->Rm, T, seq, nullptr, nullptr, e->d_mpos));
+    FNX_TRY(enqueue_mtp_input(e, T, src, tok));
+    FNX_TRY(enqueue_attention(e, e->mtp, e->Rm, T, seq, nullptr, nullptr, mpos));
     bool img = false;
     FNX_TRY(enqueue_moe(e, e->mtp, e->Rm, T, &head, e->mtp_onorm, &img));
     return enqueue_dense(e, head, e->Rm + (size_t) (T - 1) * d.H, d.H, 1, e->mtp_onorm, e->logits, e->dvn, 0,
@@ -846,12 +880,13 @@ static int enqueue_mtp(fnx_engine* e, int seq, int T, const float* src) {
 
 // lanes kept as prefixes of their chains: the kept tokens and the emitted one join each sequence's context, positions and
 // state slots advance
-__global__ void k_commit_lanes(const int* __restrict__ lane_seq, const int* __restrict__ lane_row0, const int* __restrict__ keep,
+__global__ void k_commit_lanes(const int* __restrict__ lane_seq, const int* __restrict__ lane_row0, const __grid_constant__ RowList keep,
                                const int* __restrict__ tok, const int* __restrict__ results, int* __restrict__ pos, int* __restrict__ cur, int NS,
-                               int* __restrict__ ctx, size_t ctx_stride, int* __restrict__ ctx_n, int L) {
+                               int* __restrict__ ctx, size_t ctx_stride, int* __restrict__ ctx_n, int L, int* __restrict__ mrow0, int* __restrict__ mpos_base) {
+    pdl_wait();
     const int lane = threadIdx.x;
     if (lane >= L) return;
-    const int seq = lane_seq[lane], row0 = lane_row0[lane], n = keep[lane];
+    const int seq = lane_seq[lane], row0 = lane_row0[lane], n = keep.v[lane];
     const int* res = results + (size_t) lane * (1 + 2 * FNX_MAX_ROWS);
     int* c = ctx + (size_t) seq * ctx_stride;
     const int cn = ctx_n[seq];
@@ -859,7 +894,12 @@ __global__ void k_commit_lanes(const int* __restrict__ lane_seq, const int* __re
     c[cn + n] = res[1 + FNX_MAX_ROWS + n - 1];
     ctx_n[seq] = cn + n;
     cur[seq] = (cur[seq] + n) % NS;
+    mpos_base[lane] = pos[seq];   // for the draft layer: where the lane's kept rows start, and the rows of its first call
     pos[seq] += n;
+    int m = 0;
+    for (int j = 0; j < lane; ++j) m += keep.v[j];
+    mrow0[lane] = m;
+    if (lane == L - 1) mrow0[L] = m + n;
 }
 // the draft layer's first call: its rows are the lanes' kept rows (source rows and the tokens they emitted)
 __global__ void k_mtp_gather_lanes(float* __restrict__ dst, const float* __restrict__ src, int* __restrict__ mtok, const int* __restrict__ results,
@@ -882,24 +922,14 @@ __global__ void k_last_rows(float* __restrict__ dst, const float* __restrict__ s
     const int lane = blockIdx.y, i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < H) dst[(size_t) lane * H + i] = src[(size_t) (row0[lane + 1] - 1) * H + i];
 }
-// the draft layer's positions advance per lane: by the rows of its first call, then by one
-__global__ void k_mtp_advance_lanes(int* __restrict__ mpos, const int* __restrict__ lane_seq, const int* __restrict__ row0m, int L, int first) {
+// the positions of a draft chain's k calls, [k][n_seq]: the lanes' kept rows, then one row each
+__global__ void k_mtp_positions_lanes(int* __restrict__ mpos, const int* __restrict__ lane_seq, const int* __restrict__ row0m, const int* __restrict__ base, int L, int k,
+                                      int n_seq) {
     pdl_wait();
     pdl_launch_dependents();
     const int lane = threadIdx.x;
-    if (lane < L) mpos[lane_seq[lane]] += first ? row0m[lane + 1] - row0m[lane] : 1;
-}
-__global__ void k_mtp_set_pos_lanes(int* __restrict__ mpos, const int* __restrict__ lane_seq, const int* __restrict__ base, int L) {
-    pdl_wait();
-    pdl_launch_dependents();
-    const int lane = threadIdx.x;
-    if (lane < L) mpos[lane_seq[lane]] = base[lane];
-}
-__global__ void k_scatter_drafts(int* __restrict__ out, const int* __restrict__ best, int L, int k, int j) {
-    pdl_wait();
-    pdl_launch_dependents();
-    const int lane = threadIdx.x;
-    if (lane < L) out[lane * k + j] = best[lane];
+    if (lane >= L) return;
+    for (int j = 0; j < k; ++j) mpos[(size_t) j * n_seq + lane_seq[lane]] = base[lane] + (j ? row0m[lane + 1] - row0m[lane] + j - 1 : 0);
 }
 
 // mixer of one layer over the lanes' rows: R += out_proj(mixer(in_proj(rmsnorm(R))))
@@ -966,16 +996,16 @@ static int enqueue_verify_lanes(fnx_engine* e, int n_lanes, int rows, int T) {  
 }
 
 // one draft-layer call over lanes (rows per the table d_row0, Tm in all, at most max_rows per lane); the lanes' last rows go
-// through the head and their best tokens land in best_i[0 .. n_lanes)
-static int enqueue_mtp_lanes(fnx_engine* e, int n_lanes, int Tm, int max_rows, const int* d_row0, const float* src) {
+// through the head and their best tokens land in best[0 .. n_lanes)
+static int enqueue_mtp_lanes(fnx_engine* e, int n_lanes, int Tm, int max_rows, const int* d_row0, const float* src, const int* tok, const int* mpos, int* best) {
     const Dims d = dims(e->c);
-    FNX_TRY(enqueue_mtp_input(e, Tm, src));
-    FNX_TRY(enqueue_mixer_lanes(e, e->mtp, e->Rm, Tm, n_lanes, max_rows, e->d_lane_seq, d_row0, e->d_mpos_seq));
+    FNX_TRY(enqueue_mtp_input(e, Tm, src, tok));
+    FNX_TRY(enqueue_mixer_lanes(e, e->mtp, e->Rm, Tm, n_lanes, max_rows, e->d_lane_seq, d_row0, mpos));
     FNX_TRY(enqueue_moe(e, e->mtp, e->Rm, Tm));
     launch_dep(true, k_last_rows, dim3((d.H + 255) / 256, n_lanes), 256, 0, e->st, e->Rlast, e->Rm, d_row0, d.H);
     FNX_LAUNCH_OK("draft last rows");
     FNX_TRY(enqueue_dense(e, e->mtp_head.rows ? e->mtp_head : e->head, e->Rlast, d.H, n_lanes, e->mtp_onorm, e->logits, e->dvn, 0, e->img_r));
-    return fnx_argmax_mapped(e->logits, n_lanes, e->dvn, e->d_dvocab, e->best_i, nullptr, e->err, e->st);
+    return fnx_argmax_mapped(e->logits, n_lanes, e->dvn, e->d_dvocab, best, nullptr, e->err, e->st);
 }
 
 template <typename F>
@@ -1110,38 +1140,49 @@ extern "C" int fnx_engine_create(const fnx_model_config* cfg, fnx_engine** out) 
         FNX_TRY(dalloc(e, &e->best_v, d.MAXR, "buf.best_v"));
         FNX_TRY(dalloc(e, &e->cand_v, (size_t) d.MAXR * FNX_TOPK_N, "buf.cand_v"));
         FNX_TRY(dalloc(e, &e->cand_i, (size_t) d.MAXR * FNX_TOPK_N, "buf.cand_i"));
-        FNX_TRY(dalloc(e, &e->result, 1 + 2 * FNX_MAX_ROWS, "buf.result"));
-        FNX_TRY(dalloc(e, &e->d_tok, FNX_MAX_ROWS, "buf.tok"));
-        FNX_TRY(dalloc(e, &e->d_parent, FNX_MAX_ROWS, "buf.parent"));
         FNX_TRY(dalloc(e, &e->d_depth, FNX_MAX_ROWS, "buf.depth"));
         FNX_TRY(dalloc(e, &e->d_path, FNX_MAX_ROWS, "buf.path"));
         FNX_TRY(dalloc(e, &e->d_mtok, FNX_MAX_ROWS, "buf.mtp_tok"));
-        FNX_TRY(dalloc(e, &e->d_mpos, 1, "buf.mtp_pos"));
+        FNX_TRY(dalloc(e, &e->d_mpos, FNX_MAX_ROWS, "buf.mtp_pos"));
         FNX_TRY(dalloc(e, &e->d_mpos_base, FNX_MAX_ROWS, "buf.mtp_pos_base"));
         FNX_TRY(dalloc(e, &e->d_drafts, FNX_MAX_ROWS, "buf.draft"));
         FNX_TRY(dalloc(e, &e->d_step, c.n_seq, "seq.step"));
         FNX_TRY(dalloc(e, &e->d_lk, FNX_MAX_ROWS + 4, "buf.lookup"));
-        FNX_TRY(dalloc(e, &e->d_lane_seq, FNX_MAX_ROWS, "buf.lane_seq"));
-        FNX_TRY(dalloc(e, &e->d_lane_own, FNX_MAX_ROWS));
-        FNX_TRY(dalloc(e, &e->d_lane_row0, FNX_MAX_ROWS + 1, "buf.lane_row0"));
         FNX_TRY(dalloc(e, &e->d_mlane_row0, FNX_MAX_ROWS + 1, "buf.mtp_lane_row0"));
         FNX_TRY(dalloc(e, &e->d_ident_row0, FNX_MAX_ROWS + 1, "buf.ident_row0"));
         FNX_TRY(dalloc(e, &e->d_keep, FNX_MAX_ROWS, "buf.lane_keep"));
-        FNX_TRY(dalloc(e, &e->d_results, (size_t) FNX_MAX_ROWS * (1 + 2 * FNX_MAX_ROWS), "buf.lane_results"));
-        FNX_TRY(dalloc(e, &e->d_mpos_seq, c.n_seq, "seq.mtp_pos"));
+        FNX_TRY(dalloc(e, &e->d_mpos_seq, (size_t) c.n_seq * FNX_MAX_ROWS, "seq.mtp_pos"));
         FNX_TRY(dalloc(e, &e->d_ldrafts, (size_t) FNX_MAX_ROWS * FNX_MAX_ROWS, "buf.lane_drafts"));
         FNX_TRY(dalloc(e, &e->Rlast, (size_t) d.MAXR * d.H, "buf.Rlast"));
         FNX_TRY(dalloc(e, &e->d_pos, c.n_seq, "seq.pos"));
         FNX_TRY(dalloc(e, &e->d_cur, c.n_seq, "seq.cur"));
         FNX_TRY(dalloc(e, &e->d_ctx, (size_t) c.n_seq * e->cache_rows, "seq.ctx"));
         FNX_TRY(dalloc(e, &e->d_ctx_n, c.n_seq, "seq.ctx_n"));
-        FNX_TRY(dalloc(e, &e->err, 1, "buf.err"));
         FNX_TRY(dalloc(e, &e->d_stats, 2, "buf.stats"));
         void* sc = nullptr;
         const size_t sb = fnx_attn_scratch_bytes(d.MAXR, d.nq, d.hd);
         FNX_TRY(dalloc(e, (uint8_t**) &sc, sb, "buf.attn_scratch"));
         e->att_scratch = sc;
-        FNX_CUDA_OK(cudaHostAlloc((void**) &e->h_stage, sizeof(int) * 8 * FNX_MAX_ROWS, cudaHostAllocDefault));
+        FNX_TRY(dalloc(e, &e->io, IO_TOTAL));
+        auto piece = [&](const char* name, int at, size_t n) {
+            e->tensors[name] = {e->io + at, n * sizeof(int)};
+            return e->io + at;
+        };
+        e->d_tok = piece("buf.tok", IO_TOK, IO_M);
+        e->d_parent = piece("buf.parent", IO_PAR, IO_M);
+        e->d_lane_seq = piece("buf.lane_seq", IO_LSEQ, IO_M);
+        e->d_lane_own = e->io + IO_LOWN;
+        e->d_lane_row0 = piece("buf.lane_row0", IO_LROW, IO_M + 1);
+        e->err = (unsigned*) piece("buf.err", IO_ERR, 1);
+        e->result = piece("buf.result", IO_RES, IO_NRES);
+        e->d_results = piece("buf.lane_results", IO_LRES, (size_t) IO_M * IO_NRES);
+        FNX_CUDA_OK(cudaHostAlloc((void**) &e->h_stage, sizeof(int) * (IO_TOTAL + IO_M * IO_M + 64), cudaHostAllocDefault));
+        memset(e->h_stage, 0, sizeof(int) * IO_TOTAL);
+        FNX_CUDA_OK(cudaHostAlloc((void**) &e->h_step, sizeof(uint32_t) * c.n_seq, cudaHostAllocDefault));
+        memset(e->h_step, 0, sizeof(uint32_t) * c.n_seq);
+        int ident[IO_M + 1];
+        for (int j = 0; j <= IO_M; ++j) ident[j] = j;
+        FNX_CUDA_OK(cudaMemcpy(e->d_ident_row0, ident, sizeof ident, cudaMemcpyHostToDevice));
         return FNX_OK;
     };
     rc = body();
@@ -1172,6 +1213,7 @@ extern "C" void fnx_engine_destroy(fnx_engine* e) {
     if (e->d_bias_tok) cudaFree(e->d_bias_tok);
     if (e->d_bias_val) cudaFree(e->d_bias_val);
     if (e->h_stage) cudaFreeHost(e->h_stage);
+    if (e->h_step) cudaFreeHost(e->h_step);
     for (auto& g : e->stage) stage_free(g);
     if (e->ev0) cudaEventDestroy(e->ev0);
     if (e->ev1) cudaEventDestroy(e->ev1);
@@ -1278,17 +1320,14 @@ extern "C" int fnx_engine_verify(fnx_engine* e, int seq, const int* h_tok, const
     FNX_CUDA_OK(cudaStreamSynchronize(e->st));
     // the device error word reports THIS window: whatever an earlier window left was returned with its result (or is
     // still readable through fnx_engine_error_bits until now)
-    FNX_CUDA_OK(cudaMemsetAsync(e->err, 0, sizeof(unsigned), e->st));
     int* hs = e->h_stage;
-    memcpy(hs, h_tok, sizeof(int) * T);
-    FNX_CUDA_OK(cudaMemcpyAsync(e->d_tok, hs, sizeof(int) * T, cudaMemcpyHostToDevice, e->st));
-    if (h_parent) {
-        memcpy(hs + FNX_MAX_ROWS, h_parent, sizeof(int) * T);
-        FNX_CUDA_OK(cudaMemcpyAsync(e->d_parent, hs + FNX_MAX_ROWS, sizeof(int) * T, cudaMemcpyHostToDevice, e->st));
-    }
+    memcpy(hs + IO_TOK, h_tok, sizeof(int) * T);
+    if (h_parent) memcpy(hs + IO_PAR, h_parent, sizeof(int) * T);
+    hs[IO_ERR] = 0;
+    FNX_CUDA_OK(cudaMemcpyAsync(e->io, hs, sizeof(int) * IO_RES, cudaMemcpyHostToDevice, e->st));
     if (e->sampling_on) {   // the window's Philox step is a host count: a window replayed or run twice draws the same uniforms
-        hs[2 * FNX_MAX_ROWS] = (int) s.step++;
-        FNX_CUDA_OK(cudaMemcpyAsync(e->d_step + seq, hs + 2 * FNX_MAX_ROWS, sizeof(int), cudaMemcpyHostToDevice, e->st));
+        e->h_step[seq] = s.step++;
+        FNX_CUDA_OK(cudaMemcpyAsync(e->d_step + seq, e->h_step + seq, sizeof(uint32_t), cudaMemcpyHostToDevice, e->st));
     }
     const uint64_t key = ((uint64_t) 1 << 60) | ((uint64_t) seq << 20) | ((uint64_t) T << 1) | (tree ? 1 : 0);
     FNX_TRY(run_graph(e, key, [&]() { return enqueue_verify(e, seq, T, tree); }));
@@ -1296,12 +1335,11 @@ extern "C" int fnx_engine_verify(fnx_engine* e, int seq, const int* h_tok, const
     e->last_seq = seq;
     e->lane_seqs.clear();
     if (h_result) {
-        FNX_CUDA_OK(cudaMemcpyAsync(hs + 2 * FNX_MAX_ROWS, e->result, sizeof(int) * (1 + 2 * FNX_MAX_ROWS), cudaMemcpyDeviceToHost, e->st));
-        FNX_CUDA_OK(cudaMemcpyAsync(hs + 5 * FNX_MAX_ROWS, e->err, sizeof(unsigned), cudaMemcpyDeviceToHost, e->st));
+        FNX_CUDA_OK(cudaMemcpyAsync(hs + IO_ERR, e->io + IO_ERR, sizeof(int) * (IO_RES - IO_ERR + IO_NRES), cudaMemcpyDeviceToHost, e->st));
         FNX_CUDA_OK(cudaStreamSynchronize(e->st));
         FNX_CUDA_OK(cudaEventElapsedTime(&e->last_ms, e->ev0, e->ev1));
-        memcpy(h_result, hs + 2 * FNX_MAX_ROWS, sizeof(int) * (1 + 2 * FNX_MAX_ROWS));
-        const unsigned bits = (unsigned) hs[5 * FNX_MAX_ROWS];
+        memcpy(h_result, hs + IO_RES, sizeof(int) * IO_NRES);
+        const unsigned bits = (unsigned) hs[IO_ERR];
         if (bits) return fail(FNX_E_STATE, "verify: device error bits 0x%x (1: a bounded wait gave up, 2: non-finite value, 16: non-finite logits)", bits);
     }
     return FNX_OK;
@@ -1360,7 +1398,7 @@ extern "C" int fnx_engine_set_logit_rules(fnx_engine* e, const fnx_logit_rules* 
 extern "C" int fnx_engine_lookup(fnx_engine* e, int seq, int lk, int d1, int root, int* h_out, int* h_n) {
     FNX_REQUIRE(e && h_out && h_n && seq >= 0 && seq < e->c.n_seq && lk >= 0 && lk <= FNX_MAX_ROWS, "fnx_engine_lookup: bad arguments");
     FNX_CUDA_OK(cudaStreamSynchronize(e->st));
-    int* hs = e->h_stage;
+    int* hs = e->h_stage + IO_TOTAL;
     int* out_n = e->d_lk + FNX_MAX_ROWS;
     const int* d1p = nullptr;
     if (d1 >= 0) {
@@ -1546,10 +1584,9 @@ extern "C" int fnx_engine_commit(fnx_engine* e, int seq, const int* h_path, int 
     FNX_REQUIRE(n >= 1 && n <= s.last_T && h_path[0] == 0, "fnx_engine_commit: %d rows of a window of %d (the first kept row is row 0)", n, s.last_T);
     for (int j = 1; j < n; ++j) FNX_REQUIRE(h_path[j] > h_path[j - 1] && h_path[j] < s.last_T, "fnx_engine_commit: path[%d] = %d is not increasing", j, h_path[j]);
     const Dims d = dims(e->c);
-    FNX_CUDA_OK(cudaStreamSynchronize(e->st));
-    int* hs = e->h_stage;
-    memcpy(hs, h_path, sizeof(int) * n);
-    FNX_CUDA_OK(cudaMemcpyAsync(e->d_path, hs, sizeof(int) * n, cudaMemcpyHostToDevice, e->st));
+    RowList path{};
+    memcpy(path.v, h_path, sizeof(int) * n);
+    const bool chain = h_path[n - 1] == n - 1;   // (increasing from 0: the rows lie where they belong)
     // device tables of the attention layers' caches for this sequence (built once per sequence)
     auto& tables = e->commit_tables;
     const int key = seq;
@@ -1568,14 +1605,17 @@ extern "C" int fnx_engine_commit(fnx_engine* e, int seq, const int* h_path, int 
         tables[key] = {dk, dv};
     }
     int nattn = 0;
-    for (LayerW& L : e->layers) nattn += L.attn;
-    k_commit<<<nattn + 1, 256, 0, e->st>>>(tables[key].first, tables[key].second, nattn, d.kv_rows, e->d_path, e->d_tok, e->result + 1 + FNX_MAX_ROWS, n,
-                                           e->d_pos + seq, e->d_cur + seq, e->NS, e->d_ctx + (size_t) seq * e->cache_rows, e->d_ctx_n + seq);
+    if (!chain)
+        for (LayerW& L : e->layers) nattn += L.attn;
+    launch_dep(true, k_commit_window, dim3(nattn + 1), dim3(chain ? 32 : 256), 0, e->st, tables[key].first, tables[key].second, nattn, d.kv_rows, path, e->d_tok,
+               e->result + 1 + FNX_MAX_ROWS, n, e->d_pos + seq, e->d_cur + seq, e->NS, e->d_ctx + (size_t) seq * e->cache_rows, e->d_ctx_n + seq, e->d_path,
+               e->d_mpos_base);
     FNX_LAUNCH_OK("commit");
-    launch_dep(true, k_advance_pos, 1, 1, 0, e->st, e->d_pos + seq, n);
-    FNX_LAUNCH_OK("commit (position)");
+    if (!chain) {
+        launch_dep(true, k_advance_pos, 1, 1, 0, e->st, e->d_pos + seq, n);
+        FNX_LAUNCH_OK("commit (position)");
+    }
     s.kept = n;
-    s.kept_pos0 = s.pos;
     s.cur = (s.cur + 1 + h_path[n - 1]) % e->NS;
     s.pos += n;
     s.last_T = 0;
@@ -1589,39 +1629,33 @@ extern "C" int fnx_engine_draft(fnx_engine* e, int seq, int k, int* h_drafts) {
     FNX_REQUIRE(seq == e->last_seq, "fnx_engine_draft: sequence %d, but the window buffers hold sequence %d's last window", seq, e->last_seq);
     const Dims d = dims(e->c);
     const int n = s.kept;
-    FNX_CUDA_OK(cudaStreamSynchronize(e->st));
-    int* hs = e->h_stage;
-    hs[0] = s.kept_pos0;
-    FNX_CUDA_OK(cudaMemcpyAsync(e->d_mpos_base, hs, sizeof(int), cudaMemcpyHostToDevice, e->st));
+    int* hs = e->h_stage + IO_TOTAL;
     // The whole chain is one graph: the first call on the kept rows of the main model (gathered by path) with the tokens
     // the window emitted, then k - 1 single-row calls, each from the draft layer's own last row and the previous draft;
-    // tokens and positions advance on the device, the k drafts come back in one copy.
-    auto mtp_call = [&](int T, int* out) -> int {
-        FNX_TRY(enqueue_mtp(e, seq, T, e->Rsrc));
-        return fnx_argmax_mapped(e->logits, 1, e->dvn, e->d_dvocab, out, nullptr, e->err, e->st);
-    };
+    // positions are laid out at its start (from the one that the commit left: running it again gives the same result), the k
+    // drafts come back in one copy.
     auto chain = [&]() -> int {
-        // (the chain advances the position as it goes: it starts from a copy, so that running it again gives the same result)
-        FNX_CUDA_OK(cudaMemcpyAsync(e->d_mpos, e->d_mpos_base, sizeof(int), cudaMemcpyDeviceToDevice, e->st));
-        launch_dep(true, k_gather_rows, dim3((d.H + 255) / 256, n), 256, 0, e->st, e->Rsrc, e->R, e->d_path, d.H);
-        FNX_LAUNCH_OK("draft gather");
-        FNX_CUDA_OK(cudaMemcpyAsync(e->d_mtok, e->result + 1 + FNX_MAX_ROWS, sizeof(int) * n, cudaMemcpyDeviceToDevice, e->st));
-        FNX_TRY(mtp_call(n, e->d_drafts));
-        for (int j = 1; j < k; ++j) {
-            const int src_row = j == 1 ? n - 1 : 0;
-            FNX_CUDA_OK(cudaMemcpyAsync(e->Rsrc, e->Rm + (size_t) src_row * d.H, sizeof(float) * d.H, cudaMemcpyDeviceToDevice, e->st));
-            FNX_CUDA_OK(cudaMemcpyAsync(e->d_mtok, e->d_drafts + (j - 1), sizeof(int), cudaMemcpyDeviceToDevice, e->st));
-            launch_dep(true, k_advance_pos, 1, 1, 0, e->st, e->d_mpos, j == 1 ? n : 1);
-            FNX_LAUNCH_OK("draft position");
-            FNX_TRY(mtp_call(1, e->d_drafts + j));
+        launch_dep(true, k_draft_start, dim3((d.H + 255) / 256, n), 256, 0, e->st, e->Rsrc, e->R, e->d_path, d.H, n, k, e->d_mpos_base, e->d_mpos);
+        FNX_LAUNCH_OK("draft start");
+        for (int j = 0; j < k; ++j) {
+            const float* src = e->Rsrc;
+            if (j > 0) {
+                src = e->Rm + (size_t) (j == 1 ? n - 1 : 0) * d.H;
+                if (!e->mtp_fc_hid.nat) {   // (reads the rows again while it writes Rm; the other form has their image by then)
+                    FNX_CUDA_OK(cudaMemcpyAsync(e->Rsrc, src, sizeof(float) * d.H, cudaMemcpyDeviceToDevice, e->st));
+                    src = e->Rsrc;
+                }
+            }
+            FNX_TRY(enqueue_mtp(e, seq, j ? 1 : n, src, j ? e->d_drafts + j - 1 : e->result + 1 + FNX_MAX_ROWS, e->d_mpos + j));
+            FNX_TRY(fnx_argmax_mapped(e->logits, 1, e->dvn, e->d_dvocab, e->d_drafts + j, nullptr, e->err, e->st));
         }
         return FNX_OK;
     };
     FNX_TRY(run_graph(e, ((uint64_t) 3 << 60) | ((uint64_t) seq << 20) | ((uint64_t) k << 8) | (uint64_t) n, chain));
-    FNX_CUDA_OK(cudaMemcpyAsync(hs + 8, e->d_drafts, sizeof(int) * k, cudaMemcpyDeviceToHost, e->st));
+    FNX_CUDA_OK(cudaMemcpyAsync(hs, e->d_drafts, sizeof(int) * k, cudaMemcpyDeviceToHost, e->st));
     FNX_CUDA_OK(cudaStreamSynchronize(e->st));
     FNX_CUDA_OK(cudaEventElapsedTime(&e->last_ms, e->ev0, e->ev1));
-    memcpy(h_drafts, hs + 8, sizeof(int) * k);
+    memcpy(h_drafts, hs, sizeof(int) * k);
     s.kept = 0;
     return FNX_OK;
 }
@@ -1746,26 +1780,21 @@ extern "C" int fnx_engine_verify_lanes_rows(fnx_engine* e, int n_lanes, const in
     }
     FNX_REQUIRE(T <= e->c.max_rows, "fnx_engine_verify_lanes: %d rows in all (at most %d)", T, e->c.max_rows);
     FNX_CUDA_OK(cudaStreamSynchronize(e->st));
-    FNX_CUDA_OK(cudaMemsetAsync(e->err, 0, sizeof(unsigned), e->st));
     int* hs = e->h_stage;
-    memcpy(hs, h_tok, sizeof(int) * T);
-    FNX_CUDA_OK(cudaMemcpyAsync(e->d_tok, hs, sizeof(int) * T, cudaMemcpyHostToDevice, e->st));
-    int* ht = hs + FNX_MAX_ROWS;
-    for (int j = 0; j < n_lanes; ++j) ht[j] = h_seqs[j];
-    ht[FNX_MAX_ROWS] = 0;
-    for (int j = 0; j < n_lanes; ++j) ht[FNX_MAX_ROWS + j + 1] = ht[FNX_MAX_ROWS + j] + h_rows[j];
-    FNX_CUDA_OK(cudaMemcpyAsync(e->d_lane_seq, ht, sizeof(int) * n_lanes, cudaMemcpyHostToDevice, e->st));
-    {   // the table the mixers see on expert-parallel ranks: this rank's own sequences (sequence % ranks == rank)
-        int* ho = hs + 5 * FNX_MAX_ROWS;
-        for (int j = 0; j < n_lanes; ++j) ho[j] = h_seqs[j] % e->c.ep_size == e->c.ep_rank ? h_seqs[j] : -1;
-        FNX_CUDA_OK(cudaMemcpyAsync(e->d_lane_own, ho, sizeof(int) * n_lanes, cudaMemcpyHostToDevice, e->st));
+    memcpy(hs + IO_TOK, h_tok, sizeof(int) * T);
+    hs[IO_LROW] = 0;
+    for (int j = 0; j < n_lanes; ++j) {
+        hs[IO_LSEQ + j] = h_seqs[j];
+        // the table the mixers see on expert-parallel ranks: this rank's own sequences (sequence % ranks == rank)
+        hs[IO_LOWN + j] = h_seqs[j] % e->c.ep_size == e->c.ep_rank ? h_seqs[j] : -1;
+        hs[IO_LROW + j + 1] = hs[IO_LROW + j] + h_rows[j];
     }
-    FNX_CUDA_OK(cudaMemcpyAsync(e->d_lane_row0, ht + FNX_MAX_ROWS, sizeof(int) * (n_lanes + 1), cudaMemcpyHostToDevice, e->st));
-    if (e->sampling_on)
-        for (int j = 0; j < n_lanes; ++j) {
-            ht[3 * FNX_MAX_ROWS + j] = (int) e->seqs[h_seqs[j]].step++;
-            FNX_CUDA_OK(cudaMemcpyAsync(e->d_step + h_seqs[j], ht + 3 * FNX_MAX_ROWS + j, sizeof(int), cudaMemcpyHostToDevice, e->st));
-        }
+    hs[IO_ERR] = 0;
+    FNX_CUDA_OK(cudaMemcpyAsync(e->io, hs, sizeof(int) * IO_RES, cudaMemcpyHostToDevice, e->st));
+    if (e->sampling_on) {   // (every sequence's step goes along: the others' are set again before they are read)
+        for (int j = 0; j < n_lanes; ++j) e->h_step[h_seqs[j]] = e->seqs[h_seqs[j]].step++;
+        FNX_CUDA_OK(cudaMemcpyAsync(e->d_step, e->h_step, sizeof(uint32_t) * e->c.n_seq, cudaMemcpyHostToDevice, e->st));
+    }
     // one graph per layout (each lane's rows): the key is a hash of the counts under the lanes tag
     uint64_t hsh = 1469598103934665603ull;
     for (int j = 0; j < n_lanes; ++j) hsh = (hsh ^ (uint64_t) (h_rows[j] + 8 * j)) * 1099511628211ull;
@@ -1776,14 +1805,12 @@ extern "C" int fnx_engine_verify_lanes_rows(fnx_engine* e, int n_lanes, const in
     e->last_seq = -1;
     for (int j = 0; j < n_lanes; ++j) e->seqs[h_seqs[j]].last_T = h_rows[j];
     if (h_results) {
-        const size_t n = (size_t) n_lanes * (1 + 2 * FNX_MAX_ROWS);
-        std::vector<int> tmp(n + 1);
-        FNX_CUDA_OK(cudaMemcpyAsync(tmp.data(), e->d_results, sizeof(int) * n, cudaMemcpyDeviceToHost, e->st));
-        FNX_CUDA_OK(cudaMemcpyAsync(tmp.data() + n, e->err, sizeof(unsigned), cudaMemcpyDeviceToHost, e->st));
+        const size_t n = (size_t) n_lanes * IO_NRES;
+        FNX_CUDA_OK(cudaMemcpyAsync(hs + IO_ERR, e->io + IO_ERR, sizeof(int) * (IO_LRES - IO_ERR + n), cudaMemcpyDeviceToHost, e->st));
         FNX_CUDA_OK(cudaStreamSynchronize(e->st));
         FNX_CUDA_OK(cudaEventElapsedTime(&e->last_ms, e->ev0, e->ev1));
-        memcpy(h_results, tmp.data(), sizeof(int) * n);
-        if (tmp[n]) return fail(FNX_E_STATE, "verify_lanes: device error bits 0x%x", (unsigned) tmp[n]);
+        memcpy(h_results, hs + IO_LRES, sizeof(int) * n);
+        if (hs[IO_ERR]) return fail(FNX_E_STATE, "verify_lanes: device error bits 0x%x", (unsigned) hs[IO_ERR]);
     }
     return FNX_OK;
 }
@@ -1795,17 +1822,14 @@ extern "C" int fnx_engine_commit_lanes(fnx_engine* e, int n_lanes, const int* h_
         FNX_REQUIRE(h_seqs[j] == e->lane_seqs[j], "fnx_engine_commit_lanes: lane %d is sequence %d in the window, %d here", j, e->lane_seqs[j], h_seqs[j]);
         FNX_REQUIRE(h_keep[j] >= 1 && h_keep[j] <= e->lane_rows[j], "fnx_engine_commit_lanes: lane %d keeps %d of %d rows", j, h_keep[j], e->lane_rows[j]);
     }
-    FNX_CUDA_OK(cudaStreamSynchronize(e->st));
-    int* hs = e->h_stage;
-    memcpy(hs, h_keep, sizeof(int) * n_lanes);
-    FNX_CUDA_OK(cudaMemcpyAsync(e->d_keep, hs, sizeof(int) * n_lanes, cudaMemcpyHostToDevice, e->st));
-    k_commit_lanes<<<1, 32, 0, e->st>>>(e->d_lane_seq, e->d_lane_row0, e->d_keep, e->d_tok, e->d_results, e->d_pos, e->d_cur, e->NS, e->d_ctx, (size_t) e->cache_rows,
-                                        e->d_ctx_n, n_lanes);
+    RowList keep{};
+    memcpy(keep.v, h_keep, sizeof(int) * n_lanes);
+    launch_dep(true, k_commit_lanes, dim3(1), dim3(32), 0, e->st, e->d_lane_seq, e->d_lane_row0, keep, e->d_tok, e->d_results, e->d_pos, e->d_cur, e->NS, e->d_ctx,
+               (size_t) e->cache_rows, e->d_ctx_n, n_lanes, e->d_mlane_row0, e->d_mpos_base);
     FNX_LAUNCH_OK("commit lanes");
     for (int j = 0; j < n_lanes; ++j) {
         SeqState& s = e->seqs[h_seqs[j]];
         s.kept = h_keep[j];
-        s.kept_pos0 = s.pos;
         s.cur = (s.cur + h_keep[j]) % e->NS;
         s.pos += h_keep[j];
         s.last_T = 0;
@@ -1817,43 +1841,25 @@ extern "C" int fnx_engine_draft_lanes(fnx_engine* e, int n_lanes, const int* h_s
     FNX_REQUIRE(e && h_seqs && h_drafts && k >= 1 && k < e->c.max_rows, "fnx_engine_draft_lanes: bad arguments");
     FNX_REQUIRE(n_lanes == (int) e->lane_seqs.size() && n_lanes >= 1, "fnx_engine_draft_lanes: %d lanes, the last lane window had %d", n_lanes, (int) e->lane_seqs.size());
     const Dims d = dims(e->c);
-    FNX_CUDA_OK(cudaStreamSynchronize(e->st));
-    int* hs = e->h_stage;
+    int* hs = e->h_stage + IO_TOTAL;
     int Tm = 0, maxn = 0;
     for (int j = 0; j < n_lanes; ++j) {
         FNX_REQUIRE(h_seqs[j] == e->lane_seqs[j], "fnx_engine_draft_lanes: lane %d is sequence %d in the window, %d here", j, e->lane_seqs[j], h_seqs[j]);
         const SeqState& s = e->seqs[h_seqs[j]];
         FNX_REQUIRE(s.kept >= 1, "fnx_engine_draft_lanes: sequence %d: nothing committed since the last draft", h_seqs[j]);
-        hs[j] = Tm;
         Tm += s.kept;
         maxn = s.kept > maxn ? s.kept : maxn;
-        hs[FNX_MAX_ROWS + 1 + j] = s.kept_pos0;
     }
-    hs[n_lanes] = Tm;
-    for (int j = 0; j <= n_lanes; ++j) hs[2 * FNX_MAX_ROWS + 2 + j] = j;
-    FNX_CUDA_OK(cudaMemcpyAsync(e->d_mlane_row0, hs, sizeof(int) * (n_lanes + 1), cudaMemcpyHostToDevice, e->st));
-    FNX_CUDA_OK(cudaMemcpyAsync(e->d_ident_row0, hs + 2 * FNX_MAX_ROWS + 2, sizeof(int) * (n_lanes + 1), cudaMemcpyHostToDevice, e->st));
-    FNX_CUDA_OK(cudaMemcpyAsync(e->d_mpos_base, hs + FNX_MAX_ROWS + 1, sizeof(int) * n_lanes, cudaMemcpyHostToDevice, e->st));
-    // one graph for the whole chain: the first call on every lane's kept rows, then k - 1 calls of one row per lane
+    // one graph for the whole chain: the first call on every lane's kept rows, then k - 1 calls of one row per lane (positions and the first call's
+    // lane table from what the commit left: running it again gives the same result)
     auto chain = [&]() -> int {
-        // (the chain advances the lanes' positions as it goes: it starts from a copy, so that running it again gives the same result)
-        launch_dep(true, k_mtp_set_pos_lanes, 1, 32, 0, e->st, e->d_mpos_seq, e->d_lane_seq, e->d_mpos_base, n_lanes);
+        launch_dep(true, k_mtp_positions_lanes, 1, 32, 0, e->st, e->d_mpos_seq, e->d_lane_seq, e->d_mlane_row0, e->d_mpos_base, n_lanes, k, e->c.n_seq);
         FNX_LAUNCH_OK("draft positions (lanes)");
         launch_dep(true, k_mtp_gather_lanes, dim3((d.H + 255) / 256, Tm), 256, 0, e->st, e->Rsrc, e->R, e->d_mtok, e->d_results, e->d_lane_row0, e->d_mlane_row0, n_lanes, d.H);
         FNX_LAUNCH_OK("draft gather (lanes)");
-        FNX_TRY(enqueue_mtp_lanes(e, n_lanes, Tm, maxn, e->d_mlane_row0, e->Rsrc));
-        launch_dep(true, k_scatter_drafts, 1, 32, 0, e->st, e->d_ldrafts, e->best_i, n_lanes, k, 0);
-        FNX_LAUNCH_OK("draft scatter");
-        for (int j = 1; j < k; ++j) {
-            // each lane's source row: its draft-layer last row (compact in Rlast), its token: the previous draft
-            FNX_CUDA_OK(cudaMemcpyAsync(e->Rsrc, e->Rlast, sizeof(float) * (size_t) n_lanes * d.H, cudaMemcpyDeviceToDevice, e->st));
-            FNX_CUDA_OK(cudaMemcpyAsync(e->d_mtok, e->best_i, sizeof(int) * n_lanes, cudaMemcpyDeviceToDevice, e->st));
-            launch_dep(true, k_mtp_advance_lanes, 1, 32, 0, e->st, e->d_mpos_seq, e->d_lane_seq, e->d_mlane_row0, n_lanes, j == 1 ? 1 : 0);
-            FNX_LAUNCH_OK("draft positions (lanes)");
-            FNX_TRY(enqueue_mtp_lanes(e, n_lanes, n_lanes, 1, e->d_ident_row0, e->Rsrc));
-            launch_dep(true, k_scatter_drafts, 1, 32, 0, e->st, e->d_ldrafts, e->best_i, n_lanes, k, j);
-            FNX_LAUNCH_OK("draft scatter");
-        }
+        for (int j = 0; j < k; ++j)   // each lane's source row: its draft-layer last row (compact in Rlast), its token: the previous draft
+            FNX_TRY(enqueue_mtp_lanes(e, n_lanes, j ? n_lanes : Tm, j ? 1 : maxn, j ? e->d_ident_row0 : e->d_mlane_row0, j ? e->Rlast : e->Rsrc,
+                                      j ? e->d_ldrafts + (j - 1) * n_lanes : e->d_mtok, e->d_mpos_seq + (size_t) j * e->c.n_seq, e->d_ldrafts + j * n_lanes));
         return FNX_OK;
     };
     // the graph's shape depends on the lanes' kept counts: key on all of them
@@ -1861,12 +1867,13 @@ extern "C" int fnx_engine_draft_lanes(fnx_engine* e, int n_lanes, const int* h_s
     for (int j = 0; j < n_lanes; ++j) key = key * 1000003ull + (uint64_t) e->seqs[h_seqs[j]].kept;
     key |= (uint64_t) 5 << 60;
     FNX_TRY(run_graph(e, key, chain));
-    std::vector<int> tmp((size_t) n_lanes * k);
-    FNX_CUDA_OK(cudaMemcpyAsync(tmp.data(), e->d_ldrafts, sizeof(int) * tmp.size(), cudaMemcpyDeviceToHost, e->st));
+    FNX_CUDA_OK(cudaMemcpyAsync(hs, e->d_ldrafts, sizeof(int) * (size_t) n_lanes * k, cudaMemcpyDeviceToHost, e->st));
     FNX_CUDA_OK(cudaStreamSynchronize(e->st));
     FNX_CUDA_OK(cudaEventElapsedTime(&e->last_ms, e->ev0, e->ev1));
-    memcpy(h_drafts, tmp.data(), sizeof(int) * tmp.size());
-    for (int j = 0; j < n_lanes; ++j) e->seqs[h_seqs[j]].kept = 0;
+    for (int j = 0; j < n_lanes; ++j) {   // (one row of drafts a call on the device, one a lane here)
+        for (int i = 0; i < k; ++i) h_drafts[j * k + i] = hs[i * n_lanes + j];
+        e->seqs[h_seqs[j]].kept = 0;
+    }
     return FNX_OK;
 }
 

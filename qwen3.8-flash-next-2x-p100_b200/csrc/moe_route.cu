@@ -346,11 +346,12 @@ __global__ void __launch_bounds__(32) k_combine_nat(const float* __restrict__ pa
                                                     const float* __restrict__ img_norm_w) {
     const int blk = blockIdx.x, t = blockIdx.y, lane = threadIdx.x, KB = H / 256;
     const size_t col = (size_t) blk * 256 + lane * 8;
-    pdl_wait();
-    pdl_launch_dependents();
+    // ahead of the wait: the rows (last written by the output projection), the router's results (by the kernels before the two expert products)
     float* dst = out + (size_t) t * H + col;
     const float4 o0 = *reinterpret_cast<const float4*>(dst), o1 = *reinterpret_cast<const float4*>(dst + 4);
     const float shl = logits[(size_t) t * (E + 1) + E], mw = lane < K ? topw[t * K + lane] : 0.f;
+    pdl_wait();
+    pdl_launch_dependents();
     const float4* sh = reinterpret_cast<const float4*>(part + ((size_t) T * K + t) * H + col);
     const float4 h0 = sh[0], h1 = sh[1];
     unsigned long long s[8];
