@@ -44,6 +44,8 @@ CTX, K_DRAFT, P_BAD = 4096, 4, 0.28
 C2_CTX, C2_LOOKUP = 32768, 15            # configuration 2: context and the longest lookup branch
 C3_TOKENS = 38912                          # configuration 3: the cold prompt
 C4_CTX, C4_SEQS, C4_LANES = 131072, 8, 4   # configuration 4: context per sequence, sequences, lanes per window
+# A window's copies: tokens, parents, lane tables and the error word in one block of 168 words; the error word and a result of 65 words back
+WINDOW_IN, WINDOW_OUT = 4 * 168, 4 * (4 + 65)
 E_B = 1351680          # bytes of one expert: (2*512*2048 + 2048*512) * 110 / 256
 # DRAM bytes per expert job of the gate|up launch, from an ncu capture of one launch (dram__bytes_read.sum +
 # dram__bytes_write.sum = 42.02 MB for 46 jobs; the algorithmic figure is 901,120 bytes per job)
@@ -144,7 +146,10 @@ def cpu_leg(F, O, steps, threads):
     cfg = F.flash_next_config(n_layer=4, max_ctx=CTX + 256, max_rows=8)
     eng = F.Engine(cfg)
     eng.init_synthetic(seed=0, sigma=0.02)
-    om = OracleModel(F, O, eng, cfg, with_mtp=False)
+    twin = F.Engine(cfg)   # (the oracle's weights: asking the engine itself would move its matrices to the interchange layout)
+    twin.init_synthetic(seed=0, sigma=0.02)
+    om = OracleModel(F, O, twin, cfg, with_mtp=False)
+    twin.close()
     rng = np.random.default_rng(1)
     # ---- parity at the benchmark's dimensions
     prompt = rng.integers(0, cfg.vocab, size=12).tolist()
@@ -324,8 +329,8 @@ def run_config4(a, F, eng, cfg, rank, world, local, use_peer, emit=True):
                        "timing": "per-step K/V reads (tens of GB) and expert weights far larger than the 126 MB L2; CUDA events on the engine's stream",
                        "parallelism": f"ep{world}", "layers": a.layers},
             "clocks": clk, "gpu_launches": int(c1[0] - c0[0]),
-            "e2e": {"value": tokens / (e2e_ms * 1e-3), "unit": "tok/s", "h2d_bytes_per_step": len(groups) * (4 * T + 4 * (2 * C4_LANES + 1) + 4 * C4_LANES * 2),
-                    "d2h_bytes_per_step": len(groups) * (4 * C4_LANES * 65 + 4 + 4 * C4_LANES * K_DRAFT), "wall_ms_per_step": wall * 1e3 / a.steps},
+            "e2e": {"value": tokens / (e2e_ms * 1e-3), "unit": "tok/s", "h2d_bytes_per_step": len(groups) * (WINDOW_IN + 4 * C4_SEQS),
+                    "d2h_bytes_per_step": len(groups) * (4 * (4 + 68) + 4 * C4_LANES * 65 + 4 * C4_LANES * K_DRAFT), "wall_ms_per_step": wall * 1e3 / a.steps},
             "verify_window_us": verify_ms * 1e3 / (a.steps * len(groups)), "accepted_per_offered": accepted / max(1, offered), "tokens_per_step": tokens / a.steps,
             "tokens_crc": zlib.crc32(np.asarray(stream, np.int64).tobytes()), "ep_sum": "none" if world == 1 else ("peer-memory" if use_peer else "nccl"),
             "window_bytes": {"kv_read": kv, "routed_jobs_per_window": jobs_per_window, "expert_bytes": (jobs_per_window + a.layers * 5) * E_B / max(1, world)}}
@@ -498,7 +503,7 @@ def run_config2(a, F, eng, cfg, rank, world, local, use_peer):
                                     "(seed 2: 60% of positions copy earlier spans of 20-200 tokens), greedy acceptance, rollback to the last accepted node"),
                        "timing": "inputs far larger than the 126 MB L2; CUDA events on the engine's stream", "parallelism": f"ep{world}", "layers": a.layers},
             "clocks": clk, "gpu_launches": int(c1[0] - c0[0]),
-            "e2e": {"value": tokens / (e2e_ms * 1e-3), "unit": "tok/s", "h2d_bytes_per_step": 4 * 2 * 20 + 16, "d2h_bytes_per_step": 4 * 65 + 4 + 4 * K_DRAFT + 4 * 34,
+            "e2e": {"value": tokens / (e2e_ms * 1e-3), "unit": "tok/s", "h2d_bytes_per_step": WINDOW_IN + 8, "d2h_bytes_per_step": WINDOW_OUT + 4 * K_DRAFT + 4 * 34,
                     "wall_ms_per_step": wall * 1e3 / a.steps},
             "verify_window_us": verify_ms * 1e3 / a.steps, "rows_per_window": rows / a.steps, "lookup_rows_per_window": lk_rows / a.steps,
             "lookup_rows_kept_per_window": lk_kept / a.steps, "tokens_per_step": tokens / a.steps,
@@ -750,7 +755,7 @@ def main():
             "ms_per_step": dev_ms / a.steps, "higher_is_better": True, "scaling": "strong", "vs_baseline": None, "dtype": "int8xint3->f32",
             "data": "synthetic", "config": bench_config(workload, world, a.layers),
             "clocks": clk, "gpu_launches": int(launches),
-            "e2e": {"value": e2e, "unit": "tok/s", "h2d_bytes_per_step": 4 * (1 + K_DRAFT) + 4 * (1 + K_DRAFT) + 8, "d2h_bytes_per_step": 4 * 65 + 4 + 4 * K_DRAFT,
+            "e2e": {"value": e2e, "unit": "tok/s", "h2d_bytes_per_step": WINDOW_IN, "d2h_bytes_per_step": WINDOW_OUT + 4 * K_DRAFT,
                     "wall_ms_per_step": wall * 1e3 / a.steps},
             "verify_step_us": verify_ms * 1e3, "accepted_per_offered": accepted / max(1, offered), "tokens_per_step": tokens / a.steps,
             "tokens_crc": zlib.crc32(np.asarray(want[:done], np.int64).tobytes()),
@@ -803,7 +808,7 @@ def main():
         per_launch_s = e0.elapsed_time(e1) * 1e-3 / (reps * a.layers)
         bytes_per_launch = sum(njobs) / len(njobs) * gu_b
         ach = bytes_per_launch / per_launch_s / 1e9
-        line["roofline"] = {"bound": "hbm", "kernel": "k_iq3s_mmv<1, gate|up>", "achieved": ach, "peak": hbm_peak, "unit": "GB/s", "frac": ach / hbm_peak,
+        line["roofline"] = {"bound": "hbm", "kernel": "k_iq3s_mmv<1, gate|up> (fnx_moe_gate_up; the engine's windows run k_nat_mmv on its own layout)", "achieved": ach, "peak": hbm_peak, "unit": "GB/s", "frac": ach / hbm_peak,
                             "peak_kind": peak_kind, "traffic": NCU_TRAFFIC_PER_JOB * sum(njobs) / len(njobs),
                             "traffic_source": "ncu dram__bytes_read+write of one gate|up launch (46 jobs, 4-layer case): 42.02 MB, scaled by jobs per launch", "us_per_launch": per_launch_s * 1e6, "jobs_per_launch": sum(njobs) / len(njobs),
                             "algorithmic_bytes_per_launch": bytes_per_launch}

@@ -95,6 +95,32 @@ def test_prompts_agree_between_the_layouts(n):
         b.close()
 
 
+@pytest.mark.parametrize("E,n", [(32, 1), (32, 8), (32, 9), (32, 48),          # one and two groups of eight rows to a block: 2n <= 3E, 2n <= 9E
+                                 (32, 49), (32, 64), (32, 65), (32, 144), (32, 145),
+                                 (2, 63), (2, 64), (2, 65), (2, 129)])    # weights through tensor memory: jobs of 64 rows
+def test_prompt_products_at_the_edges_of_their_jobs(E, n):
+    """Every row of a prompt, in both layouts, at the lengths where a job or a row group is full, one short or one over.
+
+    (A prompt's last token is a window's, so n rows are n + 1 tokens.)  With a router of zeros every row picks experts 0 and 1, in both engines alike, so these two have exactly n rows and no near tie
+    can part the layouts.  The keys of an attention layer behind one DeltaNet layer and its experts are compared row by row: what
+    the products read and leave is rounded to f16 three times on the way there (norms, SwiGLU, the key), 2^-11 of a value each."""
+    cfg = small(n_layer=2, attn_every=2, n_expert=E, top_k=2, max_ctx=256)
+    a, b = pair(cfg)
+    try:
+        toks = np.random.default_rng(6).integers(0, cfg.vocab, size=n + 1).tolist()
+        keys = []
+        for e in (a, b):
+            for l in range(2):
+                e.tensor(f"l{l}.router", torch.float32)[:E * cfg.hidden] = 0.0
+            e.prompt(toks)
+            keys.append(e.tensor("l1.k_cache", torch.float16).float().reshape(-1, cfg.n_kv_head * cfg.head_dim)[:n].cpu().numpy())
+        err = np.linalg.norm(keys[0] - keys[1], axis=1) / np.linalg.norm(keys[1], axis=1)
+        assert err.max() < 3 * 2.0 ** -11, (int(err.argmax()), float(err.max()))
+    finally:
+        a.close()
+        b.close()
+
+
 def test_a_matrix_asked_for_comes_back_in_the_interchange_layout():
     """Bit for bit the tiles that the same seeded weights give through the operators, padded rows included."""
     cfg = small(draft_vocab=1040)
