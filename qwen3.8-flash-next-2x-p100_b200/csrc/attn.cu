@@ -44,6 +44,7 @@ __global__ void k_attn_prep_append(const AttnPrep a) {
 // a block a row and head, with its pow and barriers, took 2.2 ms for 38,912 rows against 0.24 ms of them.
 constexpr int PREP_ROWS = 8, PREP_WARPS = 8;
 __global__ void __launch_bounds__(PREP_WARPS * 32) k_attn_prep_rows(const AttnPrep a, int T) {
+    pdl_begin();
     constexpr int HD = 256, NROT = 64;
     const int h = blockIdx.x, lane = threadIdx.x & 31, ta = ((int) blockIdx.y * PREP_WARPS + (threadIdx.x >> 5)) * PREP_ROWS, tb = min(T, ta + PREP_ROWS), pos0 = *a.pos;
     if (h >= a.nq + a.nkv) {   // a V head: store only
@@ -114,7 +115,7 @@ __global__ void __launch_bounds__(PREP_WARPS * 32) k_attn_prep_rows(const AttnPr
 
 int attn_prep(const AttnPrep& a, int rows, int n_lanes, bool early, cudaStream_t st) {
     if (rows > FNX_MAX_ROWS && !a.lane_seq && !a.depth && a.hd == 256 && a.nrot == 64) {
-        k_attn_prep_rows<<<dim3(a.nq + 2 * a.nkv, (rows + PREP_ROWS * PREP_WARPS - 1) / (PREP_ROWS * PREP_WARPS)), PREP_WARPS * 32, 0, st>>>(a, rows);
+        FNX_CUDA_OK(launch_after(k_attn_prep_rows, dim3(a.nq + 2 * a.nkv, (rows + PREP_ROWS * PREP_WARPS - 1) / (PREP_ROWS * PREP_WARPS)), dim3(PREP_WARPS * 32), 0, st, a, rows));
         FNX_LAUNCH_OK("k_attn_prep_rows");
         return FNX_OK;
     }

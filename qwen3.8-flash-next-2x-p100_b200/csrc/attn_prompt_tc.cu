@@ -57,6 +57,7 @@ __global__ void __launch_bounds__(TA_THREADS, 1) k_attn_prompt_tc(const float* _
                                                                  const __half* __restrict__ vc, float* __restrict__ out, int T, int nq, int nkv,
                                                                  const int* __restrict__ pos0p, unsigned* __restrict__ err,
                                                                  const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v) {
+    pdl_wait();   // (as in the DeltaNet scan, the successor starts at the end)
     extern __shared__ __align__(1024) uint8_t smem[];
     TaShared& sh = *reinterpret_cast<TaShared*>(smem);
     uint8_t* ring = smem + TA_HEAD;
@@ -308,7 +309,7 @@ int attn_prompt_tc_launch(const float* qg, int ldq, const __half* kc, const __ha
     CUtensorMap map_k, map_v;
     FNX_TRY(attn_kv_map(&map_k, kc, nkv, 1 << 24));
     FNX_TRY(attn_kv_map(&map_v, vc, nkv, 1 << 24));
-    k_attn_prompt_tc<<<dim3((T + TA_POS - 1) / TA_POS, nkv), TA_THREADS, TA_SMEM, st>>>(qg, ldq, kc, vc, out, T, nq, nkv, pos0, err, map_k, map_v);
+    FNX_CUDA_OK(launch_after(k_attn_prompt_tc, dim3((T + TA_POS - 1) / TA_POS, nkv), dim3(TA_THREADS), TA_SMEM, st, qg, ldq, kc, vc, out, T, nq, nkv, pos0, err, map_k, map_v));
     FNX_LAUNCH_OK("fnx_attn_prompt (tensor-core form)");
     return FNX_OK;
 }

@@ -433,10 +433,12 @@ __global__ void k_draft_start(float* __restrict__ dst, const float* __restrict__
 }
 // the prompt pass: the chunk's tokens joining the context; position and state slot afterwards
 __global__ void k_prompt_context(int* ctx, const int* ctx_n, const int* tok, int n) {
+    pdl_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) ctx[*ctx_n + i] = tok[i];
 }
 __global__ void k_prompt_advance(int* pos, int* cur, int* ctx_n, int n, int NS) {
+    pdl_begin();
     *pos += n;
     *cur = (*cur + n) % NS;
     *ctx_n += n;
@@ -453,6 +455,8 @@ int prompt_dense(const void* W, bool nat, int rows, int cols, const float* x, in
 int prompt_moe(const void* Wgu, size_t gu_stride, const void* Wsh_gu, bool gu_nat, const void* Wdn, size_t dn_stride, const void* Wsh_dn, bool dn_nat, int e_base, int E,
                int K, int e_lo, int e_hi, int add_shared, const int* topi, const float* topw, const float* logits, const float* x, const float* norm_w, float eps, int T,
                int H, int F, float* out, int accumulate, void* scratch, unsigned* err, cudaStream_t st);
+int router_rows(const float* Wr, const float* x, const float* norm_w, float eps, int T, int E, int H, int K, float* logits, int* topi, float* topw, void* scratch,
+                unsigned* err, bool early, cudaStream_t st);
 int router_window(const float* Wr, const float* x, const float* norm_w, float eps, int T, int E, int H, int K, int e_lo, int e_hi, int add_shared, float* logits, int* topi,
                   float* topw, fnx_job* jobs, int* njobs, unsigned long long* stats, unsigned* err, uint8_t* img, bool early, cudaStream_t st);
 int moe_combine_nat(const float* part, const int* topi, const float* topw, const float* logits, int T, int E, int H, int K, float* R, uint8_t* img, const float* img_norm_w,
@@ -1517,7 +1521,7 @@ extern "C" int fnx_engine_prompt(fnx_engine* e, int seq, const int* h_tok, int n
             FNX_TRY(prompt_dense(L.w_out.nat ? L.w_out.nat : L.w_out.tiles, L.w_out.nat != nullptr, d.H, mixw_l, e->pmix, nt, nullptr, e->c.eps, e->pR, d.H, 1, e->p_dense_scratch, e->err, e->st));
             mark(0, false);
             mark(PH_ROUTER, true);
-            FNX_TRY(fnx_router_rows(L.wr, e->pR, L.norm2, e->c.eps, nt, d.E, d.H, d.K, e->plogits, e->ptopi, e->ptopw, e->p_router_scratch, e->err, e->st));
+            FNX_TRY(router_rows(L.wr, e->pR, L.norm2, e->c.eps, nt, d.E, d.H, d.K, e->plogits, e->ptopi, e->ptopw, e->p_router_scratch, e->err, true, e->st));
             mark(0, false);
             mark(PH_MOE, true);
             {
@@ -1546,9 +1550,9 @@ extern "C" int fnx_engine_prompt(fnx_engine* e, int seq, const int* h_tok, int n
                 fprintf(stderr, "\n");
             }
         }
-        k_prompt_context<<<(nt + 255) / 256, 256, 0, e->st>>>(e->d_ctx + (size_t) seq * e->cache_rows, e->d_ctx_n + seq, e->d_ptok, nt);
+        FNX_CUDA_OK(launch_after(k_prompt_context, dim3((nt + 255) / 256), dim3(256), 0, e->st, e->d_ctx + (size_t) seq * e->cache_rows, e->d_ctx_n + seq, e->d_ptok, nt));
         FNX_LAUNCH_OK("prompt context");
-        k_prompt_advance<<<1, 1, 0, e->st>>>(e->d_pos + seq, e->d_cur + seq, e->d_ctx_n + seq, nt, e->NS);
+        FNX_CUDA_OK(launch_after(k_prompt_advance, dim3(1), dim3(1), 0, e->st, e->d_pos + seq, e->d_cur + seq, e->d_ctx_n + seq, nt, e->NS));
         FNX_LAUNCH_OK("prompt advance");
         e->launches += 3;   // embedding, context, advance
         FNX_CUDA_OK(cudaStreamSynchronize(e->st));   // the token copy's source and the chunk buffers are free again

@@ -61,12 +61,22 @@ inline cudaError_t launch_dep(bool early, void (*kernel)(KArgs...), dim3 grid, d
     cfg.numAttrs = early ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
 }
+// A kernel that starts with pdl_begin() reads nothing ahead and may follow anything: only its launch overlaps its predecessor's end (1 to 2 us
+// a launch in a prompt's chain of some fifteen kernels a layer).
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_after(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
+    return launch_dep(true, kernel, grid, block, smem, st, args...);
+}
 #endif
 
 #if defined(__CUDACC__)
 // ---- programmatic dependent launch (no-ops when the launch carried no such dependency)
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_begin() {
+    pdl_wait();
+    pdl_launch_dependents();
+}
 
 // ---- warp helpers
 __device__ __forceinline__ float warp_sum(float v) {

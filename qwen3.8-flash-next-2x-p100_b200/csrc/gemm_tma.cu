@@ -84,6 +84,7 @@ __device__ __forceinline__ void gt_ld32(uint32_t taddr, float (&v)[32]) {
 template <int NA, int NPROD>
 __global__ void __launch_bounds__(GT_THREADS, 1) k_gemm_tma(const GtParams p, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                                                            const __grid_constant__ CUtensorMap map_wl, const __grid_constant__ CUtensorMap map_xl) {
+    pdl_begin();
     using Sh = GtShape<NA, NPROD>;
     constexpr int STAGES = Sh::STAGES, PARTS = Sh::PARTS;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -217,6 +218,7 @@ struct GtJobParams {
 
 template <int MODE>
 __global__ void __launch_bounds__(GT_THREADS, 1) k_gemm_tma_jobs(const GtJobParams p, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x) {
+    pdl_begin();
     using Sh = GtShape<2, 1>;
     constexpr int STAGES = Sh::STAGES, NA = 2;
     const int j = blockIdx.y;
@@ -363,13 +365,13 @@ int gemm_tma_launch(const __half* w, const __half* wl, const __half* x, const __
         FNX_TRY(gt_map(&mxl, xl, T, K, GT_N));
         using Sh = GtShape<1, 3>;
         if (int rc = set_smem_limit((const void*) k_gemm_tma<1, 3>, Sh::SMEM)) return rc;
-        k_gemm_tma<1, 3><<<dim3((rows + GT_M - 1) / GT_M, (T + GT_N - 1) / GT_N), GT_THREADS, Sh::SMEM, st>>>(p, mw, mx, mwl, mxl);
+        FNX_CUDA_OK(launch_after(k_gemm_tma<1, 3>, dim3((rows + GT_M - 1) / GT_M, (T + GT_N - 1) / GT_N), dim3(GT_THREADS), Sh::SMEM, st, p, mw, mx, mwl, mxl));
     } else {
         mwl = mw;
         mxl = mx;
         using Sh = GtShape<2, 1>;
         if (int rc = set_smem_limit((const void*) k_gemm_tma<2, 1>, Sh::SMEM)) return rc;
-        k_gemm_tma<2, 1><<<dim3((rows + 2 * GT_M - 1) / (2 * GT_M), (T + GT_N - 1) / GT_N), GT_THREADS, Sh::SMEM, st>>>(p, mw, mx, mwl, mxl);
+        FNX_CUDA_OK(launch_after(k_gemm_tma<2, 1>, dim3((rows + 2 * GT_M - 1) / (2 * GT_M), (T + GT_N - 1) / GT_N), dim3(GT_THREADS), Sh::SMEM, st, p, mw, mx, mwl, mxl));
     }
     FNX_LAUNCH_OK("k_gemm_tma");
     return FNX_OK;
@@ -388,12 +390,12 @@ int gemm_tma_experts(const __half* gu16, const __half* dn16, int slots, const __
     FNX_TRY(gt_map(&mw, gu16, slots * 2 * F, H, GT_M));
     FNX_TRY(gt_map(&mx, x_sorted, entries, H, GT_N));
     p.R = 2 * F; p.F = F; p.K = H; p.h_sorted = h_sorted;
-    k_gemm_tma_jobs<1><<<dim3(F / GT_M, max_jobs), GT_THREADS, Sh::SMEM, st>>>(p, mw, mx);
+    FNX_CUDA_OK(launch_after(k_gemm_tma_jobs<1>, dim3(F / GT_M, max_jobs), dim3(GT_THREADS), Sh::SMEM, st, p, mw, mx));
     FNX_LAUNCH_OK("k_gemm_tma_jobs (gate|up)");
     FNX_TRY(gt_map(&mw, dn16, slots * H, F, GT_M));
     FNX_TRY(gt_map(&mx, h_sorted, entries, F, GT_N));
     p.R = H; p.K = F; p.part = part; p.H = H; p.h_sorted = nullptr;
-    k_gemm_tma_jobs<0><<<dim3(H / (2 * GT_M), max_jobs), GT_THREADS, Sh::SMEM, st>>>(p, mw, mx);
+    FNX_CUDA_OK(launch_after(k_gemm_tma_jobs<0>, dim3(H / (2 * GT_M), max_jobs), dim3(GT_THREADS), Sh::SMEM, st, p, mw, mx));
     FNX_LAUNCH_OK("k_gemm_tma_jobs (down)");
     return FNX_OK;
 }

@@ -210,6 +210,7 @@ struct PfParams {
 // MODE 0: out = x W^T (down).  MODE 1: out = silu(x Wg^T) * (x Wu^T) (gate|up; W = [gate (rows); up (rows)]).
 template <int MODE>
 __global__ void __launch_bounds__(PF_BLOCK, 1) k_pf_gemm(const PfParams p) {
+    pdl_begin();
     extern __shared__ __align__(128) uint8_t smem[];
     constexpr int NA = MODE == 1 ? 2 : 1;                      // weight tiles per stage
     constexpr int STAGE = NA * PF_TILE_A + PF_TILE_B;
@@ -395,6 +396,7 @@ __global__ void __launch_bounds__(PF_BLOCK, 1) k_pf_gemm(const PfParams p) {
 constexpr int PF_PAIRS = 4096, PF_MAXE = 1024;
 // per expert: how many pairs picked it (cnt starts from zeros)
 __global__ void __launch_bounds__(512) k_pf_count(const int* __restrict__ topi, int n, int e_lo, int ne, int* __restrict__ cnt) {
+    pdl_begin();
     __shared__ int hist[PF_MAXE];
     for (int e = threadIdx.x; e < ne; e += 512) hist[e] = 0;
     __syncthreads();
@@ -409,12 +411,12 @@ __global__ void __launch_bounds__(512) k_pf_count(const int* __restrict__ topi, 
         if (hist[e]) atomicAdd(&cnt[e], hist[e]);
 }
 
-// one block: the experts' first entries and jobs of `per` rows (ascending expert order, then the shared expert's)
-__global__ void __launch_bounds__(PF_MAXE) k_pf_plan(const int* __restrict__ cnt, int ne, int e_lo, int E, int T, int TKp, int add_shared, int* __restrict__ base,
-                                                     PfJob* __restrict__ jobs, int* __restrict__ njobs, int* __restrict__ order, int per) {
+// one block: the experts' first entries (e's for thread e) and jobs of `per` rows (ascending expert order, then the shared expert's)
+__device__ __forceinline__ int pf_plan(int c, int ne, int e_lo, int E, int T, int TKp, int add_shared, PfJob* __restrict__ jobs, int* __restrict__ njobs,
+                                       int* __restrict__ order, int per) {
     __shared__ int2 ws[32];
     const int e = threadIdx.x, lane = e & 31, warp = e >> 5;
-    const int c = e < ne ? cnt[e] : 0, nj = (c + per - 1) / per;
+    const int nj = (c + per - 1) / per;
     int2 s = make_int2(c, nj);   // running sums: entries, jobs
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -442,7 +444,6 @@ __global__ void __launch_bounds__(PF_MAXE) k_pf_plan(const int* __restrict__ cnt
     const int2 before = warp ? ws[warp - 1] : make_int2(0, 0), all = ws[31];
     const int entry = before.x + s.x - c;
     if (e < ne) {
-        base[e] = entry;
         for (int j = 0; j < nj; ++j) jobs[before.y + s.y - nj + j] = PfJob{e_lo + e, min(per, c - j * per), entry + j * per};
     }
     const int sj = add_shared ? (T + per - 1) / per : 0;
@@ -451,10 +452,18 @@ __global__ void __launch_bounds__(PF_MAXE) k_pf_plan(const int* __restrict__ cnt
         for (int j = e; j < sj; j += PF_MAXE) jobs[all.y + j] = PfJob{E, min(per, T - j * per), all.x + j * per};
     }
     if (e == 0) njobs[0] = all.y + sj;
+    return entry;
+}
+__global__ void __launch_bounds__(PF_MAXE) k_pf_plan(const int* __restrict__ cnt, int ne, int e_lo, int E, int T, int TKp, int add_shared, int* __restrict__ base,
+                                                     PfJob* __restrict__ jobs, int* __restrict__ njobs, int* __restrict__ order, int per) {
+    pdl_begin();
+    const int e = threadIdx.x, entry = pf_plan(e < ne ? cnt[e] : 0, ne, e_lo, E, T, TKp, add_shared, jobs, njobs, order, per);
+    if (e < ne) base[e] = entry;
 }
 
 // the experts' entries into order[base ..) (base moves on)
 __global__ void __launch_bounds__(512) k_pf_fill(const int* __restrict__ topi, int n, int e_lo, int ne, int* __restrict__ base, int* __restrict__ order) {
+    pdl_begin();
     __shared__ int hist[PF_MAXE];
     for (int e = threadIdx.x; e < ne; e += 512) hist[e] = 0;
     __syncthreads();
@@ -477,8 +486,37 @@ __global__ void __launch_bounds__(512) k_pf_fill(const int* __restrict__ topi, i
         if (ex[j] >= 0) order[hist[ex[j]] + at[j]] = i0 + threadIdx.x + j * 512;
 }
 
+// the three above for up to PF_ONE pairs, in one block: 3,330 pairs took 20 us in four launches (with the zeroing of the counts), of which 11 were
+// kernels; past PF_ONE the one block's passes over the pairs cost more than the launches
+constexpr int PF_ONE = 8192;
+__global__ void __launch_bounds__(PF_MAXE) k_pf_route(const int* __restrict__ topi, int n, int ne, int e_lo, int E, int T, int add_shared, PfJob* __restrict__ jobs,
+                                                      int* __restrict__ njobs, int* __restrict__ order, int per) {
+    pdl_begin();
+    __shared__ int hist[PF_MAXE];
+    const int tid = threadIdx.x;
+    hist[tid] = 0;
+    __syncthreads();
+    constexpr int PER = PF_ONE / PF_MAXE;
+    int ex[PER], at[PER];
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+        const int i = tid + j * PF_MAXE;
+        ex[j] = i < n ? topi[i] - e_lo : -1;
+        if (ex[j] >= ne) ex[j] = -1;
+    }
+#pragma unroll
+    for (int j = 0; j < PER; ++j) at[j] = ex[j] >= 0 ? atomicAdd(&hist[ex[j]], 1) : 0;
+    __syncthreads();
+    hist[tid] = pf_plan(hist[tid], ne, e_lo, E, T, n, add_shared, jobs, njobs, order, per);   // (only this thread read its count)
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < PER; ++j)
+        if (ex[j] >= 0) order[hist[ex[j]] + at[j]] = tid + j * PF_MAXE;
+}
+
 // xh[t] = f16(x[t] * norm_w / rms(x[t]))   (norm_w null: f16(x[t]))
 __global__ void k_pf_xnorm(const float* __restrict__ x, const float* __restrict__ norm_w, int H, float eps, __half* __restrict__ xh) {
+    pdl_begin();
     const float* xr = x + (size_t) blockIdx.x * H;
     __shared__ float ws[32], s_r;
     float ss = 0.f;
@@ -510,6 +548,7 @@ __global__ void k_pf_xnorm(const float* __restrict__ x, const float* __restrict_
 // out[t] (+)= sum_k topw[t][k] part[t Kp + k] + sigmoid(logit[t][E]) part[T Kp + t]
 __global__ void k_pf_combine(const float* __restrict__ part, const int* __restrict__ topi, const float* __restrict__ topw, const float* __restrict__ logits,
                              int T, int E, int H, int Kp, int e_lo, int e_hi, int add_shared, float* __restrict__ out, int accumulate) {
+    pdl_begin();
     // a thread owns four columns of one row; the picks' weights first, then every addend's 16-byte load in flight at once
     const int t = blockIdx.y, i = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
     if (i >= H) return;
@@ -551,6 +590,7 @@ __global__ void k_pf_combine(const float* __restrict__ part, const int* __restri
 // bytes, scales and half arithmetic), for the products that take their weights by tensor copies (gemm_tma.cu).  One warp per
 // 16 x 256 tile block.
 __global__ void __launch_bounds__(256) k_pf_decode_f16(const uint8_t* __restrict__ W, int rows, int K, __half* __restrict__ out) {
+    pdl_begin();
     __shared__ uint32_t table[512 * PF_REP];
     for (int i = threadIdx.x; i < 512 * PF_REP; i += blockDim.x) table[i] = g_grid_pf[i / PF_REP];
     __syncthreads();
@@ -578,6 +618,7 @@ __global__ void __launch_bounds__(256) k_pf_decode_f16(const uint8_t* __restrict
 }
 // the same from a matrix in the engine's own layout; one warp per half tile
 __global__ void __launch_bounds__(256) k_pf_decode_nat(const uint8_t* __restrict__ W, int rows, int K, __half* __restrict__ out) {
+    pdl_begin();
     const int lane = threadIdx.x & 31, KB = K / 256, n16 = rows / 16;
     const size_t nblk = (size_t) n16 * KB;
     const int g = lane >> 2, q = lane & 3;
@@ -600,14 +641,15 @@ __global__ void __launch_bounds__(256) k_pf_decode_nat(const uint8_t* __restrict
 static int pf_decode_f16_launch(const void* W, bool nat, int rows, int K, __half* out, cudaStream_t st) {
     const size_t nblk = (size_t) (rows / 16) * (K / 256);
     const unsigned blocks = (unsigned) (nblk / 8 < 148 * 8 ? (nblk + 7) / 8 : 148 * 8);
-    if (nat) k_pf_decode_nat<<<blocks, 256, 0, st>>>((const uint8_t*) W, rows, K, out);
-    else k_pf_decode_f16<<<blocks, 256, 0, st>>>((const uint8_t*) W, rows, K, out);
+    if (nat) FNX_CUDA_OK(launch_after(k_pf_decode_nat, dim3(blocks), dim3(256), 0, st, (const uint8_t*) W, rows, K, out));
+    else FNX_CUDA_OK(launch_after(k_pf_decode_f16, dim3(blocks), dim3(256), 0, st, (const uint8_t*) W, rows, K, out));
     FNX_LAUNCH_OK("k_pf_decode_f16");
     return FNX_OK;
 }
 
 // the job list of a dense product over T rows: job j = rows [256 j, 256 j + 256) of "expert" 0, entries in row order
 __global__ void k_pf_dense_jobs(int T, PfJob* __restrict__ jobs, int* __restrict__ njobs, int* __restrict__ order) {
+    pdl_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x, nj = (T + PF_N - 1) / PF_N;
     if (i < T) order[i] = i;
     if (i < nj) jobs[i] = PfJob{0, min(PF_N, T - i * PF_N), i * PF_N};
@@ -616,6 +658,7 @@ __global__ void k_pf_dense_jobs(int T, PfJob* __restrict__ jobs, int* __restrict
 
 // f16 rows in place between natural and slot order (pn_slot), a warp per 32 columns
 __global__ void __launch_bounds__(256) k_pf_reorder(__half* __restrict__ h, size_t groups, int to_slots) {
+    pdl_begin();
     const size_t g = (size_t) blockIdx.x * 8 + (threadIdx.x >> 5);
     if (g >= groups) return;
     const int lane = threadIdx.x & 31, slot = pn_slot(lane);
@@ -635,6 +678,7 @@ static size_t pf_align(size_t v) { return (v + 255) & ~(size_t) 255; }
 // the rows of the job list's entries, in entry order: x_sorted[pos] = xh[token of order[pos]] (a routed pair t K + k: token t; a
 // shared-expert entry n + t: token t), so that a job's rows are consecutive for the tensor copies
 __global__ void __launch_bounds__(256) k_pf_gather_rows(const __half* __restrict__ xh, const int* __restrict__ order, int n, int Kp, int H, __half* __restrict__ xs) {
+    pdl_begin();
     const int pos = blockIdx.x, pair = order[pos], t = pair < n ? pair / Kp : pair - n;
     const uint4* src = reinterpret_cast<const uint4*>(xh + (size_t) t * H);
     uint4* dst = reinterpret_cast<uint4*>(xs + (size_t) pos * H);
@@ -684,20 +728,26 @@ int prompt_moe(const void* Wgu, size_t gu_stride, const void* Wsh_gu, bool gu_na
     const int ne = e_hi - e_lo, n = T * K;
     const int few = gu_nat && dn_nat ? prompt_few_groups(n, E) : 0;
     const int per = few ? 8 * few : gu_nat || dn_nat ? PN_N : PF_N, pb = (n + PF_PAIRS - 1) / PF_PAIRS;
-    if (ne > 0) {
+    const bool one = n <= PF_ONE;
+    if (one) {
+        FNX_CUDA_OK(launch_after(k_pf_route, dim3(1), dim3(PF_MAXE), 0, st, topi, n, ne, e_lo, E, T, add_shared, jobs, njobs, order, per));
+        FNX_LAUNCH_OK("k_pf_route");
+    } else if (ne > 0) {
         FNX_CUDA_OK(cudaMemsetAsync(cnt, 0, sizeof(int) * ne, st));
-        k_pf_count<<<pb, 512, 0, st>>>(topi, n, e_lo, ne, cnt);
+        FNX_CUDA_OK(launch_after(k_pf_count, dim3(pb), dim3(512), 0, st, topi, n, e_lo, ne, cnt));
         FNX_LAUNCH_OK("k_pf_count");
     }
-    k_pf_plan<<<1, PF_MAXE, 0, st>>>(cnt, ne, e_lo, E, T, n, add_shared, base, jobs, njobs, order, per);
-    FNX_LAUNCH_OK("k_pf_plan");
-    if (ne > 0) {
-        k_pf_fill<<<pb, 512, 0, st>>>(topi, n, e_lo, ne, base, order);
+    if (!one) {
+        FNX_CUDA_OK(launch_after(k_pf_plan, dim3(1), dim3(PF_MAXE), 0, st, cnt, ne, e_lo, E, T, n, add_shared, base, jobs, njobs, order, per));
+        FNX_LAUNCH_OK("k_pf_plan");
+    }
+    if (!one && ne > 0) {
+        FNX_CUDA_OK(launch_after(k_pf_fill, dim3(pb), dim3(512), 0, st, topi, n, e_lo, ne, base, order));
         FNX_LAUNCH_OK("k_pf_fill");
     }
     if (gu_nat) FNX_TRY(prompt_nat_rows(x, norm_w, T, H, eps, xh, few != 0, st));
     else {
-        k_pf_xnorm<<<T, 256, 0, st>>>(x, norm_w, H, eps, xh);
+        FNX_CUDA_OK(launch_after(k_pf_xnorm, dim3(T), dim3(256), 0, st, x, norm_w, H, eps, xh));
         FNX_LAUNCH_OK("k_pf_xnorm");
     }
     // Interchange tiles from 1,024 rows on, with every expert on this rank and stacked without gaps: the experts' matrices decoded to f16
@@ -711,11 +761,11 @@ int prompt_moe(const void* Wgu, size_t gu_stride, const void* Wsh_gu, bool gu_na
         FNX_TRY(pf_decode_f16_launch(Wsh_gu, false, 2 * F, H, gu16 + (size_t) E * 2 * F * H, st));
         FNX_TRY(pf_decode_f16_launch(Wdn, false, E * H, F, dn16, st));
         FNX_TRY(pf_decode_f16_launch(Wsh_dn, false, H, F, dn16 + (size_t) E * H * F, st));
-        k_pf_gather_rows<<<(unsigned) pairs, 256, 0, st>>>(xh, order, n, K, H, xs);
+        FNX_CUDA_OK(launch_after(k_pf_gather_rows, dim3((unsigned) pairs), dim3(256), 0, st, xh, order, n, K, H, xs));
         FNX_LAUNCH_OK("k_pf_gather_rows");
         const int nj = (int) ((size_t) n / PF_N) + ne + (T + PF_N - 1) / PF_N;
         FNX_TRY(gemm_tma_experts(gu16, dn16, E + 1, xs, hbuf, part, jobs, njobs, order, nj, (int) pairs, H, F, err, st));
-        k_pf_combine<<<dim3((H / 4 + 255) / 256, T), 256, 0, st>>>(part, topi, topw, logits, T, E, H, K, e_lo, e_hi, add_shared, out, accumulate);
+        FNX_CUDA_OK(launch_after(k_pf_combine, dim3((H / 4 + 255) / 256, T), dim3(256), 0, st, part, topi, topw, logits, T, E, H, K, e_lo, e_hi, add_shared, out, accumulate));
         FNX_LAUNCH_OK("k_pf_combine");
         return FNX_OK;
     }
@@ -732,11 +782,11 @@ int prompt_moe(const void* Wgu, size_t gu_stride, const void* Wsh_gu, bool gu_na
     } else {
         FNX_TRY(set_smem_limit((const void*) k_pf_gemm<1>, (int) pf_smem(1)));
         p.W = (const uint8_t*) Wgu; p.expert_stride = gu_stride; p.Wsh = (const uint8_t*) Wsh_gu; p.x = xh; p.rows = F; p.K = H; p.outh = hbuf;
-        k_pf_gemm<1><<<dim3(nj, F / PF_M), PF_BLOCK, pf_smem(1), st>>>(p);
+        FNX_CUDA_OK(launch_after(k_pf_gemm<1>, dim3(nj, F / PF_M), dim3(PF_BLOCK), pf_smem(1), st, p));
         FNX_LAUNCH_OK("k_pf_gemm (gate|up)");
     }
     if (gu_nat != dn_nat) {   // (one of the two matrices was asked for in the interchange layout)
-        k_pf_reorder<<<(unsigned) ((pairs * F / 32 + 7) / 8), 256, 0, st>>>(hbuf, pairs * F / 32, dn_nat);
+        FNX_CUDA_OK(launch_after(k_pf_reorder, dim3((unsigned) ((pairs * F / 32 + 7) / 8)), dim3(256), 0, st, hbuf, pairs * F / 32, dn_nat));
         FNX_LAUNCH_OK("k_pf_reorder");
     }
     if (dn_nat) {
@@ -745,10 +795,10 @@ int prompt_moe(const void* Wgu, size_t gu_stride, const void* Wsh_gu, bool gu_na
     } else {
         FNX_TRY(set_smem_limit((const void*) k_pf_gemm<0>, (int) pf_smem(0)));
         p.W = (const uint8_t*) Wdn; p.expert_stride = dn_stride; p.Wsh = (const uint8_t*) Wsh_dn; p.x = hbuf; p.rows = H; p.K = F; p.out = part; p.outh = nullptr;
-        k_pf_gemm<0><<<dim3(nj, H / PF_M), PF_BLOCK, pf_smem(0), st>>>(p);
+        FNX_CUDA_OK(launch_after(k_pf_gemm<0>, dim3(nj, H / PF_M), dim3(PF_BLOCK), pf_smem(0), st, p));
         FNX_LAUNCH_OK("k_pf_gemm (down)");
     }
-    k_pf_combine<<<dim3((H / 4 + 255) / 256, T), 256, 0, st>>>(part, topi, topw, logits, T, E, H, K, e_lo, e_hi, add_shared, out, accumulate);
+    FNX_CUDA_OK(launch_after(k_pf_combine, dim3((H / 4 + 255) / 256, T), dim3(256), 0, st, part, topi, topw, logits, T, E, H, K, e_lo, e_hi, add_shared, out, accumulate));
     FNX_LAUNCH_OK("k_pf_combine");
     return FNX_OK;
 }
@@ -796,20 +846,20 @@ int prompt_dense(const void* W, bool nat, int rows, int cols, const float* x, in
         q.W = (const uint8_t*) W; q.T = T; q.x = xh; q.rows = rows; q.K = cols; q.out = y; q.ldo = ldy; q.accumulate = accumulate; q.err = err;
         return prompt_nat(2, q, (T + PN_N - 1) / PN_N, st);
     }
-    k_pf_xnorm<<<T, 256, 0, st>>>(x, norm_w, cols, eps, xh);
+    FNX_CUDA_OK(launch_after(k_pf_xnorm, dim3(T), dim3(256), 0, st, x, norm_w, cols, eps, xh));
     FNX_LAUNCH_OK("k_pf_xnorm");
     if (T >= pf_tma_rows()) {   // the matrix to f16 once, then one product with both operands by tensor copies
         FNX_TRY(pf_decode_f16_launch(W, nat, rows, cols, w16, st));
         return gemm_tma_launch(w16, nullptr, xh, nullptr, y, ldy, T, rows, cols, accumulate, 1.0f, err, st);
     }
-    k_pf_dense_jobs<<<(T + 255) / 256, 256, 0, st>>>(T, jobs, njobs, order);
+    FNX_CUDA_OK(launch_after(k_pf_dense_jobs, dim3((T + 255) / 256), dim3(256), 0, st, T, jobs, njobs, order));
     FNX_LAUNCH_OK("k_pf_dense_jobs");
     FNX_TRY(set_smem_limit((const void*) k_pf_gemm<0>, (int) pf_smem(0)));
     PfParams p{};
     p.W = (const uint8_t*) W; p.expert_stride = 0; p.e_base = 0; p.E = 1; p.Wsh = nullptr;
     p.jobs = jobs; p.njobs = njobs; p.order = order; p.TKp = T; p.Kp = 1; p.x = xh; p.rows = rows; p.K = cols; p.out = y; p.outh = nullptr; p.err = err;
     p.ldo = ldy; p.accumulate = accumulate;
-    k_pf_gemm<0><<<dim3(nj, (rows + PF_M - 1) / PF_M), PF_BLOCK, pf_smem(0), st>>>(p);
+    FNX_CUDA_OK(launch_after(k_pf_gemm<0>, dim3(nj, (rows + PF_M - 1) / PF_M), dim3(PF_BLOCK), pf_smem(0), st, p));
     FNX_LAUNCH_OK("k_pf_gemm (dense)");
     return FNX_OK;
 }

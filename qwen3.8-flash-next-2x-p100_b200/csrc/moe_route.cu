@@ -23,10 +23,8 @@ namespace fnxb {
 // other kernel (the weights, the norm weights) is loaded before the rows are waited for.  f32 products and sums.
 // Windows: 4 expert rows a block (129 blocks), block y = 0 of block column t also leaves row t's image (nat_image.cuh) for the experts'
 // products; bound by the rows' way to every block (T x 8 KB each) and latency: 5 rows 14 -> 4.5 us, 20 rows 34 -> 10 us (with the pick
-// 10 and 20), when one launch did both, eight rows at a time through shared memory.
-// Prompts: 16 expert rows a block, so that the rows cross L2 33 times instead of 129; bound by the products from a few hundred rows
-// on (8 rows a block walking all 513 expert rows took 145 us at any number of rows up to 1,023).
-constexpr int RT_ROWS = 4, RT_PROMPT_ROWS = 16;
+// 10 and 20), when one launch did both, eight rows at a time through shared memory.  Prompts: k_router_tiles below.
+constexpr int RT_ROWS = 4;
 
 template <int ROWS, int THREADS>
 __global__ void __launch_bounds__(THREADS, 1) k_router_logits(const float* __restrict__ Wr, const float* __restrict__ x, const float* __restrict__ norm_w, float eps, int T,
@@ -149,6 +147,139 @@ __global__ void __launch_bounds__(THREADS, 1) k_router_logits(const float* __res
     }
 }
 
+// ---- the prompt form: blocks of 16 expert rows whose weights stay in registers, 16 rows of the prompt at a time, on mma.sync.m16n8k8 in
+// tf32.  Both operands are split into a high part (the nearest 11 bits) and the 11 bits below it; high x high, high x low and low x
+// high keep the products good to 2^-22, as f32 does; sums of 16 columns go on in f32 (the tensor core's own sums are cut off, not rounded:
+// over 64 columns the logits came out up to 1.2e-6 small), those of the 128-column slices in double.  Warp = one slice; lane q of a quad holds columns 4 q .. 4 q + 3 of every 16 (the order of columns within a product is
+// free), so rows and weights are loaded 16 bytes at a time; two pieces of the rows are in flight, across row tiles.
+// Bound by the rows' way to the blocks (33 blocks read each: 128 KB a tile, two thirds of what an SM gets from L2), close behind by the splits
+// (integer-logic pipe) and the products.  333 rows x 513 x 2,048: 29 us (11 TFLOP/s of f32 products; 13 us at L2's 6.5 TB/s); f32 products with
+// their 31 shuffles per two rows took 53.
+constexpr int RP_ROWS = 16, RP_TOK = 16, RP_SLICE = 128, RP_IT = RP_SLICE / 16, RP_AHEAD = 2, RP_LD = 20, RP_WARPS = 2048 / RP_SLICE;
+
+__device__ __forceinline__ void rp_split(float v, uint32_t& hi, uint32_t& lo) {
+    hi = (__float_as_uint(v) + 0x1000u) & 0xFFFFE000u;
+    lo = __float_as_uint(v - __uint_as_float(hi)) & 0xFFFFE000u;
+}
+__device__ __forceinline__ void rp_mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+__global__ void __launch_bounds__(RP_WARPS * 32, 1) k_router_tiles(const float* __restrict__ Wr, const float* __restrict__ x, const float* __restrict__ norm_w, float eps, int T, int E,
+                                                         int H, float* __restrict__ logits, unsigned* __restrict__ err) {
+    __shared__ __align__(16) float psum_[2][RP_WARPS][RP_TOK][RP_LD];
+    __shared__ float sqs_[2][RP_WARPS][RP_TOK];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3, NW = H / RP_SLICE, row0 = blockIdx.x * RP_ROWS;
+    const int c = warp * RP_SLICE + q * 4, tiles = (T + RP_TOK - 1) / RP_TOK;
+    float4 w[2][RP_IT];   // times the norm weights
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        const bool live = row0 + 8 * j + g <= E;
+        const float* p = Wr + (size_t) (live ? row0 + 8 * j + g : 0) * H + c;
+#pragma unroll
+        for (int i = 0; i < RP_IT; ++i) w[j][i] = live ? __ldg(reinterpret_cast<const float4*>(p + 16 * i)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    if (norm_w) {
+#pragma unroll
+        for (int i = 0; i < RP_IT; ++i) {
+            const float4 n = __ldg(reinterpret_cast<const float4*>(norm_w + c + 16 * i));
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                w[j][i].x *= n.x; w[j][i].y *= n.y; w[j][i].z *= n.z; w[j][i].w *= n.w;
+            }
+        }
+    }
+    pdl_wait();
+    pdl_launch_dependents();
+    // (rows past the last one repeat it: their sums are not written)
+    auto row_of = [&](int tile, int h) { return x + (size_t) min(tile * RP_TOK + g + 8 * h, T - 1) * H + c; };
+    int tile = blockIdx.y;
+    const float *p0 = row_of(tile, 0), *p1 = row_of(tile, 1);
+    float4 xa[RP_AHEAD], xb[RP_AHEAD];
+#pragma unroll
+    for (int i = 0; i < RP_AHEAD; ++i) {
+        xa[i] = *reinterpret_cast<const float4*>(p0 + 16 * i);
+        xb[i] = *reinterpret_cast<const float4*>(p1 + 16 * i);
+    }
+    for (int buf = 0; tile < tiles; tile += gridDim.y, buf ^= 1) {
+        const int next = min(tile + (int) gridDim.y, tiles - 1);
+        const float *n0 = row_of(next, 0), *n1 = row_of(next, 1);
+        float sum[2][4] = {}, hl[2][4] = {}, ss0 = 0.f, ss1 = 0.f;
+#pragma unroll
+        for (int i0 = 0; i0 < RP_IT; i0 += RP_AHEAD) {
+#pragma unroll
+            for (int k = 0; k < RP_AHEAD; ++k) {
+                float hh[2][4] = {};
+                const int i = i0 + k;
+                const float a[4] = {xa[k].x, xa[k].y, xa[k].z, xa[k].w}, b[4] = {xb[k].x, xb[k].y, xb[k].z, xb[k].w};
+                const int ni = i + RP_AHEAD;
+                xa[k] = *reinterpret_cast<const float4*>((ni < RP_IT ? p0 : n0) + 16 * (ni % RP_IT));
+                xb[k] = *reinterpret_cast<const float4*>((ni < RP_IT ? p1 : n1) + 16 * (ni % RP_IT));
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    ss0 = fmaf(a[e], a[e], ss0);
+                    ss1 = fmaf(b[e], b[e], ss1);
+                }
+#pragma unroll
+                for (int st = 0; st < 2; ++st) {
+                    uint32_t ah[4], al[4];
+                    rp_split(a[2 * st], ah[0], al[0]);
+                    rp_split(b[2 * st], ah[1], al[1]);
+                    rp_split(a[2 * st + 1], ah[2], al[2]);
+                    rp_split(b[2 * st + 1], ah[3], al[3]);
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        uint32_t bh0, bl0, bh1, bl1;
+                        float w0 = st ? w[j][i].z : w[j][i].x, w1 = st ? w[j][i].w : w[j][i].y;
+                        asm volatile("" : "+f"(w0), "+f"(w1));   // (split here: split before the loop they would live in local memory)
+                        rp_split(w0, bh0, bl0);
+                        rp_split(w1, bh1, bl1);
+                        rp_mma(hh[j], ah, bh0, bh1);
+                        rp_mma(hl[j], ah, bl0, bl1);
+                        rp_mma(hl[j], al, bh0, bh1);
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) sum[j][e] += hh[j][e];
+            }
+        }
+        ss0 += __shfl_xor_sync(0xffffffffu, ss0, 1);
+        ss1 += __shfl_xor_sync(0xffffffffu, ss1, 1);
+        ss0 += __shfl_xor_sync(0xffffffffu, ss0, 2);
+        ss1 += __shfl_xor_sync(0xffffffffu, ss1, 2);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            *reinterpret_cast<float2*>(&psum_[buf][warp][g][8 * j + 2 * q]) = make_float2(sum[j][0] + hl[j][0], sum[j][1] + hl[j][1]);
+            *reinterpret_cast<float2*>(&psum_[buf][warp][g + 8][8 * j + 2 * q]) = make_float2(sum[j][2] + hl[j][2], sum[j][3] + hl[j][3]);
+        }
+        if (q == 0) {
+            sqs_[buf][warp][g] = ss0;
+            sqs_[buf][warp][g + 8] = ss1;
+        }
+        __syncthreads();   // (the buffers alternate: the last readers of this one passed the barrier of the tile between)
+        for (int o = tid; o < RP_TOK * RP_ROWS; o += NW * 32) {
+            const int t = o / RP_ROWS, r = o % RP_ROWS;
+            double sd = 0.0, sq = 0.0;
+            for (int j = 0; j < NW; ++j) {
+                sd += (double) psum_[buf][j][t][r];
+                sq += (double) sqs_[buf][j][t];
+            }
+            float s = (float) sd;
+            if (norm_w) s *= rsqrtf((float) sq / (float) H + eps);
+            if (tile * RP_TOK + t < T && row0 + r <= E) {
+                logits[(size_t) (tile * RP_TOK + t) * (E + 1) + row0 + r] = s;
+                if (!isfinite(s)) atomicOr(err, (unsigned) FNX_ERR_NONFINITE);
+            }
+        }
+        p0 = n0;
+        p1 = n1;
+    }
+}
+
 // the logits of T rows; windows (img may be given) or prompts
 static int router_logits(const float* Wr, const float* x, const float* norm_w, float eps, int T, int E, int H, float* logits, unsigned* err, uint8_t* img, bool early,
                          cudaStream_t st) {
@@ -159,12 +290,9 @@ static int router_logits(const float* Wr, const float* x, const float* norm_w, f
         le = launch_dep(early, H <= 2048 ? k_router_logits<RT_ROWS, 256> : k_router_logits<RT_ROWS, 512>,
                         dim3(img && blocks < T ? T : blocks, (T + FNX_MAX_ROWS - 1) / FNX_MAX_ROWS), dim3(NW * 32), (size_t) 2 * NW * (32 + 32 / RT_ROWS) * sizeof(float), st, Wr,
                         x, norm_w, eps, T, (int) FNX_MAX_ROWS, E, H, logits, err, img);
-    } else {   // about two blocks an SM, at least eight rows each (their weights are 128 KB)
-        const int blocks = (E + RT_PROMPT_ROWS) / RT_PROMPT_ROWS, want = (2 * sm_count() + blocks - 1) / blocks;
-        int per = (T + want - 1) / want;
-        per = per < 8 ? 8 : (per + 1) / 2 * 2;
-        le = launch_dep(early, k_router_logits<RT_PROMPT_ROWS, 256>, dim3(blocks, (T + per - 1) / per), dim3(NW * 32),
-                        (size_t) 2 * NW * (32 + 32 / RT_PROMPT_ROWS) * sizeof(float), st, Wr, x, norm_w, eps, T, per, E, H, logits, err, img);
+    } else {
+        const int blocks = (E + RP_ROWS) / RP_ROWS, tiles = (T + RP_TOK - 1) / RP_TOK, fit = std::max(1, sm_count() / blocks);
+        le = launch_dep(early, k_router_tiles, dim3(blocks, std::min(tiles, fit)), dim3(H / RP_SLICE * 32), 0, st, Wr, x, norm_w, eps, T, E, H, logits, err);
     }
     return le == cudaSuccess ? FNX_OK : fail(FNX_E_CUDA, "k_router_logits: launch failed: %s", cudaGetErrorString(le));
 }
@@ -217,6 +345,7 @@ int router_window(const float* Wr, const float* x, const float* norm_w, float ep
 
 // one warp per row: the top K of its E logits and their renormalised softmax weights
 __global__ void __launch_bounds__(256) k_topk_rows(const float* __restrict__ logits, int T, int E, int K, int* __restrict__ topi, float* __restrict__ topw) {
+    pdl_begin();
     __shared__ __align__(16) unsigned scr_[8][64];
     const int warp = threadIdx.x >> 5, t = blockIdx.x * 8 + warp, lane = threadIdx.x & 31;
     if (t >= T) return;
@@ -442,6 +571,7 @@ extern "C" int fnx_moe_combine_image(const float* part, const int* topi, const f
 // the logits good to a few 1e-5).  The shared expert's gate row is a plain dot.
 __global__ void __launch_bounds__(256) k_router_split_x(const float* __restrict__ x, const float* __restrict__ norm_w, const float* __restrict__ w_gate, int H,
                                                         float eps, __half* __restrict__ xh, __half* __restrict__ xl, float* __restrict__ logits, int ldl, int E) {
+    pdl_begin();
     const int t = blockIdx.x, tid = threadIdx.x;
     const float* xr = x + (size_t) t * H;
     __shared__ float ws[8], s_r;
@@ -493,6 +623,7 @@ __global__ void __launch_bounds__(256) k_router_split_x(const float* __restrict_
 }
 
 __global__ void k_router_split_w(const float* __restrict__ w, size_t n, __half* __restrict__ wh, __half* __restrict__ wl) {
+    pdl_begin();
     const size_t i = (size_t) blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float v = w[i] * 256.0f;
@@ -511,8 +642,10 @@ extern "C" size_t fnx_router_rows_scratch_bytes(int T, int E, int H) {
     return 2 * rr_align((size_t) T * H * sizeof(__half)) + 2 * rr_align((size_t) E * H * sizeof(__half));
 }
 
-extern "C" int fnx_router_rows(const float* Wr, const float* x, const float* norm_w, float eps, int T, int E, int H, int K, float* logits, int* topi,
-                               float* topw, void* scratch, unsigned* err, fnx_stream st) {
+namespace fnxb {
+// early: launch_dep's (the weights are read ahead)
+int router_rows(const float* Wr, const float* x, const float* norm_w, float eps, int T, int E, int H, int K, float* logits, int* topi, float* topw, void* scratch,
+                unsigned* err, bool early, cudaStream_t st) {
     FNX_REQUIRE(Wr && x && logits && topi && topw && err, "fnx_router_rows: null pointer");
     FNX_REQUIRE(T >= 1, "fnx_router_rows: %d rows", T);
     FNX_REQUIRE(E >= K && E <= RT_MAXE && K >= 1 && K <= 32, "fnx_router_rows: %d experts, top %d not supported", E, K);
@@ -524,16 +657,22 @@ extern "C" int fnx_router_rows(const float* Wr, const float* x, const float* nor
         __half* xl = (__half*) b; b += rr_align((size_t) T * H * sizeof(__half));
         __half* wh = (__half*) b; b += rr_align((size_t) E * H * sizeof(__half));
         __half* wl = (__half*) b;
-        k_router_split_x<<<T, 256, 0, as_stream(st)>>>(x, norm_w, Wr + (size_t) E * H, H, eps, xh, xl, logits, E + 1, E);
+        FNX_CUDA_OK(launch_after(k_router_split_x, dim3(T), dim3(256), 0, st, x, norm_w, Wr + (size_t) E * H, H, eps, xh, xl, logits, E + 1, E));
         FNX_LAUNCH_OK("k_router_split_x");
         const size_t n = (size_t) E * H;
-        k_router_split_w<<<(unsigned) ((n + 255) / 256), 256, 0, as_stream(st)>>>(Wr, n, wh, wl);
+        FNX_CUDA_OK(launch_after(k_router_split_w, dim3((unsigned) ((n + 255) / 256)), dim3(256), 0, st, Wr, n, wh, wl));
         FNX_LAUNCH_OK("k_router_split_w");
-        if (int rc = gemm_tma_launch(wh, wl, xh, xl, logits, E + 1, T, E, H, 0, 1.0f / 256.0f, err, as_stream(st))) return rc;
+        if (int rc = gemm_tma_launch(wh, wl, xh, xl, logits, E + 1, T, E, H, 0, 1.0f / 256.0f, err, st)) return rc;
     } else {
-        FNX_TRY(router_logits(Wr, x, norm_w, eps, T, E, H, logits, err, nullptr, false, as_stream(st)));
+        FNX_TRY(router_logits(Wr, x, norm_w, eps, T, E, H, logits, err, nullptr, early, st));
     }
-    k_topk_rows<<<(T + 7) / 8, 256, 0, as_stream(st)>>>(logits, T, E, K, topi, topw);
+    FNX_CUDA_OK(launch_after(k_topk_rows, dim3((T + 7) / 8), dim3(256), 0, st, logits, T, E, K, topi, topw));
     FNX_LAUNCH_OK("k_topk_rows");
     return FNX_OK;
+}
+}  // namespace fnxb
+
+extern "C" int fnx_router_rows(const float* Wr, const float* x, const float* norm_w, float eps, int T, int E, int H, int K, float* logits, int* topi,
+                               float* topw, void* scratch, unsigned* err, fnx_stream st) {
+    return router_rows(Wr, x, norm_w, eps, T, E, H, K, logits, topi, topw, scratch, err, false, as_stream(st));
 }

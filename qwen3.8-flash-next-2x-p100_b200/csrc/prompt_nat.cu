@@ -112,6 +112,7 @@ struct PnItem {
 // MODE 1: gate|up, 0: down, 2: dense (any number of 16-row groups, sums)
 template <int MODE>
 __global__ void __launch_bounds__(PN_THREADS, 1) k_prompt_nat(const PnParams p) {
+    pdl_begin();
     extern __shared__ __align__(1024) uint8_t smem[];
     PnShared& sh = *reinterpret_cast<PnShared*>(smem);
     uint8_t* Bs = smem + PN_HEAD;
@@ -416,6 +417,7 @@ __device__ __forceinline__ void pw_mma(float (&c)[4], uint32_t a0, uint32_t a1, 
 
 template <int MODE, int NG>
 __global__ void __launch_bounds__(PW_THREADS, 1) k_prompt_few(const PnParams p) {
+    pdl_begin();
     extern __shared__ __align__(128) uint8_t smem[];
     constexpr int NT = 8 * NG;   // rows
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
@@ -580,7 +582,7 @@ static int launch_few(int mode, const PnParams& p, int max_jobs, cudaStream_t st
     FNX_TRY(set_smem_limit((const void*) kernel, pw_smem<NG>()));
     const int units = mode == 1 ? p.rows / 16 : p.rows / 32;
     const long long items = (long long) max_jobs * ((units + PW_WARPS - 1) / PW_WARPS);
-    kernel<<<(unsigned) (items < sm_count() ? items : sm_count()), PW_THREADS, pw_smem<NG>(), st>>>(p);
+    FNX_CUDA_OK(launch_after(kernel, dim3((unsigned) (items < sm_count() ? items : sm_count())), dim3(PW_THREADS), pw_smem<NG>(), st, p));
     FNX_LAUNCH_OK("k_prompt_few");
     return FNX_OK;
 }
@@ -590,6 +592,7 @@ int prompt_few(int mode, int groups, const PnParams& p, int max_jobs, cudaStream
 }
 
 __global__ void __launch_bounds__(256) k_prompt_nat_rows(const float* __restrict__ x, const float* __restrict__ norm_w, int H, float eps, __half* __restrict__ xh, int few) {
+    pdl_begin();
     const float* xr = x + (size_t) blockIdx.x * H;
     __shared__ float ws[8];
     constexpr int HOLD = 4;   // the thread's pieces of up to 4,096 columns stay in registers
@@ -632,7 +635,7 @@ __global__ void __launch_bounds__(256) k_prompt_nat_rows(const float* __restrict
 }
 
 int prompt_nat_rows(const float* x, const float* norm_w, int T, int H, float eps, __half* xh, bool few, cudaStream_t st) {
-    k_prompt_nat_rows<<<T, 256, 0, st>>>(x, norm_w, H, eps, xh, few);
+    FNX_CUDA_OK(launch_after(k_prompt_nat_rows, dim3(T), dim3(256), 0, st, x, norm_w, H, eps, xh, few));
     FNX_LAUNCH_OK("k_prompt_nat_rows");
     return FNX_OK;
 }
@@ -642,7 +645,7 @@ int prompt_nat(int mode, const PnParams& p, int max_jobs, cudaStream_t st) {
     auto kernel = mode == 1 ? k_prompt_nat<1> : mode == 0 ? k_prompt_nat<0> : k_prompt_nat<2>;
     FNX_TRY(set_smem_limit((const void*) kernel, PN_SMEM));
     const long long items = (long long) max_jobs * (mode == 1 ? p.rows / 128 : (p.rows + 255) / 256);
-    kernel<<<(unsigned) (items < sm_count() ? items : sm_count()), PN_THREADS, PN_SMEM, st>>>(p);
+    FNX_CUDA_OK(launch_after(kernel, dim3((unsigned) (items < sm_count() ? items : sm_count())), dim3(PN_THREADS), PN_SMEM, st, p));
     FNX_LAUNCH_OK("k_prompt_nat");
     return FNX_OK;
 }

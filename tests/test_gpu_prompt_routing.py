@@ -1,0 +1,40 @@
+"""A prompt's routing at the edges of its kernels: the router's tiles of sixteen rows by sixteen experts, and the job lists either side of
+the number of picks that one block takes."""
+import numpy as np
+import pytest
+
+from test_gpu_ops import _moe_fixture
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+@pytest.mark.parametrize("E,H,T", [(15, 256, 33), (16, 1024, 47), (31, 2048, 48), (32, 512, 49), (512, 2048, 64), (512, 2048, 65)])
+@pytest.mark.parametrize("normed", [False, True])
+def test_router_tiles(F, E, H, T, normed):
+    """Against float64: each product is good to 3 x 2^-22 of itself (two splits, the dropped low x low), the partial sums of sixteen
+    columns and the f32 sums behind them to some 2^-21 of the sum of magnitudes together."""
+    rng = np.random.default_rng(E + T)
+    wr = (0.02 * rng.standard_normal((E + 1, H))).astype(np.float32)
+    x = (3.0 * rng.standard_normal((T, H))).astype(np.float32)
+    nw = (1.0 + 0.05 * rng.standard_normal(H)).astype(np.float32)
+    cuda = lambda a: torch.from_numpy(a).cuda()
+    _, _, lg = F.router_rows(cuda(wr), cuda(x), 4, norm_w=cuda(nw) if normed else None)
+    xn = x.astype(np.float64)
+    if normed:
+        xn = xn / np.sqrt((xn * xn).mean(axis=1, keepdims=True) + 1e-6) * nw
+    bound = (3 * 2.0 ** -22 + 2.0 ** -21) * (np.abs(xn) @ np.abs(wr.astype(np.float64)).T)
+    assert (np.abs(lg.cpu().numpy() - xn @ wr.astype(np.float64).T) < bound).all()
+
+
+@pytest.mark.parametrize("T", [1, 819])   # ten picks a row: 8,190 fill one block's list, 8,200 take the lists of several
+def test_job_lists_do_not_show_in_the_rows(F, T):
+    """A row's experts give the same bits whichever rows it comes with and wherever its entry lies."""
+    E, H, Fn, K = 16, 512, 256, 10
+    fx = _moe_fixture(F, E, H, Fn, seed=29)
+    x = torch.randn((820, H), device="cuda", generator=torch.Generator(device="cuda").manual_seed(8))
+    topi, topw, logits = F.router_rows(fx["wr"], x, K)
+    run = lambda n: F.moe_prefill(fx["gu_t"], fx["dn_t"], fx["sh_gu_t"], fx["sh_dn_t"], topi[:n].contiguous(), topw[:n].contiguous(), logits[:n].contiguous(), x[:n].contiguous(), Fn)
+    (some, err), (every, err2) = run(T), run(820)
+    assert int(err.item()) == 0 and int(err2.item()) == 0
+    assert torch.equal(some, every[:T])
