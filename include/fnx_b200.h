@@ -104,7 +104,7 @@ int fnx_router_route(const float* Wr, const float* x, const float* norm_w, float
  * weights as fnx_router_route computes them, without a job list (fnx_moe_prefill groups the pairs itself).  With scratch
  * (fnx_router_rows_scratch_bytes(T, E, H) bytes) and 1,024 rows or more the logits are a tcgen05.mma product of the rows and the
  * weights split into f16 high and low parts (three products; the tensor core's truncating f32 accumulation leaves the logits
- * good to a few 1e-5, against ~1e-6 for the f32 walk that scratch = null keeps). */
+ * good to a few 1e-5; below that, and with scratch = null, f32 products or tf32 ones of split operands: ~1e-6). */
 size_t fnx_router_rows_scratch_bytes(int T, int E, int H);
 int fnx_router_rows(const float* Wr, const float* x, const float* norm_w, float eps, int T, int E, int H, int K, float* logits,
                     int* topi, float* topw, void* scratch, unsigned* err, fnx_stream st);
@@ -215,8 +215,8 @@ int fnx_gdn_core(const float* qkvz, int ldx, const float* ab, int ldab, float* h
  * lane j is a chain from slot cur[lane_seq[j]] of that sequence's rings at hist_pool + seq * hist_seq_stride floats and
  * S_pool + seq * s_seq_stride floats. */
 /* the same over a prompt's T rows (any T), a chain of which every row is kept (gdn_prompt, engine/src/kernels.cu:2158), in three
- * launches: conv + SiLU, q / k norms and gates of every row at once; the delta rule with the state in registers from the
- * first row to the last; the gated norm of every row at once.  Starts from state slot `cur` (a host value here) and leaves the
+ * launches: conv + SiLU, q / k norms and gates of every row at once; the delta rule eight rows at a time, the state in registers
+ * from the first row to the last; the gated norm of every row at once.  Starts from state slot `cur` (a host value here) and leaves the
  * last row's state and conv history in slot (cur + T) % NS: the caller advances its slot index by T.
  * scratch: fnx_gdn_prompt_scratch_bytes(T, nk, nv, hs) bytes. */
 size_t fnx_gdn_prompt_scratch_bytes(int T, int nk, int nv, int hs);
@@ -314,7 +314,8 @@ void fnx_engine_destroy(fnx_engine* e);
 int fnx_engine_init_synthetic(fnx_engine* e, uint64_t seed, float sigma);
 /* bytes of weights + state this engine holds on its GPU */
 size_t fnx_engine_device_bytes(const fnx_engine* e);
-/* the engine's tensors by name, for tests and loaders: device pointer and byte size (0 if unknown) */
+/* the engine's tensors by name, for tests and loaders: device pointer and byte size (0 if unknown).  Matrices are held in a layout of
+ * the engine's own until they are asked for; one that was is held, and read by later windows and prompts, in the interchange layout */
 void* fnx_engine_tensor(fnx_engine* e, const char* name, size_t* bytes);
 /* resets sequence `seq` to an empty context */
 int fnx_engine_reset(fnx_engine* e, int seq);
