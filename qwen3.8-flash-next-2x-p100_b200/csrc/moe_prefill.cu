@@ -726,8 +726,8 @@ int prompt_moe(const void* Wgu, size_t gu_stride, const void* Wsh_gu, bool gu_na
     __half* xh = (__half*) b; b += pf_align((size_t) T * H * sizeof(__half));
     int* njobs = (int*) b; b += 256;
     const int ne = e_hi - e_lo, n = T * K;
-    const int few = gu_nat && dn_nat ? prompt_few_groups(n, E) : 0;
-    const int per = few ? 8 * few : gu_nat || dn_nat ? PN_N : PF_N, pb = (n + PF_PAIRS - 1) / PF_PAIRS;
+    const bool few = gu_nat && dn_nat && prompt_few_fits(n, E);
+    const int per = few ? PROMPT_FEW_ROWS : gu_nat || dn_nat ? PN_N : PF_N, pb = (n + PF_PAIRS - 1) / PF_PAIRS;
     const bool one = n <= PF_ONE;
     if (one) {
         FNX_CUDA_OK(launch_after(k_pf_route, dim3(1), dim3(PF_MAXE), 0, st, topi, n, ne, e_lo, E, T, add_shared, jobs, njobs, order, per));
@@ -745,7 +745,7 @@ int prompt_moe(const void* Wgu, size_t gu_stride, const void* Wsh_gu, bool gu_na
         FNX_CUDA_OK(launch_after(k_pf_fill, dim3(pb), dim3(512), 0, st, topi, n, e_lo, ne, base, order));
         FNX_LAUNCH_OK("k_pf_fill");
     }
-    if (gu_nat) FNX_TRY(prompt_nat_rows(x, norm_w, T, H, eps, xh, few != 0, st));
+    if (gu_nat) FNX_TRY(prompt_nat_rows(x, norm_w, T, H, eps, xh, few, st));
     else {
         FNX_CUDA_OK(launch_after(k_pf_xnorm, dim3(T), dim3(256), 0, st, x, norm_w, H, eps, xh));
         FNX_LAUNCH_OK("k_pf_xnorm");
@@ -778,7 +778,7 @@ int prompt_moe(const void* Wgu, size_t gu_stride, const void* Wsh_gu, bool gu_na
     p.e_base = e_base; p.E = E; p.jobs = jobs; p.njobs = njobs; p.order = order; p.TKp = n; p.Kp = K; p.err = err;
     if (gu_nat) {
         q.W = (const uint8_t*) Wgu; q.stride = gu_stride; q.Wsh = (const uint8_t*) Wsh_gu; q.x = xh; q.rows = F; q.K = H; q.outh = hbuf;
-        FNX_TRY(few ? prompt_few(1, few, q, nj, st) : prompt_nat(1, q, nj, st));
+        FNX_TRY(few ? prompt_few(1, q, nj, st) : prompt_nat(1, q, nj, st));
     } else {
         FNX_TRY(set_smem_limit((const void*) k_pf_gemm<1>, (int) pf_smem(1)));
         p.W = (const uint8_t*) Wgu; p.expert_stride = gu_stride; p.Wsh = (const uint8_t*) Wsh_gu; p.x = xh; p.rows = F; p.K = H; p.outh = hbuf;
@@ -791,7 +791,7 @@ int prompt_moe(const void* Wgu, size_t gu_stride, const void* Wsh_gu, bool gu_na
     }
     if (dn_nat) {
         q.W = (const uint8_t*) Wdn; q.stride = dn_stride; q.Wsh = (const uint8_t*) Wsh_dn; q.x = hbuf; q.rows = H; q.K = F; q.out = part; q.ldo = H;
-        FNX_TRY(few ? prompt_few(0, few, q, nj, st) : prompt_nat(0, q, nj, st));
+        FNX_TRY(few ? prompt_few(0, q, nj, st) : prompt_nat(0, q, nj, st));
     } else {
         FNX_TRY(set_smem_limit((const void*) k_pf_gemm<0>, (int) pf_smem(0)));
         p.W = (const uint8_t*) Wdn; p.expert_stride = dn_stride; p.Wsh = (const uint8_t*) Wsh_dn; p.x = hbuf; p.rows = H; p.K = F; p.out = part; p.outh = nullptr;
@@ -821,6 +821,17 @@ static int pf_tma_rows() {
     static const int v = []() { const char* e = getenv("FNX_PROMPT_GEMM"); return e && atoi(e) == 0 ? 1 << 30 : 1024; }();
     return v;
 }
+// Which form of the product suits a matrix in the engine's layout: prompt_nat's, which decodes again for every 64 rows (0.8 us a wave of 256
+// features x 64 rows over the SMs and 128 columns), or the matrix to f16 once and gemm_tma's tiles of 256 x 256 (0.55 us a wave and 64
+// columns, the decode 1 us per 2.5 M weights).  12,352 x 2,048: 42 against 46 us at 333 rows, 48 against 46 at 400, 63 against 48 at 600,
+// 90 against 68 at 1,020; 2,048 x 4,096 (8 tiles across only): 55 against 75 us still at 1,020 rows.
+static bool dense_decodes_as_it_goes(int T, int rows, int K) {
+    if (pf_tma_rows() > 1024) return true;
+    const long long sms = sm_count(), slabs = (rows + 255) / 256, nat = slabs * ((T + PN_N - 1) / PN_N), tma = slabs * ((T + PF_N - 1) / PF_N);
+    const double as_it_goes = 0.8 * (K / 128) * (double) ((nat + sms - 1) / sms);
+    const double once = 0.55 * (K / 64) * (double) ((tma + sms - 1) / sms) + (double) rows * K / 2.5e6;
+    return as_it_goes <= once;
+}
 }  // namespace fnxb
 
 extern "C" size_t fnx_dense_prompt_scratch_bytes(int T, int rows, int cols) {
@@ -840,7 +851,7 @@ int prompt_dense(const void* W, bool nat, int rows, int cols, const float* x, in
     int* njobs = (int*) b; b += 256;
     __half* w16 = (__half*) b;
     const int nj = (T + PF_N - 1) / PF_N;
-    if (nat && T < pf_tma_rows()) {
+    if (nat && dense_decodes_as_it_goes(T, rows, cols)) {
         FNX_TRY(prompt_nat_rows(x, norm_w, T, cols, eps, xh, false, st));
         PnParams q{};
         q.W = (const uint8_t*) W; q.T = T; q.x = xh; q.rows = rows; q.K = cols; q.out = y; q.ldo = ldy; q.accumulate = accumulate; q.err = err;
@@ -848,7 +859,7 @@ int prompt_dense(const void* W, bool nat, int rows, int cols, const float* x, in
     }
     FNX_CUDA_OK(launch_after(k_pf_xnorm, dim3(T), dim3(256), 0, st, x, norm_w, cols, eps, xh));
     FNX_LAUNCH_OK("k_pf_xnorm");
-    if (T >= pf_tma_rows()) {   // the matrix to f16 once, then one product with both operands by tensor copies
+    if (nat || T >= pf_tma_rows()) {   // the matrix to f16 once, then one product with both operands by tensor copies
         FNX_TRY(pf_decode_f16_launch(W, nat, rows, cols, w16, st));
         return gemm_tma_launch(w16, nullptr, xh, nullptr, y, ldy, T, rows, cols, accumulate, 1.0f, err, st);
     }

@@ -1,4 +1,4 @@
-// Prompt products x W^T from weights in the engine's own layout (nat_tile.h): the prompt's projections below 1,024 rows and its expert
+// Prompt products x W^T from weights in the engine's own layout (nat_tile.h): the prompt's projections of few rows (a rule in moe_prefill.cu) and its expert
 // products at every length, on tcgen05.mma with the weights as the A operand in tensor memory.
 //
 // Replaces the reference's grouped expert GEMMs for prompts, moe_gate_up_mma / moe_down_mma (engine/src/kernels.hpp:328-330,
@@ -396,18 +396,18 @@ __global__ void __launch_bounds__(PN_THREADS, 1) k_prompt_nat(const PnParams p) 
 }
 
 // ------------------------------------------------------------------------------------------------ jobs of few rows
-// The expert products where an expert has up to some nine rows on average: mma.sync with the decoded fragments in registers as the A
+// The expert products where an expert has up to four rows on average: mma.sync with the decoded fragments in registers as the A
 // operand, so that neither tensor memory nor the waits between its writers and readers are in the way.  Bound by the decode's instructions
-// (integer-logic and half pipes, two cycles each; half of either busy); the products (2 cycles an SM each) would pass it with four row groups.  An item is a job and 16
-// tiles of 32 features (gate|up: 16 gate and the 16 up of the same features), a warp each; the job's rows go through three shared-memory
-// chunks of 256 columns, a warp's tiles through two slots of its own.  513 jobs of 6 rows: 196 + 107 -> 160 + 95 us
-// (gate|up + down).
+// (integer-logic and half pipes, two cycles each; half of either busy).  An item is a job and 16 tiles of 32 features (gate|up: 16 gate
+// and the 16 up of the same features), a warp each; the job's rows go through three shared-memory chunks of 256 columns, a warp's tiles
+// through two slots of its own.  512 experts' matrices, up to eight rows each: 303 us by k_prompt_nat, 255 here (gate|up + down); two groups of
+// eight rows a job won 1% between four and five rows an expert and lost beyond.
 // The rows' columns lie in fours as (0, 2, 1, 3), the order of a decoded word's pairs.
 constexpr int PW_WARPS = 16, PW_THREADS = PW_WARPS * 32, PW_BST = 3;
+constexpr int PW_N = PROMPT_FEW_ROWS;   // rows of a job: the products' N
 constexpr int PW_ROW = 512 + 64;   // bytes of a row's chunk (neighbouring rows in different halves of the banks)
 constexpr int PW_RING = PW_WARPS * 2 * NAT_TILE_BYTES;
-template <int NG>
-constexpr int pw_smem() { return PW_RING + PW_BST * 8 * NG * PW_ROW; }
+constexpr int PW_SMEM = PW_RING + PW_BST * PW_N * PW_ROW;
 
 __device__ __forceinline__ void pw_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -415,11 +415,10 @@ __device__ __forceinline__ void pw_mma(float (&c)[4], uint32_t a0, uint32_t a1, 
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-template <int MODE, int NG>
+template <int MODE>
 __global__ void __launch_bounds__(PW_THREADS, 1) k_prompt_few(const PnParams p) {
     pdl_begin();
     extern __shared__ __align__(128) uint8_t smem[];
-    constexpr int NT = 8 * NG;   // rows
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
     const int KB = p.K / 256, units = MODE == 1 ? p.rows / 16 : p.rows / 32, parts = (units + PW_WARPS - 1) / PW_WARPS, total = *p.njobs * parts;
     if ((int) blockIdx.x >= total) return;
@@ -443,7 +442,7 @@ __global__ void __launch_bounds__(PW_THREADS, 1) k_prompt_few(const PnParams p) 
         const uint8_t* W = nx.w >= p.E ? p.Wsh : p.W + (size_t) (nx.w - p.e_base) * p.stride;
         wsrc = unit < units ? W + (size_t) unit * KB * NAT_TILE_BYTES + lane * 16 : nullptr;
         const int row = MODE == 1 ? (e >= p.TKp ? e - p.TKp : e / p.Kp) : e;
-        xsrc = warp < min(nx.n, NT) ? p.x + (size_t) row * p.K + lane * 8 : nullptr;
+        xsrc = warp < min(nx.n, PW_N) ? p.x + (size_t) row * p.K + lane * 8 : nullptr;
         if (cit + (int) gridDim.x < total) {
             nx = p.jobs[(cit + gridDim.x) / parts];
             need_e = true;
@@ -460,7 +459,7 @@ __global__ void __launch_bounds__(PW_THREADS, 1) k_prompt_few(const PnParams p) 
         }
     };
     auto fetch_rows = [&](int slot) {
-        if (cit < total && xsrc) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(b_s + slot * NT * PW_ROW), "l"(xsrc + ckb * 256) : "memory");
+        if (cit < total && xsrc) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(b_s + slot * PW_N * PW_ROW), "l"(xsrc + ckb * 256) : "memory");
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     auto fetch_tile = [&](int slot) {
@@ -491,15 +490,13 @@ __global__ void __launch_bounds__(PW_THREADS, 1) k_prompt_few(const PnParams p) 
         const PnJob job = p.jobs[it / parts];
         const int unit = it % parts * PW_WARPS + warp;
         int mine = 0;   // lane: output row `lane` of the job
-        float acc[2][NG][4];
-#pragma unroll
-        for (int i = 0; i < 2 * NG * 4; ++i) acc[i / (4 * NG)][(i / 4) % NG][i & 3] = 0.f;
+        float acc[2][4] = {};
         for (int kb = 0; kb < KB; ++kb, ++c) {
             asm volatile("cp.async.wait_group 2;" ::: "memory");
             __syncthreads();   // the chunk's rows are in, and everyone is done with the chunk before: its place is free
             fetch_rows(bslot == 0 ? PW_BST - 1 : bslot - 1);
             const uint8_t* t = ring + (c & 1) * NAT_TILE_BYTES;
-            const uint8_t* b = Bs + (bslot * NT + g) * PW_ROW + q * 16;
+            const uint8_t* b = Bs + (bslot * PW_N + g) * PW_ROW + q * 16;
             if (unit < units) {
                 const uint4 m0 = *reinterpret_cast<const uint4*>(t + NAT_META + g * 16), m1 = *reinterpret_cast<const uint4*>(t + NAT_HALF_BYTES + NAT_META + g * 16);
                 const __half2 dd[2] = {pn_as_h2(m0.z), pn_as_h2(m1.z)};
@@ -520,9 +517,7 @@ __global__ void __launch_bounds__(PW_THREADS, 1) k_prompt_few(const PnParams p) 
                         }
 #pragma unroll
                         for (int e2 = 0; e2 < 2; ++e2) {
-                            uint4 bv[NG];
-#pragma unroll
-                            for (int n = 0; n < NG; ++n) bv[n] = *reinterpret_cast<const uint4*>(b + n * 8 * PW_ROW + (4 * jj + 2 * s2 + e2) * 64);
+                            const uint4 bv = *reinterpret_cast<const uint4*>(b + (4 * jj + 2 * s2 + e2) * 64);
 #pragma unroll
                             for (int hf = 0; hf < 2; ++hf) {
                                 const uint32_t wa = s2 ? (e2 ? w[hf][0].w : w[hf][0].z) : (e2 ? w[hf][0].y : w[hf][0].x);
@@ -530,11 +525,8 @@ __global__ void __launch_bounds__(PW_THREADS, 1) k_prompt_few(const PnParams p) 
                                 uint32_t a[4], d[4];
                                 pn_decode8(C, wa, f[hf][0][e2], a[0], a[1], a[2], a[3]);
                                 pn_decode8(C, wb, f[hf][1][e2], d[0], d[1], d[2], d[3]);
-#pragma unroll
-                                for (int n = 0; n < NG; ++n) {
-                                    pw_mma(acc[hf][n], a[0], d[0], a[1], d[1], bv[n].x, bv[n].y);
-                                    pw_mma(acc[hf][n], a[2], d[2], a[3], d[3], bv[n].z, bv[n].w);
-                                }
+                                pw_mma(acc[hf], a[0], d[0], a[1], d[1], bv.x, bv.y);
+                                pw_mma(acc[hf], a[2], d[2], a[3], d[3], bv.z, bv.w);
                             }
                         }
                     }
@@ -546,49 +538,43 @@ __global__ void __launch_bounds__(PW_THREADS, 1) k_prompt_few(const PnParams p) 
             advance();
             bslot = bslot + 1 == PW_BST ? 0 : bslot + 1;
         }
-        // a lane holds the features g and g + 8 of its unit's two half tiles for the rows 8 n + 2 q, + 1
+        // a lane holds the features g and g + 8 of its unit's two half tiles for the rows 2 q, + 1
 #pragma unroll
-        for (int n = 0; n < NG; ++n)
+        for (int r = 0; r < 2; ++r) {
+            const int row = 2 * q + r;
+            const size_t o = (size_t) __shfl_sync(0xffffffffu, mine, row);
+            if (row < job.n && unit < units) {
+                if (MODE == 1) {
+                    __half* dst = p.outh + o * p.rows + unit * 16;
 #pragma unroll
-            for (int r = 0; r < 2; ++r) {
-                const int row = 8 * n + 2 * q + r;
-                const size_t o = (size_t) __shfl_sync(0xffffffffu, mine, row);
-                if (row < job.n && unit < units) {
-                    if (MODE == 1) {
-                        __half* dst = p.outh + o * p.rows + unit * 16;
+                    for (int i = 0; i < 2; ++i) {
+                        const int f = g + 8 * i;
+                        const float a = acc[0][2 * i + r], b = acc[1][2 * i + r];
+                        dst[(f & ~3) | ((f & 1) << 1) | ((f >> 1) & 1)] = __float2half_rn(__fdividef(a, 1.0f + __expf(-a)) * b);
+                    }
+                } else {
+                    float* dst = p.out + o * p.ldo + unit * 32 + g;
 #pragma unroll
-                        for (int i = 0; i < 2; ++i) {
-                            const int f = g + 8 * i;
-                            const float a = acc[0][n][2 * i + r], b = acc[1][n][2 * i + r];
-                            dst[(f & ~3) | ((f & 1) << 1) | ((f >> 1) & 1)] = __float2half_rn(__fdividef(a, 1.0f + __expf(-a)) * b);
-                        }
-                    } else {
-                        float* dst = p.out + o * p.ldo + unit * 32 + g;
-#pragma unroll
-                        for (int hf = 0; hf < 2; ++hf) {
-                            dst[16 * hf] = acc[hf][n][r];
-                            dst[16 * hf + 8] = acc[hf][n][2 + r];
-                        }
+                    for (int hf = 0; hf < 2; ++hf) {
+                        dst[16 * hf] = acc[hf][r];
+                        dst[16 * hf + 8] = acc[hf][2 + r];
                     }
                 }
             }
+        }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
-template <int NG>
-static int launch_few(int mode, const PnParams& p, int max_jobs, cudaStream_t st) {
-    auto kernel = mode == 1 ? k_prompt_few<1, NG> : k_prompt_few<0, NG>;
-    FNX_TRY(set_smem_limit((const void*) kernel, pw_smem<NG>()));
+int prompt_few(int mode, const PnParams& p, int max_jobs, cudaStream_t st) {
+    FNX_REQUIRE(p.K % 256 == 0 && p.rows % 32 == 0, "prompt product: %d features x %d", p.rows, p.K);
+    auto kernel = mode == 1 ? k_prompt_few<1> : k_prompt_few<0>;
+    FNX_TRY(set_smem_limit((const void*) kernel, PW_SMEM));
     const int units = mode == 1 ? p.rows / 16 : p.rows / 32;
     const long long items = (long long) max_jobs * ((units + PW_WARPS - 1) / PW_WARPS);
-    FNX_CUDA_OK(launch_after(kernel, dim3((unsigned) (items < sm_count() ? items : sm_count())), dim3(PW_THREADS), pw_smem<NG>(), st, p));
+    FNX_CUDA_OK(launch_after(kernel, dim3((unsigned) (items < sm_count() ? items : sm_count())), dim3(PW_THREADS), PW_SMEM, st, p));
     FNX_LAUNCH_OK("k_prompt_few");
     return FNX_OK;
-}
-int prompt_few(int mode, int groups, const PnParams& p, int max_jobs, cudaStream_t st) {
-    FNX_REQUIRE(p.K % 256 == 0 && p.rows % 32 == 0, "prompt product: %d features x %d", p.rows, p.K);
-    return groups == 1 ? launch_few<1>(mode, p, max_jobs, st) : launch_few<2>(mode, p, max_jobs, st);
 }
 
 __global__ void __launch_bounds__(256) k_prompt_nat_rows(const float* __restrict__ x, const float* __restrict__ norm_w, int H, float eps, __half* __restrict__ xh, int few) {

@@ -44,11 +44,11 @@ struct PnParams {
 int prompt_nat(int mode, const PnParams& p, int max_jobs, cudaStream_t st);
 // xh[t] = f16(x[t] norm_w / rms(x[t])) in slot order, or in prompt_few's (norm_w null: f16(x[t]))
 int prompt_nat_rows(const float* x, const float* norm_w, int T, int H, float eps, __half* xh, bool few, cudaStream_t st);
-// modes 1 and 0 for jobs of up to 8 groups rows (groups 1 or 2)
-int prompt_few(int mode, int groups, const PnParams& p, int max_jobs, cudaStream_t st);
-// row groups of eight that suit that many pairs over E experts (0: prompt_nat's jobs).  512 experts' matrices take 255 us in jobs of up to eight
-// rows, 275 us of up to sixteen, 303 us in prompt_nat's of 64 (and 382 us of up to 32 that way, where the products pass the decode): so as long as
-// nearly every expert's rows fit one job
-inline int prompt_few_groups(long long pairs, int E) { return pairs <= 3ll * E ? 1 : pairs <= 9ll * E ? 2 : 0; }
+// modes 1 and 0 for jobs of up to PROMPT_FEW_ROWS rows
+constexpr int PROMPT_FEW_ROWS = 8;
+int prompt_few(int mode, const PnParams& p, int max_jobs, cudaStream_t st);
+// where those win: up to four rows an expert.  A 12-layer prompt of 512 experts, ten a row: 100 rows 4.23 against 4.50 ms in prompt_nat's jobs of 64,
+// 150 rows 4.84 against 4.99, 200 rows 5.42 against 5.43, 333 rows 6.89 against 6.22
+inline bool prompt_few_fits(long long pairs, int E) { return pairs <= 4ll * E; }
 
 }  // namespace fnxb

@@ -95,7 +95,7 @@ def test_prompts_agree_between_the_layouts(n):
         b.close()
 
 
-@pytest.mark.parametrize("E,n", [(32, 1), (32, 8), (32, 9), (32, 48),          # one and two groups of eight rows to a block: 2n <= 3E, 2n <= 9E
+@pytest.mark.parametrize("E,n", [(32, 1), (32, 8), (32, 9), (32, 48),          # jobs of eight rows up to 2n = 4E
                                  (32, 49), (32, 64), (32, 65), (32, 144), (32, 145),
                                  (2, 63), (2, 64), (2, 65), (2, 129)])    # weights through tensor memory: jobs of 64 rows
 def test_prompt_products_at_the_edges_of_their_jobs(E, n):
@@ -112,6 +112,24 @@ def test_prompt_products_at_the_edges_of_their_jobs(E, n):
         for e in (a, b):
             for l in range(2):
                 e.tensor(f"l{l}.router", torch.float32)[:E * cfg.hidden] = 0.0
+            e.prompt(toks)
+            keys.append(e.tensor("l1.k_cache", torch.float16).float().reshape(-1, cfg.n_kv_head * cfg.head_dim)[:n].cpu().numpy())
+        err = np.linalg.norm(keys[0] - keys[1], axis=1) / np.linalg.norm(keys[1], axis=1)
+        assert err.max() < 3 * 2.0 ** -11, (int(err.argmax()), float(err.max()))
+    finally:
+        a.close()
+        b.close()
+
+
+@pytest.mark.parametrize("n", [320, 385, 513, 1100])   # in- and output projection: decoded as they go, or once; tiles of 256 rows full, one over
+def test_prompt_projections_of_both_forms(n):
+    """As above, at the benchmark's widths: the keys are a projection of rows that an output projection and experts left (f16 three times)."""
+    cfg = F.flash_next_config(n_layer=2, attn_every=2, n_expert=2, top_k=2, vocab=2048, max_ctx=1280, max_rows=32, n_seq=1)
+    a, b = pair(cfg)
+    try:
+        toks = np.random.default_rng(7).integers(0, cfg.vocab, size=n + 1).tolist()
+        keys = []
+        for e in (a, b):
             e.prompt(toks)
             keys.append(e.tensor("l1.k_cache", torch.float16).float().reshape(-1, cfg.n_kv_head * cfg.head_dim)[:n].cpu().numpy())
         err = np.linalg.norm(keys[0] - keys[1], axis=1) / np.linalg.norm(keys[1], axis=1)
