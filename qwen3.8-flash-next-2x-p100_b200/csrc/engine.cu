@@ -1493,7 +1493,8 @@ extern "C" int fnx_engine_prompt(fnx_engine* e, int seq, const int* h_tok, int n
         FNX_TRY(fnx_embed_rows(e->embed, e->d_ptok, nt, d.H, e->pR, e->st));
         for (size_t l = 0; l < e->layers.size(); ++l) {
             const LayerW& L = e->layers[l];
-            e->launches += 3 + (L.attn ? 3 : 3) + 3 + 2 + 7;   // this layer's kernels: projections 3 + 3, mixer 3, router 2, experts 7
+            // this layer's kernels, at least: projections 2 + 2, mixer 2 or 3, router 2 or 4, experts 5 or 7
+            e->launches += 4 + (L.attn ? 2 : 3) + (nt >= 1024 ? 4 : 2) + ((long long) nt * d.K > 8192 ? 7 : 5);
             mark(PH_INPROJ, true);
             FNX_TRY(prompt_dense(L.w_in.nat ? L.w_in.nat : L.w_in.tiles, L.w_in.nat != nullptr, L.in_rows, d.H, e->pR, nt, L.norm1, e->c.eps, e->pproj, e->proj_ld, 0, e->p_dense_scratch, e->err, e->st));
             mark(PH_INPROJ, false);
