@@ -124,6 +124,7 @@ struct fnx_engine {
     int *topi = nullptr, *njobs = nullptr, *best_i = nullptr, *result = nullptr, *d_tok = nullptr, *d_parent = nullptr, *d_depth = nullptr;
     int *d_pos = nullptr, *d_cur = nullptr, *d_ctx = nullptr, *d_ctx_n = nullptr, *d_path = nullptr, *d_mtok = nullptr, *d_mpos = nullptr;
     int *cand_i = nullptr, *d_drafts = nullptr, *d_mpos_base = nullptr;
+    bool in_flight = false;     // the last window's results have not been waited for
     int last_seq = -1;          // the sequence whose window the shared window buffers (tokens, result, residual rows) hold
     // batched lanes: device tables of the last lane window (sequence and first row per lane, rows kept per lane), one result
     // row per lane, the draft layer's positions per sequence and its own lane table
@@ -1012,6 +1013,15 @@ static int enqueue_mtp_lanes(fnx_engine* e, int n_lanes, int Tm, int max_rows, c
     return fnx_argmax_mapped(e->logits, n_lanes, e->dvn, e->d_dvocab, best, nullptr, e->err, e->st);
 }
 
+// A commit returns with its window complete: its logits and rows may be read then, on any stream (of a window whose results the caller
+// took, that is so already).
+static int await_window(fnx_engine* e) {
+    if (!e->in_flight) return FNX_OK;
+    FNX_CUDA_OK(cudaStreamSynchronize(e->st));
+    e->in_flight = false;
+    return FNX_OK;
+}
+
 template <typename F>
 static int run_graph(fnx_engine* e, uint64_t key, F&& enqueue) {
     auto it = e->graphs.find(key);
@@ -1334,6 +1344,7 @@ extern "C" int fnx_engine_verify(fnx_engine* e, int seq, const int* h_tok, const
         FNX_CUDA_OK(cudaMemcpyAsync(e->d_step + seq, e->h_step + seq, sizeof(uint32_t), cudaMemcpyHostToDevice, e->st));
     }
     const uint64_t key = ((uint64_t) 1 << 60) | ((uint64_t) seq << 20) | ((uint64_t) T << 1) | (tree ? 1 : 0);
+    e->in_flight = true;
     FNX_TRY(run_graph(e, key, [&]() { return enqueue_verify(e, seq, T, tree); }));
     s.last_T = T;
     e->last_seq = seq;
@@ -1341,6 +1352,7 @@ extern "C" int fnx_engine_verify(fnx_engine* e, int seq, const int* h_tok, const
     if (h_result) {
         FNX_CUDA_OK(cudaMemcpyAsync(hs + IO_ERR, e->io + IO_ERR, sizeof(int) * (IO_RES - IO_ERR + IO_NRES), cudaMemcpyDeviceToHost, e->st));
         FNX_CUDA_OK(cudaStreamSynchronize(e->st));
+        e->in_flight = false;
         FNX_CUDA_OK(cudaEventElapsedTime(&e->last_ms, e->ev0, e->ev1));
         memcpy(h_result, hs + IO_RES, sizeof(int) * IO_NRES);
         const unsigned bits = (unsigned) hs[IO_ERR];
@@ -1588,6 +1600,7 @@ extern "C" int fnx_engine_commit(fnx_engine* e, int seq, const int* h_path, int 
                 e->last_seq);
     FNX_REQUIRE(n >= 1 && n <= s.last_T && h_path[0] == 0, "fnx_engine_commit: %d rows of a window of %d (the first kept row is row 0)", n, s.last_T);
     for (int j = 1; j < n; ++j) FNX_REQUIRE(h_path[j] > h_path[j - 1] && h_path[j] < s.last_T, "fnx_engine_commit: path[%d] = %d is not increasing", j, h_path[j]);
+    FNX_TRY(await_window(e));
     const Dims d = dims(e->c);
     RowList path{};
     memcpy(path.v, h_path, sizeof(int) * n);
@@ -1804,6 +1817,7 @@ extern "C" int fnx_engine_verify_lanes_rows(fnx_engine* e, int n_lanes, const in
     uint64_t hsh = 1469598103934665603ull;
     for (int j = 0; j < n_lanes; ++j) hsh = (hsh ^ (uint64_t) (h_rows[j] + 8 * j)) * 1099511628211ull;
     const uint64_t key = ((uint64_t) 4 << 60) | ((hsh ^ (uint64_t) n_lanes) & 0x0fffffffffffffffull);
+    e->in_flight = true;
     FNX_TRY(run_graph(e, key, [&]() { return enqueue_verify_lanes(e, n_lanes, rows, T); }));
     e->lane_seqs.assign(h_seqs, h_seqs + n_lanes);
     e->lane_rows.assign(h_rows, h_rows + n_lanes);
@@ -1813,6 +1827,7 @@ extern "C" int fnx_engine_verify_lanes_rows(fnx_engine* e, int n_lanes, const in
         const size_t n = (size_t) n_lanes * IO_NRES;
         FNX_CUDA_OK(cudaMemcpyAsync(hs + IO_ERR, e->io + IO_ERR, sizeof(int) * (IO_LRES - IO_ERR + n), cudaMemcpyDeviceToHost, e->st));
         FNX_CUDA_OK(cudaStreamSynchronize(e->st));
+        e->in_flight = false;
         FNX_CUDA_OK(cudaEventElapsedTime(&e->last_ms, e->ev0, e->ev1));
         memcpy(h_results, hs + IO_LRES, sizeof(int) * n);
         if (hs[IO_ERR]) return fail(FNX_E_STATE, "verify_lanes: device error bits 0x%x", (unsigned) hs[IO_ERR]);
@@ -1827,6 +1842,7 @@ extern "C" int fnx_engine_commit_lanes(fnx_engine* e, int n_lanes, const int* h_
         FNX_REQUIRE(h_seqs[j] == e->lane_seqs[j], "fnx_engine_commit_lanes: lane %d is sequence %d in the window, %d here", j, e->lane_seqs[j], h_seqs[j]);
         FNX_REQUIRE(h_keep[j] >= 1 && h_keep[j] <= e->lane_rows[j], "fnx_engine_commit_lanes: lane %d keeps %d of %d rows", j, h_keep[j], e->lane_rows[j]);
     }
+    FNX_TRY(await_window(e));
     RowList keep{};
     memcpy(keep.v, h_keep, sizeof(int) * n_lanes);
     launch_dep(true, k_commit_lanes, dim3(1), dim3(32), 0, e->st, e->d_lane_seq, e->d_lane_row0, keep, e->d_tok, e->d_results, e->d_pos, e->d_cur, e->NS, e->d_ctx,

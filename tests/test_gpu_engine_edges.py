@@ -1,0 +1,47 @@
+"""Calls at the edges of what the engine and its operators take: sizes at which a product's form changes or its shared memory fills,
+routings that cover a part of the experts, non-finite inputs, memory that runs out."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+def _cfg(F, **over):
+    d = dict(n_layer=2, hidden=1024, n_expert=16, top_k=4, ffn=256, n_q_head=8, n_kv_head=1, gdn_k_head=2, gdn_v_head=4, vocab=2048, max_ctx=256, max_rows=32, attn_every=2, n_seq=1)
+    d.update(over)
+    return F.flash_next_config(**d)
+
+
+def _engine(F, **over):
+    cfg = _cfg(F, **over)
+    e = F.Engine(cfg)
+    e.init_synthetic(seed=3, sigma=0.02)
+    return cfg, e
+
+
+def _logits(e, cfg, T):
+    return e.tensor("buf.logits", torch.float32, (cfg.max_rows, cfg.vocab))[:T].clone()
+
+
+def test_a_window_is_complete_when_its_commit_returns(F):
+    """prompt, and windows whose results are not taken: the logits are those of the last window as soon as the commit is back, read on a
+    stream that knows nothing of the engine's."""
+    cfg, e = _engine(F, vocab=65536, n_seq=2, max_ctx=512)
+    try:
+        rng = np.random.default_rng(7)
+        draw = lambda n: rng.integers(0, cfg.vocab, size=n).tolist()
+
+        def lanes():
+            e.verify_lanes([0, 1], [draw(5), draw(5)], want_result=False)
+            e.commit_lanes([0, 1], [5, 5])
+        for warm in range(3):                        # (a window's first run is waited for: it is captured then)
+            for what in (lambda: e.prompt(draw(40)), lambda: e.prefill(draw(32)), lanes):
+                e.reset(0)
+                e.reset(1)
+                what()
+                at_once = _logits(e, cfg, 1)
+                torch.cuda.synchronize()
+                assert torch.equal(at_once, _logits(e, cfg, 1))
+    finally:
+        e.close()
