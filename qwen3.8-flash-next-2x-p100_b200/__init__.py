@@ -300,7 +300,7 @@ def router_route(Wr, x, K: int, norm_w=None, eps: float = 1e-6, e_lo: int = 0, e
     err = tail if err is None else err
     check(lib().fnx_router_route(Wr.data_ptr(), x.data_ptr(), _at(norm_w), eps, T, E, H, K, e_lo, e_hi, 1 if add_shared else 0, logits.data_ptr(), topi.data_ptr(),
                                  topw.data_ptr(), jobs.data_ptr(), njobs.data_ptr(), None, err.data_ptr(), _raw_stream(x)))
-    return dict(logits=logits, topi=topi, topw=topw, jobs=jobs, njobs=njobs, njobs_max=njobs_max, err=err)
+    return dict(logits=logits, topi=topi, topw=topw, jobs=jobs, njobs=njobs, njobs_max=njobs_max, err=err, every=e_lo == 0 and e_hi == E and bool(add_shared))
 
 
 def moe_experts(Wgu, Wdn, Wsh_gu, Wsh_dn, route, x, F: int, K: int, norm_w=None, eps: float = 1e-6, e_base: int = 0, e_lo: int = 0,
@@ -312,7 +312,7 @@ def moe_experts(Wgu, Wdn, Wsh_gu, Wsh_dn, route, x, F: int, K: int, norm_w=None,
     e_hi = E if e_hi is None else e_hi
     P = T * K + T
     gu_stride, dn_stride = iq3s_bytes(2 * F, H), iq3s_bytes(H, F)
-    new = torch.empty if e_lo <= 0 and e_hi >= E and add_shared else torch.zeros   # (rows of experts outside the range stay zero)
+    new = torch.empty if route.get("every") else torch.zeros   # (rows that the job list leaves out stay zero: the combine reads every row of its range)
     h = new((P, F), dtype=torch.float32, device=x.device)
     part = new((P, H), dtype=torch.float32, device=x.device)
     out = torch.empty((T, H), dtype=torch.float32, device=x.device)

@@ -45,3 +45,21 @@ def test_a_window_is_complete_when_its_commit_returns(F):
                 assert torch.equal(at_once, _logits(e, cfg, 1))
     finally:
         e.close()
+
+
+def test_experts_of_a_routing_that_covers_a_part(F):
+    """A routing over half of the experts, or without the shared one, and moe_experts over all of them: the rows of experts that the job
+    list leaves out count as zero, whatever the memory held before."""
+    from test_gpu_ops import _moe_fixture
+    E, H, Fn, K, T = 16, 512, 256, 4, 5
+    fx = _moe_fixture(F, E, H, Fn, seed=31)
+    x = torch.randn((T, H), device="cuda", generator=torch.Generator(device="cuda").manual_seed(9))
+    w = (fx["gu_t"], fx["dn_t"], fx["sh_gu_t"], fx["sh_dn_t"])
+    P = T * K + T
+    for rng, shared in (((0, E // 2), True), ((0, E), False), ((0, 0), True)):
+        route = F.router_route(fx["wr"], x, K, e_lo=rng[0], e_hi=rng[1], add_shared=shared)
+        want, hw, pw = F.moe_experts(*w, route, x, Fn, K, e_lo=rng[0], e_hi=rng[1], add_shared=shared)
+        dirt = [torch.full((P, n), float("nan"), device="cuda") for n in (Fn, H, Fn, H)]
+        del dirt                                     # (the caching allocator hands this memory out again)
+        got, h, part = F.moe_experts(*w, route, x, Fn, K)
+        assert torch.equal(got, want) and torch.equal(h, hw) and torch.equal(part, pw), (rng, shared)
