@@ -43,10 +43,11 @@ int sm_count();
 int set_smem_limit(const void* kernel, int bytes);
 #if defined(__CUDACC__)
 // Programmatic dependent launch: a kernel may start while its predecessor in the stream drains.
-// A kernel of an engine's window, which leaves room for its successor on the SM (registers and shared memory of two blocks fit): it may
-// start while its predecessor drains.  Before pdl_wait() it may read what no kernel since the last but one before it writes (weights,
-// the starting states); an operator of the C ABI, whose caller may have filled any input just before, is launched with early = false
-// unless the kernel reads nothing before pdl_wait().  Every block must reach pdl_wait(): a kernel's end implies its predecessors'.
+// Two rules hold for every kernel launched so.  Every block reaches pdl_wait(): a kernel's end implies its predecessors'.  And
+// pdl_launch_dependents() comes after pdl_wait(): a kernel that has started then knows that everything before its predecessor is
+// complete, so before its own pdl_wait() it may read what older kernels wrote (weights, states, positions, job lists), but nothing of
+// its predecessor's.  An operator of the C ABI, whose caller may have filled any input just before, is launched with early = false unless
+// its kernel reads nothing before pdl_wait().
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_dep(bool early, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
     cudaLaunchConfig_t cfg = {};

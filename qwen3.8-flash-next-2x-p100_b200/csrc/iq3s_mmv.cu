@@ -59,13 +59,13 @@ __global__ void __launch_bounds__(MMV_THREADS, 1) k_iq3s_mmv(const MmvParams p) 
     int nstamp = 0;
     // the codebook is replicated and the barriers are set up while the kernel before drains: five dense launches in a row of 12,352 x 2,048
     // took 18 us each one after another
-    pdl_launch_dependents();
     core_fill_table(table, tid, MMV_THREADS);
     if (lane == 0) {
         for (int i = 0; i < R; ++i) mbar_init(&S.bars[warp * R + i], 1);
         fence_barrier_init();
     }
     pdl_wait();   // from here on: what earlier kernels of the stream wrote (weights, activations, job lists)
+    pdl_launch_dependents();
     MMV_STAMP();
     StageRegs h;
     stage_begin<NG, MODE, MMV_WARPS>(p, h, tid, RowPlain());

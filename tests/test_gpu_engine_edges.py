@@ -63,3 +63,43 @@ def test_experts_of_a_routing_that_covers_a_part(F):
         del dirt                                     # (the caching allocator hands this memory out again)
         got, h, part = F.moe_experts(*w, route, x, Fn, K)
         assert torch.equal(got, want) and torch.equal(h, hw) and torch.equal(part, pw), (rng, shared)
+
+
+ASKED = {"gate|up": ["l0.experts_gu", "l1.experts_gu"], "down": ["l0.experts_dn", "l1.experts_dn"], "projections": ["l0.w_in", "l1.w_out", "mtp.fc_hid"],
+         "heads and one layer": ["head", "l1.w_in", "l1.experts_gu", "l1.experts_dn", "l1.shared_dn"]}
+
+
+@pytest.mark.parametrize("asked", sorted(ASKED))
+def test_engines_with_some_matrices_in_the_interchange_layout(F, asked):
+    """Matrices that were asked for by name among others that were not: windows, drafts and prompts take each from where it is, in one chain of
+    kernels that overlap.  The two layouts part by the order of f32 sums and by rows whose codes move one step (1 / 65,024 of a block's
+    largest value); a prompt's rows are rounded to f16 three times a layer (2^-11 each).  With routers of zeros no near tie parts them."""
+    toks = np.random.default_rng(8).integers(0, 2048, size=400).tolist()
+    got = []
+    for names in ([], ASKED[asked]):
+        cfg, e = _engine(F, max_ctx=512)
+        try:
+            for n in names:
+                e.tensor(n, torch.uint8)
+            for l in ("l0.", "l1.", "mtp."):
+                e.tensor(l + "router", torch.float32)[:cfg.n_expert * cfg.hidden] = 0.0
+            torch.cuda.synchronize()
+            r = []
+            for T in (1, 5, 20):
+                for _ in range(3):                   # (the first run, the captured one, and that again)
+                    e.verify(toks[:T])
+                    r.append(_logits(e, cfg, T))
+            assert torch.equal(r[-1], r[-2])
+            e.commit([0])
+            r.append(torch.tensor(e.draft(3), device="cuda"))
+            for n in (12, 30, 380):
+                e.reset()
+                e.prompt(toks[:n])
+                r.append(_logits(e, cfg, 1))
+            got.append(r)
+            assert e.error_bits() == 0
+        finally:
+            e.close()
+    for i, (a, b) in enumerate(zip(*got)):
+        tol = 3e-4 if i < 9 else 3 * 2.0 ** -11
+        assert torch.equal(a, b) if i == 9 else float((a - b).norm() / b.norm()) < tol, i
