@@ -243,18 +243,37 @@ static void dfree(fnx_engine* e, void* p, size_t bytes) {
             return;
         }
 }
+// A matrix and the one that the same launches read with it move to the interchange layout together or not at all.
 static int to_tiles(fnx_engine* e, Mat& m) {
-    if (!m.nat) return FNX_OK;
-    uint8_t* t = nullptr;
-    FNX_TRY(dalloc(e, &t, m.tile_stride() * m.n));
-    FNX_CUDA_OK(cudaDeviceSynchronize());   // (the zeroing above runs on another stream than the engine's)
-    for (int i = 0; i < m.n; ++i) FNX_TRY(nat_unpack(m.nat + (size_t) i * m.nat_stride(), t + (size_t) i * m.tile_stride(), m.rows, m.cols, m.gate_up, e->st));
-    FNX_CUDA_OK(cudaStreamSynchronize(e->st));
-    dfree(e, m.nat, m.nat_stride() * m.n);
-    m.nat = nullptr;
-    m.tiles = t;
-    return FNX_OK;
+    Mat* pair[2] = {&m, m.with};
+    uint8_t* t[2] = {nullptr, nullptr};
+    auto body = [&]() -> int {
+        for (int k = 0; k < 2; ++k)
+            if (pair[k] && pair[k]->nat) FNX_TRY(dalloc(e, &t[k], pair[k]->tile_stride() * pair[k]->n));
+        FNX_CUDA_OK(cudaDeviceSynchronize());   // (the zeroing above runs on another stream than the engine's)
+        for (int k = 0; k < 2; ++k)
+            for (int i = 0; t[k] && i < pair[k]->n; ++i)
+                FNX_TRY(nat_unpack(pair[k]->nat + (size_t) i * pair[k]->nat_stride(), t[k] + (size_t) i * pair[k]->tile_stride(), pair[k]->rows, pair[k]->cols, pair[k]->gate_up,
+                                   e->st));
+        FNX_CUDA_OK(cudaStreamSynchronize(e->st));
+        return FNX_OK;
+    };
+    const int rc = body();
+    if (rc != FNX_OK) cudaGetLastError();   // (memory that is not to be had: the next launch has nothing to do with it)
+    for (int k = 0; k < 2; ++k) {
+        if (!t[k]) continue;
+        if (rc != FNX_OK) {
+            dfree(e, t[k], pair[k]->tile_stride() * pair[k]->n);
+        } else {
+            dfree(e, pair[k]->nat, pair[k]->nat_stride() * pair[k]->n);
+            pair[k]->nat = nullptr;
+            pair[k]->tiles = t[k];
+        }
+    }
+    return rc;
 }
+// what a launch over a pair rests on
+static int same_layout(const Mat& a, const Mat& b) { return !a.nat == !b.nat ? FNX_OK : fail(FNX_E_STATE, "engine: two matrices of one product are held in different layouts"); }
 
 static int round_up(int v, int m) { return (v + m - 1) / m * m; }
 
@@ -739,6 +758,8 @@ static int enqueue_moe(fnx_engine* e, const LayerW& L, float* R, int T, const Ma
     FNX_TRY(router_window(L.wr, R, L.norm2, e->c.eps, T, d.E, d.H, d.K, e->e_lo, e->e_hi, 1, e->rlogits, e->topi, e->topw, e->jobs, e->njobs, e->d_stats, e->err,
                           L.wgu.nat ? e->img_x : nullptr, true, e->st));
     const int njobs_max = T * d.K + (T + FNX_JOB_TOK - 1) / FNX_JOB_TOK;
+    FNX_TRY(same_layout(L.wgu, L.wsh_gu));
+    FNX_TRY(same_layout(L.wdn, L.wsh_dn));
     if (L.wgu.nat)
         FNX_TRY(nat_gate_up(L.wgu.nat, L.wgu.nat_stride(), e->e_lo, L.wsh_gu.nat, d.E, e->jobs, e->njobs, njobs_max, e->img_x, e->c.eps, d.H, d.F, e->hbuf, e->st));
     else
@@ -855,6 +876,7 @@ static int enqueue_verify(fnx_engine* e, int seq, int T, bool tree) {
 // the draft layer's input rows: Rm = fc_hid(rms(src)) + fc_emb(rms(emb(tok)))   (fnx_mtp_input)
 static int enqueue_mtp_input(fnx_engine* e, int T, const float* src, const int* tok) {
     const Dims d = dims(e->c);
+    FNX_TRY(same_layout(e->mtp_fc_hid, e->mtp_fc_emb));
     if (!e->mtp_fc_hid.nat)
         return fnx_mtp_input(e->mtp_fc_hid.tiles, e->mtp_fc_emb.tiles, e->embed, e->mtp_hnorm, e->mtp_enorm, e->c.eps, src, d.H, tok, T, d.H, e->Emb, e->Rm, e->err,
                              e->st);
@@ -1287,11 +1309,10 @@ extern "C" void* fnx_engine_tensor(fnx_engine* e, const char* name, size_t* byte
     auto mt = e->mats.find(name);
     if (mt != e->mats.end()) {
         Mat& m = *mt->second;
-        if (m.nat) {   // the captured graphs name the layout that goes
-            cudaStreamSynchronize(e->st);
-            for (auto& g : e->graphs) cudaGraphExecDestroy(g.second);
+        if (m.nat) {
+            if (cudaStreamSynchronize(e->st) != cudaSuccess || to_tiles(e, m) != FNX_OK) return nullptr;
+            for (auto& g : e->graphs) cudaGraphExecDestroy(g.second);   // (they name the layout that is gone)
             e->graphs.clear();
-            if (to_tiles(e, m) != FNX_OK || (m.with && to_tiles(e, *m.with) != FNX_OK)) return nullptr;
         }
         if (bytes) *bytes = m.tile_stride() * m.n;
         return m.tiles;
@@ -1539,6 +1560,8 @@ extern "C" int fnx_engine_prompt(fnx_engine* e, int seq, const int* h_tok, int n
             mark(PH_MOE, true);
             {
                 const bool gn = L.wgu.nat != nullptr, dn = L.wdn.nat != nullptr;
+                FNX_TRY(same_layout(L.wgu, L.wsh_gu));
+                FNX_TRY(same_layout(L.wdn, L.wsh_dn));
                 FNX_TRY(prompt_moe(gn ? L.wgu.nat : L.wgu.tiles, gn ? L.wgu.nat_stride() : L.wgu.tile_stride(), gn ? L.wsh_gu.nat : L.wsh_gu.tiles, gn,
                                    dn ? L.wdn.nat : L.wdn.tiles, dn ? L.wdn.nat_stride() : L.wdn.tile_stride(), dn ? L.wsh_dn.nat : L.wsh_dn.tiles, dn, 0, d.E, d.K, 0, d.E, 1,
                                    e->ptopi, e->ptopw, e->plogits, e->pR, L.norm2, e->c.eps, nt, d.H, d.F, e->pR, 1, e->p_moe_scratch, e->err, e->st));

@@ -103,3 +103,36 @@ def test_engines_with_some_matrices_in_the_interchange_layout(F, asked):
     for i, (a, b) in enumerate(zip(*got)):
         tol = 3e-4 if i < 9 else 3 * 2.0 ** -11
         assert torch.equal(a, b) if i == 9 else float((a - b).norm() / b.norm()) < tol, i
+
+
+@pytest.mark.parametrize("name", ["l0.shared_gu", "l0.shared_dn"])
+def test_a_matrix_asked_for_when_its_partner_finds_no_memory(F, name):
+    """The shared expert's matrix moves to the interchange layout together with the stack of routed ones.  Where that finds no room the
+    call fails and nothing has moved: the same window and prompt give the same bits."""
+    cfg, e = _engine(F, n_layer=1, hidden=2048, ffn=512, n_expert=512)
+    try:
+        toks = np.random.default_rng(9).integers(0, cfg.vocab, size=40).tolist()
+
+        def passes():
+            e.reset()
+            e.verify(toks[:5])
+            w = _logits(e, cfg, 5)
+            e.commit([0])
+            e.draft(2)
+            e.reset()
+            e.prompt(toks)
+            return w, _logits(e, cfg, 1)
+        want, held = passes(), e.device_bytes()
+        torch.cuda.empty_cache()
+        room = 64 << 20                              # the shared matrices take 1 MB, the stacks 231 and 461
+        fill = torch.empty(torch.cuda.mem_get_info()[0] - room, dtype=torch.uint8, device="cuda")
+        with pytest.raises(KeyError):
+            e.tensor(name, torch.uint8)
+        del fill
+        torch.cuda.empty_cache()
+        assert e.device_bytes() == held
+        assert all(torch.equal(a, b) for a, b in zip(passes(), want))
+        size = e.tensor(name, torch.uint8).numel()   # with the memory back it is handed out
+        assert size == (F.iq3s_bytes(1024, 2048) if name.endswith("gu") else F.iq3s_bytes(2048, 512))
+    finally:
+        e.close()
