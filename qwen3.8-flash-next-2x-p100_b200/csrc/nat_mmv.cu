@@ -243,6 +243,8 @@ __device__ __forceinline__ float nm_row_factor(uint32_t row_s, int KB, float eps
 // A block's items are the tiles of units [u0, u1) (a unit: one tile row across the columns), dealt to its warps in equal contiguous
 // shares (mmv_core.cuh: units cut by share boundaries leave their pieces in shared memory, and after one barrier the warp with a
 // unit's first piece adds the others in warp order).
+// Dense products sum in f32, so a row's last bits show where its unit is cut, and a row gives the same bits whatever number of rows it comes with:
+// sixteen warps, which small row counts of a large matrix take, share out the eight warps' shares two by two, at the boundary of a unit.
 // C > 1 (dense, long rows): C blocks of a cluster share the units and split the columns, each holding its part of the rows' image;
 // the partial sums are added in block order through distributed shared memory.  A 2048 x 4096 product at five rows would otherwise
 // have every block copy 48 KB of image for one unit.
@@ -294,7 +296,15 @@ __device__ __forceinline__ void nm_body(const NatParams& p, uint8_t* smem) {
         }
         const int ue = min(u1, j1 * upj);
         const unsigned N = ue > uc ? (unsigned) (ue - uc) * nbu : 0u;
-        const int i0 = (int) (N * warp / NW), i1 = (int) (N * (warp + 1) / NW);
+        int i0, i1;
+        if (MODE == MAT_DENSE && NW == 16) {
+            const int a = (int) (N * (warp >> 1) / 8), b = (int) (N * ((warp >> 1) + 1) / 8), m = max(a, min(b, ((a + b) / 2 + nbu / 2) / nbu * nbu));
+            i0 = warp & 1 ? m : a;
+            i1 = warp & 1 ? b : m;
+        } else {
+            i0 = (int) (N * warp / NW);
+            i1 = (int) (N * (warp + 1) / NW);
+        }
         if (MODE == MAT_GATEUP) {   // the jobs' rows
             const int per = KB * (NI_BYTES / 16);
             for (int i = tid; i < nrow * per; i += NT) {

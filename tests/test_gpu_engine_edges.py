@@ -136,3 +136,19 @@ def test_a_matrix_asked_for_when_its_partner_finds_no_memory(F, name):
         assert size == (F.iq3s_bytes(1024, 2048) if name.endswith("gu") else F.iq3s_bytes(2048, 512))
     finally:
         e.close()
+
+
+@pytest.mark.parametrize("hidden,vocab", [(1024, 131072), (2048, 151936)])
+def test_a_row_of_a_large_head_gives_the_same_bits_in_any_window(F, hidden, vocab):
+    """A head of more than 64 MB (1,024 columns: 27 or 28 units a block; 2,048: 32 or 33): a row's logits are the same bits alone, among
+    eight rows, nine, twenty and thirty-two, whatever form of the product those take."""
+    cfg, e = _engine(F, hidden=hidden, vocab=vocab)
+    try:
+        toks = np.random.default_rng(2).integers(0, cfg.vocab, size=32).tolist()
+        e.verify(toks)
+        every = _logits(e, cfg, 32)
+        for T in (1, 4, 8, 9, 12, 16, 20, 24):
+            e.verify(toks[:T])
+            assert torch.equal(_logits(e, cfg, T), every[:T]), T
+    finally:
+        e.close()
