@@ -536,12 +536,17 @@ __global__ void __cluster_dims__(NM_SPLIT, 1, 1) __launch_bounds__(NW * 32, NW >
     nm_body<NG, MAT_DENSE, NW, SLOTS, NM_SPLIT>(p, smem);
 }
 
+constexpr size_t NM_SMEM = 220 * 1024;   // a block's at most
+// the tiles in flight and the cut units' pieces of a form, rows and jobs aside
+template <int NG, int MODE, int NW, int SLOTS>
+constexpr size_t nm_fixed_bytes() {
+    return (size_t) NW * SLOTS * NAT_TILE_BYTES + (size_t) NW * 2 * sizeof(NatPiece<NG, MODE>);
+}
+
 template <int NG, int MODE, int NW, int SLOTS>
 static int launch_nat(NatParams p, cudaStream_t st) {
-    constexpr size_t LIMIT = 220 * 1024;
-    const size_t fixed = (size_t) NW * SLOTS * NAT_TILE_BYTES + (size_t) NW * 2 * sizeof(NatPiece<NG, MODE>);
     const size_t row = ni_row_bytes(p.K / 256);
-    size_t smem = fixed;
+    size_t smem = nm_fixed_bytes<NG, MODE, NW, SLOTS>();
     if (MODE == MAT_DENSE) {
         smem += 4 * NG * row;
     } else {
@@ -552,20 +557,18 @@ static int launch_nat(NatParams p, cudaStream_t st) {
         while (p.rmax > 4 && p.rmax * row > 40 * 1024) --p.rmax;
         smem += p.rmax * row + (size_t) p.njobs_max * sizeof(fnx_job);
     }
-    if (smem > LIMIT) return fail(FNX_E_ARG, "nat_mmv: %d columns, %d rows, %d jobs need %zu bytes of shared memory", p.K, 4 * NG, p.njobs_max, smem);
-    if (int rc = set_smem_limit((const void*) k_nat_mmv<NG, MODE, NW, SLOTS>, (int) LIMIT)) return rc;
+    if (smem > NM_SMEM) return fail(FNX_E_ARG, "nat_mmv: %d columns, %d rows, %d jobs need %zu bytes of shared memory", p.K, 4 * NG, p.njobs_max, smem);
+    if (int rc = set_smem_limit((const void*) k_nat_mmv<NG, MODE, NW, SLOTS>, (int) NM_SMEM)) return rc;
     const cudaError_t le = launch_dep(true, k_nat_mmv<NG, MODE, NW, SLOTS>, dim3(sm_count()), dim3(NW * 32), smem, st, p);
     return le == cudaSuccess ? FNX_OK : fail(FNX_E_CUDA, "nat_mmv: launch failed: %s", cudaGetErrorString(le));
 }
 
 template <int NG, int NW, int SLOTS>
 static int launch_nat_split(NatParams p, cudaStream_t st) {
-    constexpr size_t LIMIT = 220 * 1024;
     const int units = (p.rows + 31) / 32, most = sm_count() / NM_SPLIT, per = (units + most - 1) / most, clusters = (units + per - 1) / per;
-    const size_t smem = (size_t) NW * SLOTS * NAT_TILE_BYTES + (size_t) NW * 2 * sizeof(NatPiece<NG, MAT_DENSE>) + 4 * NG * ni_row_bytes(p.K / 256 / NM_SPLIT) +
-                        (size_t) per * 2 * NG * 64 * sizeof(float);
-    if (smem > LIMIT) return fail(FNX_E_ARG, "nat_mmv: %d columns, %d rows need %zu bytes of shared memory", p.K, 4 * NG, smem);
-    if (int rc = set_smem_limit((const void*) k_nat_mmv_split<NG, NW, SLOTS>, (int) LIMIT)) return rc;
+    const size_t smem = nm_fixed_bytes<NG, MAT_DENSE, NW, SLOTS>() + 4 * NG * ni_row_bytes(p.K / 256 / NM_SPLIT) + (size_t) per * 2 * NG * 64 * sizeof(float);
+    if (smem > NM_SMEM) return fail(FNX_E_ARG, "nat_mmv: %d columns, %d rows need %zu bytes of shared memory", p.K, 4 * NG, smem);
+    if (int rc = set_smem_limit((const void*) k_nat_mmv_split<NG, NW, SLOTS>, (int) NM_SMEM)) return rc;
     const cudaError_t le = launch_dep(true, k_nat_mmv_split<NG, NW, SLOTS>, dim3(clusters * NM_SPLIT), dim3(NW * 32), smem, st, p);
     return le == cudaSuccess ? FNX_OK : fail(FNX_E_CUDA, "nat_mmv: launch failed: %s", cudaGetErrorString(le));
 }
@@ -575,8 +578,10 @@ int nat_dense(const uint8_t* W, int rows, int K, const uint8_t* img, bool normed
     const size_t row = ni_row_bytes(K / 256);
     // columns split over a cluster: long rows that are not normed, and few enough units that their partial sums fit
     const bool split = K >= 4096 && K % (256 * NM_SPLIT) == 0 && !normed && (rows + 31) / 32 <= 8 * (sm_count() / NM_SPLIT);
-    // a matrix that streams for some 10 us (a vocabulary's): sixteen warps, as for many expert jobs below
-    const bool large = !split && nat_bytes(rows, K) > ((size_t) 64 << 20);
+    // a matrix that streams for some 10 us (a vocabulary's): sixteen warps, as for many expert jobs below, where their tiles leave room for the
+    // rows (one group of four always, two up to 3,072 columns; three groups' sums would not leave the registers of sixteen warps).
+    // Either number of warps gives the same bits.
+    const bool large = !split && nat_bytes(rows, K) > ((size_t) 64 << 20), large2 = large && nm_fixed_bytes<2, MAT_DENSE, 16, 2>() + 8 * row <= NM_SMEM;
     // up to five groups of four rows a launch (more would leave no registers), fewer where their image would not fit beside the tiles
     int most = 5;
     while (most > 1 && 4 * most * (split ? ni_row_bytes(K / 256 / NM_SPLIT) : row) > 100 * 1024) --most;
@@ -598,7 +603,7 @@ int nat_dense(const uint8_t* W, int rows, int K, const uint8_t* img, bool normed
         } else {
             switch (ng) {
                 case 1: rc = large ? launch_nat<1, MAT_DENSE, 16, 2>(p, st) : launch_nat<1, MAT_DENSE, 8, 3>(p, st); break;
-                case 2: rc = large ? launch_nat<2, MAT_DENSE, 16, 2>(p, st) : launch_nat<2, MAT_DENSE, 8, 3>(p, st); break;
+                case 2: rc = large2 ? launch_nat<2, MAT_DENSE, 16, 2>(p, st) : launch_nat<2, MAT_DENSE, 8, 3>(p, st); break;
                 case 3: rc = launch_nat<3, MAT_DENSE, 8, 2>(p, st); break;
                 case 4: rc = launch_nat<4, MAT_DENSE, 8, 2>(p, st); break;
                 default: rc = launch_nat<5, MAT_DENSE, 8, 2>(p, st); break;

@@ -152,3 +152,20 @@ def test_a_row_of_a_large_head_gives_the_same_bits_in_any_window(F, hidden, voca
             assert torch.equal(_logits(e, cfg, T), every[:T]), T
     finally:
         e.close()
+
+
+@pytest.mark.parametrize("hidden", [3072, 3584, 4096])
+def test_a_large_head_over_wide_rows(F, hidden):
+    """A vocabulary head of more than 64 MB over rows of up to 4,096 columns, at every number of row groups: the rows' images and the tiles
+    in flight share a block's memory.  A row's logits are the same bits in all of them."""
+    cfg, e = _engine(F, hidden=hidden, vocab=40960, n_expert=4, top_k=2)
+    try:
+        toks = np.random.default_rng(1).integers(0, cfg.vocab, size=32).tolist()
+        e.verify(toks)
+        every = _logits(e, cfg, 32)
+        assert bool(torch.isfinite(every).all())
+        for T in (1, 5, 8, 13, 17, 20):
+            e.verify(toks[:T])
+            assert torch.equal(_logits(e, cfg, T), every[:T]), T
+    finally:
+        e.close()
