@@ -553,9 +553,10 @@ static int launch_nat(NatParams p, cudaStream_t st) {
         // rows of the jobs a block meets in one pass: its units lie in one to three jobs of a row or so each, one of them perhaps the shared
         // expert's four (a second pass drains the copies: four rows instead of eight cost 1.3 us at five rows); with eight a gate|up
         // and a down block fit an SM together
+        smem += (size_t) p.njobs_max * sizeof(fnx_job);
         p.rmax = 8;
-        while (p.rmax > 4 && p.rmax * row > 40 * 1024) --p.rmax;
-        smem += p.rmax * row + (size_t) p.njobs_max * sizeof(fnx_job);
+        while (p.rmax > 4 && (p.rmax * row > 40 * 1024 || smem + p.rmax * row > NM_SMEM)) --p.rmax;
+        smem += p.rmax * row;
     }
     if (smem > NM_SMEM) return fail(FNX_E_ARG, "nat_mmv: %d columns, %d rows, %d jobs need %zu bytes of shared memory", p.K, 4 * NG, p.njobs_max, smem);
     if (int rc = set_smem_limit((const void*) k_nat_mmv<NG, MODE, NW, SLOTS>, (int) NM_SMEM)) return rc;
@@ -617,13 +618,19 @@ int nat_dense(const uint8_t* W, int rows, int K, const uint8_t* img, bool normed
 // From this many jobs on the expert products stream long enough (some 15 us) that sixteen warps, which hide more of an item's latency,
 // are worth more than a second resident block: 205 jobs 50 -> 45 us (gate|up) and 28 -> 24 us (down); 52 jobs are level.
 constexpr int NM_MANY_JOBS = 80;
+// (the job list, 40 bytes a job, has to fit beside sixteen warps' tiles and four rows: 896 jobs at 2,048 columns; the bits are the same either way)
+template <int MODE>
+static int launch_nat_jobs(const NatParams& p, cudaStream_t st) {
+    const size_t least = nm_fixed_bytes<1, MODE, 16, 2>() + 4 * ni_row_bytes(p.K / 256) + (size_t) p.njobs_max * sizeof(fnx_job);
+    return p.njobs_max > NM_MANY_JOBS && least <= NM_SMEM ? launch_nat<1, MODE, 16, 2>(p, st) : launch_nat<1, MODE, 8, 2>(p, st);
+}
 
 int nat_gate_up(const uint8_t* Wgu, size_t stride, int e_base, const uint8_t* Wsh, int E, const fnx_job* jobs, const int* njobs, int njobs_max, const uint8_t* img,
                 float eps, int H, int F, float* h, cudaStream_t st) {
     NatParams p{};
     p.W = Wgu; p.expert_stride = stride; p.e_base = e_base; p.Wsh = Wsh; p.E = E; p.jobs = jobs; p.njobs = njobs; p.njobs_max = njobs_max; p.img = img; p.normed = 1;
     p.eps = eps; p.out = h; p.ldo = F; p.rows = F; p.K = H;
-    return njobs_max > NM_MANY_JOBS ? launch_nat<1, MAT_GATEUP, 16, 2>(p, st) : launch_nat<1, MAT_GATEUP, 8, 2>(p, st);
+    return launch_nat_jobs<MAT_GATEUP>(p, st);
 }
 
 int nat_down(const uint8_t* Wdn, size_t stride, int e_base, const uint8_t* Wsh, int E, const fnx_job* jobs, const int* njobs, int njobs_max, const float* h, int H,
@@ -631,7 +638,7 @@ int nat_down(const uint8_t* Wdn, size_t stride, int e_base, const uint8_t* Wsh, 
     NatParams p{};
     p.W = Wdn; p.expert_stride = stride; p.e_base = e_base; p.Wsh = Wsh; p.E = E; p.jobs = jobs; p.njobs = njobs; p.njobs_max = njobs_max; p.x = h;
     p.out = part; p.ldo = H; p.rows = H; p.K = F;
-    return njobs_max > NM_MANY_JOBS ? launch_nat<1, MAT_DOWN, 16, 2>(p, st) : launch_nat<1, MAT_DOWN, 8, 2>(p, st);
+    return launch_nat_jobs<MAT_DOWN>(p, st);
 }
 
 // ------------------------------------------------------------------------------------------------ images of rows

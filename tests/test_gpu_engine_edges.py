@@ -169,3 +169,20 @@ def test_a_large_head_over_wide_rows(F, hidden):
             assert torch.equal(_logits(e, cfg, T), every[:T]), T
     finally:
         e.close()
+
+
+@pytest.mark.parametrize("top_k,T", [(15, 32), (16, 29), (16, 32), (32, 15), (32, 32)])
+def test_wide_windows_of_many_picks(F, top_k, T):
+    """Up to 32 picks for each of 32 rows: the job list (40 bytes a job) shares a block's memory with the tiles in flight.  Against the
+    same rows one at a time: bit for bit."""
+    cfg, e = _engine(F, hidden=2048, n_expert=64, top_k=top_k)
+    try:
+        toks = np.random.default_rng(3).integers(0, cfg.vocab, size=T).tolist()
+        e.verify(toks)
+        every = _logits(e, cfg, T)
+        for t in range(3):
+            e.verify([toks[t]])
+            assert torch.equal(_logits(e, cfg, 1)[0], every[t]), t
+            e.commit([0])
+    finally:
+        e.close()
