@@ -419,20 +419,21 @@ __global__ void k_commit(__half* const* __restrict__ kcs, __half* const* __restr
     commit_body(kcs, vcs, nlayer, row_halves, path, tok, emitted, n, *pos, cur, NS, ctx, ctx_n);
 }
 // an engine's: the path comes with the launch and is left for the draft layer, with the position its rows start at; a prefix of a chain
-// (nlayer = 0) needs one block, which moves the position on as well
+// needs one block of one warp, which moves the position on as well (advance); else the blocks read it and a kernel behind them moves it
 struct RowList {
     int v[FNX_MAX_ROWS];
 };
 __global__ void k_commit_window(__half* const* __restrict__ kcs, __half* const* __restrict__ vcs, int nlayer, int row_halves, const __grid_constant__ RowList path,
                                 const int* __restrict__ tok, const int* __restrict__ emitted, int n, int* __restrict__ pos, int* __restrict__ cur, int NS,
-                                int* __restrict__ ctx, int* __restrict__ ctx_n, int* __restrict__ path_out, int* __restrict__ mpos_base) {
+                                int* __restrict__ ctx, int* __restrict__ ctx_n, int* __restrict__ path_out, int* __restrict__ mpos_base, int advance) {
     pdl_wait();
     const int p0 = *pos;
     if ((int) blockIdx.x == nlayer) {
         if ((int) threadIdx.x < n) path_out[threadIdx.x] = path.v[threadIdx.x];
+        __syncwarp();   // (every lane has read the position)
         if (threadIdx.x == 0) {
             *mpos_base = p0;
-            if (nlayer == 0) *pos = p0 + n;
+            if (advance) *pos = p0 + n;
         }
     }
     commit_body(kcs, vcs, nlayer, row_halves, path.v, tok, emitted, n, p0, cur, NS, ctx, ctx_n);
@@ -1650,7 +1651,7 @@ extern "C" int fnx_engine_commit(fnx_engine* e, int seq, const int* h_path, int 
         for (LayerW& L : e->layers) nattn += L.attn;
     launch_dep(true, k_commit_window, dim3(nattn + 1), dim3(chain ? 32 : 256), 0, e->st, tables[key].first, tables[key].second, nattn, d.kv_rows, path, e->d_tok,
                e->result + 1 + FNX_MAX_ROWS, n, e->d_pos + seq, e->d_cur + seq, e->NS, e->d_ctx + (size_t) seq * e->cache_rows, e->d_ctx_n + seq, e->d_path,
-               e->d_mpos_base);
+               e->d_mpos_base, (int) chain);
     FNX_LAUNCH_OK("commit");
     if (!chain) {
         launch_dep(true, k_advance_pos, 1, 1, 0, e->st, e->d_pos + seq, n);

@@ -186,3 +186,21 @@ def test_wide_windows_of_many_picks(F, top_k, T):
             e.commit([0])
     finally:
         e.close()
+
+
+def test_a_tree_commit_without_attention_layers(F):
+    """Every layer a DeltaNet (attn_every above the layer count): a path that is no prefix moves the device's position on by its rows, once."""
+    cfg, e = _engine(F, attn_every=5)
+    try:
+        pos = lambda: int(e.tensor("seq.pos", torch.int32)[0].item())
+        e.verify([5, 6, 7, 8], [-1, 0, 0, 2])
+        e.commit([0, 2, 3])
+        torch.cuda.synchronize()
+        d = e.draft(2)                               # (waits for the commit)
+        assert e.pos() == 3 and pos() == 3
+        e.verify([9, 10])
+        e.commit([0, 1])
+        e.draft(1)
+        assert e.pos() == 5 and pos() == 5 and len(d) == 2
+    finally:
+        e.close()
