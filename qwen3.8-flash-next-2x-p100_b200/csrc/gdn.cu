@@ -452,9 +452,9 @@ __global__ void __launch_bounds__(GDP_THREADS) k_gdn_pre(const float* __restrict
         if (on) {
             float* dst = coef + ((size_t) blockIdx.x * nv + lv) * GC_FLOATS;
             if (el < 64) {
-                float m = 0.f;
+                float m = 0.f;   // (rows after ti have no part in it: what is not finite in them stays there)
 #pragma unroll
-                for (int j = 0; j < R; ++j) m = fmaf(Qm[hf][ti][j], Ti[hf][j][tj], m);
+                for (int j = 0; j < R; ++j) m = fmaf(Qm[hf][ti][j], j <= ti ? Ti[hf][j][tj] : 0.f, m);
                 dst[GC_M + el] = m;
             } else if (el < 64 + GC_M) {
                 const int u = el - 64, i = u & 7;
@@ -591,7 +591,8 @@ __global__ void __launch_bounds__(GDS_THREADS, 2) k_gdn_scan(const float* __rest
             const float m[R] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
             float a = cf[GC_BQ + row] * qsw;
 #pragma unroll
-            for (int j = 0; j < R; ++j) a = fmaf(m[j], ws[j * C + col], a);
+            for (int j = 0; j < R; ++j)
+                if (j <= row) a = fmaf(m[j], ws[j * C + col], a);   // (m is 0 beyond, w need not be finite there)
             if (g * R + row < T) *od = a;
         }
     }

@@ -204,3 +204,25 @@ def test_a_tree_commit_without_attention_layers(F):
         assert e.pos() == 5 and pos() == 5 and len(d) == 2
     finally:
         e.close()
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("row", [5, 8, 15, 17])
+def test_a_prompts_rows_before_a_non_finite_one(F, bad, row):
+    """DeltaNet over a prompt, one value of row `row` not finite: the rows before it, of its own group of eight too, keep their bits."""
+    nk, nv, hs, NS, T = 2, 4, 128, 4, 21
+    g = torch.Generator(device="cuda").manual_seed(4)
+    rnd = lambda *s: torch.randn(s, device="cuda", generator=g)
+    ch = (2 * nk + nv) * hs
+    x, ab, hist, S = rnd(T, ch + nv * hs), rnd(T, 2 * nv), rnd(NS, 3, ch), 0.1 * rnd(NS, nv, hs, hs)
+    convw, dt, a, nw = rnd(ch, 4), rnd(nv), -rnd(nv).abs(), rnd(hs)
+    run = lambda x, ab: F.gdn_prompt(x, ab, hist.clone(), convw, dt, a, nw, S.clone(), 1, nk, nv)
+    clean = run(x, ab)
+    for what in ("q", "k", "v", "gate"):
+        y, b = x.clone(), ab.clone()
+        if what == "gate":
+            b[row, 0] = bad
+        else:
+            y[row, {"q": 0, "k": nk * hs, "v": 2 * nk * hs}[what]] = bad
+        got = run(y, b)
+        assert torch.equal(got[:row], clean[:row]), what
