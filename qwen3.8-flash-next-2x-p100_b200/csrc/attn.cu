@@ -123,13 +123,23 @@ int attn_prep(const AttnPrep& a, int rows, int n_lanes, bool early, cudaStream_t
     return le == cudaSuccess ? FNX_OK : fail(FNX_E_CUDA, "k_attn_prep_append: launch failed: %s", cudaGetErrorString(le));
 }
 
-// grid (KV heads, groups of ATT_ROWS rows); a block runs over all the positions its rows see, so there is one partial per (row, head) and
-// the merge only normalises and gates it
+// grid (KV heads, groups of ATT_ROWS rows); a block runs over all the positions its rows see, so there is one partial per (row, head), which
+// k_attn_gate normalises and gates
 __global__ void __launch_bounds__(ATT_THREADS) k_attn_part_prompt(const float* __restrict__ qg, int ldq, const __half* __restrict__ kc,
                                                                   const __half* __restrict__ vc, float* __restrict__ acc_out,
                                                                   AttPartial* __restrict__ mz_out, int T, int nq, int nkv, const int* __restrict__ pos0p) {
     extern __shared__ __align__(16) uint8_t smem[];
     attn_prompt_body(qg, ldq, kc, vc, acc_out, mz_out, T, nq, nkv, *pos0p, (int) blockIdx.x, (int) blockIdx.y * ATT_ROWS, (int) threadIdx.x, smem);
+}
+
+// grid (heads, rows).  Bound by its bytes.  500 rows of 16 heads, with the kernel before it: 66 us; 172 with the windows' merge of many partials in its
+// place, whose block of 1,024 threads has one to read here.
+__global__ void __launch_bounds__(ATT_HD) k_attn_gate(const float* __restrict__ acc, const AttPartial* __restrict__ mz, const float* __restrict__ qg, int ldq,
+                                                      float* __restrict__ out, int nq) {
+    pdl_begin();
+    const int h = blockIdx.x, t = blockIdx.y, i = threadIdx.x;
+    const size_t slot = (size_t) t * nq + h;
+    out[slot * ATT_HD + i] = acc[slot * ATT_HD + i] / mz[slot].z * sigmoidf_(qg[(size_t) t * ldq + (size_t) h * 2 * ATT_HD + ATT_HD + i]);
 }
 
 }  // namespace fnxb
@@ -186,7 +196,9 @@ extern "C" int fnx_attn_prompt(const float* qg, int ldq, const void* kc, const v
     k_attn_part_prompt<<<dim3(nkv, (T + ATT_ROWS - 1) / ATT_ROWS), ATT_THREADS, attn_prompt_smem(), as_stream(st)>>>(qg, ldq, (const __half*) kc, (const __half*) vc, acc, mz,
                                                                                                                      T, nq, nkv, pos0);
     FNX_LAUNCH_OK("fnx_attn_prompt (partials)");
-    return attn_merge(acc, mz, qg, ldq, out, T, nq, 1, as_stream(st));
+    FNX_CUDA_OK(launch_after(k_attn_gate, dim3(nq, T), dim3(ATT_HD), 0, as_stream(st), acc, mz, qg, ldq, out, nq));
+    FNX_LAUNCH_OK("fnx_attn_prompt (gate)");
+    return FNX_OK;
 }
 
 // ---- allocation-free variant: the split partials live in a file-scope device array -------------------------------------------------

@@ -439,8 +439,12 @@ __global__ void __launch_bounds__(AW_THREADS, 1) k_attn_win(const AttnWin a, flo
 // round of loads (every thread's partial sums, four dims of every sixteenth live split, and their maxima) and one exchange; the
 // one-dim-a-thread form before it took three rounds behind two barriers (7.3 us after five rows over 32,768 positions).  Groups and
 // their order do not depend on how many splits are live: a dead one adds 0.
+// TG of the sixteen groups at a time (their sums, and so the bits, are the same): all of them, or four, in blocks of a quarter the size, where
+// there are more (head, row) pairs than the SMs hold of the large blocks (two each): 64 heads, 32 rows over 3,000 positions, both kernels: 73 us
+// with the large blocks, 53 with these; 16 heads, 32 rows: 37 and 31; 8 heads, 32 rows over 131,000 positions (256 pairs): 76 and 80.
 constexpr int AM_GROUPS = 16, AM_BATCH = 5;
-__global__ void __launch_bounds__(AM_GROUPS * 64) k_attn_merge(const float* __restrict__ acc_in, const AttPartial* __restrict__ mz_in, const float* __restrict__ qg, int ldq,
+template <int TG>
+__global__ void __launch_bounds__(TG * 64) k_attn_merge(const float* __restrict__ acc_in, const AttPartial* __restrict__ mz_in, const float* __restrict__ qg, int ldq,
                                                               float* __restrict__ out, uint8_t* __restrict__ img, int T, int nq, int S, const int* __restrict__ pos,
                                                               const int* __restrict__ lane_seq, const int* __restrict__ lane_row0, int n_lanes) {
     __shared__ __align__(16) float part[AM_GROUPS][AW_HD];
@@ -454,7 +458,7 @@ __global__ void __launch_bounds__(AM_GROUPS * 64) k_attn_merge(const float* __re
         const int seq = lane_seq[j];
         skip = seq < 0;   // another rank's lane
         if (!skip) live = min(S, (pos[seq] + lane_row0[j + 1] - lane_row0[j] + AW_N - 1) / AW_N);
-    } else if (pos) live = min(S, (*pos + T + AW_N - 1) / AW_N);
+    } else live = min(S, (*pos + T + AW_N - 1) / AW_N);
     const float gate = tid < AW_HD && !skip ? qg[(size_t) t * ldq + (size_t) h * 2 * AW_HD + AW_HD + tid] : 0.f;
     pdl_wait();
     pdl_launch_dependents();
@@ -462,10 +466,10 @@ __global__ void __launch_bounds__(AM_GROUPS * 64) k_attn_merge(const float* __re
     const size_t base = ((size_t) t * nq + h) * S;
     float4 v[AM_BATCH];
     float m[AM_BATCH];
-    auto fetch = [&](int s0) {
+    auto fetch = [&](int gg, int s0) {
 #pragma unroll
         for (int i = 0; i < AM_BATCH; ++i) {
-            const int s = s0 + g + i * AM_GROUPS;
+            const int s = s0 + gg + i * AM_GROUPS;
             m[i] = -INFINITY;
             if (s < live) {
                 m[i] = mz_in[base + s].m;
@@ -473,7 +477,7 @@ __global__ void __launch_bounds__(AM_GROUPS * 64) k_attn_merge(const float* __re
             }
         }
     };
-    fetch(0);
+    fetch(g, 0);
     AttPartial p[8];   // (up to 256 splits)
     float mx = -INFINITY, z = 0.f;
 #pragma unroll
@@ -486,20 +490,24 @@ __global__ void __launch_bounds__(AM_GROUPS * 64) k_attn_merge(const float* __re
 #pragma unroll
     for (int i = 0; i < 8; ++i) z += p[i].m == -INFINITY ? 0.f : exp2f(p[i].m - mx) * p[i].z;
     z = warp_sum(z);
-    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int s0 = 0; s0 < live; s0 += AM_BATCH * AM_GROUPS) {
-        if (s0) fetch(s0);
+#pragma unroll 1
+    for (int r = 0; r < AM_GROUPS / TG; ++r) {
+        const int gg = g + r * TG;
+        float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int s0 = 0; s0 < live; s0 += AM_BATCH * AM_GROUPS) {
+            if (s0 || r) fetch(gg, s0);
 #pragma unroll
-        for (int i = 0; i < AM_BATCH; ++i)
-            if (m[i] != -INFINITY) {
-                const float w = exp2f(m[i] - mx);
-                sum.x = fmaf(w, v[i].x, sum.x);
-                sum.y = fmaf(w, v[i].y, sum.y);
-                sum.z = fmaf(w, v[i].z, sum.z);
-                sum.w = fmaf(w, v[i].w, sum.w);
-            }
+            for (int i = 0; i < AM_BATCH; ++i)
+                if (m[i] != -INFINITY) {
+                    const float w = exp2f(m[i] - mx);
+                    sum.x = fmaf(w, v[i].x, sum.x);
+                    sum.y = fmaf(w, v[i].y, sum.y);
+                    sum.z = fmaf(w, v[i].z, sum.z);
+                    sum.w = fmaf(w, v[i].w, sum.w);
+                }
+        }
+        *reinterpret_cast<float4*>(&part[gg][d4 * 4]) = sum;
     }
-    *reinterpret_cast<float4*>(&part[g][d4 * 4]) = sum;
     __syncthreads();
     if (tid >= AW_HD) return;
     float tot = part[0][tid];
@@ -516,12 +524,6 @@ __global__ void __launch_bounds__(AM_GROUPS * 64) k_attn_merge(const float* __re
     const float4 a = *reinterpret_cast<const float4*>(&row[lane * 8]), b = *reinterpret_cast<const float4*>(&row[lane * 8 + 4]);
     const float y8[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
     ni_quant(img, nq, y8, 0.f, t, h, lane);
-}
-
-int attn_merge(const float* acc, const AttPartial* mz, const float* qg, int ldq, float* out, int T, int nq, int S, cudaStream_t st) {
-    const cudaError_t le = launch_dep(false, k_attn_merge, dim3(nq, T), dim3(AM_GROUPS * 64), 0, st, acc, mz, qg, ldq, out, (uint8_t*) nullptr, T, nq, S, (const int*) nullptr,
-                                      (const int*) nullptr, (const int*) nullptr, 0);
-    return le == cudaSuccess ? FNX_OK : fail(FNX_E_CUDA, "k_attn_merge: launch failed: %s", cudaGetErrorString(le));
 }
 
 int attn_window_setup() {
@@ -547,8 +549,9 @@ int attn_window(const AttnWin& a, void* scratch, float* out, uint8_t* img, bool 
     cudaError_t le = launch_dep(early, k_attn_win, dim3(sm_count()), dim3(AW_THREADS), (size_t) AW_SMEM, st, a, acc, mz, S, map_k, map_v);
     if (le != cudaSuccess) return fail(FNX_E_CUDA, "k_attn_win: launch failed: %s", cudaGetErrorString(le));
     // (the merge reads positions, lane tables and gates ahead of its wait: all of them older than the kernel before it)
-    le = launch_dep(true, k_attn_merge, dim3(a.nq, a.T), dim3(AM_GROUPS * 64), 0, st, (const float*) acc, (const AttPartial*) mz, a.qg, a.ldq, out, img, a.T, a.nq, S, a.pos,
-                    a.lane_seq, a.lane_row0, a.n_lanes);
+    const bool many = (long long) a.T * a.nq > 2 * sm_count();
+    le = launch_dep(true, many ? k_attn_merge<4> : k_attn_merge<AM_GROUPS>, dim3(a.nq, a.T), dim3((many ? 4 : AM_GROUPS) * 64), 0, st, (const float*) acc, (const AttPartial*) mz,
+                    a.qg, a.ldq, out, img, a.T, a.nq, S, a.pos, a.lane_seq, a.lane_row0, a.n_lanes);
     return le == cudaSuccess ? FNX_OK : fail(FNX_E_CUDA, "k_attn_merge: launch failed: %s", cudaGetErrorString(le));
 }
 

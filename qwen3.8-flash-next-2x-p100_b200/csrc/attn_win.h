@@ -54,7 +54,5 @@ int attn_prep(const AttnPrep& a, int rows, int n_lanes, bool early, cudaStream_t
 int attn_window(const AttnWin& a, void* scratch, float* out, uint8_t* img, bool early, cudaStream_t st);
 // the kernels' limits and the driver's entry point, resolved outside any capture
 int attn_window_setup();
-// out = the merge of S partials (all live) of (row, head), gated
-int attn_merge(const float* acc, const AttPartial* mz, const float* qg, int ldq, float* out, int T, int nq, int S, cudaStream_t st);
 
 }  // namespace fnxb

@@ -226,3 +226,16 @@ def test_a_prompts_rows_before_a_non_finite_one(F, bad, row):
             y[row, {"q": 0, "k": nk * hs, "v": 2 * nk * hs}[what]] = bad
         got = run(y, b)
         assert torch.equal(got[:row], clean[:row]), what
+
+
+@pytest.mark.parametrize("nq,nkv", [(16, 2), (64, 8)])
+def test_many_rows_merge_to_the_bits_of_a_few(F, nq, nkv):
+    """The merge of the splits in small blocks (many rows and heads) and in large ones (few)."""
+    T, ctx = 32, 3000
+    g = torch.Generator(device="cuda").manual_seed(10)
+    qg = torch.randn((T, nq, 512), device="cuda", generator=g)
+    kc, vc = (torch.randn((ctx + T, nkv, 256), device="cuda", generator=g).half() for _ in range(2))
+    pos = torch.arange(ctx, ctx + T, dtype=torch.int32, device="cuda")
+    every = F.attn(qg, kc, vc, pos[:1])
+    for a in range(0, T, 4):
+        assert torch.equal(F.attn(qg[a:a + 4].contiguous(), kc, vc, pos[a:a + 1]), every[a:a + 4]), a
