@@ -5,11 +5,15 @@
 // top K per row with their renormalised softmax, the job list.  fnx_moe_combine replaces k_combine (engine/src/kernels.cu:412-419).
 #include <algorithm>
 
+#include <cooperative_groups.h>
+
 #include "fnx_common.cuh"
 #include <cstdlib>
 
 #include "moe_route.cuh"
 #include "nat_image.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace fnxb {
 
@@ -28,11 +32,11 @@ constexpr int RT_ROWS = 4;
 
 template <int ROWS, int THREADS>
 __global__ void __launch_bounds__(THREADS, 1) k_router_logits(const float* __restrict__ Wr, const float* __restrict__ x, const float* __restrict__ norm_w, float eps, int T,
-                                                          int per, int E, int H, float* __restrict__ logits, unsigned* __restrict__ err, uint8_t* __restrict__ img) {
+                                                          int E, int H, float* __restrict__ logits, unsigned* __restrict__ err, uint8_t* __restrict__ img) {
     constexpr int TOK = 32 / ROWS;
     extern __shared__ float sm[];                 // two buffers of psum [warps][32], ss [warps][TOK]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, NW = H / 256;
-    const int row0 = blockIdx.x * ROWS, c = warp * 256 + lane * 8, t_lo = blockIdx.y * per, t_hi = min(T, t_lo + per);
+    const int row0 = blockIdx.x * ROWS, c = warp * 256 + lane * 8;
     float w[ROWS][8], nw[8];
 #pragma unroll
     for (int r = 0; r < ROWS; ++r) {
@@ -61,7 +65,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_router_logits(const float* __res
 #pragma unroll
         for (int i = 0; i < LD; ++i) {
             xa[i] = xb[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (t + i < t_hi) {
+            if (t + i < T) {
                 const float4* p = reinterpret_cast<const float4*>(x + (size_t) (t + i) * H + c);
                 xa[i] = p[0];
                 xb[i] = p[1];
@@ -69,9 +73,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_router_logits(const float* __res
         }
     };
     constexpr bool AHEAD = THREADS <= 256;   // the next rows' loads run under the products (where the registers allow)
-    if (AHEAD) fetch(t_lo);
+    if (AHEAD) fetch(0);
     int buf = 0;
-    for (int t0 = t_lo; t0 < t_hi; t0 += TOK, buf ^= 1) {
+    for (int t0 = 0; t0 < T; t0 += TOK, buf ^= 1) {
         float v[32];   // sum t ROWS + r
         float sq[TOK];
 #pragma unroll
@@ -93,7 +97,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_router_logits(const float* __res
                     e[t][i] *= nw[i];
                 }
                 sq[h + t] = ss;
-                if (img && t0 + h + t == (int) blockIdx.x && t0 + h + t < t_hi) ni_quant(img, NW, e[t], norm_w ? ss : 0.f, t0 + h + t, warp, lane);
+                if (img && t0 + h + t == (int) blockIdx.x && t0 + h + t < T) ni_quant(img, NW, e[t], norm_w ? ss : 0.f, t0 + h + t, warp, lane);
 #pragma unroll
                 for (int r = 0; r < ROWS; ++r) {
                     float s = 0.f;
@@ -139,7 +143,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_router_logits(const float* __res
             }
             float s = (float) sd;
             if (norm_w) s *= rsqrtf((float) q / (float) H + eps);
-            if (t0 + t < t_hi && row0 + r <= E) {
+            if (t0 + t < T && row0 + r <= E) {
                 logits[(size_t) (t0 + t) * (E + 1) + row0 + r] = s;
                 if (!isfinite(s)) atomicOr(err, (unsigned) FNX_ERR_NONFINITE);
             }
@@ -155,6 +159,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_router_logits(const float* __res
 // Bound by the rows' way to the blocks (33 blocks read each: 128 KB a tile, two thirds of what an SM gets from L2), close behind by the splits
 // (integer-logic pipe) and the products.  333 rows x 513 x 2,048: 29 us (11 TFLOP/s of f32 products; 13 us at L2's 6.5 TB/s); f32 products with
 // their 31 shuffles per two rows took 53.
+// CL = 2: rows of more than 2,048 columns, each half of them in one block of a pair; each block completes half of the sums, reading
+// the other's slices through distributed shared memory.  (900 rows x 513 x 4,096: 181 us; k_router_logits over blocks of 32 rows 292, a walk of every
+// expert row by blocks of eight rows 225.)
 constexpr int RP_ROWS = 16, RP_TOK = 16, RP_SLICE = 128, RP_IT = RP_SLICE / 16, RP_AHEAD = 2, RP_LD = 20, RP_WARPS = 2048 / RP_SLICE;
 
 __device__ __forceinline__ void rp_split(float v, uint32_t& hi, uint32_t& lo) {
@@ -167,12 +174,13 @@ __device__ __forceinline__ void rp_mma(float (&d)[4], const uint32_t (&a)[4], ui
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-__global__ void __launch_bounds__(RP_WARPS * 32, 1) k_router_tiles(const float* __restrict__ Wr, const float* __restrict__ x, const float* __restrict__ norm_w, float eps, int T, int E,
+template <int CL>
+__global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(RP_WARPS * 32, 1) k_router_tiles(const float* __restrict__ Wr, const float* __restrict__ x, const float* __restrict__ norm_w, float eps, int T, int E,
                                                          int H, float* __restrict__ logits, unsigned* __restrict__ err) {
     __shared__ __align__(16) float psum_[2][RP_WARPS][RP_TOK][RP_LD];
     __shared__ float sqs_[2][RP_WARPS][RP_TOK];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3, NW = H / RP_SLICE, row0 = blockIdx.x * RP_ROWS;
-    const int c = warp * RP_SLICE + q * 4, tiles = (T + RP_TOK - 1) / RP_TOK;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3, NW = H / RP_SLICE / CL;
+    const int half = CL > 1 ? (int) blockIdx.x % CL : 0, row0 = (int) blockIdx.x / CL * RP_ROWS, c = (half * NW + warp) * RP_SLICE + q * 4, tiles = (T + RP_TOK - 1) / RP_TOK;
     float4 w[2][RP_IT];   // times the norm weights
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
@@ -260,13 +268,24 @@ __global__ void __launch_bounds__(RP_WARPS * 32, 1) k_router_tiles(const float* 
             sqs_[buf][warp][g] = ss0;
             sqs_[buf][warp][g + 8] = ss1;
         }
-        __syncthreads();   // (the buffers alternate: the last readers of this one passed the barrier of the tile between)
-        for (int o = tid; o < RP_TOK * RP_ROWS; o += NW * 32) {
+        // (the buffers alternate: the last readers of this one passed the barrier of the tile between)
+        if constexpr (CL > 1) cg::this_cluster().sync();
+        else __syncthreads();
+        for (int o = half * (RP_TOK * RP_ROWS / CL) + tid; o < (half + 1) * (RP_TOK * RP_ROWS / CL); o += NW * 32) {
             const int t = o / RP_ROWS, r = o % RP_ROWS;
             double sd = 0.0, sq = 0.0;
-            for (int j = 0; j < NW; ++j) {
-                sd += (double) psum_[buf][j][t][r];
-                sq += (double) sqs_[buf][j][t];
+#pragma unroll
+            for (int k = 0; k < CL; ++k) {
+                const float* ps = &psum_[buf][0][t][r];
+                const float* qs = &sqs_[buf][0][t];
+                if constexpr (CL > 1) {
+                    ps = cg::this_cluster().map_shared_rank(ps, k);
+                    qs = cg::this_cluster().map_shared_rank(qs, k);
+                }
+                for (int j = 0; j < NW; ++j) {
+                    sd += (double) ps[j * RP_TOK * RP_LD];
+                    sq += (double) qs[j * RP_TOK];
+                }
             }
             float s = (float) sd;
             if (norm_w) s *= rsqrtf((float) sq / (float) H + eps);
@@ -278,6 +297,7 @@ __global__ void __launch_bounds__(RP_WARPS * 32, 1) k_router_tiles(const float* 
         p0 = n0;
         p1 = n1;
     }
+    if constexpr (CL > 1) cg::this_cluster().sync();   // no block may leave while the other still reads its sums
 }
 
 // the logits of T rows; windows (img may be given) or prompts
@@ -285,14 +305,15 @@ static int router_logits(const float* Wr, const float* x, const float* norm_w, f
                          cudaStream_t st) {
     const int NW = H / 256;
     cudaError_t le;
-    if (T <= FNX_MAX_ROWS || H > 2048) {   // (sixteen rows' weights of wider slices do not fit the registers)
+    if (T <= FNX_MAX_ROWS) {
         const int blocks = (E + RT_ROWS) / RT_ROWS;
         le = launch_dep(early, H <= 2048 ? k_router_logits<RT_ROWS, 256> : k_router_logits<RT_ROWS, 512>,
-                        dim3(img && blocks < T ? T : blocks, (T + FNX_MAX_ROWS - 1) / FNX_MAX_ROWS), dim3(NW * 32), (size_t) 2 * NW * (32 + 32 / RT_ROWS) * sizeof(float), st, Wr,
-                        x, norm_w, eps, T, (int) FNX_MAX_ROWS, E, H, logits, err, img);
+                        dim3(img && blocks < T ? T : blocks), dim3(NW * 32), (size_t) 2 * NW * (32 + 32 / RT_ROWS) * sizeof(float), st, Wr,
+                        x, norm_w, eps, T, E, H, logits, err, img);
     } else {
-        const int blocks = (E + RP_ROWS) / RP_ROWS, tiles = (T + RP_TOK - 1) / RP_TOK, fit = std::max(1, sm_count() / blocks);
-        le = launch_dep(early, k_router_tiles, dim3(blocks, std::min(tiles, fit)), dim3(H / RP_SLICE * 32), 0, st, Wr, x, norm_w, eps, T, E, H, logits, err);
+        const int cl = H > RP_WARPS * RP_SLICE ? 2 : 1, blocks = (E + RP_ROWS) / RP_ROWS * cl, tiles = (T + RP_TOK - 1) / RP_TOK, fit = std::max(1, sm_count() / blocks);
+        le = launch_dep(early, cl > 1 ? k_router_tiles<2> : k_router_tiles<1>, dim3(blocks, std::min(tiles, fit)), dim3(H / RP_SLICE / cl * 32), 0, st, Wr, x, norm_w, eps, T, E, H, logits,
+                        err);
     }
     return le == cudaSuccess ? FNX_OK : fail(FNX_E_CUDA, "k_router_logits: launch failed: %s", cudaGetErrorString(le));
 }

@@ -239,3 +239,11 @@ def test_many_rows_merge_to_the_bits_of_a_few(F, nq, nkv):
     every = F.attn(qg, kc, vc, pos[:1])
     for a in range(0, T, 4):
         assert torch.equal(F.attn(qg[a:a + 4].contiguous(), kc, vc, pos[a:a + 1]), every[a:a + 4]), a
+
+
+@pytest.mark.parametrize("E,H,T", [(31, 2304, 33), (16, 3072, 64), (512, 4096, 49)])
+@pytest.mark.parametrize("normed", [False, True])
+def test_router_over_rows_of_more_than_2048_columns(F, E, H, T, normed):
+    """Pairs of blocks, a half of the columns each; the bound is that of one block's columns (the slices are added in double)."""
+    from test_gpu_prompt_routing import test_router_tiles as tiles
+    tiles(F, E, H, T, normed)
