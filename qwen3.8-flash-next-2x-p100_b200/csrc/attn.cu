@@ -11,38 +11,43 @@
 
 namespace fnxb {
 
-// grid (nq + 2 nkv heads, rows, lanes).  Bound by latency (a few hundred KB in all): the rotations, whose frequencies go through a double
-// pow, and the norm weights are ready before the rows are (3.3 us a launch with them behind the wait, in a window).
+// grid (nq + 2 nkv heads, rows, lanes).  Bound by latency (a few hundred KB in all).  EARLY: the rotations, whose frequencies go through a double
+// pow, and the norm weights are ready before the rows are (3.3 us a launch with them behind the wait, in a window).  Otherwise nothing is
+// read ahead, and the rotations come last, behind the row's barriers (before them: 17.3 against 16.2 us for 200 rows of 18 heads, 256 rotary dims).
 // Batched lanes: lane j holds the consecutive rows [lane_row0[j], lane_row0[j + 1]) of sequence lane_seq[j]: a chain that starts at that
 // sequence's position pos[seq] and appends to that sequence's caches (GdnLanes / enqueue_rows, engine/src/kernels.hpp:103-110,
 // engine/src/engine.cu:1936).
+template <bool EARLY>
 __global__ void k_attn_prep_append(const AttnPrep a) {
     extern __shared__ float xrow[];   // hd floats
     __shared__ float red[32];
     const int i = threadIdx.x, h = blockIdx.x, t = blockIdx.y, lane = blockIdx.z;
+    if (!EARLY) pdl_begin();
     const int row0 = a.lane_seq ? a.lane_row0[lane] : 0, seq = a.lane_seq ? a.lane_seq[lane] : 0;
     const bool live = !a.lane_seq || (seq >= 0 && t < a.lane_row0[lane + 1] - row0);   // (a negative sequence: another rank's lane)
-    float2 rot = make_float2(1.f, 0.f);
-    float w = 0.f;
-    int pos0 = 0;
-    if (live) {
-        pos0 = a.pos[seq];
-        if (h < a.nq + a.nkv) {
-            rot = attn_rotation(pos0 + (a.depth ? a.depth[t] : t), a.nrot, a.rope_base, i);
-            w = (h < a.nq ? a.qn : a.kn)[i];
-        }
+    const int pos0 = live ? a.pos[seq] : 0;
+    const bool normed = live && h < a.nq + a.nkv;
+    auto rotation = [&]() { return normed ? attn_rotation(pos0 + (a.depth ? a.depth[t] : t), a.nrot, a.rope_base, i) : make_float2(1.f, 0.f); };
+    auto weight = [&]() { return normed ? (h < a.nq ? a.qn : a.kn)[i] : 0.f; };
+    float2 rot;
+    float w;
+    if (EARLY) {
+        rot = rotation();
+        w = weight();
+        pdl_begin();
     }
-    pdl_wait();
-    pdl_launch_dependents();
     if (!live) return;
     const size_t crow = (a.lane_seq ? (size_t) seq * a.seq_rows : 0) + pos0 + t;
-    attn_prep_body(a.qg, a.ldq, a.k, a.ldk, a.v, a.ldv, w, a.kc, a.vc, a.nq, a.nkv, a.hd, a.nrot, crow, rot, a.eps, row0 + t, h, i, xrow, red);
+    attn_prep_body(a.qg, a.ldq, a.k, a.ldk, a.v, a.ldv, [&]() { return EARLY ? w : weight(); }, a.kc, a.vc, a.nq, a.nkv, a.hd, a.nrot, crow,
+                   [&]() { return EARLY ? rot : rotation(); }, a.eps, row0 + t, h, i, xrow, red);
 }
 
 // The same for a prompt's rows where a head has 256 dims and 64 rotary ones: a warp takes one head of PREP_ROWS rows, lane = dims lane + 32 j, so
 // that a rotated pair lies in one lane, nothing is block-wide and the frequency (a double pow) is worked out once a warp.  Bound by the rows' bytes;
 // a block a row and head, with its pow and barriers, took 2.2 ms for 38,912 rows against 0.24 ms of them.
-constexpr int PREP_ROWS = 8, PREP_WARPS = 8;
+// (Its own chain of eight rows takes 5.2 us however few there are: 20 heads, blocks a row and head against this, 48 rows: 4.2 and 5.6 us, 80 rows: 5.8 and
+// 5.8, 128 rows: 8.2 and 5.8.)
+constexpr int PREP_ROWS = 8, PREP_WARPS = 8, PREP_MANY = 1500;   // from that many (row, head) pairs on
 __global__ void __launch_bounds__(PREP_WARPS * 32) k_attn_prep_rows(const AttnPrep a, int T) {
     pdl_begin();
     constexpr int HD = 256, NROT = 64;
@@ -114,12 +119,12 @@ __global__ void __launch_bounds__(PREP_WARPS * 32) k_attn_prep_rows(const AttnPr
 }
 
 int attn_prep(const AttnPrep& a, int rows, int n_lanes, bool early, cudaStream_t st) {
-    if (rows > FNX_MAX_ROWS && !a.lane_seq && !a.depth && a.hd == 256 && a.nrot == 64) {
+    if ((long long) rows * (a.nq + 2 * a.nkv) > PREP_MANY && rows > FNX_MAX_ROWS && !a.lane_seq && !a.depth && a.hd == 256 && a.nrot == 64) {
         FNX_CUDA_OK(launch_after(k_attn_prep_rows, dim3(a.nq + 2 * a.nkv, (rows + PREP_ROWS * PREP_WARPS - 1) / (PREP_ROWS * PREP_WARPS)), dim3(PREP_WARPS * 32), 0, st, a, rows));
         FNX_LAUNCH_OK("k_attn_prep_rows");
         return FNX_OK;
     }
-    const cudaError_t le = launch_dep(early, k_attn_prep_append, dim3(a.nq + 2 * a.nkv, rows, n_lanes), dim3(a.hd), a.hd * sizeof(float), st, a);
+    const cudaError_t le = launch_dep(true, early ? k_attn_prep_append<true> : k_attn_prep_append<false>, dim3(a.nq + 2 * a.nkv, rows, n_lanes), dim3(a.hd), a.hd * sizeof(float), st, a);
     return le == cudaSuccess ? FNX_OK : fail(FNX_E_CUDA, "k_attn_prep_append: launch failed: %s", cudaGetErrorString(le));
 }
 

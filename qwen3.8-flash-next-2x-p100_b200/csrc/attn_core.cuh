@@ -19,10 +19,11 @@ __device__ __forceinline__ float2 attn_rotation(int pos, int nrot, float rope_ba
     sincosf((float) pos * fe, &sn, &cs);
     return make_float2(cs, sn);
 }
-// One (head h of nq + 2 nkv, row t) item by hd threads (i = the thread's element, rot its rotation, w its norm weight); cache row crow;
-// xrow: hd floats, red: 32 floats of shared memory.
-__device__ __forceinline__ void attn_prep_body(float* qg, int ldq, float* k, int ldk, const float* v, int ldv, float w, __half* kc, __half* vc, int nq, int nkv, int hd,
-                                               int nrot, size_t crow, float2 rot, float eps, int t, int h, int i, float* xrow, float* red) {
+// One (head h of nq + 2 nkv, row t) item by hd threads (i = the thread's element, w() its norm weight, rot() its rotation); cache row
+// crow; xrow: hd floats, red: 32 floats of shared memory.
+template <typename W, typename Rot>
+__device__ __forceinline__ void attn_prep_body(float* qg, int ldq, float* k, int ldk, const float* v, int ldv, W w, __half* kc, __half* vc, int nq, int nkv, int hd,
+                                               int nrot, size_t crow, Rot rot, float eps, int t, int h, int i, float* xrow, float* red) {
     crow *= (size_t) nkv * hd;
     if (h >= nq + nkv) {   // a V head: store only
         const int kvh = h - nq - nkv;
@@ -36,13 +37,14 @@ __device__ __forceinline__ void attn_prep_body(float* qg, int ldq, float* k, int
     __syncthreads();
     ss = 0.f;
     for (int j = 0; j < hd / 32; ++j) ss += red[j];
-    xrow[i] = val * rsqrtf(ss / (float) hd + eps) * w;
+    xrow[i] = val * rsqrtf(ss / (float) hd + eps) * w();
     __syncthreads();
     float y = xrow[i];
     if (i < nrot) {
         const int pr = i < nrot / 2 ? i : i - nrot / 2;
+        const float2 r = rot();
         const float x0 = xrow[pr], x1 = xrow[pr + nrot / 2];
-        y = i < nrot / 2 ? x0 * rot.x - x1 * rot.y : x0 * rot.y + x1 * rot.x;
+        y = i < nrot / 2 ? x0 * r.x - x1 * r.y : x0 * r.y + x1 * r.x;
     }
     x[i] = y;
     if (h >= nq) kc[crow + (size_t) (h - nq) * hd + i] = __float2half_rn(y);

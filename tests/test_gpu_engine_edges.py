@@ -247,3 +247,23 @@ def test_router_over_rows_of_more_than_2048_columns(F, E, H, T, normed):
     """Pairs of blocks, a half of the columns each; the bound is that of one block's columns (the slices are added in double)."""
     from test_gpu_prompt_routing import test_router_tiles as tiles
     tiles(F, E, H, T, normed)
+
+
+@pytest.mark.parametrize("T", [75, 76, 200])   # 20 heads: 1,500 pairs, a block each; more: eight rows a warp
+def test_prep_of_many_rows_in_both_forms(F, T):
+    """Norm, rotation and append of a prompt's rows give the bits of the same rows in windows."""
+    nq, nkv, ctx = 16, 2, 40
+    g = torch.Generator(device="cuda").manual_seed(11)
+    rnd = lambda *s: torch.randn(s, device="cuda", generator=g)
+    qg, k, v, qn, kn = rnd(T, nq, 512), rnd(T, nkv, 256), rnd(T, nkv, 256), rnd(256), rnd(256)
+
+    def run(step):
+        q, kk = qg.clone(), k.clone()
+        kc, vc = (torch.zeros((ctx + T, nkv, 256), dtype=torch.float16, device="cuda") for _ in range(2))
+        for a in range(0, T, step):
+            pos = torch.tensor([ctx + a], dtype=torch.int32, device="cuda")
+            F.attn_prep_append(q[a:a + step], kk[a:a + step], v[a:a + step], qn, kn, kc, vc, pos)
+        torch.cuda.synchronize()
+        return q, kk, kc, vc
+    for x, y in zip(run(T), run(32)):
+        assert torch.equal(x, y)
