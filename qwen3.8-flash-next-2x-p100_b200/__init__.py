@@ -259,7 +259,7 @@ def dense(W, rows: int, cols: int, x, norm_w=None, eps: float = 1e-6, out=None, 
     err = new_err(x.device) if err is None else err
     L = lib()
     per = L.fnx_dense_rows(cols)
-    if T <= per:
+    if 0 < T <= per:
         check(L.fnx_dense(W.data_ptr(), rows, cols, x.data_ptr(), x.stride(0), T, _at(norm_w), eps, out.data_ptr(), out.stride(0), 1 if accumulate else 0,
                           err.data_ptr(), _raw_stream(x)))
         return out, err

@@ -267,3 +267,10 @@ def test_prep_of_many_rows_in_both_forms(F, T):
         return q, kk, kc, vc
     for x, y in zip(run(T), run(32)):
         assert torch.equal(x, y)
+
+
+def test_dense_of_no_rows(F):
+    """No rows in, no rows out (nothing is launched)."""
+    W = F.iq3s_retile(F.iq3s_quantize(torch.zeros(16 * 256, device="cuda")), 16, 256)
+    y, err = F.dense(W, 16, 256, torch.empty((0, 256), device="cuda"))
+    assert y.shape == (0, 16) and int(err.item()) == 0
