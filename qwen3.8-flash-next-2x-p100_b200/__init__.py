@@ -804,7 +804,7 @@ class Engine:
         import mmap
         n = lib().fnx_engine_state_bytes(self._h, seq, 1 if kv else 0)
         # (fresh pages, large where the system gives them: a ctypes array of its own would be cleared first, page by page)
-        m = mmap.mmap(-1, n, flags=mmap.MAP_PRIVATE | mmap.MAP_ANONYMOUS)
+        m = mmap.mmap(-1, max(n, 1), flags=mmap.MAP_PRIVATE | mmap.MAP_ANONYMOUS)
         if hasattr(mmap, "MADV_HUGEPAGE"):
             try:
                 m.madvise(mmap.MADV_HUGEPAGE)

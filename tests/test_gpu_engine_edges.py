@@ -274,3 +274,13 @@ def test_dense_of_no_rows(F):
     W = F.iq3s_retile(F.iq3s_quantize(torch.zeros(16 * 256, device="cuda")), 16, 256)
     y, err = F.dense(W, 16, 256, torch.empty((0, 256), device="cuda"))
     assert y.shape == (0, 16) and int(err.item()) == 0
+
+
+def test_saving_a_sequence_that_is_not_there(F):
+    cfg, e = _engine(F)
+    try:
+        for seq in (-1, cfg.n_seq):
+            with pytest.raises(F.FnxError):
+                e.save_state(seq)
+    finally:
+        e.close()
