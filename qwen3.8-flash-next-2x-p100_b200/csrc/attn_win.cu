@@ -541,10 +541,10 @@ int attn_window(const AttnWin& a, void* scratch, float* out, uint8_t* img, bool 
     if (a.ldq % 4 || ((uintptr_t) a.qg & 15) || ((uintptr_t) a.kc & 15) || ((uintptr_t) a.vc & 15)) return fail(FNX_E_ARG, "attention: rows and caches must be 16-byte aligned");
     float* acc = (float*) scratch;
     AttPartial* mz = (AttPartial*) (acc + (size_t) a.T * a.nq * S * AW_HD);
-    // (nominal extents: the kernel asks only for whole chunks below a context's end)
+    // (nominal extents, as far as a copy's row number reaches: the kernel asks only for whole chunks below a context's end)
     CUtensorMap map_k, map_v;
-    FNX_TRY(attn_kv_map(&map_k, a.kc, a.nkv, 1ll << 26));
-    FNX_TRY(attn_kv_map(&map_v, a.vc, a.nkv, 1ll << 26));
+    FNX_TRY(attn_kv_map(&map_k, a.kc, a.nkv, 1ll << 31));
+    FNX_TRY(attn_kv_map(&map_v, a.vc, a.nkv, 1ll << 31));
     FNX_TRY(set_smem_limit((const void*) k_attn_win, AW_SMEM));
     cudaError_t le = launch_dep(early, k_attn_win, dim3(sm_count()), dim3(AW_THREADS), (size_t) AW_SMEM, st, a, acc, mz, S, map_k, map_v);
     if (le != cudaSuccess) return fail(FNX_E_CUDA, "k_attn_win: launch failed: %s", cudaGetErrorString(le));

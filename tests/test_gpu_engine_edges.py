@@ -284,3 +284,31 @@ def test_saving_a_sequence_that_is_not_there(F):
                 e.save_state(seq)
     finally:
         e.close()
+
+
+def test_lane_attention_far_into_a_cache(F):
+    """Lanes whose sequences start some 2^26 rows into the caches (34 GB of keys): the same bits as at the front."""
+    nq, nkv, stride, T = 8, 1, 1 << 20, 3
+    rows = (64 + 2) * stride
+    if torch.cuda.mem_get_info()[0] < 2.2 * rows * nkv * 512:
+        pytest.skip("needs 70 GB")
+    g = torch.Generator(device="cuda").manual_seed(5)
+    kc, vc = (torch.empty((rows, nkv, 256), dtype=torch.float16, device="cuda") for _ in range(2))
+    ctx = 200
+    for t in (kc, vc):
+        t[:ctx + T].normal_(0.0, 1.0, generator=g)
+        for s in (63, 64, 65):
+            t[s * stride:s * stride + ctx + T] = t[:ctx + T]
+    qg = torch.randn((T, nq, 512), device="cuda", generator=g)
+    L = F.lib()
+    scratch = torch.empty(L.fnx_attn_scratch_bytes(T, nq, 256), dtype=torch.uint8, device="cuda")
+    pos = torch.full((66,), ctx, dtype=torch.int32, device="cuda")
+    row0 = torch.tensor([0, T], dtype=torch.int32, device="cuda")
+    outs = []
+    for s in (0, 63, 64, 65):
+        out = torch.empty((T, nq, 256), device="cuda")
+        lane = torch.tensor([s], dtype=torch.int32, device="cuda")
+        F.check(L.fnx_attn_lanes(F.ptr(qg), nq * 512, F.ptr(kc), F.ptr(vc), stride, F.ptr(out), T, 1, nq, nkv, 256, F.ptr(pos), F.ptr(lane), F.ptr(row0), F.ptr(scratch), None))
+        torch.cuda.synchronize()
+        outs.append(out)
+    assert all(torch.equal(o, outs[0]) for o in outs[1:])
