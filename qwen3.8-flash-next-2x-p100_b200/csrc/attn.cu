@@ -163,7 +163,7 @@ extern "C" int fnx_attn_prep_append(float* qg, int ldq, float* k, int ldk, const
 
 extern "C" size_t fnx_attn_scratch_bytes(int T, int nq, int hd) {
     const size_t S = (size_t) sm_count();   // an upper bound of the splits for any KV-head count
-    return (size_t) T * nq * S * ((size_t) hd * sizeof(float) + sizeof(AttPartial));
+    return (size_t) T * nq * S * ((size_t) hd * sizeof(float) + sizeof(AttPartial)) + 16;   // (room to align)
 }
 
 extern "C" int fnx_attn(const float* qg, int ldq, const void* kc, const void* vc, float* out, int T, int nq, int nkv, int hd, const int* pos0,

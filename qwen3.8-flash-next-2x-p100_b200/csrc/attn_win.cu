@@ -539,7 +539,7 @@ int attn_window(const AttnWin& a, void* scratch, float* out, uint8_t* img, bool 
     const int S = sm_count() / a.nkv < 1 ? 1 : sm_count() / a.nkv;
     if (S > 256) return fail(FNX_E_ARG, "attention: %d splits", S);
     if (a.ldq % 4 || ((uintptr_t) a.qg & 15) || ((uintptr_t) a.kc & 15) || ((uintptr_t) a.vc & 15)) return fail(FNX_E_ARG, "attention: rows and caches must be 16-byte aligned");
-    float* acc = (float*) scratch;
+    float* acc = (float*) (((uintptr_t) scratch + 15) & ~(uintptr_t) 15);   // (16-byte pieces; the scratch may lie on any 8-byte boundary)
     AttPartial* mz = (AttPartial*) (acc + (size_t) a.T * a.nq * S * AW_HD);
     // (nominal extents, as far as a copy's row number reaches: the kernel asks only for whole chunks below a context's end)
     CUtensorMap map_k, map_v;

@@ -1,5 +1,7 @@
 """Calls at the edges of what the engine and its operators take: sizes at which a product's form changes or its shared memory fills,
 routings that cover a part of the experts, non-finite inputs, memory that runs out."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -312,3 +314,45 @@ def test_lane_attention_far_into_a_cache(F):
         torch.cuda.synchronize()
         outs.append(out)
     assert all(torch.equal(o, outs[0]) for o in outs[1:])
+
+
+@pytest.mark.parametrize("what", ["attention", "one KV head"])
+def test_scratch_on_an_eight_byte_boundary(F, what):
+    """Scratch of exactly the size that the library asks for, eight bytes off a 16-byte boundary: the same bits as on one, and nothing written
+    around it."""
+    g = torch.Generator(device="cuda").manual_seed(6)
+    rnd = lambda *s: torch.randn(s, device="cuda", generator=g)
+    L = F.lib()
+    if what == "DeltaNet prompt":
+        nk, nv, hs, NS, T = 2, 4, 128, 4, 20        # (back to the slot it starts from: the history's copy takes the end of the scratch)
+        ch = (2 * nk + nv) * hs
+        x, ab, hist, S = rnd(T, ch + nv * hs), rnd(T, 2 * nv), rnd(NS, 3, ch), 0.1 * rnd(NS, nv, hs, hs)
+        convw, dt, a, nw = rnd(ch, 4), rnd(nv), -rnd(nv).abs(), rnd(hs)
+        need = L.fnx_gdn_prompt_scratch_bytes(T, nk, nv, hs)
+
+        def run(at):
+            y = torch.empty((T, nv * hs), device="cuda")
+            h, s = hist.clone(), S.clone()
+            F.check(L.fnx_gdn_prompt(F.ptr(x), x.stride(0), F.ptr(ab), ab.stride(0), F.ptr(h), F.ptr(convw), F.ptr(dt), F.ptr(a), F.ptr(nw), F.ptr(s), 1, NS, F.ptr(y), nk,
+                                     nv, hs, T, 1e-6, C.c_void_p(at), None))
+            return torch.cat([y.flatten(), h.flatten(), s.flatten()])
+    else:
+        nq, nkv, T, ctx = (16, 2, 5, 700) if what == "attention" else (8, 1, 9, 9600)
+        qg, kc, vc = rnd(T, nq, 512), rnd(ctx + T, nkv, 256).half(), rnd(ctx + T, nkv, 256).half()
+        pos = torch.tensor([ctx], dtype=torch.int32, device="cuda")
+        need = L.fnx_attn_scratch_bytes(T, nq, 256)
+
+        def run(at):
+            out = torch.empty((T, nq, 256), device="cuda")
+            F.check(L.fnx_attn(F.ptr(qg), nq * 512, F.ptr(kc), F.ptr(vc), F.ptr(out), T, nq, nkv, 256, F.ptr(pos), None, C.c_void_p(at), None))
+            return out
+    mem = torch.full((need + 4096,), 0x5A, dtype=torch.uint8, device="cuda")
+    outs = []
+    torch.cuda.synchronize()
+    for off in (1024, 1032):
+        mem.fill_(0x5A)
+        torch.cuda.synchronize()
+        outs.append(run(mem.data_ptr() + off))
+        torch.cuda.synchronize()
+        assert int((mem[:off] != 0x5A).sum()) == 0 and int((mem[off + need:] != 0x5A).sum()) == 0
+    assert torch.equal(outs[0], outs[1])
