@@ -703,7 +703,7 @@ extern "C" int fnx_gdn_prompt(const float* qkvz, int ldx, const float* ab, int l
     const size_t hsz = (size_t) 3 * ch, ssz = (size_t) nv * GDN_HS * GDN_HS;
     const int ng = (T + GDP_ROWS - 1) / GDP_ROWS;
     const size_t Tp = (size_t) ng * GDP_ROWS;
-    float* xq = (float*) scratch;
+    float* xq = (float*) (((uintptr_t) scratch + 15) & ~(uintptr_t) 15);   // (16-byte pieces; the spare bytes of the scratch leave room to align)
     float* xk = xq + Tp * nk * GDN_HS;
     float* xv = xk + Tp * nk * GDN_HS;
     float* xc = xv + Tp * nv * GDN_HS;

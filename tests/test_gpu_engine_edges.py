@@ -316,7 +316,7 @@ def test_lane_attention_far_into_a_cache(F):
     assert all(torch.equal(o, outs[0]) for o in outs[1:])
 
 
-@pytest.mark.parametrize("what", ["attention", "one KV head"])
+@pytest.mark.parametrize("what", ["attention", "one KV head", "DeltaNet prompt"])
 def test_scratch_on_an_eight_byte_boundary(F, what):
     """Scratch of exactly the size that the library asks for, eight bytes off a 16-byte boundary: the same bits as on one, and nothing written
     around it."""
