@@ -15,6 +15,7 @@
 #include <cmath>
 #include <map>
 #include <string>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -2052,11 +2053,15 @@ static int copy_pieces(fnx_engine* e, const std::vector<std::pair<char*, size_t>
     std::vector<int> rcs(n, FNX_OK);
     std::vector<std::string> why(n);
     std::vector<std::thread> threads;
-    for (int w = 1; w < n; ++w)
-        threads.emplace_back([&, w]() {
-            rcs[w] = stage_worker(e, w, device, list, next, to_host);
-            if (rcs[w] != FNX_OK) why[w] = error_buf();
-        });
+    threads.reserve(n);
+    try {
+        for (int w = 1; w < n; ++w)
+            threads.emplace_back([&, w]() {
+                rcs[w] = stage_worker(e, w, device, list, next, to_host);
+                if (rcs[w] != FNX_OK) why[w] = error_buf();
+            });
+    } catch (const std::system_error&) {   // no more threads to be had: those that run, this one among them, take the whole list
+    }
     if (n > 0) rcs[0] = stage_worker(e, 0, device, list, next, to_host);
     for (auto& t : threads) t.join();
     for (int w = 0; w < n; ++w)

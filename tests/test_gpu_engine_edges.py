@@ -356,3 +356,47 @@ def test_scratch_on_an_eight_byte_boundary(F, what):
         torch.cuda.synchronize()
         assert int((mem[:off] != 0x5A).sum()) == 0 and int((mem[off + need:] != 0x5A).sum()) == 0
     assert torch.equal(outs[0], outs[1])
+
+
+def test_parking_where_no_thread_can_be_started(F, tmp_path):
+    """pthread_create refused by a shim during save and load: the calling thread moves everything itself."""
+    import os
+    import pathlib
+    import subprocess
+    import sys
+    (tmp_path / "shim.c").write_text("""
+#define _GNU_SOURCE
+#include <dlfcn.h>
+#include <errno.h>
+#include <pthread.h>
+static int refuse, refused;
+void shim_refuse(int on) { refuse = on; }
+int shim_refused(void) { return refused; }
+int pthread_create(pthread_t* t, const pthread_attr_t* a, void* (*f)(void*), void* x) {
+    static int (*real)(pthread_t*, const pthread_attr_t*, void* (*)(void*), void*);
+    if (!real) real = dlsym(RTLD_NEXT, "pthread_create");
+    if (refuse) { ++refused; return EAGAIN; }
+    return real(t, a, f, x);
+}
+""")
+    subprocess.run(["gcc", "-shared", "-fPIC", "-o", str(tmp_path / "shim.so"), str(tmp_path / "shim.c"), "-ldl"], check=True)
+    code = """
+import ctypes, sys
+sys.path[:0] = [%r, %r]
+import torch
+import fnx_b200 as F
+from test_gpu_engine_edges import _engine
+cfg, e = _engine(F, n_seq=2)
+e.prompt(list(range(150)))
+want = bytes(e.save_state(0))
+shim = ctypes.CDLL(None)
+shim.shim_refuse(1)
+image = e.save_state(0)
+e.load_state(image, 1)
+shim.shim_refuse(0)
+assert bytes(image) == want and bytes(e.save_state(1)) == want and shim.shim_refused() > 0
+e.close()
+print("same", shim.shim_refused())
+""" % (str(pathlib.Path(F.PACKAGE_DIR).parent), str(pathlib.Path(__file__).parent))
+    r = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, LD_PRELOAD=str(tmp_path / "shim.so")), capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.startswith("same"), r.stderr[-2000:]
