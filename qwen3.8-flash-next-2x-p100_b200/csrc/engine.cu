@@ -911,11 +911,12 @@ static int enqueue_mtp(fnx_engine* e, int seq, int T, const float* src, const in
 // state slots advance
 __global__ void k_commit_lanes(const int* __restrict__ lane_seq, const int* __restrict__ lane_row0, const __grid_constant__ RowList keep,
                                const int* __restrict__ tok, const int* __restrict__ results, int* __restrict__ pos, int* __restrict__ cur, int NS,
-                               int* __restrict__ ctx, size_t ctx_stride, int* __restrict__ ctx_n, int L, int* __restrict__ mrow0, int* __restrict__ mpos_base) {
+                               int* __restrict__ ctx, size_t ctx_stride, int* __restrict__ ctx_n, int L, int* __restrict__ mrow0, int* __restrict__ mpos_base, int* __restrict__ keep_out) {
     pdl_wait();
     const int lane = threadIdx.x;
     if (lane >= L) return;
     const int seq = lane_seq[lane], row0 = lane_row0[lane], n = keep.v[lane];
+    keep_out[lane] = n;
     const int* res = results + (size_t) lane * (1 + 2 * FNX_MAX_ROWS);
     int* c = ctx + (size_t) seq * ctx_stride;
     const int cn = ctx_n[seq];
@@ -1871,7 +1872,7 @@ extern "C" int fnx_engine_commit_lanes(fnx_engine* e, int n_lanes, const int* h_
     RowList keep{};
     memcpy(keep.v, h_keep, sizeof(int) * n_lanes);
     launch_dep(true, k_commit_lanes, dim3(1), dim3(32), 0, e->st, e->d_lane_seq, e->d_lane_row0, keep, e->d_tok, e->d_results, e->d_pos, e->d_cur, e->NS, e->d_ctx,
-               (size_t) e->cache_rows, e->d_ctx_n, n_lanes, e->d_mlane_row0, e->d_mpos_base);
+               (size_t) e->cache_rows, e->d_ctx_n, n_lanes, e->d_mlane_row0, e->d_mpos_base, e->d_keep);
     FNX_LAUNCH_OK("commit lanes");
     for (int j = 0; j < n_lanes; ++j) {
         SeqState& s = e->seqs[h_seqs[j]];

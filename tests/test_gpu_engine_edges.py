@@ -400,3 +400,14 @@ print("same", shim.shim_refused())
 """ % (str(pathlib.Path(F.PACKAGE_DIR).parent), str(pathlib.Path(__file__).parent))
     r = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, LD_PRELOAD=str(tmp_path / "shim.so")), capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and r.stdout.startswith("same"), r.stderr[-2000:]
+
+
+def test_the_kept_counts_of_a_lanes_commit_can_be_read(F):
+    cfg, e = _engine(F, n_seq=3)
+    try:
+        e.verify_lanes_rows([2, 0, 1], [[1, 2, 3], [4], [5, 6]])
+        e.commit_lanes([2, 0, 1], [2, 1, 2])
+        e.error_bits()                               # (waits for the commit)
+        assert e.tensor("buf.lane_keep", torch.int32)[:3].tolist() == [2, 1, 2]
+    finally:
+        e.close()
