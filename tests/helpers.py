@@ -20,6 +20,17 @@ def rel_err(a, b):
     return float(np.abs(a - b).max() / max(np.abs(b).max(), 1e-30))
 
 
+def oracle_twin(F, O, cfg, seed, sigma=0.02, **kw):
+    """The oracle on the weights of another engine of the same configuration and seed: asking the engine under test for its matrices would
+    move them to the interchange layout, and its windows and prompts to the kernels that read that."""
+    twin = F.Engine(cfg)
+    try:
+        twin.init_synthetic(seed=seed, sigma=sigma)
+        return OracleModel(F, O, twin, cfg, **kw)
+    finally:
+        twin.close()
+
+
 class OracleModel:
     """The synthetic model run through the CPU oracle, on the weights the engine holds.
 

@@ -4,7 +4,7 @@ speculative output equals plain greedy output, and a cut-back window leaves the 
 import numpy as np
 import pytest
 
-from helpers import OracleModel, rel_err
+from helpers import oracle_twin, rel_err
 
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
@@ -23,7 +23,7 @@ def model(F, O):
     cfg = small_cfg(F)
     eng = F.Engine(cfg)
     eng.init_synthetic(seed=0, sigma=0.02)
-    om = OracleModel(F, O, eng, cfg)
+    om = oracle_twin(F, O, cfg, seed=0)
     yield cfg, eng, om
     eng.close()
 
@@ -96,7 +96,7 @@ def test_drafts_over_a_draft_vocabulary_match_oracle(F, O):
     eng = F.Engine(cfg)
     try:
         eng.init_synthetic(seed=3, sigma=0.02)
-        om = OracleModel(F, O, eng, cfg)
+        om = oracle_twin(F, O, cfg, seed=3)
         assert om.dvocab.shape == (512,) and np.all(np.diff(om.dvocab) > 0) and om.dvocab[-1] < cfg.vocab
         rng = np.random.default_rng(5)
         eng.reset()
@@ -216,7 +216,7 @@ def test_full_size_layers_match_oracle(F, O):
     eng = F.Engine(cfg)
     try:
         eng.init_synthetic(seed=0, sigma=0.02)
-        om = OracleModel(F, O, eng, cfg, with_mtp=False)
+        om = oracle_twin(F, O, cfg, seed=0, with_mtp=False)
         rng = np.random.default_rng(5)
         prompt = rng.integers(0, cfg.vocab, size=21).tolist()
         eng.reset()
