@@ -198,10 +198,11 @@ def _at(t):
     return None if t is None else t.data_ptr()
 
 
-def _raw_stream(t):
-    """The current stream's handle on the current device (as _stream(), without the Stream object)."""
+def _raw_stream():
+    """What _stream() gives (the current stream of the current device), without the Stream object where torch hands out the plain handle."""
     import torch
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    get = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    return get(torch.cuda.current_device()) if get else torch.cuda.current_stream().cuda_stream
 
 
 # ------------------------------------------------------------------------------------------------ weights
@@ -261,7 +262,7 @@ def dense(W, rows: int, cols: int, x, norm_w=None, eps: float = 1e-6, out=None, 
     per = L.fnx_dense_rows(cols)
     if 0 < T <= per:
         check(L.fnx_dense(W.data_ptr(), rows, cols, x.data_ptr(), x.stride(0), T, _at(norm_w), eps, out.data_ptr(), out.stride(0), 1 if accumulate else 0,
-                          err.data_ptr(), _raw_stream(x)))
+                          err.data_ptr(), _raw_stream()))
         return out, err
     for t0 in range(0, T, per):
         nt = min(per, T - t0)
@@ -299,7 +300,7 @@ def router_route(Wr, x, K: int, norm_w=None, eps: float = 1e-6, e_lo: int = 0, e
     jobs, njobs, tail = words[:njobs_max * C.sizeof(Job) // 4].view(torch.uint8), words[jb:jb + 2], words[jb + 2:jb + 3]
     err = tail if err is None else err
     check(lib().fnx_router_route(Wr.data_ptr(), x.data_ptr(), _at(norm_w), eps, T, E, H, K, e_lo, e_hi, 1 if add_shared else 0, logits.data_ptr(), topi.data_ptr(),
-                                 topw.data_ptr(), jobs.data_ptr(), njobs.data_ptr(), None, err.data_ptr(), _raw_stream(x)))
+                                 topw.data_ptr(), jobs.data_ptr(), njobs.data_ptr(), None, err.data_ptr(), _raw_stream()))
     return dict(logits=logits, topi=topi, topw=topw, jobs=jobs, njobs=njobs, njobs_max=njobs_max, err=err, every=e_lo == 0 and e_hi == E and bool(add_shared))
 
 
@@ -316,7 +317,7 @@ def moe_experts(Wgu, Wdn, Wsh_gu, Wsh_dn, route, x, F: int, K: int, norm_w=None,
     h = new((P, F), dtype=torch.float32, device=x.device)
     part = new((P, H), dtype=torch.float32, device=x.device)
     out = torch.empty((T, H), dtype=torch.float32, device=x.device)
-    L, st = lib(), _raw_stream(x)
+    L, st = lib(), _raw_stream()
     jobs, njobs, njobs_max, err = route["jobs"].data_ptr(), route["njobs"].data_ptr(), route["njobs_max"], route["err"].data_ptr()
     hp, pp = h.data_ptr(), part.data_ptr()
     check(L.fnx_moe_gate_up(Wgu.data_ptr(), gu_stride, e_base, _at(Wsh_gu), E, jobs, njobs, njobs_max, x.data_ptr(), _at(norm_w), eps, H, F, hp, err, st))
@@ -446,7 +447,7 @@ def attn(qg, kc, vc, pos0, parent=None, scratch=None):
     out = torch.empty((T, nq, hd), dtype=torch.float32, device=qg.device)
     if scratch is None:
         scratch = torch.empty(lib().fnx_attn_scratch_bytes(T, nq, hd), dtype=torch.uint8, device=qg.device)
-    check(lib().fnx_attn(qg.data_ptr(), nq * hd2, kc.data_ptr(), vc.data_ptr(), out.data_ptr(), T, nq, nkv, hd, pos0.data_ptr(), _at(parent), scratch.data_ptr(), _raw_stream(qg)))
+    check(lib().fnx_attn(qg.data_ptr(), nq * hd2, kc.data_ptr(), vc.data_ptr(), out.data_ptr(), T, nq, nkv, hd, pos0.data_ptr(), _at(parent), scratch.data_ptr(), _raw_stream()))
     return out
 
 
