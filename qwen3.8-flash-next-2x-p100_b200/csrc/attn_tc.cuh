@@ -13,12 +13,8 @@ constexpr int ATC_HD = 256;   // head dim
 constexpr int ATC_N = 64;     // positions per step
 constexpr unsigned long long TA_WAIT_NS = 2000000000ull;   // what a wait takes at most
 
-__device__ __forceinline__ uint64_t ta_desc(uint32_t saddr, int lbo, int sbo) {
-    // shared-memory matrix descriptor: start address, leading and stride byte offsets in 16-byte units, version 1, no swizzle
-    return (uint64_t) ((saddr & 0x3FFFFu) >> 4) | ((uint64_t) (lbo >> 4) << 16) | ((uint64_t) (sbo >> 4) << 32) | (1ull << 46);
-}
-// the same for a 128-byte-swizzled tile (layout type 2); K-major: the leading offset is not used; MN-major: it is the
-// distance between the 64-element swizzle atoms along MN
+// shared-memory matrix descriptor of a 128-byte-swizzled tile (layout type 2): start address, leading and stride byte offsets in 16-byte
+// units, version 1; K-major: the leading offset is not used; MN-major: it is the distance between the 64-element swizzle atoms along MN
 __device__ __forceinline__ uint64_t ta_desc_sw(uint32_t saddr, int lbo, int sbo) {
     return (uint64_t) ((saddr & 0x3FFFFu) >> 4) | ((uint64_t) (lbo >> 4) << 16) | ((uint64_t) (sbo >> 4) << 32) | (1ull << 46) | (2ull << 61);
 }

@@ -293,7 +293,6 @@ __global__ void k_gdn_params(float* dt, float* a, int nv) {
         a[h] = -(0.5f + (float) (h % 8) / 8.0f);
     }
 }
-// dst[j] = src[idx[j]] rows of n floats
 __global__ void k_add_rows(float* __restrict__ dst, const float* __restrict__ src, size_t n) {
     const size_t i = (size_t) blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) dst[i] += src[i];
@@ -1465,7 +1464,7 @@ extern "C" int fnx_engine_lookup(fnx_engine* e, int seq, int lk, int d1, int roo
 
 // Engine::prefill (engine/src/prefill.cu: the prompt pass): the prompt's first n - 1 tokens go through the model a chunk at a time,
 // layer by layer, on the prompt-sized kernels - projections and experts on the tensor cores (fnx_dense_prompt, fnx_moe_prefill),
-// DeltaNet as one scan with the state in registers (fnx_gdn_prompt), attention over twelve rows per block (fnx_attn_prompt), the
+// DeltaNet as one scan with the state in registers (fnx_gdn_prompt), attention over sixteen rows per block (fnx_attn_prompt), the
 // router over all rows at once (fnx_router_rows) - and only caches, states and context are kept; the last token then goes through an ordinary one-row window,
 // which leaves the engine exactly as after a verify + commit (logits, emitted token, the draft layer's source row).
 extern "C" int fnx_engine_prompt(fnx_engine* e, int seq, const int* h_tok, int n) {
@@ -1475,7 +1474,7 @@ extern "C" int fnx_engine_prompt(fnx_engine* e, int seq, const int* h_tok, int n
     FNX_REQUIRE(s.pos + n <= e->c.max_ctx, "fnx_engine_prompt: %d tokens run past the context of %d rows", n, e->c.max_ctx);
     for (int t = 0; t < n; ++t) FNX_REQUIRE(h_tok[t] >= 0 && h_tok[t] < e->c.vocab, "fnx_engine_prompt: token %d outside the vocabulary", h_tok[t]);
     const Dims d = dims(e->c);
-    if (!e->pR) {   // the chunk: large enough that an expert's rows fill the 256-row tiles of the grouped product, within the context
+    if (!e->pR) {   // the chunk: large enough that an expert's rows fill many jobs of the grouped product, within the context
         if (const char* pc = getenv("FNX_PROMPT_CHUNK")) e->prompt_chunk = atoi(pc) > 0 ? atoi(pc) : e->prompt_chunk;
         if (const char* pm = getenv("FNX_ATTN_PROMPT_MMA")) e->prompt_attn_mma_sync = atoi(pm) != 0;
         if (e->prompt_chunk > e->c.max_ctx) e->prompt_chunk = e->c.max_ctx;

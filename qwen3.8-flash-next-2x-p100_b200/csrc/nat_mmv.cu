@@ -6,8 +6,9 @@
 //   - the rows come as their image (nat_image.cuh): a dense or gate|up block copies the rows it needs into shared memory and quantises
 //     nothing (read through L1 from global memory instead, the operands cost more than the weights); down quantises its few rows itself;
 //   - every lane copies its own 64 bytes of the next tiles into shared memory (cp.async): no mbarriers, no issuing lane;
-//   - a block takes half an SM's registers and shared memory at most, so that the next kernel of the window can be resident while
-//     this one drains (programmatic dependent launch): its first tiles are on their way before the rows it waits for are written.
+//   - the eight-warp forms take half an SM's registers, and most of them half its shared memory, so that the next kernel of the window can be
+//     resident while this one drains (programmatic dependent launch): its first tiles are on their way before the rows it waits for are
+//     written.  The sixteen-warp forms, for products that stream some 10 us and more, have an SM to themselves.
 // Bound by HBM for the large expert products, by the launch and its dependent loads for the small dense ones.
 #include <cooperative_groups.h>
 #include <cuda_fp16.h>

@@ -4,20 +4,22 @@
 // Replaces the reference's grouped expert GEMMs for prompts, moe_gate_up_mma / moe_down_mma (engine/src/kernels.hpp:328-330,
 // engine/src/moe_mma.cuh:301).
 //
-// What bounds it: at a few rows an expert, the weights' bytes (377 cycles of an SM's share of DRAM for 256 features x 64 columns); at
-// many, the products (8 x M128 N64 K16, 300 cycles) and the decode (16 warps x some 85 instructions, 340 cycles).  So nothing may pass
+// What it cannot do without, for 256 features x 64 columns: at a few rows an expert, the weights' bytes (377 cycles of an SM's share of
+// DRAM); at many, the products (8 x M128 N64 K16, 300 cycles) and the decode (16 warps x some 85 instructions, 340 cycles).  So nothing may pass
 // through shared memory that need not: f16 weight tiles written there by the decode and read back by the tensor core took 500 cycles
 // on their own, and 256-row tiles another 1,000 of products over rows that mostly were not there (thirteen rows an expert in a prompt
 // of 640).  Here
 //   - sixteen decode warps own a 16-row tile row each: 2,176-byte half tiles by their lanes' own async copies, four blocks ahead across
 //     items; nibbles to f16 with three shifts, four masks and twelve half operations a word of eight; the fragment layout is tcgen05.st's
 //     16x256b shape, so 64 columns leave as one store of sixteen registers;
-//   - four warps gather the job's live rows (a row of B only reaches its own column of D: the others stay what they are);
+//   - two warps gather the job's live rows (a row of B only reaches its own column of D: the others stay what they are);
 //   - one warp issues the products, one thread each, two accumulators (gate and up, or 2 x 128 features) double-buffered in tensor memory;
 //   - four warps write the item before.
 // Tensor memory: columns [0, 256) two pairs of accumulators, [256, 512) two stages of two 128 x 128 weight tiles.  Jobs have at most 64
 // rows: wider tiles pay off in the products only from some 100 rows an expert, by 20% of a bound that the decode then has alone.
-// Measured: see prompt_nat().
+// Measured: 513 jobs of gate|up (2,052 items of 256 features x 2,048 columns, fourteen an SM): 194 us, some 820 cycles a 64-column chunk, about the same
+// at six rows a job as at fifty-eight.  So none of the three sets the pace: the hand-over between the sixteen decode warps, the two weight stages in
+// tensor memory and the issuing thread does, and that is what is left here.
 #include "attn_tc.cuh"
 #include "nat_tile.h"
 #include "prompt_nat.cuh"
