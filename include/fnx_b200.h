@@ -158,7 +158,7 @@ int fnx_attn_prep_append(float* qg, int ldq, float* k, int ldk, const float* v, 
                          const int* pos0, const int* depth, float eps, float rope_base, fnx_stream st);
 /* attn (engine/src/kernels.hpp:238): softmax(q k / sqrt(hd)) v sigmoid(gate) over cache rows [0, *pos0) and the
  * window rows on row t's path to the root (parent null: a chain, the reference's causal case).
- * out [T][nq][hd].  scratch: fnx_attn_scratch_bytes(T, nq, hd) bytes (attn_scratch_floats, :131). */
+ * out [T][nq][hd].  scratch: fnx_attn_scratch_bytes(T, nq, hd) bytes on an 8-byte boundary (attn_scratch_floats, :131). */
 size_t fnx_attn_scratch_bytes(int T, int nq, int hd);
 int fnx_attn(const float* qg, int ldq, const void* kc, const void* vc, float* out, int T, int nq, int nkv, int hd,
              const int* pos0, const int* parent, void* scratch, fnx_stream st);
@@ -315,7 +315,11 @@ int fnx_engine_init_synthetic(fnx_engine* e, uint64_t seed, float sigma);
 /* bytes of weights + state this engine holds on its GPU */
 size_t fnx_engine_device_bytes(const fnx_engine* e);
 /* the engine's tensors by name, for tests and loaders: device pointer and byte size (0 if unknown).  Matrices are held in a layout of
- * the engine's own until they are asked for; one that was is held, and read by later windows and prompts, in the interchange layout */
+ * the engine's own until they are asked for; one that was (and the one that is read together with it: routed and shared experts,
+ * the two halves of the draft layer's input) is held, and read by later windows and prompts, in the interchange layout, since the
+ * caller may write to it.  That is for good, and the operators' kernels that read it are slower than those of the engine's own
+ * layout: a program that only wants to look at a served model's weights takes them from another engine of the same file or seed.
+ * The pair's copy is allocated before the old one is freed; where that fails the call returns null and nothing has changed. */
 void* fnx_engine_tensor(fnx_engine* e, const char* name, size_t* bytes);
 /* resets sequence `seq` to an empty context */
 int fnx_engine_reset(fnx_engine* e, int seq);
@@ -336,7 +340,8 @@ int fnx_engine_prompt(fnx_engine* e, int seq, const int* h_tok, int n);
 int fnx_engine_prompt_timing(fnx_engine* e, int on, float* h_phase_ms6);
 /* Engine::commit: keeps the n accepted rows h_path[0..n) of the last window of `seq`.  The window buffers (tokens,
  * acceptance result, residual rows) are shared by the engine's sequences: commit (and draft) sequence A before verifying
- * sequence B; a commit or draft for a sequence other than the one verified last returns FNX_E_STATE. */
+ * sequence B; a commit or draft for a sequence other than the one verified last returns FNX_E_STATE.  Both commits return with
+ * their window complete (its logits and rows may be read on any stream); the commit's own kernels are then on the engine's stream. */
 int fnx_engine_commit(fnx_engine* e, int seq, const int* h_path, int n);
 /* Engine::draft: the MTP layer on the rows kept by the last commit, then k - 1 chained single-row calls;
  * h_drafts receives k tokens */

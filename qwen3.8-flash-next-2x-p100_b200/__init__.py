@@ -675,7 +675,10 @@ class Engine:
         return lib().fnx_engine_device_bytes(self._h)
 
     def tensor(self, name: str, dtype, shape=None):
-        """A torch view of one of the engine's device tensors (no copy)."""
+        """A torch view of one of the engine's device tensors (no copy).
+
+        Asking for a weight matrix moves it to the interchange layout for good, and later windows and prompts to the slower kernels that
+        read that (fnx_engine_tensor); norms, routers, caches, states and buffers are handed out as they are."""
         import torch
         nbytes = C.c_size_t(0)
         p = lib().fnx_engine_tensor(self._h, name.encode(), C.byref(nbytes))
