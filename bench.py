@@ -46,7 +46,8 @@ C3_TOKENS = 38912                          # configuration 3: the cold prompt
 C4_CTX, C4_SEQS, C4_LANES = 131072, 8, 4   # configuration 4: context per sequence, sequences, lanes per window
 # A window's copies: tokens, parents, lane tables and the error word in one block of 168 words; the error word and a result of 65 words back
 WINDOW_IN, WINDOW_OUT = 4 * 168, 4 * (4 + 65)
-E_B = 1351680          # bytes of one expert: (2*512*2048 + 2048*512) * 110 / 256
+# bytes of one expert in IQ3_S blocks, (2*512*2048 + 2048*512) * 110 / 256: what the format needs (an engine's windows read 17 / 32 B a weight)
+E_B = 1351680
 # DRAM bytes per expert job of the gate|up launch, from an ncu capture of one launch (dram__bytes_read.sum +
 # dram__bytes_write.sum = 42.02 MB for 46 jobs; the algorithmic figure is 901,120 bytes per job)
 NCU_TRAFFIC_PER_JOB = 42.02e6 / 46
@@ -398,7 +399,7 @@ def run_config3(a, F, eng, cfg, rank, world, local, use_peer):
               "out_proj": 2.0 * n * H * (n_attn * cfg.n_q_head * cfg.head_dim + (L - n_attn) * cfg.gdn_v_head * cfg.gdn_head_dim),
               "attention": 4.0 * cfg.n_q_head * cfg.head_dim * (n * (n + 1) / 2.0) * n_attn}
         tf = {k: fl[k] / (phases[k] * 1e-3) / 1e12 for k in fl if phases.get(k, 0) > 0}
-        roof = {"bound": "tensor", "kernel": "k_gemm_tma_jobs (grouped expert products on tcgen05.mma, operands by tensor copies; the phase also decodes the experts to f16, copies the rows into job order and combines)", "achieved": tf.get("experts"), "peak": peak, "unit": "TFLOP/s",
+        roof = {"bound": "tensor", "kernel": "k_prompt_nat (grouped expert products on tcgen05.mma, weights decoded into tensor memory; the phase also lists the jobs, norms the rows and combines)", "achieved": tf.get("experts"), "peak": peak, "unit": "TFLOP/s",
                 "frac": tf.get("experts", 0.0) / peak, "peak_kind": "measured (sustained)" if pk else "fallback", "traffic": None,
                 "tflops_by_phase": tf, "note": "device ms per phase from CUDA events around the phases of every layer and chunk, in an extra pass of the same prompt; "
                 "projections, experts and attention run on tcgen05.mma"}
@@ -770,7 +771,7 @@ def main():
         cB = eng.counters()
         jobs_v = cB[1] - cA[1]
         prim, allb = step_bytes(jobs_v, a.ctx + done, T)
-        line["step_roofline"] = {"bound": "hbm", "primary_bytes": prim, "all_bytes": allb, "achieved_primary_gbs": prim / (verify_ms * 1e-3) / 1e9,
+        line["step_roofline"] = {"bound": "hbm", "weight_bytes": "IQ3_S blocks, 110/256 B a weight (the windows read 17/32)", "primary_bytes": prim, "all_bytes": allb, "achieved_primary_gbs": prim / (verify_ms * 1e-3) / 1e9,
                                  "achieved_all_gbs": allb / (verify_ms * 1e-3) / 1e9, "peak": hbm_peak, "peak_kind": peak_kind,
                                  "frac_primary_of_measured": prim / (verify_ms * 1e-3) / 1e9 / hbm_peak,
                                  "frac_primary_of_nominal_8TBs": prim / (verify_ms * 1e-3) / 1e9 / 8000.0,

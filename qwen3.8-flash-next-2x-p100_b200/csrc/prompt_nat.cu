@@ -18,8 +18,8 @@
 // Tensor memory: columns [0, 256) two pairs of accumulators, [256, 512) two stages of two 128 x 128 weight tiles.  Jobs have at most 64
 // rows: wider tiles pay off in the products only from some 100 rows an expert, by 20% of a bound that the decode then has alone.
 // Measured: 513 jobs of gate|up (2,052 items of 256 features x 2,048 columns, fourteen an SM): 194 us, some 820 cycles a 64-column chunk, about the same
-// at six rows a job as at fifty-eight.  So none of the three sets the pace: the hand-over between the sixteen decode warps, the two weight stages in
-// tensor memory and the issuing thread does, and that is what is left here.
+// at six rows a job as at fifty-eight.  So none of the three by itself sets the pace (issue slots 70% busy, tensor pipe 35%, DRAM 2.7 TB/s): the hand-over between the
+// sixteen decode warps, the two weight stages in tensor memory and the issuing thread comes on top, and that is what is left here.
 #include "attn_tc.cuh"
 #include "nat_tile.h"
 #include "prompt_nat.cuh"
