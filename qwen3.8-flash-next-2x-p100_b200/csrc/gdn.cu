@@ -478,147 +478,132 @@ __global__ void __launch_bounds__(GDP_THREADS) k_gdn_pre(const float* __restrict
     }
 }
 
-// block = (value head, 32 columns), one to an SM; a warp holds eight columns of the state in registers, all 128 key rows of them: lane = 16 cg + kg has
-// the key rows 4 kg .. + 3 and 64 + 4 kg .. + 3 of the columns 4 cg .. + 3, so nothing in the chain sums -> w -> state is block-wide.  What bounds it is
-// the registers' fill rate from shared memory (32 words a cycle; 73% busy), then a lone warp's own latencies on each scheduler and the products
-// (FMA pipe 53%): a lane's operands of k, q and c serve four columns.  (Two columns a lane, the state cut over four warps of two blocks an SM and the
-// sums added behind block barriers: 433 us for 3,001 rows, 372 now; 38,912 rows 5.3 ms, 4.4 now.)  A group's eight sums a column cross the
-// sixteen key lanes by halving; lane kg meets row (kg & 7) ^ i at place i, so that no lane has to choose which half it gives, and ends with sum
-// kg & 7.  The k sums first: w is on its way through shared memory under the q sums.  Groups come through four stages.
-constexpr int GDS_COLS = 32, GDS_STAGES = 4, GDS_CW = 8;
-constexpr int GDS_KQ_BYTES = 2 * GDP_ROWS * GDN_HS * 4, GDS_C = 0, GDS_V = GDP_ROWS * GDN_HS, GDS_CF = GDS_V + GDP_ROWS * GDS_COLS, GDS_REST = GDS_CF + 96;   // floats
-constexpr int GDS_W = GDS_THREADS / 32 * GDP_ROWS * GDS_CW;
-constexpr int GDS_SMEM = GDS_KQ_BYTES + GDS_STAGES * (GDS_KQ_BYTES + GDS_REST * 4) + GDS_W * 4;   // (the first term: room to align)
-constexpr int GDS_SMEM_ALONE = 116 * 1024;   // more than half an SM's
+// block = (value head, 16 columns), two to an SM so that one's loads and barriers pass while the other works: a warp holds 32 key rows
+// of the state in registers, lane = 8 of them (lane / 8) x two columns.  Bound by instructions (some 430 a warp and group) and the
+// shared memory's rate: k, q and c are broadcast, two columns a lane halve their loads; then by the chain partial sums -> sums -> w ->
+// state between two barriers.  Row by row that chain took 560 cycles a row.  Groups come through three stages of shared memory.
+constexpr int GDS_COLS = 16, GDS_STAGES = 3, GDS_PARTS = 2 * GDS_THREADS / 32, GDS_PART = 2 * GDP_ROWS * GDS_COLS + GDS_COLS;   // (the parts 16 banks apart)
+constexpr int GDS_K = 0, GDS_QO = GDP_ROWS * GDN_HS, GDS_CO = 2 * GDS_QO, GDS_V = 3 * GDS_QO, GDS_C = GDS_V + GDP_ROWS * GDS_COLS, GDS_STAGE = GDS_C + GC_FLOATS;   // floats
+constexpr int GDS_SMEM = (GDS_STAGES * GDS_STAGE + GDS_PARTS * GDS_PART + 4 * GDP_ROWS * GDS_COLS) * (int) sizeof(float);
 __global__ void __launch_bounds__(GDS_THREADS, 2) k_gdn_scan(const float* __restrict__ xq, const float* __restrict__ xk, const float* __restrict__ xv,
-                                                          const float* __restrict__ xc, const float* __restrict__ coef, const float* __restrict__ S_in,
-                                                          float* __restrict__ S_out, float* __restrict__ o, int nk, int nv, int T) {
-    pdl_begin();
-    constexpr int R = GDP_ROWS, HS = GDN_HS, C = GDS_COLS, SL = HS / C, NC = 4;
-    extern __shared__ __align__(128) uint8_t gds_raw[];
-    const uint32_t kq_s = (smem_u32(gds_raw) + GDS_KQ_BYTES - 1) & ~(uint32_t) (GDS_KQ_BYTES - 1);   // [stage][k of 8 rows, q of 8 rows][HS]
-    float* rest = reinterpret_cast<float*>(gds_raw + (kq_s - smem_u32(gds_raw)) + GDS_STAGES * GDS_KQ_BYTES);   // [stage][c, v, coefficients]
+                                                             const float* __restrict__ xc, const float* __restrict__ coef, const float* __restrict__ S_in,
+                                                             float* __restrict__ S_out, float* __restrict__ o, int nk, int nv, int T) {
+    constexpr int R = GDP_ROWS, HS = GDN_HS, C = GDS_COLS, SL = HS / C;
+    extern __shared__ __align__(16) float gds[];
+    float* red = gds + GDS_STAGES * GDS_STAGE;             // [parts][k sums, q sums of 8 rows][columns]
+    float* ws = red + GDS_PARTS * GDS_PART;                // [8][columns]
+    float2* w2 = reinterpret_cast<float2*>(ws + R * C);    // [2][8][columns / 2]: a lane's two columns, the one whose sums it keeps first
     const int lv = blockIdx.x / SL, col0 = blockIdx.x % SL * C, kh = lv % nk, tid = threadIdx.x;
-    const int warp = tid >> 5, lane = tid & 31, kg = lane & 15, cg = lane >> 4, ng = (T + R - 1) / R;
-    const int row = kg & 7;                          // of the sums that the lane ends with
-    const int mycol = warp * GDS_CW + cg * NC;       // in the block
-    float* ws = rest + GDS_STAGES * GDS_REST + warp * (R * GDS_CW);   // the warp's w: [8 rows][8 columns]
-    const size_t soff = (size_t) lv * HS * HS + col0 + mycol;
-    auto key_of = [&](int p) { return (p >> 1) * (HS / 2) + kg * 4 + (p & 1) * 2; };   // pair p: this key row and the next
-    uint64_t s[NC][4];
+    const int warp = tid >> 5, lane = tid & 31, cp = lane & 7, up = lane >> 4, ng = (T + R - 1) / R;
+    const int key0 = warp * 32 + (lane >> 3) * 8, keep = cp + 8 * up, part = warp * 2 + ((lane >> 3) & 1);
+    const int row = tid / C, col = tid % C;                // of the sums that the thread completes
+    const size_t soff = (size_t) lv * HS * HS + (size_t) key0 * HS + col0;
+    uint64_t s[2][4];   // the thread's 16 state values: its column `keep` and the other, key rows (2 i, 2 i + 1)
 #pragma unroll
-    for (int c = 0; c < NC; ++c)   // (the caller's state may lie on any 4-byte boundary)
+    for (int c = 0; c < 2; ++c)
 #pragma unroll
-        for (int p = 0; p < 4; ++p) s[c][p] = f2_pack(S_in[soff + (size_t) key_of(p) * HS + c], S_in[soff + (size_t) (key_of(p) + 1) * HS + c]);
-    // the thread's 16-byte pieces of a stage: two of k, q and c each, and one of v or the coefficients
+        for (int i = 0; i < 4; ++i) s[c][i] = f2_pack(S_in[soff + (size_t) (2 * i) * HS + (keep ^ (8 * c))], S_in[soff + (size_t) (2 * i + 1) * HS + (keep ^ (8 * c))]);
+    // the thread's 16-byte pieces of a stage: a piece of two rows of k, q and c each, and a few of v and the coefficients
     const int pr = tid >> 5, pe = lane * 4;
-    const uint32_t rest_s = smem_u32(rest);
+    const uint32_t tile_s = smem_u32(gds) + tid * 16;
     const float* gk = xk + ((size_t) pr * nk + kh) * HS + pe;
     const float* gq = xq + ((size_t) pr * nk + kh) * HS + pe;
     const float* gc = xc + ((size_t) pr * nv + lv) * HS + pe;
-    constexpr int VP = R * C / 4;
-    const float* gv = tid < VP ? xv + ((size_t) (tid / (C / 4)) * nv + lv) * HS + col0 + tid % (C / 4) * 4 : coef + (size_t) lv * GC_FLOATS + (tid - VP) * 4;
-    const size_t kstep = (size_t) R * nk * HS, cstep = (size_t) R * nv * HS, vstep = tid < VP ? cstep : (size_t) nv * GC_FLOATS;
-    const bool has_v = tid < VP + GC_FLOATS / 4;
-    static_assert(GDS_THREADS == 128 && HS == 128 && R == 8 && GDS_CF == GDS_V + VP * 4 && VP + GC_FLOATS / 4 <= GDS_THREADS && GDS_THREADS / 32 * GDS_CW == C, "the pieces above");
+    const float* gv = tid < R * C / 4 ? xv + ((size_t) (tid / (C / 4)) * nv + lv) * HS + col0 + tid % (C / 4) * 4 : coef + (size_t) lv * GC_FLOATS + (tid - R * C / 4) * 4;
+    const size_t kstep = (size_t) R * nk * HS, cstep = (size_t) R * nv * HS, vstep = tid < R * C / 4 ? cstep : (size_t) nv * GC_FLOATS;
+    const bool has_v = tid < R * C / 4 + GC_FLOATS / 4;
     auto cp16 = [](uint32_t dst, const float* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); };
     auto stage = [&](int g) {
         if (g < ng) {
-            const uint32_t dk = kq_s + g % GDS_STAGES * GDS_KQ_BYTES + tid * 16, dr = rest_s + g % GDS_STAGES * (GDS_REST * 4) + tid * 16;
-            cp16(dk, gk); cp16(dk + 2048, gk + (size_t) 4 * nk * HS);
-            cp16(dk + 4096, gq); cp16(dk + 6144, gq + (size_t) 4 * nk * HS);
-            cp16(dr, gc); cp16(dr + 2048, gc + (size_t) 4 * nv * HS);
-            if (has_v) cp16(dr + GDS_V * 4, gv);
+            const uint32_t d = tile_s + g % GDS_STAGES * (GDS_STAGE * 4);
+            cp16(d, gk); cp16(d + 2048, gk + (size_t) 4 * nk * HS);
+            cp16(d + GDS_QO * 4, gq); cp16(d + GDS_QO * 4 + 2048, gq + (size_t) 4 * nk * HS);
+            cp16(d + GDS_CO * 4, gc); cp16(d + GDS_CO * 4 + 2048, gc + (size_t) 4 * nv * HS);
+            if (has_v) cp16(d + GDS_V * 4, gv);
             gk += kstep; gq += kstep; gc += cstep; gv += vstep;
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
+    static_assert(GDS_THREADS == GDP_ROWS * GDS_COLS && GDS_THREADS * 4 == 4 * GDN_HS && GDS_C == GDS_V + GDP_ROWS * GDS_COLS, "the pieces above");
 #pragma unroll
     for (int g = 0; g < GDS_STAGES - 1; ++g) stage(g);
-    const uint32_t lane_kq = (uint32_t) row * 512u + (uint32_t) kg * 16u;
-    float* od = o + ((size_t) row * nv + lv) * HS + col0 + mycol;
+    asm volatile("cp.async.wait_group %0;" ::"n"(GDS_STAGES - 2) : "memory");
+    __syncthreads();
+    float* od = o + ((size_t) row * nv + lv) * HS + col0 + col;
     const size_t ostep = (size_t) R * nv * HS;
-    struct Sum {
-        float v[NC];
-    };
 #pragma unroll 1
     for (int g = 0; g < ng; ++g, od += ostep) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(GDS_STAGES - 2) : "memory");
-        __syncthreads();               // the group is in, and everyone is done with the one before
-        stage(g + GDS_STAGES - 1);     // (into that one's place)
-        const uint32_t base = (kq_s + g % GDS_STAGES * GDS_KQ_BYTES) | lane_kq;
-        const float* tl = rest + g % GDS_STAGES * GDS_REST;
-        const float* cf = tl + GDS_CF;
-        // row (kg & 7) ^ i of k (qo = 0) or q times the lane's part of the state
-        auto dot = [&](int i, int qo) {
-            const uint32_t a = base ^ (uint32_t) (i * 512);
-            uint64_t x0, x1, x2, x3;
-            asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(x0), "=l"(x1) : "r"(a + qo));
-            asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(x2), "=l"(x3) : "r"(a + qo + 256));
-            Sum r;
-#pragma unroll
-            for (int c = 0; c < NC; ++c) {
-                float lo, hi;
-                f2_unpack(f2_fma(s[c][3], x3, f2_fma(s[c][2], x2, f2_fma(s[c][1], x1, f2_mul(s[c][0], x0)))), lo, hi);
-                r.v[c] = lo + hi;
-            }
-            return r;
-        };
-        auto fold = [&](Sum a, const Sum& b, int o) {   // place i keeps, place i + o goes to the lane that has its row at place i
-#pragma unroll
-            for (int c = 0; c < NC; ++c) a.v[c] += __shfl_xor_sync(0xffffffffu, b.v[c], o);
-            return a;
-        };
-        auto sums = [&](int qo) {
-            const Sum a = fold(fold(dot(0, qo), dot(4, qo), 4), fold(dot(2, qo), dot(6, qo), 4), 2);
-            const Sum b = fold(fold(dot(1, qo), dot(5, qo), 4), fold(dot(3, qo), dot(7, qo), 4), 2);
-            const Sum r = fold(a, b, 1);
-            return fold(r, r, 8);
-        };
-        const Sum ks = sums(0);
-        if (kg < R) {
-            const float bv = cf[GC_BV + row], bk = cf[GC_BK + row];
-            const float4 v = *reinterpret_cast<const float4*>(tl + GDS_V + row * C + mycol);
-            *reinterpret_cast<float4*>(ws + row * GDS_CW + cg * NC) = make_float4(bv * v.x - bk * ks.v[0], bv * v.y - bk * ks.v[1], bv * v.z - bk * ks.v[2], bv * v.w - bk * ks.v[3]);
-        }
-        const Sum sum = sums(R * HS * 4);
-        float a[NC];
-        const float bq = cf[GC_BQ + row], bc = cf[GC_BC];
-        const uint64_t bc2 = f2_pack(bc, bc);
-        const float4 m0 = *reinterpret_cast<const float4*>(cf + GC_M + row * R), m1 = *reinterpret_cast<const float4*>(cf + GC_M + row * R + 4);
-        const float m[R] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
-#pragma unroll
-        for (int c = 0; c < NC; ++c) {
-            a[c] = bq * sum.v[c];
-#pragma unroll
-            for (int p = 0; p < 4; ++p) s[c][p] = f2_mul(bc2, s[c][p]);
-        }
-        __syncwarp();
+        const float* tl = gds + g % GDS_STAGES * GDS_STAGE;
+        float* rp = red + part * GDS_PART + keep;
 #pragma unroll
         for (int i = 0; i < R; ++i) {
-            const float4 w = *reinterpret_cast<const float4*>(ws + i * GDS_CW + cg * NC);
-            const ulonglong2 c0 = *reinterpret_cast<const ulonglong2*>(tl + GDS_C + i * HS + kg * 4), c1 = *reinterpret_cast<const ulonglong2*>(tl + GDS_C + i * HS + HS / 2 + kg * 4);
-            const float wc[NC] = {w.x, w.y, w.z, w.w};
+            const ulonglong2 k0 = *reinterpret_cast<const ulonglong2*>(tl + GDS_K + i * HS + key0), k1 = *reinterpret_cast<const ulonglong2*>(tl + GDS_K + i * HS + key0 + 4);
+            const ulonglong2 q0 = *reinterpret_cast<const ulonglong2*>(tl + GDS_QO + i * HS + key0), q1 = *reinterpret_cast<const ulonglong2*>(tl + GDS_QO + i * HS + key0 + 4);
+            float ks[2], qs[2];
 #pragma unroll
-            for (int c = 0; c < NC; ++c) {
-                const uint64_t ww = f2_pack(wc[c], wc[c]);
-                s[c][0] = f2_fma(c0.x, ww, s[c][0]); s[c][1] = f2_fma(c0.y, ww, s[c][1]); s[c][2] = f2_fma(c1.x, ww, s[c][2]); s[c][3] = f2_fma(c1.y, ww, s[c][3]);
+            for (int c = 0; c < 2; ++c) {
+                const uint64_t ka = f2_fma(s[c][3], k1.y, f2_fma(s[c][2], k1.x, f2_fma(s[c][1], k0.y, f2_mul(s[c][0], k0.x))));
+                const uint64_t qa = f2_fma(s[c][3], q1.y, f2_fma(s[c][2], q1.x, f2_fma(s[c][1], q0.y, f2_mul(s[c][0], q0.x))));
+                float lo, hi;
+                f2_unpack(ka, lo, hi);
+                ks[c] = lo + hi;
+                f2_unpack(qa, lo, hi);
+                qs[c] = lo + hi;
             }
-            if (i <= row) {   // (m is 0 beyond, w need not be finite there)
-#pragma unroll
-                for (int c = 0; c < NC; ++c) a[c] = fmaf(m[i], wc[c], a[c]);
-            }
+            // another eight key rows' sums of the column this lane keeps
+            rp[i * C] = ks[0] + __shfl_xor_sync(0xffffffffu, ks[1], 16);
+            rp[(R + i) * C] = qs[0] + __shfl_xor_sync(0xffffffffu, qs[1], 16);
         }
-        if (kg < R && g * R + row < T) *reinterpret_cast<float4*>(od) = make_float4(a[0], a[1], a[2], a[3]);
+        __syncthreads();
+        stage(g + GDS_STAGES - 1);   // (into the slot of the group before: its last readers passed the barrier above)
+        const float* cf = tl + GDS_C;
+        float ksw = 0.f, qsw = 0.f;
+#pragma unroll
+        for (int p = 0; p < GDS_PARTS; ++p) {
+            ksw += red[p * GDS_PART + row * C + col];
+            qsw += red[p * GDS_PART + (R + row) * C + col];
+        }
+        {
+            const float w = cf[GC_BV + row] * tl[GDS_V + row * C + col] - cf[GC_BK + row] * ksw;
+            const int h = col >> 3;
+            ws[row * C + col] = w;
+            (&w2[row * 8 + (col & 7)].x)[h] = w;
+            (&w2[(R + row) * 8 + (col & 7)].x)[h ^ 1] = w;
+        }
+        asm volatile("cp.async.wait_group %0;" ::"n"(GDS_STAGES - 2) : "memory");   // the next group is in
+        __syncthreads();
+        const float bc = cf[GC_BC];
+        const uint64_t bc2 = f2_pack(bc, bc);
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+#pragma unroll
+            for (int p = 0; p < 4; ++p) s[c][p] = f2_mul(bc2, s[c][p]);
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const float2 w = w2[(up * R + i) * 8 + cp];
+            const ulonglong2 c0 = *reinterpret_cast<const ulonglong2*>(tl + GDS_CO + i * HS + key0), c1 = *reinterpret_cast<const ulonglong2*>(tl + GDS_CO + i * HS + key0 + 4);
+            const uint64_t wx = f2_pack(w.x, w.x), wy = f2_pack(w.y, w.y);
+            s[0][0] = f2_fma(c0.x, wx, s[0][0]); s[0][1] = f2_fma(c0.y, wx, s[0][1]); s[0][2] = f2_fma(c1.x, wx, s[0][2]); s[0][3] = f2_fma(c1.y, wx, s[0][3]);
+            s[1][0] = f2_fma(c0.x, wy, s[1][0]); s[1][1] = f2_fma(c0.y, wy, s[1][1]); s[1][2] = f2_fma(c1.x, wy, s[1][2]); s[1][3] = f2_fma(c1.y, wy, s[1][3]);
+        }
+        {
+            const float4 m0 = *reinterpret_cast<const float4*>(cf + GC_M + row * R), m1 = *reinterpret_cast<const float4*>(cf + GC_M + row * R + 4);
+            const float m[R] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
+            float a = cf[GC_BQ + row] * qsw;
+#pragma unroll
+            for (int j = 0; j < R; ++j)
+                if (j <= row) a = fmaf(m[j], ws[j * C + col], a);   // (m is 0 beyond, w need not be finite there)
+            if (g * R + row < T) *od = a;
+        }
     }
 #pragma unroll
-    for (int c = 0; c < NC; ++c)
+    for (int c = 0; c < 2; ++c)
 #pragma unroll
-        for (int p = 0; p < 4; ++p) {
+        for (int i = 0; i < 4; ++i) {
             float x, y;
-            f2_unpack(s[c][p], x, y);
-            S_out[soff + (size_t) key_of(p) * HS + c] = x;
-            S_out[soff + (size_t) (key_of(p) + 1) * HS + c] = y;
+            f2_unpack(s[c][i], x, y);
+            S_out[soff + (size_t) (2 * i) * HS + (keep ^ (8 * c))] = x;
+            S_out[soff + (size_t) (2 * i + 1) * HS + (keep ^ (8 * c))] = y;
         }
 }
 
@@ -735,10 +720,9 @@ extern "C" int fnx_gdn_prompt(const float* qkvz, int ldx, const float* ab, int l
     FNX_CUDA_OK(launch_after(k_gdn_pre, dim3(ng, nk + nv * GDN_HS / GDP_THREADS), dim3(GDP_THREADS), 0, s, qkvz, ldx, ab, ldab, hin, hist_pool + (size_t) out_slot * hsz, convw, dt, a, xq, xk, xv, xc,
                                                                                coef, nk, nv, T));
     FNX_LAUNCH_OK("k_gdn_pre");
-    // blocks that all fit at once are kept to one an SM, by the shared memory they ask for: a warp has a scheduler to itself, whoever else is draining
-    const int blocks = nv * (GDN_HS / GDS_COLS), smem = blocks <= sm_count() ? GDS_SMEM_ALONE : GDS_SMEM;
-    FNX_TRY(set_smem_limit((const void*) k_gdn_scan, GDS_SMEM_ALONE));
-    FNX_CUDA_OK(launch_after(k_gdn_scan, dim3(blocks), dim3(GDS_THREADS), smem, s, xq, xk, xv, xc, coef, S_pool + (size_t) cur_host * ssz, S_pool + (size_t) out_slot * ssz, o, nk, nv, T));
+    FNX_TRY(set_smem_limit((const void*) k_gdn_scan, GDS_SMEM));
+    // (not ahead of its predecessor's end: blocks that fill the SMs as these come free sit three to some and one to others, 600 us instead of 440 for 3,001 rows)
+    FNX_CUDA_OK(launch_dep(false, k_gdn_scan, dim3(nv * (GDN_HS / GDS_COLS)), dim3(GDS_THREADS), GDS_SMEM, s, xq, xk, xv, xc, coef, S_pool + (size_t) cur_host * ssz, S_pool + (size_t) out_slot * ssz, o, nk, nv, T));
     FNX_LAUNCH_OK("k_gdn_scan");
     const bool vec = ldx % 4 == 0 && (((uintptr_t) qkvz | (uintptr_t) nw | (uintptr_t) y) & 15) == 0;
     FNX_CUDA_OK(launch_after(vec ? k_gdn_post<true> : k_gdn_post<false>, dim3(T), dim3(GDP_THREADS), 0, s, o, qkvz, ldx, nw, y, nk, nv, eps));
