@@ -546,44 +546,59 @@ __global__ void k_pf_xnorm(const float* __restrict__ x, const float* __restrict_
 }
 
 // out[t] (+)= sum_k topw[t][k] part[t Kp + k] + sigmoid(logit[t][E]) part[T Kp + t]
-__global__ void k_pf_combine(const float* __restrict__ part, const int* __restrict__ topi, const float* __restrict__ topw, const float* __restrict__ logits,
-                             int T, int E, int H, int Kp, int e_lo, int e_hi, int add_shared, float* __restrict__ out, int accumulate) {
+// A thread owns four columns of one row.  EVERY: all experts are this rank's, so no addend is left out: its load waits for nothing (asked for
+// only where the pick's weight had been seen not to be zero, the same loads took 98 us for 3,001 rows of eleven addends, 56 now; 38,912 rows 1,065 and 605).
+// Bound by the addends' way from DRAM (5.8 TB/s of them, 6.8 with the rows read and written); four blocks an SM, to whose 64 registers the loads just fit
+// (three: 68 and 682 us).
+constexpr int PC_ADD = 11;   // addends in flight a thread (top 10 and the shared expert: all of them)
+template <bool EVERY>
+__global__ void __launch_bounds__(256, 4) k_pf_combine(const float* __restrict__ part, const int* __restrict__ topi, const float* __restrict__ topw,
+                                                    const float* __restrict__ logits, int T, int E, int H, int Kp, int e_lo, int e_hi, int add_shared,
+                                                    float* __restrict__ out, int accumulate) {
     pdl_begin();
-    // a thread owns four columns of one row; the picks' weights first, then every addend's 16-byte load in flight at once
-    const int t = blockIdx.y, i = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
+    const int t = blockIdx.y, i = (blockIdx.x * blockDim.x + threadIdx.x) * 4, n = Kp + (add_shared ? 1 : 0);
     if (i >= H) return;
-    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int k0 = 0; k0 < Kp; k0 += 16) {   // sixteen picks at a time (the sum stays in pick order)
-        float w[16];
-        float4 v[16];
-#pragma unroll
-        for (int k = 0; k < 16; ++k) {
-            w[k] = 0.f;
-            if (k0 + k < Kp) {
-                const int e = topi[t * Kp + k0 + k];
-                w[k] = e >= e_lo && e < e_hi ? topw[t * Kp + k0 + k] : 0.f;
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < 16; ++k)
-            v[k] = w[k] != 0.f ? *reinterpret_cast<const float4*>(part + ((size_t) t * Kp + k0 + k) * H + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int k = 0; k < 16; ++k) {
-            s.x = fmaf(w[k], v[k].x, s.x); s.y = fmaf(w[k], v[k].y, s.y);
-            s.z = fmaf(w[k], v[k].z, s.z); s.w = fmaf(w[k], v[k].w, s.w);
-        }
-    }
-    if (add_shared) {
-        const float g = sigmoidf_(logits[(size_t) t * (E + 1) + E]);
-        const float4 sh = *reinterpret_cast<const float4*>(part + ((size_t) T * Kp + t) * H + i);
-        s.x += g * sh.x; s.y += g * sh.y; s.z += g * sh.z; s.w += g * sh.w;
-    }
     float4* o = reinterpret_cast<float4*>(out + (size_t) t * H + i);
-    if (accumulate) {
-        const float4 p0 = *o;
-        s.x += p0.x; s.y += p0.y; s.z += p0.z; s.w += p0.w;
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f), old = s;
+    if (accumulate) old = *o;
+    for (int k0 = 0; k0 < n; k0 += PC_ADD) {   // (the sum stays in pick order, the shared expert last)
+        float w[PC_ADD];
+        float4 v[PC_ADD];
+#pragma unroll
+        for (int k = 0; k < PC_ADD; ++k) {   // (past the last addend: that one again, with weight 0)
+            const int a = min(k0 + k, n - 1);
+            if (a == Kp) w[k] = sigmoidf_(logits[(size_t) t * (E + 1) + E]);
+            else {
+                w[k] = topw[(size_t) t * Kp + a];
+                if (!EVERY) {
+                    const int e = topi[(size_t) t * Kp + a];
+                    if (e < e_lo || e >= e_hi) w[k] = 0.f;
+                }
+            }
+            if (k0 + k >= n) w[k] = 0.f;
+        }
+#pragma unroll
+        for (int k = 0; k < PC_ADD; ++k) {
+            const int a = min(k0 + k, n - 1);
+            const float4* p = reinterpret_cast<const float4*>(part + (a == Kp ? (size_t) T * Kp + t : (size_t) t * Kp + a) * H + i);
+            v[k] = EVERY || w[k] != 0.f ? __ldcs(p) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int k = 0; k < PC_ADD; ++k) {
+            const bool in = w[k] != 0.f;   // (an addend of weight 0 has no part in it, whatever it holds)
+            s.x = fmaf(w[k], in ? v[k].x : 0.f, s.x); s.y = fmaf(w[k], in ? v[k].y : 0.f, s.y);
+            s.z = fmaf(w[k], in ? v[k].z : 0.f, s.z); s.w = fmaf(w[k], in ? v[k].w : 0.f, s.w);
+        }
     }
-    *o = s;
+    *o = accumulate ? make_float4(s.x + old.x, s.y + old.y, s.z + old.z, s.w + old.w) : s;
+}
+
+static int pf_combine(const float* part, const int* topi, const float* topw, const float* logits, int T, int E, int H, int K, int e_lo, int e_hi, int add_shared, float* out,
+                      int accumulate, cudaStream_t st) {
+    auto kernel = e_lo == 0 && e_hi == E ? k_pf_combine<true> : k_pf_combine<false>;
+    FNX_CUDA_OK(launch_after(kernel, dim3((H / 4 + 255) / 256, T), dim3(256), 0, st, part, topi, topw, logits, T, E, H, K, e_lo, e_hi, add_shared, out, accumulate));
+    FNX_LAUNCH_OK("k_pf_combine");
+    return FNX_OK;
 }
 
 // A tile matrix decoded once to f16, row-major [rows][K]: the values the grouped product's own decode makes (the same codebook
@@ -765,9 +780,7 @@ int prompt_moe(const void* Wgu, size_t gu_stride, const void* Wsh_gu, bool gu_na
         FNX_LAUNCH_OK("k_pf_gather_rows");
         const int nj = (int) ((size_t) n / PF_N) + ne + (T + PF_N - 1) / PF_N;
         FNX_TRY(gemm_tma_experts(gu16, dn16, E + 1, xs, hbuf, part, jobs, njobs, order, nj, (int) pairs, H, F, err, st));
-        FNX_CUDA_OK(launch_after(k_pf_combine, dim3((H / 4 + 255) / 256, T), dim3(256), 0, st, part, topi, topw, logits, T, E, H, K, e_lo, e_hi, add_shared, out, accumulate));
-        FNX_LAUNCH_OK("k_pf_combine");
-        return FNX_OK;
+        return pf_combine(part, topi, topw, logits, T, E, H, K, e_lo, e_hi, add_shared, out, accumulate, st);
     }
     // the job count is known on the device only: the grids cover the largest it can be (an expert's pairs in jobs of `per` rows:
     // at most one ragged job per expert beyond pairs / per) and the blocks past the count leave at once; nothing is read back
@@ -798,9 +811,7 @@ int prompt_moe(const void* Wgu, size_t gu_stride, const void* Wsh_gu, bool gu_na
         FNX_CUDA_OK(launch_after(k_pf_gemm<0>, dim3(nj, H / PF_M), dim3(PF_BLOCK), pf_smem(0), st, p));
         FNX_LAUNCH_OK("k_pf_gemm (down)");
     }
-    FNX_CUDA_OK(launch_after(k_pf_combine, dim3((H / 4 + 255) / 256, T), dim3(256), 0, st, part, topi, topw, logits, T, E, H, K, e_lo, e_hi, add_shared, out, accumulate));
-    FNX_LAUNCH_OK("k_pf_combine");
-    return FNX_OK;
+    return pf_combine(part, topi, topw, logits, T, E, H, K, e_lo, e_hi, add_shared, out, accumulate, st);
 }
 }  // namespace fnxb
 

@@ -38,3 +38,35 @@ def test_job_lists_do_not_show_in_the_rows(F, T):
     (some, err), (every, err2) = run(T), run(820)
     assert int(err.item()) == 0 and int(err2.item()) == 0
     assert torch.equal(some, every[:T])
+
+
+@pytest.mark.parametrize("K,add_shared", [(1, True), (10, True), (11, False), (11, True), (12, True), (24, True), (32, True)])
+def test_combine_of_many_picks(F, K, add_shared):
+    """The weighted sum of a row's addends (eleven at a time) at the edges of its passes, with every expert on this rank and with a range of
+    them; an addend of weight 0 stays out whatever it holds.  Every value is one f32 multiply-add per addend, in pick order."""
+    E, H, Fn, T = 32, 512, 256, 19
+    fx = _moe_fixture(F, E, H, Fn, seed=31)
+    g = torch.Generator(device="cuda").manual_seed(K)
+    x = torch.randn((T, H), device="cuda", generator=g)
+    topi = torch.stack([torch.randperm(E, generator=torch.Generator().manual_seed(t))[:K] for t in range(T)]).int().cuda()
+    topw = torch.rand((T, K), device="cuda", generator=g)
+    topw[3, 0] = 0.0
+    logits = torch.randn((T, E + 1), device="cuda", generator=g)
+    old = torch.randn((T, H), device="cuda", generator=g)
+    run = lambda w, **kw: F.moe_prefill(fx["gu_t"], fx["dn_t"], fx["sh_gu_t"], fx["sh_dn_t"], topi, w, logits, x, Fn, **kw)[0]
+    unit = []                                            # each addend by itself, weight 1
+    for k in range(K):
+        w = torch.zeros_like(topw)
+        w[:, k] = 1.0
+        unit.append(run(w, add_shared=False).double())
+    want = sum(topw[:, k:k + 1].double() * unit[k] for k in range(K))
+    size = sum(topw[:, k:k + 1].double() * unit[k].abs() for k in range(K))
+    if add_shared:
+        sh = run(torch.zeros_like(topw), add_shared=True).double()
+        want, size = want + sh, size + sh.abs()
+    bound = (K + 3) * 2.0 ** -24 * (size + old.abs().double()) + 1e-30
+    assert ((run(topw, add_shared=add_shared).double() - want).abs() <= bound).all()
+    assert ((run(topw, add_shared=add_shared, out=old.clone(), accumulate=True).double() - (want + old.double())).abs() <= bound).all()
+    part = run(topw, add_shared=add_shared, e_lo=0, e_hi=E // 2)
+    rest = run(topw, add_shared=False, e_lo=E // 2, e_hi=E, out=part.clone(), accumulate=True)
+    assert ((rest.double() - want).abs() <= 2 * bound).all()
