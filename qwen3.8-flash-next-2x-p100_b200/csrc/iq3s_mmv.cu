@@ -49,12 +49,11 @@ __global__ void __launch_bounds__(MMV_THREADS, 1) k_iq3s_mmv(const MmvParams p) 
     S.table_s = smem_u32(table);
     S.slots = table + CORE_TABLE_BYTES;
     S.bars = reinterpret_cast<uint64_t*>(S.slots + (size_t) MMV_WARPS * R * TILE_BYTES);
-    S.bar_stride = R;
     S.cells = reinterpret_cast<uint2*>(S.bars + MMV_WARPS * R);
     S.scales = reinterpret_cast<float*>(S.cells + (size_t) JMAX * NG * (p.K / 32) * 32);
     S.rs = S.scales + (size_t) JMAX * NG * KB * 8;
     S.pieces = S.rs + NROW * 16;
-    S.jobs_s = reinterpret_cast<fnx_job*>(reinterpret_cast<uint8_t*>(S.pieces) + (size_t) MMV_WARPS * 2 * sizeof(PieceSlotT<NG, MODE>));
+    S.jobs_s = reinterpret_cast<fnx_job*>(reinterpret_cast<uint8_t*>(S.pieces) + (size_t) MMV_WARPS * 2 * sizeof(MmvPiece<NG, MODE>));
     unsigned long long* prof = g_mmv_prof ? g_mmv_prof + (size_t) blockIdx.x * MMV_PROF_SLOTS : nullptr;
     int nstamp = 0;
     // the codebook is replicated and the barriers are set up while the kernel before drains: five dense launches in a row of 12,352 x 2,048
@@ -68,18 +67,17 @@ __global__ void __launch_bounds__(MMV_THREADS, 1) k_iq3s_mmv(const MmvParams p) 
     pdl_launch_dependents();
     MMV_STAMP();
     StageRegs h;
-    stage_begin<NG, MODE, MMV_WARPS>(p, h, tid, RowPlain());
+    stage_begin<NG, MODE>(p, h, tid);
     __syncthreads();
-    WarpRing ring;
-    ring.parity = 0;
-    stage_ring(ring, S, R, warp);
-    stage_run<NG, MODE, MMV_WARPS>(p, S, ring, h, tid, blockIdx.x, gridDim.x, RowPlain(), [&]() { MMV_STAMP(); });
+    stage_run<NG, MODE>(p, S, h, tid, blockIdx.x, gridDim.x, [&]() { MMV_STAMP(); });
     if (prof && tid == 0) prof[0] = (unsigned long long) nstamp;
 }
 
 template <int NG, int MODE>
 static int launch_mmv(const MmvParams& p0, cudaStream_t st) {
     MmvParams p = p0;
+    p.upj_inv = mmv_inverse((unsigned) p.rows / 16);
+    p.nblk_inv = mmv_inverse((unsigned) sm_count());
     p.R = 6;   // tile blocks in flight per warp: as many as the shared memory left by the codebook and the images holds
     constexpr size_t LIMIT = 227 * 1024;
     while (p.R > 2 && mmv_smem_bytes<NG, MODE>(p.K, p.R, p.njobs_max) > LIMIT) --p.R;

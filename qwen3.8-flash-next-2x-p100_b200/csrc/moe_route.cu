@@ -423,13 +423,8 @@ __global__ void __launch_bounds__(32) k_combine_image(const float* __restrict__ 
 #pragma unroll
     for (int k = 0; k < 32; ++k) w[k] = k < K ? topw[t * K + k] : 0.f;
     const float shl = logits[(size_t) t * (E + 1) + E];
-    QuantTask q[QUANT_BATCH];
-    float v[QUANT_BATCH][8], nw[QUANT_BATCH][8];
-#pragma unroll
-    for (int j = 0; j < QUANT_BATCH; ++j) {
-        q[j].src = nullptr;
-        q[j].t = q[j].blk = 0;
-    }
+    QuantTask q[1];
+    float v[1][8], nw[1][8];
     q[0].src = out + (size_t) t * H + (size_t) blk * 256;
     q[0].t = t % FNX_DENSE_ROWS;
     q[0].blk = blk;
