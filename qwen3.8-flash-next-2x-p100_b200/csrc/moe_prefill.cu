@@ -786,7 +786,7 @@ int prompt_moe(const void* Wgu, size_t gu_stride, const void* Wsh_gu, bool gu_na
     // at most one ragged job per expert beyond pairs / per) and the blocks past the count leave at once; nothing is read back
     const int nj = n / per + ne + (add_shared ? (T + per - 1) / per : 0);
     PnParams q{};
-    q.e_base = e_base; q.E = E; q.jobs = jobs; q.njobs = njobs; q.order = order; q.T = T; q.TKp = n; q.Kp = K; q.err = err;
+    q.e_base = e_base; q.E = E; q.jobs = jobs; q.njobs = njobs; q.order = order; q.T = T; q.TKp = n; q.Kp = K; q.per = per; q.err = err;
     PfParams p{};
     p.e_base = e_base; p.E = E; p.jobs = jobs; p.njobs = njobs; p.order = order; p.TKp = n; p.Kp = K; p.err = err;
     if (gu_nat) {
@@ -866,7 +866,8 @@ int prompt_dense(const void* W, bool nat, int rows, int cols, const float* x, in
         FNX_TRY(prompt_nat_rows(x, norm_w, T, cols, eps, xh, false, st));
         PnParams q{};
         q.W = (const uint8_t*) W; q.T = T; q.x = xh; q.rows = rows; q.K = cols; q.out = y; q.ldo = ldy; q.accumulate = accumulate; q.err = err;
-        return prompt_nat(2, q, (T + PN_N - 1) / PN_N, st);
+        q.per = prompt_dense_rows(T, (rows + 255) / 256, sm_count());
+        return prompt_nat(2, q, (T + q.per - 1) / q.per, st);
     }
     FNX_CUDA_OK(launch_after(k_pf_xnorm, dim3(T), dim3(256), 0, st, x, norm_w, cols, eps, xh));
     FNX_LAUNCH_OK("k_pf_xnorm");

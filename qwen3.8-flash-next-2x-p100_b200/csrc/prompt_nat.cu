@@ -9,17 +9,19 @@
 // through shared memory that need not: f16 weight tiles written there by the decode and read back by the tensor core took 500 cycles
 // on their own, and 256-row tiles another 1,000 of products over rows that mostly were not there (thirteen rows an expert in a prompt
 // of 640).  Here
-//   - sixteen decode warps own a 16-row tile row each: 2,176-byte half tiles by their lanes' own async copies, four blocks ahead across
-//     items; nibbles to f16 with three shifts, four masks and twelve half operations a word of eight; the fragment layout is tcgen05.st's
+//   - sixteen decode warps own a 16-row tile row each: 2,176-byte half tiles by their lanes' own async copies, three blocks ahead across
+//     items; nibbles to f16 with one shift, four masks and eight half operations a word of eight; the fragment layout is tcgen05.st's
 //     16x256b shape, so 64 columns leave as one store of sixteen registers;
 //   - two warps gather the job's live rows (a row of B only reaches its own column of D: the others stay what they are);
 //   - one warp issues the products, one thread each, two accumulators (gate and up, or 2 x 128 features) double-buffered in tensor memory;
 //   - four warps write the item before.
-// Tensor memory: columns [0, 256) two pairs of accumulators, [256, 512) two stages of two 128 x 128 weight tiles.  Jobs have at most 64
-// rows: wider tiles pay off in the products only from some 100 rows an expert, by 20% of a bound that the decode then has alone.
-// Measured: 513 jobs of gate|up (2,052 items of 256 features x 2,048 columns, fourteen an SM): 194 us, some 820 cycles a 64-column chunk, about the same
-// at six rows a job as at fifty-eight.  So none of the three by itself sets the pace (issue slots 70% busy, tensor pipe 35%, DRAM 2.7 TB/s): the hand-over between the
-// sixteen decode warps, the two weight stages in tensor memory and the issuing thread comes on top, and that is what is left here.
+// Tensor memory: columns [0, 256) two pairs of accumulators, [256, 512) two stages of two 128 x 128 weight tiles.  Jobs have at most 64 rows, and
+// the products' N is a job's own rows in sixteens (six rows a job: 178 us with N = 64, 166).  Jobs of 128 rows halve the decode, but leave one
+// accumulator pair, whose results (6 us an item) then lie in the next item's way: 388 us for 512 jobs of 116 rows, 339 for 1,024 of 58.
+// Measured, 512 jobs of gate|up and of down (fourteen items of 256 features x 2,048 columns an SM), us: six rows a job 162 + 92, fifty-eight 179 + 115, 6,144 jobs
+// of 760 rows an expert 1,940 + 1,244 (187 + 101, 200 + 126 and 2,172 + 1,334 with four stages of rows, N = 64 and two instructions a word more).  With neither decode nor
+// products 128: the hand-over between the decode warps, the weight stages, the rows and the issuing thread, then the decode's instructions (half of the
+// issue slots), are what is left here; DRAM would allow 88.
 #include "attn_tc.cuh"
 #include "nat_tile.h"
 #include "prompt_nat.cuh"
@@ -31,14 +33,16 @@ constexpr int PN_DECODE = 16;          // warps
 constexpr int PN_EPI = 4, PN_LOAD = 2;
 constexpr int PN_W_MMA = PN_EPI, PN_W_LOAD = PN_W_MMA + 1, PN_W_DECODE = 8;   // (warp 7 idles: the decode warps start at a multiple of four)
 constexpr int PN_THREADS = (PN_W_DECODE + PN_DECODE) * 32;
-constexpr int PN_SLOTS = 4;            // half tiles in flight a decode warp
-constexpr int PN_AST = 256 / PN_KC, PN_BST = 512 / PN_KC;  // stages of A (tensor memory) and of B (shared memory)
-constexpr int PN_LAG = 2;              // chunks of B in flight
-constexpr int PN_BBOX = PN_N * 128, PN_BBYTES = PN_KC / 64 * PN_BBOX;   // 64 rows x 64 columns, 128-byte swizzle
-constexpr int PN_RING = PN_DECODE * PN_SLOTS * NAT_HALF_BYTES;
+constexpr int PN_AST = 256 / PN_KC;    // stages of A (tensor memory)
 constexpr int PN_HEAD = 1024;
-constexpr int PN_SMEM = PN_HEAD + PN_BST * PN_BBYTES + PN_RING;
-constexpr uint32_t PN_ACC = 2 * PN_N, PN_A = 256;   // tensor memory: columns of an accumulator pair, first column of the weight stages
+constexpr uint32_t PN_A = 256;         // tensor memory: first column of the weight stages
+constexpr int PN_SLOTS = 3;            // half tiles in flight a decode warp
+// Stages of B (shared memory).  The rows come from L2 in 16-byte pieces, a chunk some 1,000 cycles after it was asked for, and pace everything where few
+// chunks are on the way: 512 jobs of 58 rows, gate|up 240 us with two stages, 198 with three, 190 with four, 179 with seven and a half tile less a warp.
+constexpr int PN_BST = 7, PN_LAG = 3;  // (of which in flight)
+constexpr int PN_BBOX = PN_N * 128, PN_BBYTES = PN_KC / 64 * PN_BBOX;   // 64 rows x 64 columns, 128-byte swizzle
+constexpr int PN_SMEM = PN_HEAD + PN_BST * PN_BBYTES + PN_DECODE * PN_SLOTS * NAT_HALF_BYTES;
+constexpr uint32_t PN_ACC = 2 * PN_N;  // tensor-memory columns of an accumulator pair
 static_assert(PN_SMEM <= 227 * 1024, "fits one block's shared memory");
 
 struct PnShared {
@@ -68,41 +72,28 @@ __device__ __forceinline__ uint32_t pn_and_xor(uint32_t a, uint32_t b, uint32_t 
     asm("lop3.b32 %0, %1, %2, %3, 0x6A;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
     return d;
 }
-__device__ __forceinline__ uint32_t pn_and_or(uint32_t a, uint32_t b, uint32_t c) {
-    uint32_t d;
-    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-    return d;
-}
-// constants that stay in registers, and factors that stay multiplications (a shift would compete for the same pipe)
-struct PnConst {
-    uint32_t two, k13, m1, m4;
-    __device__ __forceinline__ PnConst() {
-        asm("mov.u32 %0, 2;" : "=r"(two));
-        asm("mov.u32 %0, 8192;" : "=r"(k13));
-        asm("mov.u32 %0, 0x001E001E;" : "=r"(m1));
-        asm("mov.u32 %0, 0x00F000F0;" : "=r"(m4));
-    }
-};
 // The eight weights of a word times the sub-block's scale (in both halves of f): out[0], out[1] = columns (0, 2), (1, 3), out[2], out[3] =
-// (4, 6), (5, 7).  A nibble t at bits 1..4 of a half 0x6400 | .. is 1024 + 2 (t + 8) = 1039 + m; at bits 4..7 it is 1024 + 16 (t + 8) =
-// 8 (143 + m): both exact, so the one rounding is that of m f, as in the other forms of these products.
-__device__ __forceinline__ void pn_decode8(const PnConst& C, uint32_t w, __half2 f, uint32_t& o0, uint32_t& o1, uint32_t& o2, uint32_t& o3) {
+// (4, 6), (5, 7).  A nibble t at bits 0..3 of a half 0x6400 | .. is 1024 + (t + 8): twice that less 2,064 is 2 t, and one multiply-add makes
+// (2 t + 1) f of it; at bits 4..7 it is 1024 + 16 (t + 8) = 8 (143 + m).  All exact but the one rounding of m f, as in the other forms of these
+// products.  (Thirteen instructions a word; with the low nibbles moved up a bit, so that 1,039 + m was left to subtract, fifteen.)
+__device__ __forceinline__ void pn_decode8(uint32_t w, __half2 f, uint32_t& o0, uint32_t& o1, uint32_t& o2, uint32_t& o3) {
     const uint32_t s = w >> 8;
-    const uint32_t a = pn_and_xor(w * C.two, C.m1, 0x64106410u), c = pn_and_xor(w, C.m4, 0x64806480u);
-    const uint32_t b = pn_and_xor(s * C.two, C.m1, 0x64106410u), d = pn_and_xor(s, C.m4, 0x64806480u);
-    const __half2 k1 = pn_as_h2(0xE40FE40Fu);                                   // -1039
+    const uint32_t a = pn_and_xor(w, 0x000F000Fu, 0x64086408u), c = pn_and_xor(w, 0x00F000F0u, 0x64806480u);
+    const uint32_t b = pn_and_xor(s, 0x000F000Fu, 0x64086408u), d = pn_and_xor(s, 0x00F000F0u, 0x64806480u);
+    const __half2 two = pn_as_h2(0x40004000u), k1 = pn_as_h2(0xE808E808u);      // 2, -2,064
     const __half2 k8 = pn_as_h2(0x30003000u), k2 = pn_as_h2(0xD878D878u);       // 1 / 8, -143
-    o0 = pn_h2(__hmul2(__hadd2(pn_as_h2(a), k1), f));
-    o1 = pn_h2(__hmul2(__hadd2(pn_as_h2(b), k1), f));
+    o0 = pn_h2(__hfma2(__hfma2(pn_as_h2(a), two, k1), f, f));
+    o1 = pn_h2(__hfma2(__hfma2(pn_as_h2(b), two, k1), f, f));
     o2 = pn_h2(__hmul2(__hfma2(pn_as_h2(c), k8, k2), f));
     o3 = pn_h2(__hmul2(__hfma2(pn_as_h2(d), k8, k2), f));
 }
-// a row's two scales d (1 + 2 s) of sub-blocks 2 Q and 2 Q + 1 (nibbles sn >> 8 Q); d in both halves.  d has 11 bits and 1 + 2 s five: the
-// product rounds once, as from f32
-__device__ __forceinline__ void pn_scales(const PnConst& C, uint32_t sn, int Q, __half2 d, __half2& f0, __half2& f1) {
-    const uint32_t t = sn >> (8 * Q);
-    const uint32_t x = pn_and_or(t * C.k13, 0x001E0000u, pn_and_or(t * C.two, 0x0000001Eu, 0x64016401u));
-    const __half2 f = __hmul2(__hadd2(pn_as_h2(x), pn_as_h2(0xE400E400u)), d);   // (1 + 2 s, exact) d
+// a row's two scales d (1 + 2 s) of sub-blocks 2 Q and 2 Q + 1 (the nibbles of byte Q of sn); d in both halves.  The byte goes into both halves
+// 0x6400 | .., the low one keeps its low nibble (1024 + s), the high one its high nibble (1024 + 16 s); 2 s is exact, and d (1 + 2 s) rounds once, as from f32
+__device__ __forceinline__ void pn_scales(uint32_t sn, int Q, __half2 d, __half2& f0, __half2& f1) {
+    uint32_t t;
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(t) : "r"(sn), "r"(0x64u), "r"(0x4040u + 0x0101u * Q));
+    const __half2 s2 = __hfma2(pn_as_h2(t & 0xFFF0FF0Fu), pn_as_h2(0x30004000u), pn_as_h2(0xD800E800u));   // (2, 1 / 8) x - (2,048, 128)
+    const __half2 f = __hfma2(s2, d, d);
     f0 = __low2half2(f);
     f1 = __high2half2(f);
 }
@@ -146,7 +137,7 @@ __global__ void __launch_bounds__(PN_THREADS, 1) k_prompt_nat(const PnParams p) 
     const uint32_t tmem = sh.tmem;
     const int KB = p.K / 256, nchunk = p.K / PN_KC;
     const int slabs = MODE == 1 ? p.rows / 128 : (p.rows + 255) / 256;
-    const int njobs = MODE != 2 ? *p.njobs : (p.T + PN_N - 1) / PN_N, total = njobs * slabs;
+    const int njobs = MODE != 2 ? *p.njobs : (p.T + p.per - 1) / p.per, total = njobs * slabs;
     auto job_of = [&](int it) {
         const int j = it / slabs;
         PnItem x;
@@ -155,7 +146,7 @@ __global__ void __launch_bounds__(PN_THREADS, 1) k_prompt_nat(const PnParams p) 
             const PnJob jb = p.jobs[j];
             x.w = jb.w; x.n = jb.n; x.start = jb.start;
         } else {
-            x.w = 0; x.start = j * PN_N; x.n = min(PN_N, p.T - x.start);
+            x.w = 0; x.start = j * p.per; x.n = min(p.per, p.T - x.start);
         }
         return x;
     };
@@ -203,7 +194,6 @@ __global__ void __launch_bounds__(PN_THREADS, 1) k_prompt_nat(const PnParams p) 
         };
 #pragma unroll
         for (int i = 0; i < PN_SLOTS; ++i) fetch();
-        const PnConst C;
         int c = 0, slot = 0;   // chunks so far
         for (int it = blockIdx.x; it < total; it += gridDim.x) {
             for (int kb = 0; kb < KB; ++kb) {
@@ -228,12 +218,12 @@ __global__ void __launch_bounds__(PN_THREADS, 1) k_prompt_nat(const PnParams p) 
                         const int Q = PN_KC / 64 * st + q2;
                         uint32_t o[16];
                         __half2 f00, f01, f10, f11;
-                        pn_scales(C, m.x, Q, d0, f00, f01);
-                        pn_scales(C, m.y, Q, d1, f10, f11);
-                        pn_decode8(C, w[0][2 * Q], f00, o[0], o[1], o[4], o[5]);
-                        pn_decode8(C, w[1][2 * Q], f10, o[2], o[3], o[6], o[7]);
-                        pn_decode8(C, w[0][2 * Q + 1], f01, o[8], o[9], o[12], o[13]);
-                        pn_decode8(C, w[1][2 * Q + 1], f11, o[10], o[11], o[14], o[15]);
+                        pn_scales(m.x, Q, d0, f00, f01);
+                        pn_scales(m.y, Q, d1, f10, f11);
+                        pn_decode8(w[0][2 * Q], f00, o[0], o[1], o[4], o[5]);
+                        pn_decode8(w[1][2 * Q], f10, o[2], o[3], o[6], o[7]);
+                        pn_decode8(w[0][2 * Q + 1], f01, o[8], o[9], o[12], o[13]);
+                        pn_decode8(w[1][2 * Q + 1], f11, o[10], o[11], o[14], o[15]);
                         if (q2 == 0) {
                             if (ok && c >= PN_AST) ok = __all_sync(0xffffffffu, pn_wait(&sh.empty[st], (unsigned) ((c / PN_AST - 1) & 1), sh));
                             ta_fence_after();
@@ -254,12 +244,14 @@ __global__ void __launch_bounds__(PN_THREADS, 1) k_prompt_nat(const PnParams p) 
         // is reported before the wait for the next one's stage, so that neither latency lies in the products' way.
         constexpr int RJ = PN_N / (4 * PN_LOAD);
         const int lt = tid - PN_W_LOAD * 32, piece = lt & 7, r0 = lt >> 3;
-        const uint32_t b_s = smem_u32(Bs) + r0 * 128 + ((piece ^ (r0 & 7)) * 16);   // (r0 + 16 j has the same low bits)
-        int c = 0;
-        auto landed = [&](int chunk) {
+        const uint32_t b_s = smem_u32(Bs) + r0 * 128 + ((piece ^ (r0 & 7)) * 16);   // (r0 + 8 j has the same low bits)
+        int c = 0, st = 0, lst = 0;   // chunks so far; the next one's stage, the next reported one's
+        unsigned bpar = 1;            // (a stage's first use finds it free)
+        auto landed = [&]() {
             fence_proxy_async();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&sh.bfull[chunk % PN_BST]);
+            if (lane == 0) mbar_arrive(&sh.bfull[lst]);
+            lst = lst + 1 == PN_BST ? 0 : lst + 1;
         };
         PnItem x = job_of(min((int) blockIdx.x, total - 1)), nx;
         int e[RJ];   // the item's entries
@@ -269,63 +261,77 @@ __global__ void __launch_bounds__(PN_THREADS, 1) k_prompt_nat(const PnParams p) 
         };
         entries(x);
         for (int it = blockIdx.x; it < total; it += gridDim.x) {
-            const __half* src[RJ];
+            uint32_t src[RJ];   // in units of 16 bytes
+            const int live = (x.n - r0 + 4 * PN_LOAD - 1) / (4 * PN_LOAD);   // of the thread's rows
 #pragma unroll
             for (int j = 0; j < RJ; ++j) {
                 int row = e[j];
                 if (MODE == 1) row = row >= p.TKp ? row - p.TKp : row / p.Kp;
-                src[j] = r0 + 4 * PN_LOAD * j < x.n ? p.x + (size_t) row * p.K + piece * 8 : nullptr;
+                src[j] = (uint32_t) row * (uint32_t) (p.K / 8) + piece;
             }
             const bool more = it + (int) gridDim.x < total;
             if (more) nx = job_of(it + gridDim.x);
-            for (int k = 0; k < nchunk; ++k, ++c) {
+            const __half* xk = p.x;
+            for (int k = 0; k < nchunk; ++k, ++c, xk += PN_KC) {
                 if (c >= PN_LAG) {
                     asm volatile("cp.async.wait_group %0;" ::"n"(PN_LAG - 1) : "memory");
-                    landed(c - PN_LAG);
+                    landed();
                 }
-                if (ok && c >= PN_BST) ok = __all_sync(0xffffffffu, pn_wait(&sh.bempty[c % PN_BST], (unsigned) ((c / PN_BST - 1) & 1), sh));
+                if (ok && c >= PN_BST) ok = __all_sync(0xffffffffu, pn_wait(&sh.bempty[st], bpar, sh));
                 if (ok) {
-                    const uint32_t dst = b_s + (c % PN_BST) * PN_BBYTES;
+                    const uint32_t dst = b_s + st * PN_BBYTES;
 #pragma unroll
                     for (int j = 0; j < RJ; ++j)
-                        if (src[j]) {
-                            const __half* g = src[j] + k * PN_KC;
+                        if (j < live) {
+                            const __half* g = xk + (size_t) src[j] * 8;
                             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + j * (512 * PN_LOAD)), "l"(g) : "memory");
-                            if (PN_KC == 128) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + PN_BBOX + j * (512 * PN_LOAD)), "l"(g + 64) : "memory");
+                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + PN_BBOX + j * (512 * PN_LOAD)), "l"(g + 64) : "memory");
                         }
                 }
                 asm volatile("cp.async.commit_group;" ::: "memory");
+                if (++st == PN_BST) {
+                    st = 0;
+                    bpar ^= 1;
+                }
                 if (k == 0 && more) entries(nx);
             }
             x = nx;
         }
         asm volatile("cp.async.wait_group 0;" ::: "memory");
-        for (int i = max(0, c - PN_LAG); i < c; ++i) landed(i);
+        for (int i = max(0, c - PN_LAG); i < c; ++i) landed();
     } else if (warp == PN_W_MMA) {
         // ---------------------------------------------------------------------------------------- the products
-        constexpr uint32_t IDESC = (1u << 4) | ((uint32_t) (PN_N >> 3) << 17) | ((uint32_t) (128 >> 4) << 24);
         const uint32_t b_s = smem_u32(Bs);
         // (one thread all through: among sixteen decoding warps every instruction of this one is paid five or six times)
         if (ta_elect()) {
-            int c = 0, nit = 0;
+            int c = 0, nit = 0, st = 0;
+            unsigned bpar = 0;
+            int n = job_of(min((int) blockIdx.x, total - 1)).n;
             for (int it = blockIdx.x; it < total && ok; it += gridDim.x, ++nit) {
                 const int buf = nit & 1;
                 const uint32_t acc = tmem + buf * PN_ACC;
+                // N: the job's rows, in sixteens
+                const uint32_t idesc = (1u << 4) | ((uint32_t) ((n + 15) >> 4) << 18) | ((uint32_t) (128 >> 4) << 24);
+                if (it + (int) gridDim.x < total) n = job_of(it + gridDim.x).n;   // (used an item later)
                 if (nit >= 2) ok = pn_wait(&sh.acc_empty[buf], (unsigned) ((nit / 2 - 1) & 1), sh);
                 for (int k = 0; k < nchunk && ok; ++k, ++c) {
-                    ok = pn_wait(&sh.bfull[c % PN_BST], (unsigned) ((c / PN_BST) & 1), sh) && pn_wait(&sh.full[c % PN_AST], (unsigned) ((c / PN_AST) & 1), sh);
+                    ok = pn_wait(&sh.bfull[st], bpar, sh) && pn_wait(&sh.full[c % PN_AST], (unsigned) ((c / PN_AST) & 1), sh);
                     if (!ok) break;
                     ta_fence_after();
-                    const uint32_t a_t = tmem + PN_A + (c % PN_AST) * PN_KC, b = b_s + (c % PN_BST) * PN_BBYTES;
+                    const uint32_t a_t = tmem + PN_A + (c % PN_AST) * PN_KC, b = b_s + st * PN_BBYTES;
 #pragma unroll
                     for (int k16 = 0; k16 < PN_KC / 16; ++k16) {
                         const uint64_t bd = ta_desc_sw(b + (k16 >> 2) * PN_BBOX + (k16 & 3) * 32, 16, 1024);
-                        ta_mma_ta(acc, a_t + k16 * 8, bd, IDESC, (k | k16) != 0);
-                        ta_mma_ta(acc + PN_N, a_t + PN_KC / 2 + k16 * 8, bd, IDESC, (k | k16) != 0);
+                        ta_mma_ta(acc, a_t + k16 * 8, bd, idesc, (k | k16) != 0);
+                        ta_mma_ta(acc + PN_N, a_t + PN_KC / 2 + k16 * 8, bd, idesc, (k | k16) != 0);
                     }
                     ta_commit(&sh.empty[c % PN_AST]);
-                    ta_commit(&sh.bempty[c % PN_BST]);
+                    ta_commit(&sh.bempty[st]);
                     if (k == nchunk - 1) ta_commit(&sh.acc_full[buf]);
+                    if (++st == PN_BST) {
+                        st = 0;
+                        bpar ^= 1;
+                    }
                 }
             }
             if (ok && c > 0) {   // the last arrivals, before the shared memory goes
@@ -343,10 +349,11 @@ __global__ void __launch_bounds__(PN_THREADS, 1) k_prompt_nat(const PnParams p) 
         for (int it = blockIdx.x; it < total; it += gridDim.x, ++nit) {
             const PnItem x = job_of(it);
             const int buf = nit & 1;
-            int e0 = x.start + min(lane, x.n - 1), e1 = x.start + min(lane + 32, x.n - 1);   // the item's output rows, two a lane
-            if (MODE != 2) {
-                e0 = p.order[e0];
-                e1 = p.order[e1];
+            int e[PN_N / 32];   // the item's output rows
+#pragma unroll
+            for (int j = 0; j < PN_N / 32; ++j) {
+                e[j] = x.start + min(lane + 32 * j, x.n - 1);
+                if (MODE != 2) e[j] = p.order[e[j]];
             }
             if (ok) ok = __all_sync(0xffffffffu, pn_wait(&sh.acc_full[buf], (unsigned) ((nit / 2) & 1), sh));
             ta_fence_after();
@@ -356,7 +363,10 @@ __global__ void __launch_bounds__(PN_THREADS, 1) k_prompt_nat(const PnParams p) 
                 const bool in0 = f < p.rows, in1 = f + 128 < p.rows;
 #pragma unroll 1
                 for (int c0 = 0; c0 < x.n; c0 += 16) {
-                    const int mine = c0 < 32 ? e0 : e1;
+                    int mine = e[0];
+#pragma unroll
+                    for (int j = 1; j < PN_N / 32; ++j)
+                        if (c0 >= 32 * j) mine = e[j];
                     float g[16], u[16], old0[MODE == 2 ? 16 : 1], old1[MODE == 2 ? 16 : 1];
                     if (MODE == 2) {
 #pragma unroll
@@ -486,7 +496,6 @@ __global__ void __launch_bounds__(PW_THREADS, 1) k_prompt_few(const PnParams p) 
         fetch_tile(i);
         advance();
     }
-    const PnConst C;
     int c = 0, bslot = 0;
     for (int it = blockIdx.x; it < total; it += gridDim.x) {
         const PnJob job = p.jobs[it / parts];
@@ -514,8 +523,8 @@ __global__ void __launch_bounds__(PW_THREADS, 1) k_prompt_few(const PnParams p) 
                         __half2 f[2][2][2];   // [half tile][row half][sub-block]
 #pragma unroll
                         for (int hf = 0; hf < 2; ++hf) {
-                            pn_scales(C, (hf ? m1.x : m0.x) >> (16 * jj), s2, __low2half2(dd[hf]), f[hf][0][0], f[hf][0][1]);
-                            pn_scales(C, (hf ? m1.y : m0.y) >> (16 * jj), s2, __high2half2(dd[hf]), f[hf][1][0], f[hf][1][1]);
+                            pn_scales((hf ? m1.x : m0.x) >> (16 * jj), s2, __low2half2(dd[hf]), f[hf][0][0], f[hf][0][1]);
+                            pn_scales((hf ? m1.y : m0.y) >> (16 * jj), s2, __high2half2(dd[hf]), f[hf][1][0], f[hf][1][1]);
                         }
 #pragma unroll
                         for (int e2 = 0; e2 < 2; ++e2) {
@@ -525,8 +534,8 @@ __global__ void __launch_bounds__(PW_THREADS, 1) k_prompt_few(const PnParams p) 
                                 const uint32_t wa = s2 ? (e2 ? w[hf][0].w : w[hf][0].z) : (e2 ? w[hf][0].y : w[hf][0].x);
                                 const uint32_t wb = s2 ? (e2 ? w[hf][1].w : w[hf][1].z) : (e2 ? w[hf][1].y : w[hf][1].x);
                                 uint32_t a[4], d[4];
-                                pn_decode8(C, wa, f[hf][0][e2], a[0], a[1], a[2], a[3]);
-                                pn_decode8(C, wb, f[hf][1][e2], d[0], d[1], d[2], d[3]);
+                                pn_decode8(wa, f[hf][0][e2], a[0], a[1], a[2], a[3]);
+                                pn_decode8(wb, f[hf][1][e2], d[0], d[1], d[2], d[3]);
                                 pw_mma(acc[hf], a[0], d[0], a[1], d[1], bv.x, bv.y);
                                 pw_mma(acc[hf], a[2], d[2], a[3], d[3], bv.z, bv.w);
                             }
@@ -629,7 +638,7 @@ int prompt_nat_rows(const float* x, const float* norm_w, int T, int H, float eps
 }
 
 int prompt_nat(int mode, const PnParams& p, int max_jobs, cudaStream_t st) {
-    FNX_REQUIRE(p.K % 256 == 0 && p.rows % (mode == 2 ? 16 : mode == 1 ? 128 : 256) == 0, "prompt product: %d features x %d", p.rows, p.K);
+    FNX_REQUIRE(p.K % 256 == 0 && p.rows % (mode == 2 ? 16 : mode == 1 ? 128 : 256) == 0 && p.per >= 1 && p.per <= PN_N, "prompt product: %d features x %d, jobs of %d rows", p.rows, p.K, p.per);
     auto kernel = mode == 1 ? k_prompt_nat<1> : mode == 0 ? k_prompt_nat<0> : k_prompt_nat<2>;
     FNX_TRY(set_smem_limit((const void*) kernel, PN_SMEM));
     const long long items = (long long) max_jobs * (mode == 1 ? p.rows / 128 : (p.rows + 255) / 256);

@@ -16,7 +16,7 @@ __host__ __device__ __forceinline__ int pn_slot(int c) {
     return (c & ~31) + 16 * (j >> 2) + 4 * q + ((k & 1) << 1 | k >> 1);
 }
 
-constexpr int PN_N = 64;       // rows per job: the tensor core's N
+constexpr int PN_N = 64;       // rows per job at most
 
 struct PnJob {
     int w, n, start;           // expert (E: the shared one), rows, first entry of `order`
@@ -30,7 +30,7 @@ struct PnParams {
     const PnJob* jobs;         // (dense: the T rows in order)
     const int* njobs;
     const int* order;          // per entry the pair t Kp + k; shared expert: TKp + t
-    int T, TKp, Kp;
+    int T, TKp, Kp, per;       // per: the jobs' rows at most (dense: exactly, but for the last)
     const __half* x;           // gate|up, dense: [token][K]; down: [pair][K]
     int rows, K;               // features (gate|up: F), inner dimension
     float* out;                // down: [pair][rows]; dense: [token][ldo]
@@ -50,5 +50,12 @@ int prompt_few(int mode, const PnParams& p, int max_jobs, cudaStream_t st);
 // where those win: up to four rows an expert.  A 12-layer prompt of 512 experts, ten a row: 100 rows 4.23 against 4.50 ms in prompt_nat's jobs of 64,
 // 150 rows 4.84 against 4.99, 200 rows 5.42 against 5.43, 333 rows 6.89 against 6.22
 inline bool prompt_few_fits(long long pairs, int E) { return pairs <= 4ll * E; }
+// the rows of a dense product's jobs: fewer, in sixteens, as long as the items of `slabs` x the jobs all run at once (2,048 x 4,096, 332 rows: 30 us with
+// jobs of 64 on 48 SMs, 28 with jobs of 32 on 88; where they would not, 34 us become 52)
+inline int prompt_dense_rows(int T, long long slabs, int sms) {
+    int per = PN_N;
+    while (per > 16 && slabs * ((T + per - 17) / (per - 16)) <= sms) per -= 16;
+    return per;
+}
 
 }  // namespace fnxb

@@ -121,6 +121,12 @@ def test_prompt_products_at_the_edges_of_their_jobs(E, n):
         b.close()
 
 
+@pytest.mark.parametrize("n", [11, 15, 16, 17, 32, 33, 47, 63, 79, 113])
+def test_prompt_products_at_every_sixteen_rows(n):
+    """As above, where the products' N changes (a job's rows in sixteens) and where the dense jobs take fewer rows, for all of them to run at once."""
+    test_prompt_products_at_the_edges_of_their_jobs(2, n)
+
+
 @pytest.mark.parametrize("n", [320, 385, 513, 1100])   # in- and output projection: decoded as they go, or once; tiles of 256 rows full, one over
 def test_prompt_projections_of_both_forms(n):
     """As above, at the benchmark's widths: the keys are a projection of rows that an output projection and experts left (f16 three times)."""
