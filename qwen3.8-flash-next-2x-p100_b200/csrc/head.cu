@@ -2,9 +2,13 @@
 //
 // fnx_argmax replaces argmax / k_argmax (engine/src/kernels.hpp:433, engine/src/kernels.cu:1056-1083): the same
 // total order, value first and the lower index on ties.  fnx_top_tokens replaces top_tokens / k_topk_rows
-// (engine/src/kernels.hpp:445, engine/src/topk.cuh:17-155) without penalties or logit bias: a radix select over the
-// 64-bit key (ordered logit bits, ~index), which has no ties, then a rank sort of the 64 survivors.
+// (engine/src/kernels.hpp:445, engine/src/topk.cuh:17-155) without penalties or logit bias: the 64 largest by the
+// 64-bit key (ordered logit bits, ~index), which has no ties.
+#include <cooperative_groups.h>
+
 #include "fnx_common.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace fnxb {
 
@@ -88,56 +92,122 @@ __global__ void __launch_bounds__(1024) k_argmax(const float* __restrict__ logit
     }
 }
 
-__global__ void __launch_bounds__(1024) k_top_tokens(const float* __restrict__ logits, int V, float* __restrict__ out_v, int* __restrict__ out_i) {
+// The 64 candidates of a row by a cluster of TOP_NB blocks, a slice of the row each.  In its slice a warp's second largest lane maximum bounds the 64th
+// largest value of the block from below as soon as it is the smallest of the 32 warps' (64 values are at or above it), so a second look at the slice
+// leaves a few values more than needed (170 of 19,000 where they are random), which find their places by counting; the first block then merges the
+// slices' sorted 64 by searching the others for each.  A slice with more than TOP_CAP values that high (many equal logits) is selected digit by digit.
+// Bound by two looks at the row and a dozen block barriers: 20 rows of 151,936 logits 162 us with a block a row and nine looks, 18 now.
+constexpr int TOP_NB = 8, TOP_CAP = 1024, TOP_THREADS = 1024;
+constexpr int TOP_LD = 8;   // loads in flight a thread
+
+// keys of the slice [lo, hi) at or above `thr` into sel, at most cap of them; returns how many there are (every thread; ends with a barrier)
+__device__ __forceinline__ unsigned top_collect(const float* __restrict__ l, int lo, int hi, unsigned long long thr, unsigned long long* sel, unsigned cap, unsigned* count, int tid) {
+    if (tid == 0) *count = 0;
+    __syncthreads();
+    for (int i0 = lo + tid; i0 < hi; i0 += TOP_THREADS * TOP_LD) {
+        float v[TOP_LD];
+#pragma unroll
+        for (int j = 0; j < TOP_LD; ++j) v[j] = i0 + j * TOP_THREADS < hi ? l[i0 + j * TOP_THREADS] : 0.f;
+#pragma unroll
+        for (int j = 0; j < TOP_LD; ++j) {
+            const int i = i0 + j * TOP_THREADS;
+            const unsigned long long k = key64(v[j], i);
+            if (i < hi && k >= thr) {
+                const unsigned at = atomicAdd(count, 1u);
+                if (at < cap) sel[at] = k;
+            }
+        }
+    }
+    __syncthreads();
+    return *count;
+}
+
+__global__ void __cluster_dims__(TOP_NB, 1, 1) __launch_bounds__(TOP_THREADS) k_top_tokens(const float* __restrict__ logits, int V, float* __restrict__ out_v, int* __restrict__ out_i) {
     pdl_wait();
     pdl_launch_dependents();
-    __shared__ unsigned hist[256];
-    __shared__ unsigned long long prefix_s, sel[FNX_TOPK_N];
-    __shared__ unsigned need_s, nsel;
-    const int t = blockIdx.x, tid = threadIdx.x;
+    __shared__ unsigned long long sel[TOP_CAP], top[FNX_TOPK_N], every[TOP_NB][FNX_TOPK_N];
+    __shared__ unsigned low[TOP_THREADS / 32], hist[256], count, need_s;
+    __shared__ unsigned long long prefix_s;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int t = blockIdx.y, part = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const float* l = logits + (size_t) t * V;
-    if (tid == 0) { prefix_s = 0; need_s = FNX_TOPK_N; nsel = 0; }
+    const int lo = (int) ((long long) V * part / TOP_NB), hi = (int) ((long long) V * (part + 1) / TOP_NB);
+    unsigned mx = 0;
+    for (int i0 = lo + tid; i0 < hi; i0 += TOP_THREADS * TOP_LD) {
+        float v[TOP_LD];
+#pragma unroll
+        for (int j = 0; j < TOP_LD; ++j) v[j] = i0 + j * TOP_THREADS < hi ? l[i0 + j * TOP_THREADS] : l[i0];
+#pragma unroll
+        for (int j = 0; j < TOP_LD; ++j) mx = max(mx, fkey(v[j]));
+    }
+    const unsigned first = __reduce_max_sync(0xffffffffu, mx);
+    const int who = __ffs(__ballot_sync(0xffffffffu, mx == first)) - 1;
+    const unsigned second = __reduce_max_sync(0xffffffffu, lane == who ? 0u : mx);
+    if (lane == 0) low[warp] = second;
     __syncthreads();
-    // 8 passes of 8 bits from the top: after pass p the first 8 (p + 1) bits of the 64th largest key are known
-    for (int pass = 0; pass < 8; ++pass) {
-        const int shift = 56 - 8 * pass;
-        if (tid < 256) hist[tid] = 0;
-        __syncthreads();
-        const unsigned long long prefix = prefix_s;
-        const unsigned long long mask = pass == 0 ? 0ull : ~0ull << (shift + 8);
-        for (int i = tid; i < V; i += 1024) {
-            const unsigned long long k = key64(l[i], i);
-            if ((k & mask) == prefix) atomicAdd(&hist[(unsigned) (k >> shift) & 255u], 1u);
-        }
-        __syncthreads();
+    const unsigned bound = __reduce_min_sync(0xffffffffu, low[lane]);
+    unsigned n = top_collect(l, lo, hi, (unsigned long long) bound << 32, sel, TOP_CAP, &count, tid);
+    if (n > TOP_CAP) {
+        // 8 passes of 8 bits from the top: after pass p the first 8 (p + 1) bits of the slice's 64th largest key are known
         if (tid == 0) {
-            unsigned need = need_s, b = 255;
-            for (;; --b) {
-                if (hist[b] >= need) break;
-                need -= hist[b];
-                if (b == 0) break;
+            prefix_s = 0;
+            need_s = FNX_TOPK_N;
+        }
+        for (int pass = 0; pass < 8; ++pass) {
+            const int shift = 56 - 8 * pass;
+            if (tid < 256) hist[tid] = 0;
+            __syncthreads();
+            const unsigned long long prefix = prefix_s, mask = pass == 0 ? 0ull : ~0ull << (shift + 8);
+            for (int i = lo + tid; i < hi; i += TOP_THREADS) {
+                const unsigned long long k = key64(l[i], i);
+                if ((k & mask) == prefix) atomicAdd(&hist[(unsigned) (k >> shift) & 255u], 1u);
             }
-            need_s = need;
-            prefix_s = prefix | ((unsigned long long) b << shift);
+            __syncthreads();
+            if (tid == 0) {
+                unsigned need = need_s, b = 255;
+                for (;; --b) {
+                    if (hist[b] >= need) break;
+                    need -= hist[b];
+                    if (b == 0) break;
+                }
+                need_s = need;
+                prefix_s = prefix | ((unsigned long long) b << shift);
+            }
+            __syncthreads();
         }
-        __syncthreads();
+        n = top_collect(l, lo, hi, prefix_s, sel, TOP_CAP, &count, tid);   // (keys are distinct: 64)
+        if (n > TOP_CAP) n = TOP_CAP;
     }
-    const unsigned long long thr = prefix_s;   // the 64th largest key (keys are distinct)
-    for (int i = tid; i < V; i += 1024) {
-        const unsigned long long k = key64(l[i], i);
-        if (k >= thr) {
-            const unsigned at = atomicAdd(&nsel, 1u);
-            if (at < FNX_TOPK_N) sel[at] = k;
-        }
-    }
+    // the slice's 64 largest in order; fewer where the slice holds fewer (0: no key)
+    if (tid < FNX_TOPK_N) top[tid] = 0;
     __syncthreads();
-    const unsigned n = min(nsel, (unsigned) FNX_TOPK_N);
     if (tid < (int) n) {
         const unsigned long long k = sel[tid];
         unsigned rank = 0;
         for (unsigned j = 0; j < n; ++j) rank += sel[j] > k;
-        out_v[t * FNX_TOPK_N + rank] = fkey_inv((uint32_t) (k >> 32));
-        out_i[t * FNX_TOPK_N + rank] = (int) ~(uint32_t) k;
+        if (rank < FNX_TOPK_N) top[rank] = k;
+    }
+    cluster.sync();
+    if (part == 0 && tid < TOP_NB * FNX_TOPK_N) every[tid / FNX_TOPK_N][tid % FNX_TOPK_N] = cluster.map_shared_rank(top, tid / FNX_TOPK_N)[tid % FNX_TOPK_N];
+    cluster.sync();   // (no block leaves while its keys are read)
+    if (part == 0 && tid < TOP_NB * FNX_TOPK_N) {
+        const int own = tid / FNX_TOPK_N;
+        const unsigned long long k = every[own][tid % FNX_TOPK_N];
+        unsigned rank = tid % FNX_TOPK_N, at[TOP_NB];   // the larger ones: before it in its own list, and in the others
+#pragma unroll
+        for (int p = 0; p < TOP_NB; ++p) at[p] = 0;
+#pragma unroll
+        for (int step = FNX_TOPK_N / 2; step; step >>= 1)
+#pragma unroll
+            for (int p = 0; p < TOP_NB; ++p)
+                if (every[p][at[p] + step - 1] > k) at[p] += step;
+#pragma unroll
+        for (int p = 0; p < TOP_NB; ++p)
+            if (p != own) rank += at[p] + (every[p][at[p]] > k ? 1u : 0u);
+        if (k && rank < FNX_TOPK_N) {
+            out_v[t * FNX_TOPK_N + rank] = fkey_inv((uint32_t) (k >> 32));
+            out_i[t * FNX_TOPK_N + rank] = (int) ~(uint32_t) k;
+        }
     }
 }
 
@@ -186,7 +256,7 @@ extern "C" int fnx_argmax(const float* logits, int T, int V, int* best_i, float*
 extern "C" int fnx_top_tokens(const float* logits, int T, int V, float* out_v, int* out_i, fnx_stream st) {
     FNX_REQUIRE(logits && out_v && out_i && T >= 1 && V >= FNX_TOPK_N, "fnx_top_tokens: bad arguments (vocabulary of at least %d)", FNX_TOPK_N);
     {
-        const cudaError_t le_ = launch_dep(true, k_top_tokens, dim3(T), dim3(1024), 0, as_stream(st), logits, V, out_v, out_i);
+        const cudaError_t le_ = launch_dep(true, k_top_tokens, dim3(TOP_NB, T), dim3(TOP_THREADS), 0, as_stream(st), logits, V, out_v, out_i);
         if (le_ != cudaSuccess) return fail(FNX_E_CUDA, "k_top_tokens: launch failed: %s", cudaGetErrorString(le_));
     }
     FNX_LAUNCH_OK("fnx_top_tokens");

@@ -79,20 +79,39 @@ __global__ void k_accept_greedy_lanes(const int* __restrict__ tok, const int* __
     accept_greedy_walk(tok + row0, nullptr, best + row0, lane_row0[lane + 1] - row0, result + (size_t) lane * (1 + 2 * FNX_MAX_ROWS));
 }
 
-struct DistS {
-    int n;
+struct alignas(16) DistS {
+    int n, pad[3];
     int ids[FNX_TOPK_N];
     double p[FNX_TOPK_N];
 };
 
-__device__ __forceinline__ double dist_prob(const int* ids, const double* p, int n, int id) {
-    for (int i = 0; i < n; ++i)
-        if (ids[i] == id) return p[i];
-    return 0.0;
+// probability of id in a distribution of n <= 64 candidates, by a warp (every lane gets it): the first that has the id
+__device__ __forceinline__ double dist_prob(const int* ids, const double* p, int n, int id, int lane) {
+    const unsigned a = __ballot_sync(0xffffffffu, lane < n && ids[lane] == id), b = __ballot_sync(0xffffffffu, lane + 32 < n && ids[lane + 32] == id);
+    return a ? p[__ffs(a) - 1] : b ? p[31 + __ffs(b)] : 0.0;
 }
 
-// A warp per row builds the row's distribution (make_dist): the exponentials in parallel, the sums in the
-// reference's sequential order; then thread 0 walks the chain.
+// p[0] + p[1] + .. in that order, from shared memory (p on a 16-byte boundary): eight values' loads ahead of the chain of additions
+__device__ __forceinline__ double sum_in_order(const double* p, int n) {
+    double sum = 0.0;
+    int i = 0;
+    for (; i + 8 <= n; i += 8) {
+        double2 v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] = *reinterpret_cast<const double2*>(p + i + 2 * j);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            sum += v[j].x;
+            sum += v[j].y;
+        }
+    }
+    for (; i < n; ++i) sum += p[i];
+    return sum;
+}
+
+// A warp per row builds the row's distribution (make_dist): the exponentials and divisions in parallel, the sums in the
+// reference's sequential order; then the first warp walks the chain, its lanes searching the candidates.  (With the divisions and the searches
+// one after another by one thread, 23 us for four chains of five rows; 8 now.)
 __device__ __forceinline__ void accept_sample_body(const float* __restrict__ cand_v, const int* __restrict__ cand_i, const int* __restrict__ tok, int T,
                                                    fnx_sampling sp, const int* __restrict__ q_ids, const double* __restrict__ q_p,
                                                    const int* __restrict__ q_n, uint64_t seed, uint32_t seq, uint32_t step, int* __restrict__ result,
@@ -106,43 +125,39 @@ __device__ __forceinline__ void accept_sample_body(const float* __restrict__ can
         double* e = ex + (size_t) t * FNX_TOPK_N;
         const int n = FNX_TOPK_N;
         const int k = (sp.top_k <= 0 || sp.top_k > n) ? n : sp.top_k;
-        const double mx = cv[0];
-        for (int i = lane; i < n; i += 32) e[i] = exp((double) cv[i] - mx);
-        __syncwarp();
-        if (lane == 0) {
-            int keep = k;
-            if (sp.top_p < 1.f) {
-                double sum = 0.0;
-                for (int i = 0; i < k; ++i) sum += e[i];
+        int keep = k;
+        if (sp.top_p < 1.f) {
+            const double mx = cv[0];
+            for (int i = lane; i < n; i += 32) e[i] = exp((double) cv[i] - mx);
+            __syncwarp();
+            if (lane == 0) {
+                const double sum = sum_in_order(e, k);
                 double cum = 0.0;
                 for (int i = 0; i < k; ++i) {
                     cum += e[i] / sum;
                     if (cum >= (double) sp.top_p) { keep = i + 1; break; }
                 }
             }
-            if (sp.min_p > 0.f) {
-                const float thresh = cv[0] + logf(sp.min_p);
-                for (int i = 1; i < keep; ++i)
-                    if (cv[i] < thresh) { keep = i; break; }
-            }
-            dist[t].n = keep;
+            keep = __shfl_sync(0xffffffffu, keep, 0);
         }
-        __syncwarp();
-        const int keep = dist[t].n;
+        if (sp.min_p > 0.f) {   // up to the first (after the largest) below the threshold
+            const float thresh = cv[0] + logf(sp.min_p);
+            const unsigned a = __ballot_sync(0xffffffffu, lane >= 1 && lane < keep && cv[lane] < thresh), b = __ballot_sync(0xffffffffu, lane + 32 < keep && cv[lane + 32] < thresh);
+            if (a || b) keep = a ? __ffs(a) - 1 : 31 + __ffs(b);
+        }
+        if (lane == 0) dist[t].n = keep;
         const double inv_t = 1.0 / sp.temperature, smx = cv[0] * inv_t;
         for (int i = lane; i < keep; i += 32) {
             dist[t].ids[i] = ci[i];
             dist[t].p[i] = exp(cv[i] * inv_t - smx);
         }
         __syncwarp();
-        if (lane == 0) {
-            double sum = 0.0;
-            for (int i = 0; i < keep; ++i) sum += dist[t].p[i];
-            for (int i = 0; i < keep; ++i) dist[t].p[i] /= sum;
-        }
+        const double sum = sum_in_order(dist[t].p, keep);
+        __syncwarp();
+        for (int i = lane; i < keep; i += 32) dist[t].p[i] /= sum;
     }
     __syncthreads();
-    if (threadIdx.x != 0) return;
+    if (warp != 0) return;
     uint32_t slot = 0;
     int n;
     double* p = ex;   // row scratch for the residual
@@ -156,21 +171,32 @@ __device__ __forceinline__ void accept_sample_body(const float* __restrict__ can
             const double* qp = q_p ? q_p + (size_t) n * FNX_TOPK_N : nullptr;
             const bool fixed = qn == 0;
             const double u = philox_uniform(seed, seq, step, slot++);
-            if (u * (fixed ? 1.0 : dist_prob(qi, qp, qn, dr)) < dist_prob(d.ids, d.p, d.n, dr)) {
-                result[1 + n] = n;
-                result[1 + FNX_MAX_ROWS + n] = dr;
+            if (u * (fixed ? 1.0 : dist_prob(qi, qp, qn, dr, lane)) < dist_prob(d.ids, d.p, d.n, dr, lane)) {
+                if (lane == 0) {
+                    result[1 + n] = n;
+                    result[1 + FNX_MAX_ROWS + n] = dr;
+                }
                 continue;
             }
-            double rest = 0.0;
-            for (int i = 0; i < d.n; ++i) {
-                const double qv = fixed ? (d.ids[i] == dr ? 1.0 : 0.0) : dist_prob(qi, qp, qn, d.ids[i]);
+            for (int i = lane; i < d.n; i += 32) {
+                double qv = 0.0;
+                if (fixed) qv = d.ids[i] == dr ? 1.0 : 0.0;
+                else
+                    for (int j = 0; j < qn; ++j)
+                        if (qi[j] == d.ids[i]) {
+                            qv = qp[j];
+                            break;
+                        }
                 p[i] = d.p[i] - qv > 0.0 ? d.p[i] - qv : 0.0;
-                rest += p[i];
             }
+            __syncwarp();
+            const double rest = sum_in_order(p, d.n);
+            __syncwarp();
             if (rest > 1e-12) {
-                for (int i = 0; i < d.n; ++i) p[i] /= rest;
+                for (int i = lane; i < d.n; i += 32) p[i] /= rest;
                 pp = p;
             }
+            __syncwarp();
         }
         const double u = philox_uniform(seed, seq, step, slot++);
         double cum = 0.0;
@@ -179,12 +205,14 @@ __device__ __forceinline__ void accept_sample_body(const float* __restrict__ can
             cum += pp[i];
             if (u < cum) { pick = d.ids[i]; break; }
         }
-        result[1 + n] = n;
-        result[1 + FNX_MAX_ROWS + n] = pick;
+        if (lane == 0) {
+            result[1 + n] = n;
+            result[1 + FNX_MAX_ROWS + n] = pick;
+        }
         ++n;
         break;
     }
-    result[0] = n;
+    if (lane == 0) result[0] = n;
 }
 
 __global__ void __launch_bounds__(1024) k_accept_sample(const float* __restrict__ cand_v, const int* __restrict__ cand_i,

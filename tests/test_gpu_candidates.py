@@ -1,0 +1,50 @@
+"""The sampler's 64 candidates at the edges of their selection: eight slices of a row, a warp's second largest, more equal values than a slice keeps."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("V", [64, 65, 511, 513, 8191, 8200, 9000, 40003, 151936, 300007])
+def test_top_tokens_are_the_largest_keys(F, V):
+    rng = np.random.default_rng(V)
+    rows = [rng.standard_normal(V), np.zeros(V), np.round(rng.standard_normal(V) * 2), np.arange(V), -np.arange(V), rng.standard_normal(V)]
+    logits = np.stack(rows).astype(np.float32)
+    logits[5, V // 2:] = -np.inf                         # (a mask; infinities are values like others)
+    logits[5, : V // 3] = 3.0                            # more equal ones than a slice keeps, where the row is long
+    logits[0, V - 1] = np.inf
+    logits[2, :3] = [0.0, -0.0, 0.0]                     # (of two zeros the positive one is the larger)
+    bits = logits.view(np.uint32).astype(np.uint64)
+    key = np.where(bits >> 31, ~bits & 0xFFFFFFFF, bits | 0x80000000) << np.uint64(32) | (0xFFFFFFFF - np.arange(V, dtype=np.uint64))
+    want = np.argsort(key, axis=1)[:, ::-1][:, :64]      # value first, the lower index among equals
+    v, i = F.top_tokens(torch.from_numpy(logits).cuda())
+    assert np.array_equal(i.cpu().numpy(), want)
+    assert np.array_equal(v.cpu().numpy().view(np.uint32), np.take_along_axis(logits, want, 1).view(np.uint32))
+    # a row that does not start on a 16-byte boundary
+    flat = torch.from_numpy(np.concatenate([np.zeros(1, np.float32), logits[0]])).cuda()
+    _, one = F.top_tokens(flat[1:].view(1, V))
+    assert np.array_equal(one.cpu().numpy()[0], want[0])
+
+
+def test_accept_sample_with_draft_distributions(F, O):
+    """Drafts of their own distributions (up to 64 candidates, in any order) beside fixed ones: counts and tokens as the oracle's."""
+    rng = np.random.default_rng(12)
+    cuda = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    for it in range(80):
+        T, V = int(rng.integers(1, 9)), 2000
+        cv, ci = O.top_tokens((rng.standard_normal((T, V)) * 3).astype(np.float32))
+        tok = rng.integers(0, V, size=T).astype(np.int32)
+        qi, qp, qn = np.zeros((T, 64), np.int32), np.zeros((T, 64)), np.zeros(T, np.int32)
+        for t in range(T):
+            if rng.random() < 0.7:
+                m = int(rng.integers(1, 65))
+                p = rng.random(m)
+                qn[t], qi[t, :m], qp[t, :m] = m, ci[t, rng.permutation(64)[:m]], p / p.sum()
+            if t + 1 < T and rng.random() < 0.8:
+                tok[t + 1] = ci[t, int(rng.integers(0, 4))]
+        s = [O.Sampling(0.7, 1.0, 0.0, 0), O.Sampling(1.0, 0.9, 0.05, 40), O.Sampling(0.3, 1.0, 0.2, 0), O.Sampling(2.0, 0.5, 0.0, 7)][it % 4]
+        n, em = O.accept_sample(cv, ci, tok, s, seed=9, seq=it, step=3, q_ids=qi, q_p=qp, q_n=qn)
+        gn, _, gem = F.accept_sample(cuda(cv), cuda(ci), cuda(tok), F.Sampling(s.temperature, s.top_p, s.min_p, s.top_k), 9, it, cuda(np.array([3], np.int32)), cuda(qi),
+                                     cuda(qp), cuda(qn))
+        assert gn == n and gem == list(em), it
