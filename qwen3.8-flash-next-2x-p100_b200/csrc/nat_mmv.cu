@@ -6,7 +6,7 @@
 //   - the rows come as their image (nat_image.cuh): a dense or gate|up block copies the rows it needs into shared memory and quantises
 //     nothing (read through L1 from global memory instead, the operands cost more than the weights); down quantises its few rows itself;
 //   - every lane copies its own 64 bytes of the next tiles into shared memory (cp.async): no mbarriers, no issuing lane;
-//   - the eight-warp forms take half an SM's registers, and most of them half its shared memory, so that the next kernel of the window can be
+//   - the eight-warp forms of up to two row groups take half an SM's registers, and most of them half its shared memory, so that the next kernel of the window can be
 //     resident while this one drains (programmatic dependent launch): its first tiles are on their way before the rows it waits for are
 //     written.  The sixteen-warp forms, for products that stream some 10 us and more, have an SM to themselves.
 // Bound by HBM for the large expert products, by the launch and its dependent loads for the small dense ones.
@@ -141,39 +141,41 @@ __device__ __forceinline__ void nm_flush(uint32_t am, float s0, float s1, const 
         acc[3] += d1 * s1 * (float) accI[3];
     }
 }
-template <int H, int NG, typename AccT>
-__device__ __forceinline__ void nm_half_item(uint32_t a16, uint32_t am, uint32_t xb, uint32_t x0, uint32_t x1, uint32_t group, AccT (&acc)[NG][4]) {
-    int accI[NG][4];
-#pragma unroll
-    for (int ng = 0; ng < NG; ++ng)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) accI[ng][i] = 0;
-    const NmScales sc = nm_scales<H>(am);
-#pragma unroll 1
-    for (int hf = 0; hf < 2; ++hf) {
-        NmHalf w;
-        nm_decode<H>(a16, sc, hf, w);
-#pragma unroll
-        for (int ng = 0; ng < NG; ++ng) nm_products(w, lds_v4(xb + ng * group + hf * 128), lds_v4<64>(xb + ng * group + hf * 128), accI[ng]);
-    }
-#pragma unroll
-    for (int ng = 0; ng < NG; ++ng) nm_flush<H>(am, lds_f32(x0 + ng * group), lds_f32(x1 + ng * group), accI[ng], acc[ng]);
-}
-
 // One item: the tile at shared address tile_s against one block of the rows; adds into acc[half][ng][0..3] = (row g, column 2 q),
 // (g, 2 q + 1), (g + 8, 2 q), (g + 8, 2 q + 1).  xb: shared address of the lane's cells in its column's row of group 0, x0 / x1: of its
 // two C columns' scales; groups lie `group` bytes apart.  The integers are exact (8 times the sums of iq3s_mmv.cu's items).
 // AccT double (expert modes): the rounded result does not depend on where a row's K-sum was cut, as there.
-// Up to two row groups load the rows' operands once for both half tiles; more would not leave the registers.  (Most jobs have one
+// The rows' operands are loaded once for both half tiles.  (Most jobs have one
 // row, two of the eight columns; a form with half of the integer work for them was slower: 52 against 46 us for 205 jobs, the second
-// copy of the code.)  Their loop over four
-// sub-blocks stays rolled (unrolled, every load would be hoisted into registers), the short one is worth unrolling: 50 -> 47 us for 205 jobs.
+// copy of the code.)  The loop over four sub-blocks stays rolled for three row groups and more (their blocks have an SM to themselves, their rows' image
+// leaves no room for a second one, so a thread has 255 registers: a half tile at a time in 128, with spills, 8 warps waited most of the time: a head of 151,936
+// rows over 20 rows 100 us, 62 now; 12,352 x 2,048 16 and 10.7); the short one is worth unrolling: 50 -> 47 us for 205 jobs.
 template <int NG, typename AccT>
 __device__ __forceinline__ void nm_item(uint32_t tile_s, uint32_t xb, uint32_t x0, uint32_t x1, uint32_t group, int lane, AccT (&acc)[2][NG][4]) {
     const uint32_t a16 = tile_s + lane * 16, am = tile_s + (lane >> 2) * 16;
     if constexpr (NG > 2) {
-        nm_half_item<0, NG>(a16, am, xb, x0, x1, group, acc[0]);
-        nm_half_item<1, NG>(a16, am, xb, x0, x1, group, acc[1]);
+        int accI[2][NG][4];
+#pragma unroll
+        for (int i = 0; i < 2 * NG * 4; ++i) accI[i / (4 * NG)][(i / 4) % NG][i & 3] = 0;
+        const NmScales sc0 = nm_scales<0>(am), sc1 = nm_scales<1>(am);
+#pragma unroll 1
+        for (int hf = 0; hf < 2; ++hf) {
+            NmHalf w0, w1;
+            nm_decode<0>(a16, sc0, hf, w0);
+            nm_decode<1>(a16, sc1, hf, w1);
+#pragma unroll
+            for (int ng = 0; ng < NG; ++ng) {
+                const uint4 b0 = lds_v4(xb + ng * group + hf * 128), b1 = lds_v4<64>(xb + ng * group + hf * 128);
+                nm_products(w0, b0, b1, accI[0][ng]);
+                nm_products(w1, b0, b1, accI[1][ng]);
+            }
+        }
+#pragma unroll
+        for (int ng = 0; ng < NG; ++ng) {
+            const float s0 = lds_f32(x0 + ng * group), s1 = lds_f32(x1 + ng * group);
+            nm_flush<0>(am, s0, s1, accI[0][ng], acc[0][ng]);
+            nm_flush<1>(am, s0, s1, accI[1][ng], acc[1][ng]);
+        }
     } else {
         int accI[2][NG][4];
 #pragma unroll
@@ -526,13 +528,13 @@ __device__ __forceinline__ void nm_body(const NatParams& p, uint8_t* smem) {
 
 // two blocks an SM: the next kernel's may be resident while this one's drain
 template <int NG, int MODE, int NW, int SLOTS>
-__global__ void __launch_bounds__(NW * 32, NW > 12 ? 1 : 2) k_nat_mmv(const NatParams p) {
+__global__ void __launch_bounds__(NW * 32, NW > 12 || NG > 2 ? 1 : 2) k_nat_mmv(const NatParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
     nm_body<NG, MODE, NW, SLOTS, 1>(p, smem);
 }
 constexpr int NM_SPLIT = 4;
 template <int NG, int NW, int SLOTS>
-__global__ void __cluster_dims__(NM_SPLIT, 1, 1) __launch_bounds__(NW * 32, NW > 12 ? 1 : 2) k_nat_mmv_split(const NatParams p) {
+__global__ void __cluster_dims__(NM_SPLIT, 1, 1) __launch_bounds__(NW * 32, NW > 12 || NG > 2 ? 1 : 2) k_nat_mmv_split(const NatParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
     nm_body<NG, MAT_DENSE, NW, SLOTS, NM_SPLIT>(p, smem);
 }
