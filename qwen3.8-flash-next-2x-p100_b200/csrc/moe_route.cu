@@ -318,31 +318,36 @@ static int router_logits(const float* Wr, const float* x, const float* norm_w, f
     return le == cudaSuccess ? FNX_OK : fail(FNX_E_CUDA, "k_router_logits: launch failed: %s", cudaGetErrorString(le));
 }
 
-// One block: the top K of every row (a warp per row), their weights, and the job list, built in shared memory and copied out.
-constexpr int RT_PICK = 1024;   // a warp per row
-__global__ void __launch_bounds__(RT_PICK) k_router_pick(const float* __restrict__ logits, int T, int E, int K, int e_lo, int e_hi, int add_shared, int* __restrict__ topi,
-                                                         float* __restrict__ topw, fnx_job* __restrict__ jobs, int* __restrict__ njobs,
-                                                         unsigned long long* __restrict__ stats) {
+// One block: the top K of every row (a warp per row), their weights, and the job list, built in shared memory and copied out.  Bound by latency (the
+// launch, the logits' way, the ranks, four barriers): eight warps where they are enough, whose barriers cost less, what does not depend on the logits
+// before they are waited for (one row and five: 5.5 us a launch with 32 warps that cleared the list behind the picks, 4.3 now.  A list without scans
+// over the block, each entry placed by the bits of a map below its expert's: 3.9 and 4.3, 0.4% of a pass of one row).
+template <int NTH>
+__global__ void __launch_bounds__(NTH) k_router_pick(const float* __restrict__ logits, int T, int E, int K, int e_lo, int e_hi, int add_shared, int* __restrict__ topi,
+                                                     float* __restrict__ topw, fnx_job* __restrict__ jobs, int* __restrict__ njobs,
+                                                     unsigned long long* __restrict__ stats) {
     extern __shared__ __align__(16) uint8_t pick_smem[];   // the job list
     __shared__ int s_topi[FNX_MAX_ROWS * 32];
     __shared__ unsigned s_rows[RT_MAXE];
     __shared__ int s_base[RT_MAXE], wsum_[32], total_[2];
-    __shared__ __align__(16) unsigned scr_[RT_PICK / 32][64];
+    __shared__ __align__(16) unsigned scr_[NTH / 32][64];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     RtJobSmem js;
     js.s_topi = s_topi; js.s_rows = s_rows; js.s_base = s_base; js.wsum = wsum_; js.total = total_;
     js.js = reinterpret_cast<fnx_job*>(pick_smem);
+    rt_clear_jobs<NTH>(js, tid, T, K);
+    __syncthreads();
     pdl_wait();
     pdl_launch_dependents();
-    for (int t = warp; t < T; t += RT_PICK / 32) {
+    for (int t = warp; t < T; t += NTH / 32) {
         const float* l = logits + (size_t) t * (E + 1);
         int* ti = topi + t * K;
         float* tw = topw + t * K;
         if (E <= 512) rt_topk_row<16>(l, E, K, lane, scr_[warp], ti, s_topi + t * K, tw, nullptr);
         else rt_topk_row<RT_MAXE / 32>(l, E, K, lane, scr_[warp], ti, s_topi + t * K, tw, nullptr);
+        rt_note_picks(js, t, K, e_lo, e_hi, lane);
     }
-    rt_build_jobs<RT_PICK>(js, tid, T, E, K, e_lo, e_hi, add_shared);
-    __syncthreads();
+    rt_build_jobs<NTH>(js, tid, T, E, K, e_lo, e_hi, add_shared);
     const int total = total_[0];
     if (tid == 0) {
         njobs[0] = total;
@@ -352,15 +357,17 @@ __global__ void __launch_bounds__(RT_PICK) k_router_pick(const float* __restrict
         }
     }
     constexpr int JW = sizeof(fnx_job) / 4;
-    for (int w = tid; w < total * JW; w += RT_PICK) reinterpret_cast<int*>(jobs)[w] = reinterpret_cast<const int*>(js.js)[w];
+    for (int w = tid; w < total * JW; w += NTH) reinterpret_cast<int*>(jobs)[w] = reinterpret_cast<const int*>(js.js)[w];
 }
 
 int router_window(const float* Wr, const float* x, const float* norm_w, float eps, int T, int E, int H, int K, int e_lo, int e_hi, int add_shared, float* logits, int* topi,
                   float* topw, fnx_job* jobs, int* njobs, unsigned long long* stats, unsigned* err, uint8_t* img, bool early, cudaStream_t st) {
     FNX_TRY(router_logits(Wr, x, norm_w, eps, T, E, H, logits, err, img, early, st));
     const size_t smem = ((size_t) T * K + (T + FNX_JOB_TOK - 1) / FNX_JOB_TOK) * sizeof(fnx_job);
-    if (int rc = set_smem_limit((const void*) k_router_pick, 64 * 1024)) return rc;
-    const cudaError_t le = launch_dep(true, k_router_pick, dim3(1), dim3(RT_PICK), smem, st, (const float*) logits, T, E, K, e_lo, e_hi, add_shared, topi, topw, jobs, njobs, stats);
+    const int threads = T <= 8 ? 256 : 1024;   // a warp per row
+    auto kernel = T <= 8 ? k_router_pick<256> : k_router_pick<1024>;
+    if (int rc = set_smem_limit((const void*) kernel, 64 * 1024)) return rc;
+    const cudaError_t le = launch_dep(true, kernel, dim3(1), dim3(threads), smem, st, (const float*) logits, T, E, K, e_lo, e_hi, add_shared, topi, topw, jobs, njobs, stats);
     return le == cudaSuccess ? FNX_OK : fail(FNX_E_CUDA, "k_router_pick: launch failed: %s", cudaGetErrorString(le));
 }
 

@@ -126,25 +126,29 @@ struct RtJobSmem {
 // block): jobs in ascending expert order, expert e's rows in row order, 4 per job; then (add_shared) the shared expert's.
 // A row picks an expert at most once, so the rows of an expert are a bit mask: its population is their number, and the bits below a
 // row's are that row's place among them.
+// rt_clear_jobs comes first (nothing of it depends on the picks); then, behind a barrier, each row's warp leaves its picks (rt_note_picks); rt_build_jobs does the rest.
 // Thread `tid` owns experts [tid * EPT, (tid + 1) * EPT) below RT_MAXE: a block-wide exclusive scan of their job counts gives each
-// expert's first job; then one thread per (row, pick) entry places itself.  Returns the number of jobs in total[0] and
-// the routed ones in total[1] (valid after the call in every thread).
+// expert's first job; then one thread per (row, pick) entry places itself.  The number of jobs in total[0], the routed ones in
+// total[1] (valid after the call in every thread).
+template <int NTH>
+__device__ __forceinline__ void rt_clear_jobs(const RtJobSmem& s, int tid, int T, int K) {
+    for (int e = tid; e < RT_MAXE; e += NTH) s.s_rows[e] = 0u;
+    // unused row slots of the jobs stay zero
+    const int cap = (T * K + (T + FNX_JOB_TOK - 1) / FNX_JOB_TOK) * (int) (sizeof(fnx_job) / 4);
+    for (int w = tid; w < cap; w += NTH) reinterpret_cast<int*>(s.js)[w] = 0;
+}
+// row t's warp, its picks in s_topi
+__device__ __forceinline__ void rt_note_picks(const RtJobSmem& s, int t, int K, int e_lo, int e_hi, int lane) {
+    __syncwarp();
+    if (lane < K) {
+        const int e = s.s_topi[t * K + lane];
+        if (e >= e_lo && e < e_hi) atomicOr(&s.s_rows[e], 1u << t);
+    }
+}
 template <int NTH>
 __device__ __forceinline__ void rt_build_jobs(const RtJobSmem& s, int tid, int T, int E, int K, int e_lo, int e_hi, int add_shared) {
     constexpr int EPT = (RT_MAXE + NTH - 1) / NTH;
     const int warp = tid >> 5, lane = tid & 31;
-    for (int e = tid; e < RT_MAXE; e += NTH) s.s_rows[e] = 0u;
-    {   // unused row slots of the jobs stay zero
-        const int cap = (T * K + (T + FNX_JOB_TOK - 1) / FNX_JOB_TOK) * (int) (sizeof(fnx_job) / 4);
-        for (int w = tid; w < cap; w += NTH) reinterpret_cast<int*>(s.js)[w] = 0;
-    }
-    __syncthreads();
-    // the rows that picked each expert of this rank
-    for (int t = warp; t < T; t += NTH / 32)
-        if (lane < K) {
-            const int e = s.s_topi[t * K + lane];
-            if (e >= e_lo && e < e_hi) atomicOr(&s.s_rows[e], 1u << t);
-        }
     __syncthreads();
     int cnt_[EPT], mine = 0;
 #pragma unroll
@@ -165,7 +169,7 @@ __device__ __forceinline__ void rt_build_jobs(const RtJobSmem& s, int tid, int T
     for (int w = 0; w < warp; ++w) base_ += s.wsum[w];
 #pragma unroll
     for (int j = 0; j < EPT; ++j) {
-        if (tid * EPT + j < RT_MAXE) s.s_base[tid * EPT + j] = base_;
+        if (cnt_[j]) s.s_base[tid * EPT + j] = base_;
         base_ += cnt_[j];
     }
     if (tid == NTH - 1) {
