@@ -480,7 +480,7 @@ int router_rows(const float* Wr, const float* x, const float* norm_w, float eps,
                 unsigned* err, bool early, cudaStream_t st);
 int router_window(const float* Wr, const float* x, const float* norm_w, float eps, int T, int E, int H, int K, int e_lo, int e_hi, int add_shared, float* logits, int* topi,
                   float* topw, fnx_job* jobs, int* njobs, unsigned long long* stats, unsigned* err, uint8_t* img, bool early, cudaStream_t st);
-int moe_combine_nat(const float* part, const int* topi, const float* topw, const float* logits, int T, int E, int H, int K, float* R, uint8_t* img, const float* img_norm_w,
+int moe_combine_nat(const float* part, const float* topw, const float* logits, int T, int E, int H, int K, float* R, uint8_t* img, const float* img_norm_w,
                     cudaStream_t st);
 
 struct Dims {
@@ -772,7 +772,7 @@ static int enqueue_moe(fnx_engine* e, const LayerW& L, float* R, int T, const Ma
         FNX_TRY(fnx_moe_down(L.wdn.tiles, L.wdn.tile_stride(), e->e_lo, L.wsh_dn.tiles, d.E, e->jobs, e->njobs, njobs_max, e->hbuf, d.H, d.F, e->part, e->err, e->st));
     if (!ep && img) {
         if (img_ready) *img_ready = true;
-        return moe_combine_nat(e->part, e->topi, e->topw, e->rlogits, T, d.E, d.H, d.K, R, e->img_r, next_norm, e->st);
+        return moe_combine_nat(e->part, e->topw, e->rlogits, T, d.E, d.H, d.K, R, e->img_r, next_norm, e->st);
     }
     if (!ep) return fnx_moe_combine(e->part, e->topi, e->topw, e->rlogits, T, d.E, d.H, d.K, 0, d.E, 1, R, 1, e->st);
     if (e->ep_peers && e->ep_one_kernel && d.H % 256 == 0) {

@@ -491,57 +491,79 @@ __global__ void __launch_bounds__(32) k_combine_image(const float* __restrict__ 
         }
 }
 
-// k_combine for an engine's window: the new rows' image (nat_image.cuh) for the next projection rides along.  One warp per (256-column
-// block, row); the addends' loads are in flight together, sixteen picks at a time.
-__global__ void __launch_bounds__(32) k_combine_nat(const float* __restrict__ part, const int* __restrict__ topi, const float* __restrict__ topw,
-                                                    const float* __restrict__ logits, int T, int E, int H, int K, float* __restrict__ out, uint8_t* __restrict__ img,
-                                                    const float* __restrict__ img_norm_w) {
-    const int blk = blockIdx.x, t = blockIdx.y, lane = threadIdx.x, KB = H / 256;
+// k_combine for an engine's window: the new rows' image (nat_image.cuh) for the next projection rides along.  One block per (256-column
+// block, row): four warps share out the addends (integers: their order does not show), eight columns a lane, and the first one finishes.  Bound by latency: the
+// launch, one way to memory, 24 conversions to 64-bit integers a lane (a warp alone had 88 of them, and the norm weights' way on top: 4.4 us a launch for one row and for five, 2.8 and 2.4 now).
+constexpr int CN_WARPS = 4, CN_LD = 3;   // addends in flight a warp
+__global__ void __launch_bounds__(CN_WARPS * 32) k_combine_nat(const float* __restrict__ part, const float* __restrict__ topw, const float* __restrict__ logits, int T, int E, int H,
+                                                               int K, float* __restrict__ out, uint8_t* __restrict__ img, const float* __restrict__ img_norm_w) {
+    __shared__ unsigned long long sums[CN_WARPS - 1][8][32];
+    const int blk = blockIdx.x, t = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, KB = H / 256;
     const size_t col = (size_t) blk * 256 + lane * 8;
-    // ahead of the wait: the rows (last written by the output projection), the router's results (by the kernels before the two expert products)
+    // ahead of the wait: the rows (last written by the output projection), the router's results (by the kernels before the two expert products), weights
     float* dst = out + (size_t) t * H + col;
-    const float4 o0 = *reinterpret_cast<const float4*>(dst), o1 = *reinterpret_cast<const float4*>(dst + 4);
-    const float shl = logits[(size_t) t * (E + 1) + E], mw = lane < K ? topw[t * K + lane] : 0.f;
+    float v[8], nw[8];
+    if (warp == 0) {
+        const float4 o0 = *reinterpret_cast<const float4*>(dst), o1 = *reinterpret_cast<const float4*>(dst + 4);
+        const float4 w0 = *reinterpret_cast<const float4*>(img_norm_w + col), w1 = *reinterpret_cast<const float4*>(img_norm_w + col + 4);
+        v[0] = o0.x; v[1] = o0.y; v[2] = o0.z; v[3] = o0.w; v[4] = o1.x; v[5] = o1.y; v[6] = o1.z; v[7] = o1.w;
+        nw[0] = w0.x; nw[1] = w0.y; nw[2] = w0.z; nw[3] = w0.w; nw[4] = w1.x; nw[5] = w1.y; nw[6] = w1.z; nw[7] = w1.w;
+    }
+    const float mw = lane < K ? topw[t * K + lane] : 0.f, g = sigmoidf_(logits[(size_t) t * (E + 1) + E]);
     pdl_wait();
     pdl_launch_dependents();
-    const float4* sh = reinterpret_cast<const float4*>(part + ((size_t) T * K + t) * H + col);
-    const float4 h0 = sh[0], h1 = sh[1];
     unsigned long long s[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) s[i] = 0ull;
-    for (int k0 = 0; k0 < K; k0 += 16) {
-        float4 a[16][2];
+    for (int k0 = warp; k0 <= K; k0 += CN_LD * CN_WARPS) {   // (addend K: the shared expert's)
+        float4 a[CN_LD][2];
 #pragma unroll
-        for (int k = 0; k < 16; ++k)
-            if (k0 + k < K) {
-                const float4* src = reinterpret_cast<const float4*>(part + ((size_t) t * K + k0 + k) * H + col);
-                a[k][0] = src[0];
-                a[k][1] = src[1];
+        for (int j = 0; j < CN_LD; ++j) {
+            const int k = k0 + j * CN_WARPS;
+            if (k <= K) {
+                const float4* src = reinterpret_cast<const float4*>(part + (k < K ? (size_t) t * K + k : (size_t) T * K + t) * H + col);
+                a[j][0] = src[0];
+                a[j][1] = src[1];
             }
+        }
 #pragma unroll
-        for (int k = 0; k < 16; ++k)
-            if (k0 + k < K) {
-                const float wk = __shfl_sync(0xffffffffu, mw, k0 + k);
-                const float e8[8] = {a[k][0].x, a[k][0].y, a[k][0].z, a[k][0].w, a[k][1].x, a[k][1].y, a[k][1].z, a[k][1].w};
+        for (int j = 0; j < CN_LD; ++j) {
+            const int k = k0 + j * CN_WARPS;
+            if (k <= K) {
+                const float pick = __shfl_sync(0xffffffffu, mw, k & 31), wk = k < K ? pick : g;
+                const float e8[8] = {a[j][0].x, a[j][0].y, a[j][0].z, a[j][0].w, a[j][1].x, a[j][1].y, a[j][1].z, a[j][1].w};
 #pragma unroll
                 for (int i = 0; i < 8; ++i) s[i] += fix_from_float(wk * e8[i]);
             }
+        }
     }
-    const float g = sigmoidf_(shl);
-    const float e8[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
-    float v[8] = {o0.x, o0.y, o0.z, o0.w, o1.x, o1.y, o1.z, o1.w};
+    if (warp) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] += fix_to_float(s[i] + fix_from_float(g * e8[i]));
+        for (int i = 0; i < 8; ++i) sums[warp - 1][i][lane] = s[i];
+    }
+    __syncthreads();
+    if (warp) return;
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+#pragma unroll
+        for (int w = 0; w < CN_WARPS - 1; ++w) s[i] += sums[w][i][lane];
+        v[i] += fix_to_float(s[i]);
+    }
     *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
     *reinterpret_cast<float4*>(dst + 4) = make_float4(v[4], v[5], v[6], v[7]);
-    const float ss = ni_norm8(v, img_norm_w + col);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        ss = fmaf(v[i], v[i], ss);
+        v[i] *= nw[i];
+    }
     ni_quant(img, KB, v, ss, t, blk, lane);
 }
 
-int moe_combine_nat(const float* part, const int* topi, const float* topw, const float* logits, int T, int E, int H, int K, float* R, uint8_t* img, const float* img_norm_w,
+int moe_combine_nat(const float* part, const float* topw, const float* logits, int T, int E, int H, int K, float* R, uint8_t* img, const float* img_norm_w,
                     cudaStream_t st) {
     FNX_REQUIRE(T >= 1 && T <= FNX_MAX_ROWS && K >= 1 && K <= 32 && H % 256 == 0, "moe_combine_nat: %d rows of %d, top %d", T, H, K);
-    const cudaError_t le = launch_dep(true, k_combine_nat, dim3(H / 256, T), dim3(32), 0, st, part, topi, topw, logits, T, E, H, K, R, img, img_norm_w);
+    const cudaError_t le = launch_dep(true, k_combine_nat, dim3(H / 256, T), dim3(CN_WARPS * 32), 0, st, part, topw, logits, T, E, H, K, R, img, img_norm_w);
     return le == cudaSuccess ? FNX_OK : fail(FNX_E_CUDA, "k_combine_nat: launch failed: %s", cudaGetErrorString(le));
 }
 
