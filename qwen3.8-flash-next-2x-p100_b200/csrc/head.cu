@@ -20,19 +20,25 @@ __device__ __forceinline__ uint32_t fkey(float v) {
 __device__ __forceinline__ float fkey_inv(uint32_t k) { return __uint_as_float(k & 0x80000000u ? k & 0x7fffffffu : ~k); }
 __device__ __forceinline__ unsigned long long key64(float v, int i) { return ((unsigned long long) fkey(v) << 32) | (uint32_t) ~i; }
 
-// Rows are scanned by ARGMAX_NB blocks each; the blocks of a row meet in a per-row slot of device memory (largest key by
-// atomicMax, an arrival counter) and the last one to arrive writes the result and clears the slot for the next call.
-// The slots are shared by every call on the device: calls must not overlap in time (the engine's are stream-ordered).
-constexpr int ARGMAX_NB = 16, ARGMAX_ROWS = 1024;
-__device__ unsigned long long g_argmax_key[ARGMAX_ROWS];
-__device__ unsigned g_argmax_cnt[ARGMAX_ROWS];
+// the largest key of a warp's 32 (every lane gets it)
+__device__ __forceinline__ unsigned long long warp_max_key(unsigned long long k) {
+    const unsigned hi = (unsigned) (k >> 32), top = __reduce_max_sync(0xffffffffu, hi);
+    return ((unsigned long long) top << 32) | __reduce_max_sync(0xffffffffu, hi == top ? (unsigned) k : 0u);
+}
 
-__global__ void __launch_bounds__(1024) k_argmax(const float* __restrict__ logits, int V, const int* __restrict__ map, int* __restrict__ best_i,
-                                                 float* __restrict__ best_v, unsigned* __restrict__ err) {
+// A row by a cluster of ARGMAX_NB blocks, a slice each, which leave their largest keys in the first one's shared memory.  Bound by latency: the launch, the
+// slice's way, one barrier of the cluster.  (Sixteen blocks that met in device memory, an atomic maximum and an arrival counter: 6.2 us a launch for a row of
+// 151,936, one block for 40,528 6.3; 4.4 and 3.0 now.)
+constexpr int ARGMAX_NB = 8;
+
+__global__ void __cluster_dims__(1, ARGMAX_NB, 1) __launch_bounds__(1024) k_argmax(const float* __restrict__ logits, int V, const int* __restrict__ map, int* __restrict__ best_i,
+                                                                                  float* __restrict__ best_v, unsigned* __restrict__ err) {
+    __shared__ unsigned long long red[32], every[ARGMAX_NB];
+    cg::cluster_group cluster = cg::this_cluster();
+    cluster.sync();   // (the first block's shared memory is there)
     pdl_wait();
     pdl_launch_dependents();
-    __shared__ unsigned long long red[32];
-    const int t = blockIdx.x, tid = threadIdx.x, nb = gridDim.y;
+    const int t = blockIdx.x, tid = threadIdx.x, nb = ARGMAX_NB;
     const float* l = logits + (size_t) t * V;
     unsigned long long best = 0;
     bool bad = false;
@@ -56,35 +62,24 @@ __global__ void __launch_bounds__(1024) k_argmax(const float* __restrict__ logit
             }
         }
     }
-    if (blockIdx.y == nb - 1)   // what float4 units do not cover
-        for (int i = 4 * V4 + tid; i < V; i += 1024) {
-            const float v = l[i];
-            bad |= !isfinite(v);
-            const unsigned long long k = key64(v, i);
-            best = k > best ? k : best;
-        }
-    for (int o = 16; o; o >>= 1) {
-        const unsigned long long ok = __shfl_xor_sync(0xffffffffu, best, o);
-        best = ok > best ? ok : best;
+    for (int i = 4 * V4 + (int) blockIdx.y * 1024 + tid; i < V; i += nb * 1024) {   // what float4 units do not cover
+        const float v = l[i];
+        bad |= !isfinite(v);
+        const unsigned long long k = key64(v, i);
+        best = k > best ? k : best;
     }
+    best = warp_max_key(best);
     if ((tid & 31) == 0) red[tid >> 5] = best;
     if (bad) atomicOr(err, (unsigned) FNX_ERR_LOGITS);
     __syncthreads();
     if (tid < 32) {
-        best = red[tid];
-        for (int o = 16; o; o >>= 1) {
-            const unsigned long long ok = __shfl_xor_sync(0xffffffffu, best, o);
-            best = ok > best ? ok : best;
-        }
+        best = warp_max_key(red[tid]);
+        if (tid == 0) *cluster.map_shared_rank(every + blockIdx.y, 0) = best;
+    }
+    cluster.sync();
+    if (blockIdx.y == 0 && tid < 32) {
+        best = warp_max_key(tid < nb ? every[tid] : 0ull);
         if (tid == 0) {
-            if (nb > 1) {
-                atomicMax(&g_argmax_key[t], best);
-                __threadfence();
-                if (atomicAdd(&g_argmax_cnt[t], 1u) != (unsigned) nb - 1) return;
-                __threadfence();
-                best = atomicExch(&g_argmax_key[t], 0ull);
-                g_argmax_cnt[t] = 0;
-            }
             const int row = (int) ~(uint32_t) best;
             best_i[t] = map ? map[row] : row;
             if (best_v) best_v[t] = fkey_inv((uint32_t) (best >> 32));
@@ -242,7 +237,7 @@ using namespace fnxb;
 extern "C" int fnx_argmax_mapped(const float* logits, int T, int V, const int* map, int* best_i, float* best_v, unsigned* err, fnx_stream st) {
     FNX_REQUIRE(logits && best_i && err && T >= 1 && V >= 1, "fnx_argmax: bad arguments");
     {
-        const cudaError_t le_ = launch_dep(true, k_argmax, dim3(T, T <= ARGMAX_ROWS && V >= 65536 ? ARGMAX_NB : 1), dim3(1024), 0, as_stream(st), logits, V, map, best_i, best_v, err);
+        const cudaError_t le_ = launch_dep(true, k_argmax, dim3(T, ARGMAX_NB), dim3(1024), 0, as_stream(st), logits, V, map, best_i, best_v, err);
         if (le_ != cudaSuccess) return fail(FNX_E_CUDA, "k_argmax: launch failed: %s", cudaGetErrorString(le_));
     }
     FNX_LAUNCH_OK("fnx_argmax");

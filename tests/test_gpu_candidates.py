@@ -48,3 +48,14 @@ def test_accept_sample_with_draft_distributions(F, O):
         gn, _, gem = F.accept_sample(cuda(cv), cuda(ci), cuda(tok), F.Sampling(s.temperature, s.top_p, s.min_p, s.top_k), 9, it, cuda(np.array([3], np.int32)), cuda(qi),
                                      cuda(qp), cuda(qn))
         assert gn == n and gem == list(em), it
+
+
+@pytest.mark.parametrize("T,V", [(1, 1), (3, 5), (2, 31), (5, 1023), (1, 40528), (3, 40525), (32, 32771), (20, 151936), (1100, 64)])
+def test_argmax_over_a_cluster(F, T, V):
+    """Eight slices of a row, aligned to 16 bytes or not: the first of the largest values, and a row with a value that is not finite is reported."""
+    rng = np.random.default_rng(V)
+    logits = np.round(rng.standard_normal((T, V)) * 3).astype(np.float32) + 0.0    # (many ties; no negative zeros, which are below the positive one)
+    i, v, err = F.argmax(torch.from_numpy(logits).cuda())
+    assert np.array_equal(i.cpu().numpy(), logits.argmax(1)) and np.array_equal(v.cpu().numpy(), logits.max(1)) and int(err.item()) == 0
+    logits[T - 1, V - 1] = -np.inf
+    assert int(F.argmax(torch.from_numpy(logits).cuda())[2].item()) == 16
