@@ -618,9 +618,10 @@ int nat_dense(const uint8_t* W, int rows, int K, const uint8_t* img, bool normed
     return FNX_OK;
 }
 
-// From this many jobs on the expert products stream long enough (some 15 us) that sixteen warps, which hide more of an item's latency,
-// are worth more than a second resident block: 205 jobs 50 -> 45 us (gate|up) and 28 -> 24 us (down); 52 jobs are level.
-constexpr int NM_MANY_JOBS = 80;
+// From this many jobs on sixteen warps, which hide more of an item's latency, are worth more than a second resident block: 205 jobs 50 -> 45 us (gate|up)
+// and 28 -> 24 us (down).  A window of twelve layers, ten picks a row, eight and sixteen warps, us: two rows (21 jobs) 601 and 611, three (31) 657 and 654, four 700
+// and 694, five 787 and 772, six 837 and 813.
+constexpr int NM_MANY_JOBS = 30;
 // (the job list, 40 bytes a job, has to fit beside sixteen warps' tiles and four rows: 896 jobs at 2,048 columns; the bits are the same either way)
 template <int MODE>
 static int launch_nat_jobs(const NatParams& p, cudaStream_t st) {
