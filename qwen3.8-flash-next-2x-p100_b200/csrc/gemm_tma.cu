@@ -5,8 +5,8 @@
 // truncation, ~2^-24 of the running sum a step, so the logits come out to a few 1e-5).  The counterpart of the reference's
 // library GEMMs for prompts (cublasGemmEx, engine/src/prefill.cu:543-549, 626-629, 678-689; cublasSgemm for the router, :653).
 //
-// One block = NA x 128 features (tensor-memory lanes, NA accumulators) x 256 rows (columns); K in stages of 64 columns:
-// boxes of 64 x 128 (weights) and 64 x 256 (rows) with the 128-byte swizzle, which is the layout the products' shared-memory
+// One block = NA x 128 features (tensor-memory lanes, NA accumulators) x up to 256 rows (columns: gt_rows); K in stages of 64 columns:
+// boxes of 64 x 128 (weights) and 64 x that many (rows) with the 128-byte swizzle, which is the layout the products' shared-memory
 // descriptors name.  Warp 0: the loader thread; warp 1: the thread that issues the products; warps 2-5: the epilogue, a
 // feature per thread, 32 rows at a time, so that a warp's stores cover 32 consecutive features of one row.  Tensor copies
 // fill rows and features past the matrices' ends with zeros.  Every wait is bounded.
@@ -20,7 +20,7 @@
 namespace fnxb {
 
 constexpr int GT_M = 128;          // features per accumulator
-constexpr int GT_N = 256;          // rows per block
+constexpr int GT_N = 256;          // rows per block, at most
 constexpr int GT_KC = 64;          // K per stage: one 128-byte swizzle row
 constexpr int GT_THREADS = 192;
 constexpr int GT_A_BYTES = GT_M * GT_KC * 2;   // 16 KB: a box of weights
@@ -38,6 +38,7 @@ struct GtShape {
 struct GtParams {
     float* y;
     int ldy, T, rows, K, accumulate;
+    int tn;          // rows per block (a multiple of 16)
     float scale;
     unsigned* err;
 };
@@ -78,7 +79,7 @@ __device__ __forceinline__ void gt_ld32(uint32_t taddr, float (&v)[32]) {
     for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-// grid (feature tiles of NA x 128, row tiles of 256): the feature tiles of one row tile run together, so the rows' boxes are
+// grid (feature tiles of NA x 128, row tiles of p.tn): the feature tiles of one row tile run together, so the rows' boxes are
 // shared through L2 and the weights stay there from one row tile to the next.
 // map_w / map_x: the operands (NPROD = 3: their high parts), map_wl / map_xl: the low parts.
 template <int NA, int NPROD>
@@ -94,7 +95,7 @@ __global__ void __launch_bounds__(GT_THREADS, 1) k_gemm_tma(const GtParams p, co
     uint64_t* done = empty + STAGES;                                           // every product has finished
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int f0 = blockIdx.x * NA * GT_M, t0 = blockIdx.y * GT_N, nk = p.K / GT_KC;
+    const int f0 = blockIdx.x * NA * GT_M, t0 = blockIdx.y * p.tn, nk = p.K / GT_KC, t1 = min(p.T, t0 + p.tn);
     if (tid == 0) {
         for (int s = 0; s < STAGES; ++s) {
             mbar_init(&full[s], 1);
@@ -121,7 +122,7 @@ __global__ void __launch_bounds__(GT_THREADS, 1) k_gemm_tma(const GtParams p, co
                 atomicOr(p.err, (unsigned) FNX_ERR_TIMEOUT);
                 break;
             }
-            mbar_expect_tx(&full[s], (unsigned) Sh::STAGE);
+            mbar_expect_tx(&full[s], (unsigned) (PARTS * (NA * GT_A_BYTES + p.tn * GT_KC * 2)));
 #pragma unroll
             for (int part = 0; part < PARTS; ++part) {
 #pragma unroll
@@ -130,8 +131,8 @@ __global__ void __launch_bounds__(GT_THREADS, 1) k_gemm_tma(const GtParams p, co
             }
         }
     } else if (tid == 32) {
-        // f32 accumulate, f16 x f16, both operands K-major, N = 256, M = 128
-        constexpr uint32_t IDESC = (1u << 4) | ((uint32_t) (GT_N >> 3) << 17) | ((uint32_t) (GT_M >> 4) << 24);
+        // f32 accumulate, f16 x f16, both operands K-major, N = tn, M = 128
+        const uint32_t IDESC = (1u << 4) | ((uint32_t) (p.tn >> 3) << 17) | ((uint32_t) (GT_M >> 4) << 24);
         bool ok = true;
         for (int kb = 0; kb < nk && ok; ++kb) {
             const int s = kb % STAGES;
@@ -167,12 +168,12 @@ __global__ void __launch_bounds__(GT_THREADS, 1) k_gemm_tma(const GtParams p, co
                 const int f = f0 + a * GT_M + 32 * lg + lane;
 #pragma unroll 1
                 for (int c = 0; c < GT_N / 32; ++c) {
-                    if (t0 + c * 32 >= p.T) break;
+                    if (t0 + c * 32 >= t1) break;
                     float v[32];
                     gt_ld32(tmem + ((uint32_t) (32 * lg) << 16) + (uint32_t) (a * GT_N + c * 32), v);
                     if (f < p.rows) {
                         float* o = p.y + (size_t) (t0 + c * 32) * p.ldy + f;
-                        const int nt = min(32, p.T - (t0 + c * 32));
+                        const int nt = min(32, t1 - (t0 + c * 32));
                         float old[32];
                         if (p.accumulate) {   // every load first: the stores below would otherwise order them one by one
 #pragma unroll
@@ -350,28 +351,41 @@ static int gt_map(CUtensorMap* map, const __half* base, int rows, int K, int box
     return FNX_OK;
 }
 
+// Rows per block where the tiles of 256 rows leave SMs idle: what the last wave's blocks do without is worth more than the weights' boxes that smaller
+// tiles read again (32 rows' worth a block).  Twelve tiles of 256 rows, 3,001 rows in all: 2,048 x 4,096, 62 us on 96 SMs with 256 rows, 49 on 144 with 176; the
+// router's 512 experts 36 on 48, 22 on 128 with 96.  A row's sums do not depend on its tile.
+static int gt_rows(int T, int slabs) {
+    const long long sms = sm_count();
+    auto cost = [&](int n) { return (((long long) slabs * ((T + n - 1) / n) + sms - 1) / sms) * (n + 32); };
+    int best = GT_N;
+    for (int n = GT_N - 16; n >= 64; n -= 16)
+        if (cost(n) < cost(best)) best = n;
+    return 100 * cost(best) < 92 * cost(GT_N) ? best : GT_N;
+}
+
 // y[t][f] (+)= scale * W[f] . x[t] over T rows and `rows` features; wl / xl: the operands' low parts (null: one product)
 int gemm_tma_launch(const __half* w, const __half* wl, const __half* x, const __half* xl, float* y, int ldy, int T, int rows, int K, int accumulate, float scale,
                     unsigned* err, cudaStream_t st) {
     FNX_REQUIRE(w && x && y && err && T >= 1 && rows >= 1 && K >= GT_KC && K % GT_KC == 0, "gemm_tma: %d rows x %d features x %d", T, rows, K);
     FNX_REQUIRE((((uintptr_t) w | (uintptr_t) x | (uintptr_t) wl | (uintptr_t) xl) & 15) == 0, "gemm_tma: operands must be 16-byte aligned");
     FNX_REQUIRE((wl == nullptr) == (xl == nullptr), "gemm_tma: low parts of both operands or of neither");
-    GtParams p{y, ldy, T, rows, K, accumulate, scale, err};
+    const int slabs = (rows + (wl ? 1 : 2) * GT_M - 1) / ((wl ? 1 : 2) * GT_M), tn = gt_rows(T, slabs);
+    GtParams p{y, ldy, T, rows, K, accumulate, tn, scale, err};
     CUtensorMap mw, mx, mwl, mxl;
     FNX_TRY(gt_map(&mw, w, rows, K, GT_M));
-    FNX_TRY(gt_map(&mx, x, T, K, GT_N));
+    FNX_TRY(gt_map(&mx, x, T, K, tn));
     if (wl) {
         FNX_TRY(gt_map(&mwl, wl, rows, K, GT_M));
-        FNX_TRY(gt_map(&mxl, xl, T, K, GT_N));
+        FNX_TRY(gt_map(&mxl, xl, T, K, tn));
         using Sh = GtShape<1, 3>;
         if (int rc = set_smem_limit((const void*) k_gemm_tma<1, 3>, Sh::SMEM)) return rc;
-        FNX_CUDA_OK(launch_after(k_gemm_tma<1, 3>, dim3((rows + GT_M - 1) / GT_M, (T + GT_N - 1) / GT_N), dim3(GT_THREADS), Sh::SMEM, st, p, mw, mx, mwl, mxl));
+        FNX_CUDA_OK(launch_after(k_gemm_tma<1, 3>, dim3(slabs, (T + tn - 1) / tn), dim3(GT_THREADS), Sh::SMEM, st, p, mw, mx, mwl, mxl));
     } else {
         mwl = mw;
         mxl = mx;
         using Sh = GtShape<2, 1>;
         if (int rc = set_smem_limit((const void*) k_gemm_tma<2, 1>, Sh::SMEM)) return rc;
-        FNX_CUDA_OK(launch_after(k_gemm_tma<2, 1>, dim3((rows + 2 * GT_M - 1) / (2 * GT_M), (T + GT_N - 1) / GT_N), dim3(GT_THREADS), Sh::SMEM, st, p, mw, mx, mwl, mxl));
+        FNX_CUDA_OK(launch_after(k_gemm_tma<2, 1>, dim3(slabs, (T + tn - 1) / tn), dim3(GT_THREADS), Sh::SMEM, st, p, mw, mx, mwl, mxl));
     }
     FNX_LAUNCH_OK("k_gemm_tma");
     return FNX_OK;
