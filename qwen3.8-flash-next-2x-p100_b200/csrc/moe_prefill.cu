@@ -546,8 +546,9 @@ __global__ void k_pf_xnorm(const float* __restrict__ x, const float* __restrict_
 }
 
 // out[t] (+)= sum_k topw[t][k] part[t Kp + k] + sigmoid(logit[t][E]) part[T Kp + t]
-// A thread owns four columns of one row.  EVERY: all experts are this rank's, so no addend is left out: its load waits for nothing (asked for
-// only where the pick's weight had been seen not to be zero, the same loads took 98 us for 3,001 rows of eleven addends, 56 now; 38,912 rows 1,065 and 605).
+// A thread owns four columns of one row.  EVERY: all experts are this rank's, so hardly an addend is left out (a pick that names no expert, one of weight 0) and
+// its load waits for nothing (asked for only where the pick's weight had been seen not to be zero, the same loads took 98 us for 3,001 rows of eleven addends, 56
+// now; 38,912 rows 1,065 and 605).
 // Bound by the addends' way from DRAM (5.8 TB/s of them, 6.8 with the rows read and written); four blocks an SM, to whose 64 registers the loads just fit
 // (three: 68 and 682 us).
 constexpr int PC_ADD = 11;   // addends in flight a thread (top 10 and the shared expert: all of them)
@@ -569,11 +570,8 @@ __global__ void __launch_bounds__(256, 4) k_pf_combine(const float* __restrict__
             const int a = min(k0 + k, n - 1);
             if (a == Kp) w[k] = sigmoidf_(logits[(size_t) t * (E + 1) + E]);
             else {
-                w[k] = topw[(size_t) t * Kp + a];
-                if (!EVERY) {
-                    const int e = topi[(size_t) t * Kp + a];
-                    if (e < e_lo || e >= e_hi) w[k] = 0.f;
-                }
+                const int e = topi[(size_t) t * Kp + a];   // (outside the range nobody wrote the addend)
+                w[k] = e >= e_lo && e < e_hi ? topw[(size_t) t * Kp + a] : 0.f;
             }
             if (k0 + k >= n) w[k] = 0.f;
         }

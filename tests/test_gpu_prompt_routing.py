@@ -70,3 +70,24 @@ def test_combine_of_many_picks(F, K, add_shared):
     part = run(topw, add_shared=add_shared, e_lo=0, e_hi=E // 2)
     rest = run(topw, add_shared=False, e_lo=E // 2, e_hi=E, out=part.clone(), accumulate=True)
     assert ((rest.double() - want).abs() <= 2 * bound).all()
+
+
+@pytest.mark.parametrize("K,T", [(1, 3), (10, 40), (11, 19), (24, 21), (10, 830)])   # (one block's job list, one pass of addends and more; several blocks' list)
+@pytest.mark.parametrize("half", [False, True])
+def test_a_pick_that_names_no_expert_adds_nothing(F, K, T, half):
+    """Ids of -1 and E (a masked row, a masked pick) with weights that are not 0: no job has them, so nobody writes their addends, and the
+    sum is that of the other picks, bit for bit, whatever the scratch held."""
+    E, H, Fn = 32, 512, 256
+    fx = _moe_fixture(F, E, H, Fn, seed=31)
+    g = torch.Generator(device="cuda").manual_seed(K)
+    x, logits, topw = torch.randn((T, H), device="cuda", generator=g), torch.randn((T, E + 1), device="cuda", generator=g), torch.rand((T, K), device="cuda", generator=g) + 0.1
+    topi = torch.stack([torch.randperm(E, generator=torch.Generator().manual_seed(t))[:K] for t in range(T)]).int().cuda()
+    out_of_range = torch.rand((T, K), device="cuda", generator=g) < 0.3
+    out_of_range[0] = True
+    ids = torch.where(out_of_range, torch.where(topi % 2 == 0, -1, E).int(), topi)
+    nbytes = F.lib().fnx_moe_prefill_scratch_bytes(T, K, E, H, Fn)
+    run = lambda i, w, **kw: F.moe_prefill(fx["gu_t"], fx["dn_t"], fx["sh_gu_t"], fx["sh_dn_t"], i, w, logits, x, Fn, e_hi=E // 2 if half else E,
+                                           scratch=torch.full((nbytes,), 255, dtype=torch.uint8, device="cuda"), **kw)[0]   # (floats of 0xFFFFFFFF: NaN)
+    for shared in (True, False):
+        got, want = run(ids, topw, add_shared=shared), run(topi, torch.where(out_of_range, 0.0, topw), add_shared=shared)
+        assert torch.isfinite(want).all() and torch.equal(got, want), shared
