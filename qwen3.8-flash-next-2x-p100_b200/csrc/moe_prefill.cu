@@ -550,42 +550,40 @@ __global__ void k_pf_xnorm(const float* __restrict__ x, const float* __restrict_
 // its load waits for nothing (asked for only where the pick's weight had been seen not to be zero, the same loads took 98 us for 3,001 rows of eleven addends, 56
 // now; 38,912 rows 1,065 and 605).
 // Bound by the addends' way from DRAM (5.8 TB/s of them, 6.8 with the rows read and written); four blocks an SM, to whose 64 registers the loads just fit
-// (three: 68 and 682 us).
+// (three: 68 and 682 us).  A warp's lanes fetch the weights, one each, and no load goes past the last addend (a block of 32 experts of width 256, 3,001 rows in all:
+// one pick a row 181 us with every thread fetching all weights and the last addend loaded again for each place left, 169 now; two 193 and 184, ten 362 and 362, 22
+// 676 and 662).
 constexpr int PC_ADD = 11;   // addends in flight a thread (top 10 and the shared expert: all of them)
 template <bool EVERY>
 __global__ void __launch_bounds__(256, 4) k_pf_combine(const float* __restrict__ part, const int* __restrict__ topi, const float* __restrict__ topw,
                                                     const float* __restrict__ logits, int T, int E, int H, int Kp, int e_lo, int e_hi, int add_shared,
                                                     float* __restrict__ out, int accumulate) {
+    __shared__ float weights[8][32];   // the picks', a copy a warp
     pdl_begin();
-    const int t = blockIdx.y, i = (blockIdx.x * blockDim.x + threadIdx.x) * 4, n = Kp + (add_shared ? 1 : 0);
-    if (i >= H) return;
+    const int t = blockIdx.y, i = (blockIdx.x * blockDim.x + threadIdx.x) * 4, n = Kp + (add_shared ? 1 : 0), lane = threadIdx.x & 31;
+    if (i >= H) return;   // (whole warps: H is a multiple of 256)
+    float* mine = weights[threadIdx.x >> 5];
+    mine[lane] = pick_weight(topi + (size_t) t * Kp, topw + (size_t) t * Kp, Kp, e_lo, e_hi, lane);
+    __syncwarp();
+    const float gate = add_shared ? sigmoidf_(logits[(size_t) t * (E + 1) + E]) : 0.f;
     float4* o = reinterpret_cast<float4*>(out + (size_t) t * H + i);
     float4 s = make_float4(0.f, 0.f, 0.f, 0.f), old = s;
     if (accumulate) old = *o;
     for (int k0 = 0; k0 < n; k0 += PC_ADD) {   // (the sum stays in pick order, the shared expert last)
-        float w[PC_ADD];
         float4 v[PC_ADD];
 #pragma unroll
-        for (int k = 0; k < PC_ADD; ++k) {   // (past the last addend: that one again, with weight 0)
-            const int a = min(k0 + k, n - 1);
-            if (a == Kp) w[k] = sigmoidf_(logits[(size_t) t * (E + 1) + E]);
-            else {
-                const int e = topi[(size_t) t * Kp + a];   // (outside the range nobody wrote the addend)
-                w[k] = e >= e_lo && e < e_hi ? topw[(size_t) t * Kp + a] : 0.f;
-            }
-            if (k0 + k >= n) w[k] = 0.f;
-        }
-#pragma unroll
         for (int k = 0; k < PC_ADD; ++k) {
-            const int a = min(k0 + k, n - 1);
+            const int a = k0 + k;
             const float4* p = reinterpret_cast<const float4*>(part + (a == Kp ? (size_t) T * Kp + t : (size_t) t * Kp + a) * H + i);
-            v[k] = EVERY || w[k] != 0.f ? __ldcs(p) : make_float4(0.f, 0.f, 0.f, 0.f);
+            v[k] = a < n && (EVERY || a >= Kp || mine[a] != 0.f) ? __ldcs(p) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
 #pragma unroll
         for (int k = 0; k < PC_ADD; ++k) {
-            const bool in = w[k] != 0.f;   // (an addend of weight 0 has no part in it, whatever it holds)
-            s.x = fmaf(w[k], in ? v[k].x : 0.f, s.x); s.y = fmaf(w[k], in ? v[k].y : 0.f, s.y);
-            s.z = fmaf(w[k], in ? v[k].z : 0.f, s.z); s.w = fmaf(w[k], in ? v[k].w : 0.f, s.w);
+            const int a = k0 + k;
+            const float w = a < Kp ? mine[a] : a < n ? gate : 0.f;
+            const bool in = w != 0.f;   // (an addend of weight 0 has no part in it, whatever it holds)
+            s.x = fmaf(w, in ? v[k].x : 0.f, s.x); s.y = fmaf(w, in ? v[k].y : 0.f, s.y);
+            s.z = fmaf(w, in ? v[k].z : 0.f, s.z); s.w = fmaf(w, in ? v[k].w : 0.f, s.w);
         }
     }
     *o = accumulate ? make_float4(s.x + old.x, s.y + old.y, s.z + old.z, s.w + old.w) : s;
