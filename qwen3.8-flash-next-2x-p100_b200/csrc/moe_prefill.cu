@@ -581,7 +581,7 @@ __global__ void __launch_bounds__(256, 4) k_pf_combine(const float* __restrict__
         for (int k = 0; k < PC_ADD; ++k) {
             const int a = k0 + k;
             const float w = a < Kp ? mine[a] : a < n ? gate : 0.f;
-            const bool in = w != 0.f;   // (an addend of weight 0 has no part in it, whatever it holds)
+            const bool in = a >= Kp || w != 0.f;   // (a pick of weight 0 has no part in it, whatever its addend holds)
             s.x = fmaf(w, in ? v[k].x : 0.f, s.x); s.y = fmaf(w, in ? v[k].y : 0.f, s.y);
             s.z = fmaf(w, in ? v[k].z : 0.f, s.z); s.w = fmaf(w, in ? v[k].w : 0.f, s.w);
         }

@@ -43,7 +43,7 @@ def test_job_lists_do_not_show_in_the_rows(F, T):
 @pytest.mark.parametrize("K,add_shared", [(1, True), (10, True), (11, False), (11, True), (12, True), (24, True), (32, True)])
 def test_combine_of_many_picks(F, K, add_shared):
     """The weighted sum of a row's addends (eleven at a time) at the edges of its passes, with every expert on this rank and with a range of
-    them; an addend of weight 0 stays out whatever it holds.  Every value is one f32 multiply-add per addend, in pick order."""
+    them.  Every value is one f32 multiply-add per addend, in pick order."""
     E, H, Fn, T = 32, 512, 256, 19
     fx = _moe_fixture(F, E, H, Fn, seed=31)
     g = torch.Generator(device="cuda").manual_seed(K)
@@ -91,3 +91,24 @@ def test_a_pick_that_names_no_expert_adds_nothing(F, K, T, half):
     for shared in (True, False):
         got, want = run(ids, topw, add_shared=shared), run(topi, torch.where(out_of_range, 0.0, topw), add_shared=shared)
         assert torch.isfinite(want).all() and torch.equal(got, want), shared
+
+
+@pytest.mark.parametrize("lo,hi", [(0, 32), (0, 16)])
+@pytest.mark.parametrize("K", [4, 12])
+def test_addends_that_are_not_finite(F, K, lo, hi):
+    """Picks of weight 0 leave nothing of theirs in a row, finite or not; the shared expert is no pick: where its gate has gone to 0, what is
+    not finite in it still shows."""
+    E, H, Fn, T = 32, 512, 256, 9
+    fx = _moe_fixture(F, E, H, Fn, seed=31)
+    g = torch.Generator(device="cuda").manual_seed(K)
+    x, old = torch.randn((T, H), device="cuda", generator=g), torch.randn((T, H), device="cuda", generator=g)
+    x[4:6] = float("inf")                                # (every expert's results for these two rows are NaN)
+    topi = torch.stack([torch.randperm(E, generator=torch.Generator().manual_seed(t))[:K] for t in range(T)]).int().cuda()
+    topw, logits = torch.rand((T, K), device="cuda", generator=g) + 0.1, torch.randn((T, E + 1), device="cuda", generator=g)
+    topw[4:6] = 0.0
+    logits[4:6, E] = -200.0
+    run = lambda shared: F.moe_prefill(fx["gu_t"], fx["dn_t"], fx["sh_gu_t"], fx["sh_dn_t"], topi, topw, logits, x, Fn, e_lo=lo, e_hi=hi, add_shared=shared, out=old.clone(),
+                                       accumulate=True)[0]
+    routed, every = run(False), run(True)
+    assert torch.equal(routed[4:6], old[4:6]) and torch.isnan(every[4:6]).all()
+    assert torch.isfinite(routed).all() and torch.isfinite(torch.cat([every[:4], every[6:]])).all()
