@@ -687,10 +687,12 @@ using namespace fnxb;
 static size_t pf_align(size_t v) { return (v + 255) & ~(size_t) 255; }
 
 // the rows of the job list's entries, in entry order: x_sorted[pos] = xh[token of order[pos]] (a routed pair t K + k: token t; a
-// shared-expert entry n + t: token t), so that a job's rows are consecutive for the tensor copies
-__global__ void __launch_bounds__(256) k_pf_gather_rows(const __half* __restrict__ xh, const int* __restrict__ order, int n, int Kp, int H, __half* __restrict__ xs) {
+// shared-expert entry n + t: token t), so that a job's rows are consecutive for the tensor copies.  Picks that name no expert have no entry: as many
+// places at the end hold whatever they held, no job reads their rows
+__global__ void __launch_bounds__(256) k_pf_gather_rows(const __half* __restrict__ xh, const int* __restrict__ order, int n, int Kp, int T, int H, __half* __restrict__ xs) {
     pdl_begin();
     const int pos = blockIdx.x, pair = order[pos], t = pair < n ? pair / Kp : pair - n;
+    if (pair < 0 || t >= T) return;
     const uint4* src = reinterpret_cast<const uint4*>(xh + (size_t) t * H);
     uint4* dst = reinterpret_cast<uint4*>(xs + (size_t) pos * H);
     for (int i = threadIdx.x; i < H / 8; i += 256) dst[i] = src[i];
@@ -772,7 +774,7 @@ int prompt_moe(const void* Wgu, size_t gu_stride, const void* Wsh_gu, bool gu_na
         FNX_TRY(pf_decode_f16_launch(Wsh_gu, false, 2 * F, H, gu16 + (size_t) E * 2 * F * H, st));
         FNX_TRY(pf_decode_f16_launch(Wdn, false, E * H, F, dn16, st));
         FNX_TRY(pf_decode_f16_launch(Wsh_dn, false, H, F, dn16 + (size_t) E * H * F, st));
-        FNX_CUDA_OK(launch_after(k_pf_gather_rows, dim3((unsigned) pairs), dim3(256), 0, st, xh, order, n, K, H, xs));
+        FNX_CUDA_OK(launch_after(k_pf_gather_rows, dim3((unsigned) pairs), dim3(256), 0, st, xh, order, n, K, T, H, xs));
         FNX_LAUNCH_OK("k_pf_gather_rows");
         const int nj = (int) ((size_t) n / PF_N) + ne + (T + PF_N - 1) / PF_N;
         FNX_TRY(gemm_tma_experts(gu16, dn16, E + 1, xs, hbuf, part, jobs, njobs, order, nj, (int) pairs, H, F, err, st));

@@ -72,7 +72,8 @@ def test_combine_of_many_picks(F, K, add_shared):
     assert ((rest.double() - want).abs() <= 2 * bound).all()
 
 
-@pytest.mark.parametrize("K,T", [(1, 3), (10, 40), (11, 19), (24, 21), (10, 830)])   # (one block's job list, one pass of addends and more; several blocks' list)
+@pytest.mark.parametrize("K,T", [(1, 3), (10, 40), (11, 19), (24, 21),   # one block's job list, one pass of addends and more
+                                 (10, 830), (4, 1030)])                    # several blocks' list; rows by tensor copies
 @pytest.mark.parametrize("half", [False, True])
 def test_a_pick_that_names_no_expert_adds_nothing(F, K, T, half):
     """Ids of -1 and E (a masked row, a masked pick) with weights that are not 0: no job has them, so nobody writes their addends, and the
