@@ -429,9 +429,10 @@ __global__ void __launch_bounds__(32) k_combine_image(const float* __restrict__ 
     pdl_launch_dependents();
     const int blk = blockIdx.x, t = blockIdx.y, lane = threadIdx.x, KB = H / 256;
     const size_t col = (size_t) blk * 256 + lane * 8;
+    const float mw = pick_weight(topi + t * K, topw + t * K, K, 0, E, lane);
     float w[32];
 #pragma unroll
-    for (int k = 0; k < 32; ++k) w[k] = k < K ? topw[t * K + k] : 0.f;
+    for (int k = 0; k < 32; ++k) w[k] = __shfl_sync(0xffffffffu, mw, k);
     const float shl = logits[(size_t) t * (E + 1) + E];
     QuantTask q[1];
     float v[1][8], nw[1][8];
@@ -456,7 +457,7 @@ __global__ void __launch_bounds__(32) k_combine_image(const float* __restrict__ 
             }
 #pragma unroll
         for (int k = 0; k < 16; ++k)
-            if (k0 + k < K) {
+            if (k0 + k < K && w[k0 + k] != 0.f) {
                 const float wk = w[k0 + k];
                 const float e8[8] = {a[k][0].x, a[k][0].y, a[k][0].z, a[k][0].w, a[k][1].x, a[k][1].y, a[k][1].z, a[k][1].w};
 #pragma unroll

@@ -39,3 +39,12 @@ def test_picks_that_do_not_count_add_nothing(F, T, K, lo, hi, shared):
     want = combine(F, f["part"], f["topi"], f["w0"], f["logits"], lo, hi, shared, f["old"])
     got = combine(F, f["dirty"], f["ids"], f["w"], f["logits"], lo, hi, shared, f["old"])
     assert torch.isfinite(want).all() and torch.equal(got, want)
+
+
+@pytest.mark.parametrize("T,K", [(1, 1), (5, 10), (13, 17), (32, 32)])
+def test_the_form_that_leaves_the_image_leaves_them_out_too(F, T, K):
+    f = fixture(T, K)
+    want = combine(F, f["dirty"], f["ids"], f["w"], f["logits"], 0, E, True, f["old"])
+    got = f["old"].clone()
+    F.moe_combine_image(f["dirty"], dict(topi=f["ids"], topw=f["w"], logits=f["logits"]), T, E, H, K, got, torch.ones(H, device="cuda"))
+    assert torch.isfinite(want).all() and torch.equal(got, want)
