@@ -117,14 +117,14 @@ __device__ __forceinline__ unsigned top_collect(const float* __restrict__ l, int
     return *count;
 }
 
-__global__ void __cluster_dims__(TOP_NB, 1, 1) __launch_bounds__(TOP_THREADS) k_top_tokens(const float* __restrict__ logits, int V, float* __restrict__ out_v, int* __restrict__ out_i) {
+__global__ void __cluster_dims__(1, TOP_NB, 1) __launch_bounds__(TOP_THREADS) k_top_tokens(const float* __restrict__ logits, int V, float* __restrict__ out_v, int* __restrict__ out_i) {
     pdl_wait();
     pdl_launch_dependents();
     __shared__ unsigned long long sel[TOP_CAP], top[FNX_TOPK_N], every[TOP_NB][FNX_TOPK_N];
     __shared__ unsigned low[TOP_THREADS / 32], hist[256], count, need_s;
     __shared__ unsigned long long prefix_s;
     cg::cluster_group cluster = cg::this_cluster();
-    const int t = blockIdx.y, part = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int t = blockIdx.x, part = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const float* l = logits + (size_t) t * V;
     const int lo = (int) ((long long) V * part / TOP_NB), hi = (int) ((long long) V * (part + 1) / TOP_NB);
     unsigned mx = 0;
@@ -251,7 +251,7 @@ extern "C" int fnx_argmax(const float* logits, int T, int V, int* best_i, float*
 extern "C" int fnx_top_tokens(const float* logits, int T, int V, float* out_v, int* out_i, fnx_stream st) {
     FNX_REQUIRE(logits && out_v && out_i && T >= 1 && V >= FNX_TOPK_N, "fnx_top_tokens: bad arguments (vocabulary of at least %d)", FNX_TOPK_N);
     {
-        const cudaError_t le_ = launch_dep(true, k_top_tokens, dim3(TOP_NB, T), dim3(TOP_THREADS), 0, as_stream(st), logits, V, out_v, out_i);
+        const cudaError_t le_ = launch_dep(true, k_top_tokens, dim3(T, TOP_NB), dim3(TOP_THREADS), 0, as_stream(st), logits, V, out_v, out_i);
         if (le_ != cudaSuccess) return fail(FNX_E_CUDA, "k_top_tokens: launch failed: %s", cudaGetErrorString(le_));
     }
     FNX_LAUNCH_OK("fnx_top_tokens");

@@ -27,6 +27,15 @@ def test_top_tokens_are_the_largest_keys(F, V):
     assert np.array_equal(one.cpu().numpy()[0], want[0])
 
 
+def test_top_tokens_and_argmax_of_more_rows_than_a_grids_second_dimension(F):
+    T, V = 65_537, 70
+    logits = torch.randn((T, V), device="cuda", generator=torch.Generator(device="cuda").manual_seed(4))
+    v, i = F.top_tokens(logits)
+    want = logits.sort(dim=1, descending=True)   # (equal values may come in another order: the values are compared, and that the ids lead to them)
+    assert torch.equal(v, want.values[:, :64]) and torch.equal(logits.gather(1, i.long()), v)
+    assert torch.equal(F.argmax(logits)[1], want.values[:, 0])
+
+
 def test_accept_sample_with_draft_distributions(F, O):
     """Drafts of their own distributions (up to 64 candidates, in any order) beside fixed ones: counts and tokens as the oracle's."""
     rng = np.random.default_rng(12)
