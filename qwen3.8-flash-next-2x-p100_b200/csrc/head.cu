@@ -26,19 +26,28 @@ __device__ __forceinline__ unsigned long long warp_max_key(unsigned long long k)
     return ((unsigned long long) top << 32) | __reduce_max_sync(0xffffffffu, hi == top ? (unsigned) k : 0u);
 }
 
-// A row by a cluster of ARGMAX_NB blocks, a slice each, which leave their largest keys in the first one's shared memory.  Bound by latency: the launch, the
-// slice's way, one barrier of the cluster.  (Sixteen blocks that met in device memory, an atomic maximum and an arrival counter: 6.2 us a launch for a row of
-// 151,936, one block for 40,528 6.3; 4.4 and 3.0 now.)
-constexpr int ARGMAX_NB = 8;
+// Both kernels below take a row by a cluster of NB blocks, a slice each.  Few rows want many blocks; but clusters are placed whole, on SMs of one group, and the
+// chip holds 15 of eight blocks, 33 of four and 74 of two at the pace of a lone one: every further round of them costs what a block for a whole row
+// would have taken.  Argmax over rows of 40,528, us a launch with 8, 4, 2 and 1 blocks: 5 rows 2.6, 2.9, 4.1, 5.3; 16 rows 3.6, 2.9, 4.1, 5.4; 33 rows 3.8,
+// 3.6, 4.1, 5.4; 74 rows 9.3, 6.2, 4.3, 5.5; 75 rows 9.4, 6.2, 6.2, 5.5; 4,000 rows 431, 227, 161, 112.
+static int blocks_by_rows(int T) { return T <= 15 ? 8 : T <= 33 ? 4 : T <= 74 ? 2 : 1; }
+// A short row gains nothing by more blocks (1 row of 4,096: 2.0 us with eight and with one; of 8,192 2.1 and 2.3).  Where a slice takes long, a second round of
+// fours costs more than eight blocks two to an SM (28 rows of 100,000: 5.7 and 4.7, of 40,528 3.6 and 3.8; 40 rows of 262,144, two blocks 13.2, eight 12.3).
+static int argmax_blocks(int T, int V) { return V < 8192 ? 1 : V >= 100000 && T > 24 && T <= 40 ? 8 : blocks_by_rows(T); }
+// the candidates' second look and their counting cost less in one block up to here (5 rows of 8,192: 5.8 us, with eight 6.8; of 40,528 10.5 and 8.3)
+static int top_blocks(int T, int V) { return V < 16384 ? 1 : blocks_by_rows(T); }
 
-__global__ void __cluster_dims__(1, ARGMAX_NB, 1) __launch_bounds__(1024) k_argmax(const float* __restrict__ logits, int V, const int* __restrict__ map, int* __restrict__ best_i,
-                                                                                  float* __restrict__ best_v, unsigned* __restrict__ err) {
-    __shared__ unsigned long long red[32], every[ARGMAX_NB];
+// The slices' largest keys meet in the first block's shared memory.  Bound by latency: the launch, the slice's way, one barrier of the cluster.  (Sixteen blocks
+// that met in device memory, an atomic maximum and an arrival counter: 4.5 us a launch for five rows of 151,936, 7.6 for twenty; 4.0 and 5.7 now.)
+template <int NB>
+__global__ void __cluster_dims__(1, NB, 1) __launch_bounds__(1024, 2) k_argmax(const float* __restrict__ logits, int V, const int* __restrict__ map, int* __restrict__ best_i,
+                                                                            float* __restrict__ best_v, unsigned* __restrict__ err) {
+    __shared__ unsigned long long red[32], every[NB];
     cg::cluster_group cluster = cg::this_cluster();
-    cluster.sync();   // (the first block's shared memory is there)
+    if (NB > 1) cluster.sync();   // (the first block's shared memory is there)
     pdl_wait();
     pdl_launch_dependents();
-    const int t = blockIdx.x, tid = threadIdx.x, nb = ARGMAX_NB;
+    const int t = blockIdx.x, tid = threadIdx.x, nb = NB;
     const float* l = logits + (size_t) t * V;
     unsigned long long best = 0;
     bool bad = false;
@@ -74,11 +83,11 @@ __global__ void __cluster_dims__(1, ARGMAX_NB, 1) __launch_bounds__(1024) k_argm
     __syncthreads();
     if (tid < 32) {
         best = warp_max_key(red[tid]);
-        if (tid == 0) *cluster.map_shared_rank(every + blockIdx.y, 0) = best;
+        if (NB > 1 && tid == 0) *cluster.map_shared_rank(every + blockIdx.y, 0) = best;
     }
-    cluster.sync();
+    if (NB > 1) cluster.sync();
     if (blockIdx.y == 0 && tid < 32) {
-        best = warp_max_key(tid < nb ? every[tid] : 0ull);
+        if (NB > 1) best = warp_max_key(tid < nb ? every[tid] : 0ull);
         if (tid == 0) {
             const int row = (int) ~(uint32_t) best;
             best_i[t] = map ? map[row] : row;
@@ -87,12 +96,13 @@ __global__ void __cluster_dims__(1, ARGMAX_NB, 1) __launch_bounds__(1024) k_argm
     }
 }
 
-// The 64 candidates of a row by a cluster of TOP_NB blocks, a slice of the row each.  In its slice a warp's second largest lane maximum bounds the 64th
-// largest value of the block from below as soon as it is the smallest of the 32 warps' (64 values are at or above it), so a second look at the slice
-// leaves a few values more than needed (170 of 19,000 where they are random), which find their places by counting; the first block then merges the
-// slices' sorted 64 by searching the others for each.  A slice with more than TOP_CAP values that high (many equal logits) is selected digit by digit.
-// Bound by two looks at the row and a dozen block barriers: 20 rows of 151,936 logits 162 us with a block a row and nine looks, 18 now.
-constexpr int TOP_NB = 8, TOP_CAP = 1024, TOP_THREADS = 1024;
+// The 64 candidates of a row.  In a slice a warp's second largest lane maximum bounds the 64th largest value of the block from below as soon as it is the
+// smallest of the 32 warps' (64 values are at or above it), so a second look at the slice leaves a few values more than needed (170 of 19,000 where they
+// are random), which find their places by counting; the first block then merges the slices' sorted 64 by searching the others for each.  A slice with more
+// than TOP_CAP values that high (many equal logits) is selected digit by digit.
+// Bound by two looks at the row and a dozen block barriers: with a block a row and nine looks 20 rows of 151,936 logits took 162 us, 4,000 of 40,528 1,115; 14 and
+// 237 now, equal logits 178 and 40 (20 rows).
+constexpr int TOP_CAP = 1024, TOP_THREADS = 1024;
 constexpr int TOP_LD = 8;   // loads in flight a thread
 
 // keys of the slice [lo, hi) at or above `thr` into sel, at most cap of them; returns how many there are (every thread; ends with a barrier)
@@ -117,18 +127,25 @@ __device__ __forceinline__ unsigned top_collect(const float* __restrict__ l, int
     return *count;
 }
 
-__global__ void __cluster_dims__(1, TOP_NB, 1) __launch_bounds__(TOP_THREADS) k_top_tokens(const float* __restrict__ logits, int V, float* __restrict__ out_v, int* __restrict__ out_i) {
+template <int NB>
+__global__ void __cluster_dims__(1, NB, 1) __launch_bounds__(TOP_THREADS) k_top_tokens(const float* __restrict__ logits, int V, float* __restrict__ out_v, int* __restrict__ out_i) {
     pdl_wait();
     pdl_launch_dependents();
-    __shared__ unsigned long long sel[TOP_CAP], top[FNX_TOPK_N], every[TOP_NB][FNX_TOPK_N];
-    __shared__ unsigned low[TOP_THREADS / 32], hist[256], count, need_s;
+    __shared__ __align__(16) unsigned long long sel[TOP_CAP + 4];
+    __shared__ unsigned long long top[FNX_TOPK_N], every[NB][FNX_TOPK_N];
+    __shared__ unsigned low[TOP_THREADS / 32], high[TOP_THREADS / 32], hist[256], count, need_s;
     __shared__ unsigned long long prefix_s;
     cg::cluster_group cluster = cg::this_cluster();
     const int t = blockIdx.x, part = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const float* l = logits + (size_t) t * V;
-    const int lo = (int) ((long long) V * part / TOP_NB), hi = (int) ((long long) V * (part + 1) / TOP_NB);
+    const int lo = (int) ((long long) V * part / NB), hi = (int) ((long long) V * (part + 1) / NB);
     unsigned mx = 0;
-    for (int i0 = lo + tid; i0 < hi; i0 += TOP_THREADS * TOP_LD) {
+    int from = lo + tid;
+    if (hi - lo < TOP_THREADS) {   // a short slice: alike for every warp, up to a value a lane
+        const int a = (hi - lo) * warp / 32, b = (hi - lo) * (warp + 1) / 32;
+        from = lane < b - a ? lo + a + lane : hi;
+    }
+    for (int i0 = from; i0 < hi; i0 += TOP_THREADS * TOP_LD) {
         float v[TOP_LD];
 #pragma unroll
         for (int j = 0; j < TOP_LD; ++j) v[j] = i0 + j * TOP_THREADS < hi ? l[i0 + j * TOP_THREADS] : l[i0];
@@ -138,17 +155,22 @@ __global__ void __cluster_dims__(1, TOP_NB, 1) __launch_bounds__(TOP_THREADS) k_
     const unsigned first = __reduce_max_sync(0xffffffffu, mx);
     const int who = __ffs(__ballot_sync(0xffffffffu, mx == first)) - 1;
     const unsigned second = __reduce_max_sync(0xffffffffu, lane == who ? 0u : mx);
-    if (lane == 0) low[warp] = second;
+    if (lane == 0) {
+        low[warp] = second;
+        high[warp] = first;
+    }
     __syncthreads();
     const unsigned bound = __reduce_min_sync(0xffffffffu, low[lane]);
     unsigned n = top_collect(l, lo, hi, (unsigned long long) bound << 32, sel, TOP_CAP, &count, tid);
     if (n > TOP_CAP) {
-        // 8 passes of 8 bits from the top: after pass p the first 8 (p + 1) bits of the slice's 64th largest key are known
+        // passes of 8 bits from the top: after pass p the first 8 (p + 1) bits of the slice's 64th largest key are known.  It lies between the bound and the
+        // largest value: what these two have in common at the top is known before (equal logits: the value, four passes of eight)
+        const int known = __clz(bound ^ __reduce_max_sync(0xffffffffu, high[lane])) / 8;
         if (tid == 0) {
-            prefix_s = 0;
+            prefix_s = known ? ((unsigned long long) bound << 32) & ~0ull << (64 - 8 * known) : 0ull;
             need_s = FNX_TOPK_N;
         }
-        for (int pass = 0; pass < 8; ++pass) {
+        for (int pass = known; pass < 8; ++pass) {
             const int shift = 56 - 8 * pass;
             if (tid < 256) hist[tid] = 0;
             __syncthreads();
@@ -175,33 +197,45 @@ __global__ void __cluster_dims__(1, TOP_NB, 1) __launch_bounds__(TOP_THREADS) k_
     }
     // the slice's 64 largest in order; fewer where the slice holds fewer (0: no key)
     if (tid < FNX_TOPK_N) top[tid] = 0;
+    if (tid < 4) sel[n + tid] = 0;
     __syncthreads();
     if (tid < (int) n) {
         const unsigned long long k = sel[tid];
         unsigned rank = 0;
-        for (unsigned j = 0; j < n; ++j) rank += sel[j] > k;
+        for (unsigned j = 0; j < n; j += 4) {
+            const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(sel + j), b = *reinterpret_cast<const ulonglong2*>(sel + j + 2);
+            rank += (a.x > k) + (a.y > k) + (b.x > k) + (b.y > k);
+        }
         if (rank < FNX_TOPK_N) top[rank] = k;
     }
+    if (NB == 1) {
+        __syncthreads();
+        if (tid < FNX_TOPK_N) {
+            out_v[(size_t) t * FNX_TOPK_N + tid] = fkey_inv((uint32_t) (top[tid] >> 32));
+            out_i[(size_t) t * FNX_TOPK_N + tid] = (int) ~(uint32_t) top[tid];
+        }
+        return;
+    }
     cluster.sync();
-    if (part == 0 && tid < TOP_NB * FNX_TOPK_N) every[tid / FNX_TOPK_N][tid % FNX_TOPK_N] = cluster.map_shared_rank(top, tid / FNX_TOPK_N)[tid % FNX_TOPK_N];
+    if (part == 0 && tid < NB * FNX_TOPK_N) every[tid / FNX_TOPK_N][tid % FNX_TOPK_N] = cluster.map_shared_rank(top, tid / FNX_TOPK_N)[tid % FNX_TOPK_N];
     cluster.sync();   // (no block leaves while its keys are read)
-    if (part == 0 && tid < TOP_NB * FNX_TOPK_N) {
+    if (part == 0 && tid < NB * FNX_TOPK_N) {
         const int own = tid / FNX_TOPK_N;
         const unsigned long long k = every[own][tid % FNX_TOPK_N];
-        unsigned rank = tid % FNX_TOPK_N, at[TOP_NB];   // the larger ones: before it in its own list, and in the others
+        unsigned rank = tid % FNX_TOPK_N, at[NB];   // the larger ones: before it in its own list, and in the others
 #pragma unroll
-        for (int p = 0; p < TOP_NB; ++p) at[p] = 0;
+        for (int p = 0; p < NB; ++p) at[p] = 0;
 #pragma unroll
         for (int step = FNX_TOPK_N / 2; step; step >>= 1)
 #pragma unroll
-            for (int p = 0; p < TOP_NB; ++p)
+            for (int p = 0; p < NB; ++p)
                 if (every[p][at[p] + step - 1] > k) at[p] += step;
 #pragma unroll
-        for (int p = 0; p < TOP_NB; ++p)
+        for (int p = 0; p < NB; ++p)
             if (p != own) rank += at[p] + (every[p][at[p]] > k ? 1u : 0u);
         if (k && rank < FNX_TOPK_N) {
-            out_v[t * FNX_TOPK_N + rank] = fkey_inv((uint32_t) (k >> 32));
-            out_i[t * FNX_TOPK_N + rank] = (int) ~(uint32_t) k;
+            out_v[(size_t) t * FNX_TOPK_N + rank] = fkey_inv((uint32_t) (k >> 32));
+            out_i[(size_t) t * FNX_TOPK_N + rank] = (int) ~(uint32_t) k;
         }
     }
 }
@@ -237,7 +271,9 @@ using namespace fnxb;
 extern "C" int fnx_argmax_mapped(const float* logits, int T, int V, const int* map, int* best_i, float* best_v, unsigned* err, fnx_stream st) {
     FNX_REQUIRE(logits && best_i && err && T >= 1 && V >= 1, "fnx_argmax: bad arguments");
     {
-        const cudaError_t le_ = launch_dep(true, k_argmax, dim3(T, ARGMAX_NB), dim3(1024), 0, as_stream(st), logits, V, map, best_i, best_v, err);
+        const int nb = argmax_blocks(T, V);
+        auto kernel = nb == 8 ? k_argmax<8> : nb == 4 ? k_argmax<4> : nb == 2 ? k_argmax<2> : k_argmax<1>;
+        const cudaError_t le_ = launch_dep(true, kernel, dim3(T, nb), dim3(1024), 0, as_stream(st), logits, V, map, best_i, best_v, err);
         if (le_ != cudaSuccess) return fail(FNX_E_CUDA, "k_argmax: launch failed: %s", cudaGetErrorString(le_));
     }
     FNX_LAUNCH_OK("fnx_argmax");
@@ -251,7 +287,9 @@ extern "C" int fnx_argmax(const float* logits, int T, int V, int* best_i, float*
 extern "C" int fnx_top_tokens(const float* logits, int T, int V, float* out_v, int* out_i, fnx_stream st) {
     FNX_REQUIRE(logits && out_v && out_i && T >= 1 && V >= FNX_TOPK_N, "fnx_top_tokens: bad arguments (vocabulary of at least %d)", FNX_TOPK_N);
     {
-        const cudaError_t le_ = launch_dep(true, k_top_tokens, dim3(T, TOP_NB), dim3(TOP_THREADS), 0, as_stream(st), logits, V, out_v, out_i);
+        const int nb = top_blocks(T, V);
+        auto kernel = nb == 8 ? k_top_tokens<8> : nb == 4 ? k_top_tokens<4> : nb == 2 ? k_top_tokens<2> : k_top_tokens<1>;
+        const cudaError_t le_ = launch_dep(true, kernel, dim3(T, nb), dim3(TOP_THREADS), 0, as_stream(st), logits, V, out_v, out_i);
         if (le_ != cudaSuccess) return fail(FNX_E_CUDA, "k_top_tokens: launch failed: %s", cudaGetErrorString(le_));
     }
     FNX_LAUNCH_OK("fnx_top_tokens");

@@ -68,3 +68,19 @@ def test_argmax_over_a_cluster(F, T, V):
     assert np.array_equal(i.cpu().numpy(), logits.argmax(1)) and np.array_equal(v.cpu().numpy(), logits.max(1)) and int(err.item()) == 0
     logits[T - 1, V - 1] = -np.inf
     assert int(F.argmax(torch.from_numpy(logits).cuda())[2].item()) == 16
+
+
+@pytest.mark.parametrize("T", [15, 16, 25, 33, 34, 74, 75])
+@pytest.mark.parametrize("V", [65, 700, 1023, 1024, 8191, 8192, 16383, 16384, 50001, 100000])
+def test_rows_by_eight_blocks_to_one(F, T, V):
+    """Either side of where a row's blocks become fewer: the candidates and the largest of rows without ties, with many, and all alike."""
+    g = torch.Generator(device="cuda").manual_seed(T * V)
+    logits = torch.randn((T, V), device="cuda", generator=g) + 0.0
+    logits[T // 2:] = torch.round(logits[T // 2:] * 2) + 0.0             # (no negative zeros)
+    logits[T - 1] = -1.5
+    logits[T - 2] = torch.round(logits[T - 2] * 1e6) * 1e-6 + 1000.0     # (values that share most of their bits)
+    want_v, want_i = logits.sort(dim=1, descending=True, stable=True)    # the lower index among equals
+    v, i = F.top_tokens(logits)
+    assert torch.equal(v, want_v[:, :64]) and torch.equal(i.long(), want_i[:, :64])
+    i, v, err = F.argmax(logits)
+    assert torch.equal(v, want_v[:, 0]) and torch.equal(i.long(), want_i[:, 0]) and int(err.item()) == 0
