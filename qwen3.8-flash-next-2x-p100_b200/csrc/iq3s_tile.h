@@ -177,4 +177,17 @@ FNX_HD uint32_t tile_sign_mask(const uint32_t (&G)[2]) {
 // byte g, -g == g ^ 0xFE
 FNX_HD uint32_t tile_apply_sign(uint32_t mag, uint32_t mask) { return mag ^ (mask & 0xFEFEFEFEu); }
 
+// How the operators' products cut their units (16-row tiles, job after job) into blocks' shares, without a division on the device.
+// n / d for 32-bit n, from the largest 32-bit multiple of 1 / d (the product is at most one short of the quotient)
+inline unsigned mmv_inverse(unsigned d) { return d > 1 ? (unsigned) (0x100000000ull / d) : 0xFFFFFFFFu; }
+FNX_HD unsigned mmv_div(unsigned n, unsigned d, unsigned inv) {
+    const unsigned q = (unsigned) (((uint64_t) n * inv) >> 32);
+    return q + (n - q * d >= d ? 1u : 0u);
+}
+// total * bid / nblk, whatever the product's size: the quotient's share, and that of the rest (bid <= nblk < 2^16)
+FNX_HD unsigned mmv_first_unit(unsigned total, unsigned bid, unsigned nblk, unsigned inv) {
+    const unsigned q = mmv_div(total, nblk, inv);
+    return q * bid + mmv_div((total - q * nblk) * bid, nblk, inv);
+}
+
 }  // namespace fnxb

@@ -56,13 +56,6 @@ __host__ __device__ inline size_t stage_image_bytes(int NG, int K) {
     return (size_t) NG * ((size_t) (K / 32) * 32 * 8 + (size_t) (K / 256) * 8 * 4 + 4 * 16 * 4);
 }
 
-// n / d for 32-bit n, from the largest 32-bit multiple of 1 / d (the product is at most one short of the quotient)
-inline unsigned mmv_inverse(unsigned d) { return d > 1 ? (unsigned) (0x100000000ull / d) : 0xFFFFFFFFu; }
-__device__ __forceinline__ unsigned mmv_div(unsigned n, unsigned d, unsigned inv) {
-    const unsigned q = __umulhi(n, inv);
-    return q + (n - q * d >= d ? 1u : 0u);
-}
-
 // jobs whose activation images a block holds at once: its range of units spans at most two jobs of gate|up and a
 // few of down; anything wider is walked in passes
 template <int MODE>
@@ -202,8 +195,8 @@ __device__ __forceinline__ void stage_run(const MmvParams& p, const StageSmem& S
         __syncthreads();
     }
     stamp();
-    const unsigned upj = p.rows / 16, total = (unsigned) njobs * upj;   // < 2^24: the products below stay inside 32 bits
-    const int u0 = (int) mmv_div(total * bid, nblk, p.nblk_inv), u1 = (int) mmv_div(total * (bid + 1), nblk, p.nblk_inv);
+    const unsigned upj = p.rows / 16, total = (unsigned) njobs * upj;
+    const int u0 = (int) mmv_first_unit(total, bid, nblk, p.nblk_inv), u1 = (int) mmv_first_unit(total, bid + 1, nblk, p.nblk_inv);
     auto job_of = [&](int u) { return MOE ? (int) mmv_div(u, upj, p.upj_inv) : 0; };
     const float* norm_w = MODE == MAT_DOWN ? nullptr : p.norm_w;
     uint8_t* slots = S.slots + (size_t) warp * p.R * TILE_BYTES;
@@ -215,7 +208,7 @@ __device__ __forceinline__ void stage_run(const MmvParams& p, const StageSmem& S
     bool first = true, ok = true;
     for (int uc = u0; uc < u1;) {
         const int j0 = job_of(uc), j1 = min(j0 + JMAX, job_of(u1 - 1) + 1), ue = MOE ? min(u1, j1 * (int) upj) : u1;
-        const unsigned N = (unsigned) (ue - uc) << lnb;   // < 2^26 for any matrix here
+        const unsigned N = (unsigned) (ue - uc) << lnb;   // (16 N < 2^32: N tiles of 1,760 bytes a block)
         const int i0 = (int) ((N * warp) / MMV_WARPS), i1 = (int) ((N * (warp + 1)) / MMV_WARPS);
         auto item_src = [&](int item) -> const uint8_t* {
             if (!MOE) return p.W + ((size_t) uc * KB + item) * TILE_BYTES;

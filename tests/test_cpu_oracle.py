@@ -207,6 +207,16 @@ def test_tile_layout_round_trip_and_warp_replay(O, sim):
         assert np.abs(y - ref).max() <= 2e-4 * np.abs(ref).max()
 
 
+def test_units_are_cut_alike_however_many_there_are(sim):
+    """Block b's units are [total b / n, total (b + 1) / n), also where that product needs more than 32 bits."""
+    sim.sim_first_unit.restype = C.c_uint
+    rng = np.random.default_rng(2)
+    for n in (1, 2, 3, 132, 148, 160, 65535):
+        for total in [0, 1, n - 1, n, n + 1, 772, 2 ** 24, min(2 ** 32 // n, 2 ** 31 - 1), 30_000_000, 2 ** 31 - 1] + rng.integers(0, 2 ** 31, size=40).tolist():
+            for b in {0, 1, n // 2, n - 1, n}:
+                assert sim.sim_first_unit(total, b, n) == total * b // n, (total, b, n)
+
+
 def test_c_abi_exports_every_declared_symbol(F):
     hdr = (ROOT / "include" / "fnx_b200.h").read_text()
     declared = set(re.findall(r"\b(fnx_[a-z0-9_]+)\s*\(", hdr))
