@@ -93,16 +93,18 @@ __device__ __forceinline__ float warp_max(float v) {
 __device__ __forceinline__ float sigmoidf_(float x) { return 1.0f / (1.0f + expf(-x)); }
 __device__ __forceinline__ float siluf_(float x) { return x / (1.0f + expf(-x)); }
 
-// the weight of a row's pick `lane` (of K <= 32): 0 where it names no expert in [e_lo, e_hi), and past the last one
-__device__ __forceinline__ float pick_weight(const int* topi, const float* topw, int K, int e_lo, int e_hi, int lane) {
-    int e = e_lo;
-    float w = 0.f;
-    if (lane < K) {
-        e = topi[lane];
-        w = topw[lane];
+// a row's pick `lane` (of K <= 32) on its way; its weight is 0 where it names no expert in [e_lo, e_hi), and past the last one
+struct Pick {
+    int e;
+    float w;
+    __device__ __forceinline__ Pick(const int* topi, const float* topw, int K, int lane) : e(-1), w(0.f) {
+        if (lane < K) {
+            e = topi[lane];
+            w = topw[lane];
+        }
     }
-    return e >= e_lo && e < e_hi ? w : 0.f;
-}
+    __device__ __forceinline__ float weight(int e_lo, int e_hi) const { return e >= e_lo && e < e_hi ? w : 0.f; }
+};
 
 // ---- shared-memory barriers for bulk async copies.  Every wait is bounded: after `limit` polls it gives up and
 // the caller records FNX_ERR_TIMEOUT instead of hanging the GPU.

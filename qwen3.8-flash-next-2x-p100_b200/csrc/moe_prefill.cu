@@ -563,8 +563,11 @@ __global__ void __launch_bounds__(256, 4) k_pf_combine(const float* __restrict__
     const int t = blockIdx.y, i = (blockIdx.x * blockDim.x + threadIdx.x) * 4, n = Kp + (add_shared ? 1 : 0), lane = threadIdx.x & 31;
     if (i >= H) return;   // (whole warps: H is a multiple of 256)
     float* mine = weights[threadIdx.x >> 5];
-    mine[lane] = pick_weight(topi + (size_t) t * Kp, topw + (size_t) t * Kp, Kp, e_lo, e_hi, lane);
-    __syncwarp();
+    const Pick pick(topi + (size_t) t * Kp, topw + (size_t) t * Kp, Kp, lane);
+    if (!EVERY) {
+        mine[lane] = pick.weight(e_lo, e_hi);
+        __syncwarp();
+    }
     const float gate = add_shared ? sigmoidf_(logits[(size_t) t * (E + 1) + E]) : 0.f;
     float4* o = reinterpret_cast<float4*>(out + (size_t) t * H + i);
     float4 s = make_float4(0.f, 0.f, 0.f, 0.f), old = s;
@@ -576,6 +579,10 @@ __global__ void __launch_bounds__(256, 4) k_pf_combine(const float* __restrict__
             const int a = k0 + k;
             const float4* p = reinterpret_cast<const float4*>(part + (a == Kp ? (size_t) T * Kp + t : (size_t) t * Kp + a) * H + i);
             v[k] = a < n && (EVERY || a >= Kp || mine[a] != 0.f) ? __ldcs(p) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        if (EVERY && k0 == 0) {   // (behind the loads: a store waits for what it stores)
+            mine[lane] = pick.weight(e_lo, e_hi);
+            __syncwarp();
         }
 #pragma unroll
         for (int k = 0; k < PC_ADD; ++k) {

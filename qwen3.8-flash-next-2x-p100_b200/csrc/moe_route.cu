@@ -393,11 +393,12 @@ __global__ void k_combine(const float* __restrict__ part, const int* __restrict_
     pdl_launch_dependents();
     const int t = blockIdx.y, i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
     float* mine = weights[threadIdx.x >> 5];
-    mine[lane] = pick_weight(topi + t * K, topw + t * K, K, e_lo, e_hi, lane);
-    __syncwarp();
+    const Pick pick(topi + t * K, topw + t * K, K, lane);
     float w[32], v[32];
 #pragma unroll
     for (int k = 0; k < 32; ++k) v[k] = k < K && i < H ? part[((size_t) t * K + k) * H + i] : 0.f;
+    mine[lane] = pick.weight(e_lo, e_hi);
+    __syncwarp();
 #pragma unroll
     for (int k = 0; k < 32; k += 4) {
         const float4 f = *reinterpret_cast<const float4*>(mine + k);
@@ -429,7 +430,7 @@ __global__ void __launch_bounds__(32) k_combine_image(const float* __restrict__ 
     pdl_launch_dependents();
     const int blk = blockIdx.x, t = blockIdx.y, lane = threadIdx.x, KB = H / 256;
     const size_t col = (size_t) blk * 256 + lane * 8;
-    const float mw = pick_weight(topi + t * K, topw + t * K, K, 0, E, lane);
+    const float mw = Pick(topi + t * K, topw + t * K, K, lane).weight(0, E);
     float w[32];
 #pragma unroll
     for (int k = 0; k < 32; ++k) w[k] = __shfl_sync(0xffffffffu, mw, k);
