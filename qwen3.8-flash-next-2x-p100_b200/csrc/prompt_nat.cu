@@ -22,6 +22,8 @@
 // of 760 rows an expert 1,940 + 1,244 (187 + 101, 200 + 126 and 2,172 + 1,334 with four stages of rows, N = 64 and two instructions a word more).  With neither decode nor
 // products 128: the hand-over between the decode warps, the weight stages, the rows and the issuing thread, then the decode's instructions (half of the
 // issue slots), are what is left here; DRAM would allow 88.
+#include <type_traits>
+
 #include "attn_tc.cuh"
 #include "nat_tile.h"
 #include "prompt_nat.cuh"
@@ -76,24 +78,30 @@ __device__ __forceinline__ uint32_t pn_and_xor(uint32_t a, uint32_t b, uint32_t 
 // (4, 6), (5, 7).  A nibble t at bits 0..3 of a half 0x6400 | .. is 1024 + (t + 8): twice that less 2,064 is 2 t, and one multiply-add makes
 // (2 t + 1) f of it; at bits 4..7 it is 1024 + 16 (t + 8) = 8 (143 + m).  All exact but the one rounding of m f, as in the other forms of these
 // products.  (Thirteen instructions a word; with the low nibbles moved up a bit, so that 1,039 + m was left to subtract, fifteen.)
+// WIDE: the same for scales that may be infinite, where (2 t) f + f would be NaN.
+template <bool WIDE>
 __device__ __forceinline__ void pn_decode8(uint32_t w, __half2 f, uint32_t& o0, uint32_t& o1, uint32_t& o2, uint32_t& o3) {
     const uint32_t s = w >> 8;
     const uint32_t a = pn_and_xor(w, 0x000F000Fu, 0x64086408u), c = pn_and_xor(w, 0x00F000F0u, 0x64806480u);
     const uint32_t b = pn_and_xor(s, 0x000F000Fu, 0x64086408u), d = pn_and_xor(s, 0x00F000F0u, 0x64806480u);
-    const __half2 two = pn_as_h2(0x40004000u), k1 = pn_as_h2(0xE808E808u);      // 2, -2,064
+    const __half2 two = pn_as_h2(0x40004000u), k1 = pn_as_h2(0xE808E808u), one = pn_as_h2(0x3C003C00u);   // 2, -2,064, 1
     const __half2 k8 = pn_as_h2(0x30003000u), k2 = pn_as_h2(0xD878D878u);       // 1 / 8, -143
-    o0 = pn_h2(__hfma2(__hfma2(pn_as_h2(a), two, k1), f, f));
-    o1 = pn_h2(__hfma2(__hfma2(pn_as_h2(b), two, k1), f, f));
+    const __half2 ta = __hfma2(pn_as_h2(a), two, k1), tb = __hfma2(pn_as_h2(b), two, k1);
+    o0 = pn_h2(WIDE ? __hmul2(__hadd2(ta, one), f) : __hfma2(ta, f, f));
+    o1 = pn_h2(WIDE ? __hmul2(__hadd2(tb, one), f) : __hfma2(tb, f, f));
     o2 = pn_h2(__hmul2(__hfma2(pn_as_h2(c), k8, k2), f));
     o3 = pn_h2(__hmul2(__hfma2(pn_as_h2(d), k8, k2), f));
 }
+// whether one of a warp's scales d (two rows' in a word; z = d & d << 1) may overflow f16 times 31: 512 and up, infinities and NaN
+__device__ __forceinline__ bool pn_wide(uint32_t z) { return __any_sync(0xffffffffu, (z & 0x40004000u) != 0u); }
 // a row's two scales d (1 + 2 s) of sub-blocks 2 Q and 2 Q + 1 (the nibbles of byte Q of sn); d in both halves.  The byte goes into both halves
-// 0x6400 | .., the low one keeps its low nibble (1024 + s), the high one its high nibble (1024 + 16 s); 2 s is exact, and d (1 + 2 s) rounds once, as from f32
+// 0x6400 | .., the low one keeps its low nibble (1024 + s), the high one its high nibble (1024 + 16 s); 1 + 2 s is exact, and its product with d rounds once, as
+// from f32
 __device__ __forceinline__ void pn_scales(uint32_t sn, int Q, __half2 d, __half2& f0, __half2& f1) {
     uint32_t t;
     asm("prmt.b32 %0, %1, %2, %3;" : "=r"(t) : "r"(sn), "r"(0x64u), "r"(0x4040u + 0x0101u * Q));
-    const __half2 s2 = __hfma2(pn_as_h2(t & 0xFFF0FF0Fu), pn_as_h2(0x30004000u), pn_as_h2(0xD800E800u));   // (2, 1 / 8) x - (2,048, 128)
-    const __half2 f = __hfma2(s2, d, d);
+    const __half2 s2 = __hfma2(pn_as_h2(t & 0xFFF0FF0Fu), pn_as_h2(0x30004000u), pn_as_h2(0xD7F0E7FFu));   // (2, 1 / 8) x - (2,047, 127)
+    const __half2 f = __hmul2(s2, d);
     f0 = __low2half2(f);
     f1 = __high2half2(f);
 }
@@ -211,30 +219,35 @@ __global__ void __launch_bounds__(PN_THREADS, 1) k_prompt_nat(const PnParams p) 
                 __syncwarp();   // every lane has the slot
                 fetch();
                 slot = slot + 1 == PN_SLOTS ? 0 : slot + 1;
+                auto decode = [&](auto wide) {
+                    constexpr bool WIDE = decltype(wide)::value;
 #pragma unroll
-                for (int st = 0; st < PN_AST; ++st, ++c) {
+                    for (int st = 0; st < PN_AST; ++st, ++c) {
 #pragma unroll
-                    for (int q2 = 0; q2 < PN_KC / 64; ++q2) {
-                        const int Q = PN_KC / 64 * st + q2;
-                        uint32_t o[16];
-                        __half2 f00, f01, f10, f11;
-                        pn_scales(m.x, Q, d0, f00, f01);
-                        pn_scales(m.y, Q, d1, f10, f11);
-                        pn_decode8(w[0][2 * Q], f00, o[0], o[1], o[4], o[5]);
-                        pn_decode8(w[1][2 * Q], f10, o[2], o[3], o[6], o[7]);
-                        pn_decode8(w[0][2 * Q + 1], f01, o[8], o[9], o[12], o[13]);
-                        pn_decode8(w[1][2 * Q + 1], f11, o[10], o[11], o[14], o[15]);
-                        if (q2 == 0) {
-                            if (ok && c >= PN_AST) ok = __all_sync(0xffffffffu, pn_wait(&sh.empty[st], (unsigned) ((c / PN_AST - 1) & 1), sh));
-                            ta_fence_after();
+                        for (int q2 = 0; q2 < PN_KC / 64; ++q2) {
+                            const int Q = PN_KC / 64 * st + q2;
+                            uint32_t o[16];
+                            __half2 f00, f01, f10, f11;
+                            pn_scales(m.x, Q, d0, f00, f01);
+                            pn_scales(m.y, Q, d1, f10, f11);
+                            pn_decode8<WIDE>(w[0][2 * Q], f00, o[0], o[1], o[4], o[5]);
+                            pn_decode8<WIDE>(w[1][2 * Q], f10, o[2], o[3], o[6], o[7]);
+                            pn_decode8<WIDE>(w[0][2 * Q + 1], f01, o[8], o[9], o[12], o[13]);
+                            pn_decode8<WIDE>(w[1][2 * Q + 1], f11, o[10], o[11], o[14], o[15]);
+                            if (q2 == 0) {
+                                if (ok && c >= PN_AST) ok = __all_sync(0xffffffffu, pn_wait(&sh.empty[st], (unsigned) ((c / PN_AST - 1) & 1), sh));
+                                ta_fence_after();
+                            }
+                            pn_st_tile(t_lane + st * PN_KC + q2 * 32, o);
                         }
-                        pn_st_tile(t_lane + st * PN_KC + q2 * 32, o);
+                        ta_wait_st();
+                        ta_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&sh.full[st]);
                     }
-                    ta_wait_st();
-                    ta_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&sh.full[st]);
-                }
+                };
+                if (pn_wide(m.z & (m.z << 1))) decode(std::true_type{});
+                else decode(std::false_type{});
             }
         }
         asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -511,6 +524,7 @@ __global__ void __launch_bounds__(PW_THREADS, 1) k_prompt_few(const PnParams p) 
             if (unit < units) {
                 const uint4 m0 = *reinterpret_cast<const uint4*>(t + NAT_META + g * 16), m1 = *reinterpret_cast<const uint4*>(t + NAT_HALF_BYTES + NAT_META + g * 16);
                 const __half2 dd[2] = {pn_as_h2(m0.z), pn_as_h2(m1.z)};
+                const uint32_t z = (m0.z & (m0.z << 1)) | (m1.z & (m1.z << 1));
 #pragma unroll 1
                 for (int jj = 0; jj < 2; ++jj) {
                     uint4 w[2][2];
@@ -518,29 +532,33 @@ __global__ void __launch_bounds__(PW_THREADS, 1) k_prompt_few(const PnParams p) 
                     for (int hf = 0; hf < 2; ++hf)
 #pragma unroll
                         for (int h = 0; h < 2; ++h) w[hf][h] = *reinterpret_cast<const uint4*>(t + hf * NAT_HALF_BYTES + (2 * h + jj) * 512 + lane * 16);
+                    auto products = [&](auto wide) {
 #pragma unroll
-                    for (int s2 = 0; s2 < 2; ++s2) {
-                        __half2 f[2][2][2];   // [half tile][row half][sub-block]
-#pragma unroll
-                        for (int hf = 0; hf < 2; ++hf) {
-                            pn_scales((hf ? m1.x : m0.x) >> (16 * jj), s2, __low2half2(dd[hf]), f[hf][0][0], f[hf][0][1]);
-                            pn_scales((hf ? m1.y : m0.y) >> (16 * jj), s2, __high2half2(dd[hf]), f[hf][1][0], f[hf][1][1]);
-                        }
-#pragma unroll
-                        for (int e2 = 0; e2 < 2; ++e2) {
-                            const uint4 bv = *reinterpret_cast<const uint4*>(b + (4 * jj + 2 * s2 + e2) * 64);
+                        for (int s2 = 0; s2 < 2; ++s2) {
+                            __half2 f[2][2][2];   // [half tile][row half][sub-block]
 #pragma unroll
                             for (int hf = 0; hf < 2; ++hf) {
-                                const uint32_t wa = s2 ? (e2 ? w[hf][0].w : w[hf][0].z) : (e2 ? w[hf][0].y : w[hf][0].x);
-                                const uint32_t wb = s2 ? (e2 ? w[hf][1].w : w[hf][1].z) : (e2 ? w[hf][1].y : w[hf][1].x);
-                                uint32_t a[4], d[4];
-                                pn_decode8(wa, f[hf][0][e2], a[0], a[1], a[2], a[3]);
-                                pn_decode8(wb, f[hf][1][e2], d[0], d[1], d[2], d[3]);
-                                pw_mma(acc[hf], a[0], d[0], a[1], d[1], bv.x, bv.y);
-                                pw_mma(acc[hf], a[2], d[2], a[3], d[3], bv.z, bv.w);
+                                pn_scales((hf ? m1.x : m0.x) >> (16 * jj), s2, __low2half2(dd[hf]), f[hf][0][0], f[hf][0][1]);
+                                pn_scales((hf ? m1.y : m0.y) >> (16 * jj), s2, __high2half2(dd[hf]), f[hf][1][0], f[hf][1][1]);
+                            }
+#pragma unroll
+                            for (int e2 = 0; e2 < 2; ++e2) {
+                                const uint4 bv = *reinterpret_cast<const uint4*>(b + (4 * jj + 2 * s2 + e2) * 64);
+#pragma unroll
+                                for (int hf = 0; hf < 2; ++hf) {
+                                    const uint32_t wa = s2 ? (e2 ? w[hf][0].w : w[hf][0].z) : (e2 ? w[hf][0].y : w[hf][0].x);
+                                    const uint32_t wb = s2 ? (e2 ? w[hf][1].w : w[hf][1].z) : (e2 ? w[hf][1].y : w[hf][1].x);
+                                    uint32_t a[4], d[4];
+                                    pn_decode8<decltype(wide)::value>(wa, f[hf][0][e2], a[0], a[1], a[2], a[3]);
+                                    pn_decode8<decltype(wide)::value>(wb, f[hf][1][e2], d[0], d[1], d[2], d[3]);
+                                    pw_mma(acc[hf], a[0], d[0], a[1], d[1], bv.x, bv.y);
+                                    pw_mma(acc[hf], a[2], d[2], a[3], d[3], bv.z, bv.w);
+                                }
                             }
                         }
-                    }
+                    };
+                    if (pn_wide(z)) products(std::true_type{});   // (asked behind the loads)
+                    else products(std::false_type{});
                 }
             }
             if (kb == 0) mine = p.order[job.start + min(lane, job.n - 1)];   // (used after the last chunk)

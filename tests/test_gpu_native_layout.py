@@ -162,3 +162,36 @@ def test_a_matrix_asked_for_comes_back_in_the_interchange_layout():
         assert torch.equal(e.tensor("l1.experts_gu", torch.uint8)[7 * per:8 * per], F.iq3s_retile(F.iq3s_quantize(w), gu, cfg.hidden))
     finally:
         e.close()
+
+
+@pytest.mark.parametrize("n", [30, 200])
+def test_scales_past_the_largest_f16(tmp_path, n):
+    """A block scale d (1 + 2 s) that overflows f16, in a file's matrix: a prompt's weights of that block are infinite with the sign of theirs, in
+    both layouts (every value of the normed rows is 1 here, so a row of the values' projection with weights of one sign sums to that infinity)."""
+    from gguf_files import model_meta, tiny_model_tensors, write_gguf
+    cfg = small(n_layer=1, attn_every=1, n_expert=4, top_k=2, vocab=512, max_ctx=512)
+    a = F.Engine(cfg)
+    a.init_synthetic(seed=5, sigma=0.02)
+    tensors = tiny_model_tensors(F, a, cfg)
+    a.close()
+    tensors["token_embd.weight"][7] = 1.0
+    blk = tensors["blk.0.attn_v.weight"][0].reshape(-1, cfg.hidden // 256, 110)
+    for row, signs in ((0, 0x00), (1, 0xFF)):
+        blk[row, :, :2] = np.frombuffer(np.float16(60000).tobytes(), np.uint8)
+        blk[row, :, 74:106] = signs
+        blk[row, :, 106:] = 0xFF
+    path = tmp_path / "huge.gguf"
+    write_gguf(path, model_meta(cfg), tensors)
+    for asked in (False, True):
+        g = F.Gguf(path)
+        e = F.Engine(g.model_config(max_ctx=cfg.max_ctx, max_rows=cfg.max_rows))
+        try:
+            e.load_gguf(g)
+            if asked:
+                e.tensor("l0.w_in", torch.uint8)
+            with pytest.raises(F.FnxError):              # (the logits are not finite)
+                e.prompt([7] * (n + 1))
+            v = e.tensor("l0.v_cache", torch.float16).reshape(-1, cfg.n_kv_head * cfg.head_dim)[:n]
+            assert torch.isposinf(v[:, 0]).all() and torch.isneginf(v[:, 1]).all() and torch.isfinite(v[:, 2:]).all(), asked
+        finally:
+            e.close()
