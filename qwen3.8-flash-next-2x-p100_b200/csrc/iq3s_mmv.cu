@@ -6,7 +6,7 @@
 // kernel k_moe_rows (engine/src/p100_moe_rows.cuh:266-342).  Like the reference it multiplies integer codebook
 // magnitudes by int8 activations and applies the scales afterwards; unlike it
 //   - the weight stream is staged through shared memory by bulk async copies of 1,760-byte tile blocks, each warp
-//     running its own ring of them (mmv_core.cuh), from the tile layout of iq3s_tile.h;
+//     running its own ring of them (mmv_stage.cuh), from the tile layout of iq3s_tile.h;
 //   - the codebook lives in shared memory 32 times, once per bank, so the 9-bit lookups never conflict;
 //   - activations are quantised to two int8 levels per 256-column block (x ~ d (q1 + q2 / 256), error
 //     <= amax / 65024), and both levels of up to 4 rows ride in the 8 columns of one mma.sync.m16n8k32.s8, so a
@@ -78,6 +78,8 @@ static int launch_mmv(const MmvParams& p0, cudaStream_t st) {
     MmvParams p = p0;
     p.upj_inv = mmv_inverse((unsigned) p.rows / 16);
     p.nblk_inv = mmv_inverse((unsigned) sm_count());
+    p.share = (unsigned) (p.rows / 16) / (unsigned) sm_count();
+    p.rest = (unsigned) (p.rows / 16) % (unsigned) sm_count();
     p.R = 6;   // tile blocks in flight per warp: as many as the shared memory left by the codebook and the images holds
     constexpr size_t LIMIT = 227 * 1024;
     while (p.R > 2 && mmv_smem_bytes<NG, MODE>(p.K, p.R, p.njobs_max) > LIMIT) --p.R;

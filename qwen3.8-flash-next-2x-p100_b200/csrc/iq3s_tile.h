@@ -184,10 +184,7 @@ FNX_HD unsigned mmv_div(unsigned n, unsigned d, unsigned inv) {
     const unsigned q = (unsigned) (((uint64_t) n * inv) >> 32);
     return q + (n - q * d >= d ? 1u : 0u);
 }
-// total * bid / nblk, whatever the product's size: the quotient's share, and that of the rest (bid <= nblk < 2^16)
-FNX_HD unsigned mmv_first_unit(unsigned total, unsigned bid, unsigned nblk, unsigned inv) {
-    const unsigned q = mmv_div(total, nblk, inv);
-    return q * bid + mmv_div((total - q * nblk) * bid, nblk, inv);
-}
+// total * bid / nblk of total = share * nblk + rest, whatever that product's size (bid <= nblk < 2^16)
+FNX_HD unsigned mmv_first_unit(unsigned share, unsigned rest, unsigned bid, unsigned nblk, unsigned inv) { return share * bid + mmv_div(rest * bid, nblk, inv); }
 
 }  // namespace fnxb

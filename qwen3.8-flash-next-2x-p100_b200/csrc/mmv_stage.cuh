@@ -44,6 +44,7 @@ struct MmvParams {
     int accumulate;
     int R;      // ring slots per warp
     unsigned upj_inv, nblk_inv;   // mmv_inverse() of the units a job has, of the blocks
+    unsigned share, rest;         // dense: units a block, units left over
     unsigned* err;
     // dense: the rows' image, already built (stage_image_bytes() bytes in the layout of the block's own image): the
     // block copies it instead of quantising x
@@ -195,8 +196,14 @@ __device__ __forceinline__ void stage_run(const MmvParams& p, const StageSmem& S
         __syncthreads();
     }
     stamp();
-    const unsigned upj = p.rows / 16, total = (unsigned) njobs * upj;
-    const int u0 = (int) mmv_first_unit(total, bid, nblk, p.nblk_inv), u1 = (int) mmv_first_unit(total, bid + 1, nblk, p.nblk_inv);
+    const unsigned upj = p.rows / 16;
+    unsigned share = p.share, rest = p.rest;
+    if (MOE) {
+        const unsigned total = (unsigned) njobs * upj;
+        share = mmv_div(total, nblk, p.nblk_inv);
+        rest = total - share * nblk;
+    }
+    const int u0 = (int) mmv_first_unit(share, rest, bid, nblk, p.nblk_inv), u1 = (int) mmv_first_unit(share, rest, bid + 1, nblk, p.nblk_inv);
     auto job_of = [&](int u) { return MOE ? (int) mmv_div(u, upj, p.upj_inv) : 0; };
     const float* norm_w = MODE == MAT_DOWN ? nullptr : p.norm_w;
     uint8_t* slots = S.slots + (size_t) warp * p.R * TILE_BYTES;

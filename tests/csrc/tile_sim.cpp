@@ -133,4 +133,7 @@ extern "C" void sim_roundtrip(const uint8_t* ggml, int rows, int K, uint8_t* bac
             tile_get_block(tiles.data() + ((size_t) (r / 16) * KB + b) * TILE_BYTES, r % 16, back + ((size_t) r * KB + b) * IQ3S_BLOCK_BYTES);
 }
 
-extern "C" unsigned sim_first_unit(unsigned total, unsigned bid, unsigned nblk) { return mmv_first_unit(total, bid, nblk, mmv_inverse(nblk)); }
+extern "C" unsigned sim_first_unit(unsigned total, unsigned bid, unsigned nblk) {
+    const unsigned inv = mmv_inverse(nblk), share = mmv_div(total, nblk, inv);
+    return mmv_first_unit(share, total - share * nblk, bid, nblk, inv);
+}
