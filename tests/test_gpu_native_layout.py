@@ -195,3 +195,41 @@ def test_scales_past_the_largest_f16(tmp_path, n):
             assert torch.isposinf(v[:, 0]).all() and torch.isneginf(v[:, 1]).all() and torch.isfinite(v[:, 2:]).all(), asked
         finally:
             e.close()
+
+
+@pytest.mark.parametrize("n", [48, 200])   # jobs of eight rows and of 64
+def test_scales_that_are_large_but_fit(tmp_path, n):
+    """Experts with a few rows of block scales d of 1,000 (and normed rows small enough for it): the decode's form for large scales, against the
+    interchange layout, key by key as in test_prompt_products_at_the_edges_of_their_jobs."""
+    from gguf_files import model_meta, tiny_model_tensors, write_gguf
+    cfg = small(n_layer=2, attn_every=2, n_expert=32, top_k=2, vocab=512, max_ctx=512)
+    a = F.Engine(cfg)
+    a.init_synthetic(seed=5, sigma=0.02)
+    tensors = tiny_model_tensors(F, a, cfg)
+    a.close()
+    # a large row's block sums at most 1,000 x 15 x (256 x 1,024)^1/2 x 3e-5 = 230 of a normed row of 1,024: silu(gate) x up stays inside f16
+    tensors["blk.0.post_attention_norm.weight"] *= 3e-5
+    for l in range(2):
+        tensors[f"blk.{l}.ffn_gate_inp.weight"][:] = 0.0
+    for name, cols in (("ffn_gate_exps", cfg.hidden), ("ffn_up_exps", cfg.hidden), ("ffn_down_exps", cfg.ffn)):
+        blk = tensors[f"blk.0.{name}.weight"][0].reshape(cfg.n_expert, -1, cols // 256, 110)
+        blk[:, 3::40, 0, :2] = np.frombuffer(np.float16(1000).tobytes(), np.uint8)
+        blk[:, 3::40, 0, 106:] = 0
+    path = tmp_path / "large.gguf"
+    write_gguf(path, model_meta(cfg), tensors)
+    keys = []
+    for asked in (False, True):
+        g = F.Gguf(path)
+        e = F.Engine(g.model_config(max_ctx=cfg.max_ctx, max_rows=cfg.max_rows))
+        try:
+            e.load_gguf(g)
+            if asked:
+                for m in MATRICES[2:]:
+                    e.tensor("l0." + m, torch.uint8)
+            e.prompt(np.random.default_rng(6).integers(0, cfg.vocab, size=n + 1).tolist())
+            assert e.error_bits() == 0
+            keys.append(e.tensor("l1.k_cache", torch.float16).float().reshape(-1, cfg.n_kv_head * cfg.head_dim)[:n].cpu().numpy())
+        finally:
+            e.close()
+    err = np.linalg.norm(keys[0] - keys[1], axis=1) / np.linalg.norm(keys[1], axis=1)
+    assert err.max() < 3 * 2.0 ** -11, (int(err.argmax()), float(err.max()))
