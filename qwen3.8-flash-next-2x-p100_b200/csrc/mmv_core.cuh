@@ -1,4 +1,4 @@
-// The inner pieces of the IQ3_S matrix x few-rows product, shared by the persistent step kernel: codebook table,
+// The inner pieces of the operators' IQ3_S matrix x few-rows product (mmv_stage.cuh): codebook table,
 // one 16 x 256 tile against quantised activation cells, and the two-level int8 quantiser of activation rows.
 //
 // Activation image (in shared or global memory, same layout): rows in groups of four,
@@ -234,7 +234,7 @@ namespace fnxb {
 constexpr int QUANT_BATCH = 3;
 
 struct QuantTask {
-    const float* src;   // the block's 256 values; null: no task
+    const float* src;   // the block's 256 values
     int t, blk;
 };
 

@@ -837,10 +837,12 @@ static int pf_tma_rows() {
     static const int v = []() { const char* e = getenv("FNX_PROMPT_GEMM"); return e && atoi(e) == 0 ? 1 << 30 : 1024; }();
     return v;
 }
-// Which form of the product suits a matrix in the engine's layout: prompt_nat's, which decodes again for every 64 rows (0.8 us a wave of 256
-// features x 64 rows over the SMs and 128 columns), or the matrix to f16 once and gemm_tma's tiles of 256 x 256 (0.55 us a wave and 64
-// columns, the decode 1 us per 2.5 M weights).  12,352 x 2,048: 42 against 46 us at 333 rows, 48 against 46 at 400, 63 against 48 at 600,
-// 90 against 68 at 1,020; 2,048 x 4,096 (8 tiles across only): 55 against 75 us still at 1,020 rows.
+// Which form of the product suits a matrix in the engine's layout: prompt_nat's, which decodes again for every job's rows, or the matrix to f16 once and
+// gemm_tma's tiles.  The rule prices them as jobs of 64 rows (0.8 us a wave of 256 features x 64 rows over the SMs and 128 columns) and tiles of 256 x 256 (0.55
+// us a wave and 64 columns, the decode 1 us per 2.5 M weights); both take fewer rows a block where that fills the SMs (prompt_dense_rows, gt_rows), so they
+// cross a little earlier than it says.  The whole projection, as it goes and once, us.  12,352 x 2,048: 200 rows 35 and 36, 333 rows 39.5 and 37.8 (as it goes is
+// taken), 400 rows 48 and 39, 600 rows 60 and 43, 1,020 rows 89 and 65; 2,048 x 4,096: 333 rows 40 and 46, 600 rows 46.6 and 47.4, 1,020 rows 54 and 51, 1,100 rows
+// 54 and 51 (as it goes is taken), 1,184 rows 66 and 54.
 static bool dense_decodes_as_it_goes(int T, int rows, int K) {
     if (pf_tma_rows() > 1024) return true;
     const long long sms = sm_count(), slabs = (rows + 255) / 256, nat = slabs * ((T + PN_N - 1) / PN_N), tma = slabs * ((T + PF_N - 1) / PF_N);

@@ -147,9 +147,11 @@ __device__ __forceinline__ void nm_flush(uint32_t am, float s0, float s1, const 
 // AccT double (expert modes): the rounded result does not depend on where a row's K-sum was cut, as there.
 // The rows' operands are loaded once for both half tiles.  (Most jobs have one
 // row, two of the eight columns; a form with half of the integer work for them was slower: 52 against 46 us for 205 jobs, the second
-// copy of the code.)  The loop over four sub-blocks stays rolled for three row groups and more (their blocks have an SM to themselves, their rows' image
-// leaves no room for a second one, so a thread has 255 registers: a half tile at a time in 128, with spills, 8 warps waited most of the time: a head of 151,936
-// rows over 20 rows 100 us, 62 now; 12,352 x 2,048 16 and 10.7); the short one is worth unrolling: 50 -> 47 us for 205 jobs.
+// copy of the code.)  The loop over four sub-blocks stays rolled for three row groups and more, where a thread has 255 registers and its block an SM (a half tile at a
+// time in 128, with spills, 8 warps waited most of the time: a head of 151,936 rows over 20 rows 100 us, 62 now; 12,352 x 2,048 16 and 10.7.  The rows' image of the
+// plain form leaves no room for a second block anyway; the split form's, a quarter of the columns, would, but its registers are worth more than a successor
+// that waits there: windows of eight layers with that form in 128 and in 255, 9 rows 675 and 669 us, 12 rows 750 and 746, 16 rows 883 and 863, 32 rows 1,440 and
+// 1,403); the short one is worth unrolling: 50 -> 47 us for 205 jobs.
 template <int NG, typename AccT>
 __device__ __forceinline__ void nm_item(uint32_t tile_s, uint32_t xb, uint32_t x0, uint32_t x1, uint32_t group, int lane, AccT (&acc)[2][NG][4]) {
     const uint32_t a16 = tile_s + lane * 16, am = tile_s + (lane >> 2) * 16;
@@ -526,7 +528,7 @@ __device__ __forceinline__ void nm_body(const NatParams& p, uint8_t* smem) {
     }
 }
 
-// two blocks an SM: the next kernel's may be resident while this one's drain
+// two blocks an SM, up to two row groups (nm_item): the next kernel's may be resident while this one's drain
 template <int NG, int MODE, int NW, int SLOTS>
 __global__ void __launch_bounds__(NW * 32, NW > 12 || NG > 2 ? 1 : 2) k_nat_mmv(const NatParams p) {
     extern __shared__ __align__(128) uint8_t smem[];

@@ -19,7 +19,8 @@
 // the products' N is a job's own rows in sixteens (six rows a job: 178 us with N = 64, 166).  Jobs of 128 rows halve the decode, but leave one
 // accumulator pair, whose results (6 us an item) then lie in the next item's way: 388 us for 512 jobs of 116 rows, 339 for 1,024 of 58.
 // Measured, 512 jobs of gate|up and of down (fourteen items of 256 features x 2,048 columns an SM), us: six rows a job 162 + 92, fifty-eight 179 + 115, 6,144 jobs
-// of 760 rows an expert 1,940 + 1,244 (187 + 101, 200 + 126 and 2,172 + 1,334 with four stages of rows, N = 64 and two instructions a word more).  With neither decode nor
+// of 760 rows an expert 1,940 + 1,244 (187 + 101, 200 + 126 and 2,172 + 1,334 with four stages of rows, N = 64 and two instructions a word more); in a prompt of 333 rows, ten picks
+// a row, 150 + 83 a layer.  With neither decode nor
 // products 128: the hand-over between the decode warps, the weight stages, the rows and the issuing thread, then the decode's instructions (half of the
 // issue slots), are what is left here; DRAM would allow 88.
 #include <type_traits>
@@ -78,7 +79,8 @@ __device__ __forceinline__ uint32_t pn_and_xor(uint32_t a, uint32_t b, uint32_t 
 // (4, 6), (5, 7).  A nibble t at bits 0..3 of a half 0x6400 | .. is 1024 + (t + 8): twice that less 2,064 is 2 t, and one multiply-add makes
 // (2 t + 1) f of it; at bits 4..7 it is 1024 + 16 (t + 8) = 8 (143 + m).  All exact but the one rounding of m f, as in the other forms of these
 // products.  (Thirteen instructions a word; with the low nibbles moved up a bit, so that 1,039 + m was left to subtract, fifteen.)
-// WIDE: the same for scales that may be infinite, where (2 t) f + f would be NaN.
+// WIDE: the same for scales that may be infinite, where (2 t) f + f would be NaN.  A warp asks once a block of 256 columns (pn_wide): with a form of fourteen
+// instructions that holds for all scales, prompts of up to 204 rows took 2 to 3% longer, others 1.5%.
 template <bool WIDE>
 __device__ __forceinline__ void pn_decode8(uint32_t w, __half2 f, uint32_t& o0, uint32_t& o1, uint32_t& o2, uint32_t& o3) {
     const uint32_t s = w >> 8;
@@ -253,7 +255,7 @@ __global__ void __launch_bounds__(PN_THREADS, 1) k_prompt_nat(const PnParams p) 
         asm volatile("cp.async.wait_group 0;" ::: "memory");
     } else if (warp >= PN_W_LOAD && warp < PN_W_LOAD + PN_LOAD) {
         // ---------------------------------------------------------------------------------------- the rows
-        // thread: piece lt % 8 of the rows lt / 8 + 16 j, in both boxes of a stage.  Jobs and entries are loaded an item ahead, and a chunk
+        // thread: piece lt % 8 of the rows lt / 8 + 8 j, in both boxes of a stage.  Jobs and entries are loaded an item ahead, and a chunk
         // is reported before the wait for the next one's stage, so that neither latency lies in the products' way.
         constexpr int RJ = PN_N / (4 * PN_LOAD);
         const int lt = tid - PN_W_LOAD * 32, piece = lt & 7, r0 = lt >> 3;
@@ -425,8 +427,9 @@ __global__ void __launch_bounds__(PN_THREADS, 1) k_prompt_nat(const PnParams p) 
 // operand, so that neither tensor memory nor the waits between its writers and readers are in the way.  Bound by the decode's instructions
 // (integer-logic and half pipes, two cycles each; half of either busy).  An item is a job and 16 tiles of 32 features (gate|up: 16 gate
 // and the 16 up of the same features), a warp each; the job's rows go through three shared-memory chunks of 256 columns, a warp's tiles
-// through two slots of its own.  512 experts' matrices, up to eight rows each: 303 us by k_prompt_nat, 255 here (gate|up + down); two groups of
-// eight rows a job won 1% between four and five rows an expert and lost beyond.
+// through two slots of its own.  A layer's experts of a prompt (512 of them, ten picks a row; job lists, rows' copy
+// and combine included), us: 32, 64, 100, 150 and 204 rows 117, 168, 194, 222 and 257 here, 126, 175, 201, 224 and 243 by k_prompt_nat; two groups of eight rows a
+// job won 1% between four and five rows an expert and lost beyond.
 // The rows' columns lie in fours as (0, 2, 1, 3), the order of a decoded word's pairs.
 constexpr int PW_WARPS = 16, PW_THREADS = PW_WARPS * 32, PW_BST = 3;
 constexpr int PW_N = PROMPT_FEW_ROWS;   // rows of a job: the products' N

@@ -47,8 +47,10 @@ int prompt_nat_rows(const float* x, const float* norm_w, int T, int H, float eps
 // modes 1 and 0 for jobs of up to PROMPT_FEW_ROWS rows
 constexpr int PROMPT_FEW_ROWS = 8;
 int prompt_few(int mode, const PnParams& p, int max_jobs, cudaStream_t st);
-// where those win: up to four rows an expert.  A 12-layer prompt of 512 experts, ten a row: 100 rows 4.23 against 4.50 ms in prompt_nat's jobs of 64,
-// 150 rows 4.84 against 4.99, 200 rows 5.42 against 5.43, 333 rows 6.89 against 6.22
+// where those are taken: up to four rows an expert.  A layer's experts by these and by prompt_nat's jobs of 64, us, 512 experts: ten picks a row, 100 rows 194 and
+// 201, 150 rows 222 and 224, 180 rows 233 and 233, 204 rows (the line) 257 and 243, 333 rows 319 and 261; four picks, 204 rows 180 and 185, 256 rows 199 and
+// 200, 333 rows 220 and 212, 512 rows (the line) 265 and 241.  So they win up to some two and a half to three rows an expert; the line lies where it did for
+// the form of prompt_nat with four stages of rows, which came level at four
 inline bool prompt_few_fits(long long pairs, int E) { return pairs <= 4ll * E; }
 // the rows of a dense product's jobs: fewer, in sixteens, as long as the items of `slabs` x the jobs all run at once (2,048 x 4,096, 332 rows: 30 us with
 // jobs of 64 on 48 SMs, 28 with jobs of 32 on 88; where they would not, 34 us become 52)
