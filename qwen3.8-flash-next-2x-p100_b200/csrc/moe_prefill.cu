@@ -568,7 +568,8 @@ __global__ void __launch_bounds__(256, 4) k_pf_combine(const float* __restrict__
         mine[lane] = pick.weight(e_lo, e_hi);
         __syncwarp();
     }
-    const float gate = add_shared ? sigmoidf_(logits[(size_t) t * (E + 1) + E]) : 0.f;
+    const float lg = add_shared ? logits[(size_t) t * (E + 1) + E] : 0.f;
+    float gate = 0.f;
     float4* o = reinterpret_cast<float4*>(out + (size_t) t * H + i);
     float4 s = make_float4(0.f, 0.f, 0.f, 0.f), old = s;
     if (accumulate) old = *o;
@@ -580,9 +581,12 @@ __global__ void __launch_bounds__(256, 4) k_pf_combine(const float* __restrict__
             const float4* p = reinterpret_cast<const float4*>(part + (a == Kp ? (size_t) T * Kp + t : (size_t) t * Kp + a) * H + i);
             v[k] = a < n && (EVERY || a >= Kp || mine[a] != 0.f) ? __ldcs(p) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
-        if (EVERY && k0 == 0) {   // (behind the loads: a store waits for what it stores)
-            mine[lane] = pick.weight(e_lo, e_hi);
-            __syncwarp();
+        if (k0 == 0) {   // (behind the loads: what needs a value waits for it)
+            gate = sigmoidf_(lg);
+            if (EVERY) {
+                mine[lane] = pick.weight(e_lo, e_hi);
+                __syncwarp();
+            }
         }
 #pragma unroll
         for (int k = 0; k < PC_ADD; ++k) {
