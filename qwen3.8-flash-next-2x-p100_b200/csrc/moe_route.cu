@@ -382,39 +382,41 @@ __global__ void __launch_bounds__(256) k_topk_rows(const float* __restrict__ log
     else rt_topk_row<RT_MAXE / 32>(l, E, K, lane, scr_[warp], topi + (size_t) t * K, nullptr, topw + (size_t) t * K, nullptr);
 }
 
-// Every addend's load leaves at once, whether its pick counts or not (where it does not, nobody wrote the addend: its weight of 0 keeps it out), and a warp's
-// lanes fetch the weights, one each.  Bound by latency; five rows of ten picks 3.8 us a launch where the loads wait for weights that every thread fetches for
-// itself, 2.5 so; 32 rows 4.7 and 3.3 (picks of half of the experts the same).
+// Every load leaves at once: the picks' ids and weights, and every addend whether its pick counts or not (where it does not, nobody wrote the addend: nothing of
+// it enters the sum).  Bound by latency: five rows of ten picks 2.6 us a launch, 3.8 where the addends wait for the weights; 32 rows 3.7 and 4.7; the block of
+// four launches and this one, five rows, 48.5 us (without a look at the ids 48.1).  With the weights by a warp's lanes a launch among its like takes 2.4, but
+// behind a product the block takes 50.5.
 __global__ void k_combine(const float* __restrict__ part, const int* __restrict__ topi, const float* __restrict__ topw,
                           const float* __restrict__ logits, int T, int E, int H, int K, int e_lo, int e_hi, int add_shared,
                           float* __restrict__ out, int accumulate) {
-    __shared__ __align__(16) float weights[8][32];   // the picks', a copy a warp
     pdl_wait();
     pdl_launch_dependents();
-    const int t = blockIdx.y, i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
-    float* mine = weights[threadIdx.x >> 5];
-    const Pick pick(topi + t * K, topw + t * K, K, lane);
-    float w[32], v[32];
-#pragma unroll
-    for (int k = 0; k < 32; ++k) v[k] = k < K && i < H ? part[((size_t) t * K + k) * H + i] : 0.f;
-    mine[lane] = pick.weight(e_lo, e_hi);
-    __syncwarp();
-#pragma unroll
-    for (int k = 0; k < 32; k += 4) {
-        const float4 f = *reinterpret_cast<const float4*>(mine + k);
-        w[k] = f.x; w[k + 1] = f.y; w[k + 2] = f.z; w[k + 3] = f.w;
-    }
+    const int t = blockIdx.y, i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= H) return;
+    float w[32], v[32];
+    int id[32];
+#pragma unroll
+    for (int k = 0; k < 32; ++k) {
+        w[k] = v[k] = 0.f;
+        id[k] = -1;
+        if (k < K) {
+            w[k] = topw[t * K + k];
+            id[k] = topi[t * K + k];
+            v[k] = part[((size_t) t * K + k) * H + i];
+        }
+    }
     const float shv = add_shared ? part[((size_t) T * K + t) * H + i] : 0.f;
     const float shl = add_shared ? logits[(size_t) t * (E + 1) + E] : 0.f;
     float* o = out + (size_t) t * H + i;
     const float prev = accumulate ? *o : 0.f;
+    asm volatile("" ::: "memory");   // (no load behind this)
     // the addends are summed as 2^-32 fixed-point integers: the sum does not depend on their order, so a row's result does not
     // depend on how its picks are split over kernels or expert-parallel ranks
+    const unsigned span = (unsigned) max(e_hi - e_lo, 0);
     unsigned long long s = 0ull;
 #pragma unroll
     for (int k = 0; k < 32; ++k)
-        if (k < K && w[k] != 0.f) s += fix_from_float(w[k] * v[k]);
+        if (k < K && (unsigned) id[k] - (unsigned) e_lo < span && w[k] != 0.f) s += fix_from_float(w[k] * v[k]);
     if (add_shared) s += fix_from_float(sigmoidf_(shl) * shv);
     *o = prev + fix_to_float(s);
 }
