@@ -119,7 +119,8 @@ int fnx_moe_down(const void* Wdn, size_t expert_stride, int e_base, const void* 
                  const int* njobs, int njobs_max, const float* h, int H, int F, float* part, unsigned* err,
                  fnx_stream st);
 /* moe_combine (engine/src/kernels.hpp:83; the cross-card addend of ring_sum :396): out[t] (+)= sum over the picks in
- * [e_lo, e_hi) of topw * part[t K + k], + sigmoid(logits[t][E]) * part[T K + t] when add_shared */
+ * [e_lo, e_hi) of topw * part[t K + k], + sigmoid(logits[t][E]) * part[T K + t] when add_shared.  A pick of weight 0, or whose id lies
+ * outside the range (-1, E: a masked one), adds nothing, whatever its row of part holds */
 int fnx_moe_combine(const float* part, const int* topi, const float* topw, const float* logits, int T, int E, int H,
                     int K, int e_lo, int e_hi, int add_shared, float* out, int accumulate, fnx_stream st);
 /* fnx_moe_combine(part, ..., 0, E, 1, R, 1) that also leaves the image of rmsnorm(R[t]) * img_norm_w for fnx_dense_image
@@ -130,7 +131,8 @@ int fnx_moe_combine_image(const float* part, const int* topi, const float* topw,
 
 /* Prompt-sized MoE block (moe_gate_up_mma / moe_down_mma, engine/src/kernels.hpp:328-330, with the job build of
  * engine/src/prefill.cu:288-377): out[t] (+)= the routed experts in [e_lo, e_hi) and (add_shared) the shared expert of
- * rmsnorm(x[t]) * norm_w, for any number of rows T, given the routing (topi, topw [T][K], logits [T][E + 1]).  The
+ * rmsnorm(x[t]) * norm_w, for any number of rows T, given the routing (topi, topw [T][K], logits [T][E + 1]; picks of weight 0 and ids outside
+ * the range as in fnx_moe_combine).  The
  * (row, pick) pairs are grouped by expert into jobs of up to 256 rows whose products run on the tensor cores
  * (tcgen05.mma, f16 operands decoded from IQ3_S, f32 accumulators in tensor memory).  The job count stays on the device
  * (the grids cover its largest possible value; surplus blocks leave at once).  scratch: fnx_moe_prefill_scratch_bytes(T, K, E, H, F) bytes. */

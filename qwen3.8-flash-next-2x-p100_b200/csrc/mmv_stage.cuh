@@ -12,8 +12,8 @@
 // or multiplications by inverses that the host made (mmv_inverse), the ring's first copies leave from as many lanes, a row's 1 / rms is worked out
 // once a warp, and image rows that hold nothing stay whatever they are (their sums are dropped).  Up to three blocks of rows a warp are quantised
 // together, their loads on the way before the block's first barrier.  Twelve such products of five rows: 157 us with divisions, a lane that issued
-// alone and rows quantised two by two (3,100 instructions a warp, 900 of them items'), 110 now; one MoE block of five rows, its combine's shorter way included, 58.5
-// and 55.4.
+// alone and rows quantised two by two (3,100 instructions a warp, 900 of them items'), 110 now; one MoE block of five rows, its combine's shorter way included, in a
+// graph 52.4 and 48.4.
 #pragma once
 
 #include <type_traits>
