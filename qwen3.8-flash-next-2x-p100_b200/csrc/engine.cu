@@ -999,7 +999,7 @@ static int enqueue_mixer_lanes(fnx_engine* e, const LayerW& L, float* R, int T, 
     const bool mi = L.w_out.nat && d.nv % 2 == 0 && !dp;
     FNX_TRY(gdn_window_lanes(GdnArgs{e->proj, e->proj_ld, e->proj + d.gdn_ch + d.nv * d.hs, e->proj_ld, L.hist_pool, L.convw, L.dt, L.a, L.gnorm, L.S_pool, e->NS, nullptr, e->mix,
                                      mi ? e->img_m : nullptr, d.nk, d.nv, max_lane_rows, e->c.eps},
-                             (size_t) e->NS * 3 * d.gdn_ch, (size_t) e->NS * d.nv * d.hs * d.hs, e->d_cur, lanes, d_row0, n_lanes, max_lane_rows, true, e->st));
+                             (size_t) e->NS * 3 * d.gdn_ch, (size_t) e->NS * d.nv * d.hs * d.hs, e->d_cur, lanes, d_row0, n_lanes, max_lane_rows, T, true, e->st));
     if (dp) FNX_TRY(enqueue_dp_gather(e, d.nv * d.hs, n_lanes, d_row0));
     return enqueue_dense(e, L.w_out, e->mix, d.nv * d.hs, T, nullptr, R, d.H, 1, e->img_m, mi);
 }

@@ -11,6 +11,8 @@
 //     through distributed shared memory, where the reference uses a global scratch buffer and atomic counters.
 #include <cooperative_groups.h>
 
+#include <type_traits>
+
 #include "gdn_core.h"
 #include "nat_image.cuh"
 
@@ -18,7 +20,7 @@ namespace cg = cooperative_groups;
 
 namespace fnxb {
 
-constexpr int GDN_HS = 128, GDN_Q = 4, GDN_QC = GDN_HS / GDN_Q, GDN_THREADS = 2 * GDN_HS + GDN_QC, GDS_THREADS = 128;
+constexpr int GDN_HS = 128, GDN_Q = 4, GDN_QC = GDN_HS / GDN_Q, GDN_THREADS = 256, GDS_THREADS = 128;
 
 // two f32 in a 64-bit register and the packed multiply-add on them (fma.rn.f32x2: each half rounded as the scalar fmaf is, so the
 // products are those of the scalar form, at half the arithmetic instructions)
@@ -40,15 +42,19 @@ __device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
 }
 
 // One block = a quarter (32 columns) of a value head; the four blocks of a head, and with an image the two heads of a 256-column
-// block of it, form a cluster.  288 threads: one per conv channel the block needs (the head's q and k, its own v columns).  Four of the nine
-// warps run the delta rule: a warp holds 8 columns of the state, lane = 8 rg + c: column c, key rows 16 j + 4 rg + i (j < 8, i < 4),
-// so that a row's sums over the key rows are two shuffles inside the warp and nothing in the rows' chain is block-wide, and a warp's
-// 16-byte reads of k and q fall on four different bank groups.  (Eight warps of 4 columns halve the chain's instructions, but their
-// 16-byte pieces of the states' rows cost more than that: 36 us against 25 at 20 rows.)  The starting state, the history and the constants depend on no
-// kernel of this window: they are loaded before the projections are waited for.
-// Bound by latency at a few rows (the loads, the chain, the exchange over the cluster), by the states' 2 MB a row at many; one block
-// barrier a row and every load after the wait before.  (The states' stores by the five other warps, whole lines from a tile in shared memory behind named
-// barriers: 32 us against 25 at 20 rows, 5.8 against 4.8 for one: the block no longer fits beside the projection that drains.)
+// block of it, form a cluster.  Warps 0 .. 3 run the delta rule: a lane holds a column, its warp every fourth group of four key rows, so that a state's rows
+// leave in whole lines; a row's sums over the key rows are exchanged once, behind one barrier of the four warps, and what the row gives out and what the next one
+// takes from the state are summed as the state is updated.  The first four rows' conv and norms are everybody's; warps 4 .. 7 go on with the rest, four
+// rows at a time, ahead of the rule.  The starting state, the history, the constants and a tree's paths depend on no kernel of this window: they are loaded before
+// the projections are waited for.
+// Bound by latency at a few rows (the loads, the chain, the exchange over the cluster); at many by the chain and the states' way out one after the other, 520 cycles a row
+// of 16 KB at an SM's 32 bytes a cycle.  us a launch, 1, 5, 8 and 20 rows and a tree of 20, in the form before (columns eight a warp, sums by shuffles, all of the conv
+// ahead of the rule) and here: 4.5 8.8 11.6 24.6 28.2, 4.3 8.0 10.6 18.7 19.4.  Tried here: the states out of shared memory by tensor copies (20 rows 20 to 23), eight
+// warps for the rule and eight for the conv (19.0), an SM to each block (16 clusters of eight do not fit at once: 35).
+constexpr int GDN_BATCH = 4, GDN_CHANS = 2 * GDN_HS + GDN_QC;
+
+__host__ __device__ __forceinline__ bool gdn_staged(int T, bool tree) { return tree || T > GDN_BATCH; }
+
 template <int CL>
 __device__ __forceinline__ void gdn_body(const GdnArgs& p, int cur, float* sm) {
     cg::cluster_group cluster = cg::this_cluster();
@@ -59,20 +65,20 @@ __device__ __forceinline__ void gdn_body(const GdnArgs& p, int cur, float* sm) {
     float* xq = sm;                              // [T][HS] q after conv and silu (its norm's factor is applied to the sums)
     float* xk = xq + (size_t) T * GDN_HS;        // [T][HS]
     float* vs = xk + (size_t) T * GDN_HS;        // [T][QC]
-    float* os = vs + (size_t) T * GDN_QC;        // [T][QC] the rows' outputs
-    float* gates = os + (size_t) T * GDN_QC;     // [T][2]
+    float* os = vs + (size_t) T * GDN_QC;        // [T][4][QC] the rows' outputs, a warp's key rows each
+    float* ug = os + (size_t) 4 * T * GDN_QC;    // [T][QC] their gates' inputs
+    float* sk = ug + (size_t) T * GDN_QC;        // [2][4][QC] S' k of the row that is next, a warp's key rows each
+    float* gates = sk + 8 * GDN_QC;              // [T][2]
     float* fac = gates + 2 * T;                  // [T][2] 1 / |q|, 1 / |k|
     float* osum = fac + 2 * T;                   // [T][2] this block's square sums and maxima (read by the cluster)
-    float* gath = osum + 2 * T;                  // [T][2 CL] the blocks' square sums and maxima
-    float* xin = gath + 2 * CL * T;              // trees: [T + 3][2 HS + QC] conv inputs
-    constexpr int NC = GDN_THREADS;
-    int* anc = reinterpret_cast<int*>(xin + (size_t) (T + 3) * NC);   // trees: [T][3]
+    float* xin = gates + ((6 * T + 3) & ~3);     // staged inputs: [T + 3][channels], rows 0..2 = the starting history (oldest first), row 3 + t = row t
+    int* anc = reinterpret_cast<int*>(xin + (size_t) (T + 3) * GDN_CHANS);   // trees: [T][4] the last three rows before each on its path, as rows of xin
     auto slot_of = [&](int t) {   // the ring slot of row t's result (cur + 1 + t < 2 NS)
         const int v = cur + 1 + t;
         return v >= NS ? v - NS : v;
     };
-    const int cc = (warp & 3) * 8 + (lane & 7), rg = lane >> 3;
-    const size_t soff = (size_t) lv * GDN_HS * GDN_HS + (size_t) (4 * rg) * GDN_HS + qq * GDN_QC + cc;
+    const int rg = warp & 3;
+    const size_t soff = (size_t) lv * GDN_HS * GDN_HS + (size_t) (4 * rg) * GDN_HS + qq * GDN_QC + lane;
     uint64_t s[16];   // pairs of key rows: s[2 j + h] = rows 16 j + 4 rg + 2 h, + 1
     auto load_state = [&](int slot) {
         const float* src = p.S_pool + (size_t) slot * ssz + soff;
@@ -82,27 +88,63 @@ __device__ __forceinline__ void gdn_body(const GdnArgs& p, int cur, float* sm) {
             for (int h = 0; h < 2; ++h) s[2 * j + h] = f2_pack(src[(size_t) (16 * j + 2 * h) * GDN_HS], src[(size_t) (16 * j + 2 * h + 1) * GDN_HS]);
     };
     if (warp < 4) load_state(cur);
-    // this thread's channel: q, k or v element
-    const int part = tid < GDN_HS ? 0 : tid < 2 * GDN_HS ? 1 : 2, el = part < 2 ? tid - part * GDN_HS : tid - 2 * GDN_HS;
-    const int c = part == 0 ? kh * GDN_HS + el : part == 1 ? p.nk * GDN_HS + kh * GDN_HS + el : 2 * p.nk * GDN_HS + lv * GDN_HS + qq * GDN_QC + el;
+    // the thread's channel: an element of q (warps 0 .. 3) or k; warp 4 has the v columns besides
+    const int el = tid & (GDN_HS - 1);
+    const int cA = (tid < GDN_HS ? 0 : p.nk * GDN_HS) + kh * GDN_HS + el, cQ = kh * GDN_HS + el, cV = 2 * p.nk * GDN_HS + lv * GDN_HS + qq * GDN_QC + lane;
     const float* hin = p.hist_pool + (size_t) cur * hsz;
-    const float4 cw = *reinterpret_cast<const float4*>(p.convw + c * 4);
-    float h0 = hin[c], h1 = hin[ch + c], h2 = hin[2 * ch + c];
+    const float4 wA = *reinterpret_cast<const float4*>(p.convw + cA * 4);
+    float a0 = hin[cA], a1 = hin[ch + cA], a2 = hin[2 * ch + cA];
+    float4 wV = make_float4(0.f, 0.f, 0.f, 0.f);
+    float v0 = 0.f, v1 = 0.f, v2 = 0.f;
+    if (warp == 4) {
+        wV = *reinterpret_cast<const float4*>(p.convw + cV * 4);
+        v0 = hin[cV];
+        v1 = hin[ch + cV];
+        v2 = hin[2 * ch + cV];
+    }
     const float dtv = p.dt[lv], av = p.a[lv], nwv = p.nw[qq * GDN_QC + lane];
+    if (p.parent) {
+        if (tid < T) {
+            int a = tid;
+            for (int k = 0; k < 3; ++k) {
+                if (a >= 0) a = p.parent[a];
+                else --a;                  // a = -1 - (rows past the root)
+                anc[tid * 4 + k] = 3 + a;  // -1 -> row 2 (newest history), -2 -> row 1, -3 -> row 0
+            }
+        }
+        __syncthreads();
+    }
     pdl_wait();   // from here on: the projections
     pdl_launch_dependents();
-    if (tid >= NC - 32 && lane < T) {
+    auto copy4 = [](float* dst, const float* src) { asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory"); };
+    float xA[GDN_BATCH], xV[GDN_BATCH];
+#pragma unroll
+    for (int i = 0; i < GDN_BATCH; ++i) {
+        xA[i] = i < T ? p.qkvz[(size_t) i * p.stride + cA] : 0.f;
+        xV[i] = i < T && warp == 4 ? p.qkvz[(size_t) i * p.stride + cV] : 0.f;
+    }
+    if (warp == 7 && lane < T) {
         const float* abt = p.ab + (size_t) lane * p.ldab;
         const float x = abt[lv] + dtv, be = abt[p.nv + lv];
         gates[2 * lane] = expf((x > 20.0f ? x : log1pf(expf(x))) * av);
         gates[2 * lane + 1] = 1.0f / (1.0f + expf(-be));
     }
-    const bool writes = part == 2 || (lv < p.nk && qq == 0);   // one block per channel writes its history
-    float* xout = part == 0 ? xq + el : part == 1 ? xk + el : vs + el;
-    const int xstr = part < 2 ? GDN_HS : GDN_QC;
-    auto put = [&](int t, float x3, float x2, float x1, float x0) {
-        const float x = cw.x * x3 + cw.y * x2 + cw.z * x1 + cw.w * x0;
-        xout[t * xstr] = x / (1.0f + expf(-x));
+    if (warp >= 4)   // the rows after the first batch
+        for (int t = GDN_BATCH; t < T; ++t) {
+            const float* src = p.qkvz + (size_t) t * p.stride;
+            float* dst = xin + (size_t) (3 + t) * GDN_CHANS;
+            copy4(dst + el, src + cQ);
+            copy4(dst + tid, src + cA);
+            if (warp == 4) copy4(dst + 2 * GDN_HS + lane, src + cV);
+        }
+    for (int t = warp; t < T; t += GDN_THREADS / 32) copy4(ug + t * GDN_QC + lane, p.qkvz + (size_t) t * p.stride + ch + lv * GDN_HS + qq * GDN_QC + lane);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    // (one block per channel writes its history)
+    const bool own = lv < p.nk && qq == 0;
+    // (the products in the order that the compiler gave them when it chose: a row's bits stay what they were)
+    auto put = [&](int t, const float4& w, float* out, int c, bool writes, float x3, float x2, float x1, float x0) {
+        const float x = fmaf(w.w, x0, fmaf(w.z, x1, fmaf(w.x, x3, w.y * x2)));
+        *out = x / (1.0f + expf(-x));
         if (writes) {
             float* hout = p.hist_pool + (size_t) slot_of(t) * hsz + c;
             hout[0] = x2;
@@ -110,174 +152,243 @@ __device__ __forceinline__ void gdn_body(const GdnArgs& p, int cur, float* sm) {
             hout[2 * ch] = x0;
         }
     };
-    const float* src = p.qkvz + c;
-    if (!p.parent) {   // a chain: the channel's inputs pass through registers, eight rows' loads in flight
-        for (int t0 = 0; t0 < T; t0 += 8) {
-            float x[8];
+    auto put_path = [&](int t, const float4& w, float* out, int c, bool writes, const float* col) {   // from staged inputs
+        int4 at = make_int4(t + 2, t + 1, t, 0);
+        if (p.parent) at = *reinterpret_cast<const int4*>(anc + t * 4);
+        put(t, w, out, c, writes, col[at.z * GDN_CHANS], col[at.y * GDN_CHANS], col[at.x * GDN_CHANS], col[(3 + t) * GDN_CHANS]);
+    };
+    if (gdn_staged(T, p.parent != nullptr)) {   // (a thread's own columns: read back by itself, and by the others behind the barrier below)
+        float* col = xin + tid;
+        col[0] = a0;
+        col[GDN_CHANS] = a1;
+        col[2 * GDN_CHANS] = a2;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) x[i] = t0 + i < T ? src[(size_t) (t0 + i) * p.stride] : 0.f;
+        for (int i = 0; i < GDN_BATCH; ++i)
+            if (i < T) col[(3 + i) * GDN_CHANS] = xA[i];
+        if (warp == 4) {
+            col = xin + 2 * GDN_HS + lane;
+            col[0] = v0;
+            col[GDN_CHANS] = v1;
+            col[2 * GDN_CHANS] = v2;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                if (t0 + i >= T) break;
-                put(t0 + i, h0, h1, h2, x[i]);
-                h0 = h1;
-                h1 = h2;
-                h2 = x[i];
+            for (int i = 0; i < GDN_BATCH; ++i)
+                if (i < T) col[(3 + i) * GDN_CHANS] = xV[i];
+        }
+    }
+    float* outA = (tid < GDN_HS ? xq : xk) + el;
+    if (p.parent) {
+#pragma unroll 2
+        for (int t = 0; t < min(T, GDN_BATCH); ++t) {
+            put_path(t, wA, outA + t * GDN_HS, cA, own, xin + tid);
+            if (warp == 4) put_path(t, wV, vs + t * GDN_QC + lane, cV, true, xin + 2 * GDN_HS + lane);
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < GDN_BATCH; ++i) {
+            if (i >= T) break;
+            put(i, wA, outA + i * GDN_HS, cA, own, a0, a1, a2, xA[i]);
+            a0 = a1;
+            a1 = a2;
+            a2 = xA[i];
+            if (warp == 4) {
+                put(i, wV, vs + i * GDN_QC + lane, cV, true, v0, v1, v2, xV[i]);
+                v0 = v1;
+                v1 = v2;
+                v2 = xV[i];
             }
         }
-    } else {   // a tree: the inputs staged, rows 0..2 = the starting history (oldest first), row 3 + t = window row t
-        xin[tid] = h0;
-        xin[NC + tid] = h1;
-        xin[2 * NC + tid] = h2;
-        for (int t0 = 0; t0 < T; t0 += 16) {
-            float x[16];
+    }
+    // the L2 norms of n rows' q and k by w of nw warps: eight lanes a vector, four 16-byte pieces a lane
+    auto norms = [&](int r0, int n, int w, int nw) {
+        for (int i0 = 4 * w; i0 < 2 * n; i0 += 4 * nw) {
+            const int i = min(i0 + (lane >> 3), 2 * n - 1), row = r0 + (i >> 1);
+            const float* v = (i & 1 ? xk : xq) + row * GDN_HS + (lane & 7) * 4;
+            float ss[4];
 #pragma unroll
-            for (int i = 0; i < 16; ++i) x[i] = t0 + i < T ? src[(size_t) (t0 + i) * p.stride] : 0.f;
-#pragma unroll
-            for (int i = 0; i < 16; ++i)
-                if (t0 + i < T) xin[(size_t) (3 + t0 + i) * NC + tid] = x[i];
-        }
-        // the three rows before each window row on its path, as rows of xin (past the root: the history)
-        if (tid < T) {
-            int a = tid;
-            for (int k = 1; k <= 3; ++k) {
-                if (a >= 0) a = p.parent[a];
-                else --a;                      // a = -1 - (rows past the root)
-                anc[tid * 3 + k - 1] = 3 + a;  // -1 -> row 2 (newest history), -2 -> row 1, -3 -> row 0
+            for (int k = 0; k < 4; ++k) {
+                const float4 x = *reinterpret_cast<const float4*>(v + 32 * k);
+                ss[k] = (x.x * x.x + x.y * x.y) + (x.z * x.z + x.w * x.w);
             }
+            float sum = (ss[0] + ss[2]) + (ss[1] + ss[3]);
+#pragma unroll
+            for (int o = 4; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            if ((lane & 7) == 0) fac[2 * row + (i & 1)] = rsqrtf(sum + 1e-6f);
         }
-        __syncthreads();
-        for (int t = 0; t < T; ++t) put(t, xin[anc[t * 3 + 2] * NC + tid], xin[anc[t * 3 + 1] * NC + tid], xin[anc[t * 3] * NC + tid], xin[(3 + t) * NC + tid]);
-    }
+    };
     __syncthreads();
-    // ---- the L2 norms of q and k: a warp per (row, vector)
-    for (int i = warp; i < 2 * T; i += NC / 32) {
-        const float4 v = *reinterpret_cast<const float4*>((i & 1 ? xk : xq) + (i >> 1) * GDN_HS + lane * 4);
-        const float ss = warp_sum((v.x * v.x + v.y * v.y) + (v.z * v.z + v.w * v.w));
-        if (lane == 0) fac[i] = rsqrtf(ss + 1e-6f);
-    }
-    __syncthreads();
-    // ---- the delta rule
     if (warp < 4) {
-        int have = -1;   // the row whose result the registers hold (-1: the starting state)
-        const float scale = rsqrtf((float) GDN_HS);
+        // ---- the delta rule.  A row's output and the next row's S' k are sums over the same state: both are taken as it is updated.
+        norms(0, min(T, GDN_BATCH), 0, 1);   // (each of the four warps for itself: the same values)
+        __syncwarp();
+        uint64_t ak[4], aq[4];   // sums in pairs
+        auto zero = [](uint64_t (&a)[4]) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) a[i] = 0ull;
+        };
+        auto total = [](const uint64_t (&a)[4]) {
+            float a0, a1, a2, a3, a4, a5, a6, a7;
+            f2_unpack(a[0], a0, a1);
+            f2_unpack(a[1], a2, a3);
+            f2_unpack(a[2], a4, a5);
+            f2_unpack(a[3], a6, a7);
+            return ((a0 + a1) + (a2 + a3)) + ((a4 + a5) + (a6 + a7));
+        };
+        auto sums_with = [&](const float* k) {
+            zero(ak);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const ulonglong2 k2 = *reinterpret_cast<const ulonglong2*>(k + 16 * j);
+                ak[(2 * j) & 3] = f2_fma(s[2 * j], k2.x, ak[(2 * j) & 3]);
+                ak[(2 * j + 1) & 3] = f2_fma(s[2 * j + 1], k2.y, ak[(2 * j + 1) & 3]);
+            }
+        };
+        const float* kt = xk + 4 * rg;
+        const float* qt = xq + 4 * rg;
+        if (p.parent && p.parent[0] >= 0) load_state(slot_of(p.parent[0]));
+        sums_with(kt);
+        sk[rg * GDN_QC + lane] = total(ak);
 #pragma unroll 1
         for (int t = 0; t < T; ++t) {
-            if (p.parent) {
-                const int par = p.parent[t];
-                if (par != have) load_state(par < 0 ? cur : slot_of(par));
-            }
-            const float gv = gates[2 * t], bv = gates[2 * t + 1], fq = fac[2 * t], fk = fac[2 * t + 1];
-            const float* kt = xk + t * GDN_HS + 4 * rg;
-            const float* qt = xq + t * GDN_HS + 4 * rg;
-            uint64_t kp[16], acc[4];
+            const bool last = t + 1 == T;
+            if (!last && (t + 1) % GDN_BATCH == 0) asm volatile("bar.sync %0, %1;" ::"r"(2 + (t + 1) / GDN_BATCH), "n"(GDN_THREADS) : "memory");   // the next batch is ready
+            const float gv = gates[2 * t], bv = gates[2 * t + 1], fk = fac[2 * t + 1], v = vs[t * GDN_QC + lane];
+            const float* sums = sk + (t & 1) * 4 * GDN_QC + lane;
+            const float* kn = last ? kt : kt + GDN_HS;   // (the last row's sums with its own k are dropped)
+            // k, q and the next k are loaded two steps ahead, before the stores that the compiler would keep them behind
+            constexpr int AHEAD = 2;
+            ulonglong2 k1[AHEAD], q1[AHEAD], n1[AHEAD];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) acc[i] = 0ull;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const ulonglong2 k2 = *reinterpret_cast<const ulonglong2*>(kt + 16 * j);
-                kp[2 * j] = k2.x;
-                kp[2 * j + 1] = k2.y;
-                acc[(2 * j) & 3] = f2_fma(s[2 * j], k2.x, acc[(2 * j) & 3]);
-                acc[(2 * j + 1) & 3] = f2_fma(s[2 * j + 1], k2.y, acc[(2 * j + 1) & 3]);
+            for (int j = 0; j < AHEAD; ++j) {
+                k1[j] = *reinterpret_cast<const ulonglong2*>(kt + 16 * j);
+                q1[j] = *reinterpret_cast<const ulonglong2*>(qt + 16 * j);
+                n1[j] = *reinterpret_cast<const ulonglong2*>(kn + 16 * j);
             }
-            float a0, a1, a2, a3, a4, a5, a6, a7;
-            f2_unpack(acc[0], a0, a1);
-            f2_unpack(acc[1], a2, a3);
-            f2_unpack(acc[2], a4, a5);
-            f2_unpack(acc[3], a6, a7);
-            float kv = ((a0 + a1) + (a2 + a3)) + ((a4 + a5) + (a6 + a7));
-            kv += __shfl_xor_sync(0xffffffffu, kv, 8);
-            kv += __shfl_xor_sync(0xffffffffu, kv, 16);
-            const float dk = (vs[t * GDN_QC + cc] - gv * (kv * fk)) * bv * fk;
+            const int par = p.parent && !last ? anc[4 * t + 4] - 3 : t;
+            asm volatile("bar.sync 1, 128;" ::: "memory");
+            const float kv = (sums[0] + sums[GDN_QC]) + (sums[2 * GDN_QC] + sums[3 * GDN_QC]);
+            const float dk = (v - gv * (kv * fk)) * bv * fk;
             const uint64_t d2 = f2_pack(dk, dk), g2 = f2_pack(gv, gv);
             float* dst = p.S_pool + (size_t) slot_of(t) * ssz + soff;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) acc[i] = 0ull;
+            zero(ak);
+            zero(aq);
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-                const ulonglong2 q2 = *reinterpret_cast<const ulonglong2*>(qt + 16 * j);
+                const ulonglong2 k = k1[j % AHEAD], q = q1[j % AHEAD], n = n1[j % AHEAD];
+                if (j + AHEAD < 8) {
+                    k1[j % AHEAD] = *reinterpret_cast<const ulonglong2*>(kt + 16 * (j + AHEAD));
+                    q1[j % AHEAD] = *reinterpret_cast<const ulonglong2*>(qt + 16 * (j + AHEAD));
+                    n1[j % AHEAD] = *reinterpret_cast<const ulonglong2*>(kn + 16 * (j + AHEAD));
+                }
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const int i = 2 * j + h;
-                    s[i] = f2_fma(kp[i], d2, f2_mul(g2, s[i]));
-                    acc[i & 3] = f2_fma(s[i], h ? q2.y : q2.x, acc[i & 3]);
+                    s[i] = f2_fma(h ? k.y : k.x, d2, f2_mul(g2, s[i]));
+                    aq[i & 3] = f2_fma(s[i], h ? q.y : q.x, aq[i & 3]);
+                    ak[i & 3] = f2_fma(s[i], h ? n.y : n.x, ak[i & 3]);
                     float lo, hi;
                     f2_unpack(s[i], lo, hi);
-                    dst[(size_t) (16 * j + 2 * h) * GDN_HS] = lo;
-                    dst[(size_t) (16 * j + 2 * h + 1) * GDN_HS] = hi;
+                    dst[(16 * j + 2 * h) * GDN_HS] = lo;
+                    dst[(16 * j + 2 * h + 1) * GDN_HS] = hi;
                 }
             }
-            f2_unpack(acc[0], a0, a1);
-            f2_unpack(acc[1], a2, a3);
-            f2_unpack(acc[2], a4, a5);
-            f2_unpack(acc[3], a6, a7);
-            float at = ((a0 + a1) + (a2 + a3)) + ((a4 + a5) + (a6 + a7));
-            at += __shfl_xor_sync(0xffffffffu, at, 8);
-            at += __shfl_xor_sync(0xffffffffu, at, 16);
-            if (rg == 0) os[t * GDN_QC + cc] = at * fq * scale;
-            have = t;
-        }
-    }
-    // the gate inputs of the warp's output rows (warp, warp + 9, ...), fetched while the rule runs
-    constexpr int OR = (FNX_MAX_ROWS + NC / 32 - 1) / (NC / 32);
-    float u[OR];
-#pragma unroll
-    for (int j = 0; j < OR; ++j) {
-        const int t = warp + j * (NC / 32);
-        u[j] = t < T ? p.qkvz[(size_t) t * p.stride + ch + lv * GDN_HS + qq * GDN_QC + lane] : 0.f;
-    }
-    __syncthreads();
-    // ---- the outputs times their norm weight and gate; their square sums and maxima
-#pragma unroll
-    for (int j = 0; j < OR; ++j) {
-        const int t = warp + j * (NC / 32);
-        if (t >= T) break;
-        const float o = os[t * GDN_QC + lane];
-        u[j] = o * nwv / (1.0f + expf(-u[j]));
-        const float sq = warp_sum(o * o), mx = CL > GDN_Q ? warp_max(fabsf(u[j])) : 0.f;
-        if (lane == 0) *reinterpret_cast<float2*>(osum + 2 * t) = make_float2(sq, mx);
-    }
-    cluster.sync();
-    for (int i = tid; i < T * CL; i += NC) {   // every block's, one remote read per thread
-        const int t = i / CL, r = i % CL;
-        const float2 v = *reinterpret_cast<const float2*>(cluster.map_shared_rank(osum, r) + 2 * t);
-        gath[t * 2 * CL + r] = v.x;
-        gath[t * 2 * CL + CL + r] = v.y;
-    }
-    __syncthreads();
-    const int hb = CL > GDN_Q ? (lv & 1) * GDN_Q : 0;   // the head's blocks in the cluster
-#pragma unroll
-    for (int j = 0; j < OR; ++j) {
-        const int t = warp + j * (NC / 32);
-        if (t >= T) break;
-        const float* gt = gath + t * 2 * CL;
-        const float r = rsqrtf(((gt[hb] + gt[hb + 1]) + (gt[hb + 2] + gt[hb + 3])) / (float) GDN_HS + p.eps), yv = u[j] * r;
-        p.y[(size_t) t * p.nv * GDN_HS + lv * GDN_HS + qq * GDN_QC + lane] = yv;
-        if (CL > GDN_Q) {   // the image: the block's 32 columns are a sub-block of it, eight lanes a cell of each level
-            const int ob = GDN_Q - hb;
-            const float ro = rsqrtf(((gt[ob] + gt[ob + 1]) + (gt[ob + 2] + gt[ob + 3])) / (float) GDN_HS + p.eps);
-            const float* gm = gt + CL;
-            const float am = fmaxf(fmaxf(fmaxf(gm[hb], gm[hb + 1]), fmaxf(gm[hb + 2], gm[hb + 3])) * r, fmaxf(fmaxf(gm[ob], gm[ob + 1]), fmaxf(gm[ob + 2], gm[ob + 3])) * ro);
-            uint32_t w1, w2;
-            float d;
-            ni_code(yv, am, w1, w2, d);
-            w1 <<= 8 * (lane & 3);
-            w2 <<= 8 * (lane & 3);
-#pragma unroll
-            for (int o = 1; o < 4; o <<= 1) {
-                w1 |= __shfl_xor_sync(0xffffffffu, w1, o);
-                w2 |= __shfl_xor_sync(0xffffffffu, w2, o);
+            if (par != t) {   // a tree: the next row leaves from another row's state
+                load_state(par < 0 ? cur : slot_of(par));
+                sums_with(kn);
             }
-            const int KB = p.nv * GDN_HS / 256, sb = (lv & 1) * 4 + qq;
-            uint8_t* rec = p.img + (size_t) t * ni_row_bytes(KB) + (size_t) (lv >> 1) * NI_BYTES;
-            uint8_t* cell = rec + (sb >> 1) * 64 + (lane >> 3) * 16 + (sb & 1) * 8 + (lane & 4);
-            if ((lane & 3) == 0) *reinterpret_cast<uint32_t*>(cell) = w1;
-            if ((lane & 3) == 1) *reinterpret_cast<uint32_t*>(cell + 256) = w2;
-            if (sb == 0 && lane == 2) *reinterpret_cast<float4*>(rec + NI_SCALE) = make_float4(d, d * (1.0f / 256.0f), 0.f, 0.f);
+            sk[((t + 1) & 1) * 4 * GDN_QC + rg * GDN_QC + lane] = total(ak);
+            os[(t * 4 + rg) * GDN_QC + lane] = total(aq);
+            kt += GDN_HS;
+            qt += GDN_HS;
+        }
+    } else if (T > GDN_BATCH) {
+        // ---- the batches after the first, ahead of the rule
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        const float4 wQ = *reinterpret_cast<const float4*>(p.convw + cQ * 4);
+#pragma unroll 1
+        for (int t0 = GDN_BATCH; t0 < T; t0 += GDN_BATCH) {
+#pragma unroll 1
+            for (int t = t0; t < min(T, t0 + GDN_BATCH); ++t) {   // (rolled: the rule's loop runs beside it)
+                put_path(t, wA, xk + t * GDN_HS + el, cA, own, xin + tid);
+                put_path(t, wQ, xq + t * GDN_HS + el, cQ, own, xin + el);
+                if (warp == 4) put_path(t, wV, vs + t * GDN_QC + lane, cV, true, xin + 2 * GDN_HS + lane);
+            }
+            asm volatile("bar.sync 2, 128;" ::: "memory");
+            norms(t0, min(GDN_BATCH, T - t0), 7 - warp, 4);
+            asm volatile("bar.arrive %0, %1;" ::"r"(2 + t0 / GDN_BATCH), "n"(GDN_THREADS) : "memory");
         }
     }
-    cluster.sync();   // no block may leave while a neighbour still reads its shared memory
+    asm volatile("cp.async.wait_group 0;" ::: "memory");   // (a thread reads the gate inputs that it copied)
+    __syncthreads();
+    // ---- the outputs times their norm weight and gate, their square sums and maxima, and the cluster's: row warp + 8 j
+    auto results = [&](auto rows) {
+        constexpr int N = decltype(rows)::value;
+        const float scale = rsqrtf((float) GDN_HS);
+        float u[N];
+        float2 g[N];
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            const int t = min(warp + 8 * j, T - 1);
+            const float* ot = os + 4 * t * GDN_QC + lane;
+            const float o = ((ot[0] + ot[GDN_QC]) + (ot[2 * GDN_QC] + ot[3 * GDN_QC])) * fac[2 * t] * scale;
+            u[j] = o * nwv / (1.0f + expf(-ug[t * GDN_QC + lane]));
+            g[j] = make_float2(o * o, fabsf(u[j]));
+        }
+#pragma unroll
+        for (int d = 16; d; d >>= 1)
+#pragma unroll
+            for (int j = 0; j < N; ++j) {
+                g[j].x += __shfl_xor_sync(0xffffffffu, g[j].x, d);
+                if (CL > GDN_Q) g[j].y = fmaxf(g[j].y, __shfl_xor_sync(0xffffffffu, g[j].y, d));
+            }
+#pragma unroll
+        for (int j = 0; j < N; ++j)
+            if (lane == 0 && warp + 8 * j < T) *reinterpret_cast<float2*>(osum + 2 * (warp + 8 * j)) = g[j];
+        cluster.sync();
+        // every block's sums of the warp's rows, a lane each: lanes [0, 4) and [4, 8) one head's
+#pragma unroll
+        for (int j = 0; j < N; ++j) g[j] = *reinterpret_cast<const float2*>(cluster.map_shared_rank(osum, lane % CL) + 2 * min(warp + 8 * j, T - 1));
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            g[j].x += __shfl_xor_sync(0xffffffffu, g[j].x, 1);
+            g[j].x += __shfl_xor_sync(0xffffffffu, g[j].x, 2);
+            g[j].x = rsqrtf(g[j].x / (float) GDN_HS + p.eps);
+            if (CL > GDN_Q) {
+                g[j].y = fmaxf(g[j].y, __shfl_xor_sync(0xffffffffu, g[j].y, 1));
+                g[j].y = fmaxf(g[j].y, __shfl_xor_sync(0xffffffffu, g[j].y, 2)) * g[j].x;
+                g[j].y = fmaxf(g[j].y, __shfl_xor_sync(0xffffffffu, g[j].y, 4));
+            }
+        }
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // (the neighbours' shared memory is read)
+        const int hb = CL > GDN_Q ? (lv & 1) * GDN_Q : 0;   // the head's blocks in the cluster
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            const int t = warp + 8 * j;
+            const float yv = u[j] * __shfl_sync(0xffffffffu, g[j].x, hb);
+            if (t >= T) break;
+            p.y[(size_t) t * p.nv * GDN_HS + lv * GDN_HS + qq * GDN_QC + lane] = yv;
+            if (CL > GDN_Q) {   // the image: the block's 32 columns are a sub-block of it, eight lanes a cell of each level
+                uint32_t w1, w2;
+                float d;
+                ni_code(yv, g[j].y, w1, w2, d);
+                w1 <<= 8 * (lane & 3);
+                w2 <<= 8 * (lane & 3);
+#pragma unroll
+                for (int o = 1; o < 4; o <<= 1) {
+                    w1 |= __shfl_xor_sync(0xffffffffu, w1, o);
+                    w2 |= __shfl_xor_sync(0xffffffffu, w2, o);
+                }
+                const int KB = p.nv * GDN_HS / 256, sb = (lv & 1) * 4 + qq;
+                uint8_t* rec = p.img + (size_t) t * ni_row_bytes(KB) + (size_t) (lv >> 1) * NI_BYTES;
+                uint8_t* cell = rec + (sb >> 1) * 64 + (lane >> 3) * 16 + (sb & 1) * 8 + (lane & 4);
+                if ((lane & 3) == 0) *reinterpret_cast<uint32_t*>(cell) = w1;
+                if ((lane & 3) == 1) *reinterpret_cast<uint32_t*>(cell + 256) = w2;
+                if (sb == 0 && lane == 2) *reinterpret_cast<float4*>(rec + NI_SCALE) = make_float4(d, d * (1.0f / 256.0f), 0.f, 0.f);
+            }
+        }
+    };
+    if (T <= 8) results(std::integral_constant<int, 1>{});
+    else results(std::integral_constant<int, FNX_MAX_ROWS / 8>{});
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");   // no block may leave while a neighbour still reads its shared memory
 }
 
 template <int CL>
@@ -652,26 +763,38 @@ __global__ void __launch_bounds__(GDP_THREADS) k_gdn_post(const float* __restric
     }
 }
 
-static size_t gdn_smem_bytes(int T, int CL, bool tree) {
-    return sizeof(float) * ((size_t) 2 * T * GDN_HS + (size_t) 2 * T * GDN_QC + 6 * T + 2 * CL * T + (tree ? (size_t) (T + 3) * (2 * GDN_HS + GDN_QC) + 3 * T : 0));
+static size_t gdn_smem_bytes(int T, bool tree) {
+    return sizeof(float) * ((size_t) 2 * T * GDN_HS + (size_t) 6 * T * GDN_QC + 8 * GDN_QC + ((6 * T + 3) & ~3) +
+                            (gdn_staged(T, tree) ? (size_t) (T + 3) * GDN_CHANS + 4 * T : 0));
 }
+constexpr int GDN_SMEM = 112 * 1024;
 
-// an image needs the two heads of its 256-column blocks in one cluster
-int gdn_window(const GdnArgs& p, const int* cur, bool early, cudaStream_t st) {
-    const int CL = p.img ? 2 * GDN_Q : GDN_Q;
+// An image needs the two heads of its 256-column blocks in one cluster, and clusters of eight leave some SMs two blocks and others none.  From this many rows
+// on that costs more than a kernel for the image (1.3 us): 8, 12, 20 and 32 rows 10.6, 15.3, 22.4, 32.9 us in clusters of eight, 10.6, 13.6, 18.7, 26.4 in two kernels;
+// lanes of 1, 4, 3, 2, 1, 4, 3 rows 24.0 and 22.8, four lanes of five 22.7 and 18.5.  Windows of twelve layers with several lanes: 2 x 1 and 3 x 1 rows 599 and
+// 676 us in clusters of eight, 611 and 686 in two kernels; 2 x 2 rows 710 (the clusters do not all fit beside the projection) and 692, 4 x 1 725 and 727, 8 x 1 976 and 964.
+constexpr int GDN_PAIR_ROWS = 8, GDN_PAIR_LANES = 3;
+int gdn_window(const GdnArgs& p0, const int* cur, bool early, cudaStream_t st) {
+    GdnArgs p = p0;
+    const bool apart = p.img && p.T > GDN_PAIR_ROWS;
+    if (apart) p.img = nullptr;
     auto kernel = p.img ? k_gdn_core<2 * GDN_Q> : k_gdn_core<GDN_Q>;
-    if (int rc = set_smem_limit((const void*) kernel, 112 * 1024)) return rc;
-    const cudaError_t le = launch_dep(early, kernel, dim3(p.nv * GDN_Q), dim3(GDN_THREADS), gdn_smem_bytes(p.T, CL, p.parent != nullptr), st, p, cur);
-    return le == cudaSuccess ? FNX_OK : fail(FNX_E_CUDA, "k_gdn_core: launch failed: %s", cudaGetErrorString(le));
+    FNX_TRY(set_smem_limit((const void*) kernel, GDN_SMEM));
+    const cudaError_t le = launch_dep(early, kernel, dim3(p.nv * GDN_Q), dim3(GDN_THREADS), gdn_smem_bytes(p.T, p.parent != nullptr), st, p, cur);
+    if (le != cudaSuccess) return fail(FNX_E_CUDA, "k_gdn_core: launch failed: %s", cudaGetErrorString(le));
+    return apart ? nat_rows_image(p.y, p.nv * GDN_HS, p.T, p.nv * GDN_HS, nullptr, p0.img, st) : FNX_OK;
 }
-int gdn_window_lanes(const GdnArgs& p, size_t hist_seq_stride, size_t s_seq_stride, const int* cur, const int* lane_seq, const int* lane_row0, int n_lanes, int max_rows,
-                     bool early, cudaStream_t st) {
-    const int CL = p.img ? 2 * GDN_Q : GDN_Q;
+int gdn_window_lanes(const GdnArgs& p0, size_t hist_seq_stride, size_t s_seq_stride, const int* cur, const int* lane_seq, const int* lane_row0, int n_lanes, int max_rows,
+                     int rows, bool early, cudaStream_t st) {
+    GdnArgs p = p0;
+    const bool apart = p.img && rows > (n_lanes > 1 ? GDN_PAIR_LANES : GDN_PAIR_ROWS);
+    if (apart) p.img = nullptr;
     auto kernel = p.img ? k_gdn_core_lanes<2 * GDN_Q> : k_gdn_core_lanes<GDN_Q>;
-    if (int rc = set_smem_limit((const void*) kernel, 112 * 1024)) return rc;
-    const cudaError_t le = launch_dep(early, kernel, dim3(p.nv * GDN_Q, n_lanes), dim3(GDN_THREADS), gdn_smem_bytes(max_rows, CL, false), st, p, hist_seq_stride, s_seq_stride, cur,
+    FNX_TRY(set_smem_limit((const void*) kernel, GDN_SMEM));
+    const cudaError_t le = launch_dep(early, kernel, dim3(p.nv * GDN_Q, n_lanes), dim3(GDN_THREADS), gdn_smem_bytes(max_rows, false), st, p, hist_seq_stride, s_seq_stride, cur,
                                       lane_seq, lane_row0);
-    return le == cudaSuccess ? FNX_OK : fail(FNX_E_CUDA, "k_gdn_core_lanes: launch failed: %s", cudaGetErrorString(le));
+    if (le != cudaSuccess) return fail(FNX_E_CUDA, "k_gdn_core_lanes: launch failed: %s", cudaGetErrorString(le));
+    return apart ? nat_rows_image(p.y, p.nv * GDN_HS, rows, p.nv * GDN_HS, nullptr, p0.img, st) : FNX_OK;
 }
 
 }  // namespace fnxb
@@ -741,5 +864,5 @@ extern "C" int fnx_gdn_core_lanes(const float* qkvz, int ldx, const float* ab, i
                 n_lanes, max_lane_rows, NS);
     FNX_REQUIRE(nk >= 1 && nv >= nk && nv % nk == 0, "fnx_gdn_core_lanes: %d key heads, %d value heads", nk, nv);
     return gdn_window_lanes(GdnArgs{qkvz, ldx, ab, ldab, hist_pool, convw, dt, a, nw, S_pool, NS, nullptr, y, nullptr, nk, nv, max_lane_rows, eps}, hist_seq_stride,
-                            s_seq_stride, cur, lane_seq, lane_row0, n_lanes, max_lane_rows, false, as_stream(st));
+                            s_seq_stride, cur, lane_seq, lane_row0, n_lanes, max_lane_rows, 0, false, as_stream(st));
 }

@@ -23,7 +23,8 @@ struct GdnArgs {
 };
 
 int gdn_window(const GdnArgs& p, const int* cur, bool early, cudaStream_t st);
+// rows: of all the lanes
 int gdn_window_lanes(const GdnArgs& p, size_t hist_seq_stride, size_t s_seq_stride, const int* cur, const int* lane_seq, const int* lane_row0, int n_lanes, int max_rows,
-                     bool early, cudaStream_t st);
+                     int rows, bool early, cudaStream_t st);
 
 }  // namespace fnxb
