@@ -10,8 +10,8 @@
 // on their own, and 256-row tiles another 1,000 of products over rows that mostly were not there (thirteen rows an expert in a prompt
 // of 640).  Here
 //   - sixteen decode warps own a 16-row tile row each: 2,176-byte half tiles by their lanes' own async copies, three blocks ahead across
-//     items; nibbles to f16 with one shift, four masks and eight half operations a word of eight; the fragment layout is tcgen05.st's
-//     16x256b shape, so 64 columns leave as one store of sixteen registers;
+//     items; nibbles to f16 with one shift, four masks and eight half operations a word of eight; a lane's words are columns of
+//     tcgen05.st's 16x128b shape, so 64 columns leave as one store of sixteen registers;
 //   - two warps gather the job's live rows (a row of B only reaches its own column of D: the others stay what they are);
 //   - one warp issues the products, one thread each, two accumulators (gate and up, or 2 x 128 features) double-buffered in tensor memory;
 //   - four warps write the item before.
@@ -59,9 +59,10 @@ static_assert(sizeof(PnShared) <= PN_HEAD, "the head fits");
 
 __device__ __forceinline__ bool pn_wait(uint64_t* bar, unsigned parity, PnShared& S) { return ta_wait_for(bar, parity, S.gave_up); }
 
-// sixteen tensor-memory lanes x 32 columns: register 4 b + {0, 1} = columns 8 b + 2 q, + 1 of lane g, + {2, 3} the same of lane g + 8
+// sixteen tensor-memory lanes x 32 columns: register 2 b = column 4 b + q of lane g, 2 b + 1 the same of lane g + 8.  (The shape 16x256b, a fragment as mma.sync has it, takes
+// twice as long: 131 cycles a warp's store against 67 with sixteen warps at it.)
 __device__ __forceinline__ void pn_st_tile(uint32_t taddr, const uint32_t (&v)[16]) {
-    asm volatile("tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr), "r"(v[0]), "r"(v[1]),
+    asm volatile("tcgen05.st.sync.aligned.16x128b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr), "r"(v[0]), "r"(v[1]),
                  "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]),
                  "r"(v[15])
                  : "memory");
@@ -232,10 +233,10 @@ __global__ void __launch_bounds__(PN_THREADS, 1) k_prompt_nat(const PnParams p) 
                             __half2 f00, f01, f10, f11;
                             pn_scales(m.x, Q, d0, f00, f01);
                             pn_scales(m.y, Q, d1, f10, f11);
-                            pn_decode8<WIDE>(w[0][2 * Q], f00, o[0], o[1], o[4], o[5]);
-                            pn_decode8<WIDE>(w[1][2 * Q], f10, o[2], o[3], o[6], o[7]);
-                            pn_decode8<WIDE>(w[0][2 * Q + 1], f01, o[8], o[9], o[12], o[13]);
-                            pn_decode8<WIDE>(w[1][2 * Q + 1], f11, o[10], o[11], o[14], o[15]);
+                            pn_decode8<WIDE>(w[0][2 * Q], f00, o[0], o[2], o[4], o[6]);
+                            pn_decode8<WIDE>(w[1][2 * Q], f10, o[1], o[3], o[5], o[7]);
+                            pn_decode8<WIDE>(w[0][2 * Q + 1], f01, o[8], o[10], o[12], o[14]);
+                            pn_decode8<WIDE>(w[1][2 * Q + 1], f11, o[9], o[11], o[13], o[15]);
                             if (q2 == 0) {
                                 if (ok && c >= PN_AST) ok = __all_sync(0xffffffffu, pn_wait(&sh.empty[st], (unsigned) ((c / PN_AST - 1) & 1), sh));
                                 ta_fence_after();
@@ -641,8 +642,14 @@ __global__ void __launch_bounds__(256) k_prompt_nat_rows(const float* __restrict
             const float4 w = *reinterpret_cast<const float4*>(norm_w + i);
             q.x *= w.x * r; q.y *= w.y * r; q.z *= w.z * r; q.w *= w.w * r;
         }
-        const __half2 a = __floats2half2_rn(q.x, q.z), b = __floats2half2_rn(q.y, q.w);   // (pn_slot: 0, 2, 1, 3)
-        *reinterpret_cast<uint2*>(xh + (size_t) blockIdx.x * H + (few ? i : pn_slot(i))) = make_uint2(pn_h2(a), pn_h2(b));
+        const __half2 a = __floats2half2_rn(q.x, q.z), b = __floats2half2_rn(q.y, q.w);   // (pn_slot: columns 0 and 2 side by side, 1 and 3 eight slots on)
+        __half* at = xh + (size_t) blockIdx.x * H;
+        if (few) *reinterpret_cast<uint2*>(at + i) = make_uint2(pn_h2(a), pn_h2(b));
+        else {
+            at += pn_slot(i);
+            *reinterpret_cast<__half2*>(at) = a;
+            *reinterpret_cast<__half2*>(at + 8) = b;
+        }
     };
 #pragma unroll
     for (int j = 0; j < HOLD; ++j) {

@@ -10,10 +10,10 @@
 namespace fnxb {
 
 // Activations of these products are f16 rows whose columns lie, within every 32, in the order that the weight words decode in: lane q of a
-// fragment row holds the columns 8 q .. 8 q + 7, column 8 q + j at slot 16 (j / 4) + 4 q + {0, 2, 1, 3}[j % 4].
+// fragment row holds the columns 8 q .. 8 q + 7, column 8 q + j at slot 16 (j / 4) + 2 q + {0, 8, 1, 9}[j % 4].
 __host__ __device__ __forceinline__ int pn_slot(int c) {
     const int j = c & 7, q = (c >> 3) & 3, k = j & 3;
-    return (c & ~31) + 16 * (j >> 2) + 4 * q + ((k & 1) << 1 | k >> 1);
+    return (c & ~31) + 16 * (j >> 2) + 2 * q + ((k & 1) << 3 | k >> 1);
 }
 
 constexpr int PN_N = 64;       // rows per job at most
