@@ -444,8 +444,11 @@ constexpr int GC_BV = 0, GC_BK = 8, GC_BQ = 16, GC_BC = 24, GC_M = 28, GC_FLOATS
 
 // grid (groups, key heads + pairs of value heads): a key head's q and k, its dots, and its value heads' coefficients and c; or 256 channels
 // of v.  Rows past T become zeros (their coefficients leave the state as it is).  xq / xk [8 groups][nk][HS], xv / xc [..][nv][HS].
-// Bound by its reads and writes; a row's inputs are read by one block, eight rows and three before them at a time.
-__global__ void __launch_bounds__(GDP_THREADS) k_gdn_pre(const float* __restrict__ qkvz, int stride, const float* __restrict__ ab, int ldab,
+// Bound by instructions (the conv's exponentials and divisions; of a key head's the dots of the pairs j <= i alone, a row's norm over a warp in nine shuffles for all
+// eight rows) and the chain of a block's four barriers, which the gates' loads and exponentials no longer lie in; a row's inputs are read by one block, eight rows and three before them at a time.
+// Six blocks an SM, by 40 registers a thread: 333, 3,001 and 38,912 rows 13.9, 77.8, 921 us, at 64 registers 14.5, 93.0, 1,109, at 32 (with spills) 14.4, 79.2, 954; with all pairs' dots, 40
+// shuffles for the norms and the gates behind the dots 15.6, 100.5, 1,226.  The conv and the norms alone take 750 of them, the bytes 490.
+__global__ void __launch_bounds__(GDP_THREADS, 6) k_gdn_pre(const float* __restrict__ qkvz, int stride, const float* __restrict__ ab, int ldab,
                                                          const float* __restrict__ hin, float* __restrict__ hout, const float* __restrict__ convw,
                                                          const float* __restrict__ dt, const float* __restrict__ a_, float* __restrict__ xq,
                                                          float* __restrict__ xk, float* __restrict__ xv, float* __restrict__ xc, float* __restrict__ coef, int nk, int nv,
@@ -459,11 +462,32 @@ __global__ void __launch_bounds__(GDP_THREADS) k_gdn_pre(const float* __restrict
     const int c = y < nk ? hf * nk * HS + y * HS + el : 2 * nk * HS + (y - nk) * GDP_THREADS + tid;
     const float4 cw = *reinterpret_cast<const float4*>(convw + (size_t) c * 4);
     float x[R + 3], v[R];   // rows t0 - 3 ..: of this call, or the history it starts from (rows 0..2, oldest first)
+    if (t0 >= 3 && t0 + R <= T) {
+        const float* src = qkvz + (size_t) (t0 - 3) * stride + c;
 #pragma unroll
-    for (int i = 0; i < R + 3; ++i) {
-        const int r = t0 - 3 + i;
-        x[i] = r < 0 ? hin[(size_t) (3 + r) * ch + c] : r < T ? qkvz[(size_t) r * stride + c] : 0.f;
+        for (int i = 0; i < R + 3; ++i) x[i] = src[(size_t) i * stride];
+    } else {
+#pragma unroll
+        for (int i = 0; i < R + 3; ++i) {
+            const int r = t0 - 3 + i;
+            x[i] = r < 0 ? hin[(size_t) (3 + r) * ch + c] : r < T ? qkvz[(size_t) r * stride + c] : 0.f;
+        }
     }
+    auto gates = [&](int lv) {   // a value head's: one half block's head each, eight rows
+        if (el < R && lv < nv) {
+            const int t = t0 + el;
+            const float* abt = ab + (size_t) t * ldab;
+            float g = 1.f, b = 0.f;
+            if (t < T) {
+                const float p = abt[lv] + dt[lv];
+                g = expf((p > 20.0f ? p : log1pf(expf(p))) * a_[lv]);
+                b = 1.0f / (1.0f + expf(-abt[nv + lv]));
+            }
+            sg[hf][el] = g;
+            sb[hf][el] = b;
+        }
+    };
+    if (y < nk) gates(y + hf * nk);   // (their loads' way is that of the rows')
 #pragma unroll
     for (int i = 0; i < R; ++i) {
         const float s = cw.x * x[i] + cw.y * x[i + 1] + cw.z * x[i + 2] + cw.w * x[i + 3];
@@ -482,10 +506,23 @@ __global__ void __launch_bounds__(GDP_THREADS) k_gdn_pre(const float* __restrict
         for (int i = 0; i < R; ++i) dst[(size_t) i * nv * HS] = v[i];
         return;
     }
+    {   // the squares' sums over the warp, all rows at once: at each of three steps a lane keeps the half of its rows that its lane number names
+        float sq[R];
 #pragma unroll
-    for (int i = 0; i < R; ++i) {
-        const float sq = warp_sum(v[i] * v[i]);
-        if (lane == 0) red[warp][i] = sq;
+        for (int i = 0; i < R; ++i) sq[i] = v[i] * v[i];
+#pragma unroll
+        for (int o = 16, n = R / 2; n >= 1; o >>= 1, n >>= 1) {
+            const bool up = lane & o;
+#pragma unroll
+            for (int i = 0; i < n; ++i) {
+                const float keep = up ? sq[i + n] : sq[i], give = up ? sq[i] : sq[i + n];
+                sq[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+            }
+        }
+        sq[0] += __shfl_xor_sync(0xffffffffu, sq[0], 2);
+        sq[0] += __shfl_xor_sync(0xffffffffu, sq[0], 1);
+        static_assert(R == 8, "lanes 16, 8 and 4 name the row");
+        if ((lane & 3) == 0) red[warp][lane >> 2] = sq[0];
     }
     __syncthreads();
     {
@@ -500,8 +537,9 @@ __global__ void __launch_bounds__(GDP_THREADS) k_gdn_pre(const float* __restrict
         }
     }
     __syncthreads();
-    {   // four threads a pair of rows
-        const int i = tid >> 5, j = (tid >> 2) & 7, e0 = (tid & 3) * 4;
+    if (tid < 4 * R * (R + 1) / 2) {   // four threads a pair of rows j <= i (the others' have no part in anything)
+        const int pr = tid >> 2, i = (pr >= 1) + (pr >= 3) + (pr >= 6) + (pr >= 10) + (pr >= 15) + (pr >= 21) + (pr >= 28), j = pr - i * (i + 1) / 2, e0 = (tid & 3) * 4;
+        const unsigned live = __activemask();
         float dk = 0.f, dq = 0.f;
 #pragma unroll
         for (int m = 0; m < HS / 16; ++m) {
@@ -512,8 +550,8 @@ __global__ void __launch_bounds__(GDP_THREADS) k_gdn_pre(const float* __restrict
         }
 #pragma unroll
         for (int o = 1; o < 4; o <<= 1) {
-            dk += __shfl_xor_sync(0xffffffffu, dk, o);
-            dq += __shfl_xor_sync(0xffffffffu, dq, o);
+            dk += __shfl_xor_sync(live, dk, o);
+            dq += __shfl_xor_sync(live, dq, o);
         }
         if ((tid & 3) == 0) {
             kk[i][j] = dk;
@@ -525,39 +563,32 @@ __global__ void __launch_bounds__(GDP_THREADS) k_gdn_pre(const float* __restrict
     for (int lv0 = y; lv0 < nv; lv0 += 2 * nk) {   // the key head's value heads, one a half block
         const int lv = lv0 + hf * nk;
         const bool on = lv < nv;
-        if (on && el < R) {
-            const int t = t0 + el;
-            const float* abt = ab + (size_t) t * ldab;
-            float g = 1.f, b = 0.f;
-            if (t < T) {
-                const float p = abt[lv] + dt[lv];
-                g = expf((p > 20.0f ? p : log1pf(expf(p))) * a_[lv]);
-                b = 1.0f / (1.0f + expf(-abt[nv + lv]));
-            }
-            sg[hf][el] = g;
-            sb[hf][el] = b;
-        }
+        if (lv0 != y) gates(lv);
         __syncthreads();
         auto prod = [&](int a, int b) {   // g_a .. g_b
             float p = 1.f;
             for (int l = a; l <= b; ++l) p *= sg[hf][l];
             return p;
         };
-        if (on && el < 64) {
-            const float r = tj <= ti ? prod(tj + 1, ti) : 0.f;
-            Lm[hf][ti][tj] = tj < ti ? sb[hf][ti] * r * kk[ti][tj] : 0.f;
-            Qm[hf][ti][tj] = tj <= ti ? scale * r * qk[ti][tj] : 0.f;
-        }
-        __syncthreads();
-        if (on && el < R) {   // column el of the inverse
-            float t[R];
+        if (on && el < 32) {   // a warp: two entries of the matrices a lane, then column `el` of the inverse
 #pragma unroll
-            for (int i = 0; i < R; ++i) {
-                float a = i == el ? 1.f : 0.f;
+            for (int h = 0; h < 2; ++h) {
+                const int i = (el >> 3) + 4 * h, j = el & 7;
+                const float r = j <= i ? prod(j + 1, i) : 0.f;
+                Lm[hf][i][j] = j < i ? sb[hf][i] * r * kk[i][j] : 0.f;
+                Qm[hf][i][j] = j <= i ? scale * r * qk[i][j] : 0.f;
+            }
+            __syncwarp();
+            if (el < R) {
+                float t[R];
 #pragma unroll
-                for (int j = 0; j < i; ++j) a = fmaf(-Lm[hf][i][j], t[j], a);
-                t[i] = i < el ? 0.f : a;
-                Ti[hf][i][el] = t[i];
+                for (int i = 0; i < R; ++i) {
+                    float a = i == el ? 1.f : 0.f;
+#pragma unroll
+                    for (int j = 0; j < i; ++j) a = fmaf(-Lm[hf][i][j], t[j], a);
+                    t[i] = i < el ? 0.f : a;
+                    Ti[hf][i][el] = t[i];
+                }
             }
         }
         __syncthreads();
