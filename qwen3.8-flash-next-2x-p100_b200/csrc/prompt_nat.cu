@@ -20,9 +20,9 @@
 // accumulator pair, whose results (6 us an item) then lie in the next item's way: 388 us for 512 jobs of 116 rows, 339 for 1,024 of 58.
 // Measured, 512 jobs of gate|up and of down (fourteen items of 256 features x 2,048 columns an SM), us: six rows a job 162 + 92, fifty-eight 179 + 115, 6,144 jobs
 // of 760 rows an expert 1,940 + 1,244 (187 + 101, 200 + 126 and 2,172 + 1,334 with four stages of rows, N = 64 and two instructions a word more); in a prompt of 333 rows, ten picks
-// a row, 150 + 83 a layer.  With neither decode nor
-// products 128: the hand-over between the decode warps, the weight stages, the rows and the issuing thread, then the decode's instructions (half of the
-// issue slots), are what is left here; DRAM would allow 88.
+// a row, 150 + 83 a layer, 147 + 80 with the weights' stores of shape 16x128b.  By its clocks a down chunk of 128 columns takes 1,430 cycles there and 1,630 at 20,000 rows: a decode warp
+// waits 200 of them for a free stage and works the rest (13 instructions a word, half and integer-logic ones at two cycles each on pipes that overlap by half), the issuing thread waits
+// 410 to 530 for the weights.  DRAM would allow 88.
 #include <type_traits>
 
 #include "attn_tc.cuh"
