@@ -123,6 +123,12 @@ int fnx_moe_down(const void* Wdn, size_t expert_stride, int e_base, const void* 
  * outside the range (-1, E: a masked one), adds nothing, whatever its row of part holds */
 int fnx_moe_combine(const float* part, const int* topi, const float* topw, const float* logits, int T, int E, int H,
                     int K, int e_lo, int e_hi, int add_shared, float* out, int accumulate, fnx_stream st);
+/* fnx_moe_gate_up, fnx_moe_down and fnx_moe_combine (not accumulating) of one routing result, in one call: a window's three launches without a caller's way
+ * back between them.  gu_stride, dn_stride: bytes of an expert's matrices. */
+int fnx_moe_experts(const void* Wgu, size_t gu_stride, const void* Wdn, size_t dn_stride, int e_base, const void* Wsh_gu, const void* Wsh_dn,
+                    const fnx_job* jobs, const int* njobs, int njobs_max, const int* topi, const float* topw, const float* logits, const float* x,
+                    const float* norm_w, float eps, int T, int E, int H, int F, int K, int e_lo, int e_hi, int add_shared, float* h, float* part, float* out,
+                    unsigned* err, fnx_stream st);
 /* fnx_moe_combine(part, ..., 0, E, 1, R, 1) that also leaves the image of rmsnorm(R[t]) * img_norm_w for fnx_dense_image
  * (ceil(T / FNX_DENSE_ROWS) * fnx_dense_image_bytes(H) bytes, 16-byte aligned: one image per FNX_DENSE_ROWS rows): the rows are quantised once, by the kernel that completes
  * them, instead of by every block of the next projection.  R gets the same bits as from fnx_moe_combine. */

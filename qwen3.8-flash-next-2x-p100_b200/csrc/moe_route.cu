@@ -602,6 +602,15 @@ extern "C" int fnx_moe_combine(const float* part, const int* topi, const float* 
     return FNX_OK;
 }
 
+extern "C" int fnx_moe_experts(const void* Wgu, size_t gu_stride, const void* Wdn, size_t dn_stride, int e_base, const void* Wsh_gu, const void* Wsh_dn,
+                               const fnx_job* jobs, const int* njobs, int njobs_max, const int* topi, const float* topw, const float* logits, const float* x,
+                               const float* norm_w, float eps, int T, int E, int H, int F, int K, int e_lo, int e_hi, int add_shared, float* h, float* part, float* out,
+                               unsigned* err, fnx_stream st) {
+    FNX_TRY(fnx_moe_gate_up(Wgu, gu_stride, e_base, Wsh_gu, E, jobs, njobs, njobs_max, x, norm_w, eps, H, F, h, err, st));
+    FNX_TRY(fnx_moe_down(Wdn, dn_stride, e_base, Wsh_dn, E, jobs, njobs, njobs_max, h, H, F, part, err, st));
+    return fnx_moe_combine(part, topi, topw, logits, T, E, H, K, e_lo, e_hi, add_shared, out, 0, st);
+}
+
 extern "C" int fnx_moe_combine_image(const float* part, const int* topi, const float* topw, const float* logits, int T, int E, int H, int K, float* R,
                                      void* img_out, const float* img_norm_w, fnx_stream st) {
     FNX_REQUIRE(part && topi && topw && logits && R && img_out && img_norm_w, "fnx_moe_combine_image: null pointer");
