@@ -219,10 +219,7 @@ int fnx_gdn_core(const float* qkvz, int ldx, const float* ab, int ldab, float* h
                  const float* a, const float* nw, float* S_pool, const int* cur, int NS, const int* parent, float* y,
                  int nk, int nv, int hs, int T, float eps, fnx_stream st);
 
-/* Batched lanes of gdn_core (gdn_core_segs, engine/src/kernels.cu:2112-2156; GdnLanes, engine/src/kernels.hpp:103-110):
- * lane j is a chain from slot cur[lane_seq[j]] of that sequence's rings at hist_pool + seq * hist_seq_stride floats and
- * S_pool + seq * s_seq_stride floats. */
-/* the same over a prompt's T rows (any T), a chain of which every row is kept (gdn_prompt, engine/src/kernels.cu:2158), in three
+/* gdn_core over a prompt's T rows (any T), a chain of which every row is kept (gdn_prompt, engine/src/kernels.cu:2158), in three
  * launches: conv + SiLU, q / k norms and gates of every row at once; the delta rule eight rows at a time, the state in registers
  * from the first row to the last; the gated norm of every row at once.  Starts from state slot `cur` (a host value here) and leaves the
  * last row's state and conv history in slot (cur + T) % NS: the caller advances its slot index by T.
@@ -231,6 +228,9 @@ size_t fnx_gdn_prompt_scratch_bytes(int T, int nk, int nv, int hs);
 int fnx_gdn_prompt(const float* qkvz, int ldx, const float* ab, int ldab, float* hist_pool, const float* convw, const float* dt,
                    const float* a, const float* nw, float* S_pool, int cur, int NS, float* y, int nk, int nv, int hs, int T,
                    float eps, void* scratch, fnx_stream st);
+/* Batched lanes of gdn_core (gdn_core_segs, engine/src/kernels.cu:2112-2156; GdnLanes, engine/src/kernels.hpp:103-110):
+ * lane j, the rows [lane_row0[j], lane_row0[j + 1]) (at most max_lane_rows <= FNX_MAX_ROWS of them), is a chain from slot cur[lane_seq[j]] of
+ * that sequence's rings at hist_pool + seq * hist_seq_stride floats and S_pool + seq * s_seq_stride floats. */
 int fnx_gdn_core_lanes(const float* qkvz, int ldx, const float* ab, int ldab, float* hist_pool, size_t hist_seq_stride,
                        const float* convw, const float* dt, const float* a, const float* nw, float* S_pool,
                        size_t s_seq_stride, const int* cur, int NS, const int* lane_seq, const int* lane_row0, int n_lanes,

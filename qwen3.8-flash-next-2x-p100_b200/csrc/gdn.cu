@@ -891,8 +891,8 @@ extern "C" int fnx_gdn_core_lanes(const float* qkvz, int ldx, const float* ab, i
                                   fnx_stream st) {
     FNX_REQUIRE(qkvz && ab && hist_pool && convw && dt && a && nw && S_pool && cur && lane_seq && lane_row0 && y, "fnx_gdn_core_lanes: null pointer");
     FNX_REQUIRE(hs == GDN_HS, "fnx_gdn_core_lanes: head dim %d (this build: %d)", hs, GDN_HS);
-    FNX_REQUIRE(n_lanes >= 1 && n_lanes <= FNX_MAX_ROWS && max_lane_rows >= 1 && NS >= max_lane_rows + 1, "fnx_gdn_core_lanes: %d lanes of up to %d rows, %d state slots",
-                n_lanes, max_lane_rows, NS);
+    FNX_REQUIRE(n_lanes >= 1 && n_lanes <= FNX_MAX_ROWS && max_lane_rows >= 1 && max_lane_rows <= FNX_MAX_ROWS && NS >= max_lane_rows + 1,
+                "fnx_gdn_core_lanes: %d lanes of up to %d rows, %d state slots", n_lanes, max_lane_rows, NS);
     FNX_REQUIRE(nk >= 1 && nv >= nk && nv % nk == 0, "fnx_gdn_core_lanes: %d key heads, %d value heads", nk, nv);
     return gdn_window_lanes(GdnArgs{qkvz, ldx, ab, ldab, hist_pool, convw, dt, a, nw, S_pool, NS, nullptr, y, nullptr, nk, nv, max_lane_rows, eps}, hist_seq_stride,
                             s_seq_stride, cur, lane_seq, lane_row0, n_lanes, max_lane_rows, 0, false, as_stream(st));

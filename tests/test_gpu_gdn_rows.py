@@ -60,3 +60,44 @@ def test_a_row_of_an_engine_gives_the_same_bits_in_wide_windows(F, T):
             eng.commit([0], seq=0)
     finally:
         eng.close()
+
+
+def _lanes(F, d_x, d_ab, d_hist, const, d_S, cur, seqs, lens, max_rows, y, nk, nv):
+    L, P, hs = F.lib(), F.ptr, 128
+    row0 = dev(np.concatenate([[0], np.cumsum(lens)]).astype(np.int32))
+    F.check(L.fnx_gdn_core_lanes(P(d_x), d_x.stride(0), P(d_ab), d_ab.stride(0), P(d_hist), d_hist.stride(0), *map(P, const), P(d_S), d_S.stride(0), P(cur), d_S.shape[1],
+                                 P(dev(np.array(seqs, np.int32))), P(row0), len(lens), max_rows, P(y), nk, nv, hs, 1e-6, F._stream()))
+
+
+@pytest.mark.parametrize("lens,seqs", [([1], [2]), ([1, 1], [1, 0]), ([4, 5, 1], [2, 0, 1]), ([2, 3, 8, 0, 9], [4, -1, 0, 3, 1]), ([32], [0])])
+def test_lanes_of_the_operator_are_each_alone(F, lens, seqs):
+    """The lanes form against fnx_gdn_core of each lane: the same bits, from a longest lane of one row to one of FNX_MAX_ROWS; an empty lane and one of a negative sequence change nothing."""
+    nk, nv, hs, n_seq = 2, 4, 128, 5
+    NS, T = max(lens) + 1, sum(lens)
+    rng = np.random.default_rng(T)
+    ch, qkvz, ab, convw, dt, a, nw = _gdn_inputs(rng, T, nk, nv, hs)
+    const = [dev(v) for v in (convw, dt, a, nw)]
+    d_S, d_hist = dev((0.1 * rng.standard_normal((n_seq, NS, nv, hs, hs))).astype(np.float32)), dev(rng.standard_normal((n_seq, NS, 3, ch)).astype(np.float32))
+    want_S, want_hist, at = d_S.clone(), d_hist.clone(), rng.integers(0, NS, size=n_seq).astype(np.int32)
+    d_x, d_ab = dev(qkvz), dev(ab)
+    y = torch.full((T, nv * hs), 7.0, device="cuda")
+    want = y.clone()
+    _lanes(F, d_x, d_ab, d_hist, const, d_S, dev(at), seqs, lens, max(lens), y, nk, nv)
+    r = 0
+    for n, s in zip(lens, seqs):
+        if n and s >= 0:
+            want[r:r + n] = F.gdn_core(d_x[r:r + n], d_ab[r:r + n], want_hist[s], *const, want_S[s], dev(at[s:s + 1]), None, nk, nv, hs)
+        r += n
+    assert torch.equal(y, want) and torch.equal(d_S, want_S) and torch.equal(d_hist, want_hist)
+
+
+def test_lanes_of_more_rows_than_a_window_are_refused(F):
+    """FNX_MAX_ROWS + 1 rows a lane: refused whatever the lanes hold (here: nothing, so that a call that is taken has no row to work on)."""
+    nk, nv, hs, NS = 2, 4, 128, 40
+    ch, qkvz, ab, convw, dt, a, nw = _gdn_inputs(np.random.default_rng(0), 1, nk, nv, hs)
+    args = [F, dev(qkvz), dev(ab), torch.zeros((1, NS, 3, ch), device="cuda"), [dev(v) for v in (convw, dt, a, nw)], torch.zeros((1, NS, nv, hs, hs), device="cuda"),
+            dev(np.zeros(1, np.int32)), [0], [0]]
+    _lanes(*args, F.MAX_ROWS, torch.zeros((1, nv * hs), device="cuda"), nk, nv)
+    with pytest.raises(F.FnxError, match="lanes of up to 33 rows"):
+        _lanes(*args, F.MAX_ROWS + 1, torch.zeros((1, nv * hs), device="cuda"), nk, nv)
+    torch.cuda.synchronize()
