@@ -539,7 +539,8 @@ __global__ void __launch_bounds__(GDP_THREADS, 6) k_gdn_pre(const float* __restr
     __syncthreads();
     if (tid < 4 * R * (R + 1) / 2) {   // four threads a pair of rows j <= i (the others' have no part in anything)
         const int pr = tid >> 2, i = (pr >= 1) + (pr >= 3) + (pr >= 6) + (pr >= 10) + (pr >= 15) + (pr >= 21) + (pr >= 28), j = pr - i * (i + 1) / 2, e0 = (tid & 3) * 4;
-        const unsigned live = __activemask();
+        const unsigned live = tid < 128 ? 0xffffffffu : 0xffffu;   // four warps and half of the fifth
+        static_assert(4 * R * (R + 1) / 2 == 128 + 16, "the lanes above");
         float dk = 0.f, dq = 0.f;
 #pragma unroll
         for (int m = 0; m < HS / 16; ++m) {
