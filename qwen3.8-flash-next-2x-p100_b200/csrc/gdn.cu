@@ -53,7 +53,7 @@ __device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
 // warps for the rule and eight for the conv (19.0), an SM to each block (16 clusters of eight do not fit at once: 35).
 constexpr int GDN_BATCH = 4, GDN_CHANS = 2 * GDN_HS + GDN_QC;
 
-__host__ __device__ __forceinline__ bool gdn_staged(int T, bool tree) { return tree || T > GDN_BATCH; }
+__host__ __device__ constexpr bool gdn_staged(int T, bool tree) { return tree || T > GDN_BATCH; }
 
 template <int CL>
 __device__ __forceinline__ void gdn_body(const GdnArgs& p, int cur, float* sm) {
@@ -386,7 +386,8 @@ __device__ __forceinline__ void gdn_body(const GdnArgs& p, int cur, float* sm) {
             }
         }
     };
-    if (T <= 8) results(std::integral_constant<int, 1>{});
+    if constexpr (CL > GDN_Q) results(std::integral_constant<int, 1>{});   // (GDN_PAIR_ROWS at most)
+    else if (T <= 8) results(std::integral_constant<int, 1>{});
     else results(std::integral_constant<int, FNX_MAX_ROWS / 8>{});
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");   // no block may leave while a neighbour still reads its shared memory
 }
@@ -795,17 +796,20 @@ __global__ void __launch_bounds__(GDP_THREADS) k_gdn_post(const float* __restric
     }
 }
 
-static size_t gdn_smem_bytes(int T, bool tree) {
+static constexpr size_t gdn_smem_bytes(int T, bool tree) {
     return sizeof(float) * ((size_t) 2 * T * GDN_HS + (size_t) 6 * T * GDN_QC + 8 * GDN_QC + ((6 * T + 3) & ~3) +
                             (gdn_staged(T, tree) ? (size_t) (T + 3) * GDN_CHANS + 4 * T : 0));
 }
 constexpr int GDN_SMEM = 112 * 1024;
+static_assert(gdn_smem_bytes(FNX_MAX_ROWS, true) <= GDN_SMEM, "the most rows fit, two blocks an SM");
+static_assert(FNX_MAX_ROWS <= 32 && FNX_MAX_ROWS % 8 == 0 && 2 + (FNX_MAX_ROWS - 1) / GDN_BATCH < 16, "a lane a row's gates, eight warps of results, named barriers");
 
 // An image needs the two heads of its 256-column blocks in one cluster, and clusters of eight leave some SMs two blocks and others none.  From this many rows
 // on that costs more than a kernel for the image (1.3 us): 8, 12, 20 and 32 rows 10.6, 15.3, 22.4, 32.9 us in clusters of eight, 10.6, 13.6, 18.7, 26.4 in two kernels;
 // lanes of 1, 4, 3, 2, 1, 4, 3 rows 24.0 and 22.8, four lanes of five 22.7 and 18.5.  Windows of twelve layers with several lanes: 2 x 1 and 3 x 1 rows 599 and
 // 676 us in clusters of eight, 611 and 686 in two kernels; 2 x 2 rows 710 (the clusters do not all fit beside the projection) and 692, 4 x 1 725 and 727, 8 x 1 976 and 964.
 constexpr int GDN_PAIR_ROWS = 8, GDN_PAIR_LANES = 3;
+static_assert(GDN_PAIR_ROWS <= 8 && GDN_PAIR_LANES <= 8, "clusters of eight give a row to each of a block's warps");
 int gdn_window(const GdnArgs& p0, const int* cur, bool early, cudaStream_t st) {
     GdnArgs p = p0;
     const bool apart = p.img && p.T > GDN_PAIR_ROWS;
