@@ -573,10 +573,18 @@ __global__ void __launch_bounds__(GDP_THREADS, 6) k_gdn_pre(const float* __restr
             return p;
         };
         if (on && el < 32) {   // a warp: two entries of the matrices a lane, then column `el` of the inverse
+            const int j = el & 7;
+            float pr[2] = {1.f, 1.f};   // g_(j + 1) .. g_i of both in one pass, the gates' loads all at once: a value head's chain is every further one's wait
+#pragma unroll
+            for (int l = 1; l < R; ++l) {
+                const float g = l > j ? sg[hf][l] : 1.f;
+                if (l <= (el >> 3)) pr[0] *= g;
+                if (l <= (el >> 3) + 4) pr[1] *= g;
+            }
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const int i = (el >> 3) + 4 * h, j = el & 7;
-                const float r = j <= i ? prod(j + 1, i) : 0.f;
+                const int i = (el >> 3) + 4 * h;
+                const float r = j <= i ? pr[h] : 0.f;
                 Lm[hf][i][j] = j < i ? sb[hf][i] * r * kk[i][j] : 0.f;
                 Qm[hf][i][j] = j <= i ? scale * r * qk[i][j] : 0.f;
             }
