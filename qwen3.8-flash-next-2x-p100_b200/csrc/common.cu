@@ -35,9 +35,9 @@ int sm_count() {
     return n[dev];
 }
 
-// cudaFuncAttributeMaxDynamicSharedMemorySize is a per-device attribute of a kernel: set once per (device, kernel).  A thread remembers
-// the last pairs it has seen done, so that a launch usually takes no lock.
-int set_smem_limit(const void* kernel, int bytes) {
+// cudaFuncAttributeMaxDynamicSharedMemorySize and the clusters' scheduling policy are per-device attributes of a kernel: set once per (device, kernel).
+// A thread remembers the last pairs it has seen done, so that a launch usually takes no lock.
+int set_smem_limit(const void* kernel, int bytes, bool balance) {
     static std::mutex mu;
     static std::set<std::pair<int, const void*>> done;
     constexpr size_t SEEN = 64;
@@ -49,6 +49,7 @@ int set_smem_limit(const void* kernel, int bytes) {
     std::lock_guard<std::mutex> lock(mu);
     if (!done.count({dev, kernel})) {
         FNX_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+        if (balance) FNX_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeClusterSchedulingPolicyPreference, cudaClusterSchedulingPolicyLoadBalancing));
         done.insert({dev, kernel});
     }
     mine = {dev, kernel};

@@ -39,8 +39,9 @@ int fail(int code, const char* fmt, ...);
 
 inline cudaStream_t as_stream(fnx_stream s) { return (cudaStream_t) s; }
 int sm_count();
-// raises a kernel's dynamic shared-memory limit on the current device, once per (device, kernel)
-int set_smem_limit(const void* kernel, int bytes);
+// raises a kernel's dynamic shared-memory limit on the current device, once per (device, kernel); balance: its clusters' blocks go where there is
+// room, instead of to as many SMs as a cluster has blocks
+int set_smem_limit(const void* kernel, int bytes, bool balance = false);
 #if defined(__CUDACC__)
 // Programmatic dependent launch: a kernel may start while its predecessor in the stream drains.
 // Two rules hold for every kernel launched so.  Every block reaches pdl_wait(): a kernel's end implies its predecessors'.  And

@@ -809,6 +809,9 @@ static constexpr size_t gdn_smem_bytes(int T, bool tree) {
                             (gdn_staged(T, tree) ? (size_t) (T + 3) * GDN_CHANS + 4 * T : 0));
 }
 constexpr int GDN_SMEM = 112 * 1024;
+// The clusters are placed by load balancing.  The blocks start while the projection's leave (two of these or one and one of those to an SM), and by the default
+// policy, which spreads a cluster over SMs, one or two of the 32 clusters of eight of two lanes (33 fit at once) then wait for the first ones' end.
+// Windows of twelve layers, us, by the default policy and by this one: lanes of 1 and 2 rows 624 and 603, 2 and 2 668 and 647; a tree of 20 1,389 and 1,382; none slower.
 static_assert(gdn_smem_bytes(FNX_MAX_ROWS, true) <= GDN_SMEM, "the most rows fit, two blocks an SM");
 static_assert(FNX_MAX_ROWS <= 32 && FNX_MAX_ROWS % 8 == 0 && 2 + (FNX_MAX_ROWS - 1) / GDN_BATCH < 16, "a lane a row's gates, eight warps of results, named barriers");
 
@@ -823,7 +826,7 @@ int gdn_window(const GdnArgs& p0, const int* cur, bool early, cudaStream_t st) {
     const bool apart = p.img && p.T > GDN_PAIR_ROWS;
     if (apart) p.img = nullptr;
     auto kernel = p.img ? k_gdn_core<2 * GDN_Q> : k_gdn_core<GDN_Q>;
-    FNX_TRY(set_smem_limit((const void*) kernel, GDN_SMEM));
+    FNX_TRY(set_smem_limit((const void*) kernel, GDN_SMEM, true));
     const cudaError_t le = launch_dep(early, kernel, dim3(p.nv * GDN_Q), dim3(GDN_THREADS), gdn_smem_bytes(p.T, p.parent != nullptr), st, p, cur);
     if (le != cudaSuccess) return fail(FNX_E_CUDA, "k_gdn_core: launch failed: %s", cudaGetErrorString(le));
     return apart ? nat_rows_image(p.y, p.nv * GDN_HS, p.T, p.nv * GDN_HS, nullptr, p0.img, st) : FNX_OK;
@@ -834,7 +837,7 @@ int gdn_window_lanes(const GdnArgs& p0, size_t hist_seq_stride, size_t s_seq_str
     const bool apart = p.img && rows > (n_lanes > 1 ? GDN_PAIR_LANES : GDN_PAIR_ROWS);
     if (apart) p.img = nullptr;
     auto kernel = p.img ? k_gdn_core_lanes<2 * GDN_Q> : k_gdn_core_lanes<GDN_Q>;
-    FNX_TRY(set_smem_limit((const void*) kernel, GDN_SMEM));
+    FNX_TRY(set_smem_limit((const void*) kernel, GDN_SMEM, true));
     const cudaError_t le = launch_dep(early, kernel, dim3(p.nv * GDN_Q, n_lanes), dim3(GDN_THREADS), gdn_smem_bytes(max_rows, false), st, p, hist_seq_stride, s_seq_stride, cur,
                                       lane_seq, lane_row0);
     if (le != cudaSuccess) return fail(FNX_E_CUDA, "k_gdn_core_lanes: launch failed: %s", cudaGetErrorString(le));
