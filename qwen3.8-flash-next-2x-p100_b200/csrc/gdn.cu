@@ -815,15 +815,17 @@ constexpr int GDN_SMEM = 112 * 1024;
 static_assert(gdn_smem_bytes(FNX_MAX_ROWS, true) <= GDN_SMEM, "the most rows fit, two blocks an SM");
 static_assert(FNX_MAX_ROWS <= 32 && FNX_MAX_ROWS % 8 == 0 && 2 + (FNX_MAX_ROWS - 1) / GDN_BATCH < 16, "a lane a row's gates, eight warps of results, named barriers");
 
-// An image needs the two heads of its 256-column blocks in one cluster, and clusters of eight leave some SMs two blocks and others none.  From this many rows
-// on that costs more than a kernel for the image (1.3 us): 8, 12, 20 and 32 rows 10.6, 15.3, 22.4, 32.9 us in clusters of eight, 10.6, 13.6, 18.7, 26.4 in two kernels;
-// lanes of 1, 4, 3, 2, 1, 4, 3 rows 24.0 and 22.8, four lanes of five 22.7 and 18.5.  Windows of twelve layers with several lanes: 2 x 1 and 3 x 1 rows 599 and
-// 676 us in clusters of eight, 611 and 686 in two kernels; 2 x 2 rows 710 (the clusters do not all fit beside the projection) and 692, 4 x 1 725 and 727, 8 x 1 976 and 964.
-constexpr int GDN_PAIR_ROWS = 8, GDN_PAIR_LANES = 3;
-static_assert(GDN_PAIR_ROWS <= 8 && GDN_PAIR_LANES <= 8, "clusters of eight give a row to each of a block's warps");
+// An image needs the two heads of its 256-column blocks in one cluster: clusters of eight, whose warps finish a row each.  A kernel for the image takes 1.4 us; more rows, or
+// very many clusters whose blocks wait for one another in eights, cost more than that.  Windows, us, in clusters of eight and in two kernels: of twelve layers with 32 value heads,
+// 1 and 8 rows (16 clusters) 499 and 505, 832 and 841, lanes of 1 and 2 rows and of 2 and 2 (32) 603 and 614, 647 and 655, eight of one (128) 928 and 929; of eight DeltaNet layers with 64
+// value heads, lanes of 4 and 4 rows (64) 548 and 560, four, six and eight of one (128, 192, 256) 511 and 518, 630 and 628, 720 and 697; with 16, 8 rows (8) 497 and 503.
+// (A form of the clusters of eight for more rows: chains of 9 to 24 rows 3 to 10 us faster, of 1 to 5 up to 3 us slower, with 128 value heads 4 to 10 slower.)
+constexpr int GDN_PAIR_ROWS = 8, GDN_PAIR_CLUSTERS = 128;
+static_assert(GDN_PAIR_ROWS <= 8, "clusters of eight give a row to each of a block's warps");
+static bool gdn_apart(const GdnArgs& p, int n_lanes, int rows) { return p.img && (rows > GDN_PAIR_ROWS || p.nv / 2 * n_lanes > GDN_PAIR_CLUSTERS); }
 int gdn_window(const GdnArgs& p0, const int* cur, bool early, cudaStream_t st) {
     GdnArgs p = p0;
-    const bool apart = p.img && p.T > GDN_PAIR_ROWS;
+    const bool apart = gdn_apart(p, 1, p.T);
     if (apart) p.img = nullptr;
     auto kernel = p.img ? k_gdn_core<2 * GDN_Q> : k_gdn_core<GDN_Q>;
     FNX_TRY(set_smem_limit((const void*) kernel, GDN_SMEM, true));
@@ -834,7 +836,7 @@ int gdn_window(const GdnArgs& p0, const int* cur, bool early, cudaStream_t st) {
 int gdn_window_lanes(const GdnArgs& p0, size_t hist_seq_stride, size_t s_seq_stride, const int* cur, const int* lane_seq, const int* lane_row0, int n_lanes, int max_rows,
                      int rows, bool early, cudaStream_t st) {
     GdnArgs p = p0;
-    const bool apart = p.img && rows > (n_lanes > 1 ? GDN_PAIR_LANES : GDN_PAIR_ROWS);
+    const bool apart = gdn_apart(p, n_lanes, rows);
     if (apart) p.img = nullptr;
     auto kernel = p.img ? k_gdn_core_lanes<2 * GDN_Q> : k_gdn_core_lanes<GDN_Q>;
     FNX_TRY(set_smem_limit((const void*) kernel, GDN_SMEM, true));

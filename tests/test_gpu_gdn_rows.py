@@ -1,4 +1,4 @@
-"""DeltaNet windows at the edges of their batches of four rows, of the rows that a kernel leaves quantised, and of a ring's end."""
+"""DeltaNet windows at the edges of their batches of four rows, of the clusters that leave a row quantised, and of a ring's end."""
 import numpy as np
 import pytest
 
@@ -37,24 +37,25 @@ def test_rows_of_a_window_are_the_oracles_and_each_alone(F, O, T):
     assert torch.equal(d_S, together[1]) and torch.equal(d_hist, together[2])
 
 
-def _small_config(F):
-    return F.flash_next_config(n_layer=4, hidden=1024, n_expert=32, top_k=4, ffn=256, n_q_head=8, n_kv_head=1, gdn_k_head=2, gdn_v_head=4, vocab=2048, max_ctx=256, max_rows=16,
-                               n_seq=4)
+def _small_config(F, nv=4):
+    return F.flash_next_config(n_layer=4, hidden=1024, n_expert=32, top_k=4, ffn=256, n_q_head=8, n_kv_head=1, gdn_k_head=nv // 2, gdn_v_head=nv, vocab=2048, max_ctx=256, max_rows=16,
+                               n_seq=6)
 
 
-@pytest.mark.parametrize("lens", [[1, 1], [1, 2], [2, 1], [1, 1, 1], [2, 2], [1, 2, 1]])
-def test_few_rows_in_several_lanes_give_the_bits_of_each_alone(F, lens):
-    """Either side of the three rows in all from which several lanes' rows are quantised by a kernel of their own, and the next window from the states that these leave."""
-    cfg = _small_config(F)
+@pytest.mark.parametrize("nv,lens", [(4, [1, 1]), (4, [1, 2]), (4, [2, 1]), (4, [1, 1, 1]), (4, [2, 2]), (4, [4, 4]), (4, [5, 4]), (64, [1, 2, 1, 1]), (64, [1, 2, 1, 1, 1])])
+def test_rows_in_several_lanes_give_the_bits_of_each_alone(F, nv, lens):
+    """On either side of the eight rows in all, and of the 128 clusters (value heads / 2 x lanes), beyond which the rows are quantised by a kernel of their own; and the next window from the
+    states that these leave."""
+    cfg = _small_config(F, nv)
     eng = F.Engine(cfg)
     try:
         eng.init_synthetic(seed=0, sigma=0.02)
-        toks = np.random.default_rng(1).integers(0, cfg.vocab, size=8).tolist()
+        toks = np.random.default_rng(1).integers(0, cfg.vocab, size=10).tolist()
         logits = eng.tensor("buf.logits", torch.float32).view(cfg.max_rows, cfg.vocab)
-        for s in range(4):
+        for s in range(6):
             eng.reset(s)
         eng.verify(toks, seq=0)
-        together, seqs, at = logits[:8].clone(), [3, 1, 2][:len(lens)], [0] * len(lens)
+        together, seqs, at = logits[:10].clone(), [3, 1, 2, 5, 4][:len(lens)], [0] * len(lens)
         for _ in range(2):
             eng.verify_lanes_rows(seqs, [toks[a:a + n] for a, n in zip(at, lens)])
             want = torch.cat([together[a:a + n] for a, n in zip(at, lens)])
@@ -67,7 +68,7 @@ def test_few_rows_in_several_lanes_give_the_bits_of_each_alone(F, lens):
 
 @pytest.mark.parametrize("T", [8, 9, 12])
 def test_a_row_of_an_engine_gives_the_same_bits_in_wide_windows(F, T):
-    """A sequence alone, on either side of the row count from which the output projection's rows are quantised by a kernel of their own; two lanes, by that kernel."""
+    """On either side of the eight rows beyond which the output projection's rows are quantised by a kernel of their own, alone and in two lanes."""
     cfg = _small_config(F)
     eng = F.Engine(cfg)
     try:
