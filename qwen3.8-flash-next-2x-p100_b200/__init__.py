@@ -318,7 +318,8 @@ def moe_experts(Wgu, Wdn, Wsh_gu, Wsh_dn, route, x, F: int, K: int, norm_w=None,
     h = new((P, F), dtype=torch.float32, device=x.device)
     part = new((P, H), dtype=torch.float32, device=x.device)
     out = torch.empty((T, H), dtype=torch.float32, device=x.device)
-    # (one call for the three launches: a block of one row 58.7 us with three, 56.4 with one; of five 60.1 and 58.4; from twelve rows on the kernels take longer than either)
+    # (one call for the three launches: the host's way through routing and experts 55.5 us with three, 52.5 with one.  Blocks of one row, which the host paces (33 on the device),
+    # 57.6 and 54.6 us; of five (55 on the device) 59.0 and 57.3; of eight and more (70) the same)
     check(lib().fnx_moe_experts(Wgu.data_ptr(), gu_stride, Wdn.data_ptr(), dn_stride, e_base, _at(Wsh_gu), _at(Wsh_dn), route["jobs"].data_ptr(), route["njobs"].data_ptr(),
                                 route["njobs_max"], route["topi"].data_ptr(), route["topw"].data_ptr(), route["logits"].data_ptr(), x.data_ptr(), _at(norm_w), eps, T, E, H, F, K,
                                 e_lo, e_hi, 1 if add_shared else 0, h.data_ptr(), part.data_ptr(), out.data_ptr(), route["err"].data_ptr(), _raw_stream()))

@@ -47,10 +47,12 @@ __device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
 // takes from the state are summed as the state is updated.  The first four rows' conv and norms are everybody's; warps 4 .. 7 go on with the rest, four
 // rows at a time, ahead of the rule.  The starting state, the history, the constants and a tree's paths depend on no kernel of this window: they are loaded before
 // the projections are waited for.
-// Bound by latency at a few rows (the loads, the chain, the exchange over the cluster); at many by the chain and the states' way out one after the other, 520 cycles a row
-// of 16 KB at an SM's 32 bytes a cycle.  us a launch, 1, 5, 8 and 20 rows and a tree of 20, in the form before (columns eight a warp, sums by shuffles, all of the conv
-// ahead of the rule) and here: 4.5 8.8 11.6 24.6 28.2, 4.3 8.0 10.6 18.7 19.4.  Tried here: the states out of shared memory by tensor copies (20 rows 20 to 23), eight
-// warps for the rule and eight for the conv (19.0), an SM to each block (16 clusters of eight do not fit at once: 35).
+// Bound by latency at a few rows (the loads, the chain, the exchange over the cluster); at many by the rule.  By its clocks, 32 value heads (a block an SM), a row's 0.72 us between 12
+// and 32 rows are 1,000 cycles of the rule and 0.2 us ahead of it and behind it; of the rule's some 590 lie in the update with the states' stores (16 KB at an SM's 32 bytes a
+// cycle; 250 in a copy without the stores, whose row takes 880), some 400 in the totals, their exchange and the next row's loads, 45 in the wait for the conv.
+// us a launch, 1, 5, 8 and 20 rows and a tree of 20, in the form before (columns eight a warp, sums by shuffles, all of the conv ahead of the rule) and here: 4.5 8.8 11.6 24.6
+// 28.2, 4.3 8.0 10.6 18.7 19.4.  Tried here: the states out of shared memory by tensor copies (20 rows 20 to 23), eight warps for the rule and eight for the conv (19.0), an SM
+// to each block (16 clusters of eight do not fit at once: 35).
 constexpr int GDN_BATCH = 4, GDN_CHANS = 2 * GDN_HS + GDN_QC;
 
 __host__ __device__ constexpr bool gdn_staged(int T, bool tree) { return tree || T > GDN_BATCH; }
@@ -447,8 +449,9 @@ constexpr int GC_BV = 0, GC_BK = 8, GC_BQ = 16, GC_BC = 24, GC_M = 28, GC_FLOATS
 // of v.  Rows past T become zeros (their coefficients leave the state as it is).  xq / xk [8 groups][nk][HS], xv / xc [..][nv][HS].
 // Bound by instructions (the conv's exponentials and divisions; of a key head's the dots of the pairs j <= i alone, a row's norm over a warp in nine shuffles for all
 // eight rows) and the chain of a block's four barriers, which the gates' loads and exponentials no longer lie in; a row's inputs are read by one block, eight rows and three before them at a time.
-// Six blocks an SM, by 40 registers a thread: 333, 3,001 and 38,912 rows 13.9, 77.8, 921 us, at 64 registers 14.5, 93.0, 1,109, at 32 (with spills) 14.4, 79.2, 954; with all pairs' dots, 40
-// shuffles for the norms and the gates behind the dots 15.6, 100.5, 1,226.  The conv and the norms alone take 750 of them, the bytes 490.
+// Six blocks an SM, by 40 registers a thread: 333, 3,001 and 38,912 rows 10.9, 73.6, 916 us, at 64 registers 12.3, 91.6, 1,183, at 32 (with spills) 11.8, 74.9, 925.  One by one: with all
+// pairs' dots 11.8, 78.2, 970; with 40 shuffles for the norms 11.7, 77.4, 960; with the gates behind the dots 11.2, 76.1, 956; with two loops for the gates' products 11.2, 75.4,
+// 935; with none of these and no bound on the registers 13.4, 98.5, 1,243.  The conv and the norms alone take 750 of the 916, the bytes 490.
 __global__ void __launch_bounds__(GDP_THREADS, 6) k_gdn_pre(const float* __restrict__ qkvz, int stride, const float* __restrict__ ab, int ldab,
                                                          const float* __restrict__ hin, float* __restrict__ hout, const float* __restrict__ convw,
                                                          const float* __restrict__ dt, const float* __restrict__ a_, float* __restrict__ xq,

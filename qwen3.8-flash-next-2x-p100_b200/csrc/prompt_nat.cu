@@ -18,10 +18,10 @@
 // Tensor memory: columns [0, 256) two pairs of accumulators, [256, 512) two stages of two 128 x 128 weight tiles.  Jobs have at most 64 rows, and
 // the products' N is a job's own rows in sixteens (six rows a job: 178 us with N = 64, 166).  Jobs of 128 rows halve the decode, but leave one
 // accumulator pair, whose results (6 us an item) then lie in the next item's way: 388 us for 512 jobs of 116 rows, 339 for 1,024 of 58.
-// Measured, 512 jobs of gate|up and of down (fourteen items of 256 features x 2,048 columns an SM), us: six rows a job 162 + 92, fifty-eight 179 + 115, 6,144 jobs
-// of 760 rows an expert 1,940 + 1,244 (187 + 101, 200 + 126 and 2,172 + 1,334 with four stages of rows, N = 64 and two instructions a word more); in a prompt of 333 rows, ten picks
-// a row, 150 + 83 a layer, 147 + 80 with the weights' stores of shape 16x128b.  By its clocks a down chunk of 128 columns takes 1,430 cycles there and 1,630 at 20,000 rows: a decode warp
-// waits 200 of them for a free stage and works the rest (13 instructions a word, half and integer-logic ones at two cycles each on pipes that overlap by half), the issuing thread waits
+// Measured, gate|up and down of a layer of a prompt (512 experts, ten picks a row: 512 jobs of up to 64 rows are fourteen items of 256 features x 2,048 columns an SM), us: 307 rows
+// (six an expert) 147 + 79, 2,970 (58) 261 + 149, 38,912 (760, 64 a job) 2,423 + 1,430; with the weights' stores of shape 16x256b 151 + 82, 266 + 153, 2,497 + 1,432 (before these, jobs alone of six, 58 and 760 rows an
+// expert: 187 + 101, 200 + 126 and 2,172 + 1,334 with four stages of rows, N = 64 and two instructions a word more, 162 + 92, 179 + 115 and 1,940 + 1,244 without).  By its clocks a down
+// chunk of 128 columns takes 1,430 cycles at 333 rows and 1,630 at 20,000: a decode warp waits 200 of them for a free stage and works the rest (13 instructions a word, half and integer-logic ones at two cycles each on pipes that overlap by half), the issuing thread waits
 // 410 to 530 for the weights.  DRAM would allow 88.
 #include <type_traits>
 
